@@ -15,6 +15,7 @@
 #include "assign_reg.cuh"
 #include "dense_tc.hpp"
 #include "opq_tc.hpp"
+#include "ordered_sums.cuh"
 #include "pq_tc.hpp"
 #include "kernels_common.cuh"
 
@@ -1159,8 +1160,8 @@ __global__ void __launch_bounds__(256) accum_rows_moved_kernel(const float *__re
     }
 }
 
-// ORDERED: one thread per (cluster, dimension) walks all rows in ascending order and adds the members
-// of its cluster, which is exactly the serial branch of mean_vector (src/vector.rs:305-313).
+// ORDERED, more clusters than ordered_sums.cu takes: one thread per (cluster, dimension) walks all rows in ascending order
+// and adds the members of its cluster, which is exactly the serial branch of mean_vector (src/vector.rs:305-313).
 template <typename CodeT>
 __global__ void __launch_bounds__(256) accum_ordered_kernel(const float *x, unsigned long long n, unsigned long long ld, int m,
                                                             int k, int sd, const CodeT *codes, const uint32_t *active,
@@ -1338,6 +1339,10 @@ void CudaDevice::accumulate(const Shape &sh, const float *x, const void *codes, 
     // the buffer arrives zero-filled (update_centroids clears what it has read); the ordered kernel overwrites every entry
     const size_t cb = code_bytes(sh.k);
     const int cf = buf.counts_f32 ? 1 : 0;
+    if (ordered && ordered_sums_applicable(sh.k)) {
+        launch_ordered_sums(*this, sh, x, codes, cb, active, buf.sums, buf.counts, buf.counts_f32);
+        return;
+    }
     if (cb == 1) accumulate_t<uint8_t>(*this, sh, x, (const uint8_t *)codes, active, ordered, buf.sums, buf.counts, cf);
     else if (cb == 2) accumulate_t<uint16_t>(*this, sh, x, (const uint16_t *)codes, active, ordered, buf.sums, buf.counts, cf);
     else accumulate_t<uint32_t>(*this, sh, x, (const uint32_t *)codes, active, ordered, buf.sums, buf.counts, cf);

@@ -1,0 +1,236 @@
+// ordered_sums.cu -- cluster sums in ascending row order, as the reference's serial mean adds them (src/vector.rs:305-313).
+//
+// The order fixes the additions of one cluster, not the search for its rows.  So the rows are first sorted by cluster with a
+// stable counting sort (two passes over the codes), and then every cluster walks its own list:
+//   ordered_hist_kernel     rows per (chunk of rows, cluster)
+//   ordered_lists_kernel    where each chunk's rows of a cluster start, then the row numbers themselves, ascending
+//   ordered_sums_kernel     one lane per (cluster, dimension) adds the cluster's rows in list order
+// The work is O(n) per sub-space.  Walking all n codes once per (cluster, dimension), as this did before, cost 0.44 ms per pass
+// at 10,000 x 128, m 16, k 256 and 1.5 ms at 33,506 x 128, k 62; three launches of this file take ~0.02 ms and ~0.05 ms.
+#include <algorithm>
+
+#include "cuda_device.hpp"
+#include "ordered_sums.cuh"
+
+namespace vqb {
+
+namespace {
+
+constexpr int OL_WARPS = 8, OL_THREADS = 32 * OL_WARPS;
+constexpr unsigned OL_STEP = 1024;   // a chunk is a multiple of this many rows
+constexpr unsigned OL_CHUNKS = 64;   // at most about this many chunks: every list CTA reads the counts of all of them
+constexpr int OL_MAX_K = 4096;       // counters of eight warps in shared memory: 128 KiB
+constexpr int OS_WARPS = 4, OS_BATCH = 8, OS_RING = 8; // 64 rows in flight per warp, 8 KiB of shared memory each
+
+template <typename CodeT>
+__global__ void __launch_bounds__(OL_THREADS) ordered_hist_kernel(const CodeT *__restrict__ codes, unsigned n, unsigned chunk, int m, int k,
+                                                                  const uint32_t *active, uint32_t *__restrict__ hist)
+{
+    extern __shared__ uint32_t s_cnt[]; // [k]
+    const int s = blockIdx.y;
+    if (active && active[s] == 0) return;
+    for (int j = threadIdx.x; j < k; j += OL_THREADS) s_cnt[j] = 0u;
+    __syncthreads();
+    const unsigned r0 = blockIdx.x * chunk, r1 = min(n, r0 + chunk);
+    for (unsigned r = r0 + threadIdx.x; r < r1; r += OL_THREADS) atomicAdd(s_cnt + (unsigned)codes[(size_t)r * m + s], 1u);
+    __syncthreads();
+    uint32_t *h = hist + ((size_t)s * gridDim.x + blockIdx.x) * k;
+    for (int j = threadIdx.x; j < k; j += OL_THREADS) h[j] = s_cnt[j];
+}
+
+// One CTA per (chunk, sub-space).  A warp owns a contiguous eighth of the chunk, so ranking by (earlier chunks, earlier warps of
+// the CTA, earlier steps of the warp, lower lanes) is ranking by row number.
+template <typename CodeT>
+__global__ void __launch_bounds__(OL_THREADS) ordered_lists_kernel(const CodeT *__restrict__ codes, unsigned n, unsigned chunk, int m, int k,
+                                                                   const uint32_t *active, const uint32_t *__restrict__ hist,
+                                                                   uint32_t *__restrict__ start, uint32_t *__restrict__ list)
+{
+    extern __shared__ uint32_t s_at[]; // [OL_WARPS][k]: counts, then the next free place of each list
+    __shared__ uint32_t s_part[OL_WARPS];
+    const int s = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (active && active[s] == 0) return;
+    const unsigned nchunks = gridDim.x, c = blockIdx.x;
+    const unsigned per = chunk / OL_WARPS, w0 = c * chunk + warp * per, w1 = min(n, w0 + per);
+    for (int t = threadIdx.x; t < OL_WARPS * k; t += OL_THREADS) s_at[t] = 0u;
+    __syncthreads();
+    uint32_t *mine = s_at + warp * k;
+    for (unsigned r = w0 + lane; r < w1; r += 32) atomicAdd(mine + (unsigned)codes[(size_t)r * m + s], 1u);
+    __syncthreads();
+    // thread t: clusters t * jt .. t * jt + jt - 1
+    const int jt = (k + OL_THREADS - 1) / OL_THREADS, j0 = threadIdx.x * jt;
+    uint32_t total = 0;
+    for (int j = j0; j < min(k, j0 + jt); ++j) {
+        const uint32_t *h = hist + (size_t)s * nchunks * k + j;
+#pragma unroll 8
+        for (unsigned q = 0; q < nchunks; ++q) total += h[(size_t)q * k];
+    }
+    uint32_t incl = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_part[warp] = incl;
+    __syncthreads();
+    uint32_t at = incl - total;
+    for (int w = 0; w < warp; ++w) at += s_part[w];
+    for (int j = j0; j < min(k, j0 + jt); ++j) {
+        if (c == 0) start[(size_t)s * (k + 1) + j] = at;
+        const uint32_t *h = hist + (size_t)s * nchunks * k + j;
+        uint32_t before = 0, all = 0;
+#pragma unroll 8
+        for (unsigned q = 0; q < nchunks; ++q) {
+            const uint32_t v = h[(size_t)q * k];
+            all += v;
+            before += q < c ? v : 0u;
+        }
+        uint32_t place = at + before;
+        for (int w = 0; w < OL_WARPS; ++w) {
+            const uint32_t cnt = s_at[w * k + j];
+            s_at[w * k + j] = place;
+            place += cnt;
+        }
+        at += all;
+    }
+    if (c == 0 && threadIdx.x == 0) start[(size_t)s * (k + 1) + k] = n;
+    __syncthreads();
+    uint32_t *out = list + (size_t)s * n;
+    for (unsigned r = w0 + lane; r < ((w1 + 31) & ~31u); r += 32) { // per and w0 are multiples of 32: whole warps
+        const bool in = r < w1;
+        const uint32_t code = in ? (uint32_t)codes[(size_t)r * m + s] : 0xFFFFFFFFu;
+        const unsigned same = __match_any_sync(0xffffffffu, code);
+        const int rank = __popc(same & ((1u << lane) - 1u));
+        uint32_t place = 0;
+        if (in) place = mine[code] + rank;
+        __syncwarp();
+        if (in) {
+            out[place] = r;
+            if (rank == 0) mine[code] += __popc(same);
+        }
+        __syncwarp();
+    }
+}
+
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// A warp takes 32 / W clusters side by side, W lanes each (W: the power of two that covers the width, at most 32; wider rows
+// are cut into pieces of 32).  The additions of a cluster are one dependent chain, so what counts is that its rows are there
+// in time: 64 of them travel through a shared-memory ring per warp while the chain consumes earlier ones, and the row numbers
+// are read one batch further ahead.
+template <int W>
+__global__ void __launch_bounds__(32 * OS_WARPS) ordered_sums_kernel(const float *__restrict__ x, unsigned n, unsigned long long ld, int m, int k, int sd,
+                                                                     const uint32_t *active, const uint32_t *__restrict__ start,
+                                                                     const uint32_t *__restrict__ list, float *sums, uint32_t *counts, int counts_f32)
+{
+    __shared__ float ring[OS_WARPS][OS_RING][OS_BATCH][32];
+    const int s = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (active && active[s] == 0) return;
+    const int pieces = (sd + 31) / 32; // 1 unless W == 32
+    const int unit = blockIdx.x * OS_WARPS + warp;
+    const int j = (unit / pieces) * (32 / W) + lane / W, d = (unit % pieces) * 32 + lane % W;
+    uint32_t b = 0, len = 0;
+    if (j < k) {
+        b = start[(size_t)s * (k + 1) + j];
+        len = start[(size_t)s * (k + 1) + j + 1] - b;
+    }
+    const uint32_t rows = d < sd ? len : 0u;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, rows);
+    const uint32_t batches = (most + OS_BATCH - 1) / OS_BATCH;
+    const uint32_t *l = list + (size_t)s * n + b;
+    const float *xs = x + (size_t)s * sd + d;
+    float(*buf)[OS_BATCH][32] = ring[warp];
+    uint32_t idx[OS_BATCH];
+    auto fetch_idx = [&](uint32_t batch) {
+#pragma unroll
+        for (int i = 0; i < OS_BATCH; ++i) idx[i] = batch * OS_BATCH + i < rows ? __ldg(l + batch * OS_BATCH + i) : 0u;
+    };
+    auto issue = [&](uint32_t batch) { // always closes a group, so that the count of pending groups stays fixed
+#pragma unroll
+        for (int i = 0; i < OS_BATCH; ++i)
+            if (batch * OS_BATCH + i < rows)
+                cp_async4((uint32_t)__cvta_generic_to_shared(&buf[batch % OS_RING][i][lane]), xs + (size_t)idx[i] * ld);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch_idx(0);
+#pragma unroll 1
+    for (uint32_t p = 0; p + 1 < OS_RING; ++p) {
+        issue(p);
+        fetch_idx(p + 1);
+    }
+    float acc = 0.0f;
+#pragma unroll 1
+    for (uint32_t t = 0; t < batches; ++t) {
+        issue(t + OS_RING - 1);
+        fetch_idx(t + OS_RING);
+        asm volatile("cp.async.wait_group %0;" ::"n"(OS_RING - 1) : "memory"); // a lane reads only what it copied itself
+        float v[OS_BATCH];
+#pragma unroll
+        for (int i = 0; i < OS_BATCH; ++i) v[i] = buf[t % OS_RING][i][lane];
+#pragma unroll
+        for (int i = 0; i < OS_BATCH; ++i)
+            if (t * OS_BATCH + i < rows) acc = __fadd_rn(acc, v[i]);
+    }
+    if (j < k && d < sd) {
+        sums[((size_t)s * k + j) * sd + d] = acc;
+        if (d == 0) counts[(size_t)s * k + j] = counts_f32 ? __float_as_uint((float)len) : len;
+    }
+}
+
+} // namespace
+
+bool ordered_sums_applicable(size_t k) { return k <= (size_t)OL_MAX_K; }
+
+template <typename CodeT>
+static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const CodeT *codes, const uint32_t *active, float *sums, uint32_t *counts,
+                     int counts_f32)
+{
+    const unsigned n = (unsigned)sh.n_local;
+    const int m = (int)sh.m, k = (int)sh.k, sd = (int)sh.sd;
+    const unsigned chunk = std::max(1u, ((n + OL_CHUNKS - 1) / OL_CHUNKS + OL_STEP - 1) / OL_STEP) * OL_STEP;
+    const unsigned chunks = std::max(1u, (n + chunk - 1) / chunk);
+    const size_t hist_words = (size_t)m * chunks * k, start_words = (size_t)m * (k + 1), list_words = (size_t)m * n;
+    uint32_t *work = static_cast<uint32_t *>(dev.alloc((hist_words + start_words + list_words) * sizeof(uint32_t)));
+    uint32_t *hist = work, *start = hist + hist_words, *list = start + start_words;
+    {
+        KernelScope ks(dev, "ordered_lists");
+        const size_t smem = sizeof(uint32_t) * k;
+        ordered_hist_kernel<CodeT><<<dim3(chunks, m), OL_THREADS, smem, dev.stream()>>>(codes, n, chunk, m, k, active, hist);
+        VQB_CUDA_CHECK(cudaGetLastError());
+        dev.count_launch();
+        auto kernel = ordered_lists_kernel<CodeT>;
+        if (OL_WARPS * smem > 48 * 1024)
+            VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(OL_WARPS * smem)));
+        kernel<<<dim3(chunks, m), OL_THREADS, OL_WARPS * smem, dev.stream()>>>(codes, n, chunk, m, k, active, hist, start, list);
+        VQB_CUDA_CHECK(cudaGetLastError());
+        dev.count_launch();
+    }
+    {
+        KernelScope ks(dev, "ordered_sums");
+        const int w = sd <= 4 ? 4 : sd <= 8 ? 8 : sd <= 16 ? 16 : 32;
+        const size_t units = ((size_t)k + 32 / w - 1) / (32 / w) * ((sd + 31) / 32);
+        const dim3 grid((unsigned)((units + OS_WARPS - 1) / OS_WARPS), m);
+        auto go = [&](auto kernel) {
+            kernel<<<grid, 32 * OS_WARPS, 0, dev.stream()>>>(x, n, sh.ld, m, k, sd, active, start, list, sums, counts, counts_f32);
+        };
+        if (w == 4) go(ordered_sums_kernel<4>);
+        else if (w == 8) go(ordered_sums_kernel<8>);
+        else if (w == 16) go(ordered_sums_kernel<16>);
+        else go(ordered_sums_kernel<32>);
+        VQB_CUDA_CHECK(cudaGetLastError());
+        dev.count_launch();
+    }
+    dev.release(work);
+}
+
+void launch_ordered_sums(CudaDevice &dev, const Shape &sh, const float *x, const void *codes, size_t code_bytes, const uint32_t *active, float *sums,
+                         uint32_t *counts, bool counts_f32)
+{
+    const int cf = counts_f32 ? 1 : 0;
+    if (code_bytes == 1) launch_t(dev, sh, x, static_cast<const uint8_t *>(codes), active, sums, counts, cf);
+    else launch_t(dev, sh, x, static_cast<const uint16_t *>(codes), active, sums, counts, cf);
+}
+
+} // namespace vqb
