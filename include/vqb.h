@@ -267,6 +267,19 @@ int vqb_bq_fit(float threshold, uint8_t low, uint8_t high);
 int vqb_bq_quantize(vqb_ctx *ctx, float threshold, uint8_t low, uint8_t high, const float *x,
                     size_t n_elems, uint8_t *out);
 
+/* ---- stand-in row sampler ----------------------------------------------- */
+/* For hosts without the reference's StdRng: one SplitMix64 stream per LBG call, seeded `seed + stream` (src/pq.rs:119).
+ * vqb_seeder_sample draws the initial rows of `streams` sub-spaces (streams x k indices); the other three are a
+ * vqb_draw_fn, vqb_init_fn and vqb_restart_fn whose `user` is the seeder.  The restart returns every stream to where its
+ * initial sample left it (src/opq.rs:140). */
+typedef struct vqb_seeder vqb_seeder;
+int vqb_seeder_create(uint64_t seed, vqb_seeder **out);
+int vqb_seeder_destroy(vqb_seeder *sd);
+int vqb_seeder_sample(vqb_seeder *sd, size_t streams, uint64_t n, size_t k, uint64_t *idx_out);
+uint64_t vqb_seeder_draw(void *seeder, size_t stream, uint64_t n);
+void vqb_seeder_init(void *seeder, size_t stage, uint64_t n, size_t k, uint64_t *idx_out);
+void vqb_seeder_restart(void *seeder);
+
 #ifdef __cplusplus
 }
 #endif

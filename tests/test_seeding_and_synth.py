@@ -1,5 +1,6 @@
 """Host logic: the stand-in sampler, shard arithmetic and the synthetic generators."""
 import numpy as np
+import pytest
 
 from vq_b200 import synth
 from vq_b200.distributed import owner_of, shard_bounds
@@ -57,3 +58,20 @@ def test_other_generators_shapes():
     assert c.shape == (500, 8) and np.isfinite(c).all()
     z = synth.normal(20000, 4, 9)
     assert abs(float(z.mean())) < 0.03 and abs(float(z.std()) - 1.0) < 0.03
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (7, 7), (300, 256), (1_000_000, 256)])
+def test_native_seeder_draws_what_the_python_definition_draws(n, k):
+    import ctypes as C
+
+    from vq_b200 import _lib
+    lib, sd, ref = _lib.load(), C.c_void_p(), LbgSeeder(2**64 - 2)  # seed + stream wraps
+    assert lib.vqb_seeder_create(2**64 - 2, C.byref(sd)) == 0
+    idx = np.zeros((3, k), np.uint64)
+    assert lib.vqb_seeder_sample(sd, 3, n, k, idx.ctypes.data) == 0
+    assert np.array_equal(idx, np.stack([ref.init_indices(s, n, k) for s in range(3)]))
+    draws = [lib.vqb_seeder_draw(sd, s, n) for s in (0, 0, 2, 5)]
+    assert draws == [ref.draw(s, n) for s in (0, 0, 2, 5)]
+    lib.vqb_seeder_restart(sd)
+    assert [lib.vqb_seeder_draw(sd, 0, n), lib.vqb_seeder_draw(sd, 0, n)] == draws[:2]
+    lib.vqb_seeder_destroy(sd)

@@ -308,8 +308,27 @@ def _rows(training_data, ctx):
     return arr
 
 
-def _make_draw(seeder: LbgSeeder):
-    return _lib.DRAW_FN(lambda user, stream, n: seeder.draw(int(stream), int(n)))
+class _Seeder:
+    """The draws of one fit.  Without the caller's own callbacks they come from the library's copy of the stand-in sampler
+    (same numbers as seeding.LbgSeeder), so that no call of the training loop enters Python."""
+
+    def __init__(self, seed: int):
+        self._L = _lib.load()
+        self.handle = C.c_void_p()
+        self._L.vqb_seeder_create(int(seed) & 0xFFFFFFFFFFFFFFFF, C.byref(self.handle))
+
+    def sample(self, streams: int, n: int, k: int) -> np.ndarray:
+        """Initial rows, streams x k; zeros for a request that the fit is about to refuse."""
+        out = np.zeros((max(streams, 1), max(k, 1)), np.uint64)
+        if streams > 0 and 0 < k <= n:
+            self._L.vqb_seeder_sample(self.handle, streams, n, k, out.ctypes.data)
+        return out
+
+    def draw_fn(self, draw=None):
+        return _lib.DRAW_FN(lambda user, stream, n: int(draw(int(stream), int(n)))) if draw else _lib.SEEDER_DRAW
+
+    def __del__(self):
+        self._L.vqb_seeder_destroy(self.handle)
 
 
 def _global_rows(n_local: int, ctx: Context) -> int:
@@ -338,16 +357,12 @@ class ProductQuantizer:
         L = _lib.load()
         x = _rows(training_data, ctx)
         n_global = _global_rows(x.n, ctx)
-        seeder = LbgSeeder(seed)
-        if init_idx is None:
-            ok = m > 0 and 0 < k <= n_global
-            init_idx = (np.stack([seeder.init_indices(i, n_global, k) for i in range(m)]) if ok
-                        else np.zeros((max(m, 1), max(k, 1)), np.uint64))
-        init_idx = np.ascontiguousarray(init_idx, dtype=np.uint64)
-        cb = _lib.DRAW_FN(lambda user, stream, n: int(draw(int(stream), int(n)))) if draw else _make_draw(seeder)
+        seeder = _Seeder(seed)
+        init_idx = seeder.sample(m, n_global, k) if init_idx is None else np.ascontiguousarray(init_idx, dtype=np.uint64)
+        cb = seeder.draw_fn(draw)
         h = C.c_void_p()
         rc = L.vqb_pq_fit(ctx.handle, x.ptr, x.n, x.dim, m, k, max_iters, distance.metric, distance.p,
-                          init_idx.ctypes.data, cb, None, accumulate, C.byref(h))
+                          init_idx.ctypes.data, cb, seeder.handle, accumulate, C.byref(h))
         if rc:
             _raise(rc, ctx.handle)
         return cls(h, ctx, distance)
@@ -419,18 +434,18 @@ class ResidualQuantizer:
         """ResidualQuantizer::fit (src/rvq.rs:87-154).  ``init(stage, n, k)`` overrides the seeded stand-in."""
         ctx = ctx or default_context()
         x = _rows(training_data, ctx)
-        seeder = LbgSeeder(seed)
+        seeder = _Seeder(seed)
 
         def _init(user, stage, n, kk, out):
-            idx = init(int(stage), int(n), int(kk)) if init else seeder.init_indices(int(stage), int(n), int(kk))
+            idx = init(int(stage), int(n), int(kk))
             for j in range(int(kk)):
                 out[j] = int(idx[j])
 
-        icb = _lib.INIT_FN(_init)
-        dcb = _lib.DRAW_FN(lambda user, stream, n: int(draw(int(stream), int(n)))) if draw else _make_draw(seeder)
+        icb = _lib.INIT_FN(_init) if init else _lib.SEEDER_INIT
+        dcb = seeder.draw_fn(draw)
         h = C.c_void_p()
         rc = _lib.load().vqb_rvq_fit(ctx.handle, x.ptr, x.n, x.dim, stages, k, max_iters, float(epsilon),
-                                     distance.metric, distance.p, icb, dcb, None, accumulate, C.byref(h))
+                                     distance.metric, distance.p, icb, dcb, seeder.handle, accumulate, C.byref(h))
         if rc:
             _raise(rc, ctx.handle)
         return cls(h, ctx, distance)
@@ -496,31 +511,13 @@ class OptimizedProductQuantizer:
         ctx = ctx or default_context()
         x = _rows(training_data, ctx)
         n_global = _global_rows(x.n, ctx)
-        state = {"seeder": LbgSeeder(seed)}
-        ok = m > 0 and 0 < k <= n_global
-        user_idx = init_idx is not None
-        if init_idx is None:
-            init_idx = (np.stack([state["seeder"].init_indices(i, n_global, k) for i in range(m)]) if ok
-                        else np.zeros((max(m, 1), max(k, 1)), np.uint64))
-        init_idx = np.ascontiguousarray(init_idx, dtype=np.uint64)
-
-        # every outer iteration re-creates StdRng(seed + i) (src/opq.rs:140): same sample, same draws.  The streams' states
-        # right after the initial sample are the same every time, so they are recorded once and restored (drawing the
-        # 16 x 256 sample again in Python cost 2.4 ms per outer iteration of the benchmark configuration).
-        after_init = {st: r.state for st, r in state["seeder"].rngs.items()} if ok and not user_idx else {}
-
-        def _restart(user):
-            state["seeder"] = LbgSeeder(seed)
-            for st, value in after_init.items():
-                rng = StandInRng(0)
-                rng.state = value
-                state["seeder"].rngs[st] = rng
-
-        rcb = _lib.RESTART_FN(_restart)
-        dcb = _lib.DRAW_FN(lambda user, stream, n: state["seeder"].draw(int(stream), int(n)))
+        # every outer iteration re-creates StdRng(seed + i) (src/opq.rs:140): same sample, same draws
+        seeder = _Seeder(seed)
+        init_idx = seeder.sample(m, n_global, k) if init_idx is None else np.ascontiguousarray(init_idx, dtype=np.uint64)
         h = C.c_void_p()
         rc = _lib.load().vqb_opq_fit(ctx.handle, x.ptr, x.n, x.dim, m, k, max_iters, opq_iters, distance.metric,
-                                     distance.p, init_idx.ctypes.data, dcb, rcb, None, accumulate, C.byref(h))
+                                     distance.p, init_idx.ctypes.data, seeder.draw_fn(), _lib.SEEDER_RESTART, seeder.handle, accumulate,
+                                     C.byref(h))
         if rc:
             _raise(rc, ctx.handle)
         return cls(h, ctx, distance, x.dim)
@@ -709,14 +706,12 @@ def lbg_quantize(data, k: int, max_iters: int, seed: int, *, ctx: Context | None
     """lbg_quantize (src/utils.rs:32-109) on n x d rows.  Returns (centroids k x d, iterations)."""
     ctx = ctx or default_context()
     x = _rows(data, ctx)
-    seeder = LbgSeeder(seed)
-    if init_idx is None:
-        init_idx = seeder.init_indices(0, x.n, k) if 0 < k <= x.n else np.zeros(max(k, 1), np.uint64)
-    init_idx = np.ascontiguousarray(init_idx, dtype=np.uint64)
-    cb = _lib.DRAW_FN(lambda user, stream, n: int(draw(int(stream), int(n)))) if draw else _make_draw(seeder)
+    seeder = _Seeder(seed)
+    init_idx = seeder.sample(1, x.n, k) if init_idx is None else np.ascontiguousarray(init_idx, dtype=np.uint64)
+    cb = seeder.draw_fn(draw)
     out = np.empty((k, x.dim), np.float32)
     iters = C.c_size_t(0)
-    rc = _lib.load().vqb_lbg_fit(ctx.handle, x.ptr, x.n, x.dim, k, max_iters, init_idx.ctypes.data, cb, None,
+    rc = _lib.load().vqb_lbg_fit(ctx.handle, x.ptr, x.n, x.dim, k, max_iters, init_idx.ctypes.data, cb, seeder.handle,
                                  accumulate, out.ctypes.data if out.size else None, C.byref(iters))
     if rc:
         _raise(rc, ctx.handle)

@@ -78,14 +78,22 @@ SIGNATURES = {
     "vqb_sq_quantize": (C.c_int, [_P, C.c_float, C.c_float, _SZ, C.c_float, _P, _SZ, _P]),
     "vqb_bq_fit": (C.c_int, [C.c_float, C.c_uint8, C.c_uint8]),
     "vqb_bq_quantize": (C.c_int, [_P, C.c_float, C.c_uint8, C.c_uint8, _P, _SZ, _P]),
+    "vqb_seeder_create": (C.c_int, [C.c_uint64, C.POINTER(_P)]),
+    "vqb_seeder_destroy": (C.c_int, [_P]),
+    "vqb_seeder_sample": (C.c_int, [_P, _SZ, C.c_uint64, _SZ, _P]),
+    "vqb_seeder_draw": (C.c_uint64, [_P, _SZ, C.c_uint64]),
+    "vqb_seeder_init": (None, [_P, _SZ, C.c_uint64, _SZ, _P]),
+    "vqb_seeder_restart": (None, [_P]),
 }
 
 _lib = None
+# the library's own vqb_draw_fn, vqb_init_fn and vqb_restart_fn (set by load(); their `user` is a vqb_seeder)
+SEEDER_DRAW = SEEDER_INIT = SEEDER_RESTART = None
 
 
 def load():
     """Load libvqb.so and attach the signatures.  Raises if it is not built."""
-    global _lib
+    global _lib, SEEDER_DRAW, SEEDER_INIT, SEEDER_RESTART
     if _lib is not None:
         return _lib
     if not os.path.exists(LIB_PATH):
@@ -97,5 +105,7 @@ def load():
         fn = getattr(L, name)  # AttributeError here means header and library disagree
         fn.restype = res
         fn.argtypes = args
+    SEEDER_DRAW, SEEDER_INIT = C.cast(L.vqb_seeder_draw, DRAW_FN), C.cast(L.vqb_seeder_init, INIT_FN)
+    SEEDER_RESTART = C.cast(L.vqb_seeder_restart, RESTART_FN)
     _lib = L
     return L
