@@ -13,6 +13,7 @@ There is no CPU path: every call fails if the library or a B200 is missing.
 from __future__ import annotations
 
 import ctypes as C
+import sys
 import threading
 
 import numpy as np
@@ -124,6 +125,8 @@ class Context:
         self.handle = h
         self.device = int(device)
         self.rank, self.world = 0, 1
+        self._stream = None   # what set_stream() was told last
+        self._pinned = False  # use_stream() holds the stream whatever the inputs are
 
     def close(self):
         if getattr(self, "handle", None):
@@ -142,6 +145,7 @@ class Context:
         rc = L.vqb_ctx_reset_stream(self.handle) if cuda_stream is None else L.vqb_ctx_set_stream(self.handle, C.c_void_p(cuda_stream))
         if rc:
             _raise(rc, self.handle)
+        self._stream = cuda_stream
 
     def synchronize(self):
         rc = _lib.load().vqb_ctx_synchronize(self.handle)
@@ -176,7 +180,6 @@ class Context:
         """Pin all work of this context to `cuda_stream` (e.g. torch.cuda.current_stream().cuda_stream), also for
         host-memory inputs; None returns to the default behaviour (caller's torch stream for CUDA tensors, the
         context's own stream for host arrays)."""
-        self._sticky = cuda_stream
         self._pinned = cuda_stream is not None
         self.set_stream(cuda_stream)
 
@@ -204,6 +207,12 @@ _default_lock = threading.Lock()
 
 
 def default_context(device: int | None = None) -> Context:
+    torch = sys.modules.get("torch")
+    if device is None and torch is not None and torch.cuda.is_initialized():
+        device = torch._C._cuda_getDevice()
+        ctx = _default.get(device)
+        if ctx is not None:
+            return ctx
     if device is None:
         device = 0
         try:
@@ -229,28 +238,43 @@ def unique_id() -> bytes:
 
 # ---- array plumbing -----------------------------------------------------------------------------
 def _is_torch(x) -> bool:
-    return type(x).__module__.startswith("torch")
+    torch = sys.modules.get("torch")
+    return torch is not None and isinstance(x, torch.Tensor)
+
+
+_TORCH_DTYPES = {}  # numpy scalar type -> torch dtype, filled on first use (torch is not imported before the caller has)
+
+
+def _torch_dtype(np_dtype):
+    if not _TORCH_DTYPES:
+        torch = sys.modules["torch"]
+        _TORCH_DTYPES.update({np.float16: torch.float16, np.uint8: torch.uint8, np.uint32: torch.int32, np.float32: torch.float32})
+    return _TORCH_DTYPES[np_dtype]
 
 
 class _Arr:
-    """A float32 C-contiguous view of the caller's data plus where outputs should live."""
+    """A float32 C-contiguous view of the caller's data plus where outputs should live.  One is made per call, and for a single
+    vector the call lasts as long as its host code does: no torch object is created that the result does not need, and the
+    context is told of a stream only when it is another than the last one."""
+
+    __slots__ = ("cuda", "keep", "shape", "ptr", "single", "n", "dim", "size")
 
     def __init__(self, x, ctx: Context, want_2d=True):
-        self.torch = None
         if isinstance(x, Vector):
             x = x.data
-        if _is_torch(x) and x.is_cuda:
-            import torch
-            self.torch = torch
-            t = x.detach()
-            if t.dtype != torch.float32 or not t.is_contiguous():
-                t = t.to(torch.float32).contiguous()
-            self.keep = t
-            self.shape = tuple(t.shape)
-            self.ptr = t.data_ptr()
-            self.device = t.device
-            if not getattr(ctx, "_pinned", False):
-                ctx.set_stream(torch.cuda.current_stream(t.device).cuda_stream)
+        torch = sys.modules.get("torch")
+        self.cuda = torch is not None and isinstance(x, torch.Tensor) and x.is_cuda
+        if self.cuda:
+            if x.dtype is not torch.float32 or not x.is_contiguous():
+                x = x.detach().to(torch.float32).contiguous()
+            self.keep = x
+            self.shape = x.shape
+            self.ptr = x.data_ptr()
+            self.size = x.numel()
+            if not ctx._pinned:
+                stream = torch._C._cuda_getCurrentRawStream(x.get_device())
+                if stream != ctx._stream:
+                    ctx.set_stream(stream)
         else:
             if _is_torch(x):
                 x = x.detach().cpu().numpy()
@@ -258,17 +282,17 @@ class _Arr:
             self.keep = a
             self.shape = a.shape
             self.ptr = a.ctypes.data
-            if not getattr(ctx, "_pinned", False):
+            self.size = a.size
+            if not ctx._pinned and ctx._stream is not None:
                 ctx.set_stream(None)
         self.single = len(self.shape) == 1
         if want_2d:
-            if len(self.shape) == 1:
+            if self.single:
                 self.n, self.dim = 1, self.shape[0]
             elif len(self.shape) == 2:
                 self.n, self.dim = self.shape
             else:
                 raise ValueError("expected a vector or a matrix of row vectors")
-        self.size = int(np.prod(self.shape)) if len(self.shape) else 1
 
     def empty(self, shape, np_dtype, out=None):
         """A fresh result of the input's kind, or the caller's `out`: a C-contiguous array of this shape and dtype that
@@ -277,22 +301,19 @@ class _Arr:
         if out is not None:
             want = tuple(int(v) for v in shape)
             if _is_torch(out):
-                tdt = {np.float16: "float16", np.uint8: "uint8", np.uint32: "int32", np.float32: "float32"}[np_dtype]
                 on_device = bool(out.is_cuda)
-                ok = tuple(out.shape) == want and str(out.dtype) == "torch." + tdt and out.is_contiguous()
+                ok = tuple(out.shape) == want and out.dtype is _torch_dtype(np_dtype) and out.is_contiguous()
                 ptr = out.data_ptr()
             else:
                 on_device = False
                 ok = isinstance(out, np.ndarray) and out.shape == want and out.dtype == np.dtype(np_dtype) and out.flags.c_contiguous \
                     and out.flags.writeable
                 ptr = out.ctypes.data if ok else 0
-            if not ok or on_device != (self.torch is not None):
+            if not ok or on_device != self.cuda:
                 raise ValueError(f"out must be a contiguous {np.dtype(np_dtype).name} array of shape {want} on the input's side")
             return out, ptr
-        if self.torch is not None:
-            tdt = {np.float16: self.torch.float16, np.uint8: self.torch.uint8, np.uint32: self.torch.int32,
-                   np.float32: self.torch.float32}[np_dtype]
-            t = self.torch.empty(shape, dtype=tdt, device=self.device)
+        if self.cuda:
+            t = self.keep.new_empty(shape, dtype=_torch_dtype(np_dtype))
             return t, t.data_ptr()
         a = np.empty(shape, dtype=np_dtype)
         return a, a.ctypes.data
@@ -347,6 +368,7 @@ def _global_rows(n_local: int, ctx: Context) -> int:
 class ProductQuantizer:
     def __init__(self, handle, ctx: Context, distance: Distance):
         self._h, self._ctx, self.distance = handle, ctx, distance
+        self._shape = None
 
     @classmethod
     def fit(cls, training_data, m: int, k: int, max_iters: int, distance: Distance, seed: int, *,
@@ -380,9 +402,11 @@ class ProductQuantizer:
         return cls(h, ctx, distance)
 
     def shape(self):
-        m, k, sd = C.c_size_t(), C.c_size_t(), C.c_size_t()
-        _lib.load().vqb_pq_shape(self._h, C.byref(m), C.byref(k), C.byref(sd))
-        return int(m.value), int(k.value), int(sd.value)
+        if self._shape is None:
+            m, k, sd = C.c_size_t(), C.c_size_t(), C.c_size_t()
+            _lib.load().vqb_pq_shape(self._h, C.byref(m), C.byref(k), C.byref(sd))
+            self._shape = int(m.value), int(k.value), int(sd.value)
+        return self._shape
 
     @property
     def codebooks(self) -> np.ndarray:
@@ -427,6 +451,7 @@ class ProductQuantizer:
 class ResidualQuantizer:
     def __init__(self, handle, ctx: Context, distance: Distance):
         self._h, self._ctx, self.distance = handle, ctx, distance
+        self._shape = None
 
     @classmethod
     def fit(cls, training_data, stages: int, k: int, max_iters: int, epsilon: float, distance: Distance, seed: int, *,
@@ -463,9 +488,11 @@ class ResidualQuantizer:
         return cls(h, ctx, distance)
 
     def shape(self):
-        s, k, d = C.c_size_t(), C.c_size_t(), C.c_size_t()
-        _lib.load().vqb_rvq_shape(self._h, C.byref(s), C.byref(k), C.byref(d))
-        return int(s.value), int(k.value), int(d.value)
+        if self._shape is None:
+            s, k, d = C.c_size_t(), C.c_size_t(), C.c_size_t()
+            _lib.load().vqb_rvq_shape(self._h, C.byref(s), C.byref(k), C.byref(d))
+            self._shape = int(s.value), int(k.value), int(d.value)
+        return self._shape
 
     @property
     def codebooks(self) -> np.ndarray:
@@ -503,6 +530,7 @@ class ResidualQuantizer:
 class OptimizedProductQuantizer:
     def __init__(self, handle, ctx: Context, distance: Distance, dim: int):
         self._h, self._ctx, self.distance, self.dim = handle, ctx, distance, dim
+        self._shape = None
 
     @classmethod
     def fit(cls, training_data, m: int, k: int, max_iters: int, opq_iters: int, distance: Distance, seed: int, *,
@@ -536,9 +564,11 @@ class OptimizedProductQuantizer:
         return cls(h, ctx, distance, m * sd)
 
     def shape(self):
-        m, k, sd = C.c_size_t(), C.c_size_t(), C.c_size_t()
-        _lib.load().vqb_opq_shape(self._h, C.byref(m), C.byref(k), C.byref(sd))
-        return int(m.value), int(k.value), int(sd.value)
+        if self._shape is None:
+            m, k, sd = C.c_size_t(), C.c_size_t(), C.c_size_t()
+            _lib.load().vqb_opq_shape(self._h, C.byref(m), C.byref(k), C.byref(sd))
+            self._shape = int(m.value), int(k.value), int(sd.value)
+        return self._shape
 
     @property
     def rotation(self) -> np.ndarray:

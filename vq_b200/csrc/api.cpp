@@ -687,9 +687,9 @@ int vqb_pq_quantize(vqb_pq *pq, const float *x, size_t n, size_t dim, uint16_t *
         sh.sd = pq->sd;
         sh.k = pq->k;
         const size_t chunk_rows = 1u << 16;
-        const bool all_host = !dev.is_device_pointer(x) && (!out_f16 || !dev.is_device_pointer(out_f16)) &&
+        const bool all_host = n >= 2 * chunk_rows && !dev.is_device_pointer(x) && (!out_f16 || !dev.is_device_pointer(out_f16)) &&
                               (!codes || !dev.is_device_pointer(codes)) && (out_f16 || codes);
-        if (all_host && n >= 2 * chunk_rows) {
+        if (all_host) {
             // large host batch (the loop of src/bin/eval_pq.rs:51-59 in one call): chunked copy / encode / copy pipeline
             HostPipeline pipe(dev, chunk_rows);
             void *const outs[2] = {out_f16, codes};
@@ -1061,7 +1061,7 @@ int vqb_sq_quantize(vqb_ctx *ctx, float min, float max, size_t levels, float ste
         if (!x || !out) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL data pointer");
         CudaDevice &dev = *ctx->dev;
         const size_t chunk = 1u << 23; // 8 Mi values = 32 MiB in, 8 MiB out
-        if (!dev.is_device_pointer(x) && !dev.is_device_pointer(out) && n_elems >= 2 * chunk) {
+        if (n_elems >= 2 * chunk && !dev.is_device_pointer(x) && !dev.is_device_pointer(out)) {
             HostPipeline pipe(dev, chunk);
             void *const outs[2] = {out, nullptr};
             const size_t ob[2] = {1, 0};
@@ -1095,7 +1095,7 @@ int vqb_bq_quantize(vqb_ctx *ctx, float threshold, uint8_t low, uint8_t high, co
         if (!x || !out) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL data pointer");
         CudaDevice &dev = *ctx->dev;
         const size_t chunk = 1u << 23;
-        if (!dev.is_device_pointer(x) && !dev.is_device_pointer(out) && n_elems >= 2 * chunk) {
+        if (n_elems >= 2 * chunk && !dev.is_device_pointer(x) && !dev.is_device_pointer(out)) {
             HostPipeline pipe(dev, chunk);
             void *const outs[2] = {out, nullptr};
             const size_t ob[2] = {1, 0};
