@@ -3,7 +3,7 @@ import numpy as np
 import pytest
 
 import vq_b200 as vq
-from tests.util import RecordingSeeder, by_stream
+from tests.util import METRICS, RecordingSeeder, by_stream
 from vq_b200 import synth
 
 pytestmark = pytest.mark.gpu
@@ -23,3 +23,39 @@ def test_ordered_sums_bit_exact(oracle, n, m, sd, k):
     pq = vq.ProductQuantizer.fit(x, m, k, 3, vq.Distance.Euclidean, 3, init_idx=init, draw=sg.draw, accumulate=vq.ACCUM_ORDERED)
     assert np.array_equal(pq.iterations, it_o) and by_stream(so.draws) == by_stream(sg.draws)
     assert np.array_equal(pq.codebooks, cb_o)
+
+
+@pytest.mark.parametrize("name", ["SquaredEuclidean", "Euclidean", "CosineDistance", "Manhattan", "Chebyshev", "Hamming"])
+@pytest.mark.parametrize("n,m,sd,k", [(1, 3, 1, 1), (1, 16, 8, 256), (63, 2, 5, 64), (65, 2, 16, 65), (9, 1, 17, 129), (1200, 4, 8, 40)])
+def test_direct_encode_bit_exact(oracle, name, n, m, sd, k):
+    """Few rows in one launch: every number of threads per row group (32, 64, 128) and of rows per thread, chunks of the codebook
+    that are not whole, ties (duplicate centroids), a zero centroid, NaN and infinity in rows and centroids."""
+    x, cb = synth.uniform(n, m * sd, 7 + n, -1.0, 1.0), synth.uniform(k, m * sd, 11 + k, -1.0, 1.0).reshape(k, m, sd).transpose(1, 0, 2).copy()
+    if k > 4:
+        cb[:, k - 1] = cb[:, 1]
+        cb[:, 2] = 0.0
+    if n > 8:
+        x[3], x[4, 0], x[5, :sd], x[6] = 0.0, np.nan, np.inf, 1e30
+        x[8, :sd] = cb[0, min(1, k - 1)]
+        cb[0, k // 2, 0] = np.nan
+        cb[m - 1, k - 2, sd - 1] = np.inf
+    out_o, codes_o = oracle.pq_quantize(cb, x, METRICS[name])
+    out, codes = vq.ProductQuantizer.from_codebooks(cb, getattr(vq.Distance, name)).quantize(x, return_codes=True)
+    assert np.array_equal(codes, codes_o)
+    assert np.array_equal(out, out_o.view(np.float16), equal_nan=True)
+
+
+@pytest.mark.parametrize("name", ["SquaredEuclidean", "Euclidean", "CosineDistance", "Manhattan"])
+@pytest.mark.parametrize("n,dim,k,stages", [(1, 128, 256, 8), (17, 33, 64, 3), (40, 15, 7, 2), (700, 64, 130, 4)])
+def test_direct_residual_encode_bit_exact(oracle, name, n, dim, k, stages):
+    """All stages in one launch: rows that end early (their residual is a centroid), ties, NaN rows, ragged chunks."""
+    x = synth.gaussian_mixture(n, dim, 5)
+    books = 0.2 * synth.normal(stages * k, dim, 3).reshape(stages, k, dim)
+    books[0, 0] = x[0]
+    if n > 8:
+        x[5, dim - 1] = np.nan
+        books[1, k - 1] = books[1, k // 2]
+    out_o, codes_o, _ = oracle.rvq_quantize(books, 0.01, x, METRICS[name])
+    out, codes = vq.ResidualQuantizer.from_codebooks(books, 0.01, getattr(vq.Distance, name)).quantize(x, return_codes=True)
+    assert np.array_equal(codes, codes_o)
+    assert np.array_equal(out, out_o.view(np.float16), equal_nan=True)

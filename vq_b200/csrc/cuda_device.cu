@@ -14,6 +14,7 @@
 #include "assign_generic.cuh"
 #include "assign_reg.cuh"
 #include "dense_tc.hpp"
+#include "direct.cuh"
 #include "opq_tc.hpp"
 #include "ordered_sums.cuh"
 #include "pq_tc.hpp"
@@ -643,7 +644,12 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
     p.pv = (float)pm;
     p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
     p.out_vec = (!out_f16 || (aligned16(out_f16) && dim % 8 == 0)) && (!out_f32 || (aligned16(out_f32) && dim % 4 == 0));
-    if (!cuda_cores_only && pq_tensor_enabled_ && pq_tc_applicable(p, metric)) {
+    const bool tensor = !cuda_cores_only && pq_tensor_enabled_ && pq_tc_applicable(p, metric);
+    if (direct_encode_applicable(p, tensor)) {
+        launch_direct_encode(*this, p, metric);
+        return;
+    }
+    if (tensor) {
         ensure_tc_buffers(0);
         bop_fresh_ = nullptr;
         PqTcBuffers tb;
@@ -736,8 +742,26 @@ void CudaDevice::rvq_quantize(const float *x, size_t n, size_t dim, const float 
                               float epsilon, int metric, double pm, uint16_t *out_f16, uint32_t *out_codes)
 {
     if (n == 0) return;
+    GenericParams g = {};
+    g.x = x;
+    g.n = n;
+    g.ld = dim;
+    g.m = 1;
+    g.k = (int)k;
+    g.sd = (int)dim;
+    g.centroids = codebooks;
+    g.pv = (float)pm;
+    g.out_f16 = out_f16;
+    g.out_codes = out_codes;
+    g.stages = (int)stages;
+    g.epsilon = epsilon;
+    const bool tensor = tensor_enabled_ && dense_tc_applicable(n, dim, k, metric, x);
+    if (direct_rvq_applicable(g, tensor, smem_limit_)) {
+        launch_direct_rvq(*this, g, metric);
+        return;
+    }
     if (out_codes) VQB_CUDA_CHECK(cudaMemsetAsync(out_codes, 0xFF, sizeof(uint32_t) * n * stages, stream_));
-    if (tensor_enabled_ && dense_tc_applicable(n, dim, k, metric, x)) {
+    if (tensor) {
         // stage by stage: norms of the current residuals, tensor-core shortlist, exact resolve that subtracts the chosen
         // centroid, adds it to the running sum and retires rows whose residual norm fell below epsilon
         ensure_tc_buffers(n);
@@ -774,19 +798,6 @@ void CudaDevice::rvq_quantize(const float *x, size_t n, size_t dim, const float 
         release(res);
         return;
     }
-    GenericParams g = {};
-    g.x = x;
-    g.n = n;
-    g.ld = dim;
-    g.m = 1;
-    g.k = (int)k;
-    g.sd = (int)dim;
-    g.centroids = codebooks;
-    g.pv = (float)pm;
-    g.out_f16 = out_f16;
-    g.out_codes = out_codes;
-    g.stages = (int)stages;
-    g.epsilon = epsilon;
     launch_assign_generic(*this, g, metric, G_RVQ_QUANT, 4);
 }
 

@@ -89,6 +89,7 @@ class CudaDevice : public Device {
     int device() const { return device_; }
     int sm_count() const { return sm_count_; }
     size_t smem_limit() const { return smem_limit_; }
+    int *error_word() const { return tc_error_; } // null with VQB_NO_TENSOR=1
     uint64_t launches() const { return launches_.load(); }
     void count_launch(uint64_t n = 1) { launches_ += n; }
     // How often this context has asked CUDA for device or pinned memory (cudaMalloc, cudaMallocAsync, cudaHostAlloc).
