@@ -24,11 +24,20 @@
 //   => |S_j - true| <= E = 1.25 * 2^-19 (xh2 + 2 HN) = 2.4e-6 (xh2 + 2 HN)
 //   the reference prefers w over a = argmin S only if D_w <= D_a (1 + 4u) in its own arithmetic (10u relative each), i.e.
 //   S_w <= S_a + 2E + 25u (xh2 + |S_a| + E)  <=  S_a + 4.8e-6 (xh2 + 2HN) + 1.5e-6 (xh2 + |S_a|) + ...  <  limit.
-// The count uses t = sat((limit - S) * 2^p) with p chosen per row so that limit * 2^p ~ 2^60: a score differs from the
-// limit by nothing or by at least one unit in its last place (>= 2^-24 |limit|), so t is exactly 0 or 1, and the two sums
-// total = sum t * (1 + (j mod 32) / 512) and offs = sum (j / 32) * t * (1 + (j mod 32) / 512) yield count and index at once on
-// the FMA pipe.  Rows whose true distances could overflow f32 (|x|^2/2 + 2 HN >= 1e37) are marked as well: there the
+// One pass over the accumulator (3-input minima, one per score: 2 cycles of the integer pipe each, which is what bounds the
+// epilogue at 512 cycles per unit and scheduler) leaves the minima of the 16 blocks of 16 consecutive columns and of the 16
+// classes of columns equal modulo 16.  Two scores below the limit differ in their block or in their class, so exactly one score
+// lies below it <=> exactly one block minimum and exactly one class minimum do, and these two give its column.  They are counted
+// with t = sat((limit - S) * 2^p), p chosen per row so that limit * 2^p ~ 2^60: a minimum differs from the limit by nothing or
+// by at least one unit in its last place (>= 2^-24 |limit|), so t is exactly 0 or 1, and sum t * (1 + i / 512) has count and
+// index in one number.  Rows whose true distances could overflow f32 (|x|^2/2 + 2 HN >= 1e37) are marked as well: there the
 // reference's own comparisons see infinities.
+//
+// Measured, 1M x 128, m 16, k 256: 0.923 -> 0.613 ms per training pass (encode 0.942 -> 0.638 ms) against two passes over the
+// accumulator, the second of which spent two operations per score on count and index.  Per (tile, sub-space): 1456 cycles,
+// integer pipe 56 % busy, tensor pipe 35 %; the rest is the way from a commit to the epilogue and back.  Four teams (one per
+// sub-space) and eight warps per accumulator (half of the columns each) came to 0.63 - 0.81 ms: their halved registers cost
+// spills, moves or doubled tails.  Accumulators of 128 columns: 0.96 ms (an MMA of N = 128 takes as long as one of N = 256).
 //
 // CTA (1 per SM, persistent, 448 threads), owning 4 consecutive sub-spaces (m / 4 groups share the row tiles):
 //   warp 0       loads the group's four operand-B tiles once (TMA, 128B swizzle, no multicast; 32 KiB each) and, for an
@@ -88,6 +97,15 @@ __device__ __forceinline__ float to_tf32(float v)
     return __uint_as_float(r);
 }
 
+// The 11-bit head of v by Veltkamp's splitting (Dekker, Numer. Math. 18, 1971): nearest TF32 number like to_tf32, on the FMA
+// pipe; cvt.rna.tf32 costs two instructions of the integer pipe that the epilogue's minima need.  |v| > 2^114 gives NaN, which
+// sends the row to the exact scan.
+__device__ __forceinline__ float split_tf32(float v)
+{
+    const float t = __fmul_rn(v, 8193.0f);
+    return __fsub_rn(t, __fsub_rn(t, v));
+}
+
 __device__ __forceinline__ float fma_sat(float a, float b, float c)
 {
     float d;
@@ -100,7 +118,7 @@ __device__ __forceinline__ int issue_order(int p) { return ((p & 1) << 1) | (p >
 
 constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES + (size_t)NSTAGE * A_STAGE_BYTES + ((size_t)XH_RING * BM + 4 * BN * 4) * sizeof(float) + sizeof(PqBarriers) + 64;
 
-template <bool TRAIN, bool EUCLID>
+template <bool TRAIN, bool EUCLID, bool DUMP>
 __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constant__ CUtensorMap map_b, const PqTcParams Q)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -204,23 +222,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constan
         // ------------------------------------------------ operand A: split row slices into the ring
         const int r = (warp - 2) * 32 + lane; // row of the tile
         uint32_t it = 0;
-        float4 cur[8], nxt[8];
-        auto fetch = [&](float4(&dst)[8], unsigned long long tile) {
+        float4 cur[8]; // the tile's four slices; each is requested again for the next tile as soon as it has been used
+        auto fetch = [&](int ss, unsigned long long tile) {
             const unsigned long long row = tile * BM + r;
             if (tile < n_tiles && row < P.n) {
-                const float4 *src = reinterpret_cast<const float4 *>(P.x + row * P.ld + (size_t)g * 32);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) dst[i] = __ldg(src + i);
+                const float4 *src = reinterpret_cast<const float4 *>(P.x + row * P.ld + (size_t)g * 32) + 2 * ss;
+                cur[2 * ss] = __ldg(src), cur[2 * ss + 1] = __ldg(src + 1);
             } else {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) dst[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                cur[2 * ss] = cur[2 * ss + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         };
-        if (nact > 0) fetch(nxt, tile0);
-        for (unsigned long long tile = tile0; nact > 0 && tile < n_tiles && !*abort_flag; tile += tstep) {
+        if (nact > 0)
 #pragma unroll
-            for (int i = 0; i < 8; ++i) cur[i] = nxt[i];
-            fetch(nxt, tile + tstep);
+            for (int ss4 = 0; ss4 < 4; ++ss4) fetch(issue_order(ss4), tile0);
+        for (unsigned long long tile = tile0; nact > 0 && tile < n_tiles && !*abort_flag; tile += tstep) {
             bool ok = true;
 #pragma unroll
             for (int ss4 = 0; ss4 < 4; ++ss4) { // static indexing of cur[]; issue order 0, 2, 1, 3
@@ -233,11 +248,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constan
                 }
                 const float4 v0 = cur[2 * ss], v1 = cur[2 * ss + 1];
                 const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+                fetch(ss, tile + tstep);
                 float hi[8], lo[8], sq = 0.0f;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    hi[i] = to_tf32(v[i]);
-                    lo[i] = to_tf32(v[i] - hi[i]);
+                    hi[i] = split_tf32(v[i]);
+                    lo[i] = split_tf32(v[i] - hi[i]);
                     sq = fmaf(v[i], v[i], sq);
                 }
                 unsigned char *rowp = a_smem + (size_t)st * A_STAGE_BYTES + (size_t)r * 128;
@@ -262,163 +278,138 @@ __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constan
     } else {
         // ------------------------------------------------ epilogue
         const int q = warp & 3;           // TMEM lane quadrant
-        const int team = (warp - 6) >> 2; // accumulator and sub-space pair
+        const int acc = (warp - 6) >> 2;  // team = accumulator: sub-spaces 2 acc, 2 acc + 1 of the group
         const int nch = (k + 31) >> 5;    // 32-column chunks that hold centroids
-        uint32_t uu = 0, moved_mask = 0, tile_iter = 0;
-        const float hmax2_0 = 2.0f * Q.hnmax[g * 4 + team * 2], hmax2_1 = 2.0f * Q.hnmax[g * 4 + team * 2 + 1];
+        const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)acc * BN;
+        const float hmax2_0 = 2.0f * Q.hnmax[g * 4 + acc * 2], hmax2_1 = 2.0f * Q.hnmax[g * 4 + acc * 2 + 1];
+        uint32_t uu = 0, tile_iter = 0, marked_pairs = 0, moved_mask = 0;
         if (!TRAIN && nact > 0) mbar_wait(&bars->bfull, 0, abort_flag, Q.error, 16); // the f16 images arrive with operand B
         for (unsigned long long tile = tile0; nact > 0 && tile < n_tiles && !*abort_flag; tile += tstep, ++tile_iter) {
             const unsigned long long row = tile * BM + 32ull * q + lane;
             const bool valid = row < P.n;
+            uint8_t *cp = reinterpret_cast<uint8_t *>(P.codes) + row * (unsigned long long)m + g * 4 + acc * 2;
             uint32_t old2 = 0;
-            if (TRAIN && valid) old2 = *reinterpret_cast<const uint16_t *>(reinterpret_cast<const uint8_t *>(P.codes) + row * (unsigned long long)m + g * 4 + team * 2);
-            int idxs[2] = {0, 0};
-            uint32_t marked = 0, done = 0;
+            if (TRAIN && valid) old2 = *reinterpret_cast<const uint16_t *>(cp);
+            uint32_t idxs[2] = {0, 0}, done = 0, marked = 0;
 #pragma unroll 1
             for (int h = 0; h < 2; ++h) {
-                const int ss = team * 2 + h;
+                const int ss = acc * 2 + h, s = g * 4 + ss;
                 if (pos_of(ss) == 15) continue;
                 const uint32_t it = tile_iter * (uint32_t)nact + (uint32_t)pos_of(ss);
-                if (!mbar_wait(&bars->tfull[team], uu & 1u, abort_flag, Q.error, 15)) break;
+                if (!mbar_wait(&bars->tfull[acc], uu & 1u, abort_flag, Q.error, 15)) break;
                 ++uu;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)team * BN;
-                uint32_t ra[32], rb[32];
-                tmem_ld32_issue(taddr, ra);
+                if (DUMP) { // diagnostic dump of the raw scores
+                    for (int c = 0; c < nch; ++c) {
+                        uint32_t v[32];
+                        tmem_ld32_issue(taddr + c * 32, v);
+                        tmem_wait();
+                        if (valid) {
+                            float *o = Q.dbg_scores + ((size_t)row * m + s) * BN + c * 32;
+#pragma unroll
+                            for (int t = 0; t < 32; ++t) o[t] = __uint_as_float(v[t]);
+                        }
+                    }
+                }
                 const float xh2 = xh_ring[(it & (XH_RING - 1)) * BM + 32 * q + lane];
                 const float hmax2 = h ? hmax2_1 : hmax2_0;
 
-                // pass 1: the smallest score (four independent 3-input min chains)
-                float b0 = VQB_INF, b1 = VQB_INF, b2 = VQB_INF, b3 = VQB_INF;
-                bool col0_nan = false;
-                tmem_wait();
-#pragma unroll 1
-                for (int cb = 0; cb < nch; cb += 2) {
-                    if (cb + 1 < nch) tmem_ld32_issue(taddr + (cb + 1) * 32, rb);
-                    if (cb == 0) {
-                        const float s0 = __uint_as_float(ra[0]);
-                        col0_nan = !(s0 == s0);
-                    }
+                // One pass over the scores, one 3-input minimum each: the minima of the 16 blocks of 16 consecutive columns and of the 16
+                // classes of columns equal modulo 16.  Straight-line code with a way out after every chunk: without these branches the
+                // chunks' loads were scheduled ahead and the scores spilled, with a test around every chunk each register of it was
+                // moved once more.
+                uint32_t idx = 0;
+                bool single = false;
+                {
+                    constexpr int N = 8;
+                    float hb[2 * N], ga[16];
+                    bool col0_nan = false;
 #pragma unroll
-                    for (int t = 0; t < 32; t += 8) {
-                        b0 = min3f(b0, __uint_as_float(ra[t]), __uint_as_float(ra[t + 1]));
-                        b1 = min3f(b1, __uint_as_float(ra[t + 2]), __uint_as_float(ra[t + 3]));
-                        b2 = min3f(b2, __uint_as_float(ra[t + 4]), __uint_as_float(ra[t + 5]));
-                        b3 = min3f(b3, __uint_as_float(ra[t + 6]), __uint_as_float(ra[t + 7]));
-                    }
-                    tmem_wait();
-                    if (cb + 1 < nch) {
-                        tmem_ld32_issue(taddr + (cb + 2 < nch ? cb + 2 : 0) * 32, ra); // past the end: the first chunk of pass 2
+                    for (int i = 0; i < 16; ++i) hb[i] = VQB_INF;
 #pragma unroll
-                        for (int t = 0; t < 32; t += 8) {
-                            b0 = min3f(b0, __uint_as_float(rb[t]), __uint_as_float(rb[t + 1]));
-                            b1 = min3f(b1, __uint_as_float(rb[t + 2]), __uint_as_float(rb[t + 3]));
-                            b2 = min3f(b2, __uint_as_float(rb[t + 4]), __uint_as_float(rb[t + 5]));
-                            b3 = min3f(b3, __uint_as_float(rb[t + 6]), __uint_as_float(rb[t + 7]));
-                        }
-                    } else {
-                        tmem_ld32_issue(taddr, ra); // odd chunk count: the first chunk of pass 2
-                    }
-                    tmem_wait();
-                }
-                const float best = fminf(fminf(b0, b1), fminf(b2, b3));
-                const float limit = best + (MARGIN_COEF * (xh2 + hmax2 + fabsf(best)) + 1e-36f);
-                // rows the test below cannot rank: NaN / infinity anywhere that matters, or values too small to scale
-                // (nor rows whose true distances could overflow f32: there the reference's own comparisons see infinities)
-                const bool rankable = !col0_nan && (fabsf(limit) >= 8.6736174e-19f /* 2^-60 */) && (fabsf(limit) < VQB_INF) && (xh2 + hmax2 < 1e37f);
-                const uint32_t eb = (__float_as_uint(limit) >> 23) & 0xFFu;
-                const float nbig = __uint_as_float(0x80000000u | ((314u - eb) << 23)); // -2^(60 - exponent(limit))
-                const float lb = -limit * nbig;                                       // exact scaling
-
-                // pass 2: over the scores below the limit, total = sum (1 + t / 512) and offs = sum chunk * (1 + t / 512),
-                // t = column within its 32-column chunk: exactly one score below the limit <=> 1 <= total < 1.07
-                float total = 0.0f, offs = 0.0f; // chunk 0 was requested (and awaited) at the end of pass 1
-#pragma unroll 1
-                for (int cb = 0; cb < nch; cb += 2) {
-                    if (cb + 1 < nch) tmem_ld32_issue(taddr + (cb + 1) * 32, rb);
-                    {
-                        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-#pragma unroll
-                        for (int t = 0; t < 32; t += 4) {
-                            a0 = fmaf(fma_sat(__uint_as_float(ra[t]), nbig, lb), 1.0f + (float)t * 0.001953125f, a0);
-                            a1 = fmaf(fma_sat(__uint_as_float(ra[t + 1]), nbig, lb), 1.0f + (float)(t + 1) * 0.001953125f, a1);
-                            a2 = fmaf(fma_sat(__uint_as_float(ra[t + 2]), nbig, lb), 1.0f + (float)(t + 2) * 0.001953125f, a2);
-                            a3 = fmaf(fma_sat(__uint_as_float(ra[t + 3]), nbig, lb), 1.0f + (float)(t + 3) * 0.001953125f, a3);
-                        }
-                        const float cs = (a0 + a1) + (a2 + a3);
-                        total += cs;
-                        offs = fmaf(cs, (float)cb, offs);
-                    }
-                    tmem_wait();
-                    if (cb + 1 < nch) {
-                        if (cb + 2 < nch) tmem_ld32_issue(taddr + (cb + 2) * 32, ra);
-                        float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-#pragma unroll
-                        for (int t = 0; t < 32; t += 4) {
-                            a0 = fmaf(fma_sat(__uint_as_float(rb[t]), nbig, lb), 1.0f + (float)t * 0.001953125f, a0);
-                            a1 = fmaf(fma_sat(__uint_as_float(rb[t + 1]), nbig, lb), 1.0f + (float)(t + 1) * 0.001953125f, a1);
-                            a2 = fmaf(fma_sat(__uint_as_float(rb[t + 2]), nbig, lb), 1.0f + (float)(t + 2) * 0.001953125f, a2);
-                            a3 = fmaf(fma_sat(__uint_as_float(rb[t + 3]), nbig, lb), 1.0f + (float)(t + 3) * 0.001953125f, a3);
-                        }
-                        const float cs = (a0 + a1) + (a2 + a3);
-                        total += cs;
-                        offs = fmaf(cs, (float)(cb + 1), offs);
+                    for (int c = 0; c < N; ++c) {
+                        uint32_t v[32];
+                        tmem_ld32_issue(taddr + c * 32, v);
                         tmem_wait();
-                    }
-                }
-                if (Q.dbg_scores) { // diagnostic dump of the raw scores
-                    for (int cb = 0; cb < nch; ++cb) {
-                        tmem_ld32_issue(taddr + cb * 32, ra);
-                        tmem_wait();
-                        if (valid) {
-                            float *o = Q.dbg_scores + ((size_t)row * m + g * 4 + ss) * BN + cb * 32;
+                        if (c == 0) col0_nan = !(__uint_as_float(v[0]) == __uint_as_float(v[0]));
 #pragma unroll
-                            for (int t = 0; t < 32; ++t) o[t] = __uint_as_float(ra[t]);
+                        for (int t = 0; t < 16; ++t)
+                            ga[t] = c ? min3f(ga[t], __uint_as_float(v[t]), __uint_as_float(v[16 + t])) : fminf(__uint_as_float(v[t]), __uint_as_float(v[16 + t]));
+                        float b0 = __uint_as_float(v[0]), b1 = __uint_as_float(v[16]);
+#pragma unroll
+                        for (int t = 1; t < 15; t += 2) {
+                            b0 = min3f(b0, __uint_as_float(v[t]), __uint_as_float(v[t + 1]));
+                            b1 = min3f(b1, __uint_as_float(v[16 + t]), __uint_as_float(v[16 + t + 1]));
                         }
+                        hb[2 * c] = fminf(b0, __uint_as_float(v[15]));
+                        hb[2 * c + 1] = fminf(b1, __uint_as_float(v[31]));
+                        if (c + 1 == nch) break;
                     }
+                    // every score of this warp has been used: the accumulator may be overwritten
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bars->tempty[acc]);
+                    float best = hb[0];
+#pragma unroll
+                    for (int i = 1; i < 2 * N - 1; i += 2) best = min3f(best, hb[i], hb[i + 1]);
+                    best = fminf(best, hb[2 * N - 1]);
+                    const float limit = best + (MARGIN_COEF * (xh2 + hmax2 + fabsf(best)) + 1e-36f);
+                    // Rows the test below cannot rank: NaN / infinity anywhere that matters, or values too small to scale (exponent of
+                    // the limit below -60; nor rows whose true distances could overflow f32: there the reference's comparisons see
+                    // infinities).
+                    const uint32_t eb = (__float_as_uint(limit) >> 23) & 0xFFu;
+                    const bool rankable = !col0_nan && eb - 67u < 188u && (xh2 + hmax2 < 1e37f);
+                    const float nbig = __uint_as_float(0x80000000u | ((314u - eb) << 23)); // -2^(60 - exponent(limit))
+                    const float lb = -limit * nbig;                                       // exact scaling
+                    // Sums of (1 + i / 512) over the blocks and over the classes whose minimum lies below the limit (the smallest
+                    // score's always does).  Both below 1.07, i.e. one block and one class <=> exactly one score lies below the limit:
+                    // two would differ in their block or in their class.  (1 + i / 512) + 16383 has i in its low mantissa bits.
+                    float tb0 = 0.0f, tb1 = 0.0f, ta0 = 0.0f, ta1 = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < 2 * N; i += 2) {
+                        tb0 = fmaf(fma_sat(hb[i], nbig, lb), 1.0f + (float)i * 0.001953125f, tb0);
+                        tb1 = fmaf(fma_sat(hb[i + 1], nbig, lb), 1.0f + (float)(i + 1) * 0.001953125f, tb1);
+                    }
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        ta0 = fmaf(fma_sat(ga[i], nbig, lb), 1.0f + (float)i * 0.001953125f, ta0);
+                        ta1 = fmaf(fma_sat(ga[i + 1], nbig, lb), 1.0f + (float)(i + 1) * 0.001953125f, ta1);
+                    }
+                    const float tb = tb0 + tb1, ta = ta0 + ta1;
+                    idx = (__float_as_uint(tb + 16383.0f) & 15u) * 16 + (__float_as_uint(ta + 16383.0f) & 15u);
+                    single = rankable && fmaxf(tb, ta) < 1.07f && idx < (uint32_t)k;
                 }
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->tempty[team]);
-
-                const bool single = rankable && total >= 1.0f && total < 1.07f;
-                const int idx = single ? ((int)offs) * 32 + (int)((total - 1.0f) * 512.0f + 0.5f) : 0;
                 if (h == 0) idxs[0] = idx;
                 else idxs[1] = idx;
-                if (!single || idx >= k) marked |= 1u << h;
                 done |= 1u << h;
+                if (!single) marked |= 1u << h;
             }
-
             if (valid && done) {
-                if (marked) Q.marks[row * (unsigned long long)(m >> 1) + g * 2 + team] = (uint8_t)marked;
+                if (marked) Q.marks[row * (unsigned long long)(m >> 1) + g * 2 + acc] = (uint8_t)marked;
                 if (TRAIN) {
-                    uint8_t *cp = reinterpret_cast<uint8_t *>(P.codes) + row * (unsigned long long)m + g * 4 + team * 2;
                     if (done == 3u && marked == 0u) {
-                        const uint32_t nw = (uint32_t)idxs[0] | ((uint32_t)idxs[1] << 8);
+                        const uint32_t nw = idxs[0] | (idxs[1] << 8);
                         if (nw != old2) {
-                            if ((nw ^ old2) & 0xFFu) moved_mask |= 1u << (team * 2);
-                            if ((nw ^ old2) & 0xFF00u) moved_mask |= 1u << (team * 2 + 1);
+                            if ((nw ^ old2) & 0xFFu) moved_mask |= 1u;
+                            if ((nw ^ old2) & 0xFF00u) moved_mask |= 2u;
                             *reinterpret_cast<uint16_t *>(cp) = (uint16_t)nw;
                         }
                     } else {
 #pragma unroll
                         for (int h = 0; h < 2; ++h)
-                            if ((done >> h & 1u) && !(marked >> h & 1u)) {
-                                const uint32_t ob = (old2 >> (8 * h)) & 0xFFu;
-                                if (ob != (uint32_t)idxs[h]) {
-                                    moved_mask |= 1u << (team * 2 + h);
-                                    cp[h] = (uint8_t)idxs[h];
-                                }
+                            if (((done & ~marked) >> h & 1u) && ((old2 >> (8 * h)) & 0xFFu) != idxs[h]) {
+                                moved_mask |= 1u << h;
+                                cp[h] = (uint8_t)idxs[h];
                             }
                     }
                 } else {
                     const int dim = m * SDW;
 #pragma unroll
                     for (int h = 0; h < 2; ++h)
-                        if ((done >> h & 1u) && !(marked >> h & 1u)) {
-                            const int ss = team * 2 + h, s = g * 4 + ss;
-                            const int idx = idxs[h];
-                            if (P.out_codes) P.out_codes[row * m + s] = (uint32_t)idx;
+                        if ((done & ~marked) >> h & 1u) {
+                            const int ss = acc * 2 + h, s = g * 4 + ss;
+                            const uint32_t idx = idxs[h];
+                            if (P.out_codes) P.out_codes[row * m + s] = idx;
                             if (P.out_f16) // 16-byte aligned: dim % 8 == 0
                                 *reinterpret_cast<uint4 *>(P.out_f16 + row * dim + (size_t)s * SDW) = c16_s[ss * BN + idx];
                             if (P.out_f32) {
@@ -429,17 +420,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constan
                             }
                         }
                 }
-            }
-            {
-                const uint32_t nm = __reduce_add_sync(0xffffffffu, (valid && done) ? (uint32_t)__popc(marked) : 0u);
-                if (nm && lane == 0) atomicAdd(Q.stats, (unsigned long long)nm);
+                marked_pairs += __popc(marked);
             }
         }
+        marked_pairs = __reduce_add_sync(0xffffffffu, marked_pairs);
+        if (marked_pairs && lane == 0) atomicAdd(Q.stats, (unsigned long long)marked_pairs);
         if (TRAIN) {
             moved_mask = __reduce_or_sync(0xffffffffu, moved_mask);
-            if (lane == 0)
-                for (int ss = 0; ss < 4; ++ss)
-                    if (moved_mask & (1u << ss)) atomicOr(P.changed + g * 4 + ss, VQB_MOVED_BITS);
+            if (lane < 2 && (moved_mask >> lane & 1u)) atomicOr(P.changed + g * 4 + acc * 2 + lane, VQB_MOVED_BITS);
         }
     }
 
@@ -646,10 +634,10 @@ size_t pq_tc_scratch_floats() { return SCRATCH_FLOATS; }
 size_t pq_tc_stats_offset_floats() { return OFF_STATS; }
 size_t pq_tc_mark_bytes(size_t n, size_t m) { return (n * (m / 2) + 15) & ~(size_t)15; } // read 16 bytes at a time
 
-template <bool TRAIN, bool EUCLID>
+template <bool TRAIN, bool EUCLID, bool DUMP = false>
 static void launch_t(CudaDevice &dev, const CUtensorMap &mb, const PqTcParams &q, unsigned grid)
 {
-    auto kernel = pq_tc_kernel<TRAIN, EUCLID>;
+    auto kernel = pq_tc_kernel<TRAIN, EUCLID, DUMP>;
     constexpr size_t smem = PQ_TC_SMEM;
     static std::atomic<unsigned long long> configured{0}; // bit d: the attribute has been set on device d (it is per device and sticky)
     const unsigned long long bit = 1ull << (dev.device() & 63);
@@ -700,7 +688,8 @@ void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train
     const unsigned ngroups = (unsigned)p.m / 4;
     const unsigned per = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(tiles, (unsigned long long)dev.sm_count() / ngroups));
     const unsigned grid = per * ngroups;
-    if (train) launch_t<true, false>(dev, mb, q, grid);
+    if (b.dbg_scores) launch_t<false, false, true>(dev, mb, q, grid);
+    else if (train) launch_t<true, false>(dev, mb, q, grid);
     else if (metric == M_EUCLID) launch_t<false, true>(dev, mb, q, grid);
     else launch_t<false, false>(dev, mb, q, grid);
 }

@@ -39,15 +39,19 @@ __device__ __forceinline__ void mbar_expect_tx(void *bar, uint32_t bytes)
 __device__ __forceinline__ bool mbar_wait(void *bar, uint32_t parity, volatile int *abort_flag, int *err, int code, uint32_t hint_ns = VQB_WAIT_HINT_NS)
 {
     const uint32_t addr = smem_u32(bar);
-    for (uint32_t i = 0; i < UMMA_SPIN_LIMIT; ++i) {
+    for (uint32_t i = 0; i < UMMA_SPIN_LIMIT / 1024; ++i) {
         uint32_t done;
-        // the hint lets the hardware park the thread (up to ~1 us) instead of spinning through issue slots
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+        // the hint lets the hardware park the thread (up to ~1 us) instead of spinning through issue slots; the inner loop is three
+        // instructions a poll, because waiting warps share their scheduler's integer pipe with the ones that work
+        asm volatile("{\n\t.reg .pred p, q;\n\t.reg .b32 n;\n\tmov.b32 n, 1024;\n"
+                     "poll:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t@p bra over;\n\t"
+                     "sub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra poll;\n"
+                     "over:\n\tselp.b32 %0, 1, 0, p;\n\t}"
                      : "=r"(done)
                      : "r"(addr), "r"(parity), "r"(hint_ns)
                      : "memory");
         if (done) return true;
-        if ((i & 1023u) == 1023u && *abort_flag) return false;
+        if (*abort_flag) return false;
     }
     *abort_flag = 1;
     atomicCAS(err, 0, code);
