@@ -59,3 +59,23 @@ def test_direct_residual_encode_bit_exact(oracle, name, n, dim, k, stages):
     out, codes = vq.ResidualQuantizer.from_codebooks(books, 0.01, getattr(vq.Distance, name)).quantize(x, return_codes=True)
     assert np.array_equal(codes, codes_o)
     assert np.array_equal(out, out_o.view(np.float16), equal_nan=True)
+
+
+@pytest.mark.parametrize("n,m,k", [(3000, 16, 256), (4097, 12, 200), (30_000, 4, 33)])
+@pytest.mark.parametrize("special", [False, True])
+def test_cosine_encode_on_tensor_cores_bit_exact(oracle, n, m, k, special):
+    """Unit vectors on the tensor cores, near-ties to the exact scan: parallel centroids, zero, tiny, huge and NaN norms on both
+    sides (each voids what it has to)."""
+    rng = np.random.default_rng(n + k)
+    x, cb = rng.normal(size=(n, m * 8)).astype(np.float32), rng.normal(size=(m, k, 8)).astype(np.float32)
+    cb[:, 7] = 2.0 * cb[:, 3]          # the same direction: distances differ in the last bits only
+    x[:50] = cb[:, 3].reshape(-1)
+    if special:
+        cb[0, 5], cb[1, 0, 2], cb[2, 9] = 0.0, np.nan, cb[2, 9] * 1e-30
+        cb[3, 11] = 1e25
+        x[60], x[61], x[62], x[63, 1] = 0.0, x[61] * 1e-25, x[62] * 1e20, np.nan
+    q = vq.ProductQuantizer.from_codebooks(cb, vq.Distance.CosineDistance)
+    out, codes = q.quantize(x, return_codes=True)
+    out_o, codes_o = oracle.pq_quantize(cb, x, METRICS["CosineDistance"])
+    assert np.array_equal(codes, codes_o)
+    assert np.array_equal(out, out_o.view(np.float16), equal_nan=True)

@@ -1,6 +1,7 @@
 // pq_tc.cu -- product-quantizer nearest-centroid search (sub-space width 8) with the scores on the tensor cores.
 //
-// Replaces the per-point scan of src/utils.rs:59-73 (training) and src/pq.rs:159-182 (encode) for the Euclidean metrics.
+// Replaces the per-point scan of src/utils.rs:59-73 (training) and src/pq.rs:159-182 (encode) for the Euclidean metrics and,
+// when encoding, cosine.
 //
 // Scores.  S_j = |c_j|^2/2 - x.c_j ranks the centroids like the squared distance (|x - c_j|^2 = |x|^2 + 2 S_j).  Both
 // operands are split into two TF32 numbers (x = xh + xl, c = ch + cl, each part exactly representable, so the hardware's
@@ -39,6 +40,13 @@
 // sub-space) and eight warps per accumulator (half of the columns each) came to 0.63 - 0.81 ms: their halved registers cost
 // spills, moves or doubled tails.  Accumulators of 128 columns: 0.96 ms (an MMA of N = 128 takes as long as one of N = 256).
 //
+// Cosine (src/distances.rs:141-150).  1 - x.c / (|x| |c|) ranks like S_j = -x.(c_j / |c_j|), with the norm that the reference
+// computes and a zero vector for a zero norm (its distance is 1, like a score of 0).  The same split and chain with zero half
+// norms: |S_j - true| <= 2.4e-6 |x| (the unit vectors' own rounding, 2u, included).  The reference's quotient carries (2d + 6)u
+// = 22u and its difference from 1 another 2u, so it can prefer w over a only if S_w <= S_a + |x| (2 * 2.4e-6 + 2 * 24u): limit =
+// best + 7e-6 (1.25 |x| + |best|).  Norms outside [1e-17, 1e18] (products that underflow or overflow) void the row, or the
+// sub-space if it is a centroid's: everything goes to the exact scan.
+//
 // CTA (1 per SM, persistent, 448 threads), owning 4 consecutive sub-spaces (m / 4 groups share the row tiles):
 //   warp 0       loads the group's four operand-B tiles once (TMA, 128B swizzle, no multicast; 32 KiB each) and, for an
 //                encode, the binary16 images of the group's centroids (16 KiB, bulk copy)
@@ -66,6 +74,7 @@ constexpr uint32_t A_STAGE_BYTES = BM * 128; // 16 KiB
 constexpr uint32_t B_BYTES = BN * 128;       // 32 KiB per sub-space
 constexpr float PAD_SCORE = 1e30f;           // score of the columns beyond k
 constexpr float MARGIN_COEF = 7e-6f;
+constexpr float COS_MIN = 1e-17f, COS_MAX = 1e18f; // cosine: norms that the scores can be trusted for
 
 // scratch layout (floats)
 constexpr size_t OFF_BOP = 0;                                   // [MAXM][256][32] operand B
@@ -118,7 +127,7 @@ __device__ __forceinline__ int issue_order(int p) { return ((p & 1) << 1) | (p >
 
 constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES + (size_t)NSTAGE * A_STAGE_BYTES + ((size_t)XH_RING * BM + 4 * BN * 4) * sizeof(float) + sizeof(PqBarriers) + 64;
 
-template <bool TRAIN, bool EUCLID, bool DUMP>
+template <bool TRAIN, bool COSINE, bool DUMP>
 __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constant__ CUtensorMap map_b, const PqTcParams Q)
 {
     extern __shared__ unsigned char smem_raw[];
@@ -267,7 +276,12 @@ __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constan
                 *reinterpret_cast<float4 *>(rowp + ((5 ^ sw) << 4)) = make_float4(lo[4], lo[5], lo[6], lo[7]);
                 *reinterpret_cast<float4 *>(rowp + ((6 ^ sw) << 4)) = make_float4(1.0f, 1.0f, 0.0f, 0.0f);
                 *reinterpret_cast<float4 *>(rowp + ((7 ^ sw) << 4)) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                xh_ring[(it & (XH_RING - 1)) * BM + r] = 0.5f * sq;
+                float scale = 0.5f * sq;
+                if (COSINE) {
+                    const float nx = __fsqrt_rn(sq);
+                    scale = nx >= COS_MIN && nx <= COS_MAX ? 1.25f * nx : VQB_INF;
+                }
+                xh_ring[(it & (XH_RING - 1)) * BM + r] = scale;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic writes -> visible to the MMA's reads
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&bars->afull[st]);
@@ -442,7 +456,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constan
 // Operand B of one sub-space per block (thread j = centroid j): 32 TF32 numbers per centroid
 //   [-ch(8) | -cl(8) | -ch(8) | hn_h, hn_l, 0 ...]   (columns beyond k: zeros and a huge score),
 // the binary16 image of the centroid (what an encode writes, src/pq.rs:176-180) and max_j hn_j.
-__global__ void pq_operand_b_kernel(const float *cb, int k, float *bop, uint4 *c16, float *hnmax)
+// COSINE: the centroids' unit vectors, no half norms; the "largest half norm" is 0, or infinity to void the sub-space.
+template <bool COSINE> __global__ void pq_operand_b_kernel(const float *cb, int k, float *bop, uint4 *c16, float *hnmax)
 {
     __shared__ float smax[BN];
     const int s = blockIdx.x, j = threadIdx.x;
@@ -456,14 +471,25 @@ __global__ void pq_operand_b_kernel(const float *cb, int k, float *bop, uint4 *c
         const float4 c0 = c[0], c1 = c[1];
         const float v[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
         float hi[8], lo[8], a = 0.0f;
+        if (COSINE) {
+            const float norm = norm_chain(v, 8, 1);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            hi[i] = to_tf32(v[i]);
-            lo[i] = to_tf32(v[i] - hi[i]);
-            a = fmaf(v[i], v[i], a);
+            for (int i = 0; i < 8; ++i) {
+                const float unit = norm == 0.0f ? 0.0f : __fdiv_rn(v[i], norm);
+                hi[i] = to_tf32(unit);
+                lo[i] = to_tf32(unit - hi[i]);
+            }
+            hn = norm == 0.0f || !(norm == norm) || (norm >= COS_MIN && norm <= COS_MAX) ? 0.0f : VQB_INF; // a NaN score never wins
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                hi[i] = to_tf32(v[i]);
+                lo[i] = to_tf32(v[i] - hi[i]);
+                a = fmaf(v[i], v[i], a);
+            }
+            hn = 0.5f * a;
         }
-        hn = 0.5f * a;
-        const float hh = to_tf32(hn), hl = to_tf32(hn - hh);
+        const float hh = COSINE ? 0.0f : to_tf32(hn), hl = COSINE ? 0.0f : to_tf32(hn - hh);
         out[0] = out[4] = make_float4(-hi[0], -hi[1], -hi[2], -hi[3]);
         out[1] = out[5] = make_float4(-hi[4], -hi[5], -hi[6], -hi[7]);
         out[2] = make_float4(-lo[0], -lo[1], -lo[2], -lo[3]);
@@ -492,7 +518,7 @@ __global__ void pq_operand_b_kernel(const float *cb, int k, float *bop, uint4 *c
 // The marked (row, sub-space) pairs: one warp per pair scans all centroids with the reference's arithmetic
 // (src/utils.rs:59-73, src/pq.rs:159-182): strict '<' in ascending index from centroid 0, so a NaN distance never wins
 // unless it is centroid 0's, and equal distances keep the lowest index.
-template <bool TRAIN, bool EUCLID> __global__ void __launch_bounds__(256) pq_marked_kernel(const PqTcParams Q)
+template <bool TRAIN, int METRIC> __global__ void __launch_bounds__(256) pq_marked_kernel(const PqTcParams Q)
 {
     // Each step a CTA reads 256 x 16 mark bytes (all loads independent), collects the marked pairs in shared memory --
     // the list holds the worst case of a step -- and its eight warps then take the pairs in turn, so the work is balanced
@@ -558,6 +584,7 @@ template <bool TRAIN, bool EUCLID> __global__ void __launch_bounds__(256) pq_mar
                 float x[SDW];
 #pragma unroll
                 for (int t = 0; t < SDW; ++t) x[t] = s_x[i][t];
+                const float na = METRIC == M_COSINE ? norm_chain(x, SDW, 1) : 0.0f;
                 const float *cbs = P.centroids + (size_t)s * k * SDW;
                 float bd = VQB_INF, d0 = 0.0f;
                 int bi = 0x7fffffff;
@@ -575,8 +602,9 @@ template <bool TRAIN, bool EUCLID> __global__ void __launch_bounds__(256) pq_mar
 #pragma unroll
                 for (int u = 0; u < BN / 32; ++u) {
                     const int j = lane + 32 * u;
-                    float d = reg_dist<SDW, M_SQ>(x, c[u], 0.0f, 0.0f, 0.0f);
-                    if (EUCLID) d = __fsqrt_rn(d);
+                    float d = METRIC == M_COSINE ? reg_dist<SDW, M_COSINE>(x, c[u], 0.0f, na, norm_chain(c[u], SDW, 1))
+                                                 : reg_dist<SDW, M_SQ>(x, c[u], 0.0f, 0.0f, 0.0f);
+                    if (METRIC == M_EUCLID) d = __fsqrt_rn(d);
                     if (j == 0) d0 = d;
                     if (j < k && d < bd) {
                         bd = d;
@@ -624,7 +652,7 @@ template <bool TRAIN, bool EUCLID> __global__ void __launch_bounds__(256) pq_mar
 
 bool pq_tc_applicable(const AssignParams &p, int metric)
 {
-    return (metric == M_SQ || metric == M_EUCLID) && p.sd == SDW && p.m >= 4 && p.m <= MAXM && p.m % 4 == 0 && p.k >= 2 && p.k <= BN &&
+    return (metric == M_SQ || metric == M_EUCLID || metric == M_COSINE) && p.sd == SDW && p.m >= 4 && p.m <= MAXM && p.m % 4 == 0 && p.k >= 2 && p.k <= BN &&
            p.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && p.n >= 1 && (reinterpret_cast<uintptr_t>(p.codes) & 1u) == 0 &&
            (reinterpret_cast<uintptr_t>(p.centroids) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.out_f16) & 15u) == 0 &&
            (reinterpret_cast<uintptr_t>(p.out_f32) & 15u) == 0;
@@ -634,10 +662,10 @@ size_t pq_tc_scratch_floats() { return SCRATCH_FLOATS; }
 size_t pq_tc_stats_offset_floats() { return OFF_STATS; }
 size_t pq_tc_mark_bytes(size_t n, size_t m) { return (n * (m / 2) + 15) & ~(size_t)15; } // read 16 bytes at a time
 
-template <bool TRAIN, bool EUCLID, bool DUMP = false>
+template <bool TRAIN, int METRIC, bool DUMP = false>
 static void launch_t(CudaDevice &dev, const CUtensorMap &mb, const PqTcParams &q, unsigned grid)
 {
-    auto kernel = pq_tc_kernel<TRAIN, EUCLID, DUMP>;
+    auto kernel = pq_tc_kernel<TRAIN, METRIC == M_COSINE, DUMP>;
     constexpr size_t smem = PQ_TC_SMEM;
     static std::atomic<unsigned long long> configured{0}; // bit d: the attribute has been set on device d (it is per device and sticky)
     const unsigned long long bit = 1ull << (dev.device() & 63);
@@ -656,16 +684,17 @@ static void launch_t(CudaDevice &dev, const CUtensorMap &mb, const PqTcParams &q
         // one step (4 KiB of mark bytes) per CTA where the grid allows: the steps are latency-bound and independent
         const unsigned long long steps = ((q.a.n * (unsigned long long)(q.a.m / 2) + 15) / 16 + 255) / 256;
         const unsigned mgrid = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(steps, (unsigned long long)dev.sm_count() * 64));
-        pq_marked_kernel<TRAIN, EUCLID><<<mgrid, 256, 0, dev.stream()>>>(q);
+        pq_marked_kernel<TRAIN, METRIC><<<mgrid, 256, 0, dev.stream()>>>(q);
         VQB_CUDA_CHECK(cudaGetLastError());
         dev.count_launch();
     }
 }
 
-void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, float *scratch)
+static void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, bool cosine, float *scratch)
 {
     KernelScope ks(dev, "pq_operand_b");
-    pq_operand_b_kernel<<<m, BN, 0, dev.stream()>>>(centroids, k, scratch + OFF_BOP, reinterpret_cast<uint4 *>(scratch + OFF_C16), scratch + OFF_HMAX);
+    auto kernel = cosine ? pq_operand_b_kernel<true> : pq_operand_b_kernel<false>;
+    kernel<<<m, BN, 0, dev.stream()>>>(centroids, k, scratch + OFF_BOP, reinterpret_cast<uint4 *>(scratch + OFF_C16), scratch + OFF_HMAX);
     VQB_CUDA_CHECK(cudaGetLastError());
     dev.count_launch();
 }
@@ -674,7 +703,7 @@ void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train
 {
     if (train && code_bytes != 1) throw Error(100, "pq tensor path: one-byte codes expected for k <= 256");
     float *bop = b.scratch + OFF_BOP;
-    if (b.prepare_operand) launch_pq_operand_b(dev, p.centroids, p.m, p.k, b.scratch);
+    if (b.prepare_operand) launch_pq_operand_b(dev, p.centroids, p.m, p.k, metric == M_COSINE, b.scratch);
     const CUtensorMap mb = make_tensor_map_2d(bop, KOP, (unsigned long long)p.m * BN, KOP, BN, CU_TENSOR_MAP_SWIZZLE_128B);
     PqTcParams q;
     q.a = p;
@@ -688,10 +717,11 @@ void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train
     const unsigned ngroups = (unsigned)p.m / 4;
     const unsigned per = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(tiles, (unsigned long long)dev.sm_count() / ngroups));
     const unsigned grid = per * ngroups;
-    if (b.dbg_scores) launch_t<false, false, true>(dev, mb, q, grid);
-    else if (train) launch_t<true, false>(dev, mb, q, grid);
-    else if (metric == M_EUCLID) launch_t<false, true>(dev, mb, q, grid);
-    else launch_t<false, false>(dev, mb, q, grid);
+    if (b.dbg_scores) launch_t<false, M_SQ, true>(dev, mb, q, grid);
+    else if (train) launch_t<true, M_SQ>(dev, mb, q, grid);
+    else if (metric == M_EUCLID) launch_t<false, M_EUCLID>(dev, mb, q, grid);
+    else if (metric == M_COSINE) launch_t<false, M_COSINE>(dev, mb, q, grid);
+    else launch_t<false, M_SQ>(dev, mb, q, grid);
 }
 
 // ------------------------------------------------------------------------------------------------

@@ -11,7 +11,7 @@ namespace vqb {
 class CudaDevice;
 struct AssignParams;
 
-// sub-space width 8, 4 <= m <= 64 (multiple of 4), 2 <= k <= 256, 16-byte aligned row slices, Euclidean metrics
+// sub-space width 8, 4 <= m <= 64 (multiple of 4), 2 <= k <= 256, 16-byte aligned row slices, Euclidean metrics or (encode) cosine
 bool pq_tc_applicable(const AssignParams &p, int metric);
 size_t pq_tc_scratch_floats();
 // bytes of the (row, sub-space pair) mark map for n rows of m sub-spaces
