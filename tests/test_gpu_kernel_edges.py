@@ -79,3 +79,43 @@ def test_cosine_encode_on_tensor_cores_bit_exact(oracle, n, m, k, special):
     out_o, codes_o = oracle.pq_quantize(cb, x, METRICS["CosineDistance"])
     assert np.array_equal(codes, codes_o)
     assert np.array_equal(out, out_o.view(np.float16), equal_nan=True)
+
+
+@pytest.mark.parametrize("n,dim,k", [(2000, 17, 2), (1300, 33, 31), (700, 61, 256), (1025, 100, 40), (3000, 128, 200)])
+def test_full_width_training_of_any_width_bit_exact(oracle, n, dim, k):
+    """Images padded to whole K steps (dim not a multiple of 16, rows not a multiple of 16 bytes), dead clusters, residual updates
+    with the next stage's images."""
+    from tests.golden import reference_known_answers as ka
+    x = synth.gaussian_mixture(n, dim, dim, components=5)
+    x[n // 2: n // 2 + 40] = x[3]
+    so, sg = RecordingSeeder(4), RecordingSeeder(4)
+    cb_o, _res, _norms = oracle.rvq_fit(x, 3, k, 4, 1e-6, ka.EUCLID, so.init_stage, so.draw)
+    rq = vq.ResidualQuantizer.fit(x, 3, k, 4, 1e-6, vq.Distance.Euclidean, 4, init=sg.init_stage, draw=sg.draw, accumulate=vq.ACCUM_ORDERED)
+    assert np.array_equal(rq.codebooks, cb_o) and by_stream(so.draws) == by_stream(sg.draws)
+
+
+@pytest.mark.parametrize("n,dim,k", [(180_001, 61, 40), (70_000, 128, 33)])
+def test_large_residual_encode_with_rows_that_end_early_bit_exact(oracle, n, dim, k):
+    x = synth.gaussian_mixture(n, dim, 9)
+    books = 0.1 * synth.normal(3 * k, dim, 3).reshape(3, k, dim)
+    books[0, :k // 2] = x[:k // 2]
+    books[2, 5] = books[2, 1]
+    eps = float(np.float32(np.sqrt(np.sum((x[k] - books[0, 1]).astype(np.float64) ** 2))))  # some rows end within rounding of it
+    x[100:100 + k // 2] = x[:k // 2]
+    x[n - 1, dim - 1], x[n - 2, 0] = np.nan, np.inf
+    out_o, codes_o, _ = oracle.rvq_quantize(books, eps, x, METRICS["Euclidean"])
+    out, codes = vq.ResidualQuantizer.from_codebooks(books, eps, vq.Distance.Euclidean).quantize(x, return_codes=True)
+    assert np.array_equal(codes, codes_o)
+    assert np.array_equal(out, out_o.view(np.float16), equal_nan=True)
+
+
+def test_image_dot_products_within_half_of_the_bound(ctx):
+    from tests.test_gpu_dense_tc import _dots
+    for n, dim, k, scale in ((1000, 128, 256, 1.0), (777, 61, 100, 1e3), (4097, 17, 2, 1e-4)):
+        rng = np.random.default_rng(n)
+        x, cb = (scale * rng.normal(size=(n, dim))).astype(np.float32), (scale * rng.normal(size=(k, dim))).astype(np.float32)
+        dots, _ = _dots(ctx, x, cb)
+        err = np.abs(dots[:, :k] - x.astype(np.float64) @ cb.astype(np.float64).T)
+        # (the half norm is added back in f32 for this comparison: its own rounding is allowed for)
+        norm = np.linalg.norm(x, axis=1)[:, None] * np.linalg.norm(cb, axis=1).max() + (np.linalg.norm(cb, axis=1) ** 2)[None, :] * 0.01
+        assert (err <= 3.5e-6 * norm).all(), float((err / norm).max())

@@ -79,6 +79,13 @@ int set_err(vqb_ctx *ctx, int code, const std::string &msg)
 
 template <typename F> int guarded(vqb_ctx *ctx, F &&f)
 {
+    struct AtEnd { // what the kernels of one call share goes back to the pool with it
+        vqb_ctx *ctx;
+        ~AtEnd()
+        {
+            if (ctx) ctx->dev->release_dense();
+        }
+    } at_end{ctx};
     try {
         if (ctx) ctx->dev->make_current();
         f();

@@ -65,7 +65,7 @@ CudaDevice::CudaDevice(int device) : device_(device)
         opq_tensor_enabled_ = tensor_enabled_ && !(o && *o == '0');
     }
     // the small fixed-size buffers of the tensor-core kernels exist from the start, so that no later call has to create them
-    if (tensor_enabled_) ensure_tc_buffers(0);
+    if (tensor_enabled_) ensure_tc_buffers();
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess) {
         unsigned long long keep = ~0ull; // keep freed blocks cached; repeated fits reuse them
@@ -84,13 +84,9 @@ CudaDevice::~CudaDevice()
         for (cudaEvent_t e : arrival_done_) cudaEventDestroy(e);
         if (arrival_fence_) cudaEventDestroy(arrival_fence_);
         if (stage_) cudaFreeHost(stage_);
-        cudaFree(rownorm_);
-        cudaFree(hn_scratch_);
         cudaFree(rot_split_);
         cudaFree(pq_scratch_);
         cudaFree(pq_marks_);
-        cudaFree(cand_);
-        cudaFree(list_);
         cudaFree(tc_stats_);
         cudaFree(tc_error_);
         if (status_host_) cudaFreeHost(status_host_);
@@ -343,36 +339,57 @@ void CudaDevice::download(void *dst, const void *src, size_t bytes)
 // ------------------------------------------------------------------------------------------------
 // tensor-core path plumbing (kernels in dense_tc.cu / resolve.cu)
 // ------------------------------------------------------------------------------------------------
-void CudaDevice::ensure_tc_buffers(size_t n)
+void CudaDevice::ensure_tc_buffers()
 {
-    if (!hn_scratch_) {
-        device_allocs_ += 5;
-        VQB_CUDA_CHECK(cudaMalloc(&rot_split_, opq_tc_split_floats(128) * sizeof(float)));
-        VQB_CUDA_CHECK(cudaMalloc(&hn_scratch_, 260 * sizeof(float)));
-        VQB_CUDA_CHECK(cudaMalloc(&pq_scratch_, pq_tc_scratch_floats() * sizeof(float)));
-        VQB_CUDA_CHECK(cudaMemsetAsync(pq_scratch_, 0, pq_tc_scratch_floats() * sizeof(float), stream_));
-        VQB_CUDA_CHECK(cudaMalloc(&tc_stats_, 3 * sizeof(unsigned long long)));
-        VQB_CUDA_CHECK(cudaMalloc(&tc_error_, sizeof(int)));
-        VQB_CUDA_CHECK(cudaMemsetAsync(tc_stats_, 0, 3 * sizeof(unsigned long long), stream_));
-        VQB_CUDA_CHECK(cudaMemsetAsync(tc_error_, 0, sizeof(int), stream_));
-    }
-    if (n > rows_cap_) {
-        VQB_CUDA_CHECK(cudaStreamSynchronize(stream_));
-        cudaFree(rownorm_);
-        cudaFree(cand_);
-        cudaFree(list_);
-        rownorm_ = nullptr;
-        cand_ = nullptr;
-        list_ = nullptr;
-        list_count_ = nullptr;
-        rows_cap_ = 0;
-        device_allocs_ += 3;
-        VQB_CUDA_CHECK(cudaMalloc(&rownorm_, n * sizeof(float)));
-        VQB_CUDA_CHECK(cudaMalloc(&cand_, n * DENSE_MASK_WORDS * sizeof(uint32_t)));
-        VQB_CUDA_CHECK(cudaMalloc(&list_, (n + 1) * sizeof(uint32_t))); // rows left for the exact kernel, then their count
-        list_count_ = list_ + n;
-        rows_cap_ = n;
-    }
+    if (tc_error_) return;
+    device_allocs_ += 4;
+    VQB_CUDA_CHECK(cudaMalloc(&rot_split_, opq_tc_split_floats(128) * sizeof(float)));
+    VQB_CUDA_CHECK(cudaMalloc(&pq_scratch_, pq_tc_scratch_floats() * sizeof(float)));
+    VQB_CUDA_CHECK(cudaMemsetAsync(pq_scratch_, 0, pq_tc_scratch_floats() * sizeof(float), stream_));
+    VQB_CUDA_CHECK(cudaMalloc(&tc_stats_, 3 * sizeof(unsigned long long)));
+    VQB_CUDA_CHECK(cudaMemsetAsync(tc_stats_, 0, 3 * sizeof(unsigned long long), stream_));
+    VQB_CUDA_CHECK(cudaMalloc(&tc_error_, sizeof(int)));
+    VQB_CUDA_CHECK(cudaMemsetAsync(tc_error_, 0, sizeof(int), stream_));
+}
+
+// One block for everything the full-width tensor path needs besides rows and codebooks; it lives until the end of the call
+// that needed it (release_dense), so the stages of a residual quantizer share it.
+const DenseWork &CudaDevice::dense_work(size_t n, size_t dim)
+{
+    const size_t dimp = dense_padded(dim);
+    if (dense_block_ && n <= dense_rows_ && dimp == dense_dimp_) return dense_;
+    release_dense();
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    const size_t image = up(n * 4 * dimp), norms = up(n * sizeof(float)), cand = up(n * DENSE_MASK_WORDS * sizeof(uint32_t)), list = up((n + 1) * sizeof(uint32_t)),
+                 book = up(256 * 4 * dimp), hn = up(256 * sizeof(float)), frame = up(129 * sizeof(float));
+    char *p = static_cast<char *>(alloc(image + norms + cand + list + book + hn + frame));
+    dense_block_ = p;
+    dense_rows_ = n;
+    dense_dimp_ = dimp;
+    auto take = [&](size_t bytes) {
+        char *at = p;
+        p += bytes;
+        return at;
+    };
+    dense_.image = reinterpret_cast<uint16_t *>(take(image));
+    dense_.norms = reinterpret_cast<float *>(take(norms));
+    dense_.cand = reinterpret_cast<uint32_t *>(take(cand));
+    dense_.list_count = reinterpret_cast<uint32_t *>(take(list));
+    dense_.list = dense_.list_count + 1;
+    dense_.book_image = reinterpret_cast<uint16_t *>(take(book));
+    dense_.half_norms = reinterpret_cast<float *>(take(hn));
+    dense_.frame = reinterpret_cast<float *>(take(frame));
+    return dense_;
+}
+
+void CudaDevice::release_dense()
+{
+    prepared_x_ = nullptr;
+    prepared_by_apply_ = false;
+    if (!dense_block_) return;
+    release(dense_block_);
+    dense_block_ = nullptr;
+    dense_ = DenseWork();
 }
 
 uint8_t *CudaDevice::pq_mark_buffer(size_t bytes)
@@ -406,13 +423,17 @@ void CudaDevice::check_tc_error()
 
 void CudaDevice::prepare_rows(const Shape &sh, const float *x)
 {
-    prepared_x_ = nullptr;
     bop_fresh_ = nullptr;
+    const bool by_apply = prepared_by_apply_ && prepared_x_ == x && prepared_n_ == sh.n_local && prepared_dim_ == sh.sd;
+    prepared_by_apply_ = false;
+    if (by_apply && sh.m == 1 && dense_tc_applicable(sh.sd, sh.k, M_SQ)) return; // rvq_update has just written these rows and their images
+    prepared_x_ = nullptr;
     if (!tensor_enabled_ || sh.m != 1 || sh.ld != sh.sd || sh.n_local == 0) return;
-    if (!dense_tc_applicable(sh.n_local, sh.sd, sh.k, M_SQ, x)) return;
-    ensure_tc_buffers(sh.n_local);
-    if (x == arrival_.dev) end_arrival(); // the norms need all rows: the host waits for the copies
-    dense_row_norms(*this, x, sh.n_local, sh.sd, rownorm_);
+    if (!dense_tc_applicable(sh.sd, sh.k, M_SQ)) return;
+    const DenseWork &w = dense_work(sh.n_local, sh.sd);
+    if (x == arrival_.dev) end_arrival(); // the images need all rows: the host waits for the copies
+    dense_frame(*this, w, x, sh.n_local, sh.sd, nullptr, nullptr, true);
+    dense_prepare(*this, w, x, sh.n_local, sh.sd);
     prepared_x_ = x;
     prepared_n_ = sh.n_local;
     prepared_dim_ = sh.sd;
@@ -421,11 +442,12 @@ void CudaDevice::prepare_rows(const Shape &sh, const float *x)
 void CudaDevice::dense_debug(const float *x, size_t n, size_t dim, const float *codebook, size_t k, float *dots,
                              unsigned long long *stats3)
 {
-    if (!dense_tc_applicable(n, dim, k, M_SQ, x)) throw Error(103, "shape not covered by the tensor-core path");
-    ensure_tc_buffers(n);
+    if (!tensor_enabled_ || !dense_tc_applicable(dim, k, M_SQ)) throw Error(103, "shape not covered by the tensor-core path");
+    const DenseWork &w = dense_work(n, dim);
     VQB_CUDA_CHECK(cudaMemsetAsync(tc_stats_, 0, 3 * sizeof(unsigned long long), stream_));
-    dense_row_norms(*this, x, n, dim, rownorm_);
-    dense_shortlist(*this, x, n, dim, codebook, k, rownorm_, hn_scratch_, cand_, tc_stats_, tc_error_, dots);
+    dense_frame(*this, w, x, n, dim, nullptr, nullptr, false); // the caller asked for x.c
+    dense_prepare(*this, w, x, n, dim);
+    dense_shortlist(*this, w, n, dim, codebook, k, tc_stats_, tc_error_, dots, nullptr);
     download(stats3, tc_stats_, 3 * sizeof(unsigned long long));
     prepared_x_ = nullptr;
 }
@@ -444,7 +466,6 @@ void CudaDevice::pq_tensor_debug(const float *x, size_t n, size_t m, const float
     p.out_codes = codes;
     p.x_vec4 = 1;
     if (!pq_tc_applicable(p, M_SQ)) throw Error(103, "shape not covered by the product-quantizer tensor-core path");
-    ensure_tc_buffers(0);
     bop_fresh_ = nullptr;
     unsigned long long before = 0, after = 0;
     download(&before, pq_scratch_ + pq_tc_stats_offset_floats(), sizeof before);
@@ -548,42 +569,35 @@ void CudaDevice::patch_centroids(const Shape &sh, const float *x, uint64_t row_b
 // ------------------------------------------------------------------------------------------------
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// codes[r] = the reference's nearest centroid of every row whose image is in dense_
+void CudaDevice::dense_decide(const float *x, size_t n, size_t dim, const float *codebook, size_t k, bool euclid, uint8_t *codes, uint32_t *changed,
+                              unsigned long long *stats)
+{
+    VQB_CUDA_CHECK(cudaMemsetAsync(dense_.list_count, 0, sizeof(uint32_t), stream_));
+    const ShortlistTrain tr = {codes, changed};
+    dense_shortlist(*this, dense_, n, dim, codebook, k, stats, tc_error_, nullptr, &tr);
+    dense_resolve(*this, dense_, x, n, dim, codebook, k, euclid, codes, changed);
+}
+
 void CudaDevice::assign_train(const Shape &sh, const float *x, const float *centroids, void *codes, const uint32_t *active,
                               const IterBuffers &buf)
 {
     if (sh.n_local == 0) return;
     uint32_t *changed = buf.moved;
-    if (prepared_x_ == x && prepared_n_ == sh.n_local && prepared_dim_ == sh.sd && sh.m == 1 &&
-        dense_tc_applicable(sh.n_local, sh.sd, sh.k, M_SQ, x)) {
+    if (prepared_x_ == x && prepared_n_ == sh.n_local && prepared_dim_ == sh.sd && sh.m == 1 && dense_tc_applicable(sh.sd, sh.k, M_SQ)) {
         // full-width k-means step: tensor-core shortlist, then the exact decision among the candidates
         static const bool stats_on = std::getenv("VQB_TC_STATS") != nullptr; // diagnostic: shortlist sizes per training pass on stderr
         if (stats_on) VQB_CUDA_CHECK(cudaMemsetAsync(tc_stats_, 0, 3 * sizeof(unsigned long long), stream_));
-        // the shortlist kernel decides the rows with one candidate itself and lists the others for the exact kernel
         if (code_bytes(sh.k) != 1) throw Error(103, "full-width tensor path with assignments wider than one byte");
-        VQB_CUDA_CHECK(cudaMemsetAsync(list_count_, 0, sizeof(uint32_t), stream_));
-        ShortlistTrain tr = {static_cast<uint8_t *>(codes), changed, list_, list_count_};
-        dense_shortlist(*this, x, sh.n_local, sh.sd, centroids, sh.k, rownorm_, hn_scratch_, cand_, stats_on ? tc_stats_ : nullptr, tc_error_, nullptr, &tr);
+        dense_decide(x, sh.n_local, sh.sd, centroids, sh.k, false, static_cast<uint8_t *>(codes), changed, stats_on ? tc_stats_ : nullptr);
         if (stats_on) {
             unsigned long long st3[3] = {0, 0, 0};
             download(st3, tc_stats_, sizeof st3);
             uint32_t listed = 0;
-            download(&listed, list_count_, sizeof listed);
+            download(&listed, dense_.list_count, sizeof listed);
             std::fprintf(stderr, "[vqb] shortlist: rows %llu candidates %llu (%.2f per row) full scans %llu, %u rows left for the exact kernel\n", st3[0],
                          st3[1], st3[0] ? (double)st3[1] / (double)st3[0] : 0.0, st3[2], listed);
         }
-        ResolveParams r = {};
-        r.x = x;
-        r.n = sh.n_local;
-        r.dim = (int)sh.sd;
-        r.k = (int)sh.k;
-        r.codebook = centroids;
-        r.cand = cand_;
-        r.euclid = 0;
-        r.codes = codes;
-        r.changed = changed;
-        r.list = list_;
-        r.list_count = list_count_;
-        launch_resolve(*this, r, R_TRAIN, code_bytes(sh.k));
         return;
     }
     AssignParams p = {};
@@ -599,8 +613,7 @@ void CudaDevice::assign_train(const Shape &sh, const float *x, const float *cent
     p.changed = changed;
     p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
     if (pq_tensor_enabled_ && pq_tc_applicable(p, M_SQ)) {
-        ensure_tc_buffers(0);
-        PqTcBuffers tb;
+            PqTcBuffers tb;
         tb.scratch = pq_scratch_;
         tb.marks = pq_mark_buffer(pq_tc_mark_bytes(sh.n_local, sh.m));
         tb.error_word = tc_error_;
@@ -650,8 +663,7 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
         return;
     }
     if (tensor) {
-        ensure_tc_buffers(0);
-        bop_fresh_ = nullptr;
+            bop_fresh_ = nullptr;
         PqTcBuffers tb;
         tb.scratch = pq_scratch_;
         tb.marks = pq_mark_buffer(pq_tc_mark_bytes(sh.n_local, sh.m));
@@ -691,21 +703,20 @@ void CudaDevice::rvq_update(float *res, size_t n, size_t dim, const float *centr
                             double *norm_sum)
 {
     if (n == 0) return;
-    if (tensor_enabled_ && prepared_x_ == res && prepared_n_ == n && prepared_dim_ == dim && dense_tc_applicable(n, dim, k, metric, res)) {
-        // the rows have not changed since the stage's k-means announced them, so their norms are still valid
-        dense_shortlist(*this, res, n, dim, centroids, k, rownorm_, hn_scratch_, cand_, nullptr, tc_error_, nullptr);
-        ResolveParams r = {};
-        r.x = res;
-        r.res = res;
-        r.n = n;
-        r.dim = (int)dim;
-        r.k = (int)k;
-        r.codebook = centroids;
-        r.cand = cand_;
-        r.euclid = (metric == M_EUCLID);
-        r.norm_sum = norm_sum;
-        launch_resolve(*this, r, R_RVQ_UPDATE, 4);
-        prepared_x_ = nullptr; // the residuals changed
+    if (tensor_enabled_ && prepared_x_ == res && prepared_n_ == n && prepared_dim_ == dim && dense_tc_applicable(dim, k, metric)) {
+        // the rows have not changed since the stage's k-means announced them, so their images are still valid
+        uint8_t *codes = static_cast<uint8_t *>(alloc(n));
+        dense_decide(res, n, dim, centroids, k, metric == M_EUCLID, codes, nullptr, nullptr);
+        RvqApply a;
+        a.x = a.res = res;
+        a.n = n;
+        a.dim = dim;
+        a.codebook = centroids;
+        a.codes = codes;
+        a.norm_sum = norm_sum;
+        rvq_apply(*this, a, dense_);
+        release(codes);
+        prepared_by_apply_ = true; // the next stage's images are there
         return;
     }
     prepared_x_ = nullptr;
@@ -721,21 +732,6 @@ void CudaDevice::rvq_update(float *res, size_t n, size_t dim, const float *centr
     g.pv = (float)pm;
     g.norm_sum = norm_sum;
     launch_assign_generic(*this, g, metric, G_RVQ_UPDATE, 4);
-}
-
-__global__ void f32_to_f16_kernel(const float *in, unsigned long long n, uint16_t *out)
-{
-    for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < n; i += (unsigned long long)gridDim.x * blockDim.x)
-        out[i] = f32_to_f16_bits(in[i]);
-}
-
-void CudaDevice::f32_to_f16_rows(const float *in, size_t n, uint16_t *out)
-{
-    if (n == 0) return;
-    KernelScope ks(*this, "f32_to_f16");
-    f32_to_f16_kernel<<<blocks_for(n, 256, (size_t)sm_count_ * 16), 256, 0, stream_>>>(in, n, out);
-    VQB_CUDA_CHECK(cudaGetLastError());
-    count_launch();
 }
 
 void CudaDevice::rvq_quantize(const float *x, size_t n, size_t dim, const float *codebooks, size_t stages, size_t k,
@@ -755,49 +751,43 @@ void CudaDevice::rvq_quantize(const float *x, size_t n, size_t dim, const float 
     g.out_codes = out_codes;
     g.stages = (int)stages;
     g.epsilon = epsilon;
-    const bool tensor = tensor_enabled_ && dense_tc_applicable(n, dim, k, metric, x);
+    const bool tensor = tensor_enabled_ && stages < 255 && dense_tc_applicable(dim, k, metric);
     if (direct_rvq_applicable(g, tensor, smem_limit_)) {
         launch_direct_rvq(*this, g, metric);
         return;
     }
-    if (out_codes) VQB_CUDA_CHECK(cudaMemsetAsync(out_codes, 0xFF, sizeof(uint32_t) * n * stages, stream_));
     if (tensor) {
-        // stage by stage: norms of the current residuals, tensor-core shortlist, exact resolve that subtracts the chosen
-        // centroid, adds it to the running sum and retires rows whose residual norm fell below epsilon
-        ensure_tc_buffers(n);
+        // stage by stage: codes from the rows' images, then the residuals with their images for the next stage; the sums of the
+        // chosen centroids are formed from the codes at the end
+        const DenseWork &w = dense_work(n, dim);
         prepared_x_ = nullptr;
-        float *res = (float *)alloc(sizeof(float) * n * dim), *qsum = (float *)alloc(sizeof(float) * n * dim);
-        uint8_t *done = (uint8_t *)alloc(n);
-        copy(res, x, sizeof(float) * n * dim);
-        zero(qsum, sizeof(float) * n * dim);
-        zero(done, n);
+        float *res = stages > 1 ? (float *)alloc(sizeof(float) * n * dim) : nullptr;
+        uint8_t *codes = (uint8_t *)alloc(n * (stages + 1)), *ended = codes + n * stages;
+        VQB_CUDA_CHECK(cudaMemsetAsync(ended, 0xFF, n, stream_));
+        dense_frame(*this, w, x, n, dim, nullptr, nullptr, true);
+        dense_prepare(*this, w, x, n, dim);
         for (size_t st = 0; st < stages; ++st) {
-            const float *cb = codebooks + st * k * dim;
-            dense_row_norms(*this, res, n, dim, rownorm_);
-            dense_shortlist(*this, res, n, dim, cb, k, rownorm_, hn_scratch_, cand_, nullptr, tc_error_, nullptr);
-            ResolveParams r = {};
-            r.x = res;
-            r.res = res;
-            r.n = n;
-            r.dim = (int)dim;
-            r.k = (int)k;
-            r.codebook = cb;
-            r.cand = cand_;
-            r.euclid = (metric == M_EUCLID);
-            r.qsum = qsum;
-            r.done = done;
-            r.out_codes = out_codes;
-            r.stage = (int)st;
-            r.stages = (int)stages;
-            r.epsilon = epsilon;
-            launch_resolve(*this, r, R_RVQ_STAGE, 4);
+            const float *cb = codebooks + st * k * dim, *rows = st ? res : x;
+            dense_decide(rows, n, dim, cb, k, metric == M_EUCLID, codes + st * n, nullptr, nullptr);
+            if (st + 1 == stages) break; // nothing looks at the last residual
+            RvqApply a;
+            a.x = rows;
+            a.res = res;
+            a.n = n;
+            a.dim = dim;
+            a.codebook = cb;
+            a.codes = codes + st * n;
+            a.ended = ended;
+            a.stage = (int)st;
+            a.epsilon = epsilon;
+            rvq_apply(*this, a, w);
         }
-        if (out_f16) f32_to_f16_rows(qsum, n * dim, out_f16);
-        release(done);
-        release(qsum);
+        rvq_gather(*this, codes, ended, n, dim, codebooks, k, (int)stages, out_f16, out_codes);
+        release(codes);
         release(res);
         return;
     }
+    if (out_codes) VQB_CUDA_CHECK(cudaMemsetAsync(out_codes, 0xFF, sizeof(uint32_t) * n * stages, stream_));
     launch_assign_generic(*this, g, metric, G_RVQ_QUANT, 4);
 }
 

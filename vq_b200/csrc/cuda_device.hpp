@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "backend.hpp"
+#include "dense_tc.hpp"
 #include "iter_status.cuh"
 
 namespace vqb {
@@ -70,7 +71,6 @@ class CudaDevice : public Device {
     // Not part of the training loops:
     void rvq_quantize(const float *x, size_t n, size_t dim, const float *codebooks, size_t stages, size_t k,
                       float epsilon, int metric, double p, uint16_t *out_f16, uint32_t *out_codes);
-    void f32_to_f16_rows(const float *in, size_t n, uint16_t *out);
     // Raw scores, codes and the number of pairs left to the exact scan of the product-quantizer tensor-core kernel.
     void pq_tensor_debug(const float *x, size_t n, size_t m, const float *codebooks, size_t k, float *scores, uint32_t *codes,
                          unsigned long long *marked);
@@ -89,6 +89,7 @@ class CudaDevice : public Device {
     int device() const { return device_; }
     int sm_count() const { return sm_count_; }
     size_t smem_limit() const { return smem_limit_; }
+    void release_dense(); // at the end of every call of the C ABI
     int *error_word() const { return tc_error_; } // null with VQB_NO_TENSOR=1
     uint64_t launches() const { return launches_.load(); }
     void count_launch(uint64_t n = 1) { launches_ += n; }
@@ -124,22 +125,26 @@ class CudaDevice : public Device {
     void wait_status(const StatusPage &sp, size_t m, size_t k, IterStatus &out);
     // centroids whose operand B (pq_tc.cu) the scratch currently holds, written by the fused centroid update
     const float *bop_fresh_ = nullptr;
-    // tensor-core path state (dense_tc.cu): row norms of the rows announced by prepare_rows, shortlist scratch
+    // full-width tensor path (dense_tc.cu): which rows dense_ holds the images of, and the block behind dense_
     bool tensor_enabled_ = true;
     const float *prepared_x_ = nullptr;
     size_t prepared_n_ = 0, prepared_dim_ = 0;
-    float *rownorm_ = nullptr, *hn_scratch_ = nullptr, *pq_scratch_ = nullptr;
+    bool prepared_by_apply_ = false; // by rvq_update, for the k-means of the next stage
+    DenseWork dense_;
+    void *dense_block_ = nullptr;
+    size_t dense_rows_ = 0, dense_dimp_ = 0;
+    const DenseWork &dense_work(size_t n, size_t dim);
+    void dense_decide(const float *x, size_t n, size_t dim, const float *codebook, size_t k, bool euclid, uint8_t *codes, uint32_t *changed,
+                      unsigned long long *stats);
+    float *pq_scratch_ = nullptr;
     float *rot_split_ = nullptr; // TF32 high and low parts of the rotation matrix of the current rotate_rows call (dim <= 128)
     bool opq_tensor_enabled_ = true;
     uint8_t *pq_marks_ = nullptr;
     size_t pq_marks_cap_ = 0;
     bool pq_tensor_enabled_ = false;
-    uint32_t *cand_ = nullptr;
-    uint32_t *list_ = nullptr, *list_count_ = nullptr; // rows the shortlist kernel leaves to the exact kernel (training passes)
-    size_t rows_cap_ = 0;
     unsigned long long *tc_stats_ = nullptr;
     int *tc_error_ = nullptr;
-    void ensure_tc_buffers(size_t n);
+    void ensure_tc_buffers();
     void pq_encode_impl(const Shape &sh, const float *x, const float *codebooks, int metric, double p, uint16_t *out_f16,
                         uint32_t *out_codes, float *out_f32, bool cuda_cores_only);
 

@@ -3,22 +3,32 @@
 // The residual quantizer's k-means and encode (src/rvq.rs:107,111-128,186-202) compare every row with every centroid
 // over the full dimension: a dense n x k x dim contraction.  This file ranks centroids with
 //        S_j = |c_j|^2/2 - x.c_j          (|x - c_j|^2 = |x|^2 + 2 S_j)
-// where the dot products come from tcgen05.mma (TF32 inputs, f32 accumulation in tensor memory), keeps for every row
-// the SHORTLIST of centroids whose S lies within a proven error bound of the smallest one, and hands the shortlist
-// to resolve kernels (resolve.cuh) that evaluate only those candidates with the reference's exact f32 arithmetic in
-// ascending index order.  The final choice is therefore the reference's; the tensor cores only prune.
+// where the dot products come from tcgen05.mma (binary16 inputs, f32 accumulation in tensor memory), keeps for every row
+// the SHORTLIST of centroids whose S lies within a proven error bound of the smallest one, decides the rows with a single
+// candidate and hands the others to a resolve kernel (resolve.cu) that evaluates only their candidates with the reference's
+// exact f32 arithmetic.  The final choice is therefore the reference's; the tensor cores only prune.
 //
-// Bound.  TF32 keeps 10 mantissa bits of each operand (the low 13 bits of the f32 container are ignored), so
-//   |dot_tc - x.c| <= (2^-10 + 2^-10 + 2^-20 + 2 K 2^-24) sum|x_i c_ji| <= 2.1e-3 |x| |c_j|        (K <= 128)
+// Operands.  Rows and centroids move into a common frame, v = s (x - mu): distances scale by s, while |x||c|, which the error
+// bound grows with, loses the rows' common part.  mu is about the mean and s about the inverse size of a sample of 256 rows
+// (dense_frame_kernel; any values are correct).  v is split into two binary16 numbers, v = h + l + e (the "image" of a row: as many
+// bytes as the row itself), and three products are added up: h.ch + h.cl + l.ch.  With one TF32 product (bound 2.1e-3 |x||c|)
+// between 15 and 94 % of the rows of a Gaussian mixture went to the exact kernel, which then took 0.31 ms per pass over
+// 1M x 128 rows beside 0.13 ms for the shortlist; bf16 instead of binary16 (bound 5.5e-5) still left 50 % in the first stage.
+// Three products take 1.4 times as many MMAs, 24 per tile, which hide behind the row traffic.  The images are written where
+// the rows are touched anyway (dense_prepare_kernel, rvq_apply_kernel); any width up to 128 is padded to whole K steps there.
+//
+// Bound, in the frame.  |l.cl| + |e.c| + |v.ec| <= 3.01 * 2^-22 sum|v_i c_ji| (l below binary16's normal range: 2^-25 absolute
+// instead, <= 2^-25 sqrt(dim) (|v| + |c|)); 25 accumulation steps, each at most 2^-22:
+//   |dot_tc - v.c| <= 7e-6 |v| |c_j| + 4e-7 (|v| + |c_j|) =: E
 // and with the reference's own chain error (<= (dim + 2) 2^-24 relative on the distance) the winner w satisfies
-//   S_w <= S_min + 2 E + 1.05 (dim + 6) 2^-24 (|x|^2 + 2 S_min + 2 E),   E = 2.1e-3 |x| max_j |c_j|.
+//   S_w <= S_min + 2 E + 1.05 (dim + 6) 2^-24 (|v|^2 + 2 S_min + 2 E).
 // Everything not finite falls out of the comparisons and marks the row for a full exact scan.
 //
 // Kernel layout (one CTA per SM, persistent over 128-row tiles):
-//   warp 0      TMA producer: the codebook once (k x dim, resident in shared memory), then row tiles in 128-byte
+//   warp 0      TMA producer: the codebook's image once (resident in shared memory), then the rows' images in 128-byte
 //               column chunks through a 5-stage ring (cp.async.bulk.tensor, 128B swizzle, no multicast)
-//   warp 1      allocates tensor memory and issues tcgen05.mma M128 x N256 x K8 (kind::tf32); two 256-column
-//               accumulators so the next tile's MMAs overlap this tile's epilogue.  One more K = 8 step per tile multiplies
+//   warp 1      allocates tensor memory and issues tcgen05.mma M128 x N256 x K16 (kind::f16); two 256-column
+//               accumulators so the next tile's MMAs overlap this tile's epilogue.  One K = 8 step of kind::tf32 per tile multiplies
 //               a constant (1, 1, 0, ...) row operand with (-hn_h, -hn_l, 0, ...) per centroid, so the accumulator holds
 //               D = x.c - |c|^2/2 = -S and the epilogue never touches the half norms
 //   warps 2..5  epilogue: tcgen05.ld the 128 x 256 values, one row per lane; pass 1 finds the largest D (3-input max), pass 2
@@ -30,6 +40,7 @@
 #include <mutex>
 
 #include "cuda_device.hpp"
+#include "dense_image.cuh"
 #include "dense_tc.hpp"
 #include "kernels_common.cuh"
 #include "tma_host.hpp"
@@ -41,9 +52,9 @@ namespace {
 
 constexpr int BM = 128;          // rows per tile (= TMEM lanes)
 constexpr int BN = 256;          // centroids per tile (= accumulator columns)
-constexpr int CHUNK = 32;        // f32 per 128-byte swizzle row
+constexpr int CHUNK = 64;        // binary16 values per 128-byte swizzle row
 constexpr int NSTAGE = 5;        // row-tile ring depth (stages of 128 rows x 128 bytes)
-constexpr int MAX_KCHUNKS = 4;   // dim <= 128
+constexpr int MAX_KCHUNKS = 4;   // images of up to 2 x 128 values
 constexpr uint32_t X_STAGE_BYTES = BM * 128;
 constexpr uint32_t C_CHUNK_BYTES = BN * 128;
 
@@ -55,10 +66,10 @@ struct alignas(8) Barriers {
 
 struct ShortlistParams {
     unsigned long long n;
-    int dim, k, kchunks;
-    const float *hn;      // [256] |c_j|^2 / 2, +inf beyond k
-    const float *cmax;    // [1]   max_j |c_j|
-    const float *xnorm2;  // [n]   |x|^2 per row
+    int dim, k, ksteps;   // ksteps: K = 16 steps of one part (h or l) of an image
+    const float *hn;      // [256] |c_j|^2 / 2 in the frame, +inf beyond k
+    const float *frame;
+    const float *xnorm2;  // [n]   |v|^2 per row, an upper bound
     uint32_t *cand;       // [n][8] bit j set = centroid j may be the reference's choice (all k bits set: examine all)
     unsigned long long *stats; // [0] rows, [1] candidates, [2] rows needing a full scan   (may be null)
     float *debug_dots;    // [n][256] raw tensor-core dot products (may be null)
@@ -66,7 +77,7 @@ struct ShortlistParams {
     // training passes (codes != null): a row with a single candidate gets its assignment here; the others are appended to
     // `list` (and only they get their mask written)
     uint8_t *codes;        // [n] previous assignment in, new assignment out
-    uint32_t *changed;     // VQB_MOVED_BITS is OR-ed in when a row moved
+    uint32_t *changed;     // VQB_MOVED_BITS is OR-ed in when a row moved (may be null)
     uint32_t *list;        // [n] rows left for the exact decision
     uint32_t *list_count;  // [1] zero on entry
 };
@@ -88,7 +99,7 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned long long n_tiles = (P.n + BM - 1) / BM;
-    const int kchunks = P.kchunks;
+    const int kchunks = (2 * P.ksteps + 3) / 4; // 64-element pieces of an image
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
@@ -104,8 +115,12 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    __shared__ uint32_t s_hmax;
+    if (threadIdx.x == 0) s_hmax = 0u;
+    __syncthreads();
     for (int t = threadIdx.x; t < BN; t += blockDim.x) {
         const float hn = P.hn[t]; // +inf beyond k
+        if (t < P.k) atomicMax(&s_hmax, __float_as_uint(fmaxf(hn, 0.0f))); // the largest half norm (NaN counts as 0)
         hn_s[t] = hn;
         const bool pad = !(hn < VQB_DENSE_INF);
         const float hh = pad ? 1e30f : tf32_round(hn), hl = pad ? 0.0f : tf32_round(hn - hh);
@@ -180,10 +195,19 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t adesc = smem_desc_sw128(smem_u32(x_smem + (size_t)s * X_STAGE_BYTES));
-                    const uint64_t bdesc = smem_desc_sw128(smem_u32(c_smem + (size_t)kc * C_CHUNK_BYTES));
-#pragma unroll
-                    for (int k8 = 0; k8 < CHUNK / 8; ++k8) // 8 f32 = 32 bytes = 2 descriptor units per MMA step
-                        umma_tf32(d_tmem, adesc + (uint64_t)(2 * k8), bdesc + (uint64_t)(2 * k8), (kc | k8) ? 1u : 0u);
+                    auto book = [&](int step) { // descriptor of K step `step` of the codebook's image
+                        return smem_desc_sw128(smem_u32(c_smem + (size_t)(step >> 2) * C_CHUNK_BYTES)) + (uint64_t)(2 * (step & 3));
+                    };
+                    for (int i = 0; i < 4 && 4 * kc + i < 2 * P.ksteps; ++i) { // 16 bf16 = 32 bytes = 2 descriptor units per step
+                        const int j = 4 * kc + i;
+                        const uint64_t a = adesc + (uint64_t)(2 * i);
+                        if (j < P.ksteps) { // h.ch and h.cl
+                            umma_f16(d_tmem, a, book(j), j ? 1u : 0u);
+                            umma_f16(d_tmem, a, book(P.ksteps + j), 1u);
+                        } else { // l.ch
+                            umma_f16(d_tmem, a, book(j - P.ksteps), 1u);
+                        }
+                    }
                     umma_commit(&bars->empty[s]); // the stage is free once these MMAs have read it
                 }
                 if (ok) {
@@ -195,7 +219,9 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
     } else {
         // ------------------------------------------------ epilogue: one row per lane
         const int q = warp & 3; // TMEM lane quadrant this warp may read
-        const float cmax = *P.cmax;
+        const float cmax = sqrtf(2.0f * __uint_as_float(s_hmax)) * 1.00002f;
+        // in the frame: what underflows in the reference's products, and distances that could overflow there
+        const float s2 = P.frame[FRAME_SCALE] * P.frame[FRAME_SCALE], tiny = 1e-36f * s2, huge = fminf(1e37f * s2, 1e37f);
         unsigned long long cand_total = 0, full_scans = 0, rows_done = 0;
         bool moved = false;
         uint32_t local = 0;
@@ -221,7 +247,7 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
                 tmem_ld32_issue(taddr + (cb + 1) * 32, rb);
                 if (P.debug_dots && valid) {
 #pragma unroll
-                    for (int t = 0; t < 32; ++t) P.debug_dots[row * BN + cb * 32 + t] = (cb * 32 + t < P.k) ? __uint_as_float(ra[t]) + hn_s[cb * 32 + t] : 0.0f;
+                    for (int t = 0; t < 32; ++t) P.debug_dots[row * BN + cb * 32 + t] = (cb * 32 + t < P.k) ? (__uint_as_float(ra[t]) + hn_s[cb * 32 + t]) / s2 : 0.0f;
                 }
                 if (cb == 0) {
                     const float s0 = __uint_as_float(ra[0]);
@@ -239,7 +265,7 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
                 if (P.debug_dots && valid) {
 #pragma unroll
                     for (int t = 0; t < 32; ++t)
-                        P.debug_dots[row * BN + (cb + 1) * 32 + t] = ((cb + 1) * 32 + t < P.k) ? __uint_as_float(rb[t]) + hn_s[(cb + 1) * 32 + t] : 0.0f;
+                        P.debug_dots[row * BN + (cb + 1) * 32 + t] = ((cb + 1) * 32 + t < P.k) ? (__uint_as_float(rb[t]) + hn_s[(cb + 1) * 32 + t]) / s2 : 0.0f;
                 }
 #pragma unroll
                 for (int t = 0; t < 32; t += 8) {
@@ -251,16 +277,16 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
                 tmem_wait();
             }
             const float best = -fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)); // smallest score
-            // E = 2.1e-3 |x| cmax (+ the rounding of the half norms);
+            // E as above with max_j |c_j| (+ the rounding of the half norms: 10 operations in a tree, split into two TF32 numbers);
             // limit = best + 2E + 1.05 (dim + 6) u (|x|^2 + 2 best + 2E) + rounding slack of the comparison itself
-            const float e2 = 2.0f * 2.1e-3f * sqrtf(xn2) * cmax + 8e-6f * cmax * cmax;
+            const float xn = sqrtf(xn2), e2 = 2.0f * (7e-6f * xn * cmax + 4e-7f * (xn + cmax)) + 1.2e-6f * cmax * cmax;
             const float d_a = fmaxf(xn2 + 2.0f * best + e2, 0.0f);
-            const float limit = best + e2 + 1.05f * (float)(P.dim + 6) * 5.9604645e-8f * d_a + 2.4e-7f * (fabsf(best) + e2) + 1e-36f;
+            const float limit = best + e2 + 1.05f * (float)(P.dim + 6) * 5.9604645e-8f * d_a + 2.4e-7f * (fabsf(best) + e2) + tiny;
             const float lim_d = -limit; // centroid j is a candidate when D_j >= lim_d
             // a row the comparisons cannot rank (NaN / infinity somewhere, or centroid 0 not comparable, on which the
             // reference's scan depends) is handed over with every centroid marked
             // (also when a true distance could overflow f32: then the reference's own comparisons see infinities)
-            const bool scan_all = col0_nan || !(best == best) || !(limit == limit) || !(fabsf(limit) < VQB_DENSE_INF) || !(xn2 + cmax * cmax < 1e37f);
+            const bool scan_all = col0_nan || !(best == best) || !(limit == limit) || !(fabsf(limit) < VQB_DENSE_INF) || !(xn2 + cmax * cmax < huge);
 
             // pass 2: one bit per centroid, set when D_j >= lim_d.  The sign of (D_j - lim_d) is shifted into the word,
             // so the bits arrive in reverse order and inverted.
@@ -325,7 +351,7 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
                 }
             }
         }
-        if (P.codes && __any_sync(0xffffffffu, moved) && lane == 0) atomicOr(P.changed, VQB_MOVED_BITS);
+        if (P.codes && P.changed && __any_sync(0xffffffffu, moved) && lane == 0) atomicOr(P.changed, VQB_MOVED_BITS);
         if (P.stats) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
@@ -350,77 +376,115 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
     }
 }
 
-// |c_j|^2 / 2 for j < k (+inf beyond) and max_j |c_j|
-// One CTA of eight warps; a warp takes every eighth centroid, its lanes the row's 16-byte pieces (dim <= 128 on this path), so
-// all of a warp's rows are in flight together.  The order in which a row's squares are added is free: the shortlist's bound
-// carries (dim + 1) roundings of slack for the half norms.  (One thread per centroid walking its row took 23 us per launch,
-// 2 ms over a residual-quantizer fit.)
-__global__ void __launch_bounds__(256) codebook_norms_kernel(const float *c, int k, int dim, float *hn, float *cmax)
+// The frame from a sample of 256 rows (or residuals x - centroid): eight groups of 32 rows, the median of the groups' means per
+// dimension and the median of the groups' largest norms, so that a few wild rows do not move it.  Only precision depends on
+// it.  s maps that norm to [32, 64): binary16 then reaches a thousand times further up, and its l parts stay normal.
+__device__ __forceinline__ float upper_median8(float (&v)[8])
 {
-    __shared__ float smax[256];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int dim4 = dim >> 2;
-    smax[threadIdx.x] = 0.0f;
-    hn[threadIdx.x] = VQB_DENSE_INF; // entries at and beyond k stay at +inf
-    __syncthreads();
-    float part[32];
 #pragma unroll
-    for (int t = 0; t < 32; ++t) {
-        const int j = warp + 8 * t;
-        float a = 0.0f;
-        if (j < k && lane < dim4) {
-            const float4 v = __ldg(reinterpret_cast<const float4 *>(c + (size_t)j * dim) + lane);
-            a = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
+    for (int i = 1; i < 8; ++i)
+#pragma unroll
+        for (int j = 7; j >= i; --j) {
+            const float lo = fminf(v[j - 1], v[j]), hi = fmaxf(v[j - 1], v[j]);
+            v[j - 1] = lo, v[j] = hi;
         }
-        part[t] = a;
-    }
-#pragma unroll
-    for (int t = 0; t < 32; ++t) {
-        float a = part[t];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        const int j = warp + 8 * t;
-        if (lane == 0 && j < k) {
-            hn[j] = 0.5f * a;
-            smax[j] = sqrtf(a);
-        }
-    }
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) smax[threadIdx.x] = fmaxf(smax[threadIdx.x], smax[threadIdx.x + o]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *cmax = smax[0] * 1.000001f;
+    return v[4];
 }
 
-__global__ void row_norms_kernel(const float *x, unsigned long long n, int dim, float *out)
+__global__ void __launch_bounds__(1024) dense_frame_kernel(const float *__restrict__ x, unsigned long long n, int dim, const float *__restrict__ book,
+                                                           const uint8_t *__restrict__ codes, int center, float *frame)
 {
-    const int lane = threadIdx.x & 31;
-    const unsigned long long warps = (unsigned long long)gridDim.x * (blockDim.x >> 5);
-    for (unsigned long long row = blockIdx.x * (unsigned long long)(blockDim.x >> 5) + (threadIdx.x >> 5); row < n; row += warps) {
-        float a = 0.0f;
-        for (int i = lane; i < dim; i += 32) {
-            const float v = x[row * dim + i];
-            a = fmaf(v, v, a);
-        }
+    __shared__ float s_mean[8][128], s_sq[8][32][4], s_big[8], s_mu[128];
+    const int d = threadIdx.x & 127, g = threadIdx.x >> 7, lane = threadIdx.x & 31, quarter = d >> 5;
+    float v[32], sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        const unsigned long long row = (unsigned long long)(g * 32 + i) * n / 256;
+        float t = d < dim ? x[row * dim + d] : 0.0f;
+        if (codes && d < dim) t -= book[(size_t)codes[row] * dim + d];
+        v[i] = fabsf(t) < VQB_DENSE_INF ? t : 0.0f; // what is not finite has no say
+        sum += v[i] * 0.03125f;
+    }
+    s_mean[g][d] = sum;
+    __syncthreads();
+    if (g == 0) {
+        float m[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m[i] = s_mean[i][d];
+        const float mu = center ? upper_median8(m) : 0.0f;
+        s_mu[d] = fabsf(mu) < VQB_DENSE_INF ? mu : 0.0f;
+        frame[d] = s_mu[d];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        float a = d < dim ? v[i] - s_mu[d] : 0.0f;
+        a *= a;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) out[row] = a * 1.00001f; // an upper bound is what the filter needs
+        if (lane == 0) s_sq[g][i][quarter] = a;
+    }
+    __syncthreads();
+    if (d < 32) {
+        const float a = s_sq[g][d][0] + s_sq[g][d][1] + s_sq[g][d][2] + s_sq[g][d][3];
+        const uint32_t big = __reduce_max_sync(0xffffffffu, a < VQB_DENSE_INF ? __float_as_uint(a) : 0u);
+        if (d == 0) s_big[g] = __uint_as_float(big);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        float m[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m[i] = s_big[i];
+        const float norm = sqrtf(upper_median8(m));
+        const int e = norm > 0.0f && norm < VQB_DENSE_INF ? 5 - ilogbf(norm) : 0;
+        frame[FRAME_SCALE] = ldexpf(1.0f, max(-40, min(40, e)));
     }
 }
 
-CUtensorMap make_map(const float *ptr, unsigned long long rows, int dim, int box_rows)
+// A warp per centroid: image and half norm (zeros and +inf at and beyond k)
+__global__ void __launch_bounds__(256) dense_codebook_kernel(const float *c, int k, int dim, int dimp, const float *frame, uint16_t *image, float *hn)
 {
-    return make_tensor_map_2d(ptr, (unsigned long long)dim, rows, CHUNK, (unsigned)box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+    const int j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const bool in = j < k;
+    float v[4];
+    load_piece<false>(v, c, j, lane, in, dim);
+    FramePiece f = load_frame(frame, lane);
+    if (!in) f.mu[0] = f.mu[1] = f.mu[2] = f.mu[3] = 0.0f;
+    float a = store_image(image + (size_t)j * 2 * dimp, dimp, lane, v, f, true);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) hn[j] = in ? 0.5f * a : VQB_DENSE_INF;
+}
+
+// Images and (upper bounds of the) squared norms of the rows: one read, one write of the same size.  L lanes per row (8, 16 or
+// 32), four values each, so that a warp's loads and stores are whole lines.
+template <int L, bool VEC>
+__global__ void __launch_bounds__(256) dense_prepare_kernel(const float *__restrict__ x, unsigned long long n, int dim, int dimp, const float *frame,
+                                                            uint16_t *image, float *norms)
+{
+    const int lane = threadIdx.x & 31, piece = lane % L;
+    const FramePiece f = load_frame(frame, piece);
+    const unsigned long long step = (unsigned long long)gridDim.x * (256 / L);
+    for (unsigned long long row = blockIdx.x * (unsigned long long)(256 / L) + threadIdx.x / L; row - threadIdx.x / L < n; row += step) {
+        float v[4];
+        load_piece<VEC>(v, x, row, piece, row < n, dim);
+        float a = store_image(image + (size_t)row * 2 * dimp, dimp, piece, v, f, row < n);
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (row < n && piece == 0) norms[row] = a * 1.00001f; // an upper bound is what the shortlist needs
+    }
+}
+
+CUtensorMap make_map(const uint16_t *image, unsigned long long rows, int dimp, int box_rows)
+{
+    return make_tensor_map_2d(image, 2 * (unsigned long long)dimp, rows, CHUNK, (unsigned)box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 } // namespace
 
-bool dense_tc_applicable(size_t n, size_t dim, size_t k, int metric, const float *x)
+bool dense_tc_applicable(size_t dim, size_t k, int metric)
 {
-    (void)n;
-    return (metric == 0 || metric == 1) && dim >= 32 && dim <= 128 && dim % 32 == 0 && k >= 2 && k <= 256 &&
-           (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    return (metric == M_SQ || metric == M_EUCLID) && dim > 16 && dim <= 128 && k >= 2 && k <= 256;
 }
 
 size_t dense_tc_smem_bytes()
@@ -428,45 +492,61 @@ size_t dense_tc_smem_bytes()
     return 1024 + (size_t)MAX_KCHUNKS * C_CHUNK_BYTES + (size_t)NSTAGE * X_STAGE_BYTES + BN * sizeof(float) + (size_t)(BM + BN) * 32 + sizeof(Barriers) + 64;
 }
 
-void dense_row_norms(CudaDevice &dev, const float *x, size_t n, size_t dim, float *out)
+void dense_frame(CudaDevice &dev, const DenseWork &w, const float *x, size_t n, size_t dim, const float *codebook, const uint8_t *codes, bool center)
 {
     if (n == 0) return;
-    KernelScope ks(dev, "row_norms");
-    const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((n + 7) / 8, (size_t)dev.sm_count() * 8));
-    row_norms_kernel<<<grid, 256, 0, dev.stream()>>>(x, n, (int)dim, out);
+    KernelScope ks(dev, "dense_frame");
+    dense_frame_kernel<<<1, 1024, 0, dev.stream()>>>(x, n, (int)dim, codebook, codes, center ? 1 : 0, w.frame);
     VQB_CUDA_CHECK(cudaGetLastError());
     dev.count_launch();
 }
 
-void dense_shortlist(CudaDevice &dev, const float *x, size_t n, size_t dim, const float *codebook, size_t k, const float *xnorm2,
-                     float *hn_scratch /* 257 floats */, uint32_t *cand, unsigned long long *stats, int *error_word, float *debug_dots,
-                     const ShortlistTrain *train)
+void dense_prepare(CudaDevice &dev, const DenseWork &w, const float *x, size_t n, size_t dim)
 {
     if (n == 0) return;
+    KernelScope ks(dev, "dense_prepare");
+    const int dimp = (int)dense_padded(dim);
+    const bool vec = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    auto go = [&](auto kernel, int lanes) {
+        const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((n * lanes + 255) / 256, (size_t)dev.sm_count() * 32));
+        kernel<<<grid, 256, 0, dev.stream()>>>(x, n, (int)dim, dimp, w.frame, w.image, w.norms);
+    };
+    if (dimp <= 32) vec ? go(dense_prepare_kernel<8, true>, 8) : go(dense_prepare_kernel<8, false>, 8);
+    else if (dimp <= 64) vec ? go(dense_prepare_kernel<16, true>, 16) : go(dense_prepare_kernel<16, false>, 16);
+    else vec ? go(dense_prepare_kernel<32, true>, 32) : go(dense_prepare_kernel<32, false>, 32);
+    VQB_CUDA_CHECK(cudaGetLastError());
+    dev.count_launch();
+}
+
+void dense_shortlist(CudaDevice &dev, const DenseWork &w, size_t n, size_t dim, const float *codebook, size_t k, unsigned long long *stats,
+                     int *error_word, float *debug_dots, const ShortlistTrain *train)
+{
+    if (n == 0) return;
+    const int dimp = (int)dense_padded(dim);
     {
-        KernelScope ks(dev, "codebook_norms");
-        codebook_norms_kernel<<<1, 256, 0, dev.stream()>>>(codebook, (int)k, (int)dim, hn_scratch, hn_scratch + 256);
+        KernelScope ks(dev, "dense_codebook");
+        dense_codebook_kernel<<<BN / 8, 256, 0, dev.stream()>>>(codebook, (int)k, (int)dim, dimp, w.frame, w.book_image, w.half_norms);
         VQB_CUDA_CHECK(cudaGetLastError());
         dev.count_launch();
     }
-    const CUtensorMap mx = make_map(x, n, (int)dim, BM);
-    const CUtensorMap mc = make_map(codebook, k, (int)dim, BN);
+    const CUtensorMap mx = make_map(w.image, n, dimp, BM);
+    const CUtensorMap mc = make_map(w.book_image, BN, dimp, BN);
     ShortlistParams p;
     p.n = n;
     p.dim = (int)dim;
     p.k = (int)k;
-    p.kchunks = (int)(dim / CHUNK);
-    p.hn = hn_scratch;
-    p.cmax = hn_scratch + 256;
-    p.xnorm2 = xnorm2;
-    p.cand = cand;
+    p.ksteps = dimp / 16;
+    p.hn = w.half_norms;
+    p.frame = w.frame;
+    p.xnorm2 = w.norms;
+    p.cand = w.cand;
     p.stats = stats;
     p.debug_dots = debug_dots;
     p.error = error_word;
     p.codes = train ? train->codes : nullptr;
     p.changed = train ? train->changed : nullptr;
-    p.list = train ? train->list : nullptr;
-    p.list_count = train ? train->list_count : nullptr;
+    p.list = w.list;
+    p.list_count = w.list_count;
     const size_t smem = dense_tc_smem_bytes();
     VQB_CUDA_CHECK(cudaFuncSetAttribute(dense_shortlist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned long long tiles = (n + BM - 1) / BM;

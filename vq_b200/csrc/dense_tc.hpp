@@ -1,4 +1,5 @@
-// dense_tc.hpp -- tensor-core shortlist + exact resolve for full-width nearest-centroid search (dense_tc.cu, resolve.cu).
+// dense_tc.hpp -- full-width nearest-centroid search: tensor-core shortlist (dense_tc.cu), exact decision and what follows it in
+// the residual quantizer (resolve.cu).
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -10,51 +11,62 @@ class CudaDevice;
 #define DENSE_MASK_WORDS 8 /* 256 candidate bits per row (32 bytes) */
 #define VQB_DENSE_INF __int_as_float(0x7f800000)
 
-// Squared-Euclidean / Euclidean, 32 <= dim <= 128 in steps of 32, 2 <= k <= 256, 16-byte aligned rows.
-bool dense_tc_applicable(size_t n, size_t dim, size_t k, int metric, const float *x);
+// Squared-Euclidean / Euclidean, 16 < dim <= 128, 2 <= k <= 256.  (Narrower rows fill a fraction of a K step and of a line;
+// the register kernels serve them.)
+bool dense_tc_applicable(size_t dim, size_t k, int metric);
 size_t dense_tc_smem_bytes();
-// out[r] >= |x_r|^2 (tight upper bound)
-void dense_row_norms(CudaDevice &dev, const float *x, size_t n, size_t dim, float *out);
-// cand[r][0..8): 256-bit mask, bit j set for every centroid that can be the reference's choice for row r; rows that
-// cannot be ranked (NaN / infinity) come back with all k bits set.
-// With `train` (k-means passes; assignments are one byte here, k <= 256) the kernel also decides every row that has a single
-// candidate -- codes[r] is rewritten, train->changed gets VQB_MOVED_BITS when a row moved -- and appends the other rows to
-// train->list (count in *train->list_count, zero on entry); only those rows get their mask written.
+// a row's image is 2 * dense_padded(dim) binary16 values (dense_image.cuh)
+inline size_t dense_padded(size_t dim) { return (dim + 15) / 16 * 16; }
+
+// Device memory of one fit or encode, for up to a given number of rows.
+struct DenseWork {
+    uint16_t *image = nullptr;      // [n][2 * dense_padded(dim)]
+    float *norms = nullptr;         // [n] upper bounds of |s (x - mu)|^2
+    uint32_t *cand = nullptr;       // [n][8] bit j set: centroid j may be the reference's choice (all k bits set: examine all)
+    uint32_t *list = nullptr;       // [n] rows with more than one candidate
+    uint32_t *list_count = nullptr;
+    uint16_t *book_image = nullptr; // [256][2 * dense_padded(dim)]
+    float *half_norms = nullptr;    // [256]
+    float *frame = nullptr;         // [129] mu and s (dense_image.cuh)
+};
+
+// w.frame for these rows, or (codes != null) for their residuals x - centroid; center = false: mu = 0
+void dense_frame(CudaDevice &dev, const DenseWork &w, const float *x, size_t n, size_t dim, const float *codebook, const uint8_t *codes, bool center);
+// image and norms of the rows in w.frame
+void dense_prepare(CudaDevice &dev, const DenseWork &w, const float *x, size_t n, size_t dim);
+
+// Decides every row that has a single candidate -- codes[r] is rewritten, *changed gets VQB_MOVED_BITS when a row moved -- and
+// appends the other rows (also those that cannot be ranked: NaN, infinity) to w.list with their masks in w.cand
+// (*w.list_count zero on entry).  Without `train` all rows get their mask and nothing else happens (diagnostics).
 struct ShortlistTrain {
     uint8_t *codes;
     uint32_t *changed;
-    uint32_t *list;
-    uint32_t *list_count;
 };
-void dense_shortlist(CudaDevice &dev, const float *x, size_t n, size_t dim, const float *codebook, size_t k, const float *xnorm2,
-                     float *hn_scratch /* 257 floats */, uint32_t *cand, unsigned long long *stats, int *error_word, float *debug_dots,
-                     const ShortlistTrain *train = nullptr);
+void dense_shortlist(CudaDevice &dev, const DenseWork &w, size_t n, size_t dim, const float *codebook, size_t k, unsigned long long *stats,
+                     int *error_word, float *debug_dots, const ShortlistTrain *train);
 
-enum : int { R_TRAIN = 0, R_RVQ_UPDATE = 1, R_RVQ_STAGE = 2 };
+// The listed rows: the reference's own arithmetic over their candidates.
+void dense_resolve(CudaDevice &dev, const DenseWork &w, const float *x, size_t n, size_t dim, const float *codebook, size_t k, bool euclid,
+                   uint8_t *codes, uint32_t *changed);
 
-struct ResolveParams {
-    const float *x; // n rows of dim floats (R_RVQ_UPDATE / R_RVQ_STAGE: the residuals, updated in place through `res`)
-    unsigned long long n;
-    int dim, k;
-    const float *codebook; // [k][dim]
-    const uint32_t *cand;  // [n][DENSE_MASK_WORDS]
-    int euclid;            // compare square roots (Distance::Euclidean) instead of squared sums
-    // R_TRAIN: only the rows in list[0 .. *list_count) are looked at (the shortlist kernel decided the others)
-    void *codes;
-    uint32_t *changed;
-    const uint32_t *list;
-    const uint32_t *list_count;
-    // R_RVQ_UPDATE, R_RVQ_STAGE
-    float *res;
-    double *norm_sum;
-    // R_RVQ_STAGE
-    float *qsum;         // [n][dim] running sum of chosen centroids
-    uint8_t *done;       // [n] row stopped early (src/rvq.rs:204-207)
-    uint32_t *out_codes; // [n][stages] or null
-    int stage, stages;
-    float epsilon;
+// One step of the residual quantizer after a row's code is known: res = x - centroid (x may be res), and the new rows' images
+// and norms, in a new frame, for the next stage.
+struct RvqApply {
+    const float *x = nullptr;
+    float *res = nullptr;
+    size_t n = 0, dim = 0;
+    const float *codebook = nullptr;
+    const uint8_t *codes = nullptr;
+    double *norm_sum = nullptr;  // training: the residual norms are added up (src/rvq.rs:131-138)
+    uint8_t *ended = nullptr;    // encode: number of stages of rows that have ended early (src/rvq.rs:204-207), else 255
+    int stage = 0;
+    float epsilon = 0.0f;
 };
+void rvq_apply(CudaDevice &dev, const RvqApply &a, const DenseWork &w);
 
-void launch_resolve(CudaDevice &dev, const ResolveParams &p, int mode, size_t code_bytes);
+// Encode, at the end: sums of the chosen centroids in stage order as binary16 (src/rvq.rs:203,209-213) and the codes.
+// codes: [stages][n]; ended as above.
+void rvq_gather(CudaDevice &dev, const uint8_t *codes, const uint8_t *ended, size_t n, size_t dim, const float *codebooks, size_t k, int stages,
+                uint16_t *out_f16, uint32_t *out_codes);
 
 } // namespace vqb

@@ -1,13 +1,10 @@
-// resolve.cu -- exact decision among shortlisted centroids (the second half of the tensor-core path, dense_tc.cu).
-//
-// For every row the shortlist holds, in ascending order, every centroid that can be the reference's choice.  Here each
-// candidate's distance is evaluated with the reference's own f32 arithmetic (src/vector.rs:198-220, src/distances.rs:
-// 130-140) and compared with strict '<', so the outcome equals the reference's full scan; rows marked "scan all" get that
-// full scan.  The epilogue is the caller's: new assignment (training), residual update (src/rvq.rs:127,133-138), or one
-// stage of the residual encoder (src/rvq.rs:186-207).
+// resolve.cu -- exact decision among shortlisted centroids (the second half of the tensor-core path, dense_tc.cu) and what the
+// residual quantizer does once a row's centroid is known (src/rvq.rs:111-138, 186-213).
 #include <algorithm>
+#include <type_traits>
 
 #include "cuda_device.hpp"
+#include "dense_image.cuh"
 #include "dense_tc.hpp"
 #include "kernels_common.cuh"
 
@@ -15,474 +12,235 @@ namespace vqb {
 
 namespace {
 
-// Index of the lowest set bit at or above `from` in a 256-bit mask, or 256.
-__device__ __forceinline__ int next_bit(const uint32_t (&w)[8], int from)
+// One warp per listed row, one lane per candidate: each candidate's distance in the reference's own f32 arithmetic
+// (src/vector.rs:198-220, src/distances.rs:130-140), the smallest with the lowest index wins.  The shortlist leaves few rows (a
+// hundredth of a Gaussian mixture's; more only where centroids coincide, and then a warp's lanes are full), so the time is
+// the way to a few centroids in L2: 16 loads per lane are on their way at once.
+template <bool VEC>
+__global__ void __launch_bounds__(256) resolve_kernel(const float *__restrict__ x, int dim, int k, const float *__restrict__ book, int euclid,
+                                                      const uint32_t *__restrict__ cand, const uint32_t *__restrict__ list, const uint32_t *list_count,
+                                                      uint8_t *codes, uint32_t *changed)
 {
-    for (int wd = from >> 5; wd < 8; ++wd) {
-        uint32_t m = w[wd];
-        if (wd == (from >> 5)) m &= 0xFFFFFFFFu << (from & 31);
-        if (m) return wd * 32 + __ffs(m) - 1;
-    }
-    return 256;
-}
-
-// Reference distance of one row (xcol, stride XT_STRIDE) to two centroids at once: two independent serial chains.
-#define XT_STRIDE 17
-__device__ __forceinline__ void exact_dist2(const float *xcol, const float *c0, const float *c1, int dim, bool euclid, float (&out)[2])
-{
-    float a0 = 0.0f, a1 = 0.0f;
-    for (int i0 = 0; i0 < dim; i0 += 8) {
-        float xv[8], v0[8], v1[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            xv[u] = xcol[(i0 + u) * XT_STRIDE];
-            v0[u] = c0[i0 + u], v1[u] = c1[i0 + u];
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            const float d0 = __fsub_rn(xv[u], v0[u]), d1 = __fsub_rn(xv[u], v1[u]);
-            a0 = __fadd_rn(a0, __fmul_rn(d0, d0));
-            a1 = __fadd_rn(a1, __fmul_rn(d1, d1));
-        }
-    }
-    out[0] = euclid ? __fsqrt_rn(a0) : a0;
-    out[1] = euclid ? __fsqrt_rn(a1) : a1;
-}
-
-// Tiles of 16 rows, two lanes per row (see resolve_train_kernel below for why): both lanes of a row evaluate two of its next
-// four candidates each and walk through the four distances in ascending centroid order; the row's epilogue (residual, norm,
-// flags) is the first lane's.
-constexpr int RT_MAX_WARPS = 12;
-template <int MODE, typename CodeT> __global__ void __launch_bounds__(32 * RT_MAX_WARPS, 1) resolve_kernel(const ResolveParams P)
-{
-    extern __shared__ __align__(16) float smem[];
-    const int dim = P.dim, k = P.k, cstride = dim + 1; // odd stride: lanes reading different centroids hit different banks
-    const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float *cpad = smem;                                   // [k][dim + 1]
-    float *xs = smem + (size_t)k * cstride + (size_t)warp * dim * XT_STRIDE; // [dim][17] per warp
-    {
-        // codebook -> shared memory, eight 128-bit loads in flight per thread (dim is a multiple of 4 on this path)
-        const int total4 = k * dim / 4, dim4 = dim / 4;
-        const float4 *src = reinterpret_cast<const float4 *>(P.codebook);
-        for (int base = 0; base < total4; base += 8 * (int)blockDim.x) {
-            float4 v[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int t = base + u * (int)blockDim.x + (int)threadIdx.x;
-                v[u] = (t < total4) ? __ldg(src + t) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int t = base + u * (int)blockDim.x + (int)threadIdx.x;
-                if (t < total4) {
-                    float *d = cpad + (size_t)(t / dim4) * cstride + (size_t)(t % dim4) * 4;
-                    d[0] = v[u].x, d[1] = v[u].y, d[2] = v[u].z, d[3] = v[u].w;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    const bool euclid = P.euclid != 0;
-    const unsigned long long tiles = (P.n + 15) / 16;
+    __shared__ uint8_t s_number[8][256];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t total = *list_count;
     bool moved = false;
-    double warp_norm = 0.0;
-    const int r = lane & 15, half = lane >> 4;
-
-    // A warp's next tile (16 rows, up to 8 KiB) is requested into registers while the current one is worked on.
-    const int dim4 = dim / 4, total4 = 16 * dim4;
-    float4 pre[16];
-    auto request = [&](unsigned long long tile) {
-        const unsigned long long r0 = tile * 16;
+    for (uint32_t at = blockIdx.x * 8 + warp; at < total; at += gridDim.x * 8) {
+        const size_t row = list[at];
+        int cnt = 0;
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int idx = u * 32 + lane;
-            const unsigned long long rr = r0 + idx / dim4;
-            pre[u] = (tile < tiles && idx < total4 && rr < P.n) ? __ldg(reinterpret_cast<const float4 *>(P.x + rr * dim) + idx % dim4)
-                                                              : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int w = 0; w < DENSE_MASK_WORDS; ++w) {
+            const uint32_t word = __ldg(cand + row * DENSE_MASK_WORDS + w);
+            if (word >> lane & 1u) s_number[warp][cnt + __popc(word & ((1u << lane) - 1u))] = (uint8_t)(w * 32 + lane);
+            cnt += __popc(word);
         }
-    };
-    request((unsigned long long)blockIdx.x * W + warp);
-    for (unsigned long long tile = (unsigned long long)blockIdx.x * W + warp; tile < tiles; tile += (unsigned long long)gridDim.x * W) {
-        const unsigned long long row0 = tile * 16, row = row0 + r;
-        const bool valid = row < P.n;
-        bool skip = false;
-        if (MODE == R_RVQ_STAGE && valid) skip = P.done[row] != 0;
-        // stage the 16 rows dimension-major (lanes walked along a row when they were loaded: coalesced), then ask for the next tile
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int idx = u * 32 + lane;
-            if (idx < total4) {
-                float *d = xs + (size_t)(idx % dim4) * 4 * XT_STRIDE + idx / dim4;
-                d[0] = pre[u].x, d[XT_STRIDE] = pre[u].y, d[2 * XT_STRIDE] = pre[u].z, d[3 * XT_STRIDE] = pre[u].w;
-            }
-        }
-        request(tile + (unsigned long long)gridDim.x * W);
         __syncwarp();
-        const float *xcol = xs + r;
-        int best = 0;
-        uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        int ncand = 0;
-        if (valid && !skip) {
-            const uint4 lo = reinterpret_cast<const uint4 *>(P.cand + row * 8)[0], hi = reinterpret_cast<const uint4 *>(P.cand + row * 8)[1];
-            w[0] = lo.x, w[1] = lo.y, w[2] = lo.z, w[3] = lo.w, w[4] = hi.x, w[5] = hi.y, w[6] = hi.z, w[7] = hi.w;
-#pragma unroll
-            for (int t = 0; t < 8; ++t) ncand += __popc(w[t]);
-        }
-        // Rows with many candidates (or marked "examine all") are scanned by the whole warp: lane L takes centroids
-        // L, L+32, ... in ascending order, then the warp keeps the smallest distance, lowest index on ties.  A NaN never
-        // wins in the reference unless it sits at centroid 0, where the scan starts.
-        const bool wide = ncand > 12;
-        unsigned wide_rows = __ballot_sync(0xffffffffu, wide) & 0xFFFFu;
-        while (wide_rows) {
-            const int wr = __ffs(wide_rows) - 1;
-            wide_rows &= wide_rows - 1;
-            const float *xr = xs + wr;
-            float bd = VQB_DENSE_INF;
-            int bi = 0x7fffffff;
-            float d0 = 0.0f;
-            for (int j = lane; j < k; j += 32) {
-                const float *c = cpad + (size_t)j * cstride;
-                float acc = 0.0f;
-#pragma unroll 8
-                for (int i = 0; i < dim; ++i) {
-                    const float d = __fsub_rn(xr[i * XT_STRIDE], c[i]);
-                    acc = __fadd_rn(acc, __fmul_rn(d, d));
+        const float *xr = x + row * dim;
+        float best = VQB_DENSE_INF;
+        int code = 0; // stays where nothing is below +inf
+        bool stuck = false;
+        for (int base = 0; base < cnt; base += 32) {
+            const bool in = base + lane < cnt;
+            const int j = s_number[warp][in ? base + lane : 0];
+            const float *c = book + (size_t)j * dim;
+            float d = 0.0f;
+            auto add = [&](float xv, float cv) {
+                const float e = __fsub_rn(xv, cv);
+                d = __fadd_rn(d, __fmul_rn(e, e));
+            };
+            if (VEC) {
+#pragma unroll 16
+                for (int i = 0; i < dim; i += 4) {
+                    const float4 cv = __ldg(reinterpret_cast<const float4 *>(c + i)), xv = __ldg(reinterpret_cast<const float4 *>(xr + i));
+                    add(xv.x, cv.x), add(xv.y, cv.y), add(xv.z, cv.z), add(xv.w, cv.w);
                 }
-                const float d = euclid ? __fsqrt_rn(acc) : acc;
-                if (j == 0) d0 = d;
-                if (d < bd) {
-                    bd = d;
-                    bi = j;
-                }
-            }
-            d0 = __shfl_sync(0xffffffffu, d0, 0);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float od = __shfl_xor_sync(0xffffffffu, bd, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (od < bd || (od == bd && oi < bi)) {
-                    bd = od;
-                    bi = oi;
-                }
-            }
-            int res = (bi == 0x7fffffff) ? 0 : bi; // nothing finite below +inf: the reference keeps centroid 0
-            if (!(d0 == d0)) res = 0;               // NaN at centroid 0: nothing ever replaces it (src/utils.rs:62-66)
-            if (bd == VQB_DENSE_INF) res = 0;       // all distances +inf (or NaN): strict '<' never fires
-            if (r == wr) best = res;
-        }
-        // the other rows: rounds of four candidates, two per lane of the pair; every lane of the warp takes part in a round
-        {
-            float bd = VQB_DENSE_INF;
-            int bi = -1;
-            int j = (valid && !skip && !wide) ? next_bit(w, 0) : 256;
-            while (__any_sync(0xffffffffu, j < k)) {
-                int js[4];
-                js[0] = j;
-#pragma unroll
-                for (int t = 1; t < 4; ++t) js[t] = (js[t - 1] < 256) ? next_bit(w, js[t - 1] + 1) : 256;
-                const int ja = half ? js[2] : js[0], jb = half ? js[3] : js[1];
-                float mine[2];
-                exact_dist2(xcol, cpad + (size_t)min(ja, k - 1) * cstride, cpad + (size_t)min(jb, k - 1) * cstride, dim, euclid, mine);
-                const float o0 = __shfl_xor_sync(0xffffffffu, mine[0], 16), o1 = __shfl_xor_sync(0xffffffffu, mine[1], 16);
-                const float d[4] = {half ? o0 : mine[0], half ? o1 : mine[1], half ? mine[0] : o0, half ? mine[1] : o1};
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    if (js[t] >= k) break;
-                    if (js[t] == 0) { // the reference's scan starts at centroid 0 whatever its value
-                        bd = d[t];
-                        bi = 0;
-                    } else {
-                        argmin_update(d[t], js[t], bd, bi); // a skipped centroid 0 is provably farther than the winner
-                    }
-                }
-                j = (js[3] < 256) ? next_bit(w, js[3] + 1) : 256;
-            }
-            if (valid && !skip && !wide) best = bi < 0 ? 0 : bi;
-        }
-        if (valid && !skip && half == 0) {
-            if (MODE == R_TRAIN) {
-                CodeT *cp = reinterpret_cast<CodeT *>(P.codes) + row;
-                const CodeT nc = (CodeT)best;
-                if (*cp != nc) moved = true;
-                *cp = nc;
             } else {
-                const float *cw = cpad + (size_t)best * cstride;
-                float nsq = 0.0f;
-#pragma unroll 8
-                for (int i = 0; i < dim; ++i) {
-                    const float rv = __fsub_rn(xs[i * XT_STRIDE + r], cw[i]);
-                    xs[i * XT_STRIDE + r] = rv;
-                    nsq = __fadd_rn(nsq, __fmul_rn(rv, rv));
-                }
-                const float nrm = __fsqrt_rn(nsq);
-                if (MODE == R_RVQ_UPDATE) warp_norm += (double)nrm;
-                if (MODE == R_RVQ_STAGE) {
-                    if (P.out_codes) P.out_codes[row * (unsigned long long)P.stages + P.stage] = (uint32_t)best;
-                    if (nrm < P.epsilon) P.done[row] = 1;
-                }
+#pragma unroll 16
+                for (int i = 0; i < dim; ++i) add(__ldg(xr + i), __ldg(c + i));
+            }
+            if (euclid) d = __fsqrt_rn(d);
+            stuck = stuck || __any_sync(0xffffffffu, in && j == 0 && !(d == d)); // the reference's scan starts at centroid 0: a NaN there stays
+            float low = in && d < VQB_DENSE_INF ? d : VQB_DENSE_INF;
+            const float mine = low;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) low = fminf(low, __shfl_xor_sync(0xffffffffu, low, o));
+            const int jm = (int)__reduce_min_sync(0xffffffffu, mine == low ? (unsigned)j : 0xFFFFFFFFu);
+            if (low < best) best = low, code = jm; // candidates ascend: an equal distance later on loses
+        }
+        if (stuck) code = 0;
+        if (lane == 0 && codes[row] != (uint8_t)code) {
+            moved = true;
+            codes[row] = (uint8_t)code;
+        }
+        __syncwarp();
+    }
+    if (lane == 0 && moved && changed) atomicOr(changed, VQB_MOVED_BITS);
+}
+
+// L lanes per row, four values each (as dense_prepare_kernel): one read of the rows, one write of the residuals, one of their
+// images; the codebook's rows come from L2.
+template <int L, bool VEC>
+__global__ void __launch_bounds__(256) rvq_apply_kernel(const float *x, float *res, unsigned long long n, int dim, int dimp, const float *__restrict__ book,
+                                                        const uint8_t *__restrict__ codes, double *norm_sum, uint8_t *ended, int stage, float epsilon,
+                                                        const float *frame, uint16_t *image, float *norms)
+{
+    const int lane = threadIdx.x & 31, piece = lane % L;
+    const FramePiece f = load_frame(frame, piece);
+    const unsigned long long step = (unsigned long long)gridDim.x * (256 / L);
+    double total = 0.0;
+    for (unsigned long long row = blockIdx.x * (unsigned long long)(256 / L) + threadIdx.x / L; row - threadIdx.x / L < n; row += step) {
+        bool in = row < n;
+        if (ended && in) in = ended[row] > stage; // the other rows have ended: nothing of them changes
+        float v[4], c[4];
+        const int code = in ? (int)codes[row] : 0;
+        if (VEC) {
+            const float4 t = in && 4 * piece < dim ? *reinterpret_cast<const float4 *>(x + row * dim + 4 * piece) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[0] = t.x, v[1] = t.y, v[2] = t.z, v[3] = t.w;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = in && 4 * piece + e < dim ? x[row * dim + 4 * piece + e] : 0.0f;
+        }
+        load_piece<VEC>(c, book, (unsigned long long)code, piece, in, dim);
+        float a = 0.0f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            v[e] = __fsub_rn(v[e], c[e]);
+            a = fmaf(v[e], v[e], a);
+        }
+        if (in) {
+            if (VEC) {
+                if (4 * piece < dim) *reinterpret_cast<float4 *>(res + row * dim + 4 * piece) = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (4 * piece + e < dim) res[row * dim + 4 * piece + e] = v[e];
             }
         }
-        if (MODE != R_TRAIN) {
-            // write the residual tile back; R_RVQ_STAGE also adds the chosen centroid to the running sum
-            const int mybest = (valid && !skip) ? best : -1;
+        float fa = store_image(image + (size_t)row * 2 * dimp, dimp, piece, v, f, in);
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) {
+            a += __shfl_xor_sync(0xffffffffu, a, o);
+            fa += __shfl_xor_sync(0xffffffffu, fa, o);
+        }
+        if (norm_sum && in && piece == 0) total += (double)sqrtf(a);
+        if (in && piece == 0) norms[row] = fa * 1.00001f; // an upper bound is what the shortlist needs
+        if (ended) {
+            // The reference compares the root of the SERIAL sum of squares (src/rvq.rs:204-207), which lies within 2 dim 2^-24 of this
+            // one: only a row that close to epsilon is added up in order.
+            const float nrm = sqrtf(a), slack = 1e-4f * epsilon;
+            bool below = nrm < epsilon - slack;
+            const bool close = in && !below && !(nrm > epsilon + slack);
+            __syncwarp(); // the row's residual is in memory for the lane that may read it
+            if (close && piece == 0) {
+                float s = 0.0f;
+                for (int i = 0; i < dim; ++i) {
+                    const float r = *reinterpret_cast<volatile float *>(res + row * dim + i);
+                    s = __fadd_rn(s, __fmul_rn(r, r));
+                }
+                below = __fsqrt_rn(s) < epsilon;
+            }
+            if (in && piece == 0 && below) ended[row] = (uint8_t)(stage + 1);
             __syncwarp();
-            // four rows per step; the running-sum reads of a step are all issued before any is used
-            for (int r0 = 0; r0 < 16; r0 += 4) {
-                int b[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    b[u] = __shfl_sync(0xffffffffu, mybest, r0 + u);
-                    if (row0 + r0 + u >= P.n) b[u] = -1;
-                }
-                for (int i0 = 0; i0 < dim; i0 += 128) {
-                    float q[4][4];
-                    if (MODE == R_RVQ_STAGE) {
-#pragma unroll
-                        for (int u = 0; u < 4; ++u)
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const int i = i0 + e * 32 + lane;
-                                q[u][e] = (b[u] >= 0 && i < dim) ? P.qsum[(row0 + r0 + u) * dim + i] : 0.0f;
-                            }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        if (b[u] < 0) continue;
-                        const unsigned long long rr = row0 + r0 + u;
-                        const float *cw = cpad + (size_t)b[u] * cstride;
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const int i = i0 + e * 32 + lane;
-                            if (i >= dim) continue;
-                            P.res[rr * dim + i] = xs[i * XT_STRIDE + r0 + u];
-                            if (MODE == R_RVQ_STAGE) P.qsum[rr * dim + i] = __fadd_rn(q[u][e], cw[i]);
-                        }
-                    }
-                }
-            }
         }
-        __syncwarp();
     }
-    if (MODE == R_TRAIN) {
-        if (__any_sync(0xffffffffu, moved) && lane == 0) atomicOr(P.changed, VQB_MOVED_BITS);
-    }
-    if (MODE == R_RVQ_UPDATE) {
+    if (norm_sum) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) warp_norm += __shfl_xor_sync(0xffffffffu, warp_norm, o);
-        if (lane == 0 && warp_norm != 0.0) atomicAdd(P.norm_sum, warp_norm);
+        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+        if (lane == 0 && total != 0.0) atomicAdd(norm_sum, total);
     }
 }
 
-// Training assignment of the rows the shortlist kernel could not decide (more than one candidate, or "examine all"); the
-// rows with a single candidate got their assignment there and are never read here.  A warp takes 16 listed rows at a time and
-// gives every row TWO lanes, each of which evaluates two of the row's next four candidates with the exact arithmetic; the pair
-// then goes through the four distances in ascending centroid order like the reference.  Sixteen-row groups halve a warp's
-// staging buffer, which is what lets ten warps instead of four sit beside the 132 KB codebook: with one warp per scheduler
-// the serial chains ran at a quarter of the issue rate.
-template <typename CodeT> __global__ void __launch_bounds__(32 * RT_MAX_WARPS, 1) resolve_train_kernel(const ResolveParams P)
+template <int L, bool VEC>
+__global__ void __launch_bounds__(256) rvq_gather_kernel(const uint8_t *__restrict__ codes, const uint8_t *__restrict__ ended, unsigned long long n, int dim,
+                                                         const float *__restrict__ books, int k, int stages, uint16_t *out_f16, uint32_t *out_codes)
 {
-    extern __shared__ __align__(16) float smem[];
-    const int dim = P.dim, k = P.k, cstride = dim + 1;
-    const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned long long cnt = *reinterpret_cast<const volatile uint32_t *>(P.list_count);
-    const unsigned long long groups = (cnt + 15) / 16;
-    if ((unsigned long long)blockIdx.x * W >= groups) return; // nothing for this CTA: skip the codebook copy as well
-    float *cpad = smem;                                                                   // [k][dim + 1]
-    float *xs = smem + (size_t)k * cstride + (size_t)warp * dim * XT_STRIDE;              // [dim][17] per warp
-    {
-        const int total4 = k * dim / 4, dim4 = dim / 4;
-        const float4 *src = reinterpret_cast<const float4 *>(P.codebook);
-        for (int base = 0; base < total4; base += 8 * (int)blockDim.x) {
-            float4 v[8];
+    const int piece = (threadIdx.x & 31) % L;
+    const unsigned long long step = (unsigned long long)gridDim.x * (256 / L);
+    for (unsigned long long row = blockIdx.x * (unsigned long long)(256 / L) + threadIdx.x / L; row < n; row += step) {
+        const int last = min(stages, (int)ended[row]);
+        float q[4] = {0.f, 0.f, 0.f, 0.f};
+        if (out_f16) {
+#pragma unroll 4
+            for (int st = 0; st < last; ++st) {
+                float c[4];
+                load_piece<VEC>(c, books + (size_t)st * k * dim, codes[(size_t)st * n + row], piece, true, dim);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int t = base + u * (int)blockDim.x + (int)threadIdx.x;
-                v[u] = (t < total4) ? __ldg(src + t) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int e = 0; e < 4; ++e) q[e] = __fadd_rn(q[e], c[e]);
             }
+            uint16_t *o = out_f16 + row * dim + 4 * piece;
+            if (VEC) {
+                if (4 * piece < dim)
+                    *reinterpret_cast<uint2 *>(o) = make_uint2((uint32_t)f32_to_f16_bits(q[0]) | ((uint32_t)f32_to_f16_bits(q[1]) << 16),
+                                                               (uint32_t)f32_to_f16_bits(q[2]) | ((uint32_t)f32_to_f16_bits(q[3]) << 16));
+            } else {
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int t = base + u * (int)blockDim.x + (int)threadIdx.x;
-                if (t < total4) {
-                    float *d = cpad + (size_t)(t / dim4) * cstride + (size_t)(t % dim4) * 4;
-                    d[0] = v[u].x, d[1] = v[u].y, d[2] = v[u].z, d[3] = v[u].w;
-                }
+                for (int e = 0; e < 4; ++e)
+                    if (4 * piece + e < dim) o[e] = f32_to_f16_bits(q[e]);
             }
         }
+        if (out_codes)
+            for (int st = piece; st < stages; st += L) out_codes[row * stages + st] = st < last ? (uint32_t)codes[(size_t)st * n + row] : 0xFFFFFFFFu;
     }
-    __syncthreads();
-    const bool euclid = P.euclid != 0;
-    bool moved = false;
-    CodeT *codes = reinterpret_cast<CodeT *>(P.codes);
-    const int r = lane & 15, half = lane >> 4;
-    const int dim4 = dim / 4;
-    // the next group's rows are requested into registers while this one is evaluated
-    float4 pre[16];
-    auto request = [&](unsigned long long g) {
-        const int nb = g < groups ? (int)min(16ull, cnt - g * 16) : 0, total4 = nb * dim4;
-#pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int idx = u * 32 + lane;
-            pre[u] = idx < total4 ? __ldg(reinterpret_cast<const float4 *>(P.x + (unsigned long long)P.list[g * 16 + idx / dim4] * dim) + idx % dim4)
-                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-    };
-    const unsigned long long g0 = (unsigned long long)blockIdx.x * W + warp, gstep = (unsigned long long)gridDim.x * W;
-    request(g0);
-    for (unsigned long long g = g0; g < groups; g += gstep) {
-        const int nb = (int)min(16ull, cnt - g * 16);
-        {
-            const int total4 = nb * dim4;
-#pragma unroll
-            for (int u = 0; u < 16; ++u) {
-                const int idx = u * 32 + lane;
-                if (idx < total4) {
-                    float *d = xs + (size_t)(idx % dim4) * 4 * XT_STRIDE + idx / dim4;
-                    d[0] = pre[u].x, d[XT_STRIDE] = pre[u].y, d[2 * XT_STRIDE] = pre[u].z, d[3 * XT_STRIDE] = pre[u].w;
-                }
-            }
-        }
-        request(g + gstep);
-        __syncwarp();
-        const bool valid = r < nb; // both lanes of a row agree on everything below
-        const unsigned long long row = valid ? P.list[g * 16 + r] : 0ull;
-        const float *xcol = xs + r;
-        int best = 0, ncand = 0;
-        uint32_t w[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        if (valid) {
-            const uint4 lo = __ldg(reinterpret_cast<const uint4 *>(P.cand + row * 8)), hi = __ldg(reinterpret_cast<const uint4 *>(P.cand + row * 8) + 1);
-            w[0] = lo.x, w[1] = lo.y, w[2] = lo.z, w[3] = lo.w, w[4] = hi.x, w[5] = hi.y, w[6] = hi.z, w[7] = hi.w;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) ncand += __popc(w[e]);
-        }
-        // rows with many candidates (or marked "examine all"): the whole warp scans all centroids, as in resolve_kernel
-        const bool wide = valid && (ncand > 12 || ncand == 0);
-        unsigned wide_rows = __ballot_sync(0xffffffffu, wide) & 0xFFFFu;
-        while (wide_rows) {
-            const int wr = __ffs(wide_rows) - 1;
-            wide_rows &= wide_rows - 1;
-            const float *xr = xs + wr;
-            float bd = VQB_DENSE_INF, d0 = 0.0f;
-            int bi = 0x7fffffff;
-            for (int j = lane; j < k; j += 32) {
-                const float *c = cpad + (size_t)j * cstride;
-                float acc = 0.0f;
-#pragma unroll 8
-                for (int i = 0; i < dim; ++i) {
-                    const float d = __fsub_rn(xr[i * XT_STRIDE], c[i]);
-                    acc = __fadd_rn(acc, __fmul_rn(d, d));
-                }
-                const float d = euclid ? __fsqrt_rn(acc) : acc;
-                if (j == 0) d0 = d;
-                if (d < bd) {
-                    bd = d;
-                    bi = j;
-                }
-            }
-            d0 = __shfl_sync(0xffffffffu, d0, 0);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const float od = __shfl_xor_sync(0xffffffffu, bd, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (od < bd || (od == bd && oi < bi)) {
-                    bd = od;
-                    bi = oi;
-                }
-            }
-            int res = (bi == 0x7fffffff) ? 0 : bi;
-            if (!(d0 == d0)) res = 0;
-            if (bd == VQB_DENSE_INF) res = 0;
-            if (r == wr) best = res;
-        }
-        // the other rows: rounds of four candidates, two per lane of the pair
-        float bd = VQB_DENSE_INF;
-        int bi = -1;
-        int j = (valid && !wide) ? next_bit(w, 0) : 256;
-        while (__any_sync(0xffffffffu, j < k)) {
-            int js[4];
-            js[0] = j;
-#pragma unroll
-            for (int t = 1; t < 4; ++t) js[t] = (js[t - 1] < 256) ? next_bit(w, js[t - 1] + 1) : 256;
-            const int ja = half ? js[2] : js[0], jb = half ? js[3] : js[1];
-            float mine[2];
-            exact_dist2(xcol, cpad + (size_t)min(ja, k - 1) * cstride, cpad + (size_t)min(jb, k - 1) * cstride, dim, euclid, mine);
-            const float o0 = __shfl_xor_sync(0xffffffffu, mine[0], 16), o1 = __shfl_xor_sync(0xffffffffu, mine[1], 16);
-            const float d[4] = {half ? o0 : mine[0], half ? o1 : mine[1], half ? mine[0] : o0, half ? mine[1] : o1};
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                if (js[t] >= k) break;
-                if (js[t] == 0) {
-                    bd = d[t];
-                    bi = 0;
-                } else {
-                    argmin_update(d[t], js[t], bd, bi);
-                }
-            }
-            j = (js[3] < 256) ? next_bit(w, js[3] + 1) : 256;
-        }
-        if (valid && half == 0) {
-            if (!wide) best = bi < 0 ? 0 : bi;
-            const CodeT nc = (CodeT)best;
-            if (codes[row] != nc) moved = true;
-            codes[row] = nc;
-        }
-        __syncwarp();
-    }
-    if (__any_sync(0xffffffffu, moved) && lane == 0) atomicOr(P.changed, VQB_MOVED_BITS);
 }
 
-// as many warps as fit beside the padded codebook (ten at k = 256, dim = 128)
-static int resolve_warps(const ResolveParams &p, size_t extra_per_warp, size_t *smem)
+// lanes per row that a width takes, and the kernel for them
+template <typename F> void with_lanes(size_t dimp, bool vec, F &&f)
 {
-    const size_t book = (size_t)p.k * (p.dim + 1) * sizeof(float), per_warp = (size_t)p.dim * XT_STRIDE * sizeof(float) + extra_per_warp;
-    const size_t budget = 226 * 1024;
-    const int warps = (int)std::max<size_t>(1, std::min<size_t>(RT_MAX_WARPS, book < budget ? (budget - book) / per_warp : 1));
-    *smem = book + (size_t)warps * per_warp;
-    return warps;
+    if (dimp <= 32) vec ? f(std::integral_constant<int, 8>(), std::true_type()) : f(std::integral_constant<int, 8>(), std::false_type());
+    else if (dimp <= 64) vec ? f(std::integral_constant<int, 16>(), std::true_type()) : f(std::integral_constant<int, 16>(), std::false_type());
+    else vec ? f(std::integral_constant<int, 32>(), std::true_type()) : f(std::integral_constant<int, 32>(), std::false_type());
 }
 
-template <int MODE, typename CodeT> void launch_t(CudaDevice &dev, const ResolveParams &p, const char *name)
-{
-    size_t smem = 0;
-    const int warps = resolve_warps(p, 0, &smem);
-    auto kernel = resolve_kernel<MODE, CodeT>;
-    VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const unsigned long long tiles = (p.n + 15) / 16;
-    const unsigned grid = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>((tiles + warps - 1) / warps, (unsigned long long)dev.sm_count()));
-    KernelScope ks(dev, name);
-    kernel<<<grid, 32 * warps, smem, dev.stream()>>>(p);
-    VQB_CUDA_CHECK(cudaGetLastError());
-    dev.count_launch();
-}
+bool aligned(const void *p, unsigned bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
 
-template <typename CodeT> void launch_train(CudaDevice &dev, const ResolveParams &p)
+unsigned grid_rows(CudaDevice &dev, size_t n, int lanes)
 {
-    size_t smem = 0;
-    const int warps = resolve_warps(p, 0, &smem);
-    auto kernel = resolve_train_kernel<CodeT>;
-    VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    // the number of listed rows is only known on the device: CTAs without a group leave at once
-    const unsigned long long groups = (p.n + 15) / 16;
-    const unsigned grid = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>((groups + warps - 1) / warps, (unsigned long long)dev.sm_count()));
-    KernelScope ks(dev, "resolve_train");
-    kernel<<<grid, 32 * warps, smem, dev.stream()>>>(p);
-    VQB_CUDA_CHECK(cudaGetLastError());
-    dev.count_launch();
+    return (unsigned)std::max<size_t>(1, std::min<size_t>((n * lanes + 255) / 256, (size_t)dev.sm_count() * 32));
 }
 
 } // namespace
 
-void launch_resolve(CudaDevice &dev, const ResolveParams &p, int mode, size_t cb)
+void dense_resolve(CudaDevice &dev, const DenseWork &w, const float *x, size_t n, size_t dim, const float *codebook, size_t k, bool euclid,
+                   uint8_t *codes, uint32_t *changed)
 {
-    if (p.n == 0) return;
-    if (mode == R_TRAIN) {
-        if (cb == 1) launch_train<uint8_t>(dev, p);
-        else if (cb == 2) launch_train<uint16_t>(dev, p);
-        else launch_train<uint32_t>(dev, p);
-    } else if (mode == R_RVQ_UPDATE) {
-        launch_t<R_RVQ_UPDATE, uint32_t>(dev, p, "resolve_rvq_update");
-    } else {
-        launch_t<R_RVQ_STAGE, uint32_t>(dev, p, "resolve_rvq_stage");
-    }
+    if (n == 0) return;
+    const bool vec = dim % 4 == 0 && aligned(x, 16) && aligned(codebook, 16);
+    // the number of listed rows is only known on the device
+    const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((n + 7) / 8, (size_t)dev.sm_count() * 6));
+    KernelScope ks(dev, "dense_resolve");
+    auto kernel = vec ? resolve_kernel<true> : resolve_kernel<false>;
+    kernel<<<grid, 256, 0, dev.stream()>>>(x, (int)dim, (int)k, codebook, euclid ? 1 : 0, w.cand, w.list, w.list_count, codes, changed);
+    VQB_CUDA_CHECK(cudaGetLastError());
+    dev.count_launch();
+}
+
+void rvq_apply(CudaDevice &dev, const RvqApply &a, const DenseWork &w)
+{
+    if (a.n == 0) return;
+    const size_t dimp = dense_padded(a.dim);
+    dense_frame(dev, w, a.x, a.n, a.dim, a.codebook, a.codes, true);
+    KernelScope ks(dev, "rvq_apply");
+    with_lanes(dimp, a.dim % 4 == 0 && aligned(a.x, 16) && aligned(a.res, 16) && aligned(a.codebook, 16), [&](auto lanes, auto vec) {
+        constexpr int L = decltype(lanes)::value;
+        rvq_apply_kernel<L, decltype(vec)::value><<<grid_rows(dev, a.n, L), 256, 0, dev.stream()>>>(
+            a.x, a.res, a.n, (int)a.dim, (int)dimp, a.codebook, a.codes, a.norm_sum, a.ended, a.stage, a.epsilon, w.frame, w.image, w.norms);
+    });
+    VQB_CUDA_CHECK(cudaGetLastError());
+    dev.count_launch();
+}
+
+void rvq_gather(CudaDevice &dev, const uint8_t *codes, const uint8_t *ended, size_t n, size_t dim, const float *codebooks, size_t k, int stages,
+                uint16_t *out_f16, uint32_t *out_codes)
+{
+    if (n == 0) return;
+    KernelScope ks(dev, "rvq_gather");
+    with_lanes(dense_padded(dim), dim % 4 == 0 && aligned(codebooks, 16) && aligned(out_f16, 8), [&](auto lanes, auto vec) {
+        constexpr int L = decltype(lanes)::value;
+        rvq_gather_kernel<L, decltype(vec)::value><<<grid_rows(dev, n, L), 256, 0, dev.stream()>>>(codes, ended, n, (int)dim, codebooks, (int)k, stages,
+                                                                                               out_f16, out_codes);
+    });
+    VQB_CUDA_CHECK(cudaGetLastError());
+    dev.count_launch();
 }
 
 } // namespace vqb
