@@ -31,8 +31,8 @@
 //               accumulators so the next tile's MMAs overlap this tile's epilogue.  One K = 8 step of kind::tf32 per tile multiplies
 //               a constant (1, 1, 0, ...) row operand with (-hn_h, -hn_l, 0, ...) per centroid, so the accumulator holds
 //               D = x.c - |c|^2/2 = -S and the epilogue never touches the half norms
-//   warps 2..5  epilogue: tcgen05.ld the 128 x 256 values, one row per lane; pass 1 finds the largest D (3-input max), pass 2
-//               shifts the sign of (D - limit) into a 256-bit candidate mask
+//   warps 2..5  epilogue: tcgen05.ld the 128 x 256 values, one row per lane; pass 1 finds the largest D and whether it is the only
+//               candidate, and which; for a warp with an undecided row pass 2 shifts the sign of (D - limit) into a 256-bit mask
 // Every wait is bounded; on expiry the kernel records an error code, stops issuing work and frees its tensor memory.
 #include <cuda.h>
 
@@ -66,7 +66,7 @@ struct alignas(8) Barriers {
 
 struct ShortlistParams {
     unsigned long long n;
-    int dim, k, ksteps;   // ksteps: K = 16 steps of one part (h or l) of an image
+    int dim, k;
     const float *hn;      // [256] |c_j|^2 / 2 in the frame, +inf beyond k
     const float *frame;
     const float *xnorm2;  // [n]   |v|^2 per row, an upper bound
@@ -82,6 +82,9 @@ struct ShortlistParams {
     uint32_t *list_count;  // [1] zero on entry
 };
 
+// KS: K = 16 steps of one part (h or l) of an image.  A constant, because one thread issues the MMAs: with descriptors worked out
+// per step it took 260 cycles an MMA, now 200 with all waits (the tensor core alone: 134).
+template <int KS>
 __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_c,
                                                                 const ShortlistParams P)
 {
@@ -99,7 +102,7 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned long long n_tiles = (P.n + BM - 1) / BM;
-    const int kchunks = (2 * P.ksteps + 3) / 4; // 64-element pieces of an image
+    constexpr int kchunks = (2 * KS + 3) / 4; // 64-element pieces of an image
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NSTAGE; ++s) {
@@ -180,12 +183,15 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
         // ------------------------------------------------ MMA issuer
         if (lane == 0) {
             bool ok = mbar_wait(&bars->cfull, 0, abort_flag, P.error, 2);
+            const uint64_t adesc0 = smem_desc_sw128(smem_u32(x_smem)), bdesc0 = smem_desc_sw128(smem_u32(c_smem));
+            auto book_step = [](int step) { return (uint64_t)((step >> 2) * (int)(C_CHUNK_BYTES >> 4) + 2 * (step & 3)); }; // K step of the codebook's image
             uint32_t it = 0, local = 0;
             for (unsigned long long tile = blockIdx.x; ok && tile < n_tiles && !*abort_flag; tile += gridDim.x, ++local) {
                 const uint32_t b = local & 1u, buse = local >> 1;
                 if (!mbar_wait(&bars->tempty[b], (buse & 1u) ^ 1u, abort_flag, P.error, 3)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t d_tmem = tmem_base + b * BN;
+#pragma unroll
                 for (int kc = 0; kc < kchunks; ++kc, ++it) {
                     const int s = it % NSTAGE;
                     const uint32_t use = it / NSTAGE;
@@ -194,18 +200,15 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t adesc = smem_desc_sw128(smem_u32(x_smem + (size_t)s * X_STAGE_BYTES));
-                    auto book = [&](int step) { // descriptor of K step `step` of the codebook's image
-                        return smem_desc_sw128(smem_u32(c_smem + (size_t)(step >> 2) * C_CHUNK_BYTES)) + (uint64_t)(2 * (step & 3));
-                    };
-                    for (int i = 0; i < 4 && 4 * kc + i < 2 * P.ksteps; ++i) { // 16 bf16 = 32 bytes = 2 descriptor units per step
+                    const uint64_t adesc = adesc0 + (uint64_t)(s * (int)(X_STAGE_BYTES >> 4));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) { // 16 values = 32 bytes = 2 descriptor units per step
                         const int j = 4 * kc + i;
-                        const uint64_t a = adesc + (uint64_t)(2 * i);
-                        if (j < P.ksteps) { // h.ch and h.cl
-                            umma_f16(d_tmem, a, book(j), j ? 1u : 0u);
-                            umma_f16(d_tmem, a, book(P.ksteps + j), 1u);
-                        } else { // l.ch
-                            umma_f16(d_tmem, a, book(j - P.ksteps), 1u);
+                        if (j < KS) { // h.ch and h.cl
+                            umma_f16(d_tmem, adesc + 2 * i, bdesc0 + book_step(j), j ? 1u : 0u);
+                            umma_f16(d_tmem, adesc + 2 * i, bdesc0 + book_step(KS + j), 1u);
+                        } else if (j < 2 * KS) { // l.ch
+                            umma_f16(d_tmem, adesc + 2 * i, bdesc0 + book_step(j - KS), 1u);
                         }
                     }
                     umma_commit(&bars->empty[s]); // the stage is free once these MMAs have read it
@@ -235,48 +238,36 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
             const float xn2 = valid ? P.xnorm2[row] : 0.0f;
             const int old_code = (P.codes && valid) ? (int)P.codes[row] : 0; // asked for now, needed after the two passes
 
-            // pass 1: the largest D = x.c - hn, i.e. the smallest score S = -D (four chains of 3-input max); the next 32 columns
-            // are in flight while these are processed
-            float m0 = -VQB_DENSE_INF, m1 = -VQB_DENSE_INF, m2 = -VQB_DENSE_INF, m3 = -VQB_DENSE_INF;
+            // pass 1: the largest D = v.c - hn, i.e. the smallest score S = -D, as the maxima of the 16 blocks of 16 consecutive columns and
+            // of the 16 classes of columns equal modulo 16 (one 3-input maximum per score; columns beyond k hold -1e30)
+            float hb[16], ga[16];
             bool col0_nan = false;
-            uint32_t ra[32], rb[32];
-            tmem_ld32_issue(taddr, ra);
-            tmem_wait();
-#pragma unroll 1
-            for (int cb = 0; cb < BN / 32; cb += 2) {
-                tmem_ld32_issue(taddr + (cb + 1) * 32, rb);
+#pragma unroll
+            for (int c = 0; c < BN / 32; ++c) {
+                uint32_t ra[32];
+                tmem_ld32_issue(taddr + c * 32, ra);
+                tmem_wait();
+                if (c == 0) col0_nan = !(__uint_as_float(ra[0]) == __uint_as_float(ra[0]));
                 if (P.debug_dots && valid) {
 #pragma unroll
-                    for (int t = 0; t < 32; ++t) P.debug_dots[row * BN + cb * 32 + t] = (cb * 32 + t < P.k) ? (__uint_as_float(ra[t]) + hn_s[cb * 32 + t]) / s2 : 0.0f;
-                }
-                if (cb == 0) {
-                    const float s0 = __uint_as_float(ra[0]);
-                    col0_nan = !(s0 == s0);
+                    for (int t = 0; t < 32; ++t) P.debug_dots[row * BN + c * 32 + t] = (c * 32 + t < P.k) ? (__uint_as_float(ra[t]) + hn_s[c * 32 + t]) / s2 : 0.0f;
                 }
 #pragma unroll
-                for (int t = 0; t < 32; t += 8) {
-                    m0 = max3f(m0, __uint_as_float(ra[t]), __uint_as_float(ra[t + 1]));
-                    m1 = max3f(m1, __uint_as_float(ra[t + 2]), __uint_as_float(ra[t + 3]));
-                    m2 = max3f(m2, __uint_as_float(ra[t + 4]), __uint_as_float(ra[t + 5]));
-                    m3 = max3f(m3, __uint_as_float(ra[t + 6]), __uint_as_float(ra[t + 7]));
-                }
-                tmem_wait();
-                if (cb + 2 < BN / 32) tmem_ld32_issue(taddr + (cb + 2) * 32, ra);
-                if (P.debug_dots && valid) {
+                for (int t = 0; t < 16; ++t)
+                    ga[t] = c ? max3f(ga[t], __uint_as_float(ra[t]), __uint_as_float(ra[16 + t])) : fmaxf(__uint_as_float(ra[t]), __uint_as_float(ra[16 + t]));
+                float b0 = __uint_as_float(ra[0]), b1 = __uint_as_float(ra[16]);
 #pragma unroll
-                    for (int t = 0; t < 32; ++t)
-                        P.debug_dots[row * BN + (cb + 1) * 32 + t] = ((cb + 1) * 32 + t < P.k) ? (__uint_as_float(rb[t]) + hn_s[(cb + 1) * 32 + t]) / s2 : 0.0f;
+                for (int t = 1; t < 15; t += 2) {
+                    b0 = max3f(b0, __uint_as_float(ra[t]), __uint_as_float(ra[t + 1]));
+                    b1 = max3f(b1, __uint_as_float(ra[16 + t]), __uint_as_float(ra[16 + t + 1]));
                 }
-#pragma unroll
-                for (int t = 0; t < 32; t += 8) {
-                    m0 = max3f(m0, __uint_as_float(rb[t]), __uint_as_float(rb[t + 1]));
-                    m1 = max3f(m1, __uint_as_float(rb[t + 2]), __uint_as_float(rb[t + 3]));
-                    m2 = max3f(m2, __uint_as_float(rb[t + 4]), __uint_as_float(rb[t + 5]));
-                    m3 = max3f(m3, __uint_as_float(rb[t + 6]), __uint_as_float(rb[t + 7]));
-                }
-                tmem_wait();
+                hb[2 * c] = fmaxf(b0, __uint_as_float(ra[15]));
+                hb[2 * c + 1] = fmaxf(b1, __uint_as_float(ra[31]));
             }
-            const float best = -fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)); // smallest score
+            float top = hb[0];
+#pragma unroll
+            for (int i = 1; i < 15; i += 2) top = max3f(top, hb[i], hb[i + 1]);
+            const float best = -fmaxf(top, hb[15]); // smallest score
             // E as above with max_j |c_j| (+ the rounding of the half norms: 10 operations in a tree, split into two TF32 numbers);
             // limit = best + 2E + 1.05 (dim + 6) u (|x|^2 + 2 best + 2E) + rounding slack of the comparison itself
             const float xn = sqrtf(xn2), e2 = 2.0f * (7e-6f * xn * cmax + 4e-7f * (xn + cmax)) + 1.2e-6f * cmax * cmax;
@@ -288,9 +279,42 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
             // (also when a true distance could overflow f32: then the reference's own comparisons see infinities)
             const bool scan_all = col0_nan || !(best == best) || !(limit == limit) || !(fabsf(limit) < VQB_DENSE_INF) || !(xn2 + cmax * cmax < huge);
 
-            // pass 2: one bit per centroid, set when D_j >= lim_d.  The sign of (D_j - lim_d) is shifted into the word,
+
+            // Exactly one block maximum and one class maximum at or above lim_d <=> exactly one score is (two would differ in their block
+            // or in their class).  t = sat((D - lim) 2^p) is exactly 0 or 1 with lim one unit below lim_d and p such that lim 2^p ~ 2^60;
+            // sum t (1 + i / 512) has count and index in one number.
+            const float lim = lim_d - fabsf(lim_d) * 1.1920929e-7f;
+            const uint32_t eb = (__float_as_uint(lim) >> 23) & 0xFFu;
+            const float big = __uint_as_float((314u - eb) << 23), lb = -lim * big; // 2^(60 - exponent(lim)): exact
+            float tb0 = 0.0f, tb1 = 0.0f, ta0 = 0.0f, ta1 = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 16; i += 2) {
+                tb0 = fmaf(fma_sat(hb[i], big, lb), 1.0f + (float)i * 0.001953125f, tb0);
+                ta0 = fmaf(fma_sat(ga[i], big, lb), 1.0f + (float)i * 0.001953125f, ta0);
+                tb1 = fmaf(fma_sat(hb[i + 1], big, lb), 1.0f + (float)(i + 1) * 0.001953125f, tb1);
+                ta1 = fmaf(fma_sat(ga[i + 1], big, lb), 1.0f + (float)(i + 1) * 0.001953125f, ta1);
+            }
+            const float tb = tb0 + tb1, ta = ta0 + ta1;
+            const int only = (int)((__float_as_uint(tb + 16383.0f) & 15u) * 16 + (__float_as_uint(ta + 16383.0f) & 15u)); // 1 + i / 512 + 16383: i in the low bits
+            const bool single = P.codes && !scan_all && eb - 67u < 188u && tb >= 1.0f && ta >= 1.0f && fmaxf(tb, ta) < 1.07f && only < P.k;
+            if (single && valid) {
+                ++cand_total, ++rows_done;
+                if (only != old_code) {
+                    moved = true;
+                    P.codes[row] = (uint8_t)only; // the only candidate is the reference's choice
+                }
+            }
+            const bool open = valid && !single;
+            if (!__any_sync(0xffffffffu, open)) {
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->tempty[b]); // this accumulator may be overwritten
+                continue;
+            }
+
+            // pass 2, for the warps with an undecided row: one bit per centroid, set when D_j >= lim_d.  The sign of (D_j - lim_d) is shifted into the word,
             // so the bits arrive in reverse order and inverted.
-            uint32_t words[BN / 32];
+            uint32_t words[BN / 32], ra[32], rb[32];
             tmem_ld32_issue(taddr, ra);
             tmem_wait();
 #pragma unroll
@@ -312,7 +336,7 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->tempty[b]); // this accumulator may be overwritten
             bool listed = false;
-            if (valid) {
+            if (open) {
                 int cnt = 0;
 #pragma unroll
                 for (int wd = 0; wd < BN / 32; ++wd) {
@@ -535,7 +559,6 @@ void dense_shortlist(CudaDevice &dev, const DenseWork &w, size_t n, size_t dim, 
     p.n = n;
     p.dim = (int)dim;
     p.k = (int)k;
-    p.ksteps = dimp / 16;
     p.hn = w.half_norms;
     p.frame = w.frame;
     p.xnorm2 = w.norms;
@@ -548,11 +571,22 @@ void dense_shortlist(CudaDevice &dev, const DenseWork &w, size_t n, size_t dim, 
     p.list = w.list;
     p.list_count = w.list_count;
     const size_t smem = dense_tc_smem_bytes();
-    VQB_CUDA_CHECK(cudaFuncSetAttribute(dense_shortlist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const unsigned long long tiles = (n + BM - 1) / BM;
     const unsigned grid = (unsigned)std::min<unsigned long long>(tiles, (unsigned long long)dev.sm_count());
     KernelScope ks(dev, "dense_shortlist");
-    dense_shortlist_kernel<<<grid, 192, smem, dev.stream()>>>(mx, mc, p);
+    auto go = [&](auto kernel) {
+        VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<grid, 192, smem, dev.stream()>>>(mx, mc, p);
+    };
+    switch (dimp / 16) {
+    case 2: go(dense_shortlist_kernel<2>); break;
+    case 3: go(dense_shortlist_kernel<3>); break;
+    case 4: go(dense_shortlist_kernel<4>); break;
+    case 5: go(dense_shortlist_kernel<5>); break;
+    case 6: go(dense_shortlist_kernel<6>); break;
+    case 7: go(dense_shortlist_kernel<7>); break;
+    default: go(dense_shortlist_kernel<8>); break;
+    }
     VQB_CUDA_CHECK(cudaGetLastError());
     dev.count_launch();
 }

@@ -99,6 +99,14 @@ __device__ __forceinline__ float max3f(float a, float b, float c)
     return r;
 }
 
+// a b + c, clamped to [0, 1] (NaN gives 0)
+__device__ __forceinline__ float fma_sat(float a, float b, float c)
+{
+    float d;
+    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
 // nearest TF32 number (10-bit mantissa), ties away from zero
 __device__ __forceinline__ float tf32_round(float v)
 {

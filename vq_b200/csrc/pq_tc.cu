@@ -115,13 +115,6 @@ __device__ __forceinline__ float split_tf32(float v)
     return __fsub_rn(t, __fsub_rn(t, v));
 }
 
-__device__ __forceinline__ float fma_sat(float a, float b, float c)
-{
-    float d;
-    asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-
 // order in which the four sub-spaces of a group are issued: accumulator / team = ss >> 1 alternates
 __device__ __forceinline__ int issue_order(int p) { return ((p & 1) << 1) | (p >> 1); } // 0, 2, 1, 3
 
