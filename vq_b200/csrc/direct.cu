@@ -484,9 +484,9 @@ bool direct_rvq_applicable(const GenericParams &g, bool tensor, size_t smem_limi
 {
     if (g.k > DK_MAX || std::max(direct_smem(8, direct_tk(g.k), g.sd, true), direct_smem(1, direct_tk(g.k), g.sd, true)) > smem_limit - STATIC_SMEM) return false;
     // Against the CUDA-core kernel this one is ahead at every size that was measured (Manhattan, 80,000 x 128, k 256, 8 stages:
-    // 7.2 -> 2.8 ms; cosine: 10.1 -> 2.4 ms).  The tensor-core path takes 10 us and more per launch, four launches per stage, up to
-    // 20,000 rows.
-    return !tensor || (double)g.n * g.k * g.sd <= 2.6e8;
+    // 7.2 -> 2.8 ms; cosine: 10.1 -> 2.4 ms).  The tensor-core path takes about 45 us a stage up to 20,000 rows (five launches);
+    // the two meet at 12,000 rows of 128 (k 256), 50,000 of 128 (k 60), 12,000 of 61 (k 256), 80,000 of 40 (k 20).
+    return !tensor || (double)g.n * (g.k + 64) * (g.sd + 32) <= 4.5e8;
 }
 
 void launch_direct_rvq(CudaDevice &dev, const GenericParams &g, int metric)
