@@ -119,3 +119,16 @@ def test_image_dot_products_within_half_of_the_bound(ctx):
         # (the half norm is added back in f32 for this comparison: its own rounding is allowed for)
         norm = np.linalg.norm(x, axis=1)[:, None] * np.linalg.norm(cb, axis=1).max() + (np.linalg.norm(cb, axis=1) ** 2)[None, :] * 0.01
         assert (err <= 3.5e-6 * norm).all(), float((err / norm).max())
+
+
+@pytest.mark.parametrize("n,dim,depth", [(1, 5, 3), (2, 33, 3), (1025, 7, 12), (2049, 64, 4), (9000, 40, 3), (20_000, 32, 6), (5000, 1, 20)])
+def test_tree_build_bit_exact(oracle, n, dim, depth):
+    """One-warp and streaming statistics, odd widths, nodes of one CTA and of a cluster, levels beyond the ones the host launches
+    blindly, heavily repeated values (ranks inside runs of equal keys, nodes that cannot be split), negative values and zeros."""
+    x = synth.normal(n, dim, n + dim)
+    x[:, 0] = np.round(2 * x[:, 0]) * 40
+    x[n // 2:, dim // 2] = -0.0
+    cent_o, left_o, right_o = oracle.tsvq_fit(x, depth)
+    cent, left, right = vq.TSVQ(x, depth, vq.Distance.Euclidean).tree()
+    assert np.array_equal(left, left_o) and np.array_equal(right, right_o)
+    assert np.array_equal(cent, cent_o)

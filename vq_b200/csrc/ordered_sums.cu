@@ -11,6 +11,7 @@
 
 #include "cuda_device.hpp"
 #include "ordered_sums.cuh"
+#include "row_walk.cuh"
 
 namespace vqb {
 
@@ -20,7 +21,7 @@ constexpr int OL_WARPS = 8, OL_THREADS = 32 * OL_WARPS;
 constexpr unsigned OL_STEP = 1024;   // a chunk is a multiple of this many rows
 constexpr unsigned OL_CHUNKS = 64;   // at most about this many chunks: every list CTA reads the counts of all of them
 constexpr int OL_MAX_K = 4096;       // counters of eight warps in shared memory: 128 KiB
-constexpr int OS_WARPS = 4, OS_BATCH = 8, OS_RING = 8; // 64 rows in flight per warp, 8 KiB of shared memory each
+constexpr int OS_WARPS = 2; // 16 KiB of ring each
 
 template <typename CodeT>
 __global__ void __launch_bounds__(OL_THREADS) ordered_hist_kernel(const CodeT *__restrict__ codes, unsigned n, unsigned chunk, int m, int k,
@@ -111,21 +112,14 @@ __global__ void __launch_bounds__(OL_THREADS) ordered_lists_kernel(const CodeT *
     }
 }
 
-__device__ __forceinline__ void cp_async4(uint32_t dst, const float *src)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
-
 // A warp takes 32 / W clusters side by side, W lanes each (W: the power of two that covers the width, at most 32; wider rows
-// are cut into pieces of 32).  The additions of a cluster are one dependent chain, so what counts is that its rows are there
-// in time: 64 of them travel through a shared-memory ring per warp while the chain consumes earlier ones, and the row numbers
-// are read one batch further ahead.
+// are cut into pieces of 32) and walks their lists (row_walk.cuh).
 template <int W>
 __global__ void __launch_bounds__(32 * OS_WARPS) ordered_sums_kernel(const float *__restrict__ x, unsigned n, unsigned long long ld, int m, int k, int sd,
                                                                      const uint32_t *active, const uint32_t *__restrict__ start,
                                                                      const uint32_t *__restrict__ list, float *sums, uint32_t *counts, int counts_f32)
 {
-    __shared__ float ring[OS_WARPS][OS_RING][OS_BATCH][32];
+    __shared__ WalkRing ring[OS_WARPS];
     const int s = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (active && active[s] == 0) return;
     const int pieces = (sd + 31) / 32; // 1 unless W == 32
@@ -136,43 +130,8 @@ __global__ void __launch_bounds__(32 * OS_WARPS) ordered_sums_kernel(const float
         b = start[(size_t)s * (k + 1) + j];
         len = start[(size_t)s * (k + 1) + j + 1] - b;
     }
-    const uint32_t rows = d < sd ? len : 0u;
-    const uint32_t most = __reduce_max_sync(0xffffffffu, rows);
-    const uint32_t batches = (most + OS_BATCH - 1) / OS_BATCH;
-    const uint32_t *l = list + (size_t)s * n + b;
-    const float *xs = x + (size_t)s * sd + d;
-    float(*buf)[OS_BATCH][32] = ring[warp];
-    uint32_t idx[OS_BATCH];
-    auto fetch_idx = [&](uint32_t batch) {
-#pragma unroll
-        for (int i = 0; i < OS_BATCH; ++i) idx[i] = batch * OS_BATCH + i < rows ? __ldg(l + batch * OS_BATCH + i) : 0u;
-    };
-    auto issue = [&](uint32_t batch) { // always closes a group, so that the count of pending groups stays fixed
-#pragma unroll
-        for (int i = 0; i < OS_BATCH; ++i)
-            if (batch * OS_BATCH + i < rows)
-                cp_async4((uint32_t)__cvta_generic_to_shared(&buf[batch % OS_RING][i][lane]), xs + (size_t)idx[i] * ld);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    fetch_idx(0);
-#pragma unroll 1
-    for (uint32_t p = 0; p + 1 < OS_RING; ++p) {
-        issue(p);
-        fetch_idx(p + 1);
-    }
     float acc = 0.0f;
-#pragma unroll 1
-    for (uint32_t t = 0; t < batches; ++t) {
-        issue(t + OS_RING - 1);
-        fetch_idx(t + OS_RING);
-        asm volatile("cp.async.wait_group %0;" ::"n"(OS_RING - 1) : "memory"); // a lane reads only what it copied itself
-        float v[OS_BATCH];
-#pragma unroll
-        for (int i = 0; i < OS_BATCH; ++i) v[i] = buf[t % OS_RING][i][lane];
-#pragma unroll
-        for (int i = 0; i < OS_BATCH; ++i)
-            if (t * OS_BATCH + i < rows) acc = __fadd_rn(acc, v[i]);
-    }
+    walk_rows<W>(ring[warp], x + (size_t)s * sd + d, ld, list + (size_t)s * n + b, len, d < sd, [&](float v) { acc = __fadd_rn(acc, v); });
     if (j < k && d < sd) {
         sums[((size_t)s * k + j) * sd + d] = acc;
         if (d == 0) counts[(size_t)s * k + j] = counts_f32 ? __float_as_uint((float)len) : len;

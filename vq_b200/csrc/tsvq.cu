@@ -9,12 +9,13 @@
 // split dimension is the last of equal maxima (max_by, 101-105); the median is taken from the sorted values (108-116); the
 // partition is stable (119-122); children exist only when both sides are non-empty (127-141).
 //
-// Per level: chunk_sums_kernel + node_mean_kernel (centroids), node_spread_stream_kernel or node_spread_kernel (spreads of
-// the nodes that split), pick_split_kernel, a 64-bit radix sort of (node, value) keys (CUB, library code off the hot path) from which the medians
-// are read, a flag + exclusive scan (CUB) + scatter for the stable partition, and one small download of the left counts
-// from which the host numbers the children.  The build is not sharded: every rank of a multi-GPU job builds the same tree.
-#include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
+// The levels follow each other without the host: the device numbers the children and lays out the next level, the host
+// launches for as many nodes as the level can have and surplus CTAs leave at once.  Per level: centroids and spreads (one warp per
+// node and 32 dimensions where nodes are small; chunk sums, means and a streaming kernel where they are large), split_kernel (split
+// dimension, keys, median by radix selection, stable partition; one cluster of CTAs per node), next_level_kernel.  A full
+// 64-bit sort of all rows per level, and two round trips to the host, took 0.16 + 0.08 ms of the 0.39 ms of a level of 100,000 x 128.
+// The build is not sharded: every rank of a multi-GPU job builds the same tree.
+#include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cstdlib>
@@ -22,6 +23,7 @@
 
 #include "cuda_device.hpp"
 #include "kernels_common.cuh"
+#include "row_walk.cuh"
 #include "tsvq.hpp"
 #include "umma.cuh"
 
@@ -30,21 +32,22 @@ namespace vqb {
 namespace {
 
 struct NodeInfo {
-    unsigned long long start, count;
-    int split;       // 1: this node is being split at this level
-    int split_dim;
-    float median;
-    unsigned long long sorted_start; // first key of this node in the sorted key array
-    unsigned long long nleft;
-    int child_left, child_right; // ids given by the host after the partition, -1 = none
-    unsigned long long chunk0;   // first of this node's 1024-row chunks in the level's chunk table
-    unsigned int nchunks;
+    unsigned int start, count; // positions of its rows in perm
+    unsigned int chunk0, nchunks; // its 1024-row chunks in the level's chunk table
+    unsigned int nleft;
+    int split; // 1: this node is being split at this level
+};
+
+// What the host does not know of a level: written by next_level_kernel for the level after it.
+struct LevelInfo {
+    int first, count; // its nodes
+    int chunks;
+    int splits;       // nodes of it that are being split
 };
 
 constexpr unsigned MEAN_CHUNK = 1024;
 struct ChunkInfo {
-    unsigned long long start; // position of the chunk's first row in perm
-    unsigned int rows;
+    unsigned int start, rows; // position of the chunk's first row in perm
 };
 
 constexpr uint32_t DEAD = 0xFFFFFFFFu;
@@ -60,95 +63,88 @@ __device__ __forceinline__ float key_f32(uint32_t k)
     return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
 }
 
-// ---- centroids: one warp per (1024-row chunk, 32 dimensions) adds the chunk's rows in data order (lane = dimension; the
-// row numbers of the next 32 rows are requested while the current 32 rows are in flight), then one thread per (node,
-// dimension) adds the node's chunk sums in order and divides.
-__global__ void __launch_bounds__(128) chunk_sums_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
-                                                         const ChunkInfo *chunks, float *partial)
+constexpr int WR_WARPS = 2; // warps per CTA of the kernels that walk rows (16 KiB of ring each)
+
+__global__ void init_tree_kernel(size_t n, int splits, uint32_t *perm, NodeInfo *nodes, ChunkInfo *chunks, LevelInfo *level)
 {
-    const ChunkInfo ch = chunks[blockIdx.x];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t d0 = ((size_t)blockIdx.y * 4 + warp) * 32;
-    if (d0 >= dim) return;
-    const size_t d = d0 + lane;
-    const bool live = d < dim;
-    const uint32_t *rows = perm + ch.start;
-    float acc = 0.0f;
-    uint32_t next = lane < (int)ch.rows ? rows[lane] : DEAD;
-    for (unsigned r0 = 0; r0 < ch.rows; r0 += 32) {
-        const uint32_t mine = next;
-        next = r0 + 32 + lane < ch.rows ? rows[r0 + 32 + lane] : DEAD;
-        float v[32];
-#pragma unroll
-        for (int u = 0; u < 32; ++u) {
-            const uint32_t idx = __shfl_sync(0xffffffffu, mine, u);
-            v[u] = (idx != DEAD && live) ? x[(size_t)idx * dim + d] : 0.0f;
+    const size_t nchunks = (n + MEAN_CHUNK - 1) / MEAN_CHUNK;
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        perm[i] = (uint32_t)i;
+        if (i < nchunks) chunks[i] = ChunkInfo{(unsigned)(i * MEAN_CHUNK), (unsigned)min((size_t)MEAN_CHUNK, n - i * MEAN_CHUNK)};
+        if (i == 0) {
+            nodes[0] = NodeInfo{0u, (unsigned)n, 0u, (unsigned)nchunks, 0u, splits};
+            level[0] = LevelInfo{0, 1, (int)nchunks, splits};
         }
-        const int nrows = (int)min(32u, ch.rows - r0);
-#pragma unroll
-        for (int u = 0; u < 32; ++u)
-            if (u < nrows) acc = __fadd_rn(acc, v[u]);
     }
-    if (live) partial[(size_t)blockIdx.x * dim + d] = acc;
 }
 
-__global__ void node_mean_kernel(const NodeInfo *nodes, int first, int count, size_t dim, const float *partial, float *centroids)
+// ---- large nodes: one warp per (1024-row chunk, 32 dimensions), then one thread per (node, dimension) adds the node's chunk
+// sums in order and divides
+__global__ void __launch_bounds__(32 * WR_WARPS) chunk_sums_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
+                                                                   const LevelInfo *level, const ChunkInfo *chunks, float *partial)
+{
+    __shared__ WalkRing ring[WR_WARPS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t d0 = ((size_t)blockIdx.y * WR_WARPS + warp) * 32, d = d0 + lane;
+    if (blockIdx.x >= (unsigned)level->chunks || d0 >= dim) return;
+    const ChunkInfo ch = chunks[blockIdx.x];
+    float acc = 0.0f;
+    walk_rows<32>(ring[warp], x + d, dim, perm + ch.start, ch.rows, d < dim, [&](float v) { acc = __fadd_rn(acc, v); });
+    if (d < dim) partial[(size_t)blockIdx.x * dim + d] = acc;
+}
+
+__global__ void node_mean_kernel(const NodeInfo *nodes, const LevelInfo *level, size_t dim, const float *partial, float *centroids)
 {
     const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (t >= (size_t)count * dim) return;
-    const int node = first + (int)(t / dim);
+    if (t >= (size_t)level->count * dim) return;
+    const int node = level->first + (int)(t / dim);
     const size_t d = t % dim;
     const NodeInfo nd = nodes[node];
     float total = 0.0f;
-    const float *p = partial + nd.chunk0 * dim + d;
+    const float *p = partial + (size_t)nd.chunk0 * dim + d;
 #pragma unroll 8
     for (unsigned c = 0; c < nd.nchunks; ++c) total = __fadd_rn(total, p[(size_t)c * dim]);
-    centroids[(size_t)node * dim + d] = __fdiv_rn(total, __ull2float_rn(nd.count)); // sum / (len as f32)
+    centroids[(size_t)node * dim + d] = __fdiv_rn(total, __uint2float_rn(nd.count)); // sum / (len as f32)
 }
 
-// ---- spreads, any width: one thread per (node, dimension) walks the node's rows in data order; the additions form one
-// serial chain, so the loads are what can overlap: 48 rows are in flight while the previous 48 are consumed.
-// grid.x = nodes of the level (ids first .. first + gridDim.x), grid.y x 32 threads over dimensions
-__global__ void __launch_bounds__(32) node_spread_kernel(const float *x, size_t dim, const uint32_t *perm, const NodeInfo *nodes, int first,
-                                                         const float *centroids, float *spread)
+// ---- one warp per (node, 32 dimensions): the node's mean (MEAN: the sums of its 1024-row chunks one after the other) and, if
+// it is going to be split, its spread
+template <bool MEAN>
+__global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
+                                                                   const NodeInfo *nodes, const LevelInfo *level, float *centroids, float *spread)
 {
-    const int node = first + blockIdx.x;
+    __shared__ WalkRing ring[WR_WARPS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const size_t groups = (dim + 31) / 32, unit = (size_t)blockIdx.x * WR_WARPS + warp;
+    const size_t in_level = unit / groups, d = unit % groups * 32 + lane;
+    if (in_level >= (size_t)level->count) return;
+    const int node = level->first + (int)in_level;
     const NodeInfo nd = nodes[node];
-    if (!nd.split) return;
+    const bool live = d < dim;
     const uint32_t *rows = perm + nd.start;
-    constexpr int B = 48;
-    for (size_t t = blockIdx.y * 32 + threadIdx.x; t < dim; t += (size_t)gridDim.y * 32) {
-        const float c = centroids[(size_t)node * dim + t];
-        float var = 0.0f;
-        auto add = [&](float v) {
-            const float d = __fsub_rn(v, c);
-            var = __fadd_rn(var, __fmul_rn(d, d));
-        };
-        float cur[B], nxt[B];
-        unsigned long long i = 0;
-        if (nd.count >= (unsigned long long)B) {
-#pragma unroll
-            for (int u = 0; u < B; ++u) cur[u] = x[(size_t)rows[u] * dim + t];
+    float c = 0.0f;
+    if (MEAN) {
+        float total = 0.0f;
+        for (unsigned r = 0; r < nd.count; r += MEAN_CHUNK) {
+            float acc = 0.0f;
+            walk_rows<32>(ring[warp], x + d, dim, rows + r, min(MEAN_CHUNK, nd.count - r), live, [&](float v) { acc = __fadd_rn(acc, v); });
+            total = __fadd_rn(total, acc);
         }
-        for (; i + B <= nd.count; i += B) {
-            const bool more = i + 2 * B <= nd.count;
-            if (more) {
-#pragma unroll
-                for (int u = 0; u < B; ++u) nxt[u] = x[(size_t)rows[i + B + u] * dim + t];
-            }
-#pragma unroll
-            for (int u = 0; u < B; ++u) add(cur[u]);
-            if (more) {
-#pragma unroll
-                for (int u = 0; u < B; ++u) cur[u] = nxt[u];
-            }
-        }
-        for (; i < nd.count; ++i) add(x[(size_t)rows[i] * dim + t]);
-        spread[(size_t)blockIdx.x * dim + t] = var;
+        c = __fdiv_rn(total, __uint2float_rn(nd.count));
+        if (live) centroids[(size_t)node * dim + d] = c;
+    } else if (live) {
+        c = centroids[(size_t)node * dim + d];
     }
+    if (!nd.split) return;
+    float var = 0.0f;
+    walk_rows<32>(ring[warp], x + d, dim, rows, nd.count, live, [&](float v) {
+        const float e = __fsub_rn(v, c);
+        var = __fadd_rn(var, __fmul_rn(e, e));
+    });
+    if (live) spread[in_level * dim + d] = var;
 }
 
-// ---- spreads, rows whose 32-column pieces are whole 128-byte lines (dim a multiple of 32, 16-byte aligned base).  The sum
+// ---- spreads of large nodes, rows whose 32-column pieces are whole 128-byte lines (dim a multiple of 32, 16-byte aligned base).  The sum
 // stays one serial f32 chain per (node, dimension) in data order -- a dependent addition every 5.8 cycles at best -- so the
 // kernel's job is to keep that chain fed: one CTA per (node, 32 dimensions); warp 0 is the consumer (lane = dimension) and
 // does nothing but read stages from shared memory and add; eleven producer warps gather the node's rows (128-bit loads, 64
@@ -179,7 +175,7 @@ constexpr uint32_t NS_SPIN_LIMIT = 1u << 28;
 __device__ __forceinline__ int ns_swizzle(int d) { return ((d & 7) ^ (d >> 3)) & 7; }
 
 __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
-                                                                        const NodeInfo *nodes, int first, const float *centroids, float *spread, int *error)
+                                                                        const NodeInfo *nodes, const LevelInfo *level, const float *centroids, float *spread, int *error)
 {
     extern __shared__ __align__(128) unsigned char ns_smem[];
     float *ring = reinterpret_cast<float *>(ns_smem);
@@ -187,7 +183,8 @@ __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const fl
     volatile uint32_t *filled = reinterpret_cast<volatile uint32_t *>(empty + NS_GROUPS);
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int node = first + blockIdx.x;
+    if (blockIdx.x >= (unsigned)level->count) return;
+    const int node = level->first + (int)blockIdx.x;
     const NodeInfo nd = nodes[node];
     if (!nd.split) return;
     const size_t col0 = (size_t)blockIdx.y * 32;
@@ -328,101 +325,205 @@ __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const fl
     }
 }
 
-// one thread per node of the level: last of equal maxima; NaN is not comparable
-__global__ void pick_split_kernel(NodeInfo *nodes, int first, int count, size_t dim, const float *spread, int *error)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= count) return;
-    NodeInfo &nd = nodes[first + j];
-    if (!nd.split) return;
-    const float *v = spread + (size_t)j * dim;
-    size_t best = 0;
-    for (size_t t = 0; t < dim; ++t) {
-        if (!(v[t] == v[t])) atomicExch(error, 105);
-        if (t > 0 && !(v[t] < v[best])) best = t;
-    }
-    nd.split_dim = (int)best;
-}
+// Everything between a node's spreads and its two halves, one cluster of CTAs per node (one CTA where the level's nodes are
+// small): the split dimension (last of equal maxima), the rows' values along it as ordered keys, the element of rank count / 2 by
+// radix selection (11 + 11 + 10 bits; the CTAs add up their digit counts through distributed shared memory), for an even
+// count its predecessor, the median, and the stable partition.
+constexpr int SP_THREADS = 512, SP_BINS = 2048, SP_CLUSTER = 8;
 
-// key = (node << 32) | ordered value along the node's split dimension; positions outside splitting nodes sort last
-__global__ void make_keys_kernel(const float *x, size_t n, size_t dim, const uint32_t *perm, const uint32_t *pos_node, const NodeInfo *nodes,
-                                 unsigned long long *keys, int *error)
+__global__ void __launch_bounds__(SP_THREADS) split_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm, uint32_t *perm_out,
+                                                           NodeInfo *nodes, const LevelInfo *level, const float *spread, uint32_t *keys, int *error)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t node = pos_node[i];
-        unsigned long long key = ~0ull;
-        if (node != DEAD && nodes[node].split) {
-            const float v = x[(size_t)perm[i] * dim + nodes[node].split_dim];
-            if (!(v == v)) atomicExch(error, 105);
-            key = ((unsigned long long)node << 32) | f32_key(v);
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const unsigned cs = cl.num_blocks(), rank = cl.block_rank();
+    const unsigned in_level = blockIdx.x / cs;
+    if (in_level >= (unsigned)level->count) return; // the whole cluster leaves
+    const int node = level->first + (int)in_level;
+    const NodeInfo nd = nodes[node];
+    if (!nd.split) return;
+    __shared__ __align__(16) uint32_t s_hist[SP_BINS];
+    __shared__ uint32_t s_scan[SP_THREADS / 32], s_bin, s_below, s_left, s_max;
+    __shared__ unsigned long long s_best;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) s_best = 0ull, s_left = 0u, s_max = 0u;
+    __syncthreads();
+    {
+        unsigned long long best = 0ull;
+        for (size_t t = tid; t < dim; t += SP_THREADS) {
+            const float v = spread[(size_t)in_level * dim + t];
+            if (!(v == v)) atomicExch(error, 105); // not comparable
+            const unsigned long long key = ((unsigned long long)f32_key(v) << 32) | (unsigned)t;
+            best = key > best ? key : best;
         }
-        keys[i] = key;
+        atomicMax(&s_best, best);
     }
-}
+    __syncthreads();
+    const size_t split_dim = min((size_t)(uint32_t)s_best, dim - 1);
 
-__global__ void median_kernel(NodeInfo *nodes, int first, int count, const unsigned long long *sorted)
-{
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= count) return;
-    NodeInfo &nd = nodes[first + j];
-    if (!nd.split) return;
-    const unsigned long long *s = sorted + nd.sorted_start;
-    const float hi = key_f32((uint32_t)s[nd.count / 2]);
+    const unsigned per = (nd.count + cs - 1) / cs, r0 = min(nd.count, rank * per), r1 = min(nd.count, r0 + per);
+    const uint32_t *rows = perm + nd.start;
+    uint32_t *own = keys + nd.start;
+    for (unsigned i = r0 + tid; i < r1; i += SP_THREADS) {
+        const float v = __ldg(x + (size_t)rows[i] * dim + split_dim);
+        if (!(v == v)) atomicExch(error, 105);
+        own[i] = f32_key(v);
+    }
+    __syncthreads(); // from here on a CTA reads the keys of its own rows only
+
+    // inclusive scan of one value per thread; the CTA's total in s_scan[last]
+    auto block_scan = [&](uint32_t v) {
+        uint32_t incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        __syncthreads();
+        if (lane == 31) s_scan[warp] = incl;
+        __syncthreads();
+        if (warp == 0) {
+            uint32_t w = lane < SP_THREADS / 32 ? s_scan[lane] : 0u;
+#pragma unroll
+            for (int o = 1; o < SP_THREADS / 32; o <<= 1) {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, w, o);
+                if (lane >= o) w += up;
+            }
+            if (lane < SP_THREADS / 32) s_scan[lane] = w;
+        }
+        __syncthreads();
+        return incl + (warp ? s_scan[warp - 1] : 0u);
+    };
+
+    uint32_t r = nd.count / 2, prefix = 0u, mask = 0u;
+#pragma unroll 1
+    for (int pass = 0; pass < 3; ++pass) {
+        const int shift = pass == 0 ? 21 : pass == 1 ? 10 : 0;
+        const uint32_t digit = pass == 2 ? 1023u : 2047u;
+        for (int b = tid; b < SP_BINS; b += SP_THREADS) s_hist[b] = 0u;
+        __syncthreads();
+        for (unsigned i = r0 + tid; i < r1; i += SP_THREADS) {
+            const uint32_t key = own[i];
+            if ((key & mask) == prefix) atomicAdd(s_hist + ((key >> shift) & digit), 1u);
+        }
+        cl.sync();
+        uint32_t c[SP_BINS / SP_THREADS], sum = 0u;
+#pragma unroll
+        for (int b = 0; b < SP_BINS / SP_THREADS; ++b) c[b] = 0u;
+        for (unsigned q = 0; q < cs; ++q) {
+            const uint4 h = *reinterpret_cast<const uint4 *>(cl.map_shared_rank(s_hist, q) + 4 * tid);
+            c[0] += h.x, c[1] += h.y, c[2] += h.z, c[3] += h.w;
+        }
+#pragma unroll
+        for (int b = 0; b < SP_BINS / SP_THREADS; ++b) sum += c[b];
+        uint32_t below = block_scan(sum) - sum;
+#pragma unroll
+        for (int b = 0; b < SP_BINS / SP_THREADS; ++b) {
+            if (r >= below && r - below < c[b]) s_bin = 4 * tid + b, s_below = below;
+            below += c[b];
+        }
+        cl.sync(); // the counts have been read everywhere before they are cleared
+        prefix |= s_bin << shift, mask |= digit << shift;
+        r -= s_below;
+    }
+    const float hi = key_f32(prefix);
+    float median = hi;
     if (nd.count % 2 == 0) {
-        const float lo = key_f32((uint32_t)s[nd.count / 2 - 1]);
-        nd.median = __fdiv_rn(__fadd_rn(lo, hi), 2.0f);
-    } else {
-        nd.median = hi;
-    }
-}
-
-__global__ void flag_kernel(const float *x, size_t n, size_t dim, const uint32_t *perm, const uint32_t *pos_node, const NodeInfo *nodes, uint32_t *flags)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i <= n; i += (size_t)gridDim.x * blockDim.x) {
-        uint32_t f = 0;
-        if (i < n) {
-            const uint32_t node = pos_node[i];
-            if (node != DEAD && nodes[node].split) f = x[(size_t)perm[i] * dim + nodes[node].split_dim] <= nodes[node].median ? 1u : 0u;
+        float lo = hi; // r > 0: the predecessor equals it
+        if (r == 0) {  // (the same in every CTA)
+            uint32_t low = 0u;
+            for (unsigned i = r0 + tid; i < r1; i += SP_THREADS) {
+                const uint32_t key = own[i];
+                if (key < prefix) low = max(low, key);
+            }
+            low = __reduce_max_sync(0xffffffffu, low);
+            if (lane == 0) atomicMax(&s_max, low);
+            cl.sync();
+            low = 0u;
+            for (unsigned q = 0; q < cs; ++q) low = max(low, *cl.map_shared_rank(&s_max, q));
+            lo = key_f32(low);
         }
-        flags[i] = f;
+        median = __fdiv_rn(__fadd_rn(lo, hi), 2.0f);
     }
+
+    // stable partition: the rows at or below the median first, both sides in their old order
+    uint32_t mine = 0u;
+    for (unsigned i = r0 + tid; i < r1; i += SP_THREADS) mine += key_f32(own[i]) <= median ? 1u : 0u;
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) atomicAdd(&s_left, mine);
+    cl.sync();
+    uint32_t before = 0u, nleft = 0u;
+    for (unsigned q = 0; q < cs; ++q) {
+        const uint32_t l = *cl.map_shared_rank(&s_left, q);
+        before += q < rank ? l : 0u;
+        nleft += l;
+    }
+    cl.sync(); // nobody leaves while its shared memory is still being read
+    for (unsigned t0 = r0; t0 < r1; t0 += SP_THREADS) {
+        const unsigned i = t0 + tid;
+        const bool in = i < r1, left = in && key_f32(own[i]) <= median;
+        const uint32_t incl = block_scan(left ? 1u : 0u), lefts = before + incl - (left ? 1u : 0u);
+        if (in) perm_out[nd.start + (left ? lefts : nleft + (i - lefts))] = rows[i];
+        before += s_scan[SP_THREADS / 32 - 1];
+        // (block_scan's first barrier keeps s_scan until everybody has read the total)
+    }
+    if (rank == 0 && tid == 0) nodes[node].nleft = nleft;
 }
 
-__global__ void count_left_kernel(NodeInfo *nodes, int first, int count, const uint32_t *scan)
+// Numbers the children of a level in order (both or none, src/tsvq.rs:127-141), lays them and their chunks out for the next one.
+__global__ void __launch_bounds__(1024) next_level_kernel(NodeInfo *nodes, const LevelInfo *level, LevelInfo *next, int may_split, int32_t *left, int32_t *right,
+                                                          ChunkInfo *chunks)
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= count) return;
-    NodeInfo &nd = nodes[first + j];
-    if (nd.split) nd.nleft = scan[nd.start + nd.count] - scan[nd.start];
-}
-
-// stable partition of every splitting node's rows: the flagged rows first, both sides in their old order
-__global__ void scatter_kernel(size_t n, const uint32_t *perm, const uint32_t *pos_node, const NodeInfo *nodes, const uint32_t *flags, const uint32_t *scan,
-                               uint32_t *perm_out)
-{
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t node = pos_node[i];
-        size_t dst = i;
-        if (node != DEAD && nodes[node].split) {
-            const NodeInfo &nd = nodes[node];
-            const unsigned long long lr = scan[i] - scan[nd.start];
-            dst = flags[i] ? nd.start + lr : nd.start + nd.nleft + (i - nd.start - lr);
+    __shared__ unsigned long long s_scan[32], s_carry;
+    __shared__ int s_splits;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const LevelInfo li = *level;
+    if (tid == 0) s_carry = 0ull, s_splits = 0;
+    __syncthreads();
+    for (int t0 = 0; t0 < li.count; t0 += 1024) {
+        const int node = li.first + t0 + tid;
+        const bool in = t0 + tid < li.count;
+        NodeInfo nd = {};
+        if (in) nd = nodes[node];
+        const bool has = in && nd.split && nd.nleft > 0 && nd.nleft < nd.count;
+        const unsigned nl = nd.nleft, nr = nd.count - nl;
+        const unsigned cl = (nl + MEAN_CHUNK - 1) / MEAN_CHUNK, cr = (nr + MEAN_CHUNK - 1) / MEAN_CHUNK;
+        // pairs of children in the low, their chunks in the high half
+        const unsigned long long mine = has ? ((unsigned long long)(cl + cr) << 32) | 1ull : 0ull;
+        unsigned long long incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
         }
-        perm_out[dst] = perm[i];
+        if (lane == 31) s_scan[warp] = incl;
+        __syncthreads();
+        unsigned long long at = s_carry + incl - mine;
+        for (int w = 0; w < warp; ++w) at += s_scan[w];
+        if (in) {
+            int l = -1, r = -1;
+            if (has) {
+                l = li.first + li.count + 2 * (int)(uint32_t)at, r = l + 1;
+                const unsigned c0 = (unsigned)(at >> 32);
+                const NodeInfo a = {nd.start, nl, c0, cl, 0u, may_split && nl > 1 ? 1 : 0}, b = {nd.start + nl, nr, c0 + cl, cr, 0u, may_split && nr > 1 ? 1 : 0};
+                nodes[l] = a, nodes[r] = b;
+                for (unsigned c = 0; c < cl; ++c) chunks[c0 + c] = ChunkInfo{a.start + c * MEAN_CHUNK, min(MEAN_CHUNK, nl - c * MEAN_CHUNK)};
+                for (unsigned c = 0; c < cr; ++c) chunks[c0 + cl + c] = ChunkInfo{b.start + c * MEAN_CHUNK, min(MEAN_CHUNK, nr - c * MEAN_CHUNK)};
+                if (a.split + b.split) atomicAdd(&s_splits, a.split + b.split);
+            }
+            left[node] = l, right[node] = r;
+        }
+        __syncthreads();
+        if (tid == 1023) s_carry = at + mine;
+        __syncthreads();
     }
+    if (tid == 0) *next = LevelInfo{li.first + li.count, 2 * (int)(uint32_t)s_carry, (int)(s_carry >> 32), s_splits};
 }
 
-// after the host has numbered the children: every position learns its new node (or none)
-__global__ void relabel_kernel(size_t n, uint32_t *pos_node, const NodeInfo *nodes)
+__global__ void no_children_kernel(const LevelInfo *level, int32_t *left, int32_t *right) // of the deepest level
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const uint32_t node = pos_node[i];
-        if (node == DEAD) continue;
-        const NodeInfo &nd = nodes[node];
-        uint32_t nn = DEAD;
-        if (nd.split && nd.child_left >= 0) nn = (i < nd.start + nd.nleft) ? (uint32_t)nd.child_left : (uint32_t)nd.child_right;
-        pos_node[i] = nn;
-    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < level->count) left[level->first + t] = right[level->first + t] = -1;
 }
 
 template <int METRIC>
@@ -541,6 +642,20 @@ __global__ void __launch_bounds__(TQ_ROWS) tsvq_quantize_tile_kernel(const float
     }
 }
 
+struct Pool { // device memory of one build: freed in stream order, also when something throws
+    CudaDevice &dev;
+    std::vector<void *> all;
+    ~Pool()
+    {
+        for (void *p : all) dev.release(p);
+    }
+    template <typename T> T *get(size_t items)
+    {
+        all.push_back(dev.alloc(sizeof(T) * items));
+        return static_cast<T *>(all.back());
+    }
+};
+
 inline unsigned grid_for(size_t items, int threads, unsigned cap)
 {
     return (unsigned)std::max<size_t>(1, std::min<size_t>((items + threads - 1) / threads, cap));
@@ -554,154 +669,127 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
     if (n >= 0x7FFFFFFFull) throw Error(103, "tsvq: more than 2^31 - 2 rows are not supported");
     cudaStream_t st = dev.stream();
     const size_t cap_nodes = std::min<size_t>(max_depth < 40 ? ((size_t)2 << max_depth) - 1 : 2 * n, 2 * n);
-    std::vector<NodeInfo> h(1);
-    std::vector<size_t> depth_left(1, max_depth);
-    h[0] = NodeInfo{0, n, 0, 0, 0.0f, 0, 0, -1, -1, 0, 0};
-    float *cent = static_cast<float *>(dev.alloc(sizeof(float) * cap_nodes * dim));
-    NodeInfo *nodes_d = static_cast<NodeInfo *>(dev.alloc(sizeof(NodeInfo) * cap_nodes));
-    uint32_t *perm = static_cast<uint32_t *>(dev.alloc(sizeof(uint32_t) * n)), *perm2 = static_cast<uint32_t *>(dev.alloc(sizeof(uint32_t) * n));
-    uint32_t *pos_node = static_cast<uint32_t *>(dev.alloc(sizeof(uint32_t) * n));
-    uint32_t *flags = static_cast<uint32_t *>(dev.alloc(sizeof(uint32_t) * (n + 1))), *scan = static_cast<uint32_t *>(dev.alloc(sizeof(uint32_t) * (n + 1)));
-    unsigned long long *keys = static_cast<unsigned long long *>(dev.alloc(sizeof(unsigned long long) * n));
-    unsigned long long *keys2 = static_cast<unsigned long long *>(dev.alloc(sizeof(unsigned long long) * n));
-    int *error = static_cast<int *>(dev.alloc(sizeof(int)));
-    size_t sort_bytes = 0, scan_bytes = 0;
-    cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, keys, keys2, (int)n, 0, 64, st);
-    cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, flags, scan, (int)(n + 1), st);
-    void *tmp = dev.alloc(std::max(sort_bytes, scan_bytes));
-    size_t tmp_bytes = std::max(sort_bytes, scan_bytes);
-    float *spread = nullptr, *partial = nullptr;
-    ChunkInfo *chunks_d = nullptr;
+    // A level's nodes are "small" when they average at most this many rows: one warp then walks mean and spread in about 12 cycles a
+    // row, while the streaming kernel's 6 cycles cost a CTA with 200 KB of shared memory for every 32 dimensions.
+    constexpr size_t SMALL_NODE = 2048;
+    // The host does not know how many nodes a level has: it launches for the most there can be, and asks from here on, where
+    // that bound would get out of hand.
+    constexpr size_t ASK_LEVEL = 12;
+    Pool pool{dev, {}};
+    NodeInfo *nodes = pool.get<NodeInfo>(cap_nodes);
+    uint32_t *perm = pool.get<uint32_t>(n), *perm2 = pool.get<uint32_t>(n), *keys = pool.get<uint32_t>(n);
+    LevelInfo *levels = pool.get<LevelInfo>(2);
+    int *error = pool.get<int>(1);
+    const size_t n_chunks = (n + MEAN_CHUNK - 1) / MEAN_CHUNK;
+    float *partial = n > SMALL_NODE ? pool.get<float>((n_chunks + n / SMALL_NODE + 2) * dim) : nullptr, *spread = nullptr;
+    ChunkInfo *chunks = nullptr;
     size_t spread_cap = 0, chunk_cap = 0;
-    std::vector<ChunkInfo> chunks;
-    // rows in whole 128-byte pieces of 32 columns: the streaming kernel; any other shape: one thread per (node, dimension)
-    const bool stream_rows = dim % 32 == 0 && dim / 32 <= 65535 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && getenv("VQB_TSVQ_SERIAL_WALK") == nullptr;
-    if (stream_rows) VQB_CUDA_CHECK(cudaFuncSetAttribute(node_spread_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NS_SMEM));
-    auto cleanup = [&] {
-        dev.release(nodes_d), dev.release(perm), dev.release(perm2), dev.release(pos_node), dev.release(flags), dev.release(scan);
-        dev.release(keys), dev.release(keys2), dev.release(error), dev.release(tmp), dev.release(spread), dev.release(partial), dev.release(chunks_d);
+    auto room_for_chunks = [&](size_t level_nodes) {
+        if (n_chunks + level_nodes <= chunk_cap) return;
+        chunk_cap = n_chunks + 2 * level_nodes + 1024;
+        chunks = pool.get<ChunkInfo>(chunk_cap);
     };
+    const bool stream_rows = dim % 32 == 0 && dim / 32 <= 65535 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
+    if (stream_rows) VQB_CUDA_CHECK(cudaFuncSetAttribute(node_spread_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NS_SMEM));
+    const size_t groups = (dim + 31) / 32;
+    float *cent = static_cast<float *>(dev.alloc(sizeof(float) * cap_nodes * dim));
+    int32_t *left = static_cast<int32_t *>(dev.alloc(sizeof(int32_t) * cap_nodes)), *right = static_cast<int32_t *>(dev.alloc(sizeof(int32_t) * cap_nodes));
     try {
         dev.zero(error, sizeof(int));
-        dev.zero(pos_node, sizeof(uint32_t) * n); // every position belongs to node 0
-        {
-            std::vector<uint32_t> id(n);
-            for (size_t i = 0; i < n; ++i) id[i] = (uint32_t)i;
-            dev.upload(perm, id.data(), sizeof(uint32_t) * n);
-        }
-        size_t first = 0;
-        while (first < h.size()) {
-            const size_t level_count = h.size() - first;
-            size_t n_split = 0, sorted = 0;
-            chunks.clear();
-            for (size_t j = first; j < h.size(); ++j) {
-                h[j].chunk0 = chunks.size();
-                h[j].nchunks = (unsigned)((h[j].count + MEAN_CHUNK - 1) / MEAN_CHUNK);
-                for (unsigned long long r = 0; r < h[j].count; r += MEAN_CHUNK)
-                    chunks.push_back(ChunkInfo{h[j].start + r, (unsigned)std::min<unsigned long long>(MEAN_CHUNK, h[j].count - r)});
-                h[j].split = (depth_left[j] > 0 && h[j].count > 1) ? 1 : 0;
-                h[j].sorted_start = sorted;
-                if (h[j].split) {
-                    sorted += h[j].count;
-                    ++n_split;
-                }
-            }
-            dev.upload(nodes_d + first, h.data() + first, sizeof(NodeInfo) * level_count);
-            if (level_count > spread_cap) {
-                dev.release(spread);
-                spread = static_cast<float *>(dev.alloc(sizeof(float) * level_count * dim));
-                spread_cap = level_count;
-            }
-            if (chunks.size() > chunk_cap) {
-                dev.release(partial), dev.release(chunks_d);
-                chunk_cap = chunks.size() + chunks.size() / 2;
-                partial = static_cast<float *>(dev.alloc(sizeof(float) * chunk_cap * dim));
-                chunks_d = static_cast<ChunkInfo *>(dev.alloc(sizeof(ChunkInfo) * chunk_cap));
-            }
-            dev.upload(chunks_d, chunks.data(), sizeof(ChunkInfo) * chunks.size());
-            {
-                KernelScope ks(dev, "tsvq_node_means");
-                chunk_sums_kernel<<<dim3((unsigned)chunks.size(), (unsigned)((dim + 127) / 128)), 128, 0, st>>>(x, dim, perm, chunks_d, partial);
-                node_mean_kernel<<<grid_for(level_count * dim, 128, 1u << 30), 128, 0, st>>>(nodes_d, (int)first, (int)level_count, dim, partial, cent);
-                VQB_CUDA_CHECK(cudaGetLastError());
-                dev.count_launch();
-            }
-            if (n_split == 0) break;
-            {
-                KernelScope ks(dev, "tsvq_node_spreads");
-                if (stream_rows) {
-                    const dim3 grid((unsigned)level_count, (unsigned)(dim / 32));
-                    node_spread_stream_kernel<<<grid, NS_THREADS, NS_SMEM, st>>>(x, dim, perm, nodes_d, (int)first, cent, spread, error);
-                } else {
-                    const dim3 grid((unsigned)level_count, (unsigned)std::min<size_t>((dim + 31) / 32, 64));
-                    node_spread_kernel<<<grid, 32, 0, st>>>(x, dim, perm, nodes_d, (int)first, cent, spread);
-                }
-                VQB_CUDA_CHECK(cudaGetLastError());
-                dev.count_launch();
-            }
-            if (n_split == 0) break;
-            {
-                KernelScope ks(dev, "tsvq_split");
-                pick_split_kernel<<<grid_for(level_count, 128, 1u << 20), 128, 0, st>>>(nodes_d, (int)first, (int)level_count, dim, spread, error);
-                make_keys_kernel<<<grid_for(n, 256, (unsigned)dev.sm_count() * 8), 256, 0, st>>>(x, n, dim, perm, pos_node, nodes_d, keys, error);
-                VQB_CUDA_CHECK(cudaGetLastError());
-                VQB_CUDA_CHECK(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, keys, keys2, (int)n, 0, 64, st));
-                median_kernel<<<grid_for(level_count, 128, 1u << 20), 128, 0, st>>>(nodes_d, (int)first, (int)level_count, keys2);
-                flag_kernel<<<grid_for(n + 1, 256, (unsigned)dev.sm_count() * 8), 256, 0, st>>>(x, n, dim, perm, pos_node, nodes_d, flags);
-                VQB_CUDA_CHECK(cudaGetLastError());
-                VQB_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, flags, scan, (int)(n + 1), st));
-                count_left_kernel<<<grid_for(level_count, 128, 1u << 20), 128, 0, st>>>(nodes_d, (int)first, (int)level_count, scan);
-                scatter_kernel<<<grid_for(n, 256, (unsigned)dev.sm_count() * 8), 256, 0, st>>>(n, perm, pos_node, nodes_d, flags, scan, perm2);
-                VQB_CUDA_CHECK(cudaGetLastError());
-                dev.count_launch();
-            }
-            std::swap(perm, perm2);
+        room_for_chunks(2);
+        init_tree_kernel<<<grid_for(n, 256, (unsigned)dev.sm_count() * 8), 256, 0, st>>>(n, max_depth > 0 && n > 1 ? 1 : 0, perm, nodes, chunks, levels);
+        VQB_CUDA_CHECK(cudaGetLastError());
+        dev.count_launch();
+        LevelInfo known = {0, 1, 0, 0}; // the last level that the host has asked about
+        auto ask = [&](size_t l) {
             int herr = 0;
             dev.download(&herr, error, sizeof(int));
             if (herr == NS_ERR_WAIT) throw Error(100, "tsvq: a wait inside the node statistics kernel ran out");
             if (herr) throw Error(herr, "values are not comparable (NaN in the training data)");
-            dev.download(h.data() + first, nodes_d + first, sizeof(NodeInfo) * level_count);
-            const size_t level_end = h.size();
-            for (size_t j = first; j < level_end; ++j) {
-                if (!h[j].split) continue;
-                const unsigned long long nl = h[j].nleft, nr = h[j].count - nl;
-                if (nl > 0 && nr > 0) { // otherwise neither side is a proper subset: no children (src/tsvq.rs:127-141)
-                    h[j].child_left = (int)h.size();
-                    h.push_back(NodeInfo{h[j].start, nl, 0, 0, 0.0f, 0, 0, -1, -1, 0, 0});
-                    depth_left.push_back(depth_left[j] - 1);
-                    h[j].child_right = (int)h.size();
-                    h.push_back(NodeInfo{h[j].start + nl, nr, 0, 0, 0.0f, 0, 0, -1, -1, 0, 0});
-                    depth_left.push_back(depth_left[j] - 1);
+            dev.download(&known, levels + (l & 1), sizeof known);
+        };
+        size_t most = 1; // nodes that the level can have
+        for (size_t l = 0;; ++l) {
+            const LevelInfo *level = levels + (l & 1);
+            if (l >= ASK_LEVEL) {
+                ask(l);
+                if (known.count == 0) break;
+                most = (size_t)known.count;
+            }
+            const bool deepest = l >= max_depth, small = n / most <= SMALL_NODE;
+            if (!deepest && most > spread_cap) {
+                spread_cap = 2 * most;
+                spread = pool.get<float>(spread_cap * dim);
+            }
+            if (small) {
+                KernelScope ks(dev, "tsvq_node_stats");
+                node_stats_kernel<true><<<grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, nodes, level, cent, spread);
+                VQB_CUDA_CHECK(cudaGetLastError());
+                dev.count_launch();
+            } else {
+                {
+                    KernelScope ks(dev, "tsvq_node_means");
+                    chunk_sums_kernel<<<dim3((unsigned)(n_chunks + most), (unsigned)((groups + WR_WARPS - 1) / WR_WARPS)), 32 * WR_WARPS, 0, st>>>(x, dim, perm, level, chunks,
+                                                                                                                               partial);
+                    node_mean_kernel<<<grid_for(most * dim, 128, 1u << 30), 128, 0, st>>>(nodes, level, dim, partial, cent);
+                    VQB_CUDA_CHECK(cudaGetLastError());
+                    dev.count_launch();
+                    dev.count_launch();
+                }
+                if (!deepest) {
+                    KernelScope ks(dev, "tsvq_node_spreads");
+                    if (stream_rows)
+                        node_spread_stream_kernel<<<dim3((unsigned)most, (unsigned)(dim / 32)), NS_THREADS, NS_SMEM, st>>>(x, dim, perm, nodes, level, cent, spread, error);
+                    else
+                        node_stats_kernel<false><<<grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, nodes, level, cent, spread);
+                    VQB_CUDA_CHECK(cudaGetLastError());
+                    dev.count_launch();
                 }
             }
-            if (h.size() > cap_nodes) throw Error(100, "tsvq: node capacity exceeded");
-            dev.upload(nodes_d + first, h.data() + first, sizeof(NodeInfo) * level_count);
-            relabel_kernel<<<grid_for(n, 256, (unsigned)dev.sm_count() * 8), 256, 0, st>>>(n, pos_node, nodes_d);
+            if (deepest) {
+                no_children_kernel<<<grid_for(most, 256, 1u << 30), 256, 0, st>>>(level, left, right);
+                VQB_CUDA_CHECK(cudaGetLastError());
+                dev.count_launch();
+                ask(l);
+                break;
+            }
+            {
+                KernelScope ks(dev, "tsvq_split");
+                cudaLaunchConfig_t cfg = {};
+                const unsigned cluster = small ? 1u : (unsigned)SP_CLUSTER;
+                cfg.gridDim = dim3((unsigned)most * cluster);
+                cfg.blockDim = dim3(SP_THREADS);
+                cfg.stream = st;
+                cudaLaunchAttribute attr[1];
+                attr[0].id = cudaLaunchAttributeClusterDimension;
+                attr[0].val.clusterDim.x = cluster;
+                attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+                cfg.attrs = attr;
+                cfg.numAttrs = 1;
+                VQB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, split_kernel, x, dim, (const uint32_t *)perm, perm2, nodes, level, (const float *)spread, keys, error));
+                dev.count_launch();
+            }
+            room_for_chunks(std::min(2 * most, n));
+            next_level_kernel<<<1, 1024, 0, st>>>(nodes, level, levels + ((l + 1) & 1), l + 1 < max_depth ? 1 : 0, left, right, chunks);
             VQB_CUDA_CHECK(cudaGetLastError());
             dev.count_launch();
-            first = level_end;
+            std::swap(perm, perm2);
+            most = std::min(2 * most, n);
         }
+        out.dim = dim;
+        out.nodes = (size_t)(known.first + known.count);
+        out.h_left.resize(out.nodes);
+        out.h_right.resize(out.nodes);
+        dev.download(out.h_left.data(), left, sizeof(int32_t) * out.nodes);
+        dev.download(out.h_right.data(), right, sizeof(int32_t) * out.nodes);
     } catch (...) {
         cudaStreamSynchronize(st);
-        cleanup();
-        dev.release(cent);
+        dev.release(cent), dev.release(left), dev.release(right);
         throw;
     }
-    out.dim = dim;
-    out.nodes = h.size();
-    out.h_left.resize(h.size());
-    out.h_right.resize(h.size());
-    for (size_t j = 0; j < h.size(); ++j) {
-        out.h_left[j] = h[j].child_left;
-        out.h_right[j] = h[j].child_right;
-    }
     out.centroids = cent;
-    out.left = static_cast<int32_t *>(dev.alloc(sizeof(int32_t) * h.size()));
-    out.right = static_cast<int32_t *>(dev.alloc(sizeof(int32_t) * h.size()));
-    dev.upload(out.left, out.h_left.data(), sizeof(int32_t) * h.size());
-    dev.upload(out.right, out.h_right.data(), sizeof(int32_t) * h.size());
-    cudaStreamSynchronize(st);
-    cleanup();
+    out.left = left;
+    out.right = right;
 }
 
 template <int METRIC>
