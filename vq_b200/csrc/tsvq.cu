@@ -85,12 +85,12 @@ __global__ void __launch_bounds__(32 * WR_WARPS) chunk_sums_kernel(const float *
 {
     __shared__ WalkRing ring[WR_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t d0 = ((size_t)blockIdx.y * WR_WARPS + warp) * 32, d = d0 + lane;
-    if (blockIdx.x >= (unsigned)level->chunks || d0 >= dim) return;
-    const ChunkInfo ch = chunks[blockIdx.x];
+    const size_t groups = (dim + 31) / 32, unit = (size_t)blockIdx.x * WR_WARPS + warp, chunk = unit / groups, d = unit % groups * 32 + lane;
+    if (chunk >= (size_t)level->chunks) return;
+    const ChunkInfo ch = chunks[chunk];
     float acc = 0.0f;
     walk_rows<32>(ring[warp], x + d, dim, perm + ch.start, ch.rows, d < dim, [&](float v) { acc = __fadd_rn(acc, v); });
-    if (d < dim) partial[(size_t)blockIdx.x * dim + d] = acc;
+    if (d < dim) partial[chunk * dim + d] = acc;
 }
 
 __global__ void node_mean_kernel(const NodeInfo *nodes, const LevelInfo *level, size_t dim, const float *partial, float *centroids)
@@ -109,7 +109,6 @@ __global__ void node_mean_kernel(const NodeInfo *nodes, const LevelInfo *level, 
 
 // ---- one warp per (node, 32 dimensions): the node's mean (MEAN: the sums of its 1024-row chunks one after the other) and, if
 // it is going to be split, its spread
-template <bool MEAN>
 __global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
                                                                    const NodeInfo *nodes, const LevelInfo *level, float *centroids, float *spread)
 {
@@ -122,19 +121,14 @@ __global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *
     const NodeInfo nd = nodes[node];
     const bool live = d < dim;
     const uint32_t *rows = perm + nd.start;
-    float c = 0.0f;
-    if (MEAN) {
-        float total = 0.0f;
-        for (unsigned r = 0; r < nd.count; r += MEAN_CHUNK) {
-            float acc = 0.0f;
-            walk_rows<32>(ring[warp], x + d, dim, rows + r, min(MEAN_CHUNK, nd.count - r), live, [&](float v) { acc = __fadd_rn(acc, v); });
-            total = __fadd_rn(total, acc);
-        }
-        c = __fdiv_rn(total, __uint2float_rn(nd.count));
-        if (live) centroids[(size_t)node * dim + d] = c;
-    } else if (live) {
-        c = centroids[(size_t)node * dim + d];
+    float total = 0.0f;
+    for (unsigned r = 0; r < nd.count; r += MEAN_CHUNK) {
+        float acc = 0.0f;
+        walk_rows<32>(ring[warp], x + d, dim, rows + r, min(MEAN_CHUNK, nd.count - r), live, [&](float v) { acc = __fadd_rn(acc, v); });
+        total = __fadd_rn(total, acc);
     }
+    const float c = __fdiv_rn(total, __uint2float_rn(nd.count));
+    if (live) centroids[(size_t)node * dim + d] = c;
     if (!nd.split) return;
     float var = 0.0f;
     walk_rows<32>(ring[warp], x + d, dim, rows, nd.count, live, [&](float v) {
@@ -144,11 +138,11 @@ __global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *
     if (live) spread[in_level * dim + d] = var;
 }
 
-// ---- spreads of large nodes, rows whose 32-column pieces are whole 128-byte lines (dim a multiple of 32, 16-byte aligned base).  The sum
+// ---- spreads of large nodes.  The sum
 // stays one serial f32 chain per (node, dimension) in data order -- a dependent addition every 5.8 cycles at best -- so the
 // kernel's job is to keep that chain fed: one CTA per (node, 32 dimensions); warp 0 is the consumer (lane = dimension) and
-// does nothing but read stages from shared memory and add; eleven producer warps gather the node's rows (128-bit loads, 64
-// rows per warp in flight, the next stage's row numbers requested meanwhile), form (v - c)^2 with each term rounded like the
+// does nothing but read stages from shared memory and add; eleven producer warps gather the node's rows (128-bit loads where
+// rows are whole 16-byte pieces (VEC), else four 32-bit ones, which still meet the chain's pace; 64 rows per warp in flight, the next stage's row numbers requested meanwhile), form (v - c)^2 with each term rounded like the
 // reference's (src/tsvq.rs:86-98) and store that into a ring of 64-row stages, so the consumer's work per row is a
 // quarter of a shared-memory load and one addition.
 //
@@ -162,7 +156,7 @@ __global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *
 // with an ordinary load one group ahead -- the load is in flight during the additions and is looked at three stages
 // later -- and the consumer hands a group back with one relaxed arrive.  Stage numbers are padded to a multiple of four
 // (padding stages are announced without data) so that every group sees exactly four announcements.
-constexpr int NS_STAGE_ROWS = 64, NS_GROUP = 4, NS_GROUPS = 6, NS_RING = NS_GROUP * NS_GROUPS, NS_PRODUCERS = 11, NS_THREADS = 32 * (1 + NS_PRODUCERS);
+constexpr int NS_STAGE_ROWS = 64, NS_GROUP = 4, NS_GROUPS = 6, NS_RING = NS_GROUP * NS_GROUPS, NS_PRODUCERS = 12, NS_THREADS = 512;
 constexpr int NS_STAGE_BYTES = NS_STAGE_ROWS * 128;
 constexpr int NS_SMEM = NS_RING * NS_STAGE_BYTES + NS_GROUPS * 8 + NS_GROUPS * 4;
 // a producer may wait for the release of a group only when the release before that one has certainly happened (a parity
@@ -174,20 +168,22 @@ constexpr uint32_t NS_SPIN_LIMIT = 1u << 28;
 
 __device__ __forceinline__ int ns_swizzle(int d) { return ((d & 7) ^ (d >> 3)) & 7; }
 
+template <bool VEC>
 __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
                                                                         const NodeInfo *nodes, const LevelInfo *level, const float *centroids, float *spread, int *error)
 {
-    extern __shared__ __align__(128) unsigned char ns_smem[];
+    extern __shared__ __align__(256) unsigned char ns_smem[];
     float *ring = reinterpret_cast<float *>(ns_smem);
     uint64_t *empty = reinterpret_cast<uint64_t *>(ns_smem + NS_RING * NS_STAGE_BYTES);
     volatile uint32_t *filled = reinterpret_cast<volatile uint32_t *>(empty + NS_GROUPS);
     __shared__ int abort_flag;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (blockIdx.x >= (unsigned)level->count) return;
-    const int node = level->first + (int)blockIdx.x;
+    const unsigned groups = (unsigned)((dim + 31) / 32), in_level = blockIdx.x / groups;
+    if (in_level >= (unsigned)level->count) return;
+    const int node = level->first + (int)in_level;
     const NodeInfo nd = nodes[node];
     if (!nd.split) return;
-    const size_t col0 = (size_t)blockIdx.y * 32;
+    const size_t col0 = (size_t)(blockIdx.x % groups) * 32;
     const unsigned long long count = nd.count;
     const uint32_t S = (uint32_t)((count + NS_STAGE_ROWS - 1) / NS_STAGE_ROWS);      // stages with rows
     const uint32_t total = (S + NS_GROUP - 1) / NS_GROUP * NS_GROUP;                   // stage numbers
@@ -197,16 +193,14 @@ __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const fl
     }
     __syncthreads();
     if (warp == 0) {
-        float4 a[16], b[16];
+        float4 a[8], b[8];
         float acc = 0.0f;
         bool ok = true;
-        uint32_t ahead = 0; // filled[] of the group after the current one, as read at the start of the current group
         const int g = ns_swizzle(lane);
-        auto group_ready = [&](uint32_t grp, uint32_t have) { // all four stages of group `grp` announced?
-            const uint32_t need = NS_GROUP * (grp / NS_GROUPS + 1);
+        auto group_ready = [&](uint32_t slot, uint32_t need, uint32_t have) { // have: filled[slot] as read a while ago
             if (have < need) {
                 uint32_t i = 0;
-                while (filled[grp % NS_GROUPS] < need) {
+                while (filled[slot] < need) {
                     if (++i >= NS_SPIN_LIMIT || ((i & 4095u) == 0 && *(volatile int *)&abort_flag)) {
                         if (i >= NS_SPIN_LIMIT) abort_flag = 1, atomicCAS(error, 0, NS_ERR_WAIT);
                         ok = false;
@@ -216,86 +210,104 @@ __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const fl
             }
             __threadfence_block(); // the stages' values are read after their announcement
         };
-        // shared-memory address of this lane's dimension in stage s; a four-row group q sits at + ((q ^ g) << 4) bytes
-        auto stage_addr = [&](uint32_t s) { return smem_u32(ring + (size_t)(s % NS_RING) * (NS_STAGE_BYTES / 4) + lane * NS_STAGE_ROWS); };
+        // this lane's dimension in stage 0 of the ring: the four-row group q of its first (second) 32 rows sits at piece[q] (+ 128) bytes
+        uint32_t piece[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) piece[q] = smem_u32(ring + lane * NS_STAGE_ROWS) + ((q ^ g) << 4);
         // volatile, so that the loads stay where they are written: between the additions, whose issue slots they fill
-        auto load4 = [&](uint32_t addr, int q) {
+        auto load4 = [&](uint32_t at, int q) {
             float4 r;
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(addr + ((q ^ g) << 4)));
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "r"(at + piece[q]));
             return r;
         };
         auto request = [&](uint32_t s, float4(&buf)[16]) {
-            const uint32_t addr = stage_addr(s);
 #pragma unroll
-            for (int q = 0; q < 16; ++q) buf[q] = load4(addr, q);
+            for (int q = 0; q < 16; ++q) buf[q] = load4((s % NS_RING) * NS_STAGE_BYTES, q);
         };
-        // cur holds stage s (s < S)
-        auto step = [&](float4(&cur)[16], float4(&nxt)[16], uint32_t s) {
-            const bool has_next = s + 1 < S;
-            if (has_next && ((s + 1) & (NS_GROUP - 1)) == 0) {
-                group_ready((s + 1) / NS_GROUP, ahead);
-                if (!ok) return;
-            }
-            if ((s & (NS_GROUP - 1)) == 0) ahead = filled[(s / NS_GROUP + 1) % NS_GROUPS];
-            const unsigned long long left = count - (unsigned long long)s * NS_STAGE_ROWS;
-            if (left >= (unsigned long long)NS_STAGE_ROWS && has_next) {
-                const uint32_t addr = stage_addr(s + 1);
+        // adds the 32 rows in cur and loads the ones at byte `at` of the ring: the loads among the first half of the additions, so
+        // that the second half covers their latency
+        auto half_stage = [&](float4(&cur)[8], float4(&nxt)[8], uint32_t at) {
 #pragma unroll
-                for (int q = 0; q < 16; ++q) { // one load of the next stage per four additions of this one
-                    nxt[q] = load4(addr, q);
-                    acc = __fadd_rn(acc, cur[q].x), acc = __fadd_rn(acc, cur[q].y);
-                    acc = __fadd_rn(acc, cur[q].z), acc = __fadd_rn(acc, cur[q].w);
-                }
-            } else {
-                if (has_next) request(s + 1, nxt);
-                const int rows_here = left < (unsigned long long)NS_STAGE_ROWS ? (int)left : NS_STAGE_ROWS;
-#pragma unroll
-                for (int q = 0; q < 16; ++q) {
-                    if (4 * q + 0 < rows_here) acc = __fadd_rn(acc, cur[q].x);
-                    if (4 * q + 1 < rows_here) acc = __fadd_rn(acc, cur[q].y);
-                    if (4 * q + 2 < rows_here) acc = __fadd_rn(acc, cur[q].z);
-                    if (4 * q + 3 < rows_here) acc = __fadd_rn(acc, cur[q].w);
-                }
-            }
-            if ((s & (NS_GROUP - 1)) == NS_GROUP - 1 || s + 1 == S) { // the group's last stage with rows: hand the group back
-                __syncwarp();                                          // every lane has used its values
-                if (lane == 0) mbar_arrive_relaxed(&empty[(s / NS_GROUP) % NS_GROUPS]);
+            for (int q = 0; q < 8; ++q) {
+                if (q < 4) nxt[2 * q] = load4(at, 2 * q), nxt[2 * q + 1] = load4(at, 2 * q + 1);
+                acc = __fadd_rn(acc, cur[q].x), acc = __fadd_rn(acc, cur[q].y);
+                acc = __fadd_rn(acc, cur[q].z), acc = __fadd_rn(acc, cur[q].w);
             }
         };
-        group_ready(0, 0);
-        if (ok) request(0, a);
-        for (uint32_t s = 0; s < S && ok; s += 2) {
-            step(a, b, s);
-            if (s + 1 < S && ok) step(b, a, s + 1);
+        group_ready(0, NS_GROUP, 0);
+        if (ok) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) a[q] = load4(0, q);
         }
-        if (ok) spread[(size_t)blockIdx.x * dim + col0 + lane] = acc;
-    } else {
+        // Groups with another one behind them (their stages are full) run without a branch but the loop's: tests and addresses computed
+        // per stage took 240 cycles beside the 280 of its 64 additions (100,000 rows: 462 -> 310 us).
+        uint32_t at = 0, slot = 0, need = NS_GROUP, s = 0;
+        for (; ok && s + NS_GROUP < S; s += NS_GROUP) {
+            const uint32_t next_slot = slot + 1 == NS_GROUPS ? 0 : slot + 1, next = next_slot * (NS_GROUP * NS_STAGE_BYTES);
+            if (next_slot == 0) need += NS_GROUP;
+            const uint32_t have = filled[next_slot];
+#pragma unroll
+            for (int i = 0; i < NS_GROUP - 1; ++i) {
+                half_stage(a, b, at + i * NS_STAGE_BYTES + 128);
+                half_stage(b, a, at + (i + 1) * NS_STAGE_BYTES);
+            }
+            half_stage(a, b, at + (NS_GROUP - 1) * NS_STAGE_BYTES + 128);
+            group_ready(next_slot, need, have);
+            if (!ok) break;
+            half_stage(b, a, next);
+            __syncwarp(); // every lane has used its values
+            if (lane == 0) mbar_arrive_relaxed(&empty[slot]);
+            at = next, slot = next_slot;
+        }
+        for (; ok && s < S; ++s, at += NS_STAGE_BYTES) { // the last group; nobody waits for its return
+            const uint32_t left = (uint32_t)(count - (unsigned long long)s * NS_STAGE_ROWS);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const float4 v = load4(at + (q >> 3) * 128, q & 7);
+                if (4 * q + 0 < left) acc = __fadd_rn(acc, v.x);
+                if (4 * q + 1 < left) acc = __fadd_rn(acc, v.y);
+                if (4 * q + 2 < left) acc = __fadd_rn(acc, v.z);
+                if (4 * q + 3 < left) acc = __fadd_rn(acc, v.w);
+            }
+        }
+        if (ok && col0 + lane < dim) spread[(size_t)in_level * dim + col0 + lane] = acc;
+    } else if ((warp & 3) != 0) {
         const uint32_t *rows = perm + nd.start;
         const int sub = lane >> 3, piece = lane & 7;
         const float *xcol = x + col0 + piece * 4;
-        const float4 cc = *reinterpret_cast<const float4 *>(centroids + (size_t)node * dim + col0 + piece * 4);
-        // this lane's four dimensions 4 * piece + j: offset of (dimension, four-row group 0, position sub) in a stage
-        int off[4], gj[4];
+        const uint32_t ld = (uint32_t)dim;
+        const int live = (int)min((unsigned long long)4, dim > col0 + piece * 4 ? (unsigned long long)(dim - (col0 + piece * 4)) : 0ull); // this lane's columns
+        auto load_piece = [&](const float *p) {
+            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (VEC) {
+                if (live) r = __ldg(reinterpret_cast<const float4 *>(p));
+            } else {
+                if (live > 0) r.x = __ldg(p);
+                if (live > 1) r.y = __ldg(p + 1);
+                if (live > 2) r.z = __ldg(p + 2);
+                if (live > 3) r.w = __ldg(p + 3);
+            }
+            return r;
+        };
+        const float4 cc = load_piece(centroids + (size_t)node * dim + col0 + piece * 4);
+        // this lane's four dimensions 4 * piece + j, row position sub: a stage begins on 256 bytes, so the four-row group i lies at the
+        // address of group 0 with i exchanged into bits 4 to 7
+        uint32_t dst[4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) gj[j] = ns_swizzle(4 * piece + j), off[j] = (4 * piece + j) * NS_STAGE_ROWS + sub;
+        for (int j = 0; j < 4; ++j) dst[j] = smem_u32(ring + (4 * piece + j) * NS_STAGE_ROWS + sub) + (ns_swizzle(4 * piece + j) << 4);
         uint32_t idx[16];
         auto load_idx = [&](uint32_t s) { // stage numbers past the node's rows give no rows at all
-            const unsigned long long r0 = (unsigned long long)s * NS_STAGE_ROWS + sub;
+            const uint32_t left = s < S ? (uint32_t)count - s * NS_STAGE_ROWS : 0u;
+            const uint32_t *p = rows + (size_t)s * NS_STAGE_ROWS + sub;
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const unsigned long long r = r0 + 4 * i;
-                idx[i] = r < count ? rows[r] : DEAD;
-            }
+            for (int i = 0; i < 16; ++i) idx[i] = 4 * i + sub < left ? p[4 * i] : DEAD;
         };
-        uint32_t s = warp - 1;
-        if (s < total) load_idx(s);
-        for (; s < total; s += NS_PRODUCERS) {
-            const bool padding = s >= S;
-            float4 v[16];
+        auto load_rows = [&](float4(&v)[16]) {
 #pragma unroll
             for (int i = 0; i < 16; ++i)
-                v[i] = idx[i] != DEAD ? __ldg(reinterpret_cast<const float4 *>(xcol + (size_t)idx[i] * dim)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            if (s + NS_PRODUCERS < total) load_idx(s + NS_PRODUCERS);
+                v[i] = idx[i] != DEAD ? load_piece(xcol + (unsigned long long)idx[i] * ld) : make_float4(0.f, 0.f, 0.f, 0.f);
+        };
+        auto put = [&](float4(&v)[16], uint32_t s) { // false: a wait ran out
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 float d;
@@ -305,22 +317,29 @@ __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const fl
                 d = __fsub_rn(v[i].w, cc.w), v[i].w = __fmul_rn(d, d);
             }
             const uint32_t grp = s / NS_GROUP, gslot = grp % NS_GROUPS;
-            if (!mbar_wait(&empty[gslot], ((grp / NS_GROUPS) & 1u) ^ 1u, &abort_flag, error, NS_ERR_WAIT, 100u)) break;
-            if (!padding) {
-                float *dst = ring + (size_t)(s % NS_RING) * (NS_STAGE_BYTES / 4);
+            if (!mbar_wait(&empty[gslot], ((grp / NS_GROUPS) & 1u) ^ 1u, &abort_flag, error, NS_ERR_WAIT, 100u)) return false;
+            if (s < S) { // not padding
+                const uint32_t at = s % NS_RING * NS_STAGE_BYTES;
+                auto store = [&](int j, int i, float value) {
+                    asm volatile("st.shared.f32 [%0], %1;" ::"r"(((at + dst[j]) ^ ((i & 7) << 4)) + (i >> 3) * 128), "f"(value) : "memory");
+                };
 #pragma unroll
-                for (int i = 0; i < 16; ++i) { // row 4 i + sub of the stage: four-row group i, position sub
-                    dst[off[0] + ((i ^ gj[0]) << 2)] = v[i].x;
-                    dst[off[1] + ((i ^ gj[1]) << 2)] = v[i].y;
-                    dst[off[2] + ((i ^ gj[2]) << 2)] = v[i].z;
-                    dst[off[3] + ((i ^ gj[3]) << 2)] = v[i].w;
-                }
+                for (int i = 0; i < 16; ++i) store(0, i, v[i].x), store(1, i, v[i].y), store(2, i, v[i].z), store(3, i, v[i].w);
             }
             __syncwarp();
             if (lane == 0) {
                 __threadfence_block(); // the stage's values before its announcement
                 atomicAdd(const_cast<uint32_t *>(&filled[gslot]), 1u);
             }
+            return true;
+        };
+        float4 v[16];
+        uint32_t s = (warp >> 2) * 3 + (warp & 3) - 1;
+        load_idx(s);
+        for (; s < total; s += NS_PRODUCERS) {
+            load_rows(v);
+            load_idx(s + NS_PRODUCERS);
+            if (!put(v, s)) break;
         }
     }
 }
@@ -689,8 +708,8 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
         chunk_cap = n_chunks + 2 * level_nodes + 1024;
         chunks = pool.get<ChunkInfo>(chunk_cap);
     };
-    const bool stream_rows = dim % 32 == 0 && dim / 32 <= 65535 && reinterpret_cast<uintptr_t>(x) % 16 == 0;
-    if (stream_rows) VQB_CUDA_CHECK(cudaFuncSetAttribute(node_spread_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NS_SMEM));
+    const auto spread_kernel = dim % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 ? node_spread_stream_kernel<true> : node_spread_stream_kernel<false>;
+    VQB_CUDA_CHECK(cudaFuncSetAttribute(spread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NS_SMEM));
     const size_t groups = (dim + 31) / 32;
     float *cent = static_cast<float *>(dev.alloc(sizeof(float) * cap_nodes * dim));
     int32_t *left = static_cast<int32_t *>(dev.alloc(sizeof(int32_t) * cap_nodes)), *right = static_cast<int32_t *>(dev.alloc(sizeof(int32_t) * cap_nodes));
@@ -723,14 +742,13 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
             }
             if (small) {
                 KernelScope ks(dev, "tsvq_node_stats");
-                node_stats_kernel<true><<<grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, nodes, level, cent, spread);
+                node_stats_kernel<<<grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, nodes, level, cent, spread);
                 VQB_CUDA_CHECK(cudaGetLastError());
                 dev.count_launch();
             } else {
                 {
                     KernelScope ks(dev, "tsvq_node_means");
-                    chunk_sums_kernel<<<dim3((unsigned)(n_chunks + most), (unsigned)((groups + WR_WARPS - 1) / WR_WARPS)), 32 * WR_WARPS, 0, st>>>(x, dim, perm, level, chunks,
-                                                                                                                               partial);
+                    chunk_sums_kernel<<<grid_for((n_chunks + most) * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, level, chunks, partial);
                     node_mean_kernel<<<grid_for(most * dim, 128, 1u << 30), 128, 0, st>>>(nodes, level, dim, partial, cent);
                     VQB_CUDA_CHECK(cudaGetLastError());
                     dev.count_launch();
@@ -738,10 +756,7 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
                 }
                 if (!deepest) {
                     KernelScope ks(dev, "tsvq_node_spreads");
-                    if (stream_rows)
-                        node_spread_stream_kernel<<<dim3((unsigned)most, (unsigned)(dim / 32)), NS_THREADS, NS_SMEM, st>>>(x, dim, perm, nodes, level, cent, spread, error);
-                    else
-                        node_stats_kernel<false><<<grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, nodes, level, cent, spread);
+                    spread_kernel<<<grid_for(most * groups, 1, 1u << 30), NS_THREADS, NS_SMEM, st>>>(x, dim, perm, nodes, level, cent, spread, error);
                     VQB_CUDA_CHECK(cudaGetLastError());
                     dev.count_launch();
                 }
