@@ -114,24 +114,24 @@ __global__ void __launch_bounds__(OL_THREADS) ordered_lists_kernel(const CodeT *
 
 // A warp takes 32 / W clusters side by side, W lanes each (W: the power of two that covers the width, at most 32; wider rows
 // are cut into pieces of 32) and walks their lists (row_walk.cuh).
-template <int W>
+template <int W, bool VEC>
 __global__ void __launch_bounds__(32 * OS_WARPS) ordered_sums_kernel(const float *__restrict__ x, unsigned n, unsigned long long ld, int m, int k, int sd,
                                                                      const uint32_t *active, const uint32_t *__restrict__ start,
                                                                      const uint32_t *__restrict__ list, float *sums, uint32_t *counts, int counts_f32)
 {
-    __shared__ WalkRing ring[OS_WARPS];
+    __shared__ __align__(16) WalkRing ring[OS_WARPS];
     const int s = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (active && active[s] == 0) return;
     const int pieces = (sd + 31) / 32; // 1 unless W == 32
     const int unit = blockIdx.x * OS_WARPS + warp;
-    const int j = (unit / pieces) * (32 / W) + lane / W, d = (unit % pieces) * 32 + lane % W;
+    const int j = (unit / pieces) * (32 / W) + lane / W, d0 = (unit % pieces) * 32, d = d0 + lane % W;
     uint32_t b = 0, len = 0;
     if (j < k) {
         b = start[(size_t)s * (k + 1) + j];
         len = start[(size_t)s * (k + 1) + j + 1] - b;
     }
     float acc = 0.0f;
-    walk_rows<W>(ring[warp], x + (size_t)s * sd + d, ld, list + (size_t)s * n + b, len, d < sd, [&](float v) { acc = __fadd_rn(acc, v); });
+    walk_rows<W, VEC>(ring[warp], x + (size_t)s * sd + d0, ld, list + (size_t)s * n + b, len, sd - d0, [&](float v) { acc = __fadd_rn(acc, v); });
     if (j < k && d < sd) {
         sums[((size_t)s * k + j) * sd + d] = acc;
         if (d == 0) counts[(size_t)s * k + j] = counts_f32 ? __float_as_uint((float)len) : len;
@@ -174,10 +174,11 @@ static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const Cod
         auto go = [&](auto kernel) {
             kernel<<<grid, 32 * OS_WARPS, 0, dev.stream()>>>(x, n, sh.ld, m, k, sd, active, start, list, sums, counts, counts_f32);
         };
-        if (w == 4) go(ordered_sums_kernel<4>);
-        else if (w == 8) go(ordered_sums_kernel<8>);
-        else if (w == 16) go(ordered_sums_kernel<16>);
-        else go(ordered_sums_kernel<32>);
+        const bool vec = sd % 4 == 0 && sh.ld % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0; // whole 16-byte pieces
+        if (w == 4) go(vec ? ordered_sums_kernel<4, true> : ordered_sums_kernel<4, false>);
+        else if (w == 8) go(vec ? ordered_sums_kernel<8, true> : ordered_sums_kernel<8, false>);
+        else if (w == 16) go(vec ? ordered_sums_kernel<16, true> : ordered_sums_kernel<16, false>);
+        else go(vec ? ordered_sums_kernel<32, true> : ordered_sums_kernel<32, false>);
         VQB_CUDA_CHECK(cudaGetLastError());
         dev.count_launch();
     }

@@ -4,6 +4,8 @@
 // list, in order.  What is done with the values is one dependent chain of a few cycles a row, so all of the way to memory has to
 // lie ahead of it: 96 rows travel through a shared-memory ring (cp.async) and the row numbers are read another 32 rows
 // earlier, 32 at a time.  (Numbers read one batch of eight ahead cost a round trip to L2 per batch: 97 cycles a row.)
+// Rows of whole 16-byte pieces (VEC) travel four at a time, a piece per lane; others one at a time, an element per lane, which costs
+// four times the instructions.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -11,63 +13,73 @@
 namespace vqb {
 
 constexpr int WALK_BATCH = 8, WALK_BLOCK = 32, WALK_RING = 128; // rows: per commit group, per fetch of numbers, in the ring
-typedef float WalkRing[WALK_RING][32];                          // 16 KiB per warp
+typedef float WalkRing[WALK_RING][32];                          // 16 KiB per warp, 16-byte aligned
 
-// x: the list's first row number 0 at this lane's dimension; rows: this lane's list (the same for its W lanes); count: its length;
-// live: the lane has a dimension.  All lanes of the warp call it together.
-template <int W, typename Use>
-__device__ __forceinline__ void walk_rows(WalkRing &ring, const float *x, size_t ld, const uint32_t *rows, uint32_t count, bool live, Use &&use)
+// x: column 0 of row number 0; rows: this lane's list (the same for its W lanes); count: its length; cols: the list's live
+// columns, at most W of them are used (VEC: a multiple of 4, x on 16 bytes, ld a multiple of 4).  All lanes call it together.
+template <int W, bool VEC, typename Use>
+__device__ __forceinline__ void walk_rows(WalkRing &ring, const float *x, size_t ld, const uint32_t *rows, uint32_t count, int cols, Use &&use)
 {
     constexpr int NR = WALK_BLOCK / W, AHEAD = WALK_RING / WALK_BLOCK - 1; // registers of numbers per block; blocks in flight
-    const int lane = threadIdx.x & 31, sub = lane % W;
+    constexpr int STEP = VEC ? 4 : 1, LANES = W / STEP;                   // rows per copy; lanes per row of a list
+    const int lane = threadIdx.x & 31, sub = lane % W, line = sub / LANES, col = sub % LANES * STEP;
     const uint32_t most = __reduce_max_sync(0xffffffffu, count), blocks = (most + WALK_BLOCK - 1) / WALK_BLOCK;
-    uint32_t now[NR], next[NR];
-    auto numbers = [&](uint32_t(&to)[NR], uint32_t block) {
+    const bool live = col < cols;
+    x += col;
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(&ring[line][lane - sub + col]);
+    uint32_t num[AHEAD + 1][NR];
+    auto numbers = [&](uint32_t(&of)[NR], uint32_t block) {
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
             const uint32_t at = block * WALK_BLOCK + q * W + sub;
-            to[q] = at < count ? __ldg(rows + at) : 0u;
+            of[q] = at < count ? __ldg(rows + at) : 0u;
         }
     };
     auto issue = [&](const uint32_t(&of)[NR], uint32_t block, int batch) { // always closes a group: the number of pending ones stays fixed
+        if (block < blocks) {
+            const uint32_t slot = to + block * WALK_BLOCK % WALK_RING * 128, left = count - block * WALK_BLOCK; // (left is used where positive)
+            const bool some = count > block * WALK_BLOCK && live;
 #pragma unroll
-        for (int i = 0; i < WALK_BATCH; ++i) {
-            const int at = batch * WALK_BATCH + i;
-            const uint32_t row = __shfl_sync(0xffffffffu, of[at / W], at % W, W);
-            if (block * WALK_BLOCK + at < count && live)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(&ring[(block * WALK_BLOCK + at) % WALK_RING][lane])),
-                             "l"(x + (size_t)row * ld)
-                             : "memory");
+            for (int i = 0; i < WALK_BATCH; i += STEP) {
+                const int at = batch * WALK_BATCH + i;
+                const uint32_t row = __shfl_sync(0xffffffffu, of[at / W], at % W + line, W);
+                if (some && at + line < left) {
+                    const float *from = x + (size_t)row * ld;
+                    if (VEC)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(slot + at * 128), "l"(from) : "memory");
+                    else
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(slot + at * 128), "l"(from) : "memory");
+                }
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    numbers(now, 0);
-#pragma unroll 1
-    for (uint32_t b = 0; b < AHEAD; ++b) {
-        numbers(next, b + 1);
 #pragma unroll
-        for (int j = 0; j < WALK_BLOCK / WALK_BATCH; ++j) issue(now, b, j);
+    for (int b = 0; b <= AHEAD; ++b) numbers(num[b], b);
 #pragma unroll
-        for (int q = 0; q < NR; ++q) now[q] = next[q];
-    }
+    for (int b = 0; b < AHEAD; ++b)
+#pragma unroll
+        for (int j = 0; j < WALK_BLOCK / WALK_BATCH; ++j) issue(num[b], b, j);
 #pragma unroll 1
     for (uint32_t b = 0; b < blocks; ++b) {
-        numbers(next, b + AHEAD + 1);
+        numbers(num[0], b + AHEAD + 1);
 #pragma unroll
         for (int j = 0; j < WALK_BLOCK / WALK_BATCH; ++j) {
-            issue(now, b + AHEAD, j);
-            asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD * WALK_BLOCK / WALK_BATCH) : "memory"); // a lane reads only what it copied itself
+            issue(num[AHEAD], b + AHEAD, j); // over rows that every lane has used before the last __syncwarp
+            asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD * WALK_BLOCK / WALK_BATCH) : "memory");
+            __syncwarp();
             float v[WALK_BATCH];
 #pragma unroll
-            for (int i = 0; i < WALK_BATCH; ++i) v[i] = ring[(b * WALK_BLOCK + j * WALK_BATCH + i) % WALK_RING][lane];
+            for (int i = 0; i < WALK_BATCH; ++i) v[i] = ring[b * WALK_BLOCK % WALK_RING + j * WALK_BATCH + i][lane];
 #pragma unroll
             for (int i = 0; i < WALK_BATCH; ++i)
                 if (b * WALK_BLOCK + j * WALK_BATCH + i < count) use(v[i]);
         }
 #pragma unroll
-        for (int q = 0; q < NR; ++q) now[q] = next[q];
+        for (int q = 0; q < NR; ++q) num[AHEAD][q] = num[0][q];
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
 }
 
 } // namespace vqb

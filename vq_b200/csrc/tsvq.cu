@@ -80,16 +80,18 @@ __global__ void init_tree_kernel(size_t n, int splits, uint32_t *perm, NodeInfo 
 
 // ---- large nodes: one warp per (1024-row chunk, 32 dimensions), then one thread per (node, dimension) adds the node's chunk
 // sums in order and divides
+template <bool VEC>
 __global__ void __launch_bounds__(32 * WR_WARPS) chunk_sums_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
                                                                    const LevelInfo *level, const ChunkInfo *chunks, float *partial)
 {
-    __shared__ WalkRing ring[WR_WARPS];
+    __shared__ __align__(16) WalkRing ring[WR_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t groups = (dim + 31) / 32, unit = (size_t)blockIdx.x * WR_WARPS + warp, chunk = unit / groups, d = unit % groups * 32 + lane;
+    const size_t groups = (dim + 31) / 32, unit = (size_t)blockIdx.x * WR_WARPS + warp, chunk = unit / groups, d0 = unit % groups * 32, d = d0 + lane;
     if (chunk >= (size_t)level->chunks) return;
     const ChunkInfo ch = chunks[chunk];
+    const int cols = (int)min(dim - d0, (size_t)32);
     float acc = 0.0f;
-    walk_rows<32>(ring[warp], x + d, dim, perm + ch.start, ch.rows, d < dim, [&](float v) { acc = __fadd_rn(acc, v); });
+    walk_rows<32, VEC>(ring[warp], x + d0, dim, perm + ch.start, ch.rows, cols, [&](float v) { acc = __fadd_rn(acc, v); });
     if (d < dim) partial[chunk * dim + d] = acc;
 }
 
@@ -109,29 +111,31 @@ __global__ void node_mean_kernel(const NodeInfo *nodes, const LevelInfo *level, 
 
 // ---- one warp per (node, 32 dimensions): the node's mean (MEAN: the sums of its 1024-row chunks one after the other) and, if
 // it is going to be split, its spread
+template <bool VEC>
 __global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
                                                                    const NodeInfo *nodes, const LevelInfo *level, float *centroids, float *spread)
 {
-    __shared__ WalkRing ring[WR_WARPS];
+    __shared__ __align__(16) WalkRing ring[WR_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t groups = (dim + 31) / 32, unit = (size_t)blockIdx.x * WR_WARPS + warp;
-    const size_t in_level = unit / groups, d = unit % groups * 32 + lane;
+    const size_t in_level = unit / groups, d0 = unit % groups * 32, d = d0 + lane;
     if (in_level >= (size_t)level->count) return;
     const int node = level->first + (int)in_level;
     const NodeInfo nd = nodes[node];
     const bool live = d < dim;
+    const int cols = (int)min(dim - d0, (size_t)32);
     const uint32_t *rows = perm + nd.start;
     float total = 0.0f;
     for (unsigned r = 0; r < nd.count; r += MEAN_CHUNK) {
         float acc = 0.0f;
-        walk_rows<32>(ring[warp], x + d, dim, rows + r, min(MEAN_CHUNK, nd.count - r), live, [&](float v) { acc = __fadd_rn(acc, v); });
+        walk_rows<32, VEC>(ring[warp], x + d0, dim, rows + r, min(MEAN_CHUNK, nd.count - r), cols, [&](float v) { acc = __fadd_rn(acc, v); });
         total = __fadd_rn(total, acc);
     }
     const float c = __fdiv_rn(total, __uint2float_rn(nd.count));
     if (live) centroids[(size_t)node * dim + d] = c;
     if (!nd.split) return;
     float var = 0.0f;
-    walk_rows<32>(ring[warp], x + d, dim, rows, nd.count, live, [&](float v) {
+    walk_rows<32, VEC>(ring[warp], x + d0, dim, rows, nd.count, cols, [&](float v) {
         const float e = __fsub_rn(v, c);
         var = __fadd_rn(var, __fmul_rn(e, e));
     });
@@ -708,7 +712,8 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
         chunk_cap = n_chunks + 2 * level_nodes + 1024;
         chunks = pool.get<ChunkInfo>(chunk_cap);
     };
-    const auto spread_kernel = dim % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 ? node_spread_stream_kernel<true> : node_spread_stream_kernel<false>;
+    const bool vec = dim % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0; // rows of whole 16-byte pieces
+    const auto spread_kernel = vec ? node_spread_stream_kernel<true> : node_spread_stream_kernel<false>;
     VQB_CUDA_CHECK(cudaFuncSetAttribute(spread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, NS_SMEM));
     const size_t groups = (dim + 31) / 32;
     float *cent = static_cast<float *>(dev.alloc(sizeof(float) * cap_nodes * dim));
@@ -742,13 +747,13 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
             }
             if (small) {
                 KernelScope ks(dev, "tsvq_node_stats");
-                node_stats_kernel<<<grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, nodes, level, cent, spread);
+                (vec ? node_stats_kernel<true> : node_stats_kernel<false>)<<<grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, nodes, level, cent, spread);
                 VQB_CUDA_CHECK(cudaGetLastError());
                 dev.count_launch();
             } else {
                 {
                     KernelScope ks(dev, "tsvq_node_means");
-                    chunk_sums_kernel<<<grid_for((n_chunks + most) * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, level, chunks, partial);
+                    (vec ? chunk_sums_kernel<true> : chunk_sums_kernel<false>)<<<grid_for((n_chunks + most) * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, level, chunks, partial);
                     node_mean_kernel<<<grid_for(most * dim, 128, 1u << 30), 128, 0, st>>>(nodes, level, dim, partial, cent);
                     VQB_CUDA_CHECK(cudaGetLastError());
                     dev.count_launch();
