@@ -132,3 +132,17 @@ def test_tree_build_bit_exact(oracle, n, dim, depth):
     cent, left, right = vq.TSVQ(x, depth, vq.Distance.Euclidean).tree()
     assert np.array_equal(left, left_o) and np.array_equal(right, right_o)
     assert np.array_equal(cent, cent_o)
+
+
+@pytest.mark.parametrize("n,m,sd,k,skew", [(70_000, 16, 8, 256, False), (66_000, 5, 4, 17, False), (9000, 3, 16, 256, True),
+                                           (70_001, 7, 12, 100, True), (4097, 2, 32, 256, False), (1, 1, 8, 1, False), (140_000, 6, 8, 200, True)])
+def test_unordered_sums_follow_the_rows(n, m, sd, k, skew):
+    """Small whole numbers have sums that are exact in any order, so unordered sums (all rows in the first iteration, moved rows
+    after it) must train the same codebooks as ordered ones: one to four sub-spaces per CTA, rows in no whole pieces, queues
+    that run over because most rows share a cluster."""
+    x = np.round(4 * synth.normal(n, m * sd, n + sd)).astype(np.float32)
+    if skew:
+        x[: n - n // 8] = x[0]
+    init = np.stack([np.random.default_rng(s).permutation(n)[:k] for s in range(m)]).astype(np.uint32)
+    fast, ordered = (vq.ProductQuantizer.fit(x, m, k, 6, vq.Distance.SquaredEuclidean, 1, init_idx=init, accumulate=a) for a in (vq.ACCUM_FAST, vq.ACCUM_ORDERED))
+    assert np.array_equal(fast.codebooks, ordered.codebooks)
