@@ -135,7 +135,7 @@ def test_tree_build_bit_exact(oracle, n, dim, depth):
 
 
 @pytest.mark.parametrize("n,m,sd,k,skew", [(70_000, 16, 8, 256, False), (66_000, 5, 4, 17, False), (9000, 3, 16, 256, True),
-                                           (70_001, 7, 12, 100, True), (4097, 2, 32, 256, False), (1, 1, 8, 1, False), (140_000, 6, 8, 200, True)])
+                                           (70_001, 7, 12, 100, True), (4097, 2, 32, 256, False), (66_001, 1, 100, 256, True), (5000, 2, 36, 33, False), (1, 1, 8, 1, False), (140_000, 6, 8, 200, True)])
 def test_unordered_sums_follow_the_rows(n, m, sd, k, skew):
     """Small whole numbers have sums that are exact in any order, so unordered sums (all rows in the first iteration, moved rows
     after it) must train the same codebooks as ordered ones: one to four sub-spaces per CTA, rows in no whole pieces, queues

@@ -1328,9 +1328,10 @@ bool CudaDevice::accumulate_moved(const Shape &sh, const float *x, void *codes_p
     if (off || sh.n_local == 0) return !off;
     const size_t cb = code_bytes(sh.k);
     const int cf = local.counts_f32 ? 1 : 0;
-    // up to 65,536 rows (shards of a job with several ranks) 8-wide sub-spaces move their pairs directly, accum_pairs_moved_kernel: nothing
-    // to clear and to flush; 70,000 x 128: 14.5 against 15.0 us, 300,000: 41 against 30
-    if ((sh.n_local > 65536 || sh.sd != 8) && queue_sums_applicable(*this, sh, x, local.sums, cb)) {
+    // up to 65,536 rows (shards of a job with several ranks) the kernels that move their rows straight in global memory are as fast:
+    // nothing to clear and to flush.  70,000 x 128: 14.5 against 15.0 us in sub-spaces of 8, 13.5 against 15.0 in one; 300,000: 41
+    // against 30 and 37 against 30
+    if ((sh.n_local > 65536 || (sh.sd != 8 && sh.sd < 64)) && queue_sums_applicable(*this, sh, x, local.sums, cb, true)) {
         launch_queue_sums(*this, sh, x, (uint8_t *)codes_prev, (const uint8_t *)codes, active, local.sums, local.counts, local.counts_f32);
         return true;
     }
@@ -1349,7 +1350,7 @@ void CudaDevice::accumulate(const Shape &sh, const float *x, const void *codes, 
         launch_ordered_sums(*this, sh, x, codes, cb, active, buf.sums, buf.counts, buf.counts_f32);
         return;
     }
-    if (!ordered && queue_sums_applicable(*this, sh, x, buf.sums, cb)) {
+    if (!ordered && queue_sums_applicable(*this, sh, x, buf.sums, cb, false)) {
         launch_queue_sums(*this, sh, x, nullptr, (const uint8_t *)codes, active, buf.sums, buf.counts, buf.counts_f32);
         return;
     }

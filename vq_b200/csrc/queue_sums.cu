@@ -11,7 +11,7 @@
 // touch different banks.
 //
 // Measured, moves of k-means iterations, mean of nine: 1M x 128 in 16 sub-spaces, k 256: 117 -> 77 us; 500,000 x 64, 16: 98 -> 39;
-// 400,000 x 256, 8: 179 -> 57.  All rows of the first shape: 238 -> 207 us, i.e. 2.6 TB/s of rows: the integer work of the queues
+// 400,000 x 256, 8: 179 -> 57.  1M of 128, one sub-space: 95 -> 71; 400,000 of 40: 75 (all rows anew) -> 23.  All rows of the first shape: 238 -> 207 us, i.e. 2.6 TB/s of rows: the integer work of the queues
 // (2.2 instructions a cycle) and the trip to memory in front of every four additions share the time.
 #include <algorithm>
 
@@ -22,10 +22,12 @@ namespace vqb {
 
 namespace {
 
-constexpr int QS_THREADS = 512, QS_ROWS = 2048, QS_PER = QS_ROWS / QS_THREADS, QS_BATCH = 4;
+constexpr int QS_ROWS = 2048, QS_BATCH = 4;
+// two CTAs of 512 threads per SM; wide rows leave room for the sums of one
+__host__ __device__ constexpr int qs_threads(int le) { return le == 32 ? 1024 : 512; }
 // a queue entry: row within the piece (11 bits), bin / teams (4 bits), sign
 constexpr int QS_ROW_BITS = 11, QS_MAX_BINS_PER_TEAM = 16;
-static_assert(QS_PER * 8 <= 32, "a bit per entry of a thread");
+static_assert(QS_ROWS / 512 * 8 <= 32, "a bit per entry of a thread");
 static_assert(QS_ROWS == 1 << QS_ROW_BITS, "a row of a piece has to fit its bits");
 
 struct QsParams {
@@ -48,8 +50,9 @@ __device__ __forceinline__ void qs_count(const QsParams &P, size_t at, int c)
 
 // LE: lanes per team (a power of two, 4 * LE >= sd); G: sub-spaces per CTA; MOVED: codes_prev is given
 template <int LE, int G, bool MOVED>
-__global__ void __launch_bounds__(QS_THREADS, 2) queue_sums_kernel(const QsParams P)
+__global__ void __launch_bounds__(qs_threads(LE), 1024 / qs_threads(LE)) queue_sums_kernel(const QsParams P)
 {
+    constexpr int QS_THREADS = qs_threads(LE), QS_PER = QS_ROWS / QS_THREADS;
     constexpr int TEAMS = QS_THREADS / LE;
     extern __shared__ __align__(16) unsigned char qs_smem[];
     const int bins = P.k * G, g0 = blockIdx.y * G, gc = min(G, P.m - g0);
@@ -197,7 +200,8 @@ Plan plan(size_t m, size_t k, size_t sd, size_t budget)
 {
     Plan p = {1, 4, 0, 0};
     while (4 * (size_t)p.le < sd) p.le *= 2;
-    const int teams = QS_THREADS / p.le;
+    if (p.le > 8) p.le = 32, p.g = 1;
+    const int teams = qs_threads(p.le) / p.le;
     while (p.g > 1 && (size_t)p.g / 2 >= m) p.g /= 2;
     for (;; p.g /= 2) {
         p.cap = QS_ROWS * p.g / teams * 3 / 2 + 32;
@@ -210,7 +214,7 @@ template <int LE, int G> void launch(CudaDevice &dev, const QsParams &q, dim3 gr
 {
     auto kernel = q.prev ? queue_sums_kernel<LE, G, true> : queue_sums_kernel<LE, G, false>;
     VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, QS_THREADS, smem, dev.stream()>>>(q);
+    kernel<<<grid, qs_threads(LE), smem, dev.stream()>>>(q);
     VQB_CUDA_CHECK(cudaGetLastError());
     dev.count_launch();
 }
@@ -224,9 +228,10 @@ template <int LE> void launch(CudaDevice &dev, const QsParams &q, int g, dim3 gr
 
 } // namespace
 
-bool queue_sums_applicable(CudaDevice &dev, const Shape &sh, const float *x, const float *sums, size_t code_bytes)
+bool queue_sums_applicable(CudaDevice &dev, const Shape &sh, const float *x, const float *sums, size_t code_bytes, bool moved)
 {
-    if (code_bytes != 1 || sh.sd < 4 || sh.sd > 32 || sh.sd % 4 || sh.ld % 4 || sh.m > 65535u || sh.ld >> 32 || sh.n_local >= (1ull << 40)) return false;
+    // all rows of wide sub-spaces: accum_owner_kernel streams them without queues (1M x 128, k 256: 213 us against 300 and more)
+    if (code_bytes != 1 || sh.sd < 4 || sh.sd > (moved ? 128 : 32) || sh.sd % 4 || sh.ld % 4 || sh.m > 65535u || sh.ld >> 32 || sh.n_local >= (1ull << 40)) return false;
     return ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(sums)) & 15u) == 0 && plan(sh.m, sh.k, sh.sd, dev.smem_limit() - 4096).smem <= dev.smem_limit() - 1024;
 }
 
@@ -236,9 +241,9 @@ void launch_queue_sums(CudaDevice &dev, const Shape &sh, const float *x, uint8_t
     if (sh.n_local == 0) return;
     const Plan p = plan(sh.m, sh.k, sh.sd, dev.smem_limit() - 4096);
     const unsigned ny = (unsigned)((sh.m + p.g - 1) / p.g);
-    const size_t per_sm = p.smem <= (dev.smem_limit() - 4096) / 2 ? 2 : 1;
+    const size_t per_sm = p.le < 32 && p.smem <= (dev.smem_limit() - 4096) / 2 ? 2 : 1;
     size_t gx = std::max<size_t>(1, (size_t)dev.sm_count() * per_sm / ny);
-    gx = std::min<size_t>(gx, (sh.n_local + QS_THREADS - 1) / QS_THREADS);
+    gx = std::min<size_t>(gx, (sh.n_local + 511) / 512);
     gx = std::max<size_t>(gx, sh.n_local >> 30); // row numbers within a CTA are 32 bits wide
     QsParams q = {x, sh.n_local, sh.ld, (sh.n_local + gx - 1) / gx, (int)sh.m, (int)sh.k, (int)sh.sd, p.cap, codes_prev, codes, active, sums, counts, counts_f32 ? 1 : 0};
     KernelScope ks(dev, codes_prev ? "accumulate_moved" : "accumulate_fast");
@@ -246,7 +251,8 @@ void launch_queue_sums(CudaDevice &dev, const Shape &sh, const float *x, uint8_t
     if (p.le == 1) launch<1>(dev, q, p.g, grid, p.smem);
     else if (p.le == 2) launch<2>(dev, q, p.g, grid, p.smem);
     else if (p.le == 4) launch<4>(dev, q, p.g, grid, p.smem);
-    else launch<8>(dev, q, p.g, grid, p.smem);
+    else if (p.le == 8) launch<8>(dev, q, p.g, grid, p.smem);
+    else launch<32, 1>(dev, q, grid, p.smem);
 }
 
 } // namespace vqb
