@@ -146,3 +146,25 @@ def test_unordered_sums_follow_the_rows(n, m, sd, k, skew):
     init = np.stack([np.random.default_rng(s).permutation(n)[:k] for s in range(m)]).astype(np.uint32)
     fast, ordered = (vq.ProductQuantizer.fit(x, m, k, 6, vq.Distance.SquaredEuclidean, 1, init_idx=init, accumulate=a) for a in (vq.ACCUM_FAST, vq.ACCUM_ORDERED))
     assert np.array_equal(fast.codebooks, ordered.codebooks)
+
+
+@pytest.mark.parametrize("metric", ["Euclidean", "SquaredEuclidean"])
+@pytest.mark.parametrize("n,dim", [(1, 3), (5, 32), (203, 33), (130, 64), (77, 100), (66, 127), (1030, 256), (40, 260)])
+def test_tree_lookup_exact_where_the_children_are_close(oracle, n, dim, metric):
+    """Rows on the children's midplane (ties and last-bit differences decide), NaN, infinities, values whose squares vanish or
+    overflow; rows in whole 16-byte pieces and not, one to eight pieces per lane, and the width above which the tile kernel runs."""
+    x = synth.normal(n + 400, dim, n * dim)
+    distance = getattr(vq.Distance, metric)
+    tree = vq.TSVQ(x[n:], 6, distance)
+    cent, left, right = tree.tree()
+    x = x[:n].copy()
+    inner = np.flatnonzero((left >= 0) & (right >= 0))
+    for i in range(0, n, 2):
+        j = inner[i % len(inner)]
+        x[i] = (cent[left[j]] + cent[right[j]]) / 2
+    for i, v in zip(range(3, n, 7), [np.nan, np.inf, -np.inf, 1e30, 1e-30, 2e19, 0.0]):
+        x[i, i % dim:] = v
+    got, leaf = tree.quantize(x, return_leaf=True)
+    want, leaf_o = oracle.tsvq_quantize(cent, left, right, x, METRICS[metric])
+    assert np.array_equal(np.asarray(leaf), leaf_o)
+    assert np.array_equal(np.asarray(got).view(np.uint16), want)

@@ -588,6 +588,110 @@ __global__ void tsvq_quantize_kernel(const float *x, size_t n, size_t dim, const
     }
 }
 
+// The lookup for the Euclidean metrics, rows of up to 256 dimensions: eight lanes per row, four rows per warp.  The row stays in
+// registers; at each node the lanes add up their shares of both children's squared distances, and the smaller one wins where
+// the two differ by more than any order of summation could explain.  The serial chain that the reference evaluates (src/tsvq.rs:
+// 159-175) is only walked where they do not, or where values overflow, vanish or are NaN.
+//
+// Bound: all terms are >= 0, so a sum of dim of them carries a relative error of at most (dim + 2) u in either order (u = 2^-24; a
+// term's own three roundings included), and the square roots of two numbers further apart than 4 u keep their order.  Twice
+// (dim + 2) u + 4 u is well below the (4 dim + 64) u that is asked for.
+//
+// One thread per row reads 16 bytes of 32 different nodes per load: 32 wavefronts where this takes four.  1M x 64, depth 6: 505 -> 241 us;
+// 1M x 127, depth 8: 3070 -> 878 us; one row of 128, depth 8: 34 -> 15 us with the call around it.
+template <int METRIC, bool VEC, int NP>
+__global__ void __launch_bounds__(256) tsvq_quantize_group_kernel(const float *__restrict__ x, size_t n, int dim, const float *__restrict__ centroids,
+                                                                  const int32_t *__restrict__ left, const int32_t *__restrict__ right, float pv,
+                                                                  uint16_t *out_f16, uint32_t *leaf_out)
+{
+    const int lane = threadIdx.x & 31, sub = lane & 7, group = lane >> 3;
+    const float eps = (4.0f * dim + 64.0f) * 5.9604645e-8f;
+    // the lane's q-th share of a row: VEC: columns 4 (sub + 8 q) + e, else sub + 8 (4 q + e)
+    auto load = [&](const float *row, float(&v)[NP][4]) {
+#pragma unroll
+        for (int q = 0; q < NP; ++q) {
+            if (VEC) {
+                float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (4 * (sub + 8 * q) < dim) f = __ldg(reinterpret_cast<const float4 *>(row) + sub + 8 * q);
+                v[q][0] = f.x, v[q][1] = f.y, v[q][2] = f.z, v[q][3] = f.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[q][e] = sub + 8 * (4 * q + e) < dim ? __ldg(row + sub + 8 * (4 * q + e)) : 0.0f;
+            }
+        }
+    };
+    const size_t warps = (size_t)gridDim.x * (blockDim.x >> 5);
+    for (size_t row0 = (blockIdx.x * (size_t)(blockDim.x >> 5) + (threadIdx.x >> 5)) * 4; row0 < n; row0 += warps * 4) {
+        const size_t row = row0 + group;
+        const bool there = row < n;
+        const float *xr = x + (there ? row : n - 1) * dim;
+        float v[NP][4];
+        load(xr, v);
+        int node = 0, l = there ? left[0] : -1, r = there ? right[0] : -1;
+        while (__any_sync(0xffffffffu, l >= 0 || r >= 0)) {
+            const bool both = l >= 0 && r >= 0;
+            int ll = -1, lr = -1, rl = -1, rr = -1; // of the next level, on their way during the distances
+            float sl = 0.0f, sr = 0.0f;
+            if (both) {
+                ll = left[l], lr = right[l], rl = left[r], rr = right[r];
+                float a[NP][4], b[NP][4];
+                load(centroids + (size_t)l * dim, a);
+                load(centroids + (size_t)r * dim, b);
+#pragma unroll
+                for (int q = 0; q < NP; ++q)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float da = v[q][e] - a[q][e], db = v[q][e] - b[q][e];
+                        sl = fmaf(da, da, sl), sr = fmaf(db, db, sr);
+                    }
+            }
+#pragma unroll
+            for (int o = 4; o; o >>= 1) sl += __shfl_xor_sync(0xffffffffu, sl, o), sr += __shfl_xor_sync(0xffffffffu, sr, o);
+            if (both) {
+                const float most = fmaxf(sl, sr);
+                bool go_left = sl < sr;
+                if (!(fabsf(sl - sr) > eps * most && most > 1e-25f && most < 1e37f)) { // the same in the row's eight lanes
+                    const unsigned mates = 0xFFu << (8 * group);
+                    float d = 0.0f;
+                    if (sub < 2) {
+                        const float *c = centroids + (size_t)(sub ? r : l) * dim;
+                        DistAcc<METRIC> acc;
+                        acc.init();
+                        for (int t = 0; t < dim; ++t) acc.step(xr[t], c[t], pv);
+                        d = acc.finish(pv, 0.0f);
+                    }
+                    const float dl = __shfl_sync(mates, d, 8 * group), dr = __shfl_sync(mates, d, 8 * group + 1);
+                    go_left = dl <= dr; // src/tsvq.rs:172: the left child on ties; a NaN distance sends the row right
+                }
+                node = go_left ? l : r;
+                l = go_left ? ll : rl, r = go_left ? lr : rr;
+            } else if (l >= 0 || r >= 0) {
+                node = l >= 0 ? l : r;
+                l = left[node], r = right[node];
+            }
+        }
+        if (!there) continue; // no shuffle follows in this turn, and the next turn's are reached by all or by none
+        if (leaf_out && sub == 0) leaf_out[row] = (uint32_t)node;
+        if (out_f16) {
+            float c[NP][4];
+            load(centroids + (size_t)node * dim, c);
+#pragma unroll
+            for (int q = 0; q < NP; ++q) {
+                if (VEC) {
+                    if (4 * (sub + 8 * q) < dim)
+                        __stcs(reinterpret_cast<uint2 *>(out_f16 + row * dim) + sub + 8 * q,
+                               make_uint2((uint32_t)f32_to_f16_bits(c[q][0]) | ((uint32_t)f32_to_f16_bits(c[q][1]) << 16),
+                                          (uint32_t)f32_to_f16_bits(c[q][2]) | ((uint32_t)f32_to_f16_bits(c[q][3]) << 16)));
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (sub + 8 * (4 * q + e) < dim) out_f16[row * dim + sub + 8 * (4 * q + e)] = f32_to_f16_bits(c[q][e]);
+                }
+            }
+        }
+    }
+}
+
 // Tile variant of the lookup for rows in whole 16-byte pieces (dim a multiple of 8, aligned pointers): a CTA stages 128
 // rows in shared memory with coalesced 128-bit loads (row stride dim + 4 floats, so the per-thread 128-bit reads of the
 // walk are conflict-free), every thread walks the tree for its own row with the same serial distance chains as above but
@@ -812,10 +916,38 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
     out.right = right;
 }
 
+constexpr size_t TQ_GROUP_DIM = 256;
+
+template <int METRIC, bool VEC, int NP>
+static void launch_group(CudaDevice &dev, const TsvqTree &t, double p, const float *x, size_t n, uint16_t *out_f16, uint32_t *leaf)
+{
+    tsvq_quantize_group_kernel<METRIC, VEC, NP><<<grid_for(n, 32, (unsigned)dev.sm_count() * 16), 256, 0, dev.stream()>>>(x, n, (int)t.dim, t.centroids, t.left, t.right,
+                                                                                                                    (float)p, out_f16, leaf);
+    VQB_CUDA_CHECK(cudaGetLastError());
+    dev.count_launch();
+}
+
+template <int METRIC, bool VEC>
+static void launch_group(CudaDevice &dev, const TsvqTree &t, double p, const float *x, size_t n, uint16_t *out_f16, uint32_t *leaf)
+{
+    if (t.dim <= 32) launch_group<METRIC, VEC, 1>(dev, t, p, x, n, out_f16, leaf);
+    else if (t.dim <= 64) launch_group<METRIC, VEC, 2>(dev, t, p, x, n, out_f16, leaf);
+    else if (t.dim <= 128) launch_group<METRIC, VEC, 4>(dev, t, p, x, n, out_f16, leaf);
+    else launch_group<METRIC, VEC, 8>(dev, t, p, x, n, out_f16, leaf);
+}
+
 template <int METRIC>
 static void launch_quantize(CudaDevice &dev, const TsvqTree &t, double p, const float *x, size_t n, uint16_t *out_f16, uint32_t *leaf)
 {
     KernelScope ks(dev, "tsvq_quantize");
+    if constexpr (METRIC == M_SQ || METRIC == M_EUCLID) {
+        if (t.dim <= TQ_GROUP_DIM && getenv("VQB_TSVQ_SERIAL_WALK") == nullptr) {
+            const bool vec = t.dim % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(out_f16) % 8 == 0;
+            if (vec) launch_group<METRIC, true>(dev, t, p, x, n, out_f16, leaf);
+            else launch_group<METRIC, false>(dev, t, p, x, n, out_f16, leaf);
+            return;
+        }
+    }
     const size_t tile_smem = sizeof(float) * TQ_ROWS * (t.dim + 4);
     const bool aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(out_f16) % 16 == 0;
     if (t.dim % 8 == 0 && tile_smem <= 200 * 1024 && aligned && getenv("VQB_TSVQ_SERIAL_WALK") == nullptr) {
