@@ -108,12 +108,15 @@ struct In {
     CudaDevice &dev;
     const void *d = nullptr;
     void *owned = nullptr;
-    In(CudaDevice &dv, const void *p, size_t bytes) : dev(dv)
+    In(CudaDevice &dv, const void *p, size_t bytes) : In(dv, p, bytes, [](const void *) {}) {}
+    // before(d) runs ahead of a copy to d: what does not need the bytes yet overlaps with it
+    template <typename Before> In(CudaDevice &dv, const void *p, size_t bytes, Before &&before) : dev(dv)
     {
         if (bytes == 0 || dev.is_device_pointer(p)) {
             d = p;
         } else {
             owned = dev.alloc(bytes);
+            before(owned);
             VQB_CUDA_CHECK(cudaMemcpyAsync(owned, p, bytes, cudaMemcpyHostToDevice, dev.stream()));
             d = owned;
         }
@@ -186,6 +189,17 @@ struct Out {
     }
     template <typename T> T *as() const { return static_cast<T *>(d); }
 };
+
+// both outputs of an encode with one wait
+void finish(Out &a, Out &b)
+{
+    if (a.host || b.host) a.dev.download(a.host, a.d, a.host ? a.bytes : 0, b.host, b.d, b.host ? b.bytes : 0);
+    for (Out *o : {&a, &b}) {
+        if (!o->host) continue;
+        o->dev.release(o->d);
+        o->host = o->d = nullptr;
+    }
+}
 
 // Host buffers in, host buffers out: the items are cut into chunks and walked through a two-slot pipeline so that the
 // upload of chunk i+1, the kernels of chunk i and the download of chunk i-1 overlap (PCIe is full duplex).
@@ -455,8 +469,7 @@ int vqb_tsvq_quantize(vqb_tsvq *t, const float *x, size_t n, size_t dim, uint16_
         In ix(dev, x, sizeof(float) * n * dim);
         Out of(dev, out_f16, sizeof(uint16_t) * n * dim), ol(dev, leaf_out, sizeof(uint32_t) * n);
         tsvq_quantize(dev, t->tree, t->metric, t->p, ix.as<float>(), n, of.as<uint16_t>(), ol.as<uint32_t>());
-        of.finish();
-        ol.finish();
+        finish(of, ol);
     });
 }
 
@@ -708,11 +721,10 @@ int vqb_pq_quantize(vqb_pq *pq, const float *x, size_t n, size_t dim, uint16_t *
             });
             return;
         }
-        In ix(dev, x, sizeof(float) * n * dim);
         Out of(dev, out_f16, sizeof(uint16_t) * n * dim), oc(dev, codes, sizeof(uint32_t) * n * pq->m);
+        In ix(dev, x, sizeof(float) * n * dim, [&](const void *rows) { dev.pq_encode_ahead(sh, (const float *)rows, pq->codebooks, pq->metric, of.as<uint16_t>()); });
         dev.pq_encode(sh, ix.as<float>(), pq->codebooks, pq->metric, pq->p, of.as<uint16_t>(), oc.as<uint32_t>(), nullptr);
-        of.finish();
-        oc.finish();
+        finish(of, oc);
     });
 }
 
@@ -847,8 +859,7 @@ int vqb_rvq_quantize(vqb_rvq *rq, const float *x, size_t n, size_t dim, uint16_t
             dev.rvq_quantize(ix.as<float>(), n, dim, rq->codebooks, rq->stages, rq->k, rq->epsilon, rq->metric, rq->p,
                              of.as<uint16_t>(), oc.as<uint32_t>());
         }
-        of.finish();
-        oc.finish();
+        finish(of, oc);
     });
 }
 
@@ -994,8 +1005,7 @@ int vqb_opq_quantize(vqb_opq *oq, const float *x, size_t n, size_t dim, uint16_t
             throw;
         }
         dev.release(y);
-        of.finish();
-        oc.finish();
+        finish(of, oc);
     });
 }
 

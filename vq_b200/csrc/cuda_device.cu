@@ -311,18 +311,23 @@ size_t CudaDevice::await_piece(const float *x, size_t piece)
 // Small downloads sit on the critical path of every k-means iteration (counts and "changed" flags): they go through a
 // pinned staging buffer together with the tensor-core error word -- one copy, one event -- and the host polls the event
 // instead of blocking in the driver, which keeps the latency at a few microseconds whatever the host scheduler does.
-void CudaDevice::download(void *dst, const void *src, size_t bytes)
+void CudaDevice::download(void *dst, const void *src, size_t bytes) { download(dst, src, bytes, nullptr, nullptr, 0); }
+
+void CudaDevice::download(void *dst, const void *src, size_t bytes, void *dst2, const void *src2, size_t bytes2)
 {
-    if (!bytes) return;
-    if (stage_ && bytes <= STAGE_BYTES - 16) {
-        VQB_CUDA_CHECK(cudaMemcpyAsync(stage_ + 16, src, bytes, cudaMemcpyDeviceToHost, stream_));
+    if (!bytes && !bytes2) return;
+    if (stage_ && bytes <= STAGE_BYTES && bytes2 <= STAGE_BYTES && (bytes + 15) / 16 * 16 + bytes2 <= STAGE_BYTES - 16) {
+        unsigned char *second = stage_ + 16 + (bytes + 15) / 16 * 16;
+        if (bytes) VQB_CUDA_CHECK(cudaMemcpyAsync(stage_ + 16, src, bytes, cudaMemcpyDeviceToHost, stream_));
+        if (bytes2) VQB_CUDA_CHECK(cudaMemcpyAsync(second, src2, bytes2, cudaMemcpyDeviceToHost, stream_));
         if (tc_error_) VQB_CUDA_CHECK(cudaMemcpyAsync(stage_, tc_error_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
         VQB_CUDA_CHECK(cudaEventRecord(stage_event_, stream_));
         cudaError_t q;
         while ((q = cudaEventQuery(stage_event_)) == cudaErrorNotReady) {
         }
         VQB_CUDA_CHECK(q);
-        std::memcpy(dst, stage_ + 16, bytes);
+        if (bytes) std::memcpy(dst, stage_ + 16, bytes);
+        if (bytes2) std::memcpy(dst2, second, bytes2);
         if (tc_error_) {
             const int code = *reinterpret_cast<const int *>(stage_);
             if (code != 0) {
@@ -332,7 +337,8 @@ void CudaDevice::download(void *dst, const void *src, size_t bytes)
         }
         return;
     }
-    VQB_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream_));
+    if (bytes) VQB_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream_));
+    if (bytes2) VQB_CUDA_CHECK(cudaMemcpyAsync(dst2, src2, bytes2, cudaMemcpyDeviceToHost, stream_));
     VQB_CUDA_CHECK(cudaStreamSynchronize(stream_));
     check_tc_error();
 }
@@ -619,6 +625,7 @@ void CudaDevice::assign_train(const Shape &sh, const float *x, const float *cent
         tb.marks = pq_mark_buffer(pq_tc_mark_bytes(sh.n_local, sh.m));
         tb.error_word = tc_error_;
         tb.prepare_operand = (bop_fresh_ != centroids);
+        encode_operand_ = nullptr; // an announced encode that did not come about
         launch_pq_tc(*this, p, M_SQ, true, code_bytes(sh.k), tb);
         bop_fresh_ = nullptr;
         return;
@@ -639,9 +646,30 @@ void CudaDevice::assign_train(const Shape &sh, const float *x, const float *cent
     return;
 }
 
+void CudaDevice::pq_encode_ahead(const Shape &sh, const float *x, const float *codebooks, int metric, const uint16_t *out_f16)
+{
+    encode_operand_ = nullptr;
+    AssignParams p = {};
+    p.x = x;
+    p.n = sh.n_local;
+    p.ld = sh.ld;
+    p.m = (int)sh.m;
+    p.k = (int)sh.k;
+    p.sd = (int)sh.sd;
+    p.centroids = codebooks;
+    p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
+    p.out_vec = !out_f16 || (aligned16(out_f16) && sh.m * sh.sd % 8 == 0);
+    if (sh.n_local == 0 || !pq_tensor_enabled_ || !pq_tc_applicable(p, metric) || direct_encode_applicable(p, true)) return;
+    bop_fresh_ = nullptr;
+    launch_pq_operand_b(*this, codebooks, p.m, p.k, metric == M_COSINE, pq_scratch_);
+    encode_operand_ = codebooks;
+}
+
 void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *codebooks, int metric, double pm,
                                 uint16_t *out_f16, uint32_t *out_codes, float *out_f32, bool cuda_cores_only)
 {
+    const float *ahead = encode_operand_;
+    encode_operand_ = nullptr;
     if (sh.n_local == 0) return;
     const size_t dim = sh.m * sh.sd;
     AssignParams p = {};
@@ -664,8 +692,9 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
         return;
     }
     if (tensor) {
-            bop_fresh_ = nullptr;
+        bop_fresh_ = nullptr;
         PqTcBuffers tb;
+        tb.prepare_operand = ahead != codebooks;
         tb.scratch = pq_scratch_;
         tb.marks = pq_mark_buffer(pq_tc_mark_bytes(sh.n_local, sh.m));
         tb.error_word = tc_error_;

@@ -30,6 +30,11 @@ class CudaDevice : public Device {
     void release(void *p) override;
     void upload(void *dst, const void *src, size_t bytes) override;
     void download(void *dst, const void *src, size_t bytes) override;
+    // two of them with one wait (either may be empty)
+    void download(void *dst, const void *src, size_t bytes, void *dst2, const void *src2, size_t bytes2);
+    // The codebooks' operand of the next pq_encode, which has to have the same arguments: called before its rows are copied in, so
+    // that it is laid out meanwhile.
+    void pq_encode_ahead(const Shape &sh, const float *x, const float *codebooks, int metric, const uint16_t *out_f16);
     void copy(void *dst, const void *src, size_t bytes) override;
     void zero(void *dst, size_t bytes) override;
     size_t code_bytes(size_t k) const override { return k <= 256 ? 1 : (k <= 65536 ? 2 : 4); }
@@ -145,6 +150,7 @@ class CudaDevice : public Device {
     unsigned long long *tc_stats_ = nullptr;
     int *tc_error_ = nullptr;
     void ensure_tc_buffers();
+    const float *encode_operand_ = nullptr; // codebooks whose operand pq_encode_ahead has laid out
     void pq_encode_impl(const Shape &sh, const float *x, const float *codebooks, int metric, double p, uint16_t *out_f16,
                         uint32_t *out_codes, float *out_f32, bool cuda_cores_only);
 

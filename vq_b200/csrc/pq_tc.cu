@@ -683,7 +683,7 @@ static void launch_t(CudaDevice &dev, const CUtensorMap &mb, const PqTcParams &q
     }
 }
 
-static void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, bool cosine, float *scratch)
+void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, bool cosine, float *scratch)
 {
     KernelScope ks(dev, "pq_operand_b");
     auto kernel = cosine ? pq_operand_b_kernel<true> : pq_operand_b_kernel<false>;

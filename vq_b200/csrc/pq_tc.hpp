@@ -25,6 +25,7 @@ struct PqTcBuffers {
     bool prepare_operand = true;  // false: scratch already holds operand B of p.centroids (written by launch_pq_update_centroids)
     float *dbg_scores = nullptr;  // optional: n x m x 256 raw scores
 };
+void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, bool cosine, float *scratch);
 void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train, size_t code_bytes, const PqTcBuffers &b);
 // number of (row, sub-space) pairs the tensor kernel has handed to the exact scan so far (first u64 of the statistics)
 size_t pq_tc_stats_offset_floats();
