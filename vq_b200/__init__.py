@@ -81,10 +81,8 @@ class Distance:
         b = np.ascontiguousarray(b, dtype=np.float32).ravel()
         ctx = ctx or default_context()
         out = np.empty(1, np.float32)
-        rc = _lib.load().vqb_distance_rows(ctx.handle, self.metric, self.p, a.ctypes.data, a.size, b.ctypes.data,
-                                           b.size, 1, out.ctypes.data)
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(None, _lib.load().vqb_distance_rows, ctx.handle, self.metric, self.p, a.ctypes.data, a.size, b.ctypes.data,
+                 b.size, 1, out.ctypes.data)
         return float(out[0])
 
 
@@ -125,6 +123,7 @@ class Context:
         self.handle = h
         self.device = int(device)
         self.rank, self.world = 0, 1
+        self._lock = threading.RLock()  # the stream and the call that is meant for it belong together (call())
         self._stream = None   # what set_stream() was told last
         self._pinned = False  # use_stream() holds the stream whatever the inputs are
 
@@ -142,15 +141,26 @@ class Context:
     def set_stream(self, cuda_stream: int | None):
         """Run on the given cudaStream_t handle (0 = the CUDA default stream); None = the context's own stream."""
         L = _lib.load()
-        rc = L.vqb_ctx_reset_stream(self.handle) if cuda_stream is None else L.vqb_ctx_set_stream(self.handle, C.c_void_p(cuda_stream))
-        if rc:
-            _raise(rc, self.handle)
-        self._stream = cuda_stream
+        with self._lock:
+            rc = L.vqb_ctx_reset_stream(self.handle) if cuda_stream is None else L.vqb_ctx_set_stream(self.handle, C.c_void_p(cuda_stream))
+            if rc:
+                _raise(rc, self.handle)
+            self._stream = cuda_stream
+
+    def call(self, x, fn, *args):
+        """One call of the library, on the stream that the input `x` (an _Arr; None: any stream will do) was handed over on.
+
+        The stream is the context's, not the call's, and another thread may set its own between the two: ctypes lets the
+        interpreter go during every call.  So both happen under one lock, and so does reading the message of a failure."""
+        with self._lock:
+            if x is not None and not self._pinned and x.stream != self._stream:
+                self.set_stream(x.stream)
+            rc = fn(*args)
+            if rc:
+                _raise(rc, self.handle)
 
     def synchronize(self):
-        rc = _lib.load().vqb_ctx_synchronize(self.handle)
-        if rc:
-            _raise(rc, self.handle)
+        self.call(None, _lib.load().vqb_ctx_synchronize, self.handle)
 
     def launch_count(self) -> int:
         n = C.c_uint64(0)
@@ -164,31 +174,26 @@ class Context:
         return int(n.value)
 
     def timing(self, enable: bool):
-        rc = _lib.load().vqb_ctx_timing(self.handle, 1 if enable else 0)
-        if rc:
-            _raise(rc, self.handle)
+        self.call(None, _lib.load().vqb_ctx_timing, self.handle, 1 if enable else 0)
 
     def timing_report(self) -> dict:
         import json
         buf = C.create_string_buffer(1 << 16)
-        rc = _lib.load().vqb_ctx_timing_report(self.handle, buf, len(buf))
-        if rc:
-            _raise(rc, self.handle)
+        self.call(None, _lib.load().vqb_ctx_timing_report, self.handle, buf, len(buf))
         return json.loads(buf.value.decode())
 
     def use_stream(self, cuda_stream: int | None):
         """Pin all work of this context to `cuda_stream` (e.g. torch.cuda.current_stream().cuda_stream), also for
         host-memory inputs; None returns to the default behaviour (caller's torch stream for CUDA tensors, the
         context's own stream for host arrays)."""
-        self._pinned = cuda_stream is not None
-        self.set_stream(cuda_stream)
+        with self._lock:
+            self._pinned = cuda_stream is not None
+            self.set_stream(cuda_stream)
 
     def init_comm(self, unique_id: bytes, rank: int, world: int):
         """Join the NCCL communicator of a one-process-per-GPU job (see vq_b200.distributed)."""
         buf = (C.c_uint8 * _lib.UNIQUE_ID_BYTES).from_buffer_copy(unique_id)
-        rc = _lib.load().vqb_comm_init(self.handle, buf, int(rank), int(world))
-        if rc:
-            _raise(rc, self.handle)
+        self.call(None, _lib.load().vqb_comm_init, self.handle, buf, int(rank), int(world))
         self.rank, self.world = int(rank), int(world)
 
     def exchange_count(self) -> int:
@@ -253,13 +258,14 @@ def _torch_dtype(np_dtype):
 
 
 class _Arr:
-    """A float32 C-contiguous view of the caller's data plus where outputs should live.  One is made per call, and for a single
-    vector the call lasts as long as its host code does: no torch object is created that the result does not need, and the
-    context is told of a stream only when it is another than the last one."""
+    """A float32 C-contiguous view of the caller's data plus where outputs should live and which stream the call belongs on (None:
+    the context's own).  One is made per call, and for a single vector the call lasts as long as its host code does: no torch
+    object is created that the result does not need, and the context is told of a stream only when it is another than the last
+    one (Context.call)."""
 
-    __slots__ = ("cuda", "keep", "shape", "ptr", "single", "n", "dim", "size")
+    __slots__ = ("cuda", "keep", "shape", "ptr", "single", "n", "dim", "size", "stream")
 
-    def __init__(self, x, ctx: Context, want_2d=True):
+    def __init__(self, x, want_2d=True):
         if isinstance(x, Vector):
             x = x.data
         torch = sys.modules.get("torch")
@@ -271,10 +277,7 @@ class _Arr:
             self.shape = x.shape
             self.ptr = x.data_ptr()
             self.size = x.numel()
-            if not ctx._pinned:
-                stream = torch._C._cuda_getCurrentRawStream(x.get_device())
-                if stream != ctx._stream:
-                    ctx.set_stream(stream)
+            self.stream = torch._C._cuda_getCurrentRawStream(x.get_device())
         else:
             if _is_torch(x):
                 x = x.detach().cpu().numpy()
@@ -283,8 +286,7 @@ class _Arr:
             self.shape = a.shape
             self.ptr = a.ctypes.data
             self.size = a.size
-            if not ctx._pinned and ctx._stream is not None:
-                ctx.set_stream(None)
+            self.stream = None
         self.single = len(self.shape) == 1
         if want_2d:
             if self.single:
@@ -319,14 +321,13 @@ class _Arr:
         return a, a.ctypes.data
 
 
-def _rows(training_data, ctx):
+def _rows(training_data):
     """Pack the reference's ``&[Vector<f32>]`` (list of rows) or take an n x dim array as is."""
     if isinstance(training_data, (list, tuple)):
         if len(training_data) == 0:
-            return _Arr(np.zeros((0, 0), np.float32), ctx)
+            return _Arr(np.zeros((0, 0), np.float32))
         training_data = np.stack([v.data if isinstance(v, Vector) else np.asarray(v) for v in training_data])
-    arr = _Arr(training_data, ctx)
-    return arr
+    return _Arr(training_data)
 
 
 class _Seeder:
@@ -377,16 +378,14 @@ class ProductQuantizer:
         shard.  ``init_idx`` (m x k global row indices) and ``draw(stream, n)`` override the seeded stand-in."""
         ctx = ctx or default_context()
         L = _lib.load()
-        x = _rows(training_data, ctx)
+        x = _rows(training_data)
         n_global = _global_rows(x.n, ctx)
         seeder = _Seeder(seed)
         init_idx = seeder.sample(m, n_global, k) if init_idx is None else np.ascontiguousarray(init_idx, dtype=np.uint64)
         cb = seeder.draw_fn(draw)
         h = C.c_void_p()
-        rc = L.vqb_pq_fit(ctx.handle, x.ptr, x.n, x.dim, m, k, max_iters, distance.metric, distance.p,
-                          init_idx.ctypes.data, cb, seeder.handle, accumulate, C.byref(h))
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(x, L.vqb_pq_fit, ctx.handle, x.ptr, x.n, x.dim, m, k, max_iters, distance.metric, distance.p,
+                 init_idx.ctypes.data, cb, seeder.handle, accumulate, C.byref(h))
         return cls(h, ctx, distance)
 
     @classmethod
@@ -395,10 +394,8 @@ class ProductQuantizer:
         cbk = np.ascontiguousarray(codebooks, dtype=np.float32)
         m, k, sd = cbk.shape
         h = C.c_void_p()
-        rc = _lib.load().vqb_pq_from_codebooks(ctx.handle, cbk.ctypes.data, m, k, sd, distance.metric, distance.p,
-                                                C.byref(h))
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(None, _lib.load().vqb_pq_from_codebooks, ctx.handle, cbk.ctypes.data, m, k, sd, distance.metric, distance.p,
+                 C.byref(h))
         return cls(h, ctx, distance)
 
     def shape(self):
@@ -412,9 +409,7 @@ class ProductQuantizer:
     def codebooks(self) -> np.ndarray:
         m, k, sd = self.shape()
         out = np.empty((m, k, sd), np.float32)
-        rc = _lib.load().vqb_pq_codebooks(self._h, out.ctypes.data)
-        if rc:
-            _raise(rc, self._ctx.handle)
+        self._ctx.call(None, _lib.load().vqb_pq_codebooks, self._h, out.ctypes.data)
         return out
 
     @property
@@ -427,12 +422,10 @@ class ProductQuantizer:
     def quantize(self, vector, return_codes: bool = False, out=None):
         """ProductQuantizer::quantize (src/pq.rs:146-187): f16 reconstruction, one row per input vector (written to `out`
         when given: n x dim float16)."""
-        x = _Arr(vector, self._ctx)
+        x = _Arr(vector)
         out, optr = x.empty((x.n, x.dim), np.float16, out)
         codes, cptr = (x.empty((x.n, self.shape()[0]), np.uint32) if return_codes else (None, None))
-        rc = _lib.load().vqb_pq_quantize(self._h, x.ptr, x.n, x.dim, optr, cptr)
-        if rc:
-            _raise(rc, self._ctx.handle)
+        self._ctx.call(x, _lib.load().vqb_pq_quantize, self._h, x.ptr, x.n, x.dim, optr, cptr)
         if x.single:
             out = out[0]
             codes = codes[0] if codes is not None else None
@@ -458,7 +451,7 @@ class ResidualQuantizer:
             ctx: Context | None = None, accumulate: int = ACCUM_AUTO, init=None, draw=None):
         """ResidualQuantizer::fit (src/rvq.rs:87-154).  ``init(stage, n, k)`` overrides the seeded stand-in."""
         ctx = ctx or default_context()
-        x = _rows(training_data, ctx)
+        x = _rows(training_data)
         seeder = _Seeder(seed)
 
         def _init(user, stage, n, kk, out):
@@ -469,10 +462,8 @@ class ResidualQuantizer:
         icb = _lib.INIT_FN(_init) if init else _lib.SEEDER_INIT
         dcb = seeder.draw_fn(draw)
         h = C.c_void_p()
-        rc = _lib.load().vqb_rvq_fit(ctx.handle, x.ptr, x.n, x.dim, stages, k, max_iters, float(epsilon),
-                                     distance.metric, distance.p, icb, dcb, seeder.handle, accumulate, C.byref(h))
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(x, _lib.load().vqb_rvq_fit, ctx.handle, x.ptr, x.n, x.dim, stages, k, max_iters, float(epsilon),
+                 distance.metric, distance.p, icb, dcb, seeder.handle, accumulate, C.byref(h))
         return cls(h, ctx, distance)
 
     @classmethod
@@ -481,10 +472,8 @@ class ResidualQuantizer:
         cbk = np.ascontiguousarray(codebooks, dtype=np.float32)
         stages, k, dim = cbk.shape
         h = C.c_void_p()
-        rc = _lib.load().vqb_rvq_from_codebooks(ctx.handle, cbk.ctypes.data, stages, k, dim, float(epsilon),
-                                                 distance.metric, distance.p, C.byref(h))
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(None, _lib.load().vqb_rvq_from_codebooks, ctx.handle, cbk.ctypes.data, stages, k, dim, float(epsilon),
+                 distance.metric, distance.p, C.byref(h))
         return cls(h, ctx, distance)
 
     def shape(self):
@@ -499,19 +488,15 @@ class ResidualQuantizer:
         s, k, d = self.shape()
         out = np.empty((s, k, d), np.float32)
         if out.size:
-            rc = _lib.load().vqb_rvq_codebooks(self._h, out.ctypes.data)
-            if rc:
-                _raise(rc, self._ctx.handle)
+            self._ctx.call(None, _lib.load().vqb_rvq_codebooks, self._h, out.ctypes.data)
         return out
 
     def quantize(self, vector, return_codes: bool = False, out=None):
         """ResidualQuantizer::quantize (src/rvq.rs:171-215); `out` as in ProductQuantizer.quantize."""
-        x = _Arr(vector, self._ctx)
+        x = _Arr(vector)
         out, optr = x.empty((x.n, x.dim), np.float16, out)
         codes, cptr = (x.empty((x.n, self.shape()[0]), np.uint32) if return_codes else (None, None))
-        rc = _lib.load().vqb_rvq_quantize(self._h, x.ptr, x.n, x.dim, optr, cptr)
-        if rc:
-            _raise(rc, self._ctx.handle)
+        self._ctx.call(x, _lib.load().vqb_rvq_quantize, self._h, x.ptr, x.n, x.dim, optr, cptr)
         if x.single:
             out = out[0]
             codes = codes[0] if codes is not None else None
@@ -537,17 +522,15 @@ class OptimizedProductQuantizer:
             ctx: Context | None = None, accumulate: int = ACCUM_AUTO, init_idx=None):
         """OptimizedProductQuantizer::fit (src/opq.rs:90-205)."""
         ctx = ctx or default_context()
-        x = _rows(training_data, ctx)
+        x = _rows(training_data)
         n_global = _global_rows(x.n, ctx)
         # every outer iteration re-creates StdRng(seed + i) (src/opq.rs:140): same sample, same draws
         seeder = _Seeder(seed)
         init_idx = seeder.sample(m, n_global, k) if init_idx is None else np.ascontiguousarray(init_idx, dtype=np.uint64)
         h = C.c_void_p()
-        rc = _lib.load().vqb_opq_fit(ctx.handle, x.ptr, x.n, x.dim, m, k, max_iters, opq_iters, distance.metric,
-                                     distance.p, init_idx.ctypes.data, seeder.draw_fn(), _lib.SEEDER_RESTART, seeder.handle, accumulate,
-                                     C.byref(h))
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(x, _lib.load().vqb_opq_fit, ctx.handle, x.ptr, x.n, x.dim, m, k, max_iters, opq_iters, distance.metric,
+                 distance.p, init_idx.ctypes.data, seeder.draw_fn(), _lib.SEEDER_RESTART, seeder.handle, accumulate,
+                 C.byref(h))
         return cls(h, ctx, distance, x.dim)
 
     @classmethod
@@ -557,10 +540,8 @@ class OptimizedProductQuantizer:
         cbk = np.ascontiguousarray(codebooks, dtype=np.float32)
         m, k, sd = cbk.shape
         h = C.c_void_p()
-        rc = _lib.load().vqb_opq_from_parts(ctx.handle, rot.ctypes.data, cbk.ctypes.data, m, k, sd, distance.metric,
-                                             distance.p, C.byref(h))
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(None, _lib.load().vqb_opq_from_parts, ctx.handle, rot.ctypes.data, cbk.ctypes.data, m, k, sd, distance.metric,
+                 distance.p, C.byref(h))
         return cls(h, ctx, distance, m * sd)
 
     def shape(self):
@@ -573,9 +554,7 @@ class OptimizedProductQuantizer:
     @property
     def rotation(self) -> np.ndarray:
         out = np.empty((self.dim, self.dim), np.float32)
-        rc = _lib.load().vqb_opq_rotation(self._h, out.ctypes.data)
-        if rc:
-            _raise(rc, self._ctx.handle)
+        self._ctx.call(None, _lib.load().vqb_opq_rotation, self._h, out.ctypes.data)
         return out
 
     @property
@@ -583,23 +562,19 @@ class OptimizedProductQuantizer:
         m, k, sd = self.shape()
         out = np.empty((m, k, sd), np.float32)
         if out.size:
-            rc = _lib.load().vqb_opq_codebooks(self._h, out.ctypes.data)
-            if rc:
-                _raise(rc, self._ctx.handle)
+            self._ctx.call(None, _lib.load().vqb_opq_codebooks, self._h, out.ctypes.data)
         return out
 
     def quantize(self, vector, return_codes: bool = False, out=None):
         """OptimizedProductQuantizer::quantize (src/opq.rs:222-264).  Without codebooks (opq_iters == 0)
         the result is empty, as in the reference.  `out` as in ProductQuantizer.quantize."""
-        x = _Arr(vector, self._ctx)
+        x = _Arr(vector)
         m = self.shape()[0]
         width = x.dim if m else 0
         out, optr = x.empty((x.n, width), np.float16, out)
         codes, cptr = (x.empty((x.n, m), np.uint32) if return_codes else (None, None))
-        rc = _lib.load().vqb_opq_quantize(self._h, x.ptr, x.n, x.dim, optr if width else None,
-                                           cptr if (return_codes and m) else None)
-        if rc:
-            _raise(rc, self._ctx.handle)
+        self._ctx.call(x, _lib.load().vqb_opq_quantize, self._h, x.ptr, x.n, x.dim, optr if width else None,
+                       cptr if (return_codes and m) else None)
         if x.single:
             out = out[0]
             codes = codes[0] if codes is not None else None
@@ -631,11 +606,9 @@ class ScalarQuantizer:
     def quantize(self, vector, out=None):
         """ScalarQuantizer::quantize (src/sq.rs:89-106); any shape, element-wise (into `out` when given: uint8, the input's shape)."""
         ctx = self._ctx or default_context()
-        x = _Arr(vector, ctx, want_2d=False)
+        x = _Arr(vector, want_2d=False)
         out, optr = x.empty(x.shape, np.uint8, out)
-        rc = _lib.load().vqb_sq_quantize(ctx.handle, self.min, self.max, self.levels, self.step, x.ptr, x.size, optr)
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(x, _lib.load().vqb_sq_quantize, ctx.handle, self.min, self.max, self.levels, self.step, x.ptr, x.size, optr)
         return out
 
 
@@ -654,11 +627,9 @@ class BinaryQuantizer:
     def quantize(self, vector, out=None):
         """BinaryQuantizer::quantize (src/bq.rs:75-104); any shape, element-wise (into `out` when given: uint8, the input's shape)."""
         ctx = self._ctx or default_context()
-        x = _Arr(vector, ctx, want_2d=False)
+        x = _Arr(vector, want_2d=False)
         out, optr = x.empty(x.shape, np.uint8, out)
-        rc = _lib.load().vqb_bq_quantize(ctx.handle, self.threshold, self.low, self.high, x.ptr, x.size, optr)
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(x, _lib.load().vqb_bq_quantize, ctx.handle, self.threshold, self.low, self.high, x.ptr, x.size, optr)
         return out
 
 
@@ -668,11 +639,9 @@ class TSVQ:
 
     def __init__(self, training_data, max_depth: int, distance: Distance, *, ctx: Context | None = None):
         ctx = ctx or default_context()
-        x = _rows(training_data, ctx)
+        x = _rows(training_data)
         h = C.c_void_p()
-        rc = _lib.load().vqb_tsvq_fit(ctx.handle, x.ptr, x.n, x.dim, int(max_depth), distance.metric, distance.p, C.byref(h))
-        if rc:
-            _raise(rc, ctx.handle)
+        ctx.call(x, _lib.load().vqb_tsvq_fit, ctx.handle, x.ptr, x.n, x.dim, int(max_depth), distance.metric, distance.p, C.byref(h))
         self._h, self._ctx, self.distance = h, ctx, distance
 
     def shape(self):
@@ -685,19 +654,15 @@ class TSVQ:
         cent = np.empty((nodes, dim), np.float32)
         left = np.empty(nodes, np.int32)
         right = np.empty(nodes, np.int32)
-        rc = _lib.load().vqb_tsvq_tree(self._h, cent.ctypes.data, left.ctypes.data, right.ctypes.data)
-        if rc:
-            _raise(rc, self._ctx.handle)
+        self._ctx.call(None, _lib.load().vqb_tsvq_tree, self._h, cent.ctypes.data, left.ctypes.data, right.ctypes.data)
         return cent, left, right
 
     def quantize(self, vector, return_leaf: bool = False, out=None):
         """TSVQ::quantize (src/tsvq.rs:231-249): one f16 row per input vector; `out` as in ProductQuantizer.quantize."""
-        x = _Arr(vector, self._ctx)
+        x = _Arr(vector)
         out, optr = x.empty((x.n, x.dim), np.float16, out)
         leaf, lptr = (x.empty((x.n,), np.uint32) if return_leaf else (None, None))
-        rc = _lib.load().vqb_tsvq_quantize(self._h, x.ptr, x.n, x.dim, optr, lptr)
-        if rc:
-            _raise(rc, self._ctx.handle)
+        self._ctx.call(x, _lib.load().vqb_tsvq_quantize, self._h, x.ptr, x.n, x.dim, optr, lptr)
         if x.single:
             out = out[0]
             leaf = leaf[0] if leaf is not None else None
@@ -717,7 +682,7 @@ def evaluate(original, quantized_f16, k: int = 10, *, ctx: Context | None = None
     calculate_reconstruction_error and calculate_recall of src/bin/utils.rs:50-127 applied to the f16 output of a
     ``quantize`` call (numpy float16 array or CUDA float16 tensor, one row per vector)."""
     ctx = ctx or default_context()
-    x = _Arr(original, ctx)
+    x = _Arr(original)
     if _is_torch(quantized_f16) and quantized_f16.is_cuda:
         qk = quantized_f16.contiguous()
         qptr = qk.data_ptr()
@@ -725,9 +690,7 @@ def evaluate(original, quantized_f16, k: int = 10, *, ctx: Context | None = None
         qk = np.ascontiguousarray(quantized_f16, dtype=np.float16)
         qptr = qk.ctypes.data
     mse, rec = C.c_float(), C.c_float()
-    rc = _lib.load().vqb_evaluate_f16(ctx.handle, x.ptr, qptr, x.n, x.dim, int(k), C.byref(mse), C.byref(rec))
-    if rc:
-        _raise(rc, ctx.handle)
+    ctx.call(x, _lib.load().vqb_evaluate_f16, ctx.handle, x.ptr, qptr, x.n, x.dim, int(k), C.byref(mse), C.byref(rec))
     return float(mse.value), float(rec.value)
 
 
@@ -735,14 +698,12 @@ def lbg_quantize(data, k: int, max_iters: int, seed: int, *, ctx: Context | None
                  init_idx=None, draw=None):
     """lbg_quantize (src/utils.rs:32-109) on n x d rows.  Returns (centroids k x d, iterations)."""
     ctx = ctx or default_context()
-    x = _rows(data, ctx)
+    x = _rows(data)
     seeder = _Seeder(seed)
     init_idx = seeder.sample(1, x.n, k) if init_idx is None else np.ascontiguousarray(init_idx, dtype=np.uint64)
     cb = seeder.draw_fn(draw)
     out = np.empty((k, x.dim), np.float32)
     iters = C.c_size_t(0)
-    rc = _lib.load().vqb_lbg_fit(ctx.handle, x.ptr, x.n, x.dim, k, max_iters, init_idx.ctypes.data, cb, seeder.handle,
-                                 accumulate, out.ctypes.data if out.size else None, C.byref(iters))
-    if rc:
-        _raise(rc, ctx.handle)
+    ctx.call(x, _lib.load().vqb_lbg_fit, ctx.handle, x.ptr, x.n, x.dim, k, max_iters, init_idx.ctypes.data, cb, seeder.handle,
+             accumulate, out.ctypes.data if out.size else None, C.byref(iters))
     return out, int(iters.value)
