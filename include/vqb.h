@@ -21,7 +21,10 @@
  *   - there is no CPU fallback: without a usable GPU vqb_ctx_create fails.
  *   - a context (and the quantizers made from it) may be used from several
  *     host threads, one call at a time per context (calls are serialised by an
- *     internal lock), matching the reference's `Send + Sync` plain-data types.
+ *     internal lock), matching the reference's `Send + Sync` plain-data types;
+ *   - a callback of a fit (below) may destroy quantizers of the same context (a
+ *     garbage collector may run there); every other call of that context from
+ *     inside it returns VQB_ERR_CALLBACK.
  */
 #ifndef VQB_H
 #define VQB_H

@@ -6,12 +6,12 @@
 #include <algorithm>
 #include <cstring>
 #include <memory>
-#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
 
 #include "../../include/vqb.h"
+#include "call_lock.hpp"
 #include "cuda_device.hpp"
 #include "opq_parts.hpp"
 #include "tsvq.hpp"
@@ -26,7 +26,7 @@ using namespace vqb;
 struct vqb_ctx {
     std::unique_ptr<CudaDevice> dev;
     std::unique_ptr<Comm> comm;
-    std::mutex mu;
+    CallLock lock;
     std::string err;
 };
 
@@ -99,6 +99,33 @@ template <typename F> int guarded(vqb_ctx *ctx, F &&f)
     } catch (...) {
         return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "unknown error");
     }
+}
+
+// One call of a context.
+template <typename F> int locked(vqb_ctx *ctx, F &&f)
+{
+    CallLock::Hold hold(ctx->lock);
+    if (!hold) return set_err(ctx, VQB_ERR_CALLBACK, "a callback may not call the context that is calling it");
+    return guarded(ctx, f);
+}
+
+// What a destroy function frees.  Inside a callback (a garbage collector may run there) only that happens: what the fit in
+// progress shares between its kernels stays, and so does its thread's current device.
+template <typename F> void destroyed(vqb_ctx *ctx, F &&f)
+{
+    int before = -1;
+    if (cudaGetDevice(&before) != cudaSuccess) before = -1;
+    CallLock::Hold hold(ctx->lock);
+    try {
+        if (hold) {
+            guarded(ctx, f);
+        } else {
+            ctx->dev->make_current();
+            f();
+        }
+    } catch (...) {
+    }
+    if (before >= 0 && before != ctx->dev->device()) cudaSetDevice(before);
 }
 
 bool metric_ok(int m) { return m >= 0 && m <= 6; }
@@ -281,7 +308,7 @@ OpqParts opq_parts(vqb_opq *oq)
 {
     OpqParts v;
     v.dev = oq->ctx->dev.get();
-    v.mu = &oq->ctx->mu;
+    v.lock = &oq->ctx->lock;
     v.err = &oq->ctx->err;
     v.rotation = oq->rotation_d;
     v.codebooks = oq->codebooks;
@@ -317,6 +344,7 @@ int vqb_ctx_create(int device, vqb_ctx **out)
 int vqb_ctx_destroy(vqb_ctx *ctx)
 {
     if (!ctx) return VQB_OK;
+    if (!CallLock::Hold(ctx->lock)) return set_err(ctx, VQB_ERR_CALLBACK, "a callback may not destroy the context that is calling it");
     try {
         ctx->dev->make_current();
         ctx->dev->synchronize();
@@ -332,24 +360,19 @@ const char *vqb_last_error(const vqb_ctx *ctx) { return ctx ? ctx->err.c_str() :
 int vqb_ctx_set_stream(vqb_ctx *ctx, void *cuda_stream)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    ctx->dev->set_stream(static_cast<cudaStream_t>(cuda_stream));
-    return VQB_OK;
+    return locked(ctx, [&] { ctx->dev->set_stream(static_cast<cudaStream_t>(cuda_stream)); });
 }
 
 int vqb_ctx_reset_stream(vqb_ctx *ctx)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    ctx->dev->reset_stream();
-    return VQB_OK;
+    return locked(ctx, [&] { ctx->dev->reset_stream(); });
 }
 
 int vqb_ctx_synchronize(vqb_ctx *ctx)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] { ctx->dev->synchronize(); });
+    return locked(ctx, [&] { ctx->dev->synchronize(); });
 }
 
 int vqb_ctx_launch_count(const vqb_ctx *ctx, uint64_t *out)
@@ -369,15 +392,13 @@ int vqb_ctx_alloc_count(const vqb_ctx *ctx, uint64_t *out)
 int vqb_ctx_timing(vqb_ctx *ctx, int enable)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] { ctx->dev->set_timing(enable != 0); });
+    return locked(ctx, [&] { ctx->dev->set_timing(enable != 0); });
 }
 
 int vqb_ctx_timing_report(vqb_ctx *ctx, char *buf, size_t cap)
 {
     if (!ctx || !buf || cap == 0) return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "NULL argument");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         std::string r = ctx->dev->timing_report();
         if (r.size() + 1 > cap) throw Error(VQB_ERR_BAD_ARGUMENT, "report buffer too small");
         std::memcpy(buf, r.c_str(), r.size() + 1);
@@ -394,8 +415,7 @@ int vqb_comm_init(vqb_ctx *ctx, const uint8_t *unique_id, int rank, int world)
 {
     if (!ctx || !unique_id) return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     if (world < 1 || rank < 0 || rank >= world) return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "rank/world out of range");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         ctx->comm.reset();
         ctx->comm.reset(make_nccl_comm(*ctx->dev, unique_id, rank, world));
     });
@@ -411,8 +431,7 @@ int vqb_comm_exchange_count(const vqb_ctx *ctx, uint64_t *out)
 int vqb_comm_destroy(vqb_ctx *ctx)
 {
     if (!ctx) return VQB_OK;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         ctx->dev->synchronize();
         ctx->comm.reset();
     });
@@ -422,8 +441,7 @@ int vqb_distance_rows(vqb_ctx *ctx, int metric, double p, const float *a, size_t
                       float *out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!metric_ok(metric)) throw Error(VQB_ERR_BAD_ARGUMENT, "unknown metric");
         if (da != db) throw Error(VQB_ERR_DIMENSION_MISMATCH, dim_mismatch(da, db)); // src/distances.rs:119-127
         check_minkowski(metric, p);
@@ -440,8 +458,7 @@ int vqb_distance_rows(vqb_ctx *ctx, int metric, double p, const float *a, size_t
 int vqb_tsvq_fit(vqb_ctx *ctx, const float *x, size_t n, size_t dim, size_t max_depth, int metric, double p, vqb_tsvq **out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!out) throw Error(VQB_ERR_BAD_ARGUMENT, "out is NULL");
         *out = nullptr;
         if (metric < 0 || metric > 6) throw Error(VQB_ERR_BAD_ARGUMENT, "unknown metric");
@@ -459,8 +476,7 @@ int vqb_tsvq_quantize(vqb_tsvq *t, const float *x, size_t n, size_t dim, uint16_
 {
     if (!t) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "tsvq is NULL");
     vqb_ctx *ctx = t->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (dim != t->tree.dim) throw Error(VQB_ERR_DIMENSION_MISMATCH, dim_mismatch(t->tree.dim, dim)); // src/tsvq.rs:232-240
         if (n == 0) return;
         if (!x) throw Error(VQB_ERR_BAD_ARGUMENT, "x is NULL");
@@ -485,8 +501,7 @@ int vqb_tsvq_tree(const vqb_tsvq *t, float *centroids_out, int32_t *left_out, in
 {
     if (!t) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "tsvq is NULL");
     vqb_ctx *ctx = t->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (centroids_out) {
             const size_t bytes = sizeof(float) * t->tree.nodes * t->tree.dim;
             if (ctx->dev->is_device_pointer(centroids_out)) ctx->dev->copy(centroids_out, t->tree.centroids, bytes);
@@ -501,8 +516,7 @@ int vqb_tsvq_destroy(vqb_tsvq *t)
 {
     if (!t) return VQB_OK;
     vqb_ctx *ctx = t->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    guarded(ctx, [&] { tsvq_release(*ctx->dev, t->tree); });
+    destroyed(ctx, [&] { tsvq_release(*ctx->dev, t->tree); });
     delete t;
     return VQB_OK;
 }
@@ -511,8 +525,7 @@ int vqb_evaluate_f16(vqb_ctx *ctx, const float *x, const uint16_t *q_f16, size_t
                      float *recall_out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!x || !q_f16 || !mse_out || !recall_out) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL argument");
         CudaDevice &dev = *ctx->dev;
         In ix(dev, x, sizeof(float) * n * dim), iq(dev, q_f16, sizeof(uint16_t) * n * dim);
@@ -524,8 +537,7 @@ int vqb_dense_dots(vqb_ctx *ctx, const float *x, size_t n, size_t dim, const flo
                    unsigned long long *stats_out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!x || !codebook || !stats_out || n == 0) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL or empty argument");
         CudaDevice &dev = *ctx->dev;
         In ix(dev, x, sizeof(float) * n * dim), ic(dev, codebook, sizeof(float) * k * dim);
@@ -539,8 +551,7 @@ int vqb_pq_tensor_scores(vqb_ctx *ctx, const float *x, size_t n, size_t m, const
                          uint32_t *codes_out, unsigned long long *marked_out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!x || !codebooks || !codes_out || !marked_out || n == 0) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL or empty argument");
         CudaDevice &dev = *ctx->dev;
         In ix(dev, x, sizeof(float) * n * m * 8), ic(dev, codebooks, sizeof(float) * m * k * 8);
@@ -554,8 +565,7 @@ int vqb_pq_tensor_scores(vqb_ctx *ctx, const float *x, size_t n, size_t m, const
 int vqb_opq_rotate_rows(vqb_ctx *ctx, const float *rot, size_t dim, const float *x, size_t n, float *y_out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!rot || !x || !y_out || n == 0 || dim == 0) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL or empty argument");
         CudaDevice &dev = *ctx->dev;
         In ir(dev, rot, sizeof(float) * dim * dim), ix(dev, x, sizeof(float) * n * dim);
@@ -569,8 +579,7 @@ int vqb_opq_rotate_rows(vqb_ctx *ctx, const float *rot, size_t dim, const float 
 int vqb_opq_cross_cov(vqb_ctx *ctx, const float *y, const float *x, size_t n, size_t dim, double *a_out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!y || !x || !a_out || n == 0 || dim == 0) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL or empty argument");
         CudaDevice &dev = *ctx->dev;
         In iy(dev, y, sizeof(float) * n * dim), ix(dev, x, sizeof(float) * n * dim);
@@ -585,8 +594,7 @@ int vqb_lbg_fit(vqb_ctx *ctx, const float *x, size_t n, size_t d, size_t k, size
                 vqb_draw_fn draw, void *user, int flags, float *centroids_out, size_t *iterations_out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         CudaDevice &dev = *ctx->dev;
         if (n && !x) throw Error(VQB_ERR_BAD_ARGUMENT, "x is NULL");
         In ix(dev, x, sizeof(float) * n * d);
@@ -620,8 +628,7 @@ int vqb_pq_fit(vqb_ctx *ctx, const float *x, size_t n, size_t dim, size_t m, siz
 {
     if (!ctx || !out) return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     *out = nullptr;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!metric_ok(metric)) throw Error(VQB_ERR_BAD_ARGUMENT, "unknown metric");
         const bool multi = ctx->comm && ctx->comm->world() > 1;
         if (n == 0 && !multi) // src/pq.rs:87-89
@@ -666,8 +673,7 @@ int vqb_pq_from_codebooks(vqb_ctx *ctx, const float *codebooks, size_t m, size_t
 {
     if (!ctx || !out) return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     *out = nullptr;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!metric_ok(metric)) throw Error(VQB_ERR_BAD_ARGUMENT, "unknown metric");
         if (!codebooks || m == 0 || k == 0 || sub_dim == 0) throw Error(VQB_ERR_BAD_ARGUMENT, "empty codebooks");
         CudaDevice &dev = *ctx->dev;
@@ -692,8 +698,7 @@ int vqb_pq_quantize(vqb_pq *pq, const float *x, size_t n, size_t dim, uint16_t *
 {
     if (!pq) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "pq is NULL");
     vqb_ctx *ctx = pq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         const size_t full = pq->m * pq->sd;
         if (dim != full) throw Error(VQB_ERR_DIMENSION_MISMATCH, dim_mismatch(full, dim)); // src/pq.rs:147-156
         check_minkowski(pq->metric, pq->p);
@@ -741,8 +746,7 @@ int vqb_pq_codebooks(const vqb_pq *pq, float *out)
 {
     if (!pq || !out) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     vqb_ctx *ctx = pq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         const size_t bytes = sizeof(float) * pq->m * pq->k * pq->sd;
         if (ctx->dev->is_device_pointer(out)) ctx->dev->copy(out, pq->codebooks, bytes);
         else ctx->dev->download(out, pq->codebooks, bytes);
@@ -760,8 +764,7 @@ int vqb_pq_destroy(vqb_pq *pq)
 {
     if (!pq) return VQB_OK;
     vqb_ctx *ctx = pq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    guarded(ctx, [&] { ctx->dev->release(pq->codebooks); });
+    destroyed(ctx, [&] { ctx->dev->release(pq->codebooks); });
     delete pq;
     return VQB_OK;
 }
@@ -774,8 +777,7 @@ int vqb_rvq_fit(vqb_ctx *ctx, const float *x, size_t n, size_t dim, size_t stage
 {
     if (!ctx || !out) return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     *out = nullptr;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!metric_ok(metric)) throw Error(VQB_ERR_BAD_ARGUMENT, "unknown metric");
         const bool multi = ctx->comm && ctx->comm->world() > 1;
         if (n == 0 && !multi) // src/rvq.rs:96-98
@@ -816,8 +818,7 @@ int vqb_rvq_from_codebooks(vqb_ctx *ctx, const float *codebooks, size_t stages, 
 {
     if (!ctx || !out) return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     *out = nullptr;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!metric_ok(metric)) throw Error(VQB_ERR_BAD_ARGUMENT, "unknown metric");
         if (dim == 0 || (stages > 0 && (k == 0 || !codebooks))) throw Error(VQB_ERR_BAD_ARGUMENT, "empty codebooks");
         CudaDevice &dev = *ctx->dev;
@@ -844,8 +845,7 @@ int vqb_rvq_quantize(vqb_rvq *rq, const float *x, size_t n, size_t dim, uint16_t
 {
     if (!rq) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "rvq is NULL");
     vqb_ctx *ctx = rq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (dim != rq->dim) throw Error(VQB_ERR_DIMENSION_MISMATCH, dim_mismatch(rq->dim, dim)); // src/rvq.rs:172-180
         if (rq->stages > 0 && rq->k >= 2) check_minkowski(rq->metric, rq->p);
         if (n == 0) return;
@@ -876,8 +876,7 @@ int vqb_rvq_codebooks(const vqb_rvq *rq, float *out)
 {
     if (!rq || !out) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     vqb_ctx *ctx = rq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         const size_t bytes = sizeof(float) * rq->stages * rq->k * rq->dim;
         if (ctx->dev->is_device_pointer(out)) ctx->dev->copy(out, rq->codebooks, bytes);
         else ctx->dev->download(out, rq->codebooks, bytes);
@@ -888,8 +887,7 @@ int vqb_rvq_destroy(vqb_rvq *rq)
 {
     if (!rq) return VQB_OK;
     vqb_ctx *ctx = rq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    guarded(ctx, [&] { ctx->dev->release(rq->codebooks); });
+    destroyed(ctx, [&] { ctx->dev->release(rq->codebooks); });
     delete rq;
     return VQB_OK;
 }
@@ -902,8 +900,7 @@ int vqb_opq_fit(vqb_ctx *ctx, const float *x, size_t n, size_t dim, size_t m, si
 {
     if (!ctx || !out) return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     *out = nullptr;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!metric_ok(metric)) throw Error(VQB_ERR_BAD_ARGUMENT, "unknown metric");
         const bool multi = ctx->comm && ctx->comm->world() > 1;
         if (n == 0 && !multi) // src/opq.rs:99-101
@@ -947,8 +944,7 @@ int vqb_opq_from_parts(vqb_ctx *ctx, const float *rotation, const float *codeboo
 {
     if (!ctx || !out) return set_err(ctx, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     *out = nullptr;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (!metric_ok(metric)) throw Error(VQB_ERR_BAD_ARGUMENT, "unknown metric");
         if (!rotation || !codebooks || m == 0 || k == 0 || sub_dim == 0) throw Error(VQB_ERR_BAD_ARGUMENT, "empty parts");
         CudaDevice &dev = *ctx->dev;
@@ -980,8 +976,7 @@ int vqb_opq_quantize(vqb_opq *oq, const float *x, size_t n, size_t dim, uint16_t
 {
     if (!oq) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "opq is NULL");
     vqb_ctx *ctx = oq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (dim != oq->dim) throw Error(VQB_ERR_DIMENSION_MISMATCH, dim_mismatch(oq->dim, dim)); // src/opq.rs:223-231
         if (oq->empty) return; // no codebooks: the reference returns an empty vector (src/opq.rs:244-263)
         check_minkowski(oq->metric, oq->p);
@@ -1022,8 +1017,7 @@ int vqb_opq_rotation(const vqb_opq *oq, float *out)
 {
     if (!oq || !out) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     vqb_ctx *ctx = oq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         const size_t bytes = sizeof(float) * oq->dim * oq->dim;
         if (ctx->dev->is_device_pointer(out)) ctx->dev->copy(out, oq->rotation_d, bytes);
         else std::memcpy(out, oq->rotation.data(), bytes);
@@ -1034,8 +1028,7 @@ int vqb_opq_codebooks(const vqb_opq *oq, float *out)
 {
     if (!oq || !out) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "NULL argument");
     vqb_ctx *ctx = oq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (oq->empty) return;
         const size_t bytes = sizeof(float) * oq->m * oq->k * oq->sd;
         if (ctx->dev->is_device_pointer(out)) ctx->dev->copy(out, oq->codebooks, bytes);
@@ -1047,8 +1040,7 @@ int vqb_opq_destroy(vqb_opq *oq)
 {
     if (!oq) return VQB_OK;
     vqb_ctx *ctx = oq->ctx;
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    guarded(ctx, [&] {
+    destroyed(ctx, [&] {
         ctx->dev->release(oq->codebooks);
         ctx->dev->release(oq->rotation_d);
     });
@@ -1071,8 +1063,7 @@ int vqb_sq_quantize(vqb_ctx *ctx, float min, float max, size_t levels, float ste
                     uint8_t *out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (levels < 2 || levels > 256) throw Error(VQB_ERR_INVALID_PARAMETER, "Invalid parameter: levels must be between 2 and 256");
         if (n_elems == 0) return;
         if (!x || !out) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL data pointer");
@@ -1106,8 +1097,7 @@ int vqb_bq_fit(float threshold, uint8_t low, uint8_t high)
 int vqb_bq_quantize(vqb_ctx *ctx, float threshold, uint8_t low, uint8_t high, const float *x, size_t n_elems, uint8_t *out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
-    std::lock_guard<std::mutex> lk(ctx->mu);
-    return guarded(ctx, [&] {
+    return locked(ctx, [&] {
         if (n_elems == 0) return;
         if (!x || !out) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL data pointer");
         CudaDevice &dev = *ctx->dev;

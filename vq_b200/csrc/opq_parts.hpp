@@ -1,8 +1,8 @@
 // opq_parts.hpp -- read-only view of a trained OPQ handle for translation units other than api.cpp.
 #pragma once
-#include <mutex>
 #include <string>
 
+#include "call_lock.hpp"
 #include "cuda_device.hpp"
 
 struct vqb_opq;
@@ -11,7 +11,7 @@ namespace vqb {
 
 struct OpqParts {
     CudaDevice *dev;
-    std::mutex *mu;
+    CallLock *lock;
     std::string *err;
     const float *rotation; // device, dim x dim row-major
     const float *codebooks; // device, m x k x sd

@@ -45,7 +45,11 @@ extern "C" int vqb_opq_quantize_static(vqb_opq *oq, const float *x, size_t n, si
 {
     if (!oq) return VQB_ERR_BAD_ARGUMENT;
     vqb::OpqParts P = vqb::opq_parts(oq);
-    std::lock_guard<std::mutex> lk(*P.mu);
+    vqb::CallLock::Hold hold(*P.lock);
+    if (!hold) {
+        *P.err = "a callback may not call the context that is calling it";
+        return VQB_ERR_CALLBACK;
+    }
     try {
         vqb::CudaDevice &dev = *P.dev;
         dev.make_current();
