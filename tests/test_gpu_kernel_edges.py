@@ -45,6 +45,45 @@ def test_direct_encode_bit_exact(oracle, name, n, m, sd, k):
     assert np.array_equal(out, out_o.view(np.float16), equal_nan=True)
 
 
+@pytest.mark.parametrize("m,sd,k,last", [(16, 8, 256, 686), (4, 8, 100, 4540), (8, 8, 33, 3371), (5, 4, 256, 11_200), (3, 8, 20, 6666), (4, 5, 100, 7000)])
+def test_encode_on_both_sides_of_the_line_between_the_kernels(oracle, ctx, m, sd, k, last):
+    """`last` rows are the most that one launch encodes, one more goes to the kernels for many rows (three launches where the tensor
+    cores take the shape): both give the oracle's codes."""
+    cb = synth.uniform(k, m * sd, 11 + k, -1.0, 1.0).reshape(k, m, sd).transpose(1, 0, 2).copy()
+    cb[:, k - 1] = cb[:, 1]
+    x = synth.uniform(last + 1, m * sd, 7, -1.0, 1.0)
+    x[5] = cb[:, 1].reshape(-1)
+    x[last // 2, 0] = np.nan
+    out_o, codes_o = oracle.pq_quantize(cb, x, METRICS["Euclidean"])
+    q = vq.ProductQuantizer.from_codebooks(cb, vq.Distance.Euclidean)
+    launches = []
+    for n in (last, last + 1):
+        before = ctx.launch_count()
+        out, codes = q.quantize(x[:n], return_codes=True)
+        launches.append(ctx.launch_count() - before)
+        assert np.array_equal(codes, codes_o[:n])
+        assert np.array_equal(out, out_o[:n].view(np.float16), equal_nan=True)
+    assert launches[0] == 1 and (launches[1] == 3 if sd == 8 and m % 4 == 0 else launches[1] >= 1)
+
+
+@pytest.mark.parametrize("dim,k,last", [(128, 256, 12_500), (61, 256, 12_499), (33, 90, 34_500), (24, 5, 106_250)])
+def test_residual_encode_on_both_sides_of_the_line_between_the_kernels(oracle, ctx, dim, k, last):
+    """As above: one launch for all stages, or several per stage."""
+    x = synth.gaussian_mixture(last + 1, dim, 5)
+    books = 0.2 * synth.normal(2 * k, dim, 3).reshape(2, k, dim)
+    books[0, 0], books[1, k - 1] = x[0], books[1, k // 2]
+    out_o, codes_o, _ = oracle.rvq_quantize(books, 0.01, x, METRICS["Euclidean"])
+    q = vq.ResidualQuantizer.from_codebooks(books, 0.01, vq.Distance.Euclidean)
+    launches = []
+    for n in (last, last + 1):
+        before = ctx.launch_count()
+        out, codes = q.quantize(x[:n], return_codes=True)
+        launches.append(ctx.launch_count() - before)
+        assert np.array_equal(codes, codes_o[:n])
+        assert np.array_equal(out, out_o[:n].view(np.float16), equal_nan=True)
+    assert launches[0] == 1 < launches[1]
+
+
 @pytest.mark.parametrize("name", ["SquaredEuclidean", "Euclidean", "CosineDistance", "Manhattan"])
 @pytest.mark.parametrize("n,dim,k,stages", [(1, 128, 256, 8), (17, 33, 64, 3), (40, 15, 7, 2), (700, 64, 130, 4)])
 def test_direct_residual_encode_bit_exact(oracle, name, n, dim, k, stages):

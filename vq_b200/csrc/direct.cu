@@ -459,15 +459,23 @@ static void launch_any(CudaDevice &dev, DirectParams &p, int metric, int m)
     }
 }
 
-// Measured (us, 2000 .. 64,000 rows of 5 .. 32 sub-spaces): this kernel takes about 0.35 + 0.003 k ns per (row, sub-space).  The
-// tensor-core kernel for 8-wide sub-spaces takes 21 us (k = 256) and 16 us (k = 20) up to some thousand rows, three launches
-// of which the rows are the smaller part; the CUDA-core kernels take 57 - 121 us (k = 256) and 10 - 23 us (k = 20 .. 40) until
-// their grids are full, which is a few thousand rows later.
+// Where the other kernels take over.  A thread looks at two centroids whatever k is, so this kernel's time follows (row, sub-space)
+// pairs and 2 tk = 64, 128 or 256.  Measured with rows on the GPU, from the call to its result and as one of many in a row (the
+// two agree within a few per cent):
+//   the tensor-core kernel (8-wide sub-spaces; 19 us in three launches as one of many, hardly dependent on the rows) passes at
+//       k 256: 10,900 .. 11,100 pairs (m 4, 8, 16, 32), k 200: 10,750, k 128: 15,900 .. 20,000, k 20, 40, 64: 27,100 .. 27,400
+//   the CUDA-core kernels (19 us up to k 20, 33 at 64, 40 .. 46 at 128, 66 .. 83 at 256, until their grids are full, some thousand
+//       rows later) pass at  k 256: 57,800 .. 64,400 pairs (4- and 16-wide), 68,600 (8-wide), 78,900 (Manhattan), k 128: 67,000,
+//       k 64: 63,700 (cosine), 70,000 (24-wide), k 48: 48,000, k 40: 28,000 (cosine), k 32: 32,000, k 2 .. 20: 16,000 (16-wide) .. 30,000,
+//       and k 100 of 5 values, which are no whole 16-byte pieces: 29,000
+static bool whole_pieces(int sd, const float *centroids) { return sd % 4 == 0 && (reinterpret_cast<uintptr_t>(centroids) & 15u) == 0; }
+
 bool direct_encode_applicable(const AssignParams &p, bool tensor)
 {
     if (p.k > DK_MAX || p.sd > 256 || p.m > 65535) return false;
-    const double us = 1e-3 * (double)p.n * p.m * (0.35 + 0.003 * p.k);
-    return us <= (tensor ? 10.0 : 0.25 * p.k);
+    const double pairs = (double)p.n * p.m;
+    if (tensor) return pairs * (2 * direct_tk(p.k) + 68) <= 3.56e6;
+    return pairs <= (p.k < 48 ? 20e3 : 56e3) * (whole_pieces(p.sd, p.centroids) ? 1.0 : 0.5);
 }
 
 void launch_direct_encode(CudaDevice &dev, const AssignParams &a, int metric)
@@ -476,7 +484,7 @@ void launch_direct_encode(CudaDevice &dev, const AssignParams &a, int metric)
     p.x = a.x, p.n = a.n, p.ld = a.ld, p.m = a.m, p.k = a.k, p.sd = a.sd, p.tk = direct_tk(a.k);
     p.centroids = a.centroids;
     p.out_f16 = a.out_f16, p.out_codes = a.out_codes, p.out_f32 = a.out_f32, p.pv = a.pv;
-    p.vec4 = a.sd % 4 == 0 && (reinterpret_cast<uintptr_t>(a.centroids) & 15u) == 0;
+    p.vec4 = whole_pieces(a.sd, a.centroids);
     launch_any(dev, p, metric, a.m);
 }
 
@@ -484,9 +492,14 @@ bool direct_rvq_applicable(const GenericParams &g, bool tensor, size_t smem_limi
 {
     if (g.k > DK_MAX || std::max(direct_smem(8, direct_tk(g.k), g.sd, true), direct_smem(1, direct_tk(g.k), g.sd, true)) > smem_limit - STATIC_SMEM) return false;
     // Against the CUDA-core kernel this one is ahead at every size that was measured (Manhattan, 80,000 x 128, k 256, 8 stages:
-    // 7.2 -> 2.8 ms; cosine: 10.1 -> 2.4 ms).  The tensor-core path takes about 45 us a stage up to 20,000 rows (five launches);
-    // the two meet at 12,000 rows of 128 (k 256), 50,000 of 128 (k 60), 12,000 of 61 (k 256), 80,000 of 40 (k 20).
-    return !tensor || (double)g.n * (g.k + 64) * (g.sd + 32) <= 4.5e8;
+    // 7.2 -> 2.8 ms; cosine: 10.1 -> 2.4 ms).  The tensor-core path takes about 45 us a stage up to 20,000 rows (five launches), of
+    // which little depends on the rows' width or on k; the two meet at these rows (8 stages; 2 stages within 6 %):
+    //   2 tk 256:  12,700 of 128, 16,600 of 96, 22,400 of 64, 31,700 of 32, 12,300 of 61 (no whole 16-byte pieces: no TMA)
+    //   2 tk 128:  29,900 of 128, 34,400 of 61          2 tk 64:  46,400 of 128, 107,000 of 40, 115,000 of 32, 97,000 of 24
+    if (!tensor) return true;
+    const int tk = direct_tk(g.k), dc = chunk_dims(g.sd), width = (g.sd + dc - 1) / dc * dc;
+    const double rows = (tk == 128 ? 2.0e6 : tk == 64 ? 4.6e6 : 6.8e6) / (width + 32);
+    return (double)g.n <= (whole_pieces(g.sd, g.centroids) ? rows : 0.6 * rows);
 }
 
 void launch_direct_rvq(CudaDevice &dev, const GenericParams &g, int metric)
@@ -495,7 +508,7 @@ void launch_direct_rvq(CudaDevice &dev, const GenericParams &g, int metric)
     p.x = g.x, p.n = g.n, p.ld = g.ld, p.m = 1, p.k = g.k, p.sd = g.sd, p.tk = direct_tk(g.k);
     p.centroids = g.centroids;
     p.out_f16 = g.out_f16, p.out_codes = g.out_codes, p.pv = g.pv, p.epsilon = g.epsilon, p.stages = g.stages;
-    p.vec4 = g.sd % 4 == 0 && (reinterpret_cast<uintptr_t>(g.centroids) & 15u) == 0;
+    p.vec4 = whole_pieces(g.sd, g.centroids);
     launch_any(dev, p, metric, 1);
 }
 
