@@ -79,11 +79,11 @@ int set_err(vqb_ctx *ctx, int code, const std::string &msg)
 
 template <typename F> int guarded(vqb_ctx *ctx, F &&f)
 {
-    struct AtEnd { // what the kernels of one call share goes back to the pool with it
+    struct AtEnd {
         vqb_ctx *ctx;
         ~AtEnd()
         {
-            if (ctx) ctx->dev->release_dense();
+            if (ctx) ctx->dev->end_call();
         }
     } at_end{ctx};
     try {

@@ -42,6 +42,7 @@ CudaDevice::CudaDevice(int device) : device_(device)
     smem_limit_ = prop.sharedMemPerBlockOptin;
     VQB_CUDA_CHECK(cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking));
     stream_ = own_stream_;
+    VQB_CUDA_CHECK(cudaEventCreateWithFlags(&order_event_, cudaEventDisableTiming));
     ++device_allocs_;
     if (cudaHostAlloc(reinterpret_cast<void **>(&stage_), STAGE_BYTES, cudaHostAllocMapped) != cudaSuccess) {
         stage_ = nullptr; // pinned memory is an optimisation only
@@ -82,6 +83,7 @@ CudaDevice::~CudaDevice()
         for (int i = 0; i < 2; ++i)
             if (aux_[i]) cudaStreamDestroy(aux_[i]);
         if (stage_event_) cudaEventDestroy(stage_event_);
+        if (order_event_) cudaEventDestroy(order_event_);
         for (cudaEvent_t e : arrival_done_) cudaEventDestroy(e);
         if (arrival_fence_) cudaEventDestroy(arrival_fence_);
         if (stage_) cudaFreeHost(stage_);
@@ -164,6 +166,43 @@ std::string CudaDevice::timing_report()
     return out + "}";
 }
 
+// A stream that is being captured into a graph takes no part in the order of calls: an event from outside may not be waited for
+// there, and one from inside not outside.  (The query fails for the default stream while another one is being captured.)
+static bool captured(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
+// The scratch of the tensor-core kernels, the map of marked pairs and the memory of a quantizer that is being destroyed are the
+// context's, whatever stream a call runs on.  The caller may destroy a stream of its own as soon as its work is done, so
+// such a stream gets the event while the call is still there (end_call); the context's own and the default stream get it here,
+// so that programs that never change streams pay nothing.
+void CudaDevice::set_stream(cudaStream_t s)
+{
+    const cudaStream_t old = stream_;
+    if (s == old) return;
+    stream_ = s;
+    if (!unfinished_ || captured(s)) return;
+    if (lasting(old)) {
+        if (captured(old)) return;
+        VQB_CUDA_CHECK(cudaEventRecord(order_event_, old));
+    }
+    VQB_CUDA_CHECK(cudaStreamWaitEvent(s, order_event_, 0));
+}
+
+bool CudaDevice::lasting(cudaStream_t s) const { return s == own_stream_ || s == nullptr || s == cudaStreamLegacy; }
+
+void CudaDevice::end_call()
+{
+    release_dense();
+    if (!unfinished_ || lasting(stream_)) return;
+    if (captured(stream_)) unfinished_ = false;
+    else cudaEventRecord(order_event_, stream_);
+}
+
 cudaStream_t CudaDevice::aux_stream(int i)
 {
     if (!aux_[i]) VQB_CUDA_CHECK(cudaStreamCreateWithFlags(&aux_[i], cudaStreamNonBlocking));
@@ -178,6 +217,7 @@ void CudaDevice::synchronize()
 {
     if (tc_error_) check_tc_error();
     else VQB_CUDA_CHECK(cudaStreamSynchronize(stream_));
+    unfinished_ = false;
 }
 
 bool CudaDevice::is_device_pointer(const void *p) const
@@ -326,6 +366,7 @@ void CudaDevice::download(void *dst, const void *src, size_t bytes, void *dst2, 
         while ((q = cudaEventQuery(stage_event_)) == cudaErrorNotReady) {
         }
         VQB_CUDA_CHECK(q);
+        unfinished_ = false;
         if (bytes) std::memcpy(dst, stage_ + 16, bytes);
         if (bytes2) std::memcpy(dst2, second, bytes2);
         if (tc_error_) {
@@ -340,6 +381,7 @@ void CudaDevice::download(void *dst, const void *src, size_t bytes, void *dst2, 
     if (bytes) VQB_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, stream_));
     if (bytes2) VQB_CUDA_CHECK(cudaMemcpyAsync(dst2, src2, bytes2, cudaMemcpyDeviceToHost, stream_));
     VQB_CUDA_CHECK(cudaStreamSynchronize(stream_));
+    unfinished_ = false;
     check_tc_error();
 }
 
@@ -357,6 +399,7 @@ void CudaDevice::ensure_tc_buffers()
     VQB_CUDA_CHECK(cudaMemsetAsync(tc_stats_, 0, 3 * sizeof(unsigned long long), stream_));
     VQB_CUDA_CHECK(cudaMalloc(&tc_error_, sizeof(int)));
     VQB_CUDA_CHECK(cudaMemsetAsync(tc_error_, 0, sizeof(int), stream_));
+    unfinished_ = true; // the first call may come on another stream
 }
 
 // One block for everything the full-width tensor path needs besides rows and codebooks; it lives until the end of the call
@@ -490,12 +533,14 @@ void CudaDevice::copy(void *dst, const void *src, size_t bytes)
 {
     if (!bytes) return;
     VQB_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, stream_));
+    unfinished_ = true;
 }
 
 void CudaDevice::zero(void *dst, size_t bytes)
 {
     if (!bytes) return;
     VQB_CUDA_CHECK(cudaMemsetAsync(dst, 0, bytes, stream_));
+    unfinished_ = true;
 }
 
 static inline unsigned blocks_for(size_t items, int threads, size_t cap = 1u << 20)

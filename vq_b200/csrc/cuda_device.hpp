@@ -87,17 +87,17 @@ class CudaDevice : public Device {
 
     // Two helper streams for overlapping host<->device copies with kernels (created on first use).
     cudaStream_t aux_stream(int i);
-    void set_stream(cudaStream_t s) { stream_ = s; } // nullptr = the CUDA default stream
-    void reset_stream() { stream_ = own_stream_; }
+    void set_stream(cudaStream_t s); // nullptr = the CUDA default stream
+    void reset_stream() { set_stream(own_stream_); }
     cudaStream_t stream() const { return stream_; }
     void synchronize();
     int device() const { return device_; }
     int sm_count() const { return sm_count_; }
     size_t smem_limit() const { return smem_limit_; }
-    void release_dense(); // at the end of every call of the C ABI
+    void end_call(); // at the end of every call of the C ABI
     int *error_word() const { return tc_error_; } // null with VQB_NO_TENSOR=1
     uint64_t launches() const { return launches_.load(); }
-    void count_launch(uint64_t n = 1) { launches_ += n; }
+    void count_launch(uint64_t n = 1) { launches_ += n, unfinished_ = true; }
     // How often this context has asked CUDA for device or pinned memory (cudaMalloc, cudaMallocAsync, cudaHostAlloc).
     uint64_t device_allocs() const { return device_allocs_.load(); }
     void make_current() const;
@@ -118,6 +118,11 @@ class CudaDevice : public Device {
     int sm_count_ = 148;
     size_t smem_limit_ = 0;
     cudaStream_t own_stream_ = nullptr, stream_ = nullptr, aux_[2] = {nullptr, nullptr};
+    // A call may leave work behind on its stream that uses the context's scratch, and the next call may run on another one: set_stream
+    // puts that one behind order_event_.
+    bool unfinished_ = false; // nothing has waited for stream_ since the last launch or copy
+    cudaEvent_t order_event_ = nullptr;
+    bool lasting(cudaStream_t s) const;
     static constexpr size_t STAGE_BYTES = 1u << 20; // pinned staging for small downloads
     unsigned char *stage_ = nullptr, *stage_dev_ = nullptr; // stage_dev_: the same bytes as kernels on this GPU address them
     cudaEvent_t stage_event_ = nullptr;
@@ -139,6 +144,7 @@ class CudaDevice : public Device {
     void *dense_block_ = nullptr;
     size_t dense_rows_ = 0, dense_dimp_ = 0;
     const DenseWork &dense_work(size_t n, size_t dim);
+    void release_dense();
     void dense_decide(const float *x, size_t n, size_t dim, const float *codebook, size_t k, bool euclid, uint8_t *codes, uint32_t *changed,
                       unsigned long long *stats);
     float *pq_scratch_ = nullptr;
