@@ -727,8 +727,9 @@ int vqb_pq_quantize(vqb_pq *pq, const float *x, size_t n, size_t dim, uint16_t *
             return;
         }
         Out of(dev, out_f16, sizeof(uint16_t) * n * dim), oc(dev, codes, sizeof(uint32_t) * n * pq->m);
-        In ix(dev, x, sizeof(float) * n * dim, [&](const void *rows) { dev.pq_encode_ahead(sh, (const float *)rows, pq->codebooks, pq->metric, of.as<uint16_t>()); });
-        dev.pq_encode(sh, ix.as<float>(), pq->codebooks, pq->metric, pq->p, of.as<uint16_t>(), oc.as<uint32_t>(), nullptr);
+        bool ahead = false;
+        In ix(dev, x, sizeof(float) * n * dim, [&](const void *rows) { ahead = dev.pq_encode_ahead(sh, (const float *)rows, pq->codebooks, pq->metric, of.as<uint16_t>()); });
+        dev.pq_encode_prepared(sh, ix.as<float>(), pq->codebooks, pq->metric, pq->p, of.as<uint16_t>(), oc.as<uint32_t>(), ahead);
         finish(of, oc);
     });
 }

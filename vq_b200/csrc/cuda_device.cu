@@ -198,6 +198,7 @@ bool CudaDevice::lasting(cudaStream_t s) const { return s == own_stream_ || s ==
 void CudaDevice::end_call()
 {
     release_dense();
+    bop_fresh_ = nullptr; // the next call's centroids may have the same address
     if (!unfinished_ || lasting(stream_)) return;
     if (captured(stream_)) unfinished_ = false;
     else cudaEventRecord(order_event_, stream_);
@@ -665,12 +666,11 @@ void CudaDevice::assign_train(const Shape &sh, const float *x, const float *cent
     p.changed = changed;
     p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
     if (pq_tensor_enabled_ && pq_tc_applicable(p, M_SQ)) {
-            PqTcBuffers tb;
+        PqTcBuffers tb;
         tb.scratch = pq_scratch_;
         tb.marks = pq_mark_buffer(pq_tc_mark_bytes(sh.n_local, sh.m));
         tb.error_word = tc_error_;
         tb.prepare_operand = (bop_fresh_ != centroids);
-        encode_operand_ = nullptr; // an announced encode that did not come about
         launch_pq_tc(*this, p, M_SQ, true, code_bytes(sh.k), tb);
         bop_fresh_ = nullptr;
         return;
@@ -691,9 +691,8 @@ void CudaDevice::assign_train(const Shape &sh, const float *x, const float *cent
     return;
 }
 
-void CudaDevice::pq_encode_ahead(const Shape &sh, const float *x, const float *codebooks, int metric, const uint16_t *out_f16)
+bool CudaDevice::pq_encode_ahead(const Shape &sh, const float *x, const float *codebooks, int metric, const uint16_t *out_f16)
 {
-    encode_operand_ = nullptr;
     AssignParams p = {};
     p.x = x;
     p.n = sh.n_local;
@@ -704,17 +703,15 @@ void CudaDevice::pq_encode_ahead(const Shape &sh, const float *x, const float *c
     p.centroids = codebooks;
     p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
     p.out_vec = !out_f16 || (aligned16(out_f16) && sh.m * sh.sd % 8 == 0);
-    if (sh.n_local == 0 || !pq_tensor_enabled_ || !pq_tc_applicable(p, metric) || direct_encode_applicable(p, true)) return;
+    if (sh.n_local == 0 || !pq_tensor_enabled_ || !pq_tc_applicable(p, metric) || direct_encode_applicable(p, true)) return false;
     bop_fresh_ = nullptr;
     launch_pq_operand_b(*this, codebooks, p.m, p.k, metric == M_COSINE, pq_scratch_);
-    encode_operand_ = codebooks;
+    return true;
 }
 
 void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *codebooks, int metric, double pm,
-                                uint16_t *out_f16, uint32_t *out_codes, float *out_f32, bool cuda_cores_only)
+                                uint16_t *out_f16, uint32_t *out_codes, float *out_f32, bool cuda_cores_only, bool operand_there)
 {
-    const float *ahead = encode_operand_;
-    encode_operand_ = nullptr;
     if (sh.n_local == 0) return;
     const size_t dim = sh.m * sh.sd;
     AssignParams p = {};
@@ -739,7 +736,7 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
     if (tensor) {
         bop_fresh_ = nullptr;
         PqTcBuffers tb;
-        tb.prepare_operand = ahead != codebooks;
+        tb.prepare_operand = !operand_there;
         tb.scratch = pq_scratch_;
         tb.marks = pq_mark_buffer(pq_tc_mark_bytes(sh.n_local, sh.m));
         tb.error_word = tc_error_;
@@ -765,13 +762,19 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
 void CudaDevice::pq_encode(const Shape &sh, const float *x, const float *codebooks, int metric, double pm, uint16_t *out_f16,
                            uint32_t *out_codes, float *out_f32)
 {
-    pq_encode_impl(sh, x, codebooks, metric, pm, out_f16, out_codes, out_f32, false);
+    pq_encode_impl(sh, x, codebooks, metric, pm, out_f16, out_codes, out_f32, false, false);
+}
+
+void CudaDevice::pq_encode_prepared(const Shape &sh, const float *x, const float *codebooks, int metric, double pm, uint16_t *out_f16,
+                                    uint32_t *out_codes, bool operand_there)
+{
+    pq_encode_impl(sh, x, codebooks, metric, pm, out_f16, out_codes, nullptr, false, operand_there);
 }
 
 void CudaDevice::pq_encode_no_scratch(const Shape &sh, const float *x, const float *codebooks, int metric, double pm, uint16_t *out_f16,
                                       uint32_t *out_codes)
 {
-    pq_encode_impl(sh, x, codebooks, metric, pm, out_f16, out_codes, nullptr, true);
+    pq_encode_impl(sh, x, codebooks, metric, pm, out_f16, out_codes, nullptr, true, false);
 }
 
 void CudaDevice::rvq_update(float *res, size_t n, size_t dim, const float *centroids, size_t k, int metric, double pm,

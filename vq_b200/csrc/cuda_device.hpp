@@ -32,9 +32,9 @@ class CudaDevice : public Device {
     void download(void *dst, const void *src, size_t bytes) override;
     // two of them with one wait (either may be empty)
     void download(void *dst, const void *src, size_t bytes, void *dst2, const void *src2, size_t bytes2);
-    // The codebooks' operand of the next pq_encode, which has to have the same arguments: called before its rows are copied in, so
-    // that it is laid out meanwhile.
-    void pq_encode_ahead(const Shape &sh, const float *x, const float *codebooks, int metric, const uint16_t *out_f16);
+    // The codebooks' operand of an encode with the same arguments, laid out before its rows are copied in; what it returns is the
+    // operand_there of pq_encode_prepared.
+    bool pq_encode_ahead(const Shape &sh, const float *x, const float *codebooks, int metric, const uint16_t *out_f16);
     void copy(void *dst, const void *src, size_t bytes) override;
     void zero(void *dst, size_t bytes) override;
     size_t code_bytes(size_t k) const override { return k <= 256 ? 1 : (k <= 65536 ? 2 : 4); }
@@ -66,6 +66,8 @@ class CudaDevice : public Device {
                     double *norm_sum) override;
     void pq_encode(const Shape &sh, const float *x, const float *codebooks, int metric, double p, uint16_t *out_f16,
                    uint32_t *out_codes, float *out_f32) override;
+    void pq_encode_prepared(const Shape &sh, const float *x, const float *codebooks, int metric, double p, uint16_t *out_f16,
+                            uint32_t *out_codes, bool operand_there);
     // The same encode on the CUDA-core kernels only: they work out of shared memory and registers and need no device
     // memory besides inputs and outputs.  Results are identical to pq_encode.
     void pq_encode_no_scratch(const Shape &sh, const float *x, const float *codebooks, int metric, double p, uint16_t *out_f16,
@@ -156,9 +158,8 @@ class CudaDevice : public Device {
     unsigned long long *tc_stats_ = nullptr;
     int *tc_error_ = nullptr;
     void ensure_tc_buffers();
-    const float *encode_operand_ = nullptr; // codebooks whose operand pq_encode_ahead has laid out
     void pq_encode_impl(const Shape &sh, const float *x, const float *codebooks, int metric, double p, uint16_t *out_f16,
-                        uint32_t *out_codes, float *out_f32, bool cuda_cores_only);
+                        uint32_t *out_codes, float *out_f32, bool cuda_cores_only, bool operand_there);
 
     void check_tc_error();
     // rows on their way from a host buffer (begin_arrival): piece i is complete when arrival_done_[i] has fired
