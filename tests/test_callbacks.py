@@ -8,9 +8,11 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
-def test_lock_of_a_context_knows_its_holder(tmp_path):
-    exe = os.path.join(str(tmp_path), "test_call_lock")
-    subprocess.check_call(["/usr/bin/g++", "-std=c++17", "-O1", "-Wall", "-pthread", "-o", exe, os.path.join(ROOT, "tests", "cpp", "test_call_lock.cpp")])
+@pytest.mark.parametrize("name", ["test_call_lock", "test_host_wait"])
+def test_host_side_waits(tmp_path, name):
+    """The lock of a context knows its holder; the host's wait for a result has an end and says what it waited for."""
+    exe = os.path.join(str(tmp_path), name)
+    subprocess.check_call(["/usr/bin/g++", "-std=c++17", "-O1", "-Wall", "-pthread", "-o", exe, os.path.join(ROOT, "tests", "cpp", name + ".cpp")])
     res = subprocess.run([exe], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, timeout=60)
     assert res.returncode == 0, res.stdout.decode()
 

@@ -15,6 +15,7 @@
 #include "assign_reg.cuh"
 #include "dense_tc.hpp"
 #include "direct.cuh"
+#include "host_wait.hpp"
 #include "opq_tc.hpp"
 #include "ordered_sums.cuh"
 #include "queue_sums.cuh"
@@ -363,9 +364,9 @@ void CudaDevice::download(void *dst, const void *src, size_t bytes, void *dst2, 
         if (bytes2) VQB_CUDA_CHECK(cudaMemcpyAsync(second, src2, bytes2, cudaMemcpyDeviceToHost, stream_));
         if (tc_error_) VQB_CUDA_CHECK(cudaMemcpyAsync(stage_, tc_error_, sizeof(int), cudaMemcpyDeviceToHost, stream_));
         VQB_CUDA_CHECK(cudaEventRecord(stage_event_, stream_));
-        cudaError_t q;
-        while ((q = cudaEventQuery(stage_event_)) == cudaErrorNotReady) {
-        }
+        cudaError_t q = cudaSuccess;
+        wait_until([&] { return (q = cudaEventQuery(stage_event_)) != cudaErrorNotReady; },
+                   [&] { return std::to_string(bytes + bytes2) + " bytes from the GPU, behind kernel " + last_kernel_; });
         VQB_CUDA_CHECK(q);
         unfinished_ = false;
         if (bytes) std::memcpy(dst, stage_ + 16, bytes);
@@ -1588,7 +1589,7 @@ void CudaDevice::wait_status(const StatusPage &sp, size_t m, size_t k, IterStatu
                 throw Error(100, "centroid update finished without reporting its status");
             }
             if (std::chrono::steady_clock::now() - t0 > std::chrono::seconds(120))
-                throw Error(100, "timed out waiting for the centroid update's status");
+                throw Error(100, std::string("timed out waiting for the centroid update's status, behind kernel ") + last_kernel_);
         }
     }
     std::atomic_thread_fence(std::memory_order_acquire);

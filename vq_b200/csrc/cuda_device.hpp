@@ -106,6 +106,7 @@ class CudaDevice : public Device {
     // Optional per-kernel timing with CUDA events on the launching stream (off by default).
     void set_timing(bool on);
     bool timing() const { return timing_; }
+    void note_kernel(const char *name) { last_kernel_ = name; }
     void timing_begin(const char *name);
     void timing_end();
     // {"name": {"launches": L, "ms": T}, ...}; clears the record.
@@ -170,6 +171,7 @@ class CudaDevice : public Device {
     std::vector<cudaEvent_t> arrival_done_; // created once, re-used
     cudaEvent_t arrival_fence_ = nullptr;
     bool timing_ = false;
+    const char *last_kernel_ = "(none)"; // for the message of a wait that was given up
     struct Span {
         const char *name;
         cudaEvent_t a, b;
@@ -184,6 +186,7 @@ struct KernelScope {
     CudaDevice &dev;
     KernelScope(CudaDevice &d, const char *name) : dev(d)
     {
+        dev.note_kernel(name);
         if (dev.timing()) dev.timing_begin(name);
     }
     ~KernelScope()
