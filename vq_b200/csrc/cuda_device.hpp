@@ -145,11 +145,13 @@ class CudaDevice : public Device {
     bool prepared_by_apply_ = false; // by rvq_update, for the k-means of the next stage
     DenseWork dense_;
     void *dense_block_ = nullptr;
-    size_t dense_rows_ = 0, dense_dimp_ = 0;
-    const DenseWork &dense_work(size_t n, size_t dim);
+    size_t dense_rows_ = 0, dense_for_ = 0, dense_dimp_ = 0; // rows it has room for, rows it was asked for
+    // At most n rows at a time (dense_rows_; a multiple of 128 when fewer); `beside`: bytes a row that the caller allocates next.
+    const DenseWork &dense_work(size_t n, size_t dim, size_t beside);
     void release_dense();
     void dense_decide(const float *x, size_t n, size_t dim, const float *codebook, size_t k, bool euclid, uint8_t *codes, uint32_t *changed,
                       unsigned long long *stats);
+    void *try_alloc(size_t bytes); // null when there is no room
     float *pq_scratch_ = nullptr;
     float *rot_split_ = nullptr; // TF32 high and low parts of the rotation matrix of the current rotate_rows call (dim <= 128)
     bool opq_tensor_enabled_ = true;
