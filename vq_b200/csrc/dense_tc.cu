@@ -14,8 +14,9 @@
 // bytes as the row itself), and three products are added up: h.ch + h.cl + l.ch.  With one TF32 product (bound 2.1e-3 |x||c|)
 // between 15 and 94 % of the rows of a Gaussian mixture went to the exact kernel, which then took 0.31 ms per pass over
 // 1M x 128 rows beside 0.13 ms for the shortlist; bf16 instead of binary16 (bound 5.5e-5) still left 50 % in the first stage.
-// Three products take 1.4 times as many MMAs, 24 per tile, which hide behind the row traffic.  The images are written where
-// the rows are touched anyway (dense_prepare_kernel, rvq_apply_kernel); any width up to 128 is padded to whole K steps there.
+// Three products take 24 MMAs per tile of 128 dimensions and bound the kernel together with the epilogue: 0.148 ms per pass over
+// 1M x 128 (0.84 of the measured bf16 rate) beside 0.079 ms of row traffic.  The images are written where the rows are touched
+// anyway (dense_prepare_kernel, rvq_apply_kernel); any width up to 128 is padded to whole K steps there.
 //
 // Bound, in the frame.  |l.cl| + |e.c| + |v.ec| <= 3.01 * 2^-22 sum|v_i c_ji| (l below binary16's normal range: 2^-25 absolute
 // instead, <= 2^-25 sqrt(dim) (|v| + |c|)); 25 accumulation steps, each at most 2^-22:

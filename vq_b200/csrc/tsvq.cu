@@ -142,13 +142,13 @@ __global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *
     if (live) spread[in_level * dim + d] = var;
 }
 
-// ---- spreads of large nodes.  The sum
-// stays one serial f32 chain per (node, dimension) in data order -- a dependent addition every 5.8 cycles at best -- so the
-// kernel's job is to keep that chain fed: one CTA per (node, 32 dimensions); warp 0 is the consumer (lane = dimension) and
-// does nothing but read stages from shared memory and add; eleven producer warps gather the node's rows (128-bit loads where
-// rows are whole 16-byte pieces (VEC), else four 32-bit ones, which still meet the chain's pace; 64 rows per warp in flight, the next stage's row numbers requested meanwhile), form (v - c)^2 with each term rounded like the
-// reference's (src/tsvq.rs:86-98) and store that into a ring of 64-row stages, so the consumer's work per row is a
-// quarter of a shared-memory load and one addition.
+// ---- spreads of large nodes.  The sum stays one serial f32 chain per (node, dimension) in data order -- a dependent addition every
+// 4.1 cycles at best, 5.0 here (root of 100,000 x 128: 258 us) -- so the kernel's job is to keep that chain fed: one CTA per
+// (node, 32 dimensions); warp 0 is the consumer (lane = dimension, alone on its scheduler) and does nothing but read stages from
+// shared memory and add; twelve producer warps on the other three schedulers gather the node's rows (128-bit loads where rows are
+// whole 16-byte pieces (VEC), else four 32-bit ones, which still meet the chain's pace; 64 rows per warp in flight, the next
+// stage's row numbers requested meanwhile), form (v - c)^2 with each term rounded like the reference's (src/tsvq.rs:86-98) and
+// store that into a ring of 64-row stages, so the consumer's work per row is a quarter of a shared-memory load and one addition.
 //
 // A stage is stored dimension-major, [32 dimensions][64 rows], so that the consumer fetches four consecutive rows of its
 // dimension with one 128-bit load; the 16 four-row groups of a dimension are permuted by ns_swizzle(d), which keeps both
@@ -797,7 +797,7 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
     cudaStream_t st = dev.stream();
     const size_t cap_nodes = std::min<size_t>(max_depth < 40 ? ((size_t)2 << max_depth) - 1 : 2 * n, 2 * n);
     // A level's nodes are "small" when they average at most this many rows: one warp then walks mean and spread in about 12 cycles a
-    // row, while the streaming kernel's 6 cycles cost a CTA with 200 KB of shared memory for every 32 dimensions.
+    // row, while the streaming kernel's 5 cycles cost a CTA with 200 KB of shared memory for every 32 dimensions.
     constexpr size_t SMALL_NODE = 2048;
     // The host does not know how many nodes a level has: it launches for the most there can be, and asks from here on, where
     // that bound would get out of hand.
