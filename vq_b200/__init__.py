@@ -281,7 +281,8 @@ class _Arr:
             self.keep = x
             self.shape = x.shape
             self.ptr = x.data_ptr()
-            self.size = x.numel()
+            if not want_2d:
+                self.size = x.numel()
             self.stream = torch._C._cuda_getCurrentRawStream(x.get_device())
         else:
             if _is_torch(x):
@@ -292,12 +293,13 @@ class _Arr:
             self.ptr = a.ctypes.data
             self.size = a.size
             self.stream = None
-        self.single = len(self.shape) == 1
         if want_2d:
+            shape = self.shape
+            self.single = len(shape) == 1
             if self.single:
-                self.n, self.dim = 1, self.shape[0]
-            elif len(self.shape) == 2:
-                self.n, self.dim = self.shape
+                self.n, self.dim = 1, shape[0]
+            elif len(shape) == 2:
+                self.n, self.dim = shape
             else:
                 raise ValueError("expected a vector or a matrix of row vectors")
 
