@@ -64,7 +64,7 @@ enum vqb_metric {
 /* ---- fit flags --------------------------------------------------------- */
 #define VQB_ACCUM_AUTO 0    /* ordered when the global row count is <= 65536, else fast */
 #define VQB_ACCUM_ORDERED 1 /* cluster sums in ascending row order == src/vector.rs:305-313 (bit-exact on one GPU) */
-#define VQB_ACCUM_FAST 2    /* shared-memory atomics; order unspecified, like src/vector.rs:298-304 */
+#define VQB_ACCUM_FAST 2    /* any order, like src/vector.rs:298-304 */
 
 typedef struct vqb_ctx vqb_ctx;
 typedef struct vqb_pq vqb_pq;

@@ -202,7 +202,7 @@ void CudaDevice::end_call()
     bop_fresh_ = nullptr; // the next call's centroids may have the same address
     if (!unfinished_ || lasting(stream_)) return;
     if (captured(stream_)) unfinished_ = false;
-    else cudaEventRecord(order_event_, stream_);
+    else if (cudaEventRecord(order_event_, stream_) != cudaSuccess) cudaGetLastError(); // (not the next launch's error)
 }
 
 cudaStream_t CudaDevice::aux_stream(int i)
