@@ -163,9 +163,9 @@ int vqb_dense_dots(vqb_ctx *ctx, const float *x, size_t n, size_t dim, const flo
 int vqb_opq_rotate_rows(vqb_ctx *ctx, const float *rot, size_t dim, const float *x, size_t n, float *y_out);
 int vqb_opq_cross_cov(vqb_ctx *ctx, const float *y, const float *x, size_t n, size_t dim, double *a_out);
 
-/* Diagnostic for the tensor-core path of the product quantizer (sub-space width 8): the raw split-TF32 scores
- * |c_j|^2/2 - x.c_j (scores_out: n x m x 256, may be NULL), the codes the path produces (codes_out: n x m) and the number
- * of (row, sub-space) pairs it left to the exact scan.  Requires m % 4 == 0, 4 <= m <= 64, 2 <= k <= 256.
+/* Diagnostic for the tensor-core path of the product quantizer (sub-space width 8): the raw scores
+ * |c_j|^2/2 - x.c_j of its operands (scores_out: n x m x 256, may be NULL), the codes the path produces (codes_out: n x m) and the number
+ * of (row, sub-space) pairs it left to the reference's arithmetic.  Requires m % 4 == 0, 4 <= m <= 64, 2 <= k <= 256.
  * No counterpart in the reference. */
 int vqb_pq_tensor_scores(vqb_ctx *ctx, const float *x, size_t n, size_t m, const float *codebooks, size_t k,
                          float *scores_out, uint32_t *codes_out, unsigned long long *marked_out);

@@ -1,0 +1,97 @@
+"""The product quantizer's tensor-core kernel where its fixed-point scores could go wrong: edges of the column tiles, centroids and rows
+far from the rest, offsets, sub-spaces and rows that only the full scan can decide, queues that fill up.  Codes and codebooks are
+the oracle's bit for bit."""
+import numpy as np
+import pytest
+
+import vq_b200 as vq
+from tests.golden import reference_known_answers as ka
+from tests.util import RecordingSeeder
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(oracle, cb, x, metric=(vq.Distance.Euclidean, ka.EUCLID)):
+    q = vq.ProductQuantizer.from_codebooks(cb, metric[0])
+    out, codes = q.quantize(x, return_codes=True)
+    out_o, codes_o = oracle.pq_quantize(cb, x, metric[1])
+    assert np.array_equal(codes, codes_o)
+    assert np.array_equal(out, out_o.view(np.float16), equal_nan=True)
+
+
+@pytest.mark.parametrize("k", [2, 15, 16, 17, 63, 64, 65, 127, 128, 129, 192, 255, 256])
+@pytest.mark.parametrize("m", [4, 20])
+def test_edges_of_the_column_tiles(oracle, k, m):
+    rng = np.random.default_rng(k * 100 + m)
+    n = 90_000 // m + 1  # past the one-launch path, a ragged last tile
+    x = rng.random((n, m * 8), dtype=np.float32)
+    cb = rng.random((m, k, 8), dtype=np.float32)
+    cb[1, k - 1] = cb[1, 0]                 # a tie between the first and the last column
+    x[n - 3:, 8:16] = cb[1, 0]
+    _check(oracle, cb, x)
+
+
+CASES = ["far", "very_far", "many_far", "offset", "tight", "equal", "nan", "tiny", "huge", "far_rows"]
+
+
+def _crafted(case, rng, n, m, k):
+    x = rng.normal(size=(n, m * 8)).astype(np.float32)
+    cb = rng.normal(size=(m, k, 8)).astype(np.float32)
+    if case == "far":                       # one centroid far away; rows near it, on the way to it and beyond
+        cb[:, 7] *= 100
+        x[: n // 4] = cb[:, 7].reshape(-1) * rng.random((n // 4, 1), dtype=np.float32) * 1.5
+    elif case == "very_far":
+        cb[:, 7] *= 1e6
+        x[: n // 4] = cb[:, 7].reshape(-1) * rng.random((n // 4, 1), dtype=np.float32)
+    elif case == "many_far":
+        cb[:, ::5] *= 30
+        x[::3] *= 30
+    elif case == "offset":                  # far from the origin: only the distances to the centroids' mean count
+        x += 1000
+        cb += 1000
+    elif case == "tight":                   # tight clusters far apart: most rows have several centroids within reach
+        where = rng.normal(size=(8, m * 8)).astype(np.float32) * 10
+        x = (where[rng.integers(8, size=n)] + rng.normal(size=(n, m * 8)) * 1e-3).astype(np.float32)
+        cb = np.ascontiguousarray(x[rng.permutation(n)[:k]].reshape(k, m, 8).transpose(1, 0, 2))
+    elif case == "equal":                   # every row ties with every centroid
+        x[:] = 0.25
+        cb[:] = 0.25
+    elif case == "nan":
+        cb[1, 3, 2] = np.nan
+        cb[2, 0, 0] = np.nan
+        cb[3, 5] = np.inf
+        x[5, 3], x[6, 9] = np.nan, -np.inf
+    elif case == "tiny":
+        x *= np.float32(1e-16)
+        cb *= np.float32(1e-16)
+    elif case == "huge":
+        x *= np.float32(1e16)
+        cb *= np.float32(1e16)
+    elif case == "far_rows":
+        x[::2] *= np.float32(1e4)
+        x[1::4] *= np.float32(1e19)
+    return x, cb
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_values_that_strain_the_fixed_point(oracle, case):
+    n, m, k = 22_500, 4, 200
+    x, cb = _crafted(case, np.random.default_rng(len(case)), n, m, k)
+    with np.errstate(all="ignore"):
+        _check(oracle, cb, x)
+        _check(oracle, cb, x, (vq.Distance.SquaredEuclidean, ka.SQ))
+        _check(oracle, cb, x, (vq.Distance.CosineDistance, ka.COSINE))
+
+
+@pytest.mark.parametrize("case", ["far", "many_far", "offset", "tight", "equal", "far_rows"])
+def test_training_on_values_that_strain_the_fixed_point(oracle, case):
+    n, m, k, iters = 12_000, 4, 150, 4
+    x, _ = _crafted(case, np.random.default_rng(len(case) + 1), n, m, k)
+    if case == "far_rows":
+        x = np.minimum(np.abs(x), np.float32(1e12))
+    so, sg = RecordingSeeder(3), RecordingSeeder(3)
+    init = so.init_pq(n, m, k)
+    sg.init_pq(n, m, k)
+    cb_o, _ = oracle.pq_fit(x, m, k, iters, init, so.draw)
+    pq = vq.ProductQuantizer.fit(x, m, k, iters, vq.Distance.Euclidean, 3, init_idx=init, draw=sg.draw, accumulate=vq.ACCUM_ORDERED)
+    assert np.array_equal(pq.codebooks, cb_o, equal_nan=True)

@@ -90,7 +90,7 @@ CudaDevice::~CudaDevice()
         if (stage_) cudaFreeHost(stage_);
         cudaFree(rot_split_);
         cudaFree(pq_scratch_);
-        cudaFree(pq_marks_);
+        cudaFree(pq_codes_);
         cudaFree(tc_stats_);
         cudaFree(tc_error_);
         if (status_host_) cudaFreeHost(status_host_);
@@ -479,20 +479,20 @@ void CudaDevice::release_dense()
     dense_ = DenseWork();
 }
 
-uint8_t *CudaDevice::pq_mark_buffer(size_t bytes)
+// Working memory of encodes on the tensor path, kept by the context: grown when a larger call comes.
+uint8_t *CudaDevice::pq_code_buffer(size_t bytes)
 {
-    if (bytes > pq_marks_cap_) {
+    if (bytes > pq_codes_cap_) {
         VQB_CUDA_CHECK(cudaStreamSynchronize(stream_));
-        cudaFree(pq_marks_);
-        pq_marks_ = nullptr;
-        pq_marks_cap_ = 0;
+        cudaFree(pq_codes_);
+        pq_codes_ = nullptr;
+        pq_codes_cap_ = 0;
         const size_t cap = bytes + bytes / 4;
         ++device_allocs_;
-        VQB_CUDA_CHECK(cudaMalloc(&pq_marks_, cap));
-        pq_marks_cap_ = cap;
-        VQB_CUDA_CHECK(cudaMemsetAsync(pq_marks_, 0, cap, stream_));
+        VQB_CUDA_CHECK(cudaMalloc(&pq_codes_, cap));
+        pq_codes_cap_ = cap;
     }
-    return pq_marks_;
+    return pq_codes_;
 }
 
 // Called at host synchronisation points: a tensor-core kernel whose bounded wait expired leaves a code here.
@@ -559,7 +559,7 @@ void CudaDevice::pq_tensor_debug(const float *x, size_t n, size_t m, const float
     download(&before, pq_scratch_ + pq_tc_stats_offset_floats(), sizeof before);
     PqTcBuffers tb;
     tb.scratch = pq_scratch_;
-    tb.marks = pq_mark_buffer(pq_tc_mark_bytes(n, m));
+    tb.codes = pq_code_buffer(pq_tc_code_bytes(n, m));
     tb.error_word = tc_error_;
     tb.dbg_scores = scores;
     launch_pq_tc(*this, p, M_SQ, false, 4, tb);
@@ -710,7 +710,6 @@ void CudaDevice::assign_train(const Shape &sh, const float *x, const float *cent
     if (pq_tensor_enabled_ && pq_tc_applicable(p, M_SQ)) {
         PqTcBuffers tb;
         tb.scratch = pq_scratch_;
-        tb.marks = pq_mark_buffer(pq_tc_mark_bytes(sh.n_local, sh.m));
         tb.error_word = tc_error_;
         tb.prepare_operand = (bop_fresh_ != centroids);
         launch_pq_tc(*this, p, M_SQ, true, code_bytes(sh.k), tb);
@@ -747,7 +746,7 @@ bool CudaDevice::pq_encode_ahead(const Shape &sh, const float *x, const float *c
     p.out_vec = !out_f16 || (aligned16(out_f16) && sh.m * sh.sd % 8 == 0);
     if (sh.n_local == 0 || !pq_tensor_enabled_ || !pq_tc_applicable(p, metric) || direct_encode_applicable(p, true)) return false;
     bop_fresh_ = nullptr;
-    launch_pq_operand_b(*this, codebooks, p.m, p.k, metric == M_COSINE, pq_scratch_);
+    launch_pq_operand_b(*this, codebooks, p.m, p.k, p.sd, metric == M_COSINE, pq_scratch_);
     return true;
 }
 
@@ -780,7 +779,7 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
         PqTcBuffers tb;
         tb.prepare_operand = !operand_there;
         tb.scratch = pq_scratch_;
-        tb.marks = pq_mark_buffer(pq_tc_mark_bytes(sh.n_local, sh.m));
+        tb.codes = pq_code_buffer(pq_tc_code_bytes(sh.n_local, sh.m));
         tb.error_word = tc_error_;
         launch_pq_tc(*this, p, metric, false, 4, tb);
         return;
@@ -1679,7 +1678,7 @@ void CudaDevice::update_centroids(const Shape &sh, const IterBuffers &buf, const
     const PeerView pv = peer_view(px, sh, tc_error_);
     if (pq8) {
         const StatusPage sp = status_page(m, k);
-        launch_pq_update_centroids(*this, (int)m, (int)k, buf.sums, buf.counts, buf.moved, buf.counts_f32, active, centroids, pq_scratch_, sp, pv);
+        launch_pq_update_centroids(*this, (int)m, (int)k, (int)sh.sd, buf.sums, buf.counts, buf.moved, buf.counts_f32, active, centroids, pq_scratch_, sp, pv);
         bop_fresh_ = centroids;
         wait_status(sp, m, k, status);
         return;

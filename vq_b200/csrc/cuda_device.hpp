@@ -51,7 +51,6 @@ class CudaDevice : public Device {
     bool svd_sweeps(double *gt, double *vt, size_t n) override;
     bool polar_rotation(const double *a_dev, size_t n, float *rot_dev) override;
     // Zero-filled map of at least `bytes` bytes for the product-quantizer tensor kernel; its users leave it zero-filled.
-    uint8_t *pq_mark_buffer(size_t bytes);
     void patch_centroids(const Shape &sh, const float *x, uint64_t row_begin, const RowPatch *patches, size_t n_patches,
                          float *centroids, Comm *comm) override;
     void assign_train(const Shape &sh, const float *x, const float *centroids, void *codes, const uint32_t *active,
@@ -153,10 +152,11 @@ class CudaDevice : public Device {
                       unsigned long long *stats);
     void *try_alloc(size_t bytes); // null when there is no room
     float *pq_scratch_ = nullptr;
+    uint8_t *pq_codes_ = nullptr;
+    size_t pq_codes_cap_ = 0;
+    uint8_t *pq_code_buffer(size_t bytes);
     float *rot_split_ = nullptr; // TF32 high and low parts of the rotation matrix of the current rotate_rows call (dim <= 128)
     bool opq_tensor_enabled_ = true;
-    uint8_t *pq_marks_ = nullptr;
-    size_t pq_marks_cap_ = 0;
     bool pq_tensor_enabled_ = false;
     unsigned long long *tc_stats_ = nullptr;
     int *tc_error_ = nullptr;

@@ -1,63 +1,80 @@
-// pq_tc.cu -- product-quantizer nearest-centroid search (sub-space width 8) with the scores on the tensor cores.
+// pq_tc.cu -- product-quantizer nearest-centroid search (sub-spaces of 4 or 8 values) with the scores on the tensor cores.
 //
 // Replaces the per-point scan of src/utils.rs:59-73 (training) and src/pq.rs:159-182 (encode) for the Euclidean metrics and,
 // when encoding, cosine.
 //
-// Scores.  S_j = |c_j|^2/2 - x.c_j ranks the centroids like the squared distance (|x - c_j|^2 = |x|^2 + 2 S_j).  Both
-// operands are split into two TF32 numbers (x = xh + xl, c = ch + cl, each part exactly representable, so the hardware's
-// treatment of the low mantissa bits does not matter) and one K = 32 tcgen05.mma chain per (128-row tile, sub-space)
-// accumulates, in f32,
-//     xh.(-ch) + xh.(-cl) + xl.(-ch) + 1*hn_h + 1*hn_l            (hn = |c|^2/2 split the same way)
-// into tensor memory: 128 x 256 scores with about 2^-21 relative accuracy instead of TF32's 2^-11.
+// Scores.  S_j = |c_j|^2/2 - x.c_j ranks the centroids like the squared distance (|x - c_j|^2 = |x|^2 + 2 S_j), for x and c
+// taken relative to any common point mu (the mean of the sub-space's centroids here).  Both operands are split into two
+// binary16 numbers, x = xh + xl and c = ch + cl, after scaling by powers of two that keep them in range, and tcgen05.mma
+// accumulates xh.(-ch) + xh.(-cl) + xl.(-ch) + the half norm (two parts) in f32 in tensor memory: half the MMAs of a split into TF32
+// numbers (K = 16 instead of 8 per step at the same cycles).
 //
-// Decision.  Per row the epilogue finds the smallest score, then counts the scores below
-//     limit = best + 7e-6 (|x|^2/2 + 2 max_j hn_j + |best|)
-// If exactly one score lies below the limit its centroid is the reference's answer; otherwise (two or more within the
-// limit, NaN / infinity, values too small to rank) the (row, sub-space) pair is marked and a second kernel decides it with
-// the reference's own f32 arithmetic over all centroids (ascending index, strict '<', sqrt inside the comparison for the
-// Euclidean metric, scan started at centroid 0).  The result equals the exact scan's bit for bit.
+// Fixed point.  What a row needs is the index of its smallest score and whether a second one is close.  The last step of the
+// chain adds 2^23 and a row constant K0, and the row's operand carries a factor sigma such that
+//     T_j = sigma S_j + K0   lies in [8, 65400]   for every centroid (Cauchy-Schwarz: -min(|x|^2/2, |x| rho) <= S_j <= |x| rho + rho^2/2).
+// 2^23 + T_j has T_j, rounded to an integer, in the low 16 bits of its f32 representation: tcgen05.ld.pack::16b delivers two of
+// them per register and one 3-input packed minimum (2 cycles of the integer pipe, like the f32 one) looks at four values
+// instead of two.  The minimum of every score, which bounded this kernel, costs half, and so does reading tensor memory.
 //
-// Bound behind 7e-6.  u = 2^-24, xh2 = |x|^2/2, HN = max_j hn_j.
-//   operand split:   dropped xl.cl and the rounding of xl, cl to TF32: <= 3 * 2^-22 sum|x_i c_ji| <= 3 * 2^-22 (xh2 + hn_j)
-//   half norm:       f32 chain 9u hn_j, split 2^-22 hn_j
-//   accumulation:    26 exact products summed by the tensor core in f32; assumed error <= 2^-20 (hn_j + sum|x_i c_ji|),
-//                    sixteen times what is measured (tests/test_gpu_pq_tensor.py measures it against f64)
-//   => |S_j - true| <= E = 1.25 * 2^-19 (xh2 + 2 HN) = 2.4e-6 (xh2 + 2 HN)
-//   the reference prefers w over a = argmin S only if D_w <= D_a (1 + 4u) in its own arithmetic (10u relative each), i.e.
-//   S_w <= S_a + 2E + 25u (xh2 + |S_a| + E)  <=  S_a + 4.8e-6 (xh2 + 2HN) + 1.5e-6 (xh2 + |S_a|) + ...  <  limit.
-// One pass over the accumulator (3-input minima, one per score: 2 cycles of the integer pipe each, which is what bounds the
-// epilogue at 512 cycles per unit and scheduler) leaves the minima of the 16 blocks of 16 consecutive columns and of the 16
-// classes of columns equal modulo 16.  Two scores below the limit differ in their block or in their class, so exactly one score
-// lies below it <=> exactly one block minimum and exactly one class minimum do, and these two give its column.  They are counted
-// with t = sat((limit - S) * 2^p), p chosen per row so that limit * 2^p ~ 2^60: a minimum differs from the limit by nothing or
-// by at least one unit in its last place (>= 2^-24 |limit|), so t is exactly 0 or 1, and sum t * (1 + i / 512) has count and
-// index in one number.  Rows whose true distances could overflow f32 (|x|^2/2 + 2 HN >= 1e37) are marked as well: there the
-// reference's own comparisons see infinities.
+// Decision.  Minima of the 16 blocks of 16 consecutive columns and of the 16 classes of columns equal modulo 16, even and odd
+// columns side by side in a register.  Two columns differ in their block or in their class, so exactly one T_j lies within M of
+// the smallest <=> exactly one block minimum and exactly one class minimum do, and they give its column.  Everything else
+// (close scores, ties, NaN / infinity) is put into a queue of the warp in shared memory, with the set of blocks and classes that
+// came close; every 32 entries the warp evaluates those columns with the reference's own f32 arithmetic, one entry per lane
+// (strict '<' in ascending index, sqrt inside the comparison for the Euclidean metric).  The result equals the exact scan's bit
+// for bit.
 //
-// Measured, 1M x 128, m 16, k 256: 0.923 -> 0.613 ms per training pass (encode 0.942 -> 0.638 ms) against two passes over the
-// accumulator, the second of which spent two operations per score on count and index.  Per (tile, sub-space): 1456 cycles,
-// integer pipe 56 % busy, tensor pipe 35 %; the rest is the way from a commit to the epilogue and back.  Four teams (one per
-// sub-space) and eight warps per accumulator (half of the columns each) came to 0.63 - 0.81 ms: their halved registers cost
-// spills, moves or doubled tails.  Accumulators of 128 columns: 0.96 ms (an MMA of N = 128 takes as long as one of N = 256).
+// Bound behind M.  In units of T (sigma (|x|^2 + rho^2) <= 65300, which covers sigma (|x| + rho)^2 / 2):
+//   last step: the tensor core aligns its addends to 2^23 and cuts each towards zero two bits below the unit (measured: 1, 2, 8 and
+//   16 fractional addends beside 2^23 give errors of 0.25 per addend and one unit downwards for the result).  2^23, K0 and the
+//   padding are whole numbers, so that only the accumulator of the steps before is cut: error in (-1.25, 0.25)
+//   steps before: partial sums up to 2^16 in f32: 0.02 each; dropped xl.cl: sd * 8 * 4 * 2^-12 = 0.06, the low parts' rounding as much
+//   again; half norm in f32 9u and in two parts 2^-24: 0.04; x - mu and c - mu, u each: 0.01
+//   the reference's own arithmetic prefers w over a only if D_w <= D_a (1 + 4u) with (sd + 2)u each: 24u * 65300 = 0.1
+//   => T_w <= T_best + 1.5 + 2 * 0.17 + 0.1, i.e. a difference of at most 1.  M = 3 leaves room for twice what was measured.
+//
+// Far centroids.  One centroid far from the others would stretch the range for all.  Those farther from mu than four times the
+// mean distance (mu: the mean of the rest, found in up to six rounds) are left out: rho covers the others.  The producers leave a
+// lower bound of what a far one can score against the row, lim^2/2 - lim |x|, in shared memory; a row that has it within reach is
+// queued and looks at the far ones as well.  Columns beyond k, far ones and those that are not finite hold T = 57344; a smallest
+// value up there is decided by a scan of all centroids.  Rows that are not finite, too far or too large for f32 get an operand of
+// zeros: all columns tie, everything is scanned.  So does a sub-space whose
+// radius leaves f32; with a NaN in centroid 0, where the reference's scan starts, the answer is 0 without one.
+// (500,000 x 128, m 16, k 256, encode, before -> now: rows of normal values 358 -> 260 us; 64 clusters of standard deviation 0.05 / 0.001
+// and distance 1: 666 -> 480 / 6100 -> 1640 us; values around 100: 6400 -> 255 us, which the uncentred scores could not separate.)
 //
 // Cosine (src/distances.rs:141-150).  1 - x.c / (|x| |c|) ranks like S_j = -x.(c_j / |c_j|), with the norm that the reference
-// computes and a zero vector for a zero norm (its distance is 1, like a score of 0).  The same split and chain with zero half
-// norms: |S_j - true| <= 2.4e-6 |x| (the unit vectors' own rounding, 2u, included).  The reference's quotient carries (2d + 6)u
-// = 22u and its difference from 1 another 2u, so it can prefer w over a only if S_w <= S_a + |x| (2 * 2.4e-6 + 2 * 24u): limit =
-// best + 7e-6 (1.25 |x| + |best|).  Norms outside [1e-17, 1e18] (products that underflow or overflow) void the row, or the
-// sub-space if it is a centroid's: everything goes to the exact scan.
+// computes and a zero vector for a zero norm (its distance is 1, like a score of 0): no half norms, mu = 0, rho = 1.  The
+// reference's quotient carries (2d + 6)u and its difference from 1 another 2u: 48u |x|, 0.1 units of T.  Norms outside
+// [1e-17, 1e18] (products that underflow or overflow) void the row, or the sub-space if it is a centroid's.
 //
-// CTA (1 per SM, persistent, 448 threads), owning 4 consecutive sub-spaces (m / 4 groups share the row tiles):
-//   warp 0       loads the group's four operand-B tiles once (TMA, 128B swizzle, no multicast; 32 KiB each) and, for an
-//                encode, the binary16 images of the group's centroids (16 KiB, bulk copy)
-//   warp 1       owns tensor memory (two 128 x 256 f32 accumulators) and issues the MMAs
-//   warps 2-5    read row slices from global memory, split them and write operand-A tiles (128 rows x 128 bytes, 128B
-//                swizzle) into a 4-stage ring, plus |x|^2/2 per row
-//   warps 6-13   epilogue: two teams of four warps (one row per lane, one TMEM lane quadrant per warp); team t serves
-//                sub-spaces 2t, 2t+1 of the group through accumulator t
+// CTA (1 per SM, persistent, 896 threads), owning up to 4 consecutive sub-spaces (groups share the row tiles).  A unit is one
+// 128-row tile of one sub-space; it uses one of the two 128 x 256 f32 accumulators, in two halves of 128 columns.
+//   warps 0-3    MMA issuers, one per accumulator half; warp 0 first loads the group's operand-B tiles (TMA, no multicast), warp 1
+//                owns tensor memory
+//   warps 4-11   take the row tile that TMA has brought into shared memory (two buffers), scale and split the slices (two sub-spaces a
+//                warp) and write operand-A tiles, one stage per sub-space
+//   warps 12-27  epilogue: a team of four warps per sub-space (one row per lane, one TMEM lane quadrant per warp)
 // Every wait is bounded; on expiry the CTA records a code, stops issuing, frees tensor memory and the host raises an error.
+//
+// Measured, 1M x 128, m 16, k 256: a training pass 0.643 (0.613 and 0.030 for the pairs left to an exact kernel) -> 0.40 ms, an
+// encode 0.698 -> 0.47 ms, against f32 scores of split-TF32 operands with one f32 minimum each.  Per unit 930 cycles; the parts
+// alone: hand-over of the barriers 500, with the producers 720, with the epilogue 860; the MMAs take 385, the minima 256 of a
+// scheduler's integer pipe.  What each choice brought (ms a pass, the others as they are):
+//   * one issuer per accumulator half instead of one per accumulator (0.46), and those instead of one in all (0.71): a half is idle
+//     from its release until its issuer has seen it, and an issuer that waits for one half keeps the other waiting
+//   * eight producer warps instead of four (0.48): 150 dependent instructions a slice, 5 cycles each, are what a warp takes
+//   * four teams of four warps with 72 registers, whose loads wait for the first half's minima, instead of three with 96 that load a
+//     half at once (0.49): more warps in flight count for more than the time a half stays occupied
+//   * rows by TMA, and 64- and 32-byte operand rows, which make room for them: loaded by the producers' lanes, 32 rows an
+//     instruction, they keep the L1 cache busy for 256 cycles a unit (0.40)
+//   * an encode leaves one byte per pair; pq_expand_kernel turns them into rows and 32-bit codes with whole-line stores, 0.08 ms
+//     (16-byte pieces stored from here: 0.49 in all)
+// The constant in a step of its own (K = 48) rather than beside the last products (K = 32): ten cut addends instead of one would
+// need M = 8 and triple the share of queued rows.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "assign_reg.cuh"
 #include "cuda_device.hpp"
@@ -69,109 +86,285 @@ namespace vqb {
 
 namespace {
 
-constexpr int BM = 128, BN = 256, SDW = 8, KOP = 32, NSTAGE = 4, MAXM = 64, XH_RING = 8, NTHREADS = 448;
-constexpr uint32_t A_STAGE_BYTES = BM * 128; // 16 KiB
-constexpr uint32_t B_BYTES = BN * 128;       // 32 KiB per sub-space
-constexpr float PAD_SCORE = 1e30f;           // score of the columns beyond k
-constexpr float MARGIN_COEF = 7e-6f;
-constexpr float COS_MIN = 1e-17f, COS_MAX = 1e18f; // cosine: norms that the scores can be trusted for
+constexpr int BM = 128, BN = 256, MAXM = 64, NTHREADS = 32 * (4 + 8 + 16);
+constexpr int QCAP = 64; // queue entries per epilogue warp: fewer than 32 wait, at most 32 are added at a time
+constexpr float COS_MIN = 1e-17f, COS_MAX = 1e18f;  // cosine: norms that the scores can be trusted for
+constexpr float RHO_MIN = 1e-14f, RHO_MAX = 1e15f;  // Euclidean: radii for which neither 2^+-96 scalings nor distances leave f32
+constexpr float SQ_MAX = 5e36f;               // rows beyond: the reference's own distances could overflow
+constexpr float T_RANGE = 65300.0f;
+constexpr float CR_MIN = 6.2e-5f;             // below: no longer a normal binary16 number
+constexpr float SPLIT = 1.5f * 134217728.0f;  // 1.5 2^27: adding it rounds to a multiple of 16
+constexpr uint32_t T_HIGH = 57344u - 16u;     // the padding columns' T, less the window
+
+// per-sub-space constants (32 floats): mu[16], then
+constexpr int SUB_RHO2 = 16, SUB_SCALE = 17, SUB_SCALE2 = 18, SUB_FLAGS = 19, SUB_LIM = 20, SUB_MASK = 24, SUB_FLOATS = 32;
+constexpr uint32_t SUB_VOID = 1u, SUB_FAR = 2u, SUB_NAN0 = 4u; // NAN0: every distance to centroid 0 is NaN, where the scan starts and stays
 
 // scratch layout (floats)
-constexpr size_t OFF_BOP = 0;                                   // [MAXM][256][32] operand B
-constexpr size_t OFF_C16 = OFF_BOP + (size_t)MAXM * BN * KOP;   // [MAXM][256] 8 halves (uint4)
-constexpr size_t OFF_HMAX = OFF_C16 + (size_t)MAXM * BN * 4;    // [MAXM]
-constexpr size_t OFF_STATS = OFF_HMAX + MAXM;                   // 2 x u64: marked pairs, launches
+constexpr size_t OFF_B1 = 0;                                      // [MAXM][256] rows of 32 halves: operand B, K slots 0 .. 31
+constexpr size_t OFF_B2 = OFF_B1 + (size_t)MAXM * BN * 16;        // [MAXM][256] rows of 16 halves: K slots 32 .. 47
+constexpr size_t OFF_C16 = OFF_B2 + (size_t)MAXM * BN * 8;        // [MAXM][256] rows of up to 8 halves
+constexpr size_t OFF_SUB = OFF_C16 + (size_t)MAXM * BN * 4;       // [MAXM][32]
+constexpr size_t OFF_STATS = OFF_SUB + (size_t)MAXM * SUB_FLOATS; // 2 x u64: pairs that went through the queues, unused
 constexpr size_t SCRATCH_FLOATS = OFF_STATS + 4;
 
+// How the chain's K slots (16 per MMA) are used for each width.  Slots 0 .. 31 lie in a tile of 64-byte rows (64B swizzle), the rest
+// in one of 32-byte rows (32B swizzle): 128-byte rows would leave no room for the row tiles.
+template <int SD> struct Slots;
+template <> struct Slots<4> {
+    static constexpr int STEPS = 2, NORM = 12, CONST = 16, M = 3;
+};
+template <> struct Slots<8> {
+    static constexpr int STEPS = 3, NORM = 24, CONST = 32, M = 3;
+};
+template <int SD> constexpr uint32_t A1_BYTES = BM * 64;                            // a stage
+template <int SD> constexpr uint32_t A2_BYTES = Slots<SD>::STEPS == 3 ? BM * 32 : 0;
+template <int SD> constexpr uint32_t A_BYTES = A1_BYTES<SD> + A2_BYTES<SD>;
+template <int SD> constexpr uint32_t B1_BYTES = BN * 64;                            // a sub-space
+template <int SD> constexpr uint32_t B2_BYTES = Slots<SD>::STEPS == 3 ? BN * 32 : 0;
+template <int SD> constexpr uint32_t B_BYTES = B1_BYTES<SD> + B2_BYTES<SD>;
+template <int SD> constexpr uint32_t RAW_BYTES = BM * 4 * SD * 4;                   // a row tile
+
 struct alignas(8) PqBarriers {
-    unsigned long long afull[NSTAGE], aempty[NSTAGE], bfull, tfull[2], tempty[2];
+    unsigned long long afull[4], aempty[4], bfull, rfull[2], rempty[2]; // a...: per sub-space; r...: per row-tile buffer
+    unsigned long long tfull[8], tempty[8];                             // [2 ss + half]
     uint32_t tmem_base;
     int abort_flag;
 };
 
 struct PqTcParams {
     AssignParams a;
-    const uint4 *c16;   // [m][256] centroid values as 8 binary16
-    const float *hnmax; // [m]
-    uint8_t *marks;     // [n][m/2]: bit h of byte (g, team) = pair (row, 4g + 2 team + h) needs the exact scan
+    const float *sub; // [m][32]
     unsigned long long *stats;
     int *error;
-    float *dbg_scores; // optional [n][m][256]
+    float *dbg_scores;              // optional [n][m][256]
+    uint16_t first[MAXM / 4 + 1];   // CTAs first[g] .. first[g + 1] - 1 serve group g
 };
 
-__device__ __forceinline__ float to_tf32(float v)
+__device__ __forceinline__ uint32_t pack_f16(float lo, float hi)
 {
     uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
-    return __uint_as_float(r);
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
 }
 
-// The 11-bit head of v by Veltkamp's splitting (Dekker, Numer. Math. 18, 1971): nearest TF32 number like to_tf32, on the FMA
-// pipe; cvt.rna.tf32 costs two instructions of the integer pipe that the epilogue's minima need.  |v| > 2^114 gives NaN, which
-// sends the row to the exact scan.
-__device__ __forceinline__ float split_tf32(float v)
+__device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b)
 {
-    const float t = __fmul_rn(v, 8193.0f);
-    return __fsub_rn(t, __fsub_rn(t, v));
+    uint32_t r;
+    asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
 }
 
-// order in which the four sub-spaces of a group are issued: accumulator / team = ss >> 1 alternates
-__device__ __forceinline__ int issue_order(int p) { return ((p & 1) << 1) | (p >> 1); } // 0, 2, 1, 3
+__device__ __forceinline__ uint32_t min3_u16x2(uint32_t a, uint32_t b, uint32_t c) { return __vimin3_u16x2(a, b, c); } // one instruction on sm_100
 
-constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES + (size_t)NSTAGE * A_STAGE_BYTES + ((size_t)XH_RING * BM + 4 * BN * 4) * sizeof(float) + sizeof(PqBarriers) + 64;
-
-template <bool TRAIN, bool COSINE, bool DUMP>
-__global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constant__ CUtensorMap map_b, const PqTcParams Q)
+__device__ __forceinline__ float sqrt_approx(float v)
 {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+template <int SD>
+constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES<SD> + 4 * (size_t)A_BYTES<SD> + 2 * (size_t)RAW_BYTES<SD> + 4 * SUB_FLOATS * sizeof(float) +
+                              16 * QCAP * sizeof(uint4) + 4 * 4 * BM * sizeof(uint16_t) + sizeof(PqBarriers) + 64;
+
+// What a row contributes besides its (shifted) values: the factor of its operand, the half-norm factor and the two row constants.
+struct RowFrame {
+    float mul, cr, k0;
+    uint32_t far; // no far centroid can have a T below this
+    bool ok;
+};
+
+template <int SD, bool COSINE> __device__ __forceinline__ RowFrame row_frame(const float (&y)[SD], const float *sub)
+{
+    RowFrame f;
+    float sq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < SD; ++i) sq = fmaf(y[i], y[i], sq);
+    const float4 c = *reinterpret_cast<const float4 *>(sub + SUB_RHO2); // rho^2 (rounded up), scale, scale^2, flags
+    const uint32_t flags = __float_as_uint(c.w);
+    float low, sigma;
+    if (COSINE) {
+        const float norm = sqrt_approx(sq) * 1.000002f; // not below |x| |unit vector|
+        low = norm;
+        sigma = __fdividef(T_RANGE, 2.0f * norm);
+        f.cr = 0.0f;
+        f.mul = 0.5f * sigma;
+        f.ok = norm >= COS_MIN && norm <= COS_MAX && !(flags & SUB_VOID);
+    } else {
+        // eleven significant bits, rounded down: cr is a binary16 number as well
+        f.cr = __uint_as_float(__float_as_uint(__fdividef(T_RANGE, (sq * 1.000001f + c.x) * c.z)) & 0xFFFFE000u);
+        low = 0.5f * sq;
+        sigma = f.cr * c.z;
+        f.mul = f.cr * c.y;
+        f.ok = sq < SQ_MAX && f.cr >= CR_MIN && !(flags & SUB_VOID);
+    }
+    // a whole number (1.5 2^23 rounds it), 12 to spare after rounding to binary16
+    f.k0 = fmaf(low, sigma * 1.001f, 12582912.0f + 12.0f) - 12582912.0f;
+    f.far = 0xFFFFu;
+    if (flags & SUB_FAR) {
+        const float lim = sub[SUB_LIM], norm = sqrt_approx(sq) * 1.000001f;
+        const float t = norm < lim ? (0.5f * lim - norm) * lim * sigma + 0.999f * f.k0 - 16.0f : 0.0f;
+        f.far = (uint32_t)fminf(fmaxf(t, 0.0f), 65535.0f);
+    }
+    return f;
+}
+
+// Minima of 64 more columns (two per register): hb = their four blocks of 16, ga = the classes.
+template <bool FIRST> __device__ __forceinline__ void fold64(const uint32_t (&v)[32], uint32_t *hb, uint32_t (&ga)[8])
+{
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        if (FIRST) {
+            ga[t] = min3_u16x2(v[t], v[8 + t], v[16 + t]);
+            ga[t] = min_u16x2(ga[t], v[24 + t]);
+        } else {
+            ga[t] = min3_u16x2(ga[t], v[t], v[8 + t]);
+            ga[t] = min3_u16x2(ga[t], v[16 + t], v[24 + t]);
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const uint32_t *w = v + 8 * b;
+        hb[b] = min3_u16x2(min3_u16x2(w[0], w[1], w[2]), min3_u16x2(w[3], w[4], w[5]), min_u16x2(w[6], w[7]));
+    }
+}
+
+// The queued rows of one warp, one per lane, with the reference's arithmetic.  Entry: x = tile, y = row in the tile | classes << 16
+// (bit c: columns = c modulo 16 are candidates), z = blocks (bit 2 i + p: block i, columns of parity p), w = Q_WHOLE: all centroids;
+// Q_FAR: the far ones as well.  Returns whether this lane's assignment changed.
+constexpr uint32_t Q_WHOLE = 1u, Q_FAR = 2u;
+
+template <int SD, bool TRAIN, int METRIC>
+__device__ __noinline__ bool pq_queue_drain(const PqTcParams &Q, const uint4 *queue, const float *sub, int count, int s, int lane)
+{
+    const AssignParams &P = Q.a;
+    bool moved = false;
+    const bool mine = lane < count;
+    uint4 e = make_uint4(0u, 0u, 0u, 0u);
+    if (mine) e = queue[lane];
+    const unsigned long long row = (unsigned long long)e.x * BM + (e.y & 127u);
+    float x[SD];
+    if (mine) {
+        load_slice<SD>(x, P.x + row * P.ld + (size_t)s * SD, true);
+    } else {
+#pragma unroll
+        for (int i = 0; i < SD; ++i) x[i] = 0.0f;
+    }
+    const float na = METRIC == M_COSINE ? norm_chain(x, SD, 1) : 0.0f;
+    const float *cbs = P.centroids + (size_t)s * P.k * SD;
+    float bd = VQB_INF;
+    int bi = 0x7fffffff;
+    bool nan0 = false;
+    auto look = [&](int j) {
+        float cv[SD];
+        load_centroid<SD>(cv, cbs + (size_t)j * SD);
+        float d = METRIC == M_COSINE ? reg_dist<SD, M_COSINE>(x, cv, 0.0f, na, norm_chain(cv, SD, 1)) : reg_dist<SD, M_SQ>(x, cv, 0.0f, 0.0f, 0.0f);
+        if (METRIC == M_EUCLID) d = __fsqrt_rn(d);
+        if (j == 0) nan0 = !(d == d);
+        if (d < bd || (d == bd && j < bi)) {
+            bd = d;
+            bi = j;
+        }
+    };
+    // many candidates (ties): the lanes go through all centroids together, whose loads are then the same for all
+    const bool all = (e.w & Q_WHOLE) || __popc(e.z) * __popc(e.y >> 16) >= 256;
+    if (__float_as_uint(sub[SUB_FLAGS]) & SUB_NAN0) {
+        nan0 = true;
+    } else if (__any_sync(0xffffffffu, all)) {
+#pragma unroll 4
+        for (int j = 0; j < P.k; ++j) look(j);
+    }
+    if (!all) {
+        bd = VQB_INF, bi = 0x7fffffff, nan0 = false;
+        uint32_t blocks = e.z;
+        while (blocks) {
+            const int bit = __ffs(blocks) - 1;
+            blocks &= blocks - 1;
+            uint32_t c = (e.y >> 16) & ((bit & 1) ? 0xAAAAu : 0x5555u);
+            while (c) {
+                const int j = (bit >> 1) * 16 + __ffs(c) - 1;
+                c &= c - 1;
+                if (j < P.k) look(j);
+            }
+        }
+        if (e.w & Q_FAR)
+            for (int w = 0; w < BN / 32; ++w) {
+                uint32_t far = __float_as_uint(sub[SUB_MASK + w]);
+                while (far) {
+                    look(w * 32 + __ffs(far) - 1);
+                    far &= far - 1;
+                }
+            }
+    }
+    if (mine) {
+        const int idx = (bi == 0x7fffffff || nan0) ? 0 : bi; // nothing below +inf, or the reference's scan starts at a NaN
+        uint8_t *cp = reinterpret_cast<uint8_t *>(P.codes) + row * (unsigned long long)P.m + s;
+        if (!TRAIN || *cp != (uint8_t)idx) {
+            moved = true;
+            *cp = (uint8_t)idx;
+        }
+    }
+    if (lane == 0) atomicAdd(Q.stats, (unsigned long long)count);
+    __syncwarp(); // the entries are read: the caller may add new ones
+    return moved;
+}
+
+template <int SD, bool TRAIN, int METRIC, bool WIDE, bool DUMP>
+__global__ void __launch_bounds__(NTHREADS, 1)
+    pq_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
+                 const __grid_constant__ PqTcParams Q)
+{
+    constexpr bool COSINE = METRIC == M_COSINE;
+    constexpr int halves = WIDE ? 2 : 1; // accumulator halves that hold centroids
+    using SL = Slots<SD>;
     extern __shared__ unsigned char smem_raw[];
     const AssignParams &P = Q.a;
     unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    unsigned char *b_smem = base;                                           // 4 x 32 KiB
-    unsigned char *a_smem = base + 4 * (size_t)B_BYTES;                     // NSTAGE x 16 KiB
-    float *xh_ring = reinterpret_cast<float *>(a_smem + (size_t)NSTAGE * A_STAGE_BYTES); // [XH_RING][128]
-    const uint4 *c16_s = reinterpret_cast<const uint4 *>(xh_ring + XH_RING * BM);         // [4][256] binary16 images
-    PqBarriers *bars = reinterpret_cast<PqBarriers *>(xh_ring + XH_RING * BM + 4 * BN * 4);
+    unsigned char *b_smem = base;                                                    // [4] 64-byte rows, then [4] 32-byte rows
+    unsigned char *a_smem = base + 4 * (size_t)B_BYTES<SD>;                          // the same
+    unsigned char *raw_smem = a_smem + 4 * (size_t)A_BYTES<SD>;                      // [2] row tiles
+    float *sub_s = reinterpret_cast<float *>(raw_smem + 2 * (size_t)RAW_BYTES<SD>);  // [4][32]
+    uint4 *queues = reinterpret_cast<uint4 *>(sub_s + 4 * SUB_FLOATS);               // [16][QCAP]
+    uint16_t *far_s = reinterpret_cast<uint16_t *>(queues + 16 * QCAP);              // [4][4][128] RowFrame::far of four tiles
+    PqBarriers *bars = reinterpret_cast<PqBarriers *>(far_s + 4 * 4 * BM);
     volatile int *abort_flag = &bars->abort_flag;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31; // (the shuffle: uniform by construction)
     const int m = P.m, k = P.k;
-    const int ngroups = m >> 2;
-    const int g = blockIdx.x % ngroups;
-    const unsigned long long tile0 = blockIdx.x / ngroups, tstep = gridDim.x / ngroups;
-    const unsigned long long n_tiles = (P.n + BM - 1) / BM;
+    int g = 0;
+    while (blockIdx.x >= Q.first[g + 1]) ++g;
+    const uint32_t tile0 = blockIdx.x - Q.first[g], tstep = Q.first[g + 1] - Q.first[g];
+    const uint32_t n_tiles = (uint32_t)((P.n + BM - 1) / BM);
+    const uint32_t last_rows = (uint32_t)(P.n - (unsigned long long)(n_tiles - 1) * BM); // rows of the last tile
+    const int here = min(4, m - 4 * g); // sub-spaces of this group
 
-    // the active sub-spaces of this group in issue order (identical in every thread), packed four bits apiece so that the
-    // lookups below are shifts on a register: indexed local arrays would go through the L1 cache, which the row stream of
-    // the producer warps keeps flushing (each lookup then costs a trip to L2 on the critical path of a unit)
-    uint32_t list_p = 0, pos_p = 0xFFFFu; // list_p: nibble p = sub-space issued p-th; pos_p: nibble ss = its position, 0xF = inactive
-    int nact = 0;
+    uint32_t act = 0; // bit ss: sub-space ss of the group takes part (identical in every thread)
 #pragma unroll
-    for (int p = 0; p < 4; ++p) {
-        const int ss = issue_order(p);
-        const bool act = !(TRAIN && P.active && P.active[g * 4 + ss] == 0);
-        if (act) {
-            pos_p = (pos_p & ~(0xFu << (4 * ss))) | ((uint32_t)nact << (4 * ss));
-            list_p |= (uint32_t)ss << (4 * nact);
-            ++nact;
-        }
-    }
-    auto list_at = [&](int p) { return (int)((list_p >> (4 * p)) & 0xFu); };
-    auto pos_of = [&](int ss) { return (int)((pos_p >> (4 * ss)) & 0xFu); }; // 15 = inactive
+    for (int ss = 0; ss < 4; ++ss)
+        if (ss < here && !(TRAIN && P.active && P.active[g * 4 + ss] == 0)) act |= 1u << ss;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NSTAGE; ++s) {
+        for (int s = 0; s < 4; ++s) {
             mbar_init(&bars->afull[s], 4);
-            mbar_init(&bars->aempty[s], 1);
+            mbar_init(&bars->aempty[s], halves); // one commit per accumulator half
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&bars->rfull[b], 1);
+            mbar_init(&bars->rempty[b], 8);
         }
         mbar_init(&bars->bfull, 1);
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < 8; ++b) {
             mbar_init(&bars->tfull[b], 1);
             mbar_init(&bars->tempty[b], 4);
         }
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    if (threadIdx.x < here * SUB_FLOATS) sub_s[threadIdx.x] = Q.sub[(size_t)g * 4 * SUB_FLOATS + threadIdx.x];
+    for (uint32_t i = threadIdx.x; i < 4 * A_BYTES<SD> / 16; i += NTHREADS) // the slots that no row uses stay zero
+        reinterpret_cast<uint4 *>(a_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -181,261 +374,281 @@ __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constan
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = bars->tmem_base;
 
-    if (warp == 0) {
-        // ------------------------------------------------ operand B: the group's four sub-spaces, once
-        if (lane == 0 && nact > 0) {
-            mbar_expect_tx(&bars->bfull, 4 * B_BYTES + (TRAIN ? 0u : 4u * BN * 16u));
-            for (int ss = 0; ss < 4; ++ss) tma_load_2d(b_smem + (size_t)ss * B_BYTES, &map_b, 0, (g * 4 + ss) * BN, &bars->bfull);
-            if (!TRAIN) bulk_load_1d(const_cast<uint4 *>(c16_s), Q.c16 + (size_t)g * 4 * BN, 4u * BN * 16u, &bars->bfull);
+    if (warp < 4) {
+        // ------------------------------------------------ operand B: the group's sub-spaces, once
+        const bool leader = elect_one();
+        if (warp == 0 && leader && act) {
+            mbar_expect_tx(&bars->bfull, (uint32_t)here * B_BYTES<SD>);
+            for (int ss = 0; ss < here; ++ss) {
+                tma_load_2d(b_smem + (size_t)ss * B1_BYTES<SD>, &map_b1, 0, (g * 4 + ss) * BN, &bars->bfull);
+                if (B2_BYTES<SD>) tma_load_2d(b_smem + 4 * (size_t)B1_BYTES<SD> + (size_t)ss * B2_BYTES<SD>, &map_b2, 0, (g * 4 + ss) * BN, &bars->bfull);
+            }
         }
-    } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer
-        if (lane == 0 && nact > 0) {
+        __syncwarp();
+        // ------------------------------------------------ MMA issuer of half warp % 2 of accumulator warp / 2: the whole warp walks the loop,
+        // so that what it works out is uniform, and one lane issues
+        const int acc = warp >> 1, half = warp & 1;
+        const uint32_t mine = half < halves ? act >> (2 * acc) & 3u : 0u;
+        if (mine) {
             bool ok = mbar_wait(&bars->bfull, 0, abort_flag, Q.error, 12);
-            uint32_t it = 0, uses0 = 0, uses1 = 0;
-            for (unsigned long long tile = tile0; ok && tile < n_tiles && !*abort_flag; tile += tstep) {
-                for (int p = 0; ok && p < nact; ++p, ++it) {
-                    const int ss = list_at(p);
-                    const uint32_t b = (uint32_t)ss >> 1;
-                    const int st = it % NSTAGE;
-                    if (!mbar_wait(&bars->afull[st], (it / NSTAGE) & 1u, abort_flag, Q.error, 14)) {
-                        ok = false;
-                        break;
-                    }
-                    const uint32_t ub = b ? uses1 : uses0;
-                    if (!mbar_wait(&bars->tempty[b], (ub & 1u) ^ 1u, abort_flag, Q.error, 13)) {
-                        ok = false;
-                        break;
-                    }
-                    if (b) ++uses1;
-                    else ++uses0;
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t adesc = smem_desc_sw128(smem_u32(a_smem + (size_t)st * A_STAGE_BYTES));
-                    const uint64_t bdesc = smem_desc_sw128(smem_u32(b_smem + (size_t)ss * B_BYTES));
+            const uint32_t a1 = (smem_u32(a_smem) + 2 * acc * A1_BYTES<SD>) >> 4, a2 = (smem_u32(a_smem) + 4 * A1_BYTES<SD> + 2 * acc * A2_BYTES<SD>) >> 4;
+            const uint32_t b1 = (smem_u32(b_smem) + 2 * acc * B1_BYTES<SD> + half * (B1_BYTES<SD> / 2)) >> 4;
+            const uint32_t b2 = (smem_u32(b_smem) + 4 * B1_BYTES<SD> + 2 * acc * B2_BYTES<SD> + half * (B2_BYTES<SD> / 2)) >> 4;
+            const uint32_t td = tmem_base + acc * BN + half * 128;
+            uint32_t phase = 0; // parity of the tile's phases
+            for (uint32_t tile = tile0; ok && tile < n_tiles && !*abort_flag; tile += tstep, phase ^= 1u) {
 #pragma unroll
-                    for (int k8 = 0; k8 < KOP / 8; ++k8) // 8 f32 = 32 bytes = 2 descriptor units per step
-                        umma_tf32(tmem_base + b * BN, adesc + (uint64_t)(2 * k8), bdesc + (uint64_t)(2 * k8), k8 ? 1u : 0u);
-                    umma_commit(&bars->aempty[st]);
-                    umma_commit(&bars->tfull[b]);
+                for (int h = 0; h < 2; ++h) {
+                    if (!(mine >> h & 1u) || !ok) continue;
+                    const int ss = 2 * acc + h;
+                    // the columns' last user: the other sub-space if it takes part (in this tile for h = 1), else this one in the tile before
+                    const int before = mine == 3u ? ss ^ 1 : ss;
+                    const uint32_t parity = (h == 1 && mine == 3u) ? phase : phase ^ 1u;
+                    if (!mbar_wait(&bars->afull[ss], phase, abort_flag, Q.error, 14) || !mbar_wait(&bars->tempty[2 * before + half], parity, abort_flag, Q.error, 13)) {
+                        ok = false;
+                        continue;
+                    }
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    if (leader) {
+                        const uint32_t o = (uint32_t)h; // 16 halves = 32 bytes = 2 descriptor units per step
+                        umma_f16_n128(td, smem_desc_sw64_at(a1 + o * (A1_BYTES<SD> >> 4)), smem_desc_sw64_at(b1 + o * (B1_BYTES<SD> >> 4)), 0u);
+                        umma_f16_n128(td, smem_desc_sw64_at(a1 + o * (A1_BYTES<SD> >> 4) + 2), smem_desc_sw64_at(b1 + o * (B1_BYTES<SD> >> 4) + 2), 1u);
+                        if (SL::STEPS == 3) umma_f16_n128(td, smem_desc_sw32_at(a2 + o * (A2_BYTES<SD> >> 4)), smem_desc_sw32_at(b2 + o * (B2_BYTES<SD> >> 4)), 1u);
+                        umma_commit(&bars->tfull[2 * ss + half]);
+                        umma_commit(&bars->aempty[ss]);
+                    }
+                    __syncwarp();
                 }
             }
         }
-    } else if (warp < 6) {
-        // ------------------------------------------------ operand A: split row slices into the ring
-        const int r = (warp - 2) * 32 + lane; // row of the tile
-        uint32_t it = 0;
-        float4 cur[8]; // the tile's four slices; each is requested again for the next tile as soon as it has been used
-        auto fetch = [&](int ss, unsigned long long tile) {
-            const unsigned long long row = tile * BM + r;
-            if (tile < n_tiles && row < P.n) {
-                const float4 *src = reinterpret_cast<const float4 *>(P.x + row * P.ld + (size_t)g * 32) + 2 * ss;
-                cur[2 * ss] = __ldg(src), cur[2 * ss + 1] = __ldg(src + 1);
-            } else {
-                cur[2 * ss] = cur[2 * ss + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+    } else if (warp < 12) {
+        // ------------------------------------------------ operand A: scaled and split row slices
+        const int r = (warp & 3) * 32 + lane; // row of the tile
+        const int pair = (warp - 4) >> 2;     // this warp's sub-spaces: 2 pair, 2 pair + 1
+        auto load_tile = [&](uint32_t tile, uint32_t buf) { // rows and columns beyond the matrix arrive as zeros
+            mbar_expect_tx(&bars->rfull[buf], RAW_BYTES<SD>);
+            tma_load_2d(raw_smem + buf * RAW_BYTES<SD>, &map_x, g * 4 * SD, (int)(tile * BM), &bars->rfull[buf]);
         };
-        if (nact > 0)
+        if (warp == 4 && lane == 0 && act) {
+            if (tile0 < n_tiles) load_tile(tile0, 0);
+            if (tile0 + tstep < n_tiles) load_tile(tile0 + tstep, 1);
+        }
+        __syncwarp();
+        uint32_t step = 0, buf = 0, rphase = 0; // tiles so far (parity: that of the stages); row-tile buffer and its parity
+        bool ok = true;
+        for (uint32_t tile = tile0; act && ok && tile < n_tiles && !*abort_flag; tile += tstep, ++step) {
+            if (!mbar_wait(&bars->rfull[buf], rphase, abort_flag, Q.error, 10)) break;
+            const unsigned char *raw = raw_smem + buf * RAW_BYTES<SD> + r * (16 * SD);
 #pragma unroll
-            for (int ss4 = 0; ss4 < 4; ++ss4) fetch(issue_order(ss4), tile0);
-        for (unsigned long long tile = tile0; nact > 0 && tile < n_tiles && !*abort_flag; tile += tstep) {
-            bool ok = true;
+            for (int h = 0; h < 2; ++h) {
+                const int ss = 2 * pair + h;
+                if (!(act >> ss & 1u) || !ok) continue;
+                const float *sub = sub_s + ss * SUB_FLOATS;
+                float y[SD];
 #pragma unroll
-            for (int ss4 = 0; ss4 < 4; ++ss4) { // static indexing of cur[]; issue order 0, 2, 1, 3
-                const int ss = issue_order(ss4);
-                if (pos_of(ss) == 15 || !ok) continue;
-                const int st = it % NSTAGE;
-                if (!mbar_wait(&bars->aempty[st], ((it / NSTAGE) & 1u) ^ 1u, abort_flag, Q.error, 11)) {
+                for (int c = 0; c < SD / 4; ++c) {
+                    const int chunk = ss * (SD / 4) + c;
+                    const float4 v = *reinterpret_cast<const float4 *>(raw + ((SD == 8 ? chunk ^ (r & 7) : chunk ^ ((r >> 1) & 3)) << 4));
+                    const float4 mu = COSINE ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4 *>(sub)[c];
+                    y[4 * c] = v.x - mu.x, y[4 * c + 1] = v.y - mu.y, y[4 * c + 2] = v.z - mu.z, y[4 * c + 3] = v.w - mu.w;
+                }
+                const RowFrame f = row_frame<SD, COSINE>(y, sub);
+                uint32_t hi[SD / 2], lo[SD / 2], cc, k0;
+#pragma unroll
+                for (int i = 0; i < SD / 2; ++i) {
+                    // |y mul| < 2^15: the multiple of 16 next to it and the rest (at most 8) are both binary16 numbers, the rest to 2^-9
+                    const float ah = fmaf(y[2 * i], f.mul, SPLIT) - SPLIT, bh = fmaf(y[2 * i + 1], f.mul, SPLIT) - SPLIT;
+                    hi[i] = pack_f16(ah, bh);
+                    lo[i] = pack_f16(fmaf(y[2 * i], f.mul, -ah), fmaf(y[2 * i + 1], f.mul, -bh));
+                }
+                cc = pack_f16(f.cr, f.cr);
+                k0 = DUMP ? 0u : pack_f16(2048.0f, f.k0);
+                if (!f.ok) {
+#pragma unroll
+                    for (int i = 0; i < SD / 2; ++i) hi[i] = lo[i] = 0u;
+                    cc = k0 = 0u;
+                }
+                if (!mbar_wait(&bars->aempty[ss], (step & 1u) ^ 1u, abort_flag, Q.error, 11)) {
                     ok = false;
                     continue;
                 }
-                const float4 v0 = cur[2 * ss], v1 = cur[2 * ss + 1];
-                const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-                fetch(ss, tile + tstep);
-                float hi[8], lo[8], sq = 0.0f;
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    hi[i] = split_tf32(v[i]);
-                    lo[i] = split_tf32(v[i] - hi[i]);
-                    sq = fmaf(v[i], v[i], sq);
+                unsigned char *row1 = a_smem + (size_t)ss * A1_BYTES<SD> + (size_t)r * 64;
+                const int s1 = (r >> 1) & 3;
+                if (SD == 4) {
+                    *reinterpret_cast<uint4 *>(row1 + ((0 ^ s1) << 4)) = make_uint4(hi[0], hi[1], hi[0], hi[1]);
+                    *reinterpret_cast<uint4 *>(row1 + ((1 ^ s1) << 4)) = make_uint4(lo[0], lo[1], cc, 0u);
+                    *reinterpret_cast<uint4 *>(row1 + ((2 ^ s1) << 4)) = make_uint4(k0, 0u, 0u, 0u);
+                } else {
+                    const uint4 h4 = make_uint4(hi[0], hi[1], hi[2 % (SD / 2)], hi[3 % (SD / 2)]);
+                    *reinterpret_cast<uint4 *>(row1 + ((0 ^ s1) << 4)) = h4;
+                    *reinterpret_cast<uint4 *>(row1 + ((1 ^ s1) << 4)) = h4;
+                    *reinterpret_cast<uint4 *>(row1 + ((2 ^ s1) << 4)) = make_uint4(lo[0], lo[1], lo[2 % (SD / 2)], lo[3 % (SD / 2)]);
+                    *reinterpret_cast<uint4 *>(row1 + ((3 ^ s1) << 4)) = make_uint4(cc, 0u, 0u, 0u);
+                    unsigned char *row2 = a_smem + 4 * (size_t)A1_BYTES<SD> + (size_t)ss * A2_BYTES<SD> + (size_t)r * 32;
+                    *reinterpret_cast<uint4 *>(row2 + (((r >> 2) & 1) << 4)) = make_uint4(k0, 0u, 0u, 0u);
                 }
-                unsigned char *rowp = a_smem + (size_t)st * A_STAGE_BYTES + (size_t)r * 128;
-                const int sw = r & 7;
-                const float4 h0 = make_float4(hi[0], hi[1], hi[2], hi[3]), h1 = make_float4(hi[4], hi[5], hi[6], hi[7]);
-                *reinterpret_cast<float4 *>(rowp + ((0 ^ sw) << 4)) = h0;
-                *reinterpret_cast<float4 *>(rowp + ((1 ^ sw) << 4)) = h1;
-                *reinterpret_cast<float4 *>(rowp + ((2 ^ sw) << 4)) = h0;
-                *reinterpret_cast<float4 *>(rowp + ((3 ^ sw) << 4)) = h1;
-                *reinterpret_cast<float4 *>(rowp + ((4 ^ sw) << 4)) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-                *reinterpret_cast<float4 *>(rowp + ((5 ^ sw) << 4)) = make_float4(lo[4], lo[5], lo[6], lo[7]);
-                *reinterpret_cast<float4 *>(rowp + ((6 ^ sw) << 4)) = make_float4(1.0f, 1.0f, 0.0f, 0.0f);
-                *reinterpret_cast<float4 *>(rowp + ((7 ^ sw) << 4)) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                float scale = 0.5f * sq;
-                if (COSINE) {
-                    const float nx = __fsqrt_rn(sq);
-                    scale = nx >= COS_MIN && nx <= COS_MAX ? 1.25f * nx : VQB_INF;
-                }
-                xh_ring[(it & (XH_RING - 1)) * BM + r] = scale;
+                if (__float_as_uint(sub[SUB_FLAGS]) & SUB_FAR) far_s[(ss * 4 + (step & 3u)) * BM + r] = (uint16_t)f.far;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic writes -> visible to the MMA's reads
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&bars->afull[st]);
-                ++it;
+                if (lane == 0) mbar_arrive(&bars->afull[ss]);
             }
             if (!ok) break;
+            // the row tile is used up: once all eight warps say so, its buffer takes the tile after the next
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->rempty[buf]);
+            if (warp == 4 && tile + 2 * tstep < n_tiles) {
+                ok = mbar_wait(&bars->rempty[buf], rphase, abort_flag, Q.error, 17);
+                if (ok && lane == 0) load_tile(tile + 2 * tstep, buf);
+                __syncwarp();
+            }
+            buf ^= 1u;
+            if (buf == 0) rphase ^= 1u;
         }
     } else {
-        // ------------------------------------------------ epilogue
-        const int q = warp & 3;           // TMEM lane quadrant
-        const int acc = (warp - 6) >> 2;  // team = accumulator: sub-spaces 2 acc, 2 acc + 1 of the group
-        const int nch = (k + 31) >> 5;    // 32-column chunks that hold centroids
-        const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)acc * BN;
-        const float hmax2_0 = 2.0f * Q.hnmax[g * 4 + acc * 2], hmax2_1 = 2.0f * Q.hnmax[g * 4 + acc * 2 + 1];
-        uint32_t uu = 0, tile_iter = 0, marked_pairs = 0, moved_mask = 0;
-        if (!TRAIN && nact > 0) mbar_wait(&bars->bfull, 0, abort_flag, Q.error, 16); // the f16 images arrive with operand B
-        for (unsigned long long tile = tile0; nact > 0 && tile < n_tiles && !*abort_flag; tile += tstep, ++tile_iter) {
-            const unsigned long long row = tile * BM + 32ull * q + lane;
-            const bool valid = row < P.n;
-            uint8_t *cp = reinterpret_cast<uint8_t *>(P.codes) + row * (unsigned long long)m + g * 4 + acc * 2;
-            uint32_t old2 = 0;
-            if (TRAIN && valid) old2 = *reinterpret_cast<const uint16_t *>(cp);
-            uint32_t idxs[2] = {0, 0}, done = 0, marked = 0;
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                const int ss = acc * 2 + h, s = g * 4 + ss;
-                if (pos_of(ss) == 15) continue;
-                const uint32_t it = tile_iter * (uint32_t)nact + (uint32_t)pos_of(ss);
-                if (!mbar_wait(&bars->tfull[acc], uu & 1u, abort_flag, Q.error, 15)) break;
-                ++uu;
+        // ------------------------------------------------ epilogue: team (warp - 12) / 4 serves that sub-space of the group
+        const int q = warp & 3; // TMEM lane quadrant
+        const int ss = (warp - 12) >> 2, s = g * 4 + ss;
+        const uint32_t taddr = tmem_base + ((uint32_t)(32 * q) << 16) + (uint32_t)(ss >> 1) * BN;
+        const float *sub = sub_s + ss * SUB_FLOATS;
+        uint4 *queue = queues + (warp - 12) * QCAP;
+        const bool any_far = (__float_as_uint(sub[SUB_FLAGS]) & SUB_FAR) != 0;
+        uint32_t waiting = 0; // entries in the queue
+        bool moved = false;
+        const bool on = act >> ss & 1u;
+        const uint32_t r = 32u * q + lane;
+        auto there = [&](uint32_t t) { return t + 1 < n_tiles || (t < n_tiles && r < last_rows); };
+        uint8_t *next_code = reinterpret_cast<uint8_t *>(P.codes) + ((unsigned long long)tile0 * BM + r) * m + s;
+        const unsigned long long code_step = (unsigned long long)tstep * BM * m;
+        // the previous code of a row is requested while the tile before it is decided: a trip to memory is longer than a unit
+        uint32_t next_old = 0;
+        if (TRAIN && on && there(tile0)) next_old = *next_code;
+        uint32_t step = 0; // tiles so far
+        for (uint32_t tile = tile0; on && tile < n_tiles && !*abort_flag; tile += tstep, ++step) {
+            const bool valid = there(tile);
+            uint8_t *cp = next_code;
+            const uint32_t old = next_old;
+            next_code += code_step;
+            if (TRAIN && there(tile + tstep)) next_old = *next_code;
+            uint32_t hb[16], ga[8];
+            bool ok = true;
+#pragma unroll
+            for (int half = 0; half < halves; ++half) {
+                if (!ok) continue;
+                if (!mbar_wait(&bars->tfull[2 * ss + half], step & 1u, abort_flag, Q.error, 15)) {
+                    ok = false;
+                    continue;
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (DUMP) { // diagnostic dump of the raw scores
-                    for (int c = 0; c < nch; ++c) {
-                        uint32_t v[32];
-                        tmem_ld32_issue(taddr + c * 32, v);
+                uint32_t v[32];
+                if (DUMP) { // diagnostic: the chain's result without the fixed-point constants, as scores
+                    const unsigned long long row = (unsigned long long)tile * BM + r;
+                    float x[SD], y[SD], shift = 0.0f;
+#pragma unroll
+                    for (int i = 0; i < SD; ++i) x[i] = y[i] = 0.0f;
+                    if (valid) load_slice<SD>(x, P.x + row * P.ld + (size_t)s * SD, true);
+#pragma unroll
+                    for (int i = 0; i < SD; ++i) {
+                        y[i] = x[i] - sub[i];
+                        shift = fmaf(sub[i], x[i] - 0.5f * sub[i], shift); // S = S' - y.mu - |mu|^2 / 2
+                    }
+                    const RowFrame f = row_frame<SD, COSINE>(y, sub);
+                    const float sigma = f.cr * sub[SUB_SCALE2];
+                    for (int c = 0; c < 4; ++c) {
+                        tmem_ld32_issue(taddr + half * 128 + c * 32, v);
                         tmem_wait();
                         if (valid) {
-                            float *o = Q.dbg_scores + ((size_t)row * m + s) * BN + c * 32;
+                            float *o = Q.dbg_scores + ((size_t)row * m + s) * BN + half * 128 + c * 32;
 #pragma unroll
-                            for (int t = 0; t < 32; ++t) o[t] = __uint_as_float(v[t]);
+                            for (int t = 0; t < 32; ++t) o[t] = half * 128 + c * 32 + t < k ? __uint_as_float(v[t]) / sigma - shift : 1e30f;
                         }
-                    }
-                }
-                const float xh2 = xh_ring[(it & (XH_RING - 1)) * BM + 32 * q + lane];
-                const float hmax2 = h ? hmax2_1 : hmax2_0;
-
-                // One pass over the scores, one 3-input minimum each: the minima of the 16 blocks of 16 consecutive columns and of the 16
-                // classes of columns equal modulo 16.  Straight-line code with a way out after every chunk: without these branches the
-                // chunks' loads were scheduled ahead and the scores spilled, with a test around every chunk each register of it was
-                // moved once more.
-                uint32_t idx = 0;
-                bool single = false;
-                {
-                    constexpr int N = 8;
-                    float hb[2 * N], ga[16];
-                    bool col0_nan = false;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) hb[i] = VQB_INF;
-#pragma unroll
-                    for (int c = 0; c < N; ++c) {
-                        uint32_t v[32];
-                        tmem_ld32_issue(taddr + c * 32, v);
-                        tmem_wait();
-                        if (c == 0) col0_nan = !(__uint_as_float(v[0]) == __uint_as_float(v[0]));
-#pragma unroll
-                        for (int t = 0; t < 16; ++t)
-                            ga[t] = c ? min3f(ga[t], __uint_as_float(v[t]), __uint_as_float(v[16 + t])) : fminf(__uint_as_float(v[t]), __uint_as_float(v[16 + t]));
-                        float b0 = __uint_as_float(v[0]), b1 = __uint_as_float(v[16]);
-#pragma unroll
-                        for (int t = 1; t < 15; t += 2) {
-                            b0 = min3f(b0, __uint_as_float(v[t]), __uint_as_float(v[t + 1]));
-                            b1 = min3f(b1, __uint_as_float(v[16 + t]), __uint_as_float(v[16 + t + 1]));
-                        }
-                        hb[2 * c] = fminf(b0, __uint_as_float(v[15]));
-                        hb[2 * c + 1] = fminf(b1, __uint_as_float(v[31]));
-                        if (c + 1 == nch) break;
-                    }
-                    // every score of this warp has been used: the accumulator may be overwritten
-                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&bars->tempty[acc]);
-                    float best = hb[0];
-#pragma unroll
-                    for (int i = 1; i < 2 * N - 1; i += 2) best = min3f(best, hb[i], hb[i + 1]);
-                    best = fminf(best, hb[2 * N - 1]);
-                    const float limit = best + (MARGIN_COEF * (xh2 + hmax2 + fabsf(best)) + 1e-36f);
-                    // Rows the test below cannot rank: NaN / infinity anywhere that matters, or values too small to scale (exponent of
-                    // the limit below -60; nor rows whose true distances could overflow f32: there the reference's comparisons see
-                    // infinities).
-                    const uint32_t eb = (__float_as_uint(limit) >> 23) & 0xFFu;
-                    const bool rankable = !col0_nan && eb - 67u < 188u && (xh2 + hmax2 < 1e37f);
-                    const float nbig = __uint_as_float(0x80000000u | ((314u - eb) << 23)); // -2^(60 - exponent(limit))
-                    const float lb = -limit * nbig;                                       // exact scaling
-                    // Sums of (1 + i / 512) over the blocks and over the classes whose minimum lies below the limit (the smallest
-                    // score's always does).  Both below 1.07, i.e. one block and one class <=> exactly one score lies below the limit:
-                    // two would differ in their block or in their class.  (1 + i / 512) + 16383 has i in its low mantissa bits.
-                    float tb0 = 0.0f, tb1 = 0.0f, ta0 = 0.0f, ta1 = 0.0f;
-#pragma unroll
-                    for (int i = 0; i < 2 * N; i += 2) {
-                        tb0 = fmaf(fma_sat(hb[i], nbig, lb), 1.0f + (float)i * 0.001953125f, tb0);
-                        tb1 = fmaf(fma_sat(hb[i + 1], nbig, lb), 1.0f + (float)(i + 1) * 0.001953125f, tb1);
-                    }
-#pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                        ta0 = fmaf(fma_sat(ga[i], nbig, lb), 1.0f + (float)i * 0.001953125f, ta0);
-                        ta1 = fmaf(fma_sat(ga[i + 1], nbig, lb), 1.0f + (float)(i + 1) * 0.001953125f, ta1);
-                    }
-                    const float tb = tb0 + tb1, ta = ta0 + ta1;
-                    idx = (__float_as_uint(tb + 16383.0f) & 15u) * 16 + (__float_as_uint(ta + 16383.0f) & 15u);
-                    single = rankable && fmaxf(tb, ta) < 1.07f && idx < (uint32_t)k;
-                }
-                if (h == 0) idxs[0] = idx;
-                else idxs[1] = idx;
-                done |= 1u << h;
-                if (!single) marked |= 1u << h;
-            }
-            if (valid && done) {
-                if (marked) Q.marks[row * (unsigned long long)(m >> 1) + g * 2 + acc] = (uint8_t)marked;
-                if (TRAIN) {
-                    if (done == 3u && marked == 0u) {
-                        const uint32_t nw = idxs[0] | (idxs[1] << 8);
-                        if (nw != old2) {
-                            if ((nw ^ old2) & 0xFFu) moved_mask |= 1u;
-                            if ((nw ^ old2) & 0xFF00u) moved_mask |= 2u;
-                            *reinterpret_cast<uint16_t *>(cp) = (uint16_t)nw;
-                        }
-                    } else {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            if (((done & ~marked) >> h & 1u) && ((old2 >> (8 * h)) & 0xFFu) != idxs[h]) {
-                                moved_mask |= 1u << h;
-                                cp[h] = (uint8_t)idxs[h];
-                            }
                     }
                 } else {
-                    const int dim = m * SDW;
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        if ((done & ~marked) >> h & 1u) {
-                            const int ss = acc * 2 + h, s = g * 4 + ss;
-                            const uint32_t idx = idxs[h];
-                            if (P.out_codes) P.out_codes[row * m + s] = idx;
-                            if (P.out_f16) // 16-byte aligned: dim % 8 == 0
-                                *reinterpret_cast<uint4 *>(P.out_f16 + row * dim + (size_t)s * SDW) = c16_s[ss * BN + idx];
-                            if (P.out_f32) {
-                                const float4 *c = reinterpret_cast<const float4 *>(P.centroids + ((size_t)s * k + idx) * SDW);
-                                float4 *o = reinterpret_cast<float4 *>(P.out_f32 + row * dim + (size_t)s * SDW);
-                                o[0] = __ldg(c);
-                                o[1] = __ldg(c + 1);
-                            }
-                        }
+                    tmem_ld32_pack16_issue(taddr + half * 128, v);
+                    tmem_wait();
+                    if (half == 0) fold64<true>(v, hb, ga);
+                    else fold64<false>(v, hb + 8, ga);
+                    tmem_ld32_pack16_issue(taddr + half * 128 + 64, v);
+                    tmem_wait();
                 }
-                marked_pairs += __popc(marked);
+                // the half is in registers: its columns may be overwritten
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->tempty[2 * ss + half]);
+                if (!DUMP) fold64<false>(v, hb + 8 * half + 4, ga);
+            }
+            if (!ok) break;
+            if (DUMP) continue;
+
+            uint32_t best2 = 0xFFFFFFFFu;
+            {
+                constexpr int NB = 8 * halves;
+                uint32_t b[NB / 3 + 1];
+#pragma unroll
+                for (int i = 0; i < NB / 3; ++i) b[i] = min3_u16x2(hb[3 * i], hb[3 * i + 1], hb[3 * i + 2]);
+                if (WIDE) best2 = min_u16x2(min3_u16x2(b[0], b[1], b[2]), min3_u16x2(b[3], b[NB / 3 - 1], hb[NB - 1]));
+                else best2 = min_u16x2(min3_u16x2(b[0], b[1], hb[6]), hb[7]);
+            }
+            const uint32_t best = min(best2 & 0xFFFFu, best2 >> 16);
+            const uint32_t minus = ((0u - best) & 0xFFFFu) * 0x10001u; // adding it: the distance from the best, never negative
+            constexpr uint32_t MM = SL::M * 0x10001u;
+            // Sums of weight * min(distance, M) over the blocks (weight W0 + block) and over the classes (W0 + class), both halves of a word
+            // at once.  What they lack of M times all weights is the sum of weight * (M - distance) over those within M: one with distance 0
+            // gives M weights, two or more at least W0 (M + 1) > M (W0 + 15).
+            constexpr uint32_t W0 = 16 * SL::M, NBLK = 8 * halves;
+            constexpr uint32_t WB = 2 * SL::M * (NBLK * W0 + NBLK * (NBLK - 1) / 2), WA = SL::M * (16 * W0 + 120);
+            uint32_t sb = 0, sb1 = 0, sa = 0, sa1 = 0;
+#pragma unroll
+            for (uint32_t i = 0; i < NBLK; i += 2) {
+                sb = __dp2a_lo(__viaddmin_u16x2(hb[i], minus, MM), (W0 + i) * 0x101u, sb);
+                sb1 = __dp2a_lo(__viaddmin_u16x2(hb[i + 1], minus, MM), (W0 + i + 1) * 0x101u, sb1);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 8; i += 2) {
+                sa = __dp2a_lo(__viaddmin_u16x2(ga[i], minus, MM), (W0 + 2 * i) + ((W0 + 2 * i + 1) << 8), sa);
+                sa1 = __dp2a_lo(__viaddmin_u16x2(ga[i + 1], minus, MM), (W0 + 2 * i + 2) + ((W0 + 2 * i + 3) << 8), sa1);
+            }
+            const uint32_t lb = WB - sb - sb1, la = WA - sa - sa1;
+            const uint32_t idx = ((lb / SL::M - W0) * 16u + (la / SL::M - W0)) & 0xFFu;
+            const bool whole = best == 0u || best >= T_HIGH; // nothing to tell apart, or nothing but padding: all centroids
+            bool single = max(lb, la) <= SL::M * (W0 + 15u) && idx < (uint32_t)k && !whole;
+            // a far centroid may be as close (the entry is written again four tiles on, which takes this unit's end)
+            const bool far = any_far && best + SL::M > far_s[(ss * 4 + (step & 3u)) * BM + r];
+            single = single && !far;
+            const bool later = valid && !single;
+            const uint32_t vote = __ballot_sync(0xffffffffu, later);
+            if (vote) {
+                // one bit per half of a word: min(distance, M) + (65536 - M) wraps to 0 for M and stays at least 1 otherwise
+                constexpr uint32_t LESS = (0x10000u - SL::M) * 0x10001u;
+                uint32_t blocks = 0, classes = 0;
+#pragma unroll
+                for (int c = 0; c < 2 * halves; ++c) { // four words at a time: eight bits, weighted by the bytes of dp2a
+                    uint32_t bits = 0;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) bits = __dp2a_lo(__viaddmin_u16x2(__viaddmin_u16x2(hb[4 * c + i], minus, MM), LESS, 0x10001u), 0x201u << (2 * i), bits);
+                    blocks |= bits << (8 * c);
+                }
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    uint32_t bits = 0;
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) bits = __dp2a_lo(__viaddmin_u16x2(__viaddmin_u16x2(ga[4 * c + i], minus, MM), LESS, 0x10001u), 0x201u << (2 * i), bits);
+                    classes |= bits << (8 * c);
+                }
+                if (later) queue[waiting + __popc(vote & ((1u << lane) - 1u))] = make_uint4(tile, r | (classes << 16), blocks, (whole ? Q_WHOLE : 0u) | (far ? Q_FAR : 0u));
+                waiting += __popc(vote);
+                __syncwarp();
+                if (waiting >= 32) {
+                    waiting -= 32;
+                    moved |= pq_queue_drain<SD, TRAIN, METRIC>(Q, queue + waiting, sub, 32, s, lane);
+                }
+            }
+            if (valid && single && (!TRAIN || idx != old)) {
+                moved = true;
+                *cp = (uint8_t)idx;
             }
         }
-        marked_pairs = __reduce_add_sync(0xffffffffu, marked_pairs);
-        if (marked_pairs && lane == 0) atomicAdd(Q.stats, (unsigned long long)marked_pairs);
-        if (TRAIN) {
-            moved_mask = __reduce_or_sync(0xffffffffu, moved_mask);
-            if (lane < 2 && (moved_mask >> lane & 1u)) atomicOr(P.changed + g * 4 + acc * 2 + lane, VQB_MOVED_BITS);
-        }
+        if (waiting) moved |= pq_queue_drain<SD, TRAIN, METRIC>(Q, queue, sub, (int)waiting, s, lane);
+        if (TRAIN && __any_sync(0xffffffffu, moved) && lane == 0) atomicOr(P.changed + s, VQB_MOVED_BITS);
     }
 
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -446,248 +659,283 @@ __global__ void __launch_bounds__(NTHREADS, 1) pq_tc_kernel(const __grid_constan
     }
 }
 
-// Operand B of one sub-space per block (thread j = centroid j): 32 TF32 numbers per centroid
-//   [-ch(8) | -cl(8) | -ch(8) | hn_h, hn_l, 0 ...]   (columns beyond k: zeros and a huge score),
-// the binary16 image of the centroid (what an encode writes, src/pq.rs:176-180) and max_j hn_j.
-// COSINE: the centroids' unit vectors, no half norms; the "largest half norm" is 0, or infinity to void the sub-space.
-template <bool COSINE> __global__ void pq_operand_b_kernel(const float *cb, int k, float *bop, uint4 *c16, float *hnmax)
+// The encode's outputs from its one-byte codes (codes [n][m]): thread = one (row, sub-space) pair at a time, neighbours in memory next
+// to each other, so that every store covers whole lines.  The images of the centroids (c16 [m][256][SD]) are gathered from shared memory
+// when they fit (TABLE): 16 bytes per lane from 32 different lines would take 32 cycles of the L1 cache.
+template <int SD, bool TABLE>
+__global__ void __launch_bounds__(512) pq_expand_kernel(const uint8_t *codes, unsigned long long pairs, int m, int k, const uint16_t *c16, const float *centroids,
+                                                        uint16_t *out_f16, uint32_t *out_codes, float *out_f32)
 {
-    __shared__ float smax[BN];
-    const int s = blockIdx.x, j = threadIdx.x;
-    float4 out[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    float hn = 0.0f;
-    uint4 img = make_uint4(0, 0, 0, 0);
-    if (j < k) {
-        const float4 *c = reinterpret_cast<const float4 *>(cb + ((size_t)s * k + j) * SDW);
-        const float4 c0 = c[0], c1 = c[1];
-        const float v[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-        float hi[8], lo[8], a = 0.0f;
-        if (COSINE) {
-            const float norm = norm_chain(v, 8, 1);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float unit = norm == 0.0f ? 0.0f : __fdiv_rn(v[i], norm);
-                hi[i] = to_tf32(unit);
-                lo[i] = to_tf32(unit - hi[i]);
-            }
-            hn = norm == 0.0f || !(norm == norm) || (norm >= COS_MIN && norm <= COS_MAX) ? 0.0f : VQB_INF; // a NaN score never wins
-        } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                hi[i] = to_tf32(v[i]);
-                lo[i] = to_tf32(v[i] - hi[i]);
-                a = fmaf(v[i], v[i], a);
-            }
-            hn = 0.5f * a;
-        }
-        const float hh = COSINE ? 0.0f : to_tf32(hn), hl = COSINE ? 0.0f : to_tf32(hn - hh);
-        out[0] = out[4] = make_float4(-hi[0], -hi[1], -hi[2], -hi[3]);
-        out[1] = out[5] = make_float4(-hi[4], -hi[5], -hi[6], -hi[7]);
-        out[2] = make_float4(-lo[0], -lo[1], -lo[2], -lo[3]);
-        out[3] = make_float4(-lo[4], -lo[5], -lo[6], -lo[7]);
-        out[6] = make_float4(hh, hl, 0.f, 0.f);
-        img.x = f32_to_f16_bits(v[0]) | ((uint32_t)f32_to_f16_bits(v[1]) << 16);
-        img.y = f32_to_f16_bits(v[2]) | ((uint32_t)f32_to_f16_bits(v[3]) << 16);
-        img.z = f32_to_f16_bits(v[4]) | ((uint32_t)f32_to_f16_bits(v[5]) << 16);
-        img.w = f32_to_f16_bits(v[6]) | ((uint32_t)f32_to_f16_bits(v[7]) << 16);
-    } else {
-        out[6] = make_float4(to_tf32(PAD_SCORE), 0.f, 0.f, 0.f);
-    }
-    float4 *o = reinterpret_cast<float4 *>(bop + ((size_t)s * BN + j) * KOP);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) o[i] = out[i];
-    c16[(size_t)s * BN + j] = img;
-    smax[j] = (j < k) ? fabsf(hn) : 0.0f;
-    __syncthreads();
-    for (int o2 = BN / 2; o2 > 0; o2 >>= 1) {
-        if (j < o2) smax[j] = fmaxf(smax[j], smax[j + o2]); // a NaN half norm is dropped here; its column scores NaN and is never counted
+    extern __shared__ __align__(16) uint16_t table[];
+    using Piece = typename std::conditional<SD == 4, uint2, uint4>::type; // SD halves
+    if (TABLE) {
+        for (uint32_t i = threadIdx.x; i < (uint32_t)m * BN * SD / 8; i += blockDim.x) reinterpret_cast<uint4 *>(table)[i] = __ldg(reinterpret_cast<const uint4 *>(c16) + i);
         __syncthreads();
     }
-    if (j == 0) hnmax[s] = smax[0];
+    const uint32_t step = (uint32_t)(((unsigned long long)gridDim.x * blockDim.x) % (uint32_t)m);
+    unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+    uint32_t s = (uint32_t)(i % (uint32_t)m);
+    for (; i < pairs; i += (unsigned long long)gridDim.x * blockDim.x) {
+        const uint32_t idx = codes[i];
+        if (out_codes) __stcs(out_codes + i, idx);
+        if (out_f16) __stcs(reinterpret_cast<Piece *>(out_f16) + i, reinterpret_cast<const Piece *>(TABLE ? table : c16)[s * BN + idx]);
+        if (out_f32) {
+#pragma unroll
+            for (int c = 0; c < SD / 4; ++c)
+                reinterpret_cast<float4 *>(out_f32)[i * (SD / 4) + c] = __ldg(reinterpret_cast<const float4 *>(centroids) + ((size_t)s * k + min(idx, (uint32_t)k - 1u)) * (SD / 4) + c);
+        }
+        s += step;
+        if (s >= (uint32_t)m) s -= (uint32_t)m;
+    }
 }
 
-// The marked (row, sub-space) pairs: one warp per pair scans all centroids with the reference's arithmetic
-// (src/utils.rs:59-73, src/pq.rs:159-182): strict '<' in ascending index from centroid 0, so a NaN distance never wins
-// unless it is centroid 0's, and equal distances keep the lowest index.
-template <bool TRAIN, int METRIC> __global__ void __launch_bounds__(256) pq_marked_kernel(const PqTcParams Q)
+// ------------------------------------------------------------------------------------------------
+// Operand B of one sub-space by one block of 256 threads (thread j = centroid j, v its values)
+// ------------------------------------------------------------------------------------------------
+template <int SD> struct OperandSmem {
+    float part[8][SD + 1];
+    float part1[8];
+};
+
+__device__ __forceinline__ float warp_sum(float v)
 {
-    // Each step a CTA reads 256 x 16 mark bytes (all loads independent), collects the marked pairs in shared memory --
-    // the list holds the worst case of a step -- and its eight warps then take the pairs in turn, so the work is balanced
-    // whatever the distribution of the marks.
-    __shared__ uint16_t s_list[256 * 16 * 2];
-    __shared__ float s_x[256][SDW];
-    __shared__ uint8_t s_old[256];
-    __shared__ uint32_t s_count;
-    const AssignParams &P = Q.a;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int m = P.m, k = P.k, half = m >> 1;
-    const unsigned long long total = P.n * (unsigned long long)half; // mark bytes; the buffer is zero-padded to 16
-    const unsigned long long total16 = (total + 15) / 16;
-    uint32_t moved_lo = 0, moved_hi = 0;
-    for (unsigned long long base = (unsigned long long)blockIdx.x * 256ull; base < total16; base += (unsigned long long)gridDim.x * 256ull) {
-        if (threadIdx.x == 0) s_count = 0u;
-        __syncthreads();
-        const unsigned long long mine = base + threadIdx.x;
-        if (mine < total16) {
-            const uint4 f = reinterpret_cast<const uint4 *>(Q.marks)[mine];
-            const uint32_t w[4] = {f.x, f.y, f.z, f.w};
-            // the map is handed back all zero, so the next launch needs no memset
-            if (f.x | f.y | f.z | f.w) reinterpret_cast<uint4 *>(Q.marks)[mine] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-            for (int wi = 0; wi < 4; ++wi) {
-                uint32_t word = w[wi];
-                while (word) {
-                    const int bit = __ffs(word) - 1; // bit (8 byte + h): pair h of mark byte `byte`
-                    word &= word - 1;
-                    if ((bit & 7) < 2) s_list[atomicAdd(&s_count, 1u)] = (uint16_t)((threadIdx.x * 16u + (uint32_t)(wi * 4 + (bit >> 3))) * 2u + (uint32_t)(bit & 7));
-                }
-            }
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// Row j of operand B (64 halves, see Slots), the binary16 image that an encode writes (src/pq.rs:176-180) and the sub-space's constants.
+template <int SD, bool COSINE>
+__device__ __forceinline__ void write_operand(const float (&v)[SD], int s, int k, float *scratch, OperandSmem<SD> &sm)
+{
+    using SL = Slots<SD>;
+    const int j = threadIdx.x, warp = j >> 5, lane = j & 31;
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < SD; ++i) finite = finite && fabsf(v[i]) < VQB_INF;
+    // A distance to a centroid that is not finite is never below another (src/utils.rs:66): its column is like one beyond k.  But the
+    // scan starts at centroid 0, and at a NaN it stays.
+    const bool mine = j < k && finite;
+    bool nan = false;
+#pragma unroll
+    for (int i = 0; i < SD; ++i) nan = nan || !(v[i] == v[i]);
+    const bool lost = __syncthreads_or(j == 0 && (COSINE ? !finite : nan)) != 0;
+    float y[SD], mu[SD], norm = 0.0f, rho = 0.0f, lim = 0.0f, half_norm = 0.0f;
+    bool far = false, void_sub = false;
+    if (COSINE) {
+        const float len = norm_chain(v, SD, 1);
+#pragma unroll
+        for (int i = 0; i < SD; ++i) {
+            mu[i] = 0.0f;
+            y[i] = mine && len != 0.0f ? __fdiv_rn(v[i], len) : 0.0f;
         }
-        __syncthreads();
-        const uint32_t cnt = s_count;
-        // rounds of up to 256 pairs: first every thread fetches one pair's row slice (and previous code) -- one trip to memory
-        // for the whole round instead of one per pair and warp -- then the warps take the pairs in turn
-        for (uint32_t r0 = 0; r0 < cnt; r0 += 256) {
-            const uint32_t rc = min(256u, cnt - r0);
-            if (threadIdx.x < rc) {
-                const uint32_t ent = s_list[r0 + threadIdx.x];
-                const unsigned long long e = base * 16ull + (ent >> 1);
-                if (e < total) {
-                    const unsigned long long row = e / half;
-                    const int rem = (int)(e % half);
-                    const int s = (rem >> 1) * 4 + (rem & 1) * 2 + (int)(ent & 1u);
-                    float x[SDW];
-                    load_slice<SDW>(x, P.x + row * P.ld + (size_t)s * SDW, P.x_vec4 != 0);
+        void_sub = lost || __syncthreads_or(mine && !(len == 0.0f || (len >= COS_MIN && len <= COS_MAX))) != 0;
+        rho = 1.000001f;
+    } else {
+        bool in = mine;
+#pragma unroll 1
+        for (int round = 0;; ++round) { // mu = the mean of those that are not far from it
+            const float cnt = warp_sum(in ? 1.0f : 0.0f);
 #pragma unroll
-                    for (int i = 0; i < SDW; ++i) s_x[threadIdx.x][i] = x[i];
-                    if (TRAIN) s_old[threadIdx.x] = reinterpret_cast<const uint8_t *>(P.codes)[row * (unsigned long long)m + s];
-                }
+            for (int i = 0; i < SD; ++i) {
+                const float t = warp_sum(in ? v[i] : 0.0f);
+                if (lane == 0) sm.part[warp][i] = t;
             }
+            if (lane == 0) sm.part[warp][SD] = cnt;
             __syncthreads();
-            for (uint32_t i = warp; i < rc; i += 8) {
-                const uint32_t ent = s_list[r0 + i];
-                const unsigned long long e = base * 16ull + (ent >> 1);
-                const int h = (int)(ent & 1u);
-                if (e >= total) continue;
-                const unsigned long long row = e / half;
-                const int rem = (int)(e % half);
-                const int s = (rem >> 1) * 4 + (rem & 1) * 2 + h;
-                float x[SDW];
+            float c = 0.0f;
 #pragma unroll
-                for (int t = 0; t < SDW; ++t) x[t] = s_x[i][t];
-                const float na = METRIC == M_COSINE ? norm_chain(x, SDW, 1) : 0.0f;
-                const float *cbs = P.centroids + (size_t)s * k * SDW;
-                float bd = VQB_INF, d0 = 0.0f;
-                int bi = 0x7fffffff;
-                float c[BN / 32][SDW]; // this lane's centroids j = lane, lane + 32, ...: all requested before the first is used
+            for (int w = 0; w < 8; ++w) c += sm.part[w][SD];
+            const float inv = __fdividef(1.0f, c);
+            float sq = 0.0f;
 #pragma unroll
-                for (int u = 0; u < BN / 32; ++u) {
-                    const int j = lane + 32 * u;
-                    if (j < k) {
-                        load_centroid<SDW>(c[u], cbs + (size_t)j * SDW);
-                    } else {
+            for (int i = 0; i < SD; ++i) {
+                float t = 0.0f;
 #pragma unroll
-                        for (int t = 0; t < SDW; ++t) c[u][t] = 0.0f;
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < BN / 32; ++u) {
-                    const int j = lane + 32 * u;
-                    float d = METRIC == M_COSINE ? reg_dist<SDW, M_COSINE>(x, c[u], 0.0f, na, norm_chain(c[u], SDW, 1))
-                                                 : reg_dist<SDW, M_SQ>(x, c[u], 0.0f, 0.0f, 0.0f);
-                    if (METRIC == M_EUCLID) d = __fsqrt_rn(d);
-                    if (j == 0) d0 = d;
-                    if (j < k && d < bd) {
-                        bd = d;
-                        bi = j;
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
-                    const float od = __shfl_xor_sync(0xffffffffu, bd, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                    if (od < bd || (od == bd && oi < bi)) {
-                        bd = od;
-                        bi = oi;
-                    }
-                }
-                d0 = __shfl_sync(0xffffffffu, d0, 0);
-                const int idx = (bi == 0x7fffffff || !(d0 == d0)) ? 0 : bi; // nothing below +inf, or the scan started at a NaN
-                if (lane == 0) {
-                    bool moved = false;
-                    if (TRAIN) {
-                        if (s_old[i] != (uint8_t)idx) {
-                            moved = true;
-                            reinterpret_cast<uint8_t *>(P.codes)[row * (unsigned long long)m + s] = (uint8_t)idx;
-                        }
-                    } else {
-                        store_result<SDW, uint8_t, TRAIN>(P, row, s, idx, cbs, moved);
-                    }
-                    if (moved) {
-                        if (s < 32) moved_lo |= 1u << s;
-                        else moved_hi |= 1u << (s - 32);
-                    }
-                }
+                for (int w = 0; w < 8; ++w) t += sm.part[w][i];
+                mu[i] = t * inv;
+                y[i] = mine ? v[i] - mu[i] : 0.0f;
+                sq = fmaf(y[i], y[i], sq);
             }
-            __syncthreads(); // the staged slices are rewritten by the next round
+            half_norm = 0.5f * sq;
+            norm = sqrt_approx(sq) * 1.000001f;
+            const float t = warp_sum(in ? norm : 0.0f);
+            if (lane == 0) sm.part1[warp] = t;
+            __syncthreads();
+            float sum = 0.0f;
+#pragma unroll
+            for (int w = 0; w < 8; ++w) sum += sm.part1[w];
+            lim = 4.0f * (sum * inv);
+            far = mine && !(norm <= lim);
+            const bool again = __syncthreads_or(in && far) != 0; // also: the partial sums may be overwritten
+            if (!again || round == 5) break;
+            in = mine && !far;
+            if (!__syncthreads_or(in)) break; // overflow: void below
         }
-        __syncthreads(); // the list is rewritten by the next step
+        float t = far ? 0.0f : norm;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t = fmaxf(t, __shfl_xor_sync(0xffffffffu, t, o));
+        if (lane == 0) sm.part1[warp] = t;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < 8; ++w) rho = fmaxf(rho, sm.part1[w]);
+        void_sub = lost || !(rho >= RHO_MIN && rho <= RHO_MAX && lim <= 4.0f * RHO_MAX);
     }
-    if (TRAIN && lane == 0) {
-        for (int s = 0; s < m; ++s)
-            if ((s < 32 ? moved_lo >> s : moved_hi >> (s - 32)) & 1u) atomicOr(P.changed + s, VQB_MOVED_BITS);
+    const uint32_t e = (__float_as_uint(rho) >> 23) & 0xFFu;                     // rho in [2^(e - 127), 2^(e - 126))
+    const float scale = void_sub ? 1.0f : __uint_as_float((255u - e) << 23);     // rho * scale in [2, 4)
+    constexpr int KROW = 16 * SL::STEPS;
+    uint16_t row[KROW];
+#pragma unroll
+    for (int i = 0; i < KROW; ++i) row[i] = 0;
+    const uint16_t one = 0x3C00u;
+    if (void_sub) {
+        // zeros: the rows' operands are zero as well, every column ties
+    } else if (!mine || far) {
+        row[SL::CONST] = f32_to_f16_bits(4096.0f + 28.0f); // 2048 * 28 = 57344
+    } else {
+#pragma unroll
+        for (int i = 0; i < SD; ++i) {
+            const float c = y[i] * scale;
+            const uint16_t h = f32_to_f16_bits(-c);
+            const uint16_t l = f32_to_f16_bits(-c - __half2float(__ushort_as_half(h)));
+            row[i] = row[2 * SD + i] = h;
+            row[SD + i] = l;
+        }
+        if (!COSINE) {
+            const float hn = half_norm * scale * scale;
+            row[SL::NORM] = f32_to_f16_bits(hn);
+            row[SL::NORM + 1] = f32_to_f16_bits(hn - __half2float(__ushort_as_half(row[SL::NORM])));
+        }
+        row[SL::CONST] = f32_to_f16_bits(4096.0f);
+        row[SL::CONST + 1] = one;
     }
+    uint4 *o1 = reinterpret_cast<uint4 *>(scratch + OFF_B1) + ((size_t)s * BN + j) * 4, *o2 = reinterpret_cast<uint4 *>(scratch + OFF_B2) + ((size_t)s * BN + j) * 2;
+#pragma unroll
+    for (int i = 0; i < KROW / 8; ++i) {
+        const uint16_t *w = row + 8 * i;
+        (i < 4 ? o1[i] : o2[i - 4]) = make_uint4(w[0] | ((uint32_t)w[1] << 16), w[2] | ((uint32_t)w[3] << 16), w[4] | ((uint32_t)w[5] << 16), w[6] | ((uint32_t)w[7] << 16));
+    }
+    uint16_t *img = reinterpret_cast<uint16_t *>(scratch + OFF_C16) + ((size_t)s * BN + j) * SD;
+#pragma unroll
+    for (int i = 0; i < SD; i += 4) {
+        uint2 w = make_uint2(0u, 0u);
+        if (j < k) {
+            w.x = f32_to_f16_bits(v[i]) | ((uint32_t)f32_to_f16_bits(v[i + 1]) << 16);
+            w.y = f32_to_f16_bits(v[i + 2]) | ((uint32_t)f32_to_f16_bits(v[i + 3]) << 16);
+        }
+        *reinterpret_cast<uint2 *>(img + i) = w;
+    }
+    float *sub = scratch + OFF_SUB + (size_t)s * SUB_FLOATS;
+    const uint32_t mask = __ballot_sync(0xffffffffu, far && !void_sub);
+    if (lane == 0) sub[SUB_MASK + warp] = __uint_as_float(mask);
+    const bool any_far = __syncthreads_or(far && !void_sub) != 0;
+    if (j == 0) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) sub[i] = void_sub || i >= SD ? 0.0f : mu[i % SD];
+        sub[SUB_RHO2] = 1.000001f * rho * rho;
+        sub[SUB_SCALE] = scale;
+        sub[SUB_SCALE2] = scale * scale;
+        sub[SUB_FLAGS] = __uint_as_float((void_sub ? SUB_VOID : 0u) | (any_far ? SUB_FAR : 0u) | (lost && !COSINE ? SUB_NAN0 : 0u));
+        sub[SUB_LIM] = 0.99999f * lim;
+    }
+}
+
+template <int SD> __device__ __forceinline__ void read_centroid(float (&v)[SD], const float *cb, int s, int k, int j)
+{
+    if (j < k) {
+        load_centroid<SD>(v, cb + ((size_t)s * k + j) * SD);
+    } else {
+#pragma unroll
+        for (int i = 0; i < SD; ++i) v[i] = 0.0f;
+    }
+}
+
+template <int SD, bool COSINE> __global__ void __launch_bounds__(BN) pq_operand_b_kernel(const float *cb, int k, float *scratch)
+{
+    __shared__ OperandSmem<SD> sm;
+    float v[SD];
+    read_centroid<SD>(v, cb, blockIdx.x, k, threadIdx.x);
+    write_operand<SD, COSINE>(v, blockIdx.x, k, scratch, sm);
 }
 
 } // namespace
 
 bool pq_tc_applicable(const AssignParams &p, int metric)
 {
-    return (metric == M_SQ || metric == M_EUCLID || metric == M_COSINE) && p.sd == SDW && p.m >= 4 && p.m <= MAXM && p.m % 4 == 0 && p.k >= 2 && p.k <= BN &&
-           p.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && p.n >= 1 && (reinterpret_cast<uintptr_t>(p.codes) & 1u) == 0 &&
+    return (metric == M_SQ || metric == M_EUCLID || metric == M_COSINE) && p.sd == 8 && p.m >= 4 && p.m <= MAXM && p.m % 4 == 0 && p.k >= 2 && p.k <= BN &&
+           p.n < (1ull << 32) && p.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && p.n >= 1 && (reinterpret_cast<uintptr_t>(p.codes) & 1u) == 0 &&
            (reinterpret_cast<uintptr_t>(p.centroids) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.out_f16) & 15u) == 0 &&
            (reinterpret_cast<uintptr_t>(p.out_f32) & 15u) == 0;
 }
 
 size_t pq_tc_scratch_floats() { return SCRATCH_FLOATS; }
 size_t pq_tc_stats_offset_floats() { return OFF_STATS; }
-size_t pq_tc_mark_bytes(size_t n, size_t m) { return (n * (m / 2) + 15) & ~(size_t)15; } // read 16 bytes at a time
+size_t pq_tc_code_bytes(size_t n, size_t m) { return n * m; }
 
-template <bool TRAIN, int METRIC, bool DUMP = false>
-static void launch_t(CudaDevice &dev, const CUtensorMap &mb, const PqTcParams &q, unsigned grid)
+struct PqMaps {
+    CUtensorMap x, b1, b2;
+};
+
+template <int SD, bool TRAIN, int METRIC, bool WIDE, bool DUMP = false>
+static void launch_w(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
 {
-    auto kernel = pq_tc_kernel<TRAIN, METRIC == M_COSINE, DUMP>;
-    constexpr size_t smem = PQ_TC_SMEM;
+    auto kernel = pq_tc_kernel<SD, TRAIN, METRIC, WIDE, DUMP>;
+    constexpr size_t smem = PQ_TC_SMEM<SD>;
     static std::atomic<unsigned long long> configured{0}; // bit d: the attribute has been set on device d (it is per device and sticky)
     const unsigned long long bit = 1ull << (dev.device() & 63);
     if (!(configured.load(std::memory_order_relaxed) & bit)) {
         VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured.fetch_or(bit, std::memory_order_relaxed);
     }
-    {
-        KernelScope ks(dev, TRAIN ? "assign_train" : "pq_encode");
-        kernel<<<grid, NTHREADS, smem, dev.stream()>>>(mb, q);
-        VQB_CUDA_CHECK(cudaGetLastError());
-        dev.count_launch();
-    }
-    {
-        KernelScope ks(dev, TRAIN ? "assign_train_marked" : "pq_encode_marked");
-        // one step (4 KiB of mark bytes) per CTA where the grid allows: the steps are latency-bound and independent
-        const unsigned long long steps = ((q.a.n * (unsigned long long)(q.a.m / 2) + 15) / 16 + 255) / 256;
-        const unsigned mgrid = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(steps, (unsigned long long)dev.sm_count() * 64));
-        pq_marked_kernel<TRAIN, METRIC><<<mgrid, 256, 0, dev.stream()>>>(q);
-        VQB_CUDA_CHECK(cudaGetLastError());
-        dev.count_launch();
-    }
+    KernelScope ks(dev, TRAIN ? "assign_train" : "pq_encode");
+    kernel<<<grid, NTHREADS, smem, dev.stream()>>>(mp.x, mp.b1, mp.b2, q);
+    VQB_CUDA_CHECK(cudaGetLastError());
+    dev.count_launch();
 }
 
-void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, bool cosine, float *scratch)
+template <int SD, bool TRAIN, int METRIC> static void launch_t(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
+{
+    if (q.a.k > 128) launch_w<SD, TRAIN, METRIC, true>(dev, mp, q, grid);
+    else launch_w<SD, TRAIN, METRIC, false>(dev, mp, q, grid);
+}
+
+template <int SD> static void launch_expand(CudaDevice &dev, const AssignParams &p, const uint16_t *c16)
+{
+    const size_t table = (size_t)p.m * BN * SD * sizeof(uint16_t);
+    const bool in_smem = table <= 100u * 1024u; // two CTAs of 512 threads per SM
+    auto kernel = in_smem ? pq_expand_kernel<SD, true> : pq_expand_kernel<SD, false>;
+    static std::atomic<unsigned long long> configured{0};
+    const unsigned long long bit = 1ull << (dev.device() & 63);
+    if (!(configured.load(std::memory_order_relaxed) & bit)) {
+        VQB_CUDA_CHECK(cudaFuncSetAttribute(pq_expand_kernel<SD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        configured.fetch_or(bit, std::memory_order_relaxed);
+    }
+    const unsigned long long pairs = p.n * (unsigned long long)p.m;
+    const unsigned grid = (unsigned)std::min<unsigned long long>((pairs + 511) / 512, (unsigned long long)dev.sm_count() * (in_smem ? 2 : 4));
+    KernelScope ks(dev, "pq_expand");
+    kernel<<<grid, 512, in_smem ? table : 0, dev.stream()>>>(reinterpret_cast<const uint8_t *>(p.codes), pairs, p.m, p.k, c16, p.centroids, p.out_f16, p.out_codes, p.out_f32);
+    VQB_CUDA_CHECK(cudaGetLastError());
+    dev.count_launch();
+}
+
+template <int SD> static void launch_sd(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid, int metric, bool train, const uint16_t *c16)
+{
+    if (q.dbg_scores) launch_w<SD, false, M_SQ, true, true>(dev, mp, q, grid);
+    if (train) {
+        launch_t<SD, true, M_SQ>(dev, mp, q, grid);
+        return;
+    }
+    if (metric == M_EUCLID) launch_t<SD, false, M_EUCLID>(dev, mp, q, grid);
+    else if (metric == M_COSINE) launch_t<SD, false, M_COSINE>(dev, mp, q, grid);
+    else launch_t<SD, false, M_SQ>(dev, mp, q, grid);
+    launch_expand<SD>(dev, q.a, c16);
+}
+
+void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, int sd, bool cosine, float *scratch)
 {
     KernelScope ks(dev, "pq_operand_b");
-    auto kernel = cosine ? pq_operand_b_kernel<true> : pq_operand_b_kernel<false>;
-    kernel<<<m, BN, 0, dev.stream()>>>(centroids, k, scratch + OFF_BOP, reinterpret_cast<uint4 *>(scratch + OFF_C16), scratch + OFF_HMAX);
+    auto kernel = sd == 4 ? (cosine ? pq_operand_b_kernel<4, true> : pq_operand_b_kernel<4, false>) : (cosine ? pq_operand_b_kernel<8, true> : pq_operand_b_kernel<8, false>);
+    kernel<<<m, BN, 0, dev.stream()>>>(centroids, k, scratch);
     VQB_CUDA_CHECK(cudaGetLastError());
     dev.count_launch();
 }
@@ -695,38 +943,48 @@ void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, 
 void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train, size_t code_bytes, const PqTcBuffers &b)
 {
     if (train && code_bytes != 1) throw Error(100, "pq tensor path: one-byte codes expected for k <= 256");
-    float *bop = b.scratch + OFF_BOP;
-    if (b.prepare_operand) launch_pq_operand_b(dev, p.centroids, p.m, p.k, metric == M_COSINE, b.scratch);
-    const CUtensorMap mb = make_tensor_map_2d(bop, KOP, (unsigned long long)p.m * BN, KOP, BN, CU_TENSOR_MAP_SWIZZLE_128B);
-    PqTcParams q;
+    if (b.prepare_operand) launch_pq_operand_b(dev, p.centroids, p.m, p.k, p.sd, metric == M_COSINE, b.scratch);
+    PqMaps mp;
+    // the rows as they lie: a box is one tile of a group's columns
+    mp.x = make_tensor_map_2d(p.x, (unsigned long long)p.m * p.sd, p.n, 4 * p.sd, BM, p.sd == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, p.ld);
+    mp.b1 = make_tensor_map_2d(reinterpret_cast<const uint16_t *>(b.scratch + OFF_B1), 32, (unsigned long long)p.m * BN, 32, BN, CU_TENSOR_MAP_SWIZZLE_64B);
+    mp.b2 = make_tensor_map_2d(reinterpret_cast<const uint16_t *>(b.scratch + OFF_B2), 16, (unsigned long long)p.m * BN, 16, BN, CU_TENSOR_MAP_SWIZZLE_32B);
+    PqTcParams q = {};
     q.a = p;
-    q.c16 = reinterpret_cast<uint4 *>(b.scratch + OFF_C16);
-    q.hnmax = b.scratch + OFF_HMAX;
-    q.marks = b.marks; // all zero between launches: the follow-up kernel clears what it reads
+    if (!train) q.a.codes = b.codes;
+    q.sub = b.scratch + OFF_SUB;
     q.stats = reinterpret_cast<unsigned long long *>(b.scratch + OFF_STATS);
     q.error = b.error_word;
     q.dbg_scores = b.dbg_scores;
+    // one CTA per SM, shared out among the groups of four sub-spaces by what they hold: the last one may have fewer than four
     const unsigned long long tiles = (p.n + BM - 1) / BM;
-    const unsigned ngroups = (unsigned)p.m / 4;
-    const unsigned per = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(tiles, (unsigned long long)dev.sm_count() / ngroups));
-    const unsigned grid = per * ngroups;
-    if (b.dbg_scores) launch_t<false, M_SQ, true>(dev, mb, q, grid);
-    else if (train) launch_t<true, M_SQ>(dev, mb, q, grid);
-    else if (metric == M_EUCLID) launch_t<false, M_EUCLID>(dev, mb, q, grid);
-    else if (metric == M_COSINE) launch_t<false, M_COSINE>(dev, mb, q, grid);
-    else launch_t<false, M_SQ>(dev, mb, q, grid);
+    const unsigned ngroups = ((unsigned)p.m + 3) / 4;
+    unsigned left = (unsigned)std::max(dev.sm_count(), (int)ngroups), subs = (unsigned)p.m, at = 0;
+    for (unsigned g = 0; g < ngroups; ++g) {
+        const unsigned here = std::min(4u, (unsigned)p.m - 4 * g);
+        const unsigned share = std::max(1u, std::min((left * here + subs / 2) / subs, left - (ngroups - 1 - g)));
+        q.first[g] = (uint16_t)at;
+        at += (unsigned)std::min<unsigned long long>(tiles, share);
+        left -= share;
+        subs -= here;
+    }
+    q.first[ngroups] = (uint16_t)at;
+    const uint16_t *c16 = reinterpret_cast<const uint16_t *>(b.scratch + OFF_C16);
+    if (p.sd == 4) launch_sd<4>(dev, mp, q, at, metric, train, c16);
+    else launch_sd<8>(dev, mp, q, at, metric, train, c16);
 }
 
 // ------------------------------------------------------------------------------------------------
 // Centroid update of one k-means iteration for the shapes this file serves, in one launch (one CTA per sub-space, thread j =
-// cluster j): centroid = sum / count (src/vector.rs:315-316), the operand-B row, binary16 image and largest half norm the next
+// cluster j): centroid = sum / count (src/vector.rs:315-316), the operand-B row, binary16 image and constants the next
 // assignment pass needs, the iteration's flags for the host, and the sums / counts / flags cleared for the next iteration.
 // ------------------------------------------------------------------------------------------------
+template <int SD>
 __global__ void __launch_bounds__(BN) pq_update_centroids_kernel(float *sums, uint32_t *counts, uint32_t *moved, int counts_f32, const uint32_t *active,
-                                                                 int k, float *centroids, float *bop, uint4 *c16, float *hnmax, StatusPage sp,
-                                                                 const PeerView pv)
+                                                                 int k, float *centroids, float *scratch, StatusPage sp, const PeerView pv)
 {
-    __shared__ float smax[BN];
+    constexpr int V = SD / 4;
+    __shared__ OperandSmem<SD> sm;
     const int s = blockIdx.x, j = threadIdx.x;
     const bool act = !active || active[s] != 0;
     const bool direct = pv.world > 1; // the parts of all ranks are added here, in rank order (peer_exchange.cuh)
@@ -736,102 +994,75 @@ __global__ void __launch_bounds__(BN) pq_update_centroids_kernel(float *sums, ui
     for (int q = 0; q < VQB_MAX_PEERS; ++q) mv_parts[q] = (direct && j == 0 && q < pv.world) ? peer_ld(pv.words[q] + pv.off_moved + s) : 0u;
     bool empty = false;
     if (act) {
-        float4 out[8];
+        float v[SD];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) out[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        float hn = 0.0f;
-        uint4 img = make_uint4(0, 0, 0, 0);
+        for (int i = 0; i < SD; ++i) v[i] = 0.0f;
         if (j < k) {
             const size_t cj = (size_t)s * k + j;
-            float4 *cp = reinterpret_cast<float4 *>(centroids + cj * SDW);
-            float4 *sp4 = reinterpret_cast<float4 *>(sums + cj * SDW);
-            float4 a, b;
+            float4 *cp = reinterpret_cast<float4 *>(centroids + cj * SD);
+            float4 *sp4 = reinterpret_cast<float4 *>(sums + cj * SD);
+            float4 a[V];
             float cf;
             if (direct) {
                 // Every peer load is issued before the first one is used.  A warp stops at the first instruction that needs a
                 // pending load, so "load rank q, add, load rank q + 1" pays one NVLink round trip (about 2 us) per rank:
                 // 30 us of a 44 us kernel at eight ranks.  The parts are then added in rank order as before.
-                float4 pa[VQB_MAX_PEERS], pb[VQB_MAX_PEERS];
+                float4 part[VQB_MAX_PEERS][V];
                 uint32_t pc[VQB_MAX_PEERS];
 #pragma unroll
                 for (int q = 0; q < VQB_MAX_PEERS; ++q) {
-                    pa[q] = pb[q] = make_float4(0.f, 0.f, 0.f, 0.f);
                     pc[q] = 0u;
+#pragma unroll
+                    for (int i = 0; i < V; ++i) part[q][i] = make_float4(0.f, 0.f, 0.f, 0.f);
                     if (q < pv.world) {
                         const uint32_t *w = pv.words[q];
-                        pa[q] = peer_ld4(w + cj * SDW);
-                        pb[q] = peer_ld4(w + cj * SDW + 4);
+#pragma unroll
+                        for (int i = 0; i < V; ++i) part[q][i] = peer_ld4(w + cj * SD + 4 * i);
                         pc[q] = peer_ld(w + pv.off_counts + cj);
                     }
                 }
                 uint32_t cnt = pc[0];
-                a = pa[0], b = pb[0];
+#pragma unroll
+                for (int i = 0; i < V; ++i) a[i] = part[0][i];
 #pragma unroll
                 for (int q = 1; q < VQB_MAX_PEERS; ++q) {
                     if (q < pv.world) {
                         cnt += pc[q];
-                        a.x = __fadd_rn(a.x, pa[q].x), a.y = __fadd_rn(a.y, pa[q].y), a.z = __fadd_rn(a.z, pa[q].z), a.w = __fadd_rn(a.w, pa[q].w);
-                        b.x = __fadd_rn(b.x, pb[q].x), b.y = __fadd_rn(b.y, pb[q].y), b.z = __fadd_rn(b.z, pb[q].z), b.w = __fadd_rn(b.w, pb[q].w);
+#pragma unroll
+                        for (int i = 0; i < V; ++i) {
+                            a[i].x = __fadd_rn(a[i].x, part[q][i].x), a[i].y = __fadd_rn(a[i].y, part[q][i].y);
+                            a[i].z = __fadd_rn(a[i].z, part[q][i].z), a[i].w = __fadd_rn(a[i].w, part[q][i].w);
+                        }
                     }
                 }
                 cf = __uint2float_rn(cnt);
-                float4 *st4 = reinterpret_cast<float4 *>(pv.stale + cj * SDW);
-                st4[0] = st4[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 *st4 = reinterpret_cast<float4 *>(pv.stale + cj * SD);
+#pragma unroll
+                for (int i = 0; i < V; ++i) st4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
                 pv.stale[pv.off_counts + cj] = 0u;
             } else {
                 const uint32_t cw = counts[cj];
                 cf = counts_f32 ? __uint_as_float(cw) : __uint2float_rn(cw);
-                a = sp4[0], b = sp4[1];
+#pragma unroll
+                for (int i = 0; i < V; ++i) a[i] = sp4[i];
             }
-            float4 c0, c1;
             if (cf != 0.0f) {
-                c0 = make_float4(__fdiv_rn(a.x, cf), __fdiv_rn(a.y, cf), __fdiv_rn(a.z, cf), __fdiv_rn(a.w, cf));
-                c1 = make_float4(__fdiv_rn(b.x, cf), __fdiv_rn(b.y, cf), __fdiv_rn(b.z, cf), __fdiv_rn(b.w, cf));
-                cp[0] = c0;
-                cp[1] = c1;
-                if (!direct) {
-                    sp4[0] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    sp4[1] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    counts[cj] = 0u;
+#pragma unroll
+                for (int i = 0; i < V; ++i) {
+                    a[i] = make_float4(__fdiv_rn(a[i].x, cf), __fdiv_rn(a[i].y, cf), __fdiv_rn(a[i].z, cf), __fdiv_rn(a[i].w, cf));
+                    cp[i] = a[i];
+                    if (!direct) sp4[i] = make_float4(0.f, 0.f, 0.f, 0.f);
                 }
+                if (!direct) counts[cj] = 0u;
             } else { // an empty cluster keeps its centroid until the host re-seeds it (src/utils.rs:99-101)
                 empty = true;
-                c0 = cp[0];
-                c1 = cp[1];
-            }
-            const float v[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-            float hi[8], lo[8], a2 = 0.0f;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                hi[i] = to_tf32(v[i]);
-                lo[i] = to_tf32(v[i] - hi[i]);
-                a2 = fmaf(v[i], v[i], a2);
+                for (int i = 0; i < V; ++i) a[i] = cp[i];
             }
-            hn = 0.5f * a2;
-            const float hh = to_tf32(hn), hl = to_tf32(hn - hh);
-            out[0] = out[4] = make_float4(-hi[0], -hi[1], -hi[2], -hi[3]);
-            out[1] = out[5] = make_float4(-hi[4], -hi[5], -hi[6], -hi[7]);
-            out[2] = make_float4(-lo[0], -lo[1], -lo[2], -lo[3]);
-            out[3] = make_float4(-lo[4], -lo[5], -lo[6], -lo[7]);
-            out[6] = make_float4(hh, hl, 0.f, 0.f);
-            img.x = f32_to_f16_bits(v[0]) | ((uint32_t)f32_to_f16_bits(v[1]) << 16);
-            img.y = f32_to_f16_bits(v[2]) | ((uint32_t)f32_to_f16_bits(v[3]) << 16);
-            img.z = f32_to_f16_bits(v[4]) | ((uint32_t)f32_to_f16_bits(v[5]) << 16);
-            img.w = f32_to_f16_bits(v[6]) | ((uint32_t)f32_to_f16_bits(v[7]) << 16);
-        } else {
-            out[6] = make_float4(to_tf32(PAD_SCORE), 0.f, 0.f, 0.f);
-        }
-        float4 *o = reinterpret_cast<float4 *>(bop + ((size_t)s * BN + j) * KOP);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = out[i];
-        c16[(size_t)s * BN + j] = img;
-        smax[j] = (j < k) ? fabsf(hn) : 0.0f;
-        __syncthreads();
-        for (int o2 = BN / 2; o2 > 0; o2 >>= 1) {
-            if (j < o2) smax[j] = fmaxf(smax[j], smax[j + o2]);
-            __syncthreads();
+            for (int i = 0; i < V; ++i) v[4 * i] = a[i].x, v[4 * i + 1] = a[i].y, v[4 * i + 2] = a[i].z, v[4 * i + 3] = a[i].w;
         }
-        if (j == 0) hnmax[s] = smax[0];
+        write_operand<SD, false>(v, s, k, scratch, sm);
     }
     // flags of this sub-space for the host: 8 bitmap words (bit = cluster without rows) and the "some row moved" word
     const uint32_t bits = __ballot_sync(0xffffffffu, empty);
@@ -851,12 +1082,12 @@ __global__ void __launch_bounds__(BN) pq_update_centroids_kernel(float *sums, ui
     }
 }
 
-void launch_pq_update_centroids(CudaDevice &dev, int m, int k, float *sums, uint32_t *counts, uint32_t *moved, bool counts_f32,
+void launch_pq_update_centroids(CudaDevice &dev, int m, int k, int sd, float *sums, uint32_t *counts, uint32_t *moved, bool counts_f32,
                                 const uint32_t *active, float *centroids, float *scratch, const StatusPage &sp, const PeerView &pv)
 {
     KernelScope ks(dev, "update_centroids");
-    pq_update_centroids_kernel<<<m, BN, 0, dev.stream()>>>(sums, counts, moved, counts_f32 ? 1 : 0, active, k, centroids, scratch + OFF_BOP,
-                                                            reinterpret_cast<uint4 *>(scratch + OFF_C16), scratch + OFF_HMAX, sp, pv);
+    auto kernel = sd == 4 ? pq_update_centroids_kernel<4> : pq_update_centroids_kernel<8>;
+    kernel<<<m, BN, 0, dev.stream()>>>(sums, counts, moved, counts_f32 ? 1 : 0, active, k, centroids, scratch, sp, pv);
     VQB_CUDA_CHECK(cudaGetLastError());
     dev.count_launch();
 }

@@ -11,9 +11,9 @@
 
 namespace vqb {
 
-// T: float, or uint16_t for binary16 bits
+// T: float, or uint16_t for binary16 bits.  ld: elements from row to row (0: the rows follow each other)
 template <typename T> inline CUtensorMap make_tensor_map_2d(const T *ptr, unsigned long long inner, unsigned long long rows, unsigned box_inner,
-                                      unsigned box_rows, CUtensorMapSwizzle swizzle)
+                                      unsigned box_rows, CUtensorMapSwizzle swizzle, unsigned long long ld = 0)
 {
     typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
                                       const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -29,7 +29,7 @@ template <typename T> inline CUtensorMap make_tensor_map_2d(const T *ptr, unsign
     if (!fn) throw Error(100, "cuTensorMapEncodeTiled is not available from this driver");
     CUtensorMap m;
     cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)inner * sizeof(T)};
+    cuuint64_t strides[1] = {(cuuint64_t)(ld ? ld : inner) * sizeof(T)};
     cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
     CUresult r = fn(&m, sizeof(T) == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<T *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
