@@ -20,15 +20,40 @@ def _check(oracle, cb, x, metric=(vq.Distance.Euclidean, ka.EUCLID)):
 
 
 @pytest.mark.parametrize("k", [2, 15, 16, 17, 63, 64, 65, 127, 128, 129, 192, 255, 256])
-@pytest.mark.parametrize("m", [4, 20])
-def test_edges_of_the_column_tiles(oracle, k, m):
+@pytest.mark.parametrize("m,sd", [(4, 8), (20, 8), (7, 8), (9, 4)])
+def test_edges_of_the_column_tiles(oracle, k, m, sd):
     rng = np.random.default_rng(k * 100 + m)
     n = 90_000 // m + 1  # past the one-launch path, a ragged last tile
-    x = rng.random((n, m * 8), dtype=np.float32)
-    cb = rng.random((m, k, 8), dtype=np.float32)
+    x = rng.random((n, m * sd), dtype=np.float32)
+    cb = rng.random((m, k, sd), dtype=np.float32)
     cb[1, k - 1] = cb[1, 0]                 # a tie between the first and the last column
-    x[n - 3:, 8:16] = cb[1, 0]
+    x[n - 3:, sd:2 * sd] = cb[1, 0]
     _check(oracle, cb, x)
+
+
+@pytest.mark.parametrize("m,sd", [(4, 4), (5, 8), (6, 4), (13, 8), (31, 4), (63, 8), (64, 4)])
+def test_groups_that_are_not_full(oracle, m, sd):
+    """Numbers of sub-spaces that leave the last group of a launch with one to three, both widths, against the oracle: encode with each
+    metric of the path (rows and outputs in host memory and on the GPU) and training."""
+    import torch
+
+    rng = np.random.default_rng(m * sd)
+    n, k = 90_000 // m + 77, 100
+    x = rng.normal(size=(n, m * sd)).astype(np.float32)
+    cb = rng.normal(size=(m, k, sd)).astype(np.float32)
+    for metric in ((vq.Distance.Euclidean, ka.EUCLID), (vq.Distance.SquaredEuclidean, ka.SQ), (vq.Distance.CosineDistance, ka.COSINE)):
+        _check(oracle, cb, x, metric)
+    q = vq.ProductQuantizer.from_codebooks(cb, vq.Distance.Euclidean)
+    out, codes = q.quantize(torch.from_numpy(x).cuda(), return_codes=True)
+    out_o, codes_o = oracle.pq_quantize(cb, x, ka.EUCLID)
+    assert np.array_equal(codes.cpu().numpy(), codes_o) and np.array_equal(out.cpu().numpy(), out_o.view(np.float16))
+    rows, iters = min(n, 3000), 5
+    so, sg = RecordingSeeder(7), RecordingSeeder(7)
+    init = so.init_pq(rows, m, k)
+    sg.init_pq(rows, m, k)
+    cb_o, _ = oracle.pq_fit(x[:rows], m, k, iters, init, so.draw)
+    pq = vq.ProductQuantizer.fit(x[:rows], m, k, iters, vq.Distance.Euclidean, 7, init_idx=init, draw=sg.draw, accumulate=vq.ACCUM_ORDERED)
+    assert np.array_equal(pq.codebooks, cb_o)
 
 
 CASES = ["far", "very_far", "many_far", "offset", "tight", "equal", "nan", "tiny", "huge", "far_rows"]

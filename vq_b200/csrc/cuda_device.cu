@@ -397,6 +397,7 @@ void CudaDevice::ensure_tc_buffers()
     VQB_CUDA_CHECK(cudaMalloc(&rot_split_, opq_tc_split_floats(128) * sizeof(float)));
     VQB_CUDA_CHECK(cudaMalloc(&pq_scratch_, pq_tc_scratch_floats() * sizeof(float)));
     VQB_CUDA_CHECK(cudaMemsetAsync(pq_scratch_, 0, pq_tc_scratch_floats() * sizeof(float), stream_));
+    pq_maps_.reset(new PqTcMaps(pq_tc_make_maps(pq_scratch_)));
     VQB_CUDA_CHECK(cudaMalloc(&tc_stats_, 3 * sizeof(unsigned long long)));
     VQB_CUDA_CHECK(cudaMemsetAsync(tc_stats_, 0, 3 * sizeof(unsigned long long), stream_));
     VQB_CUDA_CHECK(cudaMalloc(&tc_error_, sizeof(int)));
@@ -559,6 +560,7 @@ void CudaDevice::pq_tensor_debug(const float *x, size_t n, size_t m, const float
     download(&before, pq_scratch_ + pq_tc_stats_offset_floats(), sizeof before);
     PqTcBuffers tb;
     tb.scratch = pq_scratch_;
+    tb.maps = pq_maps_.get();
     tb.codes = pq_code_buffer(pq_tc_code_bytes(n, m));
     tb.error_word = tc_error_;
     tb.dbg_scores = scores;
@@ -710,6 +712,7 @@ void CudaDevice::assign_train(const Shape &sh, const float *x, const float *cent
     if (pq_tensor_enabled_ && pq_tc_applicable(p, M_SQ)) {
         PqTcBuffers tb;
         tb.scratch = pq_scratch_;
+        tb.maps = pq_maps_.get();
         tb.error_word = tc_error_;
         tb.prepare_operand = (bop_fresh_ != centroids);
         launch_pq_tc(*this, p, M_SQ, true, code_bytes(sh.k), tb);
@@ -744,7 +747,7 @@ bool CudaDevice::pq_encode_ahead(const Shape &sh, const float *x, const float *c
     p.centroids = codebooks;
     p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
     p.out_vec = !out_f16 || (aligned16(out_f16) && sh.m * sh.sd % 8 == 0);
-    if (sh.n_local == 0 || !pq_tensor_enabled_ || !pq_tc_applicable(p, metric) || direct_encode_applicable(p, true)) return false;
+    if (sh.n_local == 0 || !pq_tensor_enabled_ || !pq_tc_applicable(p, metric) || direct_encode_applicable(p, p.sd == 8 && p.m % 4 == 0)) return false;
     bop_fresh_ = nullptr;
     launch_pq_operand_b(*this, codebooks, p.m, p.k, p.sd, metric == M_COSINE, pq_scratch_);
     return true;
@@ -770,7 +773,8 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
     p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
     p.out_vec = (!out_f16 || (aligned16(out_f16) && dim % 8 == 0)) && (!out_f32 || (aligned16(out_f32) && dim % 4 == 0));
     const bool tensor = !cuda_cores_only && pq_tensor_enabled_ && pq_tc_applicable(p, metric);
-    if (direct_encode_applicable(p, tensor)) {
+    // (the lines of the one-launch kernel lie where it meets the other path; narrow or odd shapes keep that of the CUDA cores' kernels)
+    if (direct_encode_applicable(p, tensor && p.sd == 8 && p.m % 4 == 0)) {
         launch_direct_encode(*this, p, metric);
         return;
     }
@@ -779,6 +783,7 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
         PqTcBuffers tb;
         tb.prepare_operand = !operand_there;
         tb.scratch = pq_scratch_;
+        tb.maps = pq_maps_.get();
         tb.codes = pq_code_buffer(pq_tc_code_bytes(sh.n_local, sh.m));
         tb.error_word = tc_error_;
         launch_pq_tc(*this, p, metric, false, 4, tb);
@@ -1673,10 +1678,10 @@ void CudaDevice::update_centroids(const Shape &sh, const IterBuffers &buf, const
         return;
     }
     // shapes of the product-quantizer tensor kernel: the same launch writes the operand of the next assignment pass
-    const bool pq8 = pq_tensor_enabled_ && sh.sd == 8 && sh.m >= 4 && sh.m <= 64 && sh.m % 4 == 0 && k >= 2 && k <= 256 && pq_scratch_ != nullptr &&
+    const bool pq_shape = pq_tensor_enabled_ && pq_tc_shape(m, sh.sd, k) && pq_scratch_ != nullptr &&
                      (reinterpret_cast<uintptr_t>(centroids) & 15u) == 0 && (reinterpret_cast<uintptr_t>(buf.sums) & 15u) == 0;
     const PeerView pv = peer_view(px, sh, tc_error_);
-    if (pq8) {
+    if (pq_shape) {
         const StatusPage sp = status_page(m, k);
         launch_pq_update_centroids(*this, (int)m, (int)k, (int)sh.sd, buf.sums, buf.counts, buf.moved, buf.counts_f32, active, centroids, pq_scratch_, sp, pv);
         bop_fresh_ = centroids;

@@ -4,12 +4,14 @@
 
 #include <atomic>
 #include <map>
+#include <memory>
 #include <string>
 #include <vector>
 
 #include "backend.hpp"
 #include "dense_tc.hpp"
 #include "iter_status.cuh"
+#include "pq_tc.hpp"
 
 namespace vqb {
 
@@ -152,6 +154,7 @@ class CudaDevice : public Device {
                       unsigned long long *stats);
     void *try_alloc(size_t bytes); // null when there is no room
     float *pq_scratch_ = nullptr;
+    std::unique_ptr<PqTcMaps> pq_maps_; // of pq_scratch_
     uint8_t *pq_codes_ = nullptr;
     size_t pq_codes_cap_ = 0;
     uint8_t *pq_code_buffer(size_t bytes);

@@ -68,7 +68,7 @@
 //     half at once (0.49): more warps in flight count for more than the time a half stays occupied
 //   * rows by TMA, and 64- and 32-byte operand rows, which make room for them: loaded by the producers' lanes, 32 rows an
 //     instruction, they keep the L1 cache busy for 256 cycles a unit (0.40)
-//   * an encode leaves one byte per pair; pq_expand_kernel turns them into rows and 32-bit codes with whole-line stores, 0.08 ms
+//   * an encode leaves one byte per pair; pq_expand_kernel turns them into rows and 32-bit codes with whole-line stores, 0.06 ms
 //     (16-byte pieces stored from here: 0.49 in all)
 // The constant in a step of its own (K = 48) rather than beside the last products (K = 32): ten cut addends instead of one would
 // need M = 8 and triple the share of queued rows.
@@ -672,20 +672,31 @@ __global__ void __launch_bounds__(512) pq_expand_kernel(const uint8_t *codes, un
         for (uint32_t i = threadIdx.x; i < (uint32_t)m * BN * SD / 8; i += blockDim.x) reinterpret_cast<uint4 *>(table)[i] = __ldg(reinterpret_cast<const uint4 *>(c16) + i);
         __syncthreads();
     }
-    const uint32_t step = (uint32_t)(((unsigned long long)gridDim.x * blockDim.x) % (uint32_t)m);
-    unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
-    uint32_t s = (uint32_t)(i % (uint32_t)m);
-    for (; i < pairs; i += (unsigned long long)gridDim.x * blockDim.x) {
-        const uint32_t idx = codes[i];
-        if (out_codes) __stcs(out_codes + i, idx);
-        if (out_f16) __stcs(reinterpret_cast<Piece *>(out_f16) + i, reinterpret_cast<const Piece *>(TABLE ? table : c16)[s * BN + idx]);
-        if (out_f32) {
+    // eight codes are requested before the first is used: with one at a time a thread waits for memory once per pair (85 us for 1M x 16)
+    constexpr int U = 8;
+    const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+    const uint32_t step = (uint32_t)(stride % (uint32_t)m);
+    unsigned long long i0 = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+    uint32_t s = (uint32_t)(i0 % (uint32_t)m);
+    for (; i0 < pairs; i0 += U * stride) {
+        uint32_t idx[U];
 #pragma unroll
-            for (int c = 0; c < SD / 4; ++c)
-                reinterpret_cast<float4 *>(out_f32)[i * (SD / 4) + c] = __ldg(reinterpret_cast<const float4 *>(centroids) + ((size_t)s * k + min(idx, (uint32_t)k - 1u)) * (SD / 4) + c);
+        for (int u = 0; u < U; ++u) idx[u] = i0 + u * stride < pairs ? __ldcs(codes + i0 + u * stride) : 0u;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const unsigned long long i = i0 + u * stride;
+            if (i < pairs) {
+                if (out_codes) __stcs(out_codes + i, idx[u]);
+                if (out_f16) __stcs(reinterpret_cast<Piece *>(out_f16) + i, reinterpret_cast<const Piece *>(TABLE ? table : c16)[s * BN + idx[u]]);
+                if (out_f32) {
+#pragma unroll
+                    for (int c = 0; c < SD / 4; ++c)
+                        reinterpret_cast<float4 *>(out_f32)[i * (SD / 4) + c] = __ldg(reinterpret_cast<const float4 *>(centroids) + ((size_t)s * k + min(idx[u], (uint32_t)k - 1u)) * (SD / 4) + c);
+                }
+            }
+            s += step;
+            if (s >= (uint32_t)m) s -= (uint32_t)m;
         }
-        s += step;
-        if (s >= (uint32_t)m) s -= (uint32_t)m;
     }
 }
 
@@ -860,12 +871,16 @@ template <int SD, bool COSINE> __global__ void __launch_bounds__(BN) pq_operand_
 
 } // namespace
 
+// Every number of sub-spaces from four on: the last group of a launch may hold fewer than four, and gets as many CTAs as it has work.
+// Against the CUDA-core kernels (assign_filter.cuh), encode / fit of 5 iterations: 1M rows, 32 of 4: 4.05 -> 0.82 / 18.8 -> 5.2 ms;
+// 300,000 rows, 13 of 8: 0.79 -> 0.23 / 4.1 -> 1.6 ms; 100,000 rows, 7 of 4, k 100, cosine: 124 -> 38 us.
+bool pq_tc_shape(size_t m, size_t sd, size_t k) { return (sd == 4 || sd == 8) && m >= 4 && m <= MAXM && k >= 2 && k <= BN; }
+
 bool pq_tc_applicable(const AssignParams &p, int metric)
 {
-    return (metric == M_SQ || metric == M_EUCLID || metric == M_COSINE) && p.sd == 8 && p.m >= 4 && p.m <= MAXM && p.m % 4 == 0 && p.k >= 2 && p.k <= BN &&
-           p.n < (1ull << 32) && p.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && p.n >= 1 && (reinterpret_cast<uintptr_t>(p.codes) & 1u) == 0 &&
-           (reinterpret_cast<uintptr_t>(p.centroids) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.out_f16) & 15u) == 0 &&
-           (reinterpret_cast<uintptr_t>(p.out_f32) & 15u) == 0;
+    return (metric == M_SQ || metric == M_EUCLID || metric == M_COSINE) && pq_tc_shape(p.m, p.sd, p.k) && p.n >= 1 && p.n < (1ull << 32) &&
+           p.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.centroids) & 15u) == 0 &&
+           (reinterpret_cast<uintptr_t>(p.out_f16) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.out_f32) & 15u) == 0;
 }
 
 size_t pq_tc_scratch_floats() { return SCRATCH_FLOATS; }
@@ -902,16 +917,17 @@ template <int SD, bool TRAIN, int METRIC> static void launch_t(CudaDevice &dev, 
 template <int SD> static void launch_expand(CudaDevice &dev, const AssignParams &p, const uint16_t *c16)
 {
     const size_t table = (size_t)p.m * BN * SD * sizeof(uint16_t);
-    const bool in_smem = table <= 100u * 1024u; // two CTAs of 512 threads per SM
+    const bool in_smem = table <= 200u * 1024u;
     auto kernel = in_smem ? pq_expand_kernel<SD, true> : pq_expand_kernel<SD, false>;
     static std::atomic<unsigned long long> configured{0};
     const unsigned long long bit = 1ull << (dev.device() & 63);
     if (!(configured.load(std::memory_order_relaxed) & bit)) {
-        VQB_CUDA_CHECK(cudaFuncSetAttribute(pq_expand_kernel<SD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        VQB_CUDA_CHECK(cudaFuncSetAttribute(pq_expand_kernel<SD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         configured.fetch_or(bit, std::memory_order_relaxed);
     }
     const unsigned long long pairs = p.n * (unsigned long long)p.m;
-    const unsigned grid = (unsigned)std::min<unsigned long long>((pairs + 511) / 512, (unsigned long long)dev.sm_count() * (in_smem ? 2 : 4));
+    const unsigned per_sm = in_smem ? (unsigned)std::min<size_t>(4, 200u * 1024u / table) : 4u;
+    const unsigned grid = (unsigned)std::min<unsigned long long>((pairs + 511) / 512, (unsigned long long)dev.sm_count() * per_sm);
     KernelScope ks(dev, "pq_expand");
     kernel<<<grid, 512, in_smem ? table : 0, dev.stream()>>>(reinterpret_cast<const uint8_t *>(p.codes), pairs, p.m, p.k, c16, p.centroids, p.out_f16, p.out_codes, p.out_f32);
     VQB_CUDA_CHECK(cudaGetLastError());
@@ -940,15 +956,22 @@ void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, 
     dev.count_launch();
 }
 
+PqTcMaps pq_tc_make_maps(const float *scratch)
+{
+    PqTcMaps maps;
+    maps.b1 = make_tensor_map_2d(reinterpret_cast<const uint16_t *>(scratch + OFF_B1), 32, (unsigned long long)MAXM * BN, 32, BN, CU_TENSOR_MAP_SWIZZLE_64B);
+    maps.b2 = make_tensor_map_2d(reinterpret_cast<const uint16_t *>(scratch + OFF_B2), 16, (unsigned long long)MAXM * BN, 16, BN, CU_TENSOR_MAP_SWIZZLE_32B);
+    return maps;
+}
+
 void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train, size_t code_bytes, const PqTcBuffers &b)
 {
     if (train && code_bytes != 1) throw Error(100, "pq tensor path: one-byte codes expected for k <= 256");
     if (b.prepare_operand) launch_pq_operand_b(dev, p.centroids, p.m, p.k, p.sd, metric == M_COSINE, b.scratch);
     PqMaps mp;
+    mp.b1 = b.maps->b1, mp.b2 = b.maps->b2;
     // the rows as they lie: a box is one tile of a group's columns
     mp.x = make_tensor_map_2d(p.x, (unsigned long long)p.m * p.sd, p.n, 4 * p.sd, BM, p.sd == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, p.ld);
-    mp.b1 = make_tensor_map_2d(reinterpret_cast<const uint16_t *>(b.scratch + OFF_B1), 32, (unsigned long long)p.m * BN, 32, BN, CU_TENSOR_MAP_SWIZZLE_64B);
-    mp.b2 = make_tensor_map_2d(reinterpret_cast<const uint16_t *>(b.scratch + OFF_B2), 16, (unsigned long long)p.m * BN, 16, BN, CU_TENSOR_MAP_SWIZZLE_32B);
     PqTcParams q = {};
     q.a = p;
     if (!train) q.a.codes = b.codes;

@@ -3,6 +3,8 @@
 #include <cstddef>
 #include <cstdint>
 
+#include <cuda.h>
+
 #include "iter_status.cuh"
 #include "peer_exchange.cuh"
 
@@ -11,15 +13,24 @@ namespace vqb {
 class CudaDevice;
 struct AssignParams;
 
-// sub-space width 8, 4 <= m <= 64 (multiple of 4), 2 <= k <= 256, 16-byte aligned row slices, Euclidean metrics or (encode) cosine
+// sub-space widths 4 and 8, 4 <= m <= 64, 2 <= k <= 256: what the kernels and the fused centroid update take ...
+bool pq_tc_shape(size_t m, size_t sd, size_t k);
+// ... with 16-byte aligned row slices, for the Euclidean metrics or (encode) cosine
 bool pq_tc_applicable(const AssignParams &p, int metric);
 size_t pq_tc_scratch_floats();
 // bytes of the one-byte codes that an encode of n rows of m sub-spaces goes through
 size_t pq_tc_code_bytes(size_t n, size_t m);
 
+// How TMA reads operand B from the scratch memory; made once for it.
+struct PqTcMaps {
+    CUtensorMap b1, b2;
+};
+PqTcMaps pq_tc_make_maps(const float *scratch);
+
 // Device memory one launch works with besides its inputs and outputs.
 struct PqTcBuffers {
     float *scratch = nullptr;     // pq_tc_scratch_floats() floats, zero-filled once: operand B, binary16 images, constants, statistics
+    const PqTcMaps *maps = nullptr; // of scratch
     uint8_t *codes = nullptr;     // encode: pq_tc_code_bytes(n, m) bytes of working memory
     int *error_word = nullptr;    // set when a bounded wait expires
     bool prepare_operand = true;  // false: scratch already holds operand B of p.centroids (written by launch_pq_update_centroids)
