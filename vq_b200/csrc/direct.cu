@@ -187,7 +187,7 @@ template <int METRIC, int R> __global__ void __launch_bounds__(DT, 3) direct_ker
 #pragma unroll
         for (int r = 0; r < R; ++r) a0[r] = a1[r] = 0.0f, p0[r] = p1[r] = 0ull;
         for (int ch = 0; ch < nch; ++ch) {
-            if (P.tma) mbar_wait(&s_full[slot], phase, &s_abort, P.error, 21, 200u);
+            if (P.tma) mbar_wait<200u>(&s_full[slot], phase, &s_abort, P.error, 21);
             else asm volatile("cp.async.wait_group %0;" ::"n"(NBUF - 2) : "memory");
             __syncthreads(); // this chunk is there for everybody, and the one before is used up
             load_chunk();

@@ -57,8 +57,8 @@
 //   warps 12-27  epilogue: a team of four warps per sub-space (one row per lane, one TMEM lane quadrant per warp)
 // Every wait is bounded; on expiry the CTA records a code, stops issuing, frees tensor memory and the host raises an error.
 //
-// Measured, 1M x 128, m 16, k 256: a training pass 0.643 (0.613 and 0.030 for the pairs left to an exact kernel) -> 0.40 ms, an
-// encode 0.698 -> 0.47 ms, against f32 scores of split-TF32 operands with one f32 minimum each.  Per unit 930 cycles; the parts
+// Measured, 1M x 128, m 16, k 256: a training pass 0.643 (0.613 and 0.030 for the pairs left to an exact kernel) -> 0.38 ms, an
+// encode 0.682 -> 0.43 ms, against f32 scores of split-TF32 operands with one f32 minimum each.  Per unit 880 cycles; the parts
 // alone: hand-over of the barriers 500, with the producers 720, with the epilogue 860; the MMAs take 385, the minima 256 of a
 // scheduler's integer pipe.  What each choice brought (ms a pass, the others as they are):
 //   * one issuer per accumulator half instead of one per accumulator (0.46), and those instead of one in all (0.71): a half is idle
@@ -96,7 +96,7 @@ constexpr float CR_MIN = 6.2e-5f;             // below: no longer a normal binar
 constexpr float SPLIT = 1.5f * 134217728.0f;  // 1.5 2^27: adding it rounds to a multiple of 16
 constexpr uint32_t T_HIGH = 57344u - 16u;     // the padding columns' T, less the window
 
-// per-sub-space constants (32 floats): mu[16], then
+// per-sub-space constants (32 floats): -mu[16], then
 constexpr int SUB_RHO2 = 16, SUB_SCALE = 17, SUB_SCALE2 = 18, SUB_FLAGS = 19, SUB_LIM = 20, SUB_MASK = 24, SUB_FLOATS = 32;
 constexpr uint32_t SUB_VOID = 1u, SUB_FAR = 2u, SUB_NAN0 = 4u; // NAN0: every distance to centroid 0 is NaN, where the scan starts and stays
 
@@ -157,6 +157,35 @@ __device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b)
 
 __device__ __forceinline__ uint32_t min3_u16x2(uint32_t a, uint32_t b, uint32_t c) { return __vimin3_u16x2(a, b, c); } // one instruction on sm_100
 
+// two f32 numbers in one register pair, and what the FMA pipe does with both at once
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 pair2(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float lo2(F2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float hi2(F2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 __device__ __forceinline__ float sqrt_approx(float v)
 {
     float r;
@@ -175,12 +204,10 @@ struct RowFrame {
     bool ok;
 };
 
-template <int SD, bool COSINE> __device__ __forceinline__ RowFrame row_frame(const float (&y)[SD], const float *sub)
+// sq = |x - mu|^2
+template <bool COSINE> __device__ __forceinline__ RowFrame row_frame(float sq, const float *sub)
 {
     RowFrame f;
-    float sq = 0.0f;
-#pragma unroll
-    for (int i = 0; i < SD; ++i) sq = fmaf(y[i], y[i], sq);
     const float4 c = *reinterpret_cast<const float4 *>(sub + SUB_RHO2); // rho^2 (rounded up), scale, scale^2, flags
     const uint32_t flags = __float_as_uint(c.w);
     float low, sigma;
@@ -396,7 +423,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             const uint32_t b2 = (smem_u32(b_smem) + 4 * B1_BYTES<SD> + 2 * acc * B2_BYTES<SD> + half * (B2_BYTES<SD> / 2)) >> 4;
             const uint32_t td = tmem_base + acc * BN + half * 128;
             uint32_t phase = 0; // parity of the tile's phases
-            for (uint32_t tile = tile0; ok && tile < n_tiles && !*abort_flag; tile += tstep, phase ^= 1u) {
+            for (uint32_t tile = tile0; ok && tile < n_tiles; tile += tstep, phase ^= 1u) { // (after an abort the next wait fails)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     if (!(mine >> h & 1u) || !ok) continue;
@@ -436,7 +463,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         __syncwarp();
         uint32_t step = 0, buf = 0, rphase = 0; // tiles so far (parity: that of the stages); row-tile buffer and its parity
         bool ok = true;
-        for (uint32_t tile = tile0; act && ok && tile < n_tiles && !*abort_flag; tile += tstep, ++step) {
+        for (uint32_t tile = tile0; act && ok && tile < n_tiles; tile += tstep, ++step) {
             if (!mbar_wait(&bars->rfull[buf], rphase, abort_flag, Q.error, 10)) break;
             const unsigned char *raw = raw_smem + buf * RAW_BYTES<SD> + r * (16 * SD);
 #pragma unroll
@@ -444,29 +471,37 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 const int ss = 2 * pair + h;
                 if (!(act >> ss & 1u) || !ok) continue;
                 const float *sub = sub_s + ss * SUB_FLOATS;
-                float y[SD];
+                // two values per instruction where the FMA pipe has one (add, fma .f32x2)
+                F2 y[SD / 2];
 #pragma unroll
                 for (int c = 0; c < SD / 4; ++c) {
                     const int chunk = ss * (SD / 4) + c;
-                    const float4 v = *reinterpret_cast<const float4 *>(raw + ((SD == 8 ? chunk ^ (r & 7) : chunk ^ ((r >> 1) & 3)) << 4));
-                    const float4 mu = COSINE ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4 *>(sub)[c];
-                    y[4 * c] = v.x - mu.x, y[4 * c + 1] = v.y - mu.y, y[4 * c + 2] = v.z - mu.z, y[4 * c + 3] = v.w - mu.w;
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(raw + ((SD == 8 ? chunk ^ (r & 7) : chunk ^ ((r >> 1) & 3)) << 4));
+                    y[2 * c] = v.x, y[2 * c + 1] = v.y;
+                    if (!COSINE) {
+                        const ulonglong2 mu = reinterpret_cast<const ulonglong2 *>(sub)[c]; // the mean with its sign changed
+                        y[2 * c] = add2(y[2 * c], mu.x), y[2 * c + 1] = add2(y[2 * c + 1], mu.y);
+                    }
                 }
-                const RowFrame f = row_frame<SD, COSINE>(y, sub);
+                F2 sq2 = mul2(y[0], y[0]);
+#pragma unroll
+                for (int i = 1; i < SD / 2; ++i) sq2 = fma2(y[i], y[i], sq2);
+                const RowFrame f = row_frame<COSINE>(lo2(sq2) + hi2(sq2), sub);
                 uint32_t hi[SD / 2], lo[SD / 2], cc, k0;
+                const F2 mul = pair2(f.mul, f.mul), up = pair2(SPLIT, SPLIT), down = pair2(-SPLIT, -SPLIT);
 #pragma unroll
                 for (int i = 0; i < SD / 2; ++i) {
                     // |y mul| < 2^15: the multiple of 16 next to it and the rest (at most 8) are both binary16 numbers, the rest to 2^-9
-                    const float ah = fmaf(y[2 * i], f.mul, SPLIT) - SPLIT, bh = fmaf(y[2 * i + 1], f.mul, SPLIT) - SPLIT;
-                    hi[i] = pack_f16(ah, bh);
-                    lo[i] = pack_f16(fmaf(y[2 * i], f.mul, -ah), fmaf(y[2 * i + 1], f.mul, -bh));
+                    const F2 head = add2(fma2(y[i], mul, up), down);
+                    hi[i] = pack_f16(lo2(head), hi2(head));
+                    lo[i] = pack_f16(fmaf(lo2(y[i]), f.mul, -lo2(head)), fmaf(hi2(y[i]), f.mul, -hi2(head)));
                 }
                 cc = pack_f16(f.cr, f.cr);
                 k0 = DUMP ? 0u : pack_f16(2048.0f, f.k0);
-                if (!f.ok) {
+                if (__any_sync(0xffffffffu, !f.ok)) { // (rarely: a vote instead of a select per word)
 #pragma unroll
-                    for (int i = 0; i < SD / 2; ++i) hi[i] = lo[i] = 0u;
-                    cc = k0 = 0u;
+                    for (int i = 0; i < SD / 2; ++i) hi[i] = f.ok ? hi[i] : 0u, lo[i] = f.ok ? lo[i] : 0u;
+                    cc = f.ok ? cc : 0u, k0 = f.ok ? k0 : 0u;
                 }
                 if (!mbar_wait(&bars->aempty[ss], (step & 1u) ^ 1u, abort_flag, Q.error, 11)) {
                     ok = false;
@@ -516,19 +551,18 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         bool moved = false;
         const bool on = act >> ss & 1u;
         const uint32_t r = 32u * q + lane;
-        auto there = [&](uint32_t t) { return t + 1 < n_tiles || (t < n_tiles && r < last_rows); };
-        uint8_t *next_code = reinterpret_cast<uint8_t *>(P.codes) + ((unsigned long long)tile0 * BM + r) * m + s;
-        const unsigned long long code_step = (unsigned long long)tstep * BM * m;
+        const uint32_t n_steps = tile0 < n_tiles ? (n_tiles - tile0 + tstep - 1) / tstep : 0u; // tiles of this CTA
+        const bool in_last = r < (tile0 + (n_steps - 1) * tstep == n_tiles - 1 ? last_rows : (uint32_t)BM);
+        auto there = [&](uint32_t t) { return t + 1 < n_steps || (t < n_steps && in_last); };
+        uint8_t *code = reinterpret_cast<uint8_t *>(P.codes) + ((unsigned long long)tile0 * BM + r) * m + s; // this lane's row of the tile
+        const uint32_t code_step = tstep * BM * (uint32_t)m;
         // the previous code of a row is requested while the tile before it is decided: a trip to memory is longer than a unit
         uint32_t next_old = 0;
-        if (TRAIN && on && there(tile0)) next_old = *next_code;
-        uint32_t step = 0; // tiles so far
-        for (uint32_t tile = tile0; on && tile < n_tiles && !*abort_flag; tile += tstep, ++step) {
-            const bool valid = there(tile);
-            uint8_t *cp = next_code;
+        if (TRAIN && on && there(0)) next_old = *code;
+        for (uint32_t step = 0; on && step < n_steps; ++step, code += code_step) {
+            const bool valid = there(step);
             const uint32_t old = next_old;
-            next_code += code_step;
-            if (TRAIN && there(tile + tstep)) next_old = *next_code;
+            if (TRAIN && there(step + 1)) next_old = code[code_step];
             uint32_t hb[16], ga[8];
             bool ok = true;
 #pragma unroll
@@ -541,17 +575,18 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t v[32];
                 if (DUMP) { // diagnostic: the chain's result without the fixed-point constants, as scores
-                    const unsigned long long row = (unsigned long long)tile * BM + r;
-                    float x[SD], y[SD], shift = 0.0f;
+                    const unsigned long long row = (unsigned long long)(tile0 + step * tstep) * BM + r;
+                    float x[SD], sq[2] = {0.0f, 0.0f}, shift = 0.0f;
 #pragma unroll
-                    for (int i = 0; i < SD; ++i) x[i] = y[i] = 0.0f;
+                    for (int i = 0; i < SD; ++i) x[i] = 0.0f;
                     if (valid) load_slice<SD>(x, P.x + row * P.ld + (size_t)s * SD, true);
 #pragma unroll
                     for (int i = 0; i < SD; ++i) {
-                        y[i] = x[i] - sub[i];
-                        shift = fmaf(sub[i], x[i] - 0.5f * sub[i], shift); // S = S' - y.mu - |mu|^2 / 2
+                        const float mu = -sub[i], y = x[i] - mu;
+                        sq[i & 1] = fmaf(y, y, sq[i & 1]); // (in the producers' order: cr is cut to eleven bits)
+                        shift = fmaf(mu, x[i] - 0.5f * mu, shift); // S = S' - y.mu - |mu|^2 / 2
                     }
-                    const RowFrame f = row_frame<SD, COSINE>(y, sub);
+                    const RowFrame f = row_frame<COSINE>(sq[0] + sq[1], sub);
                     const float sigma = f.cr * sub[SUB_SCALE2];
                     for (int c = 0; c < 4; ++c) {
                         tmem_ld32_issue(taddr + half * 128 + c * 32, v);
@@ -608,9 +643,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 sa1 = __dp2a_lo(__viaddmin_u16x2(ga[i + 1], minus, MM), (W0 + 2 * i + 2) + ((W0 + 2 * i + 3) << 8), sa1);
             }
             const uint32_t lb = WB - sb - sb1, la = WA - sa - sa1;
-            const uint32_t idx = ((lb / SL::M - W0) * 16u + (la / SL::M - W0)) & 0xFFu;
-            const bool whole = best == 0u || best >= T_HIGH; // nothing to tell apart, or nothing but padding: all centroids
-            bool single = max(lb, la) <= SL::M * (W0 + 15u) && idx < (uint32_t)k && !whole;
+            const uint32_t idx = ((lb * 16u + la - SL::M * 17u * W0) / SL::M) & 0xFFu; // 16 block + class
+            const bool whole = best - 1u >= T_HIGH - 1u; // 0: nothing to tell apart; high up: nothing but columns without a centroid
+            bool single = max(lb, la) <= SL::M * (W0 + 15u) && !whole;
             // a far centroid may be as close (the entry is written again four tiles on, which takes this unit's end)
             const bool far = any_far && best + SL::M > far_s[(ss * 4 + (step & 3u)) * BM + r];
             single = single && !far;
@@ -634,7 +669,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     for (int i = 0; i < 4; ++i) bits = __dp2a_lo(__viaddmin_u16x2(__viaddmin_u16x2(ga[4 * c + i], minus, MM), LESS, 0x10001u), 0x201u << (2 * i), bits);
                     classes |= bits << (8 * c);
                 }
-                if (later) queue[waiting + __popc(vote & ((1u << lane) - 1u))] = make_uint4(tile, r | (classes << 16), blocks, (whole ? Q_WHOLE : 0u) | (far ? Q_FAR : 0u));
+                if (later) queue[waiting + __popc(vote & ((1u << lane) - 1u))] = make_uint4(tile0 + step * tstep, r | (classes << 16), blocks, (whole ? Q_WHOLE : 0u) | (far ? Q_FAR : 0u));
                 waiting += __popc(vote);
                 __syncwarp();
                 if (waiting >= 32) {
@@ -644,7 +679,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             }
             if (valid && single && (!TRAIN || idx != old)) {
                 moved = true;
-                *cp = (uint8_t)idx;
+                *code = (uint8_t)idx;
             }
         }
         if (waiting) moved |= pq_queue_drain<SD, TRAIN, METRIC>(Q, queue, sub, (int)waiting, s, lane);
@@ -842,7 +877,7 @@ __device__ __forceinline__ void write_operand(const float (&v)[SD], int s, int k
     const bool any_far = __syncthreads_or(far && !void_sub) != 0;
     if (j == 0) {
 #pragma unroll
-        for (int i = 0; i < 16; ++i) sub[i] = void_sub || i >= SD ? 0.0f : mu[i % SD];
+        for (int i = 0; i < 16; ++i) sub[i] = void_sub || i >= SD ? 0.0f : -mu[i % SD]; // (added to the rows)
         sub[SUB_RHO2] = 1.000001f * rho * rho;
         sub[SUB_SCALE] = scale;
         sub[SUB_SCALE2] = scale * scale;

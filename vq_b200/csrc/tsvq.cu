@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const fl
                 d = __fsub_rn(v[i].w, cc.w), v[i].w = __fmul_rn(d, d);
             }
             const uint32_t grp = s / NS_GROUP, gslot = grp % NS_GROUPS;
-            if (!mbar_wait(&empty[gslot], ((grp / NS_GROUPS) & 1u) ^ 1u, &abort_flag, error, NS_ERR_WAIT, 100u)) return false;
+            if (!mbar_wait<100u>(&empty[gslot], ((grp / NS_GROUPS) & 1u) ^ 1u, &abort_flag, error, NS_ERR_WAIT)) return false;
             if (s < S) { // not padding
                 const uint32_t at = s % NS_RING * NS_STAGE_BYTES;
                 auto store = [&](int j, int i, float value) {
