@@ -17,6 +17,12 @@ enum : int { M_SQ = 0, M_EUCLID = 1, M_COSINE = 2, M_MANHATTAN = 3, M_CHEBYSHEV 
 // as an integer and, when the words of several ranks are added up as f32 in one all-reduce with the cluster sums, as a float.
 #define VQB_MOVED_BITS 0x3F800000u
 
+// A kernel launched by launch_following: all earlier work of the stream is complete and visible from here on.  Every thread calls it,
+// before it touches global memory or leaves.
+__device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// All blocks that have got here (or left) let the next kernel of the stream, if launched that way, take the free places.
+__device__ __forceinline__ void next_kernel_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- running state of one distance evaluation, advanced one dimension at a time ----------------
 // `b` carries the centroid's sum of squares for the cosine metric (src/distances.rs:141-144).
 template <int METRIC> struct DistAcc {

@@ -10,6 +10,7 @@
 #include <algorithm>
 
 #include "cuda_device.hpp"
+#include "kernels_common.cuh"
 #include "ordered_sums.cuh"
 #include "row_walk.cuh"
 
@@ -17,6 +18,8 @@ namespace vqb {
 
 namespace {
 
+// (what an earlier kernel of the chain wrote is read through plain pointers: loads that the compiler may take for invariant could move
+// above after_previous_kernel())
 constexpr int OL_WARPS = 8, OL_THREADS = 32 * OL_WARPS;
 constexpr unsigned OL_STEP = 1024;   // a chunk is a multiple of this many rows
 constexpr unsigned OL_CHUNKS = 64;   // at most about this many chunks: every list CTA reads the counts of all of them
@@ -24,11 +27,13 @@ constexpr int OL_MAX_K = 4096;       // counters of eight warps in shared memory
 constexpr int OS_WARPS = 2; // 16 KiB of ring each
 
 template <typename CodeT>
-__global__ void __launch_bounds__(OL_THREADS) ordered_hist_kernel(const CodeT *__restrict__ codes, unsigned n, unsigned chunk, int m, int k,
+__global__ void __launch_bounds__(OL_THREADS) ordered_hist_kernel(const CodeT *codes, unsigned n, unsigned chunk, int m, int k,
                                                                   const uint32_t *active, uint32_t *__restrict__ hist)
 {
     extern __shared__ uint32_t s_cnt[]; // [k]
     const int s = blockIdx.y;
+    after_previous_kernel();
+    next_kernel_may_start();
     if (active && active[s] == 0) return;
     for (int j = threadIdx.x; j < k; j += OL_THREADS) s_cnt[j] = 0u;
     __syncthreads();
@@ -42,13 +47,15 @@ __global__ void __launch_bounds__(OL_THREADS) ordered_hist_kernel(const CodeT *_
 // One CTA per (chunk, sub-space).  A warp owns a contiguous eighth of the chunk, so ranking by (earlier chunks, earlier warps of
 // the CTA, earlier steps of the warp, lower lanes) is ranking by row number.
 template <typename CodeT>
-__global__ void __launch_bounds__(OL_THREADS) ordered_lists_kernel(const CodeT *__restrict__ codes, unsigned n, unsigned chunk, int m, int k,
-                                                                   const uint32_t *active, const uint32_t *__restrict__ hist,
+__global__ void __launch_bounds__(OL_THREADS) ordered_lists_kernel(const CodeT *codes, unsigned n, unsigned chunk, int m, int k,
+                                                                   const uint32_t *active, const uint32_t *hist,
                                                                    uint32_t *__restrict__ start, uint32_t *__restrict__ list)
 {
     extern __shared__ uint32_t s_at[]; // [OL_WARPS][k]: counts, then the next free place of each list
     __shared__ uint32_t s_part[OL_WARPS];
     const int s = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    after_previous_kernel();
+    next_kernel_may_start();
     if (active && active[s] == 0) return;
     const unsigned nchunks = gridDim.x, c = blockIdx.x;
     const unsigned per = chunk / OL_WARPS, w0 = c * chunk + warp * per, w1 = min(n, w0 + per);
@@ -116,11 +123,13 @@ __global__ void __launch_bounds__(OL_THREADS) ordered_lists_kernel(const CodeT *
 // are cut into pieces of 32) and walks their lists (row_walk.cuh).
 template <int W, bool VEC>
 __global__ void __launch_bounds__(32 * OS_WARPS) ordered_sums_kernel(const float *__restrict__ x, unsigned n, unsigned long long ld, int m, int k, int sd,
-                                                                     const uint32_t *active, const uint32_t *__restrict__ start,
-                                                                     const uint32_t *__restrict__ list, float *sums, uint32_t *counts, int counts_f32)
+                                                                     const uint32_t *active, const uint32_t *start,
+                                                                     const uint32_t *list, float *sums, uint32_t *counts, int counts_f32)
 {
     __shared__ __align__(16) WalkRing ring[OS_WARPS];
     const int s = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    after_previous_kernel();
+    next_kernel_may_start();
     if (active && active[s] == 0) return;
     const int pieces = (sd + 31) / 32; // 1 unless W == 32
     const int unit = blockIdx.x * OS_WARPS + warp;
@@ -156,14 +165,12 @@ static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const Cod
     {
         KernelScope ks(dev, "ordered_lists");
         const size_t smem = sizeof(uint32_t) * k;
-        ordered_hist_kernel<CodeT><<<dim3(chunks, m), OL_THREADS, smem, dev.stream()>>>(codes, n, chunk, m, k, active, hist);
-        VQB_CUDA_CHECK(cudaGetLastError());
+        launch_following(ordered_hist_kernel<CodeT>, dim3(chunks, m), OL_THREADS, smem, dev.stream(), codes, n, chunk, m, k, active, hist);
         dev.count_launch();
         auto kernel = ordered_lists_kernel<CodeT>;
         if (OL_WARPS * smem > 48 * 1024)
             VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(OL_WARPS * smem)));
-        kernel<<<dim3(chunks, m), OL_THREADS, OL_WARPS * smem, dev.stream()>>>(codes, n, chunk, m, k, active, hist, start, list);
-        VQB_CUDA_CHECK(cudaGetLastError());
+        launch_following(kernel, dim3(chunks, m), OL_THREADS, OL_WARPS * smem, dev.stream(), codes, n, chunk, m, k, active, hist, start, list);
         dev.count_launch();
     }
     {
@@ -172,14 +179,13 @@ static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const Cod
         const size_t units = ((size_t)k + 32 / w - 1) / (32 / w) * ((sd + 31) / 32);
         const dim3 grid((unsigned)((units + OS_WARPS - 1) / OS_WARPS), m);
         auto go = [&](auto kernel) {
-            kernel<<<grid, 32 * OS_WARPS, 0, dev.stream()>>>(x, n, sh.ld, m, k, sd, active, start, list, sums, counts, counts_f32);
+            launch_following(kernel, grid, 32 * OS_WARPS, 0, dev.stream(), x, n, sh.ld, m, k, sd, active, start, list, sums, counts, counts_f32);
         };
         const bool vec = sd % 4 == 0 && sh.ld % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0; // whole 16-byte pieces
         if (w == 4) go(vec ? ordered_sums_kernel<4, true> : ordered_sums_kernel<4, false>);
         else if (w == 8) go(vec ? ordered_sums_kernel<8, true> : ordered_sums_kernel<8, false>);
         else if (w == 16) go(vec ? ordered_sums_kernel<16, true> : ordered_sums_kernel<16, false>);
         else go(vec ? ordered_sums_kernel<32, true> : ordered_sums_kernel<32, false>);
-        VQB_CUDA_CHECK(cudaGetLastError());
         dev.count_launch();
     }
     dev.release(work);

@@ -366,11 +366,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     const uint32_t last_rows = (uint32_t)(P.n - (unsigned long long)(n_tiles - 1) * BM); // rows of the last tile
     const int here = min(4, m - 4 * g); // sub-spaces of this group
 
-    uint32_t act = 0; // bit ss: sub-space ss of the group takes part (identical in every thread)
-#pragma unroll
-    for (int ss = 0; ss < 4; ++ss)
-        if (ss < here && !(TRAIN && P.active && P.active[g * 4 + ss] == 0)) act |= 1u << ss;
-
     if (threadIdx.x == 0) {
         for (int s = 0; s < 4; ++s) {
             mbar_init(&bars->afull[s], 4);
@@ -388,7 +383,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (threadIdx.x < here * SUB_FLOATS) sub_s[threadIdx.x] = Q.sub[(size_t)g * 4 * SUB_FLOATS + threadIdx.x];
     for (uint32_t i = threadIdx.x; i < 4 * A_BYTES<SD> / 16; i += NTHREADS) // the slots that no row uses stay zero
         reinterpret_cast<uint4 *>(a_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -396,6 +390,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_base)), "r"(512u) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    after_previous_kernel();
+    next_kernel_may_start();
+    uint32_t act = 0; // bit ss: sub-space ss of the group takes part (identical in every thread)
+#pragma unroll
+    for (int ss = 0; ss < 4; ++ss)
+        if (ss < here && !(TRAIN && P.active && P.active[g * 4 + ss] == 0)) act |= 1u << ss;
+    if (threadIdx.x < here * SUB_FLOATS) sub_s[threadIdx.x] = Q.sub[(size_t)g * 4 * SUB_FLOATS + threadIdx.x];
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -703,6 +704,8 @@ __global__ void __launch_bounds__(512) pq_expand_kernel(const uint8_t *codes, un
 {
     extern __shared__ __align__(16) uint16_t table[];
     using Piece = typename std::conditional<SD == 4, uint2, uint4>::type; // SD halves
+    after_previous_kernel();
+    next_kernel_may_start();
     if (TABLE) {
         for (uint32_t i = threadIdx.x; i < (uint32_t)m * BN * SD / 8; i += blockDim.x) reinterpret_cast<uint4 *>(table)[i] = __ldg(reinterpret_cast<const uint4 *>(c16) + i);
         __syncthreads();
@@ -900,6 +903,8 @@ template <int SD, bool COSINE> __global__ void __launch_bounds__(BN) pq_operand_
 {
     __shared__ OperandSmem<SD> sm;
     float v[SD];
+    after_previous_kernel();
+    next_kernel_may_start();
     read_centroid<SD>(v, cb, blockIdx.x, k, threadIdx.x);
     write_operand<SD, COSINE>(v, blockIdx.x, k, scratch, sm);
 }
@@ -938,8 +943,7 @@ static void launch_w(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, uns
         configured.fetch_or(bit, std::memory_order_relaxed);
     }
     KernelScope ks(dev, TRAIN ? "assign_train" : "pq_encode");
-    kernel<<<grid, NTHREADS, smem, dev.stream()>>>(mp.x, mp.b1, mp.b2, q);
-    VQB_CUDA_CHECK(cudaGetLastError());
+    launch_following(kernel, grid, NTHREADS, smem, dev.stream(), mp.x, mp.b1, mp.b2, q);
     dev.count_launch();
 }
 
@@ -964,8 +968,7 @@ template <int SD> static void launch_expand(CudaDevice &dev, const AssignParams 
     const unsigned per_sm = in_smem ? (unsigned)std::min<size_t>(4, 200u * 1024u / table) : 4u;
     const unsigned grid = (unsigned)std::min<unsigned long long>((pairs + 511) / 512, (unsigned long long)dev.sm_count() * per_sm);
     KernelScope ks(dev, "pq_expand");
-    kernel<<<grid, 512, in_smem ? table : 0, dev.stream()>>>(reinterpret_cast<const uint8_t *>(p.codes), pairs, p.m, p.k, c16, p.centroids, p.out_f16, p.out_codes, p.out_f32);
-    VQB_CUDA_CHECK(cudaGetLastError());
+    launch_following(kernel, grid, 512, in_smem ? table : 0, dev.stream(), reinterpret_cast<const uint8_t *>(p.codes), pairs, p.m, p.k, c16, p.centroids, p.out_f16, p.out_codes, p.out_f32);
     dev.count_launch();
 }
 
@@ -986,8 +989,7 @@ void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, 
 {
     KernelScope ks(dev, "pq_operand_b");
     auto kernel = sd == 4 ? (cosine ? pq_operand_b_kernel<4, true> : pq_operand_b_kernel<4, false>) : (cosine ? pq_operand_b_kernel<8, true> : pq_operand_b_kernel<8, false>);
-    kernel<<<m, BN, 0, dev.stream()>>>(centroids, k, scratch);
-    VQB_CUDA_CHECK(cudaGetLastError());
+    launch_following(kernel, m, BN, 0, dev.stream(), centroids, k, scratch);
     dev.count_launch();
 }
 
@@ -1044,6 +1046,8 @@ __global__ void __launch_bounds__(BN) pq_update_centroids_kernel(float *sums, ui
     constexpr int V = SD / 4;
     __shared__ OperandSmem<SD> sm;
     const int s = blockIdx.x, j = threadIdx.x;
+    after_previous_kernel();
+    next_kernel_may_start();
     const bool act = !active || active[s] != 0;
     const bool direct = pv.world > 1; // the parts of all ranks are added here, in rank order (peer_exchange.cuh)
     peer_arrive_and_wait(pv);
@@ -1145,8 +1149,7 @@ void launch_pq_update_centroids(CudaDevice &dev, int m, int k, int sd, float *su
 {
     KernelScope ks(dev, "update_centroids");
     auto kernel = sd == 4 ? pq_update_centroids_kernel<4> : pq_update_centroids_kernel<8>;
-    kernel<<<m, BN, 0, dev.stream()>>>(sums, counts, moved, counts_f32 ? 1 : 0, active, k, centroids, scratch, sp, pv);
-    VQB_CUDA_CHECK(cudaGetLastError());
+    launch_following(kernel, m, BN, 0, dev.stream(), sums, counts, moved, counts_f32 ? 1 : 0, active, k, centroids, scratch, sp, pv);
     dev.count_launch();
 }
 
