@@ -1503,6 +1503,8 @@ __global__ void __launch_bounds__(256) update_centroids_kernel(float *sums, uint
     __shared__ uint32_t s_bits;
     const int s = blockIdx.x, word = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    after_previous_kernel();
+    next_kernel_may_start();
     const bool act = !active || active[s] != 0;
     const bool direct = pv.world > 1; // the parts of all ranks are added here, in rank order (peer_exchange.cuh)
     if (threadIdx.x == 0) s_bits = 0u;
@@ -1693,9 +1695,8 @@ void CudaDevice::update_centroids(const Shape &sh, const IterBuffers &buf, const
     const StatusPage sp = status_page(m, k);
     {
         KernelScope ks(*this, "update_centroids");
-        update_centroids_kernel<<<dim3((unsigned)m, wps), 256, 0, stream_>>>(buf.sums, buf.counts, buf.moved, buf.counts_f32 ? 1 : 0, active, (int)k,
-                                                                            (int)sh.sd, centroids, sp, pv);
-        VQB_CUDA_CHECK(cudaGetLastError());
+        launch_following(update_centroids_kernel, dim3((unsigned)m, wps), 256, 0, stream_, buf.sums, buf.counts, buf.moved, buf.counts_f32 ? 1 : 0, active, (int)k,
+                         (int)sh.sd, centroids, sp, pv);
         count_launch();
     }
     wait_status(sp, m, k, status);

@@ -122,6 +122,8 @@ __global__ void __launch_bounds__(192, 1) dense_shortlist_kernel(const __grid_co
     __shared__ uint32_t s_hmax;
     if (threadIdx.x == 0) s_hmax = 0u;
     __syncthreads();
+    after_previous_kernel();
+    next_kernel_may_start();
     for (int t = threadIdx.x; t < BN; t += blockDim.x) {
         const float hn = P.hn[t]; // +inf beyond k
         if (t < P.k) atomicMax(&s_hmax, __float_as_uint(fmaxf(hn, 0.0f))); // the largest half norm (NaN counts as 0)
@@ -469,6 +471,8 @@ __global__ void __launch_bounds__(1024) dense_frame_kernel(const float *__restri
 // A warp per centroid: image and half norm (zeros and +inf at and beyond k)
 __global__ void __launch_bounds__(256) dense_codebook_kernel(const float *c, int k, int dim, int dimp, const float *frame, uint16_t *image, float *hn)
 {
+    after_previous_kernel();
+    next_kernel_may_start();
     const int j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const bool in = j < k;
     float v[4];
@@ -550,8 +554,7 @@ void dense_shortlist(CudaDevice &dev, const DenseWork &w, size_t n, size_t dim, 
     const int dimp = (int)dense_padded(dim);
     {
         KernelScope ks(dev, "dense_codebook");
-        dense_codebook_kernel<<<BN / 8, 256, 0, dev.stream()>>>(codebook, (int)k, (int)dim, dimp, w.frame, w.book_image, w.half_norms);
-        VQB_CUDA_CHECK(cudaGetLastError());
+        launch_following(dense_codebook_kernel, BN / 8, 256, 0, dev.stream(), codebook, (int)k, (int)dim, dimp, w.frame, w.book_image, w.half_norms);
         dev.count_launch();
     }
     const CUtensorMap mx = make_map(w.image, n, dimp, BM);
@@ -577,7 +580,7 @@ void dense_shortlist(CudaDevice &dev, const DenseWork &w, size_t n, size_t dim, 
     KernelScope ks(dev, "dense_shortlist");
     auto go = [&](auto kernel) {
         VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<grid, 192, smem, dev.stream()>>>(mx, mc, p);
+        launch_following(kernel, grid, 192, smem, dev.stream(), mx, mc, p);
     };
     switch (dimp / 16) {
     case 2: go(dense_shortlist_kernel<2>); break;
@@ -588,7 +591,6 @@ void dense_shortlist(CudaDevice &dev, const DenseWork &w, size_t n, size_t dim, 
     case 7: go(dense_shortlist_kernel<7>); break;
     default: go(dense_shortlist_kernel<8>); break;
     }
-    VQB_CUDA_CHECK(cudaGetLastError());
     dev.count_launch();
 }
 

@@ -16,6 +16,7 @@
 #include <algorithm>
 
 #include "cuda_device.hpp"
+#include "kernels_common.cuh"
 #include "queue_sums.cuh"
 
 namespace vqb {
@@ -63,6 +64,8 @@ __global__ void __launch_bounds__(qs_threads(LE), 1024 / qs_threads(LE)) queue_s
     for (int t = threadIdx.x; t < bins * P.sd; t += QS_THREADS) ssum[t] = 0.0f;
     for (int t = threadIdx.x; t < bins; t += QS_THREADS) scnt[t] = 0;
     if (threadIdx.x < TEAMS) fill[threadIdx.x] = 0;
+    after_previous_kernel();
+    next_kernel_may_start();
     uint32_t live = 0; // byte mask of the sub-spaces that take part
     for (int sl = 0; sl < gc; ++sl)
         if (!P.active || P.active[g0 + sl] != 0) live |= 0xFFu << (8 * sl);
@@ -214,8 +217,7 @@ template <int LE, int G> void launch(CudaDevice &dev, const QsParams &q, dim3 gr
 {
     auto kernel = q.prev ? queue_sums_kernel<LE, G, true> : queue_sums_kernel<LE, G, false>;
     VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kernel<<<grid, qs_threads(LE), smem, dev.stream()>>>(q);
-    VQB_CUDA_CHECK(cudaGetLastError());
+    launch_following(kernel, grid, qs_threads(LE), smem, dev.stream(), q);
     dev.count_launch();
 }
 

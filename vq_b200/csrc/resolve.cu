@@ -18,11 +18,13 @@ namespace {
 // the way to a few centroids in L2: 16 loads per lane are on their way at once.
 template <bool VEC>
 __global__ void __launch_bounds__(256) resolve_kernel(const float *__restrict__ x, int dim, int k, const float *__restrict__ book, int euclid,
-                                                      const uint32_t *__restrict__ cand, const uint32_t *__restrict__ list, const uint32_t *list_count,
+                                                      const uint32_t *cand, const uint32_t *list, const uint32_t *list_count,
                                                       uint8_t *codes, uint32_t *changed)
 {
     __shared__ uint8_t s_number[8][256];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    after_previous_kernel();
+    next_kernel_may_start();
     const uint32_t total = *list_count;
     bool moved = false;
     for (uint32_t at = blockIdx.x * 8 + warp; at < total; at += gridDim.x * 8) {
@@ -30,7 +32,7 @@ __global__ void __launch_bounds__(256) resolve_kernel(const float *__restrict__ 
         int cnt = 0;
 #pragma unroll
         for (int w = 0; w < DENSE_MASK_WORDS; ++w) {
-            const uint32_t word = __ldg(cand + row * DENSE_MASK_WORDS + w);
+            const uint32_t word = cand[row * DENSE_MASK_WORDS + w];
             if (word >> lane & 1u) s_number[warp][cnt + __popc(word & ((1u << lane) - 1u))] = (uint8_t)(w * 32 + lane);
             cnt += __popc(word);
         }
@@ -209,8 +211,7 @@ void dense_resolve(CudaDevice &dev, const DenseWork &w, const float *x, size_t n
     const unsigned grid = (unsigned)std::max<size_t>(1, std::min<size_t>((n + 7) / 8, (size_t)dev.sm_count() * 6));
     KernelScope ks(dev, "dense_resolve");
     auto kernel = vec ? resolve_kernel<true> : resolve_kernel<false>;
-    kernel<<<grid, 256, 0, dev.stream()>>>(x, (int)dim, (int)k, codebook, euclid ? 1 : 0, w.cand, w.list, w.list_count, codes, changed);
-    VQB_CUDA_CHECK(cudaGetLastError());
+    launch_following(kernel, grid, 256, 0, dev.stream(), x, (int)dim, (int)k, codebook, euclid ? 1 : 0, w.cand, w.list, w.list_count, codes, changed);
     dev.count_launch();
 }
 

@@ -67,6 +67,8 @@ constexpr int WR_WARPS = 2; // warps per CTA of the kernels that walk rows (16 K
 
 __global__ void init_tree_kernel(size_t n, int splits, uint32_t *perm, NodeInfo *nodes, ChunkInfo *chunks, LevelInfo *level)
 {
+    after_previous_kernel();
+    next_kernel_may_start();
     const size_t nchunks = (n + MEAN_CHUNK - 1) / MEAN_CHUNK;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         perm[i] = (uint32_t)i;
@@ -85,6 +87,8 @@ __global__ void __launch_bounds__(32 * WR_WARPS) chunk_sums_kernel(const float *
                                                                    const LevelInfo *level, const ChunkInfo *chunks, float *partial)
 {
     __shared__ __align__(16) WalkRing ring[WR_WARPS];
+    after_previous_kernel();
+    next_kernel_may_start();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t groups = (dim + 31) / 32, unit = (size_t)blockIdx.x * WR_WARPS + warp, chunk = unit / groups, d0 = unit % groups * 32, d = d0 + lane;
     if (chunk >= (size_t)level->chunks) return;
@@ -97,6 +101,8 @@ __global__ void __launch_bounds__(32 * WR_WARPS) chunk_sums_kernel(const float *
 
 __global__ void node_mean_kernel(const NodeInfo *nodes, const LevelInfo *level, size_t dim, const float *partial, float *centroids)
 {
+    after_previous_kernel();
+    next_kernel_may_start();
     const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (t >= (size_t)level->count * dim) return;
     const int node = level->first + (int)(t / dim);
@@ -116,6 +122,8 @@ __global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *
                                                                    const NodeInfo *nodes, const LevelInfo *level, float *centroids, float *spread)
 {
     __shared__ __align__(16) WalkRing ring[WR_WARPS];
+    after_previous_kernel();
+    next_kernel_may_start();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t groups = (dim + 31) / 32, unit = (size_t)blockIdx.x * WR_WARPS + warp;
     const size_t in_level = unit / groups, d0 = unit % groups * 32, d = d0 + lane;
@@ -181,6 +189,8 @@ __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const fl
     uint64_t *empty = reinterpret_cast<uint64_t *>(ns_smem + NS_RING * NS_STAGE_BYTES);
     volatile uint32_t *filled = reinterpret_cast<volatile uint32_t *>(empty + NS_GROUPS);
     __shared__ int abort_flag;
+    after_previous_kernel();
+    next_kernel_may_start();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned groups = (unsigned)((dim + 31) / 32), in_level = blockIdx.x / groups;
     if (in_level >= (unsigned)level->count) return;
@@ -357,6 +367,8 @@ constexpr int SP_THREADS = 512, SP_BINS = 2048, SP_CLUSTER = 8;
 __global__ void __launch_bounds__(SP_THREADS) split_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm, uint32_t *perm_out,
                                                            NodeInfo *nodes, const LevelInfo *level, const float *spread, uint32_t *keys, int *error)
 {
+    after_previous_kernel();
+    next_kernel_may_start();
     namespace cg = cooperative_groups;
     cg::cluster_group cl = cg::this_cluster();
     const unsigned cs = cl.num_blocks(), rank = cl.block_rank();
@@ -499,6 +511,8 @@ __global__ void __launch_bounds__(1024) next_level_kernel(NodeInfo *nodes, const
 {
     __shared__ unsigned long long s_scan[32], s_carry;
     __shared__ int s_splits;
+    after_previous_kernel();
+    next_kernel_may_start();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const LevelInfo li = *level;
     if (tid == 0) s_carry = 0ull, s_splits = 0;
@@ -545,6 +559,8 @@ __global__ void __launch_bounds__(1024) next_level_kernel(NodeInfo *nodes, const
 
 __global__ void no_children_kernel(const LevelInfo *level, int32_t *left, int32_t *right) // of the deepest level
 {
+    after_previous_kernel();
+    next_kernel_may_start();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < level->count) left[level->first + t] = right[level->first + t] = -1;
 }
@@ -825,8 +841,7 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
     try {
         dev.zero(error, sizeof(int));
         room_for_chunks(2);
-        init_tree_kernel<<<grid_for(n, 256, (unsigned)dev.sm_count() * 8), 256, 0, st>>>(n, max_depth > 0 && n > 1 ? 1 : 0, perm, nodes, chunks, levels);
-        VQB_CUDA_CHECK(cudaGetLastError());
+        launch_following(init_tree_kernel, grid_for(n, 256, (unsigned)dev.sm_count() * 8), 256, 0, st, n, max_depth > 0 && n > 1 ? 1 : 0, perm, nodes, chunks, levels);
         dev.count_launch();
         LevelInfo known = {0, 1, 0, 0}; // the last level that the host has asked about
         auto ask = [&](size_t l) {
@@ -851,28 +866,24 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
             }
             if (small) {
                 KernelScope ks(dev, "tsvq_node_stats");
-                (vec ? node_stats_kernel<true> : node_stats_kernel<false>)<<<grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, nodes, level, cent, spread);
-                VQB_CUDA_CHECK(cudaGetLastError());
+                launch_following(vec ? node_stats_kernel<true> : node_stats_kernel<false>, grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st, x, dim, perm, nodes, level, cent, spread);
                 dev.count_launch();
             } else {
                 {
                     KernelScope ks(dev, "tsvq_node_means");
-                    (vec ? chunk_sums_kernel<true> : chunk_sums_kernel<false>)<<<grid_for((n_chunks + most) * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st>>>(x, dim, perm, level, chunks, partial);
-                    node_mean_kernel<<<grid_for(most * dim, 128, 1u << 30), 128, 0, st>>>(nodes, level, dim, partial, cent);
-                    VQB_CUDA_CHECK(cudaGetLastError());
+                    launch_following(vec ? chunk_sums_kernel<true> : chunk_sums_kernel<false>, grid_for((n_chunks + most) * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st, x, dim, perm, level, chunks, partial);
+                    launch_following(node_mean_kernel, grid_for(most * dim, 128, 1u << 30), 128, 0, st, nodes, level, dim, partial, cent);
                     dev.count_launch();
                     dev.count_launch();
                 }
                 if (!deepest) {
                     KernelScope ks(dev, "tsvq_node_spreads");
-                    spread_kernel<<<grid_for(most * groups, 1, 1u << 30), NS_THREADS, NS_SMEM, st>>>(x, dim, perm, nodes, level, cent, spread, error);
-                    VQB_CUDA_CHECK(cudaGetLastError());
+                    launch_following(spread_kernel, grid_for(most * groups, 1, 1u << 30), NS_THREADS, NS_SMEM, st, x, dim, perm, nodes, level, cent, spread, error);
                     dev.count_launch();
                 }
             }
             if (deepest) {
-                no_children_kernel<<<grid_for(most, 256, 1u << 30), 256, 0, st>>>(level, left, right);
-                VQB_CUDA_CHECK(cudaGetLastError());
+                launch_following(no_children_kernel, grid_for(most, 256, 1u << 30), 256, 0, st, level, left, right);
                 dev.count_launch();
                 ask(l);
                 break;
@@ -884,18 +895,19 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
                 cfg.gridDim = dim3((unsigned)most * cluster);
                 cfg.blockDim = dim3(SP_THREADS);
                 cfg.stream = st;
-                cudaLaunchAttribute attr[1];
+                cudaLaunchAttribute attr[2] = {};
                 attr[0].id = cudaLaunchAttributeClusterDimension;
                 attr[0].val.clusterDim.x = cluster;
                 attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+                attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization; // like launch_following
+                attr[1].val.programmaticStreamSerializationAllowed = 1;
                 cfg.attrs = attr;
-                cfg.numAttrs = 1;
+                cfg.numAttrs = 2;
                 VQB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, split_kernel, x, dim, (const uint32_t *)perm, perm2, nodes, level, (const float *)spread, keys, error));
                 dev.count_launch();
             }
             room_for_chunks(std::min(2 * most, n));
-            next_level_kernel<<<1, 1024, 0, st>>>(nodes, level, levels + ((l + 1) & 1), l + 1 < max_depth ? 1 : 0, left, right, chunks);
-            VQB_CUDA_CHECK(cudaGetLastError());
+            launch_following(next_level_kernel, 1, 1024, 0, st, nodes, level, levels + ((l + 1) & 1), l + 1 < max_depth ? 1 : 0, left, right, chunks);
             dev.count_launch();
             std::swap(perm, perm2);
             most = std::min(2 * most, n);
