@@ -191,6 +191,13 @@ class Device {
     // PQ encode (src/pq.rs:159-186 per row; also the OPQ reconstruction src/opq.rs:146-168 via out_f32).
     virtual void pq_encode(const Shape &sh, const float *x, const float *codebooks, int metric, double p,
                            uint16_t *out_f16, uint32_t *out_codes, float *out_f32) = 0;
+    // pq_encode's f32 reconstruction y of the rows and a = y^T x in one step (src/opq.rs:146-179), without y in memory.  Returns false,
+    // having done nothing, when the device does not take the shape.
+    virtual bool encode_cross_cov(const Shape &sh, const float *x, const float *codebooks, int metric, double *a)
+    {
+        (void)sh, (void)x, (void)codebooks, (void)metric, (void)a;
+        return false;
+    }
     // y[r] = R * x[r] (src/opq.rs:186-194, 232-234); R row-major dim x dim.
     virtual void rotate_rows(const float *rot, size_t dim, const float *x, size_t n, float *y) = 0;
     // a[i][j] += sum_r y[r][i] * x[r][j]  (A = Y * X^T, src/opq.rs:172-179), f64 dim x dim, cleared here.

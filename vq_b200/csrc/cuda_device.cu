@@ -58,8 +58,8 @@ CudaDevice::CudaDevice(int device) : device_(device)
     {
         const char *e = std::getenv("VQB_NO_TENSOR"); // VQB_NO_TENSOR=1: CUDA-core kernels only (A/B comparisons)
         tensor_enabled_ = !(e && *e && *e != '0');
-        // The product quantizer's 8-wide sub-spaces run on the tcgen05 kernel of pq_tc.cu (about twice as fast as the
-        // CUDA-core filter kernel); VQB_PQ_TENSOR=0 selects the filter kernel (A/B comparisons).
+        // The product quantizer's sub-spaces of 4 and 8 values run on the tcgen05 kernel of pq_tc.cu (1M x 128, m 16, k 256: 0.38 ms a
+        // training pass against 2.25 of the CUDA-core filter kernel); VQB_PQ_TENSOR=0 selects the filter kernel (A/B comparisons).
         const char *f = std::getenv("VQB_PQ_TENSOR");
         pq_tensor_enabled_ = tensor_enabled_ && !(f && *f == '0');
     }
@@ -177,7 +177,7 @@ static bool captured(cudaStream_t s)
     return true;
 }
 
-// The scratch of the tensor-core kernels, the map of marked pairs and the memory of a quantizer that is being destroyed are the
+// The scratch of the tensor-core kernels, the one-byte codes of an encode and the memory of a quantizer that is being destroyed are the
 // context's, whatever stream a call runs on.  The caller may destroy a stream of its own as soon as its work is done, so
 // such a stream gets the event while the call is still there (end_call); the context's own and the default stream get it here,
 // so that programs that never change streams pay nothing.
@@ -1839,6 +1839,33 @@ void CudaDevice::cross_cov(const float *y, const float *x, size_t n, size_t dim,
         VQB_CUDA_CHECK(cudaGetLastError());
         count_launch();
     }
+}
+
+bool CudaDevice::encode_cross_cov(const Shape &sh, const float *x, const float *codebooks, int metric, double *a)
+{
+    const size_t dim = sh.m * sh.sd;
+    AssignParams p = {};
+    p.x = x;
+    p.n = sh.n_local;
+    p.ld = sh.ld;
+    p.m = (int)sh.m;
+    p.k = (int)sh.k;
+    p.sd = (int)sh.sd;
+    p.centroids = codebooks;
+    // (few rows: one launch encodes them faster)
+    if (sh.n_local == 0 || sh.ld != dim || !pq_tensor_enabled_ || !opq_tensor_enabled_ || !pq_tc_applicable(p, metric) || !opq_tc_applicable(dim, x, x) ||
+        direct_encode_applicable(p, sh.sd == 8 && sh.m % 4 == 0))
+        return false;
+    zero(a, sizeof(double) * dim * dim);
+    bop_fresh_ = nullptr;
+    PqTcBuffers tb;
+    tb.scratch = pq_scratch_;
+    tb.maps = pq_maps_.get();
+    tb.codes = pq_code_buffer(pq_tc_code_bytes(sh.n_local, sh.m));
+    tb.error_word = tc_error_;
+    launch_pq_tc(*this, p, metric, false, 4, tb);
+    launch_opq_cross_cov_codes(*this, tb.codes, codebooks, sh.m, sh.k, x, sh.n_local, dim, a, tc_error_);
+    return true;
 }
 
 // ------------------------------------------------------------------------------------------------

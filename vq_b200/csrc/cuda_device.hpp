@@ -74,6 +74,7 @@ class CudaDevice : public Device {
     void pq_encode_no_scratch(const Shape &sh, const float *x, const float *codebooks, int metric, double p, uint16_t *out_f16,
                               uint32_t *out_codes);
     void rotate_rows(const float *rot, size_t dim, const float *x, size_t n, float *y) override;
+    bool encode_cross_cov(const Shape &sh, const float *x, const float *codebooks, int metric, double *a) override;
     void cross_cov(const float *y, const float *x, size_t n, size_t dim, double *a) override;
 
     // Not part of the training loops:

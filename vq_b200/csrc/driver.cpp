@@ -9,6 +9,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include "../../include/vqb.h"
@@ -296,7 +297,8 @@ bool opq_fit(Device &dev, Comm *comm, const float *x, size_t n_local, size_t dim
     sh.sd = dim / m;
     sh.k = k;
     const size_t bytes = sizeof(float) * n_local * dim;
-    DevBuf rotated(dev, bytes), rec(dev, bytes);
+    DevBuf rotated(dev, bytes);
+    std::unique_ptr<DevBuf> rec; // the reconstruction, where the device wants it in memory
     DevBuf a_d(dev, sizeof(double) * dim * dim), rot_d(dev, sizeof(float) * dim * dim);
     dev.copy(rotated.p, x, bytes); // src/opq.rs:121
     std::vector<double> a(dim * dim), u(dim * dim), sv(dim), v(dim * dim);
@@ -306,8 +308,11 @@ bool opq_fit(Device &dev, Comm *comm, const float *x, size_t n_local, size_t dim
         lbg_fit(dev, comm, sh, rotated.as<float>(), max_iters, init_idx, draw, user, 0, flags, codebooks, nullptr);
         if (k >= 2 && metric == VQB_MINKOWSKI && p <= 0.0)
             throw Error(VQB_ERR_INVALID_METRIC_PARAMETER, "Invalid metric parameter for Minkowski: p must be positive");
-        dev.pq_encode(sh, rotated.as<float>(), codebooks, metric, p, nullptr, nullptr, rec.as<float>()); // 146-168
-        dev.cross_cov(rec.as<float>(), rotated.as<float>(), n_local, dim, a_d.as<double>());            // 172-179
+        if (!dev.encode_cross_cov(sh, rotated.as<float>(), codebooks, metric, a_d.as<double>())) {
+            if (!rec) rec.reset(new DevBuf(dev, bytes));
+            dev.pq_encode(sh, rotated.as<float>(), codebooks, metric, p, nullptr, nullptr, rec->as<float>()); // 146-168
+            dev.cross_cov(rec->as<float>(), rotated.as<float>(), n_local, dim, a_d.as<double>());            // 172-179
+        }
         if (multi) comm->allreduce_sum_f64(a_d.as<double>(), dim * dim);
         // 180-183: rotation = V U^T.  On the device as the polar factor of A^T when that converges (full-rank A), else the SVD.
         if (dev.polar_rotation(a_d.as<double>(), dim, rot_d.as<float>())) {

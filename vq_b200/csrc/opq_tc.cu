@@ -41,7 +41,7 @@ namespace {
 constexpr int BM = 128;                    // rows per rotate tile = accumulator lanes
 constexpr int CHUNK = 32;                  // f32 per 128-byte swizzle row
 constexpr int NST = 2;                     // stage ring depth (rotate: hi + lo tile of one K chunk; cross_cov: four operand tiles)
-constexpr int NCONV = 8;                   // converter warps
+constexpr int NCONV = 16;                  // converter warps
 constexpr int PF = 3;                      // stages of global loads a converter thread keeps in flight (registers)
 constexpr int NTHREADS = 32 * (2 + NCONV + 4);
 constexpr uint32_t STAGE_ROW_BYTES = 144;  // epilogue staging: 32 floats of a row + 16 bytes, so that rows start in different banks
@@ -200,25 +200,26 @@ __global__ void __launch_bounds__(NTHREADS, 1) opq_rotate_kernel(const __grid_co
         const int cw = warp - 2, sub = lane >> 3, e16 = lane & 7;
         const unsigned long long my_tiles = (n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;
         const unsigned long long total = my_tiles * (unsigned long long)kchunks;
-        auto fetch = [&](float4(&dst)[4], unsigned long long gidx) {
+        constexpr int RPL = BM / NCONV / 4; // rows of a stage per lane
+        auto fetch = [&](float4(&dst)[RPL], unsigned long long gidx) {
             const unsigned long long tile = blockIdx.x + (gidx / kchunks) * gridDim.x;
             const int kc = (int)(gidx % kchunks);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = cw * 16 + i * 4 + sub;
+            for (int i = 0; i < RPL; ++i) {
+                const int r = cw * (BM / NCONV) + i * 4 + sub;
                 const unsigned long long row = tile * BM + r;
                 dst[i] = (gidx < total && row < P.n) ? __ldg(reinterpret_cast<const float4 *>(P.x + row * dim + kc * CHUNK) + e16)
                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
             }
         };
-        auto convert = [&](const float4(&src)[4], unsigned long long gidx) -> bool {
+        auto convert = [&](const float4(&src)[RPL], unsigned long long gidx) -> bool {
             const uint32_t it = (uint32_t)gidx;
             const int st = it % NST;
             if (!mbar_wait(&bars->aempty[st], ((it / NST) & 1u) ^ 1u, abort_flag, P.error, 25)) return false;
             unsigned char *hi_t = a_smem + (size_t)st * 2 * TILE_BYTES, *lo_t = hi_t + TILE_BYTES;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = cw * 16 + i * 4 + sub;
+            for (int i = 0; i < RPL; ++i) {
+                const int r = cw * (BM / NCONV) + i * 4 + sub;
                 float4 h, l;
                 split4(src[i], h, l);
                 const uint32_t off = (uint32_t)r * 128u + (uint32_t)((e16 ^ (r & 7)) << 4);
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) opq_rotate_kernel(const __grid_co
             if (lane == 0) mbar_arrive(&bars->afull[st]);
             return true;
         };
-        float4 p0[4], p1[4], p2[4];
+        float4 p0[RPL], p1[RPL], p2[RPL];
         static_assert(PF == 3, "the ring below is written out for three stages");
         fetch(p0, 0);
         fetch(p1, 1);
@@ -307,13 +308,17 @@ __global__ void opq_split_matrix_kernel(const float *r, int count, float *hi, fl
 // ------------------------------------------------------------------------------------------------
 struct CrossParams {
     const float *y, *x;
+    // CODES: y is not in memory; row r's values are those of the centroids that its codes name
+    const uint8_t *codes;   // [n][m]
+    const float *centroids; // [m][k][sd]
+    int m, k, sd;
     unsigned long long n;
     int dim, kchunks;
     double *a; // [dim][dim], zero-filled by the caller
     int *error;
 };
 
-__global__ void __launch_bounds__(NTHREADS, 1) opq_cross_cov_kernel(const CrossParams P)
+template <bool CODES> __global__ void __launch_bounds__(NTHREADS, 1) opq_cross_cov_kernel(const CrossParams P)
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -381,15 +386,30 @@ __global__ void __launch_bounds__(NTHREADS, 1) opq_cross_cov_kernel(const CrossP
         const int c = lane >> 3, e16 = lane & 7; // column chunk and 16-byte unit of this lane's float4
         const bool lane_in = lane * 4 < dim;
         constexpr int RPW = XC_ROWS / NCONV; // rows of a stage per warp
+        // CODES: this lane's sub-space and place in it; the codes of a stage are requested one stage before its values
+        const int sub = CODES && lane_in ? 4 * lane / P.sd : 0;
+        const float4 *book = CODES ? reinterpret_cast<const float4 *>(P.centroids + (size_t)sub * P.k * P.sd + (lane_in ? 4 * lane % P.sd : 0)) : nullptr;
+        uint32_t next_code[RPW];
+        auto fetch_codes = [&](unsigned long long j) {
+            const unsigned long long blk = blk_begin + j;
+#pragma unroll
+            for (int i = 0; i < RPW; ++i) {
+                const unsigned long long row = blk * XC_ROWS + (unsigned long long)(cw + NCONV * i);
+                next_code[i] = lane_in && blk < blk_end && row < P.n ? P.codes[row * P.m + sub] : 0u;
+            }
+        };
+        if (CODES) fetch_codes(0);
         auto fetch = [&](float4(&dy)[RPW], float4(&dx)[RPW], unsigned long long j) {
             const unsigned long long blk = blk_begin + j;
 #pragma unroll
             for (int i = 0; i < RPW; ++i) {
                 const unsigned long long row = blk * XC_ROWS + (unsigned long long)(cw + NCONV * i);
                 const bool in = lane_in && blk < blk_end && row < P.n;
-                dy[i] = in ? __ldg(reinterpret_cast<const float4 *>(P.y + row * dim) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+                if (CODES) dy[i] = in ? __ldg(book + min(next_code[i], (uint32_t)P.k - 1u) * (uint32_t)(P.sd / 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                else dy[i] = in ? __ldg(reinterpret_cast<const float4 *>(P.y + row * dim) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
                 dx[i] = in ? __ldg(reinterpret_cast<const float4 *>(P.x + row * dim) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
+            if (CODES) fetch_codes(j + 1);
         };
         auto convert = [&](const float4(&sy)[RPW], const float4(&sx)[RPW], unsigned long long j) -> bool {
             const uint32_t it = (uint32_t)j;
@@ -516,11 +536,8 @@ void launch_opq_rotate(CudaDevice &dev, const float *rot, size_t dim, const floa
     dev.count_launch();
 }
 
-void launch_opq_cross_cov(CudaDevice &dev, const float *y, const float *x, size_t n, size_t dim, double *a, int *error_word)
+template <bool CODES> static void launch_cross(CudaDevice &dev, CrossParams p, size_t n, size_t dim, double *a, int *error_word)
 {
-    CrossParams p;
-    p.y = y;
-    p.x = x;
     p.n = n;
     p.dim = (int)dim;
     p.kchunks = (int)(dim / CHUNK);
@@ -528,13 +545,34 @@ void launch_opq_cross_cov(CudaDevice &dev, const float *y, const float *x, size_
     p.error = error_word;
     const size_t smem = 1024 + (size_t)NST * 4 * 4 * XC_ROWS * 128 + 128 * 128 * sizeof(float) + sizeof(OpqBarriers) + 64;
     static std::atomic<unsigned long long> configured{0};
-    set_smem_once(opq_cross_cov_kernel, smem, dev.device(), configured);
+    set_smem_once(opq_cross_cov_kernel<CODES>, smem, dev.device(), configured);
     const unsigned long long blocks = (n + XC_ROWS - 1) / XC_ROWS;
     const unsigned grid = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>(blocks, (unsigned long long)dev.sm_count()));
     KernelScope ks(dev, "cross_cov");
-    opq_cross_cov_kernel<<<grid, NTHREADS, smem, dev.stream()>>>(p);
+    opq_cross_cov_kernel<CODES><<<grid, NTHREADS, smem, dev.stream()>>>(p);
     VQB_CUDA_CHECK(cudaGetLastError());
     dev.count_launch();
+}
+
+void launch_opq_cross_cov(CudaDevice &dev, const float *y, const float *x, size_t n, size_t dim, double *a, int *error_word)
+{
+    CrossParams p = {};
+    p.y = y;
+    p.x = x;
+    launch_cross<false>(dev, p, n, dim, a, error_word);
+}
+
+void launch_opq_cross_cov_codes(CudaDevice &dev, const uint8_t *codes, const float *centroids, size_t m, size_t k, const float *x, size_t n, size_t dim, double *a,
+                                int *error_word)
+{
+    CrossParams p = {};
+    p.codes = codes;
+    p.centroids = centroids;
+    p.m = (int)m;
+    p.k = (int)k;
+    p.sd = (int)(dim / m);
+    p.x = x;
+    launch_cross<true>(dev, p, n, dim, a, error_word);
 }
 
 } // namespace vqb

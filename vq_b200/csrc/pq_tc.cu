@@ -982,7 +982,7 @@ template <int SD> static void launch_sd(CudaDevice &dev, const PqMaps &mp, const
     if (metric == M_EUCLID) launch_t<SD, false, M_EUCLID>(dev, mp, q, grid);
     else if (metric == M_COSINE) launch_t<SD, false, M_COSINE>(dev, mp, q, grid);
     else launch_t<SD, false, M_SQ>(dev, mp, q, grid);
-    launch_expand<SD>(dev, q.a, c16);
+    if (q.a.out_f16 || q.a.out_codes || q.a.out_f32) launch_expand<SD>(dev, q.a, c16); // else the caller wants the one-byte codes
 }
 
 void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, int sd, bool cosine, float *scratch)
