@@ -16,14 +16,20 @@
 //   cross_cov  the contraction runs over ROWS, so both operands are MN-major: a stage holds 32 rows (K) of Y and of X as
 //              dim/32 column chunks of 32 rows x 128 bytes, which is how the rows lie in memory -- no transposition anywhere
 //              (128-byte swizzle with 32-byte base, the one swizzled MN-major layout the tensor core takes for 32-bit elements).
+//               In a fit whose assignment leaves one-byte codes Y is not in memory: the converters gather its values from the
+//               codebooks (128 KiB, in L2), the codes requested a stage ahead.
 // The split needs a pass through registers, so the row tiles are read from global memory by converter warps (coalesced 128-bit
 // loads, one stage ahead) and written as hi / lo tiles with the swizzle applied; fence.proxy.async + mbarrier hand them to the
 // MMA thread.  One persistent CTA per SM:
 //   warp 0      operand B by TMA (rotate only)
 //   warp 1      owns tensor memory (two accumulators) and issues the MMAs
-//   warps 2-9   converters (three stages of global loads in flight per thread)
-//   warps 10-13 epilogue: tcgen05.ld, one accumulator row per lane; rotate writes Y through a shared-memory transposition (whole
+//   warps 2-17  converters (three stages of global loads in flight per thread)
+//   warps 18-21 epilogue: tcgen05.ld, one accumulator row per lane; rotate writes Y through a shared-memory transposition (whole
 //               128-byte row pieces per store), cross_cov adds the accumulator to an f32 partial sum and, at the end, to the f64 result
+// Measured, 1M x 128 (no unit is busy more than two thirds of the time; the conversion of a stage and its hand-over take most of it): rotation
+// 0.226 -> 0.215 ms, cross-covariance from codes (16 x 256 centroids) 0.331 -> 0.276 ms with sixteen converter warps instead of eight (0.220 /
+// 0.288: half as many rows of a stage for each) and with the high parts in integer instructions (the conversion instruction has a fraction of
+// their rate).  With Y in memory 0.29 ms, and 0.20 for writing it.
 // Every wait is bounded; on expiry the CTA records a code, stops issuing, frees tensor memory and the host raises an error.
 #include <algorithm>
 #include <atomic>
@@ -90,9 +96,12 @@ __device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t addr, uint32_t c
 // byte offset of 16-byte unit e16 (0..7) of K row r inside its 128-byte row under that swizzle
 __device__ __forceinline__ uint32_t mn_swizzle_unit(int e16, int r) { return (uint32_t)((((e16 >> 1) ^ (r & 3)) << 5) | ((e16 & 1) << 4)); }
 
+// tf32_round in two integer instructions.  A NaN may come out as something else here, but not v - high_part(v).
+__device__ __forceinline__ float high_part(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u); }
+
 __device__ __forceinline__ void split4(const float4 v, float4 &hi, float4 &lo)
 {
-    hi.x = tf32_round(v.x), hi.y = tf32_round(v.y), hi.z = tf32_round(v.z), hi.w = tf32_round(v.w);
+    hi.x = high_part(v.x), hi.y = high_part(v.y), hi.z = high_part(v.z), hi.w = high_part(v.w);
     lo.x = tf32_round(v.x - hi.x), lo.y = tf32_round(v.y - hi.y), lo.z = tf32_round(v.z - hi.z), lo.w = tf32_round(v.w - hi.w);
 }
 
