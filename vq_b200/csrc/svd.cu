@@ -7,6 +7,7 @@
 // __syncthreads.  The sweeps end when no pair rotated (|g_p . g_q| <= 1e-15 |g_p| |g_q| for all pairs) or after 60 sweeps;
 // singular values, U and the completion of a rank-deficient U are computed by the caller from the converged G.
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 
@@ -142,6 +143,10 @@ bool CudaDevice::svd_sweeps(double *gt, double *vt, size_t n)
 // same sequence); small singular values then grow by up to 2.6 instead of 1.5 per step.  The interval starts at l = 1e-4, a
 // guess: a smaller true value only means the last steps run with the plain coefficients.  One launch and about 16 steps
 // replace some 25 steps of three stream operations each and a host round trip every eighth step (1.23 -> 0.37 ms at n = 128).
+// A step is a chain of trips to L2 and of barriers, so a product waits for one trip (all operands of a tile requested at once; one per
+// 16 values of the contraction before), the residual arrives with the next product's operands, a thread keeps its own entry of the
+// iterate, the coefficients come with the launch and the barrier is a release and an acquire instead of two full fences: 0.325 -> 0.148 ms
+// at n = 128 (the products alone 0.185).
 // The step-by-step kernels below remain for matrices whose tiles cannot all be resident.  If the iteration has not converged
 // after 96 steps (rank-deficient or extremely ill-conditioned A) the caller falls back to the Jacobi SVD, which also
 // completes a null space.
@@ -238,9 +243,32 @@ __global__ void __launch_bounds__(POLAR_TILE *POLAR_TILE) polar_update_kernel(co
 }
 
 // ---- the whole iteration in one cooperative launch ---------------------------------------------
+// The coefficients of the steps: the cubic a x - b x^3 that maps [l, 1] into the narrowest [l', 1], until l has reached 1; (1.5, 0.5) beyond
+struct PolarSteps {
+    static constexpr int N = 24;
+    double a[N], b[N];
+};
+
+PolarSteps polar_steps(double l)
+{
+    PolarSteps st;
+    for (int i = 0; i < PolarSteps::N; ++i) {
+        st.a[i] = 1.5, st.b[i] = 0.5;
+        if (l < 0.999) {
+            const double s = 1.0 + l + l * l, xs = std::sqrt(s / 3.0);
+            const double pa = 2.0 / ((2.0 / 3.0) * xs + 1.0 - 1.0 / s), pe = (2.0 * pa / 3.0) * xs - 1.0;
+            st.a[i] = pa / (1.0 + pe);
+            st.b[i] = pa / s / (1.0 + pe);
+            l = (1.0 - pe) / (1.0 + pe);
+        }
+    }
+    return st;
+}
+
 struct PolarWork {
     double *x0, *x1, *b;             // n x n each
     unsigned long long *resid;       // [max_steps + 1] bits of max |X^T X - I| per step, zero on entry
+    unsigned long long *scale;       // [2] bits of |A|_inf and |A|_1, zero on entry
     unsigned int *arrivals;          // grid barrier counter, zero on entry
     int *status;                     // [0] 1 = converged, 0 = not, -1 = a barrier wait ran out; [1] steps taken
 };
@@ -251,114 +279,154 @@ __device__ __forceinline__ bool polar_grid_barrier(const PolarWork &w, unsigned 
 {
     __syncthreads();
     if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(w.arrivals, 1u);
+        // release and acquire on the counter itself: no fence waits for anything else
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(w.arrivals) : "memory");
         const unsigned int target = round * ctas;
-        unsigned int i = 0;
-        while ((int)(*reinterpret_cast<volatile unsigned int *>(w.arrivals) - target) < 0) {
-            if (++i > (1u << 26) || *reinterpret_cast<volatile int *>(w.status) < 0) {
+        for (unsigned int i = 0;;) {
+            unsigned int seen;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(w.arrivals) : "memory");
+            if ((int)(seen - target) >= 0) break;
+            if (++i > (1u << 26) || ((i & 63u) == 0 && *reinterpret_cast<volatile int *>(w.status) < 0)) {
                 *reinterpret_cast<volatile int *>(w.status) = -1;
                 *failed_sh = 1;
                 break;
             }
         }
-        __threadfence();
     }
     __syncthreads();
     return *failed_sh == 0;
 }
 
-__global__ void __launch_bounds__(POLAR_TILE *POLAR_TILE) polar_iterate_kernel(const double *a, int n, PolarWork w, float *rot, int max_steps, double l0)
+// Sum over r of left(r, i) * right(r, j) for the CTA's 16 x 16 tile: thread t gets entry (t / 16, t % 16).  KC values of r at a time lie in shared
+// memory, all of a thread's loads of them in flight at once (one trip to L2 instead of one per 16); four groups of 64 threads take every
+// fourth r with 2 x 2 entries per thread, which are added up at the end.
+//   left(r, i) = TRANSPOSED ? left[(i0 + i) n + r] : left[r n + i0 + i];   right(r, j) = right[r n + j0 + j]
+constexpr int POLAR_LD = POLAR_TILE + 2; // doubles of a row in shared memory: 16-byte pieces stay whole, transposed stores spread over the banks
+template <int KC> struct PolarTiles {
+    double l[KC][POLAR_LD], r[KC][POLAR_LD];
+};
+
+template <int KC, bool TRANSPOSED>
+__device__ __forceinline__ double polar_tile(const double *left, const double *right, int n, int i0, int j0, PolarTiles<KC> &sh)
 {
-    __shared__ double sa[POLAR_TILE][POLAR_TILE + 1], sb[POLAR_TILE][POLAR_TILE + 1];
-    __shared__ double red[POLAR_TILE * POLAR_TILE];
+    constexpr int PIECES = KC * POLAR_TILE / 2 / 256; // 16-byte pieces of either operand per thread and chunk
+    const int t = threadIdx.x, g = t >> 6, ti = (t >> 3) & 7, tj = t & 7;
+    double acc[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+    for (int r0 = 0; r0 < n; r0 += KC) {
+        const int kc = min(KC, n - r0); // a multiple of 16
+        double2 lv[PIECES], rv[PIECES];
+#pragma unroll
+        for (int u = 0; u < PIECES; ++u) {
+            const int r = (t >> 3) + 32 * u;                // row of the chunk, piece t & 7 of its 128 bytes
+            const int r2 = 2 * ((t & 15) + POLAR_TILE * u); // TRANSPOSED: values r2, r2 + 1 of row t / 16
+            if (r < kc) rv[u] = __ldcg(reinterpret_cast<const double2 *>(right + (size_t)(r0 + r) * n + j0) + (t & 7));
+            if (TRANSPOSED) {
+                if (r2 < kc) lv[u] = __ldcg(reinterpret_cast<const double2 *>(left + (size_t)(i0 + (t >> 4)) * n + r0 + r2));
+            } else if (r < kc) {
+                lv[u] = __ldcg(reinterpret_cast<const double2 *>(left + (size_t)(r0 + r) * n + i0) + (t & 7));
+            }
+        }
+        if (r0) __syncthreads(); // the chunk before has been used
+#pragma unroll
+        for (int u = 0; u < PIECES; ++u) {
+            const int r = (t >> 3) + 32 * u, r2 = 2 * ((t & 15) + POLAR_TILE * u);
+            if (r < kc) *reinterpret_cast<double2 *>(&sh.r[r][2 * (t & 7)]) = rv[u];
+            if (TRANSPOSED) {
+                if (r2 < kc) sh.l[r2][t >> 4] = lv[u].x, sh.l[r2 + 1][t >> 4] = lv[u].y;
+            } else if (r < kc) {
+                *reinterpret_cast<double2 *>(&sh.l[r][2 * (t & 7)]) = lv[u];
+            }
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int r = g; r < kc; r += 4) {
+            const double2 a = *reinterpret_cast<const double2 *>(&sh.l[r][2 * ti]), b = *reinterpret_cast<const double2 *>(&sh.r[r][2 * tj]);
+            acc[0][0] = fma(a.x, b.x, acc[0][0]), acc[0][1] = fma(a.x, b.y, acc[0][1]);
+            acc[1][0] = fma(a.y, b.x, acc[1][0]), acc[1][1] = fma(a.y, b.y, acc[1][1]);
+        }
+    }
+    __syncthreads();
+    double *part = reinterpret_cast<double *>(&sh); // [4][16][16]
+    static_assert(4 * POLAR_TILE * POLAR_TILE * sizeof(double) <= sizeof(PolarTiles<KC>), "the partial sums fit into the operands' place");
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) part[(g * POLAR_TILE + 2 * ti + a) * POLAR_TILE + 2 * tj + b] = acc[a][b];
+    __syncthreads();
+    const double sum = (part[t] + part[t + 256]) + (part[t + 512] + part[t + 768]);
+    __syncthreads();
+    return sum;
+}
+
+// max over the CTA of a non-negative value into *out (bits of a non-negative double are ordered like integers), by thread 0, whose
+// grid barrier follows
+__device__ __forceinline__ void polar_max(double v, unsigned long long *out, double *red)
+{
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = 1; q < 8; ++q) v = fmax(v, red[q]);
+        atomicMax(out, (unsigned long long)__double_as_longlong(v));
+    }
+}
+
+template <int KC, int CTAS_PER_SM>
+__global__ void __launch_bounds__(POLAR_TILE *POLAR_TILE, CTAS_PER_SM)
+    polar_iterate_kernel(const double *a, int n, PolarWork w, float *rot, int max_steps, const __grid_constant__ PolarSteps steps)
+{
+    __shared__ __align__(16) PolarTiles<KC> tiles;
+    __shared__ double red[8];
     __shared__ int failed_sh;
-    const int tx = threadIdx.x % POLAR_TILE, ty = threadIdx.x / POLAR_TILE;
-    const int i = blockIdx.y * POLAR_TILE + ty, j = blockIdx.x * POLAR_TILE + tx;
+    const int i0 = blockIdx.y * POLAR_TILE, j0 = blockIdx.x * POLAR_TILE;
+    const int i = i0 + threadIdx.x / POLAR_TILE, j = j0 + threadIdx.x % POLAR_TILE;
     const unsigned int ctas = gridDim.x * gridDim.y;
     unsigned int round = 0;
     if (threadIdx.x == 0) failed_sh = 0;
-    // scale^2 = |a|_1 |a|_inf, computed by every CTA for itself (the same value everywhere)
-    double best_row = 0.0, best_col = 0.0;
-    for (int t = threadIdx.x; t < n; t += POLAR_TILE * POLAR_TILE) {
-        double r = 0.0, c = 0.0;
-        for (int u = 0; u < n; ++u) {
-            r += fabs(__ldcg(a + (size_t)t * n + u));
-            c += fabs(__ldcg(a + (size_t)u * n + t));
-        }
-        best_row = fmax(best_row, r);
-        best_col = fmax(best_col, c);
+    // scale^2 = |a|_1 |a|_inf: a warp per row sum or column sum
+    double best[2] = {0.0, 0.0};
+    for (unsigned int v = (blockIdx.y * gridDim.x + blockIdx.x) * 8u + (threadIdx.x >> 5); v < 2u * (unsigned)n; v += 8u * ctas) {
+        const bool column = v >= (unsigned)n;
+        const size_t first = column ? v - (unsigned)n : (size_t)v * n, step = column ? (size_t)n : 1;
+        double sum = 0.0;
+#pragma unroll 4
+        for (int u = threadIdx.x & 31; u < n; u += 32) sum += fabs(__ldcg(a + first + u * step));
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        best[column] = fmax(best[column], sum); // (a NaN is passed over)
     }
-    red[threadIdx.x] = best_row;
-    __syncthreads();
-    for (int o = POLAR_TILE * POLAR_TILE / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);
-        __syncthreads();
-    }
-    const double rmax = red[0];
-    __syncthreads();
-    red[threadIdx.x] = best_col;
-    __syncthreads();
-    for (int o = POLAR_TILE * POLAR_TILE / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);
-        __syncthreads();
-    }
-    const double f = sqrt(rmax * red[0]);
-    __syncthreads();
     double *cur = w.x0, *nxt = w.x1;
-    cur[(size_t)i * n + j] = (f > 0.0 && f == f) ? __ldcg(a + (size_t)j * n + i) / f : 0.0; // X_0 = A^T / f
+    double own = __ldcg(a + (size_t)j * n + i); // this thread's entry of the iterate; X_0 = A^T inv, the factor applied in step 0
+    cur[(size_t)i * n + j] = own;
+    polar_max(best[0], w.scale, red);
+    __syncthreads();
+    polar_max(best[1], w.scale + 1, red);
     if (!polar_grid_barrier(w, ++round, ctas, &failed_sh)) return;
-    double l = l0, resid = 1.0;
+    const double f = sqrt(__longlong_as_double((long long)__ldcg(w.scale)) * __longlong_as_double((long long)__ldcg(w.scale + 1)));
+    double inv = (f > 0.0 && f == f) ? 1.0 / f : 0.0;
+    double resid = 1.0;
     int step = 0;
     for (; step <= max_steps; ++step) {
-        // b = cur^T cur, tile (i-block, j-block), and the step's residual
-        double acc = 0.0;
-        for (int r0 = 0; r0 < n; r0 += POLAR_TILE) {
-            sa[ty][tx] = __ldcg(cur + (size_t)(r0 + ty) * n + blockIdx.y * POLAR_TILE + tx);
-            sb[ty][tx] = __ldcg(cur + (size_t)(r0 + ty) * n + blockIdx.x * POLAR_TILE + tx);
-            __syncthreads();
-#pragma unroll
-            for (int r = 0; r < POLAR_TILE; ++r) acc = fma(sa[r][ty], sb[r][tx], acc);
-            __syncthreads();
-        }
-        w.b[(size_t)i * n + j] = acc;
-        const double dev = fabs(acc - (i == j ? 1.0 : 0.0));
-        red[threadIdx.x] = dev == dev ? dev : 1e300;
-        __syncthreads();
-        for (int o = POLAR_TILE * POLAR_TILE / 2; o > 0; o >>= 1) {
-            if ((int)threadIdx.x < o) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + o]);
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) atomicMax(w.resid + step, (unsigned long long)__double_as_longlong(red[0]));
+        // b = X^T X, tile (i-block, j-block), and the step's residual
+        const double b = polar_tile<KC, false>(cur, cur, n, i0, j0, tiles) * inv * inv;
+        w.b[(size_t)i * n + j] = b;
+        const double dev = fabs(b - (i == j ? 1.0 : 0.0));
+        polar_max(dev == dev ? dev : 1e300, w.resid + step, red);
         if (!polar_grid_barrier(w, ++round, ctas, &failed_sh)) return;
-        resid = __longlong_as_double((long long)__ldcg(w.resid + step));
+        // nxt = ca X - cb X b, tile (i-block, j-block); the residual arrives with its operands
+        const unsigned long long bits = __ldcg(w.resid + step);
+        const double xb = polar_tile<KC, true>(cur, w.b, n, i0, j0, tiles);
+        resid = __longlong_as_double((long long)bits);
         if (resid < POLAR_TOL || step == max_steps) break; // the same value in every CTA
-        // coefficients: the cubic that maps [l, 1] into the narrowest [l', 1]; (1.5, 0.5) once l has reached 1
-        double ca = 1.5, cb = 0.5;
-        if (l < 0.999) {
-            const double s = 1.0 + l + l * l, xs = sqrt(s / 3.0);
-            const double pa = 2.0 / ((2.0 / 3.0) * xs + 1.0 - 1.0 / s), pe = (2.0 * pa / 3.0) * xs - 1.0;
-            ca = pa / (1.0 + pe);
-            cb = pa / s / (1.0 + pe);
-            l = (1.0 - pe) / (1.0 + pe);
-        }
-        // nxt = ca cur - cb cur b, tile (i-block, j-block)
-        acc = 0.0;
-        for (int r0 = 0; r0 < n; r0 += POLAR_TILE) {
-            sa[ty][tx] = __ldcg(cur + (size_t)i * n + r0 + tx);
-            sb[ty][tx] = __ldcg(w.b + (size_t)(r0 + ty) * n + j);
-            __syncthreads();
-#pragma unroll
-            for (int r = 0; r < POLAR_TILE; ++r) acc = fma(sa[ty][r], sb[r][tx], acc);
-            __syncthreads();
-        }
-        nxt[(size_t)i * n + j] = ca * __ldcg(cur + (size_t)i * n + j) - cb * acc;
+        const double ca = step < PolarSteps::N ? steps.a[step] : 1.5, cb = step < PolarSteps::N ? steps.b[step] : 0.5;
+        own = (ca * own - cb * xb) * inv;
+        nxt[(size_t)i * n + j] = own;
+        inv = 1.0;
         if (!polar_grid_barrier(w, ++round, ctas, &failed_sh)) return;
         double *t = cur;
         cur = nxt;
         nxt = t;
     }
-    rot[(size_t)i * n + j] = (float)__ldcg(cur + (size_t)i * n + j);
+    rot[(size_t)i * n + j] = (float)(own * inv);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         w.status[0] = resid < 1e-11 ? 1 : 0;
         w.status[1] = step;
@@ -383,17 +451,24 @@ bool CudaDevice::polar_rotation(const double *a_dev, size_t n, float *rot_dev)
         int per_sm = 0, coop = 0, dev_id = 0;
         cudaGetDevice(&dev_id);
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev_id);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, polar_iterate_kernel, POLAR_TILE * POLAR_TILE, 0);
+        // 128 values of the contraction at a time while all CTAs fit beside each other with the registers that takes (n <= 272 on 148 SMs), else 32
         const size_t ctas = (n / POLAR_TILE) * (n / POLAR_TILE);
+        auto kernel = polar_iterate_kernel<128, 2>;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, POLAR_TILE * POLAR_TILE, 0);
+        if ((size_t)per_sm * (size_t)sm_count() < ctas) {
+            kernel = polar_iterate_kernel<32, 7>;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, POLAR_TILE * POLAR_TILE, 0);
+        }
         if (coop && (size_t)per_sm * (size_t)sm_count() >= ctas && std::getenv("VQB_POLAR_STEPWISE") == nullptr) {
-            const size_t extra = sizeof(unsigned long long) * (max_steps + 2) + 64;
+            const size_t extra = sizeof(unsigned long long) * (max_steps + 4) + 64;
             unsigned char *blk = static_cast<unsigned char *>(alloc(3 * bytes + extra));
             PolarWork w;
             w.x0 = reinterpret_cast<double *>(blk);
             w.x1 = w.x0 + n * n;
             w.b = w.x1 + n * n;
             w.resid = reinterpret_cast<unsigned long long *>(blk + 3 * bytes);
-            w.arrivals = reinterpret_cast<unsigned int *>(w.resid + max_steps + 2);
+            w.scale = w.resid + max_steps + 2;
+            w.arrivals = reinterpret_cast<unsigned int *>(w.scale + 2);
             w.status = reinterpret_cast<int *>(w.arrivals + 2);
             int status[2] = {0, 0};
             {
@@ -401,9 +476,9 @@ bool CudaDevice::polar_rotation(const double *a_dev, size_t n, float *rot_dev)
                 VQB_CUDA_CHECK(cudaMemsetAsync(w.resid, 0, extra, stream_));
                 const dim3 grid((unsigned)(n / POLAR_TILE), (unsigned)(n / POLAR_TILE));
                 int n_i = (int)n, steps_i = max_steps;
-                double l0 = 1e-4;
-                void *args[] = {(void *)&a_dev, (void *)&n_i, (void *)&w, (void *)&rot_dev, (void *)&steps_i, (void *)&l0};
-                VQB_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)polar_iterate_kernel, grid, dim3(POLAR_TILE * POLAR_TILE), args, 0, stream_));
+                PolarSteps steps = polar_steps(1e-4);
+                void *args[] = {(void *)&a_dev, (void *)&n_i, (void *)&w, (void *)&rot_dev, (void *)&steps_i, (void *)&steps};
+                VQB_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)kernel, grid, dim3(POLAR_TILE * POLAR_TILE), args, 0, stream_));
                 count_launch();
             }
             download(status, w.status, sizeof status);
