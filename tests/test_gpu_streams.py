@@ -16,7 +16,7 @@ def _quantizers():
 
 
 def test_calls_on_two_streams_follow_each_other():
-    """Two quantizers, two streams, nobody waits: the operand tiles and the map of marked pairs of one call are the next one's, and a
+    """Two quantizers, two streams, nobody waits: the operand tiles of one call are the next one's, and a
     quantizer is destroyed while its last call may still run."""
     import torch
     x = torch.from_numpy(synth.uniform01(300_000, 128, 9)).cuda()
@@ -75,3 +75,31 @@ def test_a_captured_call_stays_out_of_the_order():
     got_b = b.quantize(x, return_codes=True)[1]
     graph.replay()
     assert torch.equal(codes, want_a) and torch.equal(got_b, want_b)
+
+
+@pytest.mark.parametrize("m,sd,k", [(16, 8, 256), (7, 8, 100), (9, 4, 60)])
+def test_a_captured_encode_has_working_memory_of_its_own(m, sd, k):
+    """The first call of a context may be a captured one, and its graph replays correctly after larger calls of the context and between
+    them: nothing that it works with is the context's to free."""
+    import torch
+    x = torch.from_numpy(synth.uniform01(60_000, m * sd, 9)).cuda()
+    books = synth.uniform01(m * k, sd, 3).reshape(m, k, sd)
+    rows = x[:30_000].clone()
+    want, want_all = (vq.ProductQuantizer.from_codebooks(books, vq.Distance.Euclidean).quantize(r, return_codes=True) for r in (rows, x))
+    ctx = vq.Context(0)
+    q = vq.ProductQuantizer.from_codebooks(books, vq.Distance.Euclidean, ctx=ctx)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out, codes = q.quantize(rows, return_codes=True)
+    for turn in range(3):
+        out.zero_(), codes.zero_()
+        graph.replay()
+        assert torch.equal(codes, want[1]) and torch.equal(out, want[0])
+        got = q.quantize(x, return_codes=True)  # larger than anything before it
+        assert torch.equal(got[1], want_all[1]) and torch.equal(got[0], want_all[0])
+        rows.copy_(x[30_000:] if turn == 0 else x[:30_000])  # the graph reads its rows anew
+        graph.replay()
+        assert torch.equal(codes, want_all[1][30_000:] if turn == 0 else want[1])
+        rows.copy_(x[:30_000])
+    del graph

@@ -90,7 +90,6 @@ CudaDevice::~CudaDevice()
         if (stage_) cudaFreeHost(stage_);
         cudaFree(rot_split_);
         cudaFree(pq_scratch_);
-        cudaFree(pq_codes_);
         cudaFree(tc_stats_);
         cudaFree(tc_error_);
         if (status_host_) cudaFreeHost(status_host_);
@@ -177,8 +176,8 @@ static bool captured(cudaStream_t s)
     return true;
 }
 
-// The scratch of the tensor-core kernels, the one-byte codes of an encode and the memory of a quantizer that is being destroyed are the
-// context's, whatever stream a call runs on.  The caller may destroy a stream of its own as soon as its work is done, so
+// The scratch of the tensor-core kernels and the memory of a quantizer that is being destroyed are the context's, whatever stream a call
+// runs on.  The caller may destroy a stream of its own as soon as its work is done, so
 // such a stream gets the event while the call is still there (end_call); the context's own and the default stream get it here,
 // so that programs that never change streams pay nothing.
 void CudaDevice::set_stream(cudaStream_t s)
@@ -480,22 +479,6 @@ void CudaDevice::release_dense()
     dense_ = DenseWork();
 }
 
-// Working memory of encodes on the tensor path, kept by the context: grown when a larger call comes.
-uint8_t *CudaDevice::pq_code_buffer(size_t bytes)
-{
-    if (bytes > pq_codes_cap_) {
-        VQB_CUDA_CHECK(cudaStreamSynchronize(stream_));
-        cudaFree(pq_codes_);
-        pq_codes_ = nullptr;
-        pq_codes_cap_ = 0;
-        const size_t cap = bytes + bytes / 4;
-        ++device_allocs_;
-        VQB_CUDA_CHECK(cudaMalloc(&pq_codes_, cap));
-        pq_codes_cap_ = cap;
-    }
-    return pq_codes_;
-}
-
 // Called at host synchronisation points: a tensor-core kernel whose bounded wait expired leaves a code here.
 void CudaDevice::check_tc_error()
 {
@@ -541,6 +524,16 @@ void CudaDevice::dense_debug(const float *x, size_t n, size_t dim, const float *
     prepared_x_ = nullptr;
 }
 
+// The one-byte codes that an encode on the tensor path goes through.  They belong to the call, in the order of its stream: a call that is
+// being captured makes them part of its graph, which may then be replayed whatever other calls do meanwhile (a buffer that the
+// context keeps and grows is freed under a graph that holds its address, and cannot grow at all during a capture).
+struct PqCodes {
+    CudaDevice &dev;
+    uint8_t *const codes;
+    PqCodes(CudaDevice &d, size_t n, size_t m) : dev(d), codes(static_cast<uint8_t *>(d.alloc(pq_tc_code_bytes(n, m)))) {}
+    ~PqCodes() { dev.release(codes); }
+};
+
 void CudaDevice::pq_tensor_debug(const float *x, size_t n, size_t m, const float *codebooks, size_t k, float *scores, uint32_t *codes,
                                  unsigned long long *marked)
 {
@@ -561,7 +554,8 @@ void CudaDevice::pq_tensor_debug(const float *x, size_t n, size_t m, const float
     PqTcBuffers tb;
     tb.scratch = pq_scratch_;
     tb.maps = pq_maps_.get();
-    tb.codes = pq_code_buffer(pq_tc_code_bytes(n, m));
+    const PqCodes work(*this, n, m);
+    tb.codes = work.codes;
     tb.error_word = tc_error_;
     tb.dbg_scores = scores;
     launch_pq_tc(*this, p, M_SQ, false, 4, tb);
@@ -784,7 +778,8 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
         tb.prepare_operand = !operand_there;
         tb.scratch = pq_scratch_;
         tb.maps = pq_maps_.get();
-        tb.codes = pq_code_buffer(pq_tc_code_bytes(sh.n_local, sh.m));
+        const PqCodes work(*this, sh.n_local, sh.m);
+        tb.codes = work.codes;
         tb.error_word = tc_error_;
         launch_pq_tc(*this, p, metric, false, 4, tb);
         return;
@@ -1861,7 +1856,8 @@ bool CudaDevice::encode_cross_cov(const Shape &sh, const float *x, const float *
     PqTcBuffers tb;
     tb.scratch = pq_scratch_;
     tb.maps = pq_maps_.get();
-    tb.codes = pq_code_buffer(pq_tc_code_bytes(sh.n_local, sh.m));
+    const PqCodes work(*this, sh.n_local, sh.m);
+    tb.codes = work.codes;
     tb.error_word = tc_error_;
     launch_pq_tc(*this, p, metric, false, 4, tb);
     launch_opq_cross_cov_codes(*this, tb.codes, codebooks, sh.m, sh.k, x, sh.n_local, dim, a, tc_error_);

@@ -156,9 +156,6 @@ class CudaDevice : public Device {
     void *try_alloc(size_t bytes); // null when there is no room
     float *pq_scratch_ = nullptr;
     std::unique_ptr<PqTcMaps> pq_maps_; // of pq_scratch_
-    uint8_t *pq_codes_ = nullptr;
-    size_t pq_codes_cap_ = 0;
-    uint8_t *pq_code_buffer(size_t bytes);
     float *rot_split_ = nullptr; // TF32 high and low parts of the rotation matrix of the current rotate_rows call (dim <= 128)
     bool opq_tensor_enabled_ = true;
     bool pq_tensor_enabled_ = false;
