@@ -529,8 +529,20 @@ void CudaDevice::dense_debug(const float *x, size_t n, size_t dim, const float *
 // context keeps and grows is freed under a graph that holds its address, and cannot grow at all during a capture).
 struct PqCodes {
     CudaDevice &dev;
-    uint8_t *const codes;
-    PqCodes(CudaDevice &d, size_t n, size_t m) : dev(d), codes(static_cast<uint8_t *>(d.alloc(pq_tc_code_bytes(n, m)))) {}
+    size_t rows; // at a time: all of them, or a multiple of 128
+    uint8_t *codes;
+    PqCodes(CudaDevice &d, size_t n, size_t m) : dev(d), rows(n), codes(static_cast<uint8_t *>(d.alloc(pq_tc_code_bytes(n, m)))) {}
+    // As many rows as there is room for, but not less than `least`: none then, and codes is null.
+    PqCodes(CudaDevice &d, size_t n, size_t m, size_t least) : dev(d), rows(n), codes(nullptr)
+    {
+        static const char *cap = std::getenv("VQB_CODE_ROWS"); // at most so many rows' codes at a time (tests)
+        if (cap) rows = std::min(n, (size_t)std::strtoull(cap, nullptr, 10) / 128 * 128), least = std::min<size_t>(least, 128);
+        for (; rows >= std::min(n, least) && rows; rows = rows / 256 * 128) {
+            codes = static_cast<uint8_t *>(dev.try_alloc(pq_tc_code_bytes(rows, m)));
+            if (codes) return;
+        }
+    }
+    PqCodes(const PqCodes &) = delete;
     ~PqCodes() { dev.release(codes); }
 };
 
@@ -773,16 +785,29 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
         return;
     }
     if (tensor) {
-        bop_fresh_ = nullptr;
-        PqTcBuffers tb;
-        tb.prepare_operand = !operand_there;
-        tb.scratch = pq_scratch_;
-        tb.maps = pq_maps_.get();
-        const PqCodes work(*this, sh.n_local, sh.m);
-        tb.codes = work.codes;
-        tb.error_word = tc_error_;
-        launch_pq_tc(*this, p, metric, false, 4, tb);
-        return;
+        // Where memory is short the rows are taken piece by piece, and pieces of less than 32,768 rows (each is three launches) are left to
+        // the kernels that need no working memory.
+        const PqCodes work(*this, sh.n_local, sh.m, 32768);
+        if (work.codes) {
+            bop_fresh_ = nullptr;
+            PqTcBuffers tb;
+            tb.prepare_operand = !operand_there;
+            tb.scratch = pq_scratch_;
+            tb.maps = pq_maps_.get();
+            tb.codes = work.codes;
+            tb.error_word = tc_error_;
+            for (size_t r0 = 0; r0 < sh.n_local; r0 += work.rows) {
+                AssignParams piece = p;
+                piece.n = std::min(work.rows, sh.n_local - r0);
+                piece.x = x + r0 * sh.ld;
+                piece.out_f16 = out_f16 ? out_f16 + r0 * dim : nullptr;
+                piece.out_codes = out_codes ? out_codes + r0 * sh.m : nullptr;
+                piece.out_f32 = out_f32 ? out_f32 + r0 * dim : nullptr;
+                launch_pq_tc(*this, piece, metric, false, 4, tb);
+                tb.prepare_operand = false;
+            }
+            return;
+        }
     }
     if (launch_assign_reg(*this, p, metric, false, 4)) return;
     GenericParams g = {};

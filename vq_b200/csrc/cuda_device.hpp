@@ -29,6 +29,7 @@ class CudaDevice : public Device {
     ~CudaDevice() override;
 
     void *alloc(size_t bytes) override;
+    void *try_alloc(size_t bytes); // null when there is no room
     void release(void *p) override;
     void upload(void *dst, const void *src, size_t bytes) override;
     void download(void *dst, const void *src, size_t bytes) override;
@@ -153,7 +154,6 @@ class CudaDevice : public Device {
     void release_dense();
     void dense_decide(const float *x, size_t n, size_t dim, const float *codebook, size_t k, bool euclid, uint8_t *codes, uint32_t *changed,
                       unsigned long long *stats);
-    void *try_alloc(size_t bytes); // null when there is no room
     float *pq_scratch_ = nullptr;
     std::unique_ptr<PqTcMaps> pq_maps_; // of pq_scratch_
     float *rot_split_ = nullptr; // TF32 high and low parts of the rotation matrix of the current rotate_rows call (dim <= 128)
