@@ -56,6 +56,39 @@ def test_groups_that_are_not_full(oracle, m, sd):
     assert np.array_equal(pq.codebooks, cb_o)
 
 
+@pytest.mark.parametrize("k", [2, 16, 17, 33])
+@pytest.mark.parametrize("m,sd", [(7, 8), (5, 4)])
+def test_training_with_few_centroids_in_groups_that_are_not_full(oracle, m, sd, k):
+    """Encodes of these shapes leave few centroids to the CUDA-core kernels; training does not."""
+    rng = np.random.default_rng(k)
+    n, iters = 2_500, 5
+    x = rng.normal(size=(n, m * sd)).astype(np.float32)
+    so, sg = RecordingSeeder(7), RecordingSeeder(7)
+    init = so.init_pq(n, m, k)
+    sg.init_pq(n, m, k)
+    cb_o, _ = oracle.pq_fit(x, m, k, iters, init, so.draw)
+    pq = vq.ProductQuantizer.fit(x, m, k, iters, vq.Distance.Euclidean, 7, init_idx=init, draw=sg.draw, accumulate=vq.ACCUM_ORDERED)
+    assert np.array_equal(pq.codebooks, cb_o)
+
+
+@pytest.mark.parametrize("m,sd,n,euclid,cosine", [(7, 8, 30_000, 36, 20), (5, 4, 60_000, 40, 24), (4, 4, 60_000, 40, 24), (4, 4, 150_000, 2, 2), (9, 4, 20_000, 40, 24),
+                                                  (9, 4, 30_000, 2, 2), (8, 8, 30_000, 2, 2)])
+def test_encodes_take_the_kernels_that_are_faster(m, sd, n, euclid, cosine):
+    """One launch on the CUDA cores up to the line, three on the tensor cores from there on."""
+    import torch
+
+    ctx = vq.Context(0)
+    x = torch.rand(n, m * sd, device="cuda")
+    for distance, line in ((vq.Distance.Euclidean, euclid), (vq.Distance.SquaredEuclidean, euclid), (vq.Distance.CosineDistance, cosine)):
+        for k in (line - 1, line):
+            if k < 2:
+                continue
+            q = vq.ProductQuantizer.from_codebooks(np.random.default_rng(k).random((m, k, sd), dtype=np.float32), distance, ctx=ctx)
+            before = ctx.launch_count()
+            q.quantize(x)
+            assert ctx.launch_count() - before == (3 if k >= line else 1), (distance, k)
+
+
 CASES = ["far", "very_far", "many_far", "offset", "tight", "equal", "nan", "tiny", "huge", "far_rows"]
 
 

@@ -753,7 +753,8 @@ bool CudaDevice::pq_encode_ahead(const Shape &sh, const float *x, const float *c
     p.centroids = codebooks;
     p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
     p.out_vec = !out_f16 || (aligned16(out_f16) && sh.m * sh.sd % 8 == 0);
-    if (sh.n_local == 0 || !pq_tensor_enabled_ || !pq_tc_applicable(p, metric) || direct_encode_applicable(p, p.sd == 8 && p.m % 4 == 0)) return false;
+    if (sh.n_local == 0 || !pq_tensor_enabled_ || !pq_tc_applicable(p, metric) || !pq_tc_encode_pays(p, metric) || direct_encode_applicable(p, p.sd == 8 && p.m % 4 == 0))
+        return false;
     bop_fresh_ = nullptr;
     launch_pq_operand_b(*this, codebooks, p.m, p.k, p.sd, metric == M_COSINE, pq_scratch_);
     return true;
@@ -778,7 +779,7 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
     p.pv = (float)pm;
     p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
     p.out_vec = (!out_f16 || (aligned16(out_f16) && dim % 8 == 0)) && (!out_f32 || (aligned16(out_f32) && dim % 4 == 0));
-    const bool tensor = !cuda_cores_only && pq_tensor_enabled_ && pq_tc_applicable(p, metric);
+    const bool tensor = !cuda_cores_only && pq_tensor_enabled_ && pq_tc_applicable(p, metric) && pq_tc_encode_pays(p, metric);
     // (the lines of the one-launch kernel lie where it meets the other path; narrow or odd shapes keep that of the CUDA cores' kernels)
     if (direct_encode_applicable(p, tensor && p.sd == 8 && p.m % 4 == 0)) {
         launch_direct_encode(*this, p, metric);

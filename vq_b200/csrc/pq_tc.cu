@@ -923,6 +923,24 @@ bool pq_tc_applicable(const AssignParams &p, int metric)
            (reinterpret_cast<uintptr_t>(p.out_f16) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.out_f32) & 15u) == 0;
 }
 
+// The tensor kernel computes 128 columns whatever k is, in three launches; the CUDA-core kernels' one takes a time that grows with k.  Multiples
+// of four sub-spaces of 8 values stay here for every k.  Where the others meet, k for the CUDA-core kernels' time over this one's (15,000,
+// 60,000 and 300,000 rows):
+//   8-wide, Euclidean: m 5 .. 30 at k 24: 0.64 .. 0.92, 0.71 .. 1.05, 0.65 .. 1.01; 32: 0.73 .. 1.14, 0.86 .. 1.21, 0.78 .. 1.18;
+//       40: 0.83 .. 1.21, 1.04 .. 1.38, 0.92 .. 1.34 (m 13, 300,000 rows, k 16: 92 us there, 172 here; k 64: 227 and 173)
+//   8-wide, cosine: k 16: 0.63 .. 0.98, 0.80 .. 1.31, 0.97 .. 1.63; 24: 0.79 .. 1.23, 1.04 .. 1.70, 1.21 .. 2.04
+//   4-wide, m 4 .. 6, Euclidean: k 32: 0.68 .. 0.93, 0.74 .. 0.91, 0.91 .. 1.37; 40: 0.76 .. 0.93, 0.83 .. 0.99, 1.02 .. 1.48 (the last of
+//       each is m 4, whose group is full: 1.0 from k 2 on with 300,000 rows); cosine: k 24: 0.77 .. 1.04, 0.82 .. 1.14, 1.33 .. 1.81
+//   4-wide, m from 7 on: below 200,000 pairs (m 7 .. 13, 15,000 rows) k 16: 0.79 .. 1.07, 32: 0.89 .. 1.21, cosine k 16: 0.99 .. 1.20;
+//       above, every k of the range is faster here (m 16: 1.15 .. 2.4; m 9, 60,000 rows, k 16: 0.95)
+// Training passes are faster here for every k (2 .. 64, 30,000 and 300,000 rows: 0.97 .. 2.2).
+bool pq_tc_encode_pays(const AssignParams &p, int metric)
+{
+    if (p.sd == 8) return p.m % 4 == 0 || p.k >= (metric == M_COSINE ? 20 : 36);
+    const bool few = p.n * (unsigned long long)p.m < 200000u || p.m == 5 || p.m == 6 || (p.m == 4 && p.n < 150000u);
+    return !few || p.k >= (metric == M_COSINE ? 24 : 40);
+}
+
 size_t pq_tc_scratch_floats() { return SCRATCH_FLOATS; }
 size_t pq_tc_stats_offset_floats() { return OFF_STATS; }
 size_t pq_tc_code_bytes(size_t n, size_t m) { return n * m; }

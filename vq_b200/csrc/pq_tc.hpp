@@ -17,6 +17,8 @@ struct AssignParams;
 bool pq_tc_shape(size_t m, size_t sd, size_t k);
 // ... with 16-byte aligned row slices, for the Euclidean metrics or (encode) cosine
 bool pq_tc_applicable(const AssignParams &p, int metric);
+// whether an encode that the kernels can take is faster with them than on the CUDA cores
+bool pq_tc_encode_pays(const AssignParams &p, int metric);
 size_t pq_tc_scratch_floats();
 // bytes of the one-byte codes that an encode of n rows of m sub-spaces goes through
 size_t pq_tc_code_bytes(size_t n, size_t m);
