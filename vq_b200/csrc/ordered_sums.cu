@@ -178,8 +178,16 @@ static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const Cod
         const int w = sd <= 4 ? 4 : sd <= 8 ? 8 : sd <= 16 ? 16 : 32;
         const size_t units = ((size_t)k + 32 / w - 1) / (32 / w) * ((sd + 31) / 32);
         const dim3 grid((unsigned)((units + OS_WARPS - 1) / OS_WARPS), m);
+        // Up to a block per SM: launched while the kernel before them runs, the blocks would gather on the SMs that are free first and share
+        // one port for their scattered 16-byte copies.  They ask for half of an SM's shared memory, so that no two share one.  Fits of 5
+        // iterations, launched after the kernel before / overlapping it / like this: 60,000 rows, 16 sub-spaces of 4, k 16 1151 / 1545 / 962 us;
+        // 30,000 rows, 32 of 4, k 16 808 / 984 / 728; 10,000 rows, 8 of 4, k 16 371 / 321 / 321.  (Two to six blocks spread the same
+        // way: 64 of 4, k 64 8 % faster, 32 of 8, 2500 rows, k 256 3 % slower.)
+        const size_t rings = sizeof(WalkRing) * OS_WARPS;
+        const size_t spread = (size_t)grid.x * grid.y <= (size_t)dev.sm_count() && dev.smem_limit() / 2 > rings ? dev.smem_limit() / 2 - rings : 0;
         auto go = [&](auto kernel) {
-            launch_following(kernel, grid, 32 * OS_WARPS, 0, dev.stream(), x, n, sh.ld, m, k, sd, active, start, list, sums, counts, counts_f32);
+            if (spread) VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spread));
+            launch_following(kernel, grid, 32 * OS_WARPS, spread, dev.stream(), x, n, sh.ld, m, k, sd, active, start, list, sums, counts, counts_f32);
         };
         const bool vec = sd % 4 == 0 && sh.ld % 4 == 0 && reinterpret_cast<uintptr_t>(x) % 16 == 0; // whole 16-byte pieces
         if (w == 4) go(vec ? ordered_sums_kernel<4, true> : ordered_sums_kernel<4, false>);
