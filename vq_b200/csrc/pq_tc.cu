@@ -86,7 +86,7 @@ namespace vqb {
 
 namespace {
 
-constexpr int BM = 128, BN = 256, MAXM = 64, NTHREADS = 32 * (4 + 8 + 16);
+constexpr int BM = (int)PQ_TC_TILE, BN = 256, MAXM = 64, NTHREADS = 32 * (4 + 8 + 16);
 constexpr int QCAP = 64; // queue entries per epilogue warp: fewer than 32 wait, at most 32 are added at a time
 constexpr float COS_MIN = 1e-17f, COS_MAX = 1e18f;  // cosine: norms that the scores can be trusted for
 constexpr float RHO_MIN = 1e-14f, RHO_MAX = 1e15f;  // Euclidean: radii for which neither 2^+-96 scalings nor distances leave f32
@@ -911,14 +911,9 @@ template <int SD, bool COSINE> __global__ void __launch_bounds__(BN) pq_operand_
 
 } // namespace
 
-// Every number of sub-spaces from four on: the last group of a launch may hold fewer than four, and gets as many CTAs as it has work.
-// Against the CUDA-core kernels (assign_filter.cuh), encode / fit of 5 iterations: 1M rows, 32 of 4: 4.05 -> 0.82 / 18.8 -> 5.2 ms;
-// 300,000 rows, 13 of 8: 0.79 -> 0.23 / 4.1 -> 1.6 ms; 100,000 rows, 7 of 4, k 100, cosine: 124 -> 38 us.
-bool pq_tc_shape(size_t m, size_t sd, size_t k) { return (sd == 4 || sd == 8) && m >= 4 && m <= MAXM && k >= 2 && k <= BN; }
-
 bool pq_tc_applicable(const AssignParams &p, int metric)
 {
-    return (metric == M_SQ || metric == M_EUCLID || metric == M_COSINE) && pq_tc_shape(p.m, p.sd, p.k) && p.n >= 1 && p.n < (1ull << 32) &&
+    return (metric == M_SQ || metric == M_EUCLID || metric == M_COSINE) && pq_tc_shape(p.m, p.sd, p.k) && pq_tc_rows(p.n) &&
            p.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.centroids) & 15u) == 0 &&
            (reinterpret_cast<uintptr_t>(p.out_f16) & 15u) == 0 && (reinterpret_cast<uintptr_t>(p.out_f32) & 15u) == 0;
 }

@@ -7,15 +7,15 @@
 
 #include "iter_status.cuh"
 #include "peer_exchange.cuh"
+#include "pq_tc_shape.hpp"
 
 namespace vqb {
 
 class CudaDevice;
 struct AssignParams;
 
-// sub-space widths 4 and 8, 4 <= m <= 64, 2 <= k <= 256: what the kernels and the fused centroid update take ...
-bool pq_tc_shape(size_t m, size_t sd, size_t k);
-// ... with 16-byte aligned row slices, for the Euclidean metrics or (encode) cosine
+// pq_tc_shape is what the kernels and the fused centroid update take: for an assignment with pq_tc_rows and 16-byte aligned row slices, for the
+// Euclidean metrics or (encode) cosine
 bool pq_tc_applicable(const AssignParams &p, int metric);
 // whether an encode that the kernels can take is faster with them than on the CUDA cores
 bool pq_tc_encode_pays(const AssignParams &p, int metric);
