@@ -475,8 +475,9 @@ __global__ void __launch_bounds__(256) dense_codebook_kernel(const float *c, int
     next_kernel_may_start();
     const int j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const bool in = j < k;
-    float v[4];
-    load_piece<false>(v, c, j, lane, in, dim);
+    float v[4]; // (ordinary loads: a centroid update may come directly before)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = in && 4 * lane + e < dim ? c[(size_t)j * dim + 4 * lane + e] : 0.0f;
     FramePiece f = load_frame(frame, lane);
     if (!in) f.mu[0] = f.mu[1] = f.mu[2] = f.mu[3] = 0.0f;
     float a = store_image(image + (size_t)j * 2 * dimp, dimp, lane, v, f, true);

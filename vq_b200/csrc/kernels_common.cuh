@@ -18,7 +18,9 @@ enum : int { M_SQ = 0, M_EUCLID = 1, M_COSINE = 2, M_MANHATTAN = 3, M_CHEBYSHEV 
 #define VQB_MOVED_BITS 0x3F800000u
 
 // A kernel launched by launch_following: all earlier work of the stream is complete and visible from here on.  Every thread calls it,
-// before it touches global memory or leaves.
+// before it touches global memory or leaves.  What the kernel directly before may have written is not read through __ldg or const
+// __restrict__ pointers: those loads are for memory that nobody writes while the kernel is there, and it is there before its predecessor
+// ends.  (The work before that has ended when the predecessor lets this kernel start.)
 __device__ __forceinline__ void after_previous_kernel() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // All blocks that have got here (or left) let the next kernel of the stream, if launched that way, take the free places.
 __device__ __forceinline__ void next_kernel_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -18,8 +18,7 @@ namespace vqb {
 
 namespace {
 
-// (what an earlier kernel of the chain wrote is read through plain pointers: loads that the compiler may take for invariant could move
-// above after_previous_kernel())
+// (what the kernel before wrote is read with ordinary loads, also in row_walk.cuh: kernels_common.cuh, after_previous_kernel)
 constexpr int OL_WARPS = 8, OL_THREADS = 32 * OL_WARPS;
 constexpr unsigned OL_STEP = 1024;   // a chunk is a multiple of this many rows
 constexpr unsigned OL_CHUNKS = 64;   // at most about this many chunks: every list CTA reads the counts of all of them

@@ -32,7 +32,7 @@ __device__ __forceinline__ void walk_rows(WalkRing &ring, const float *x, size_t
 #pragma unroll
         for (int q = 0; q < NR; ++q) {
             const uint32_t at = block * WALK_BLOCK + q * W + sub;
-            of[q] = at < count ? __ldg(rows + at) : 0u;
+            of[q] = at < count ? rows[at] : 0u;
         }
     };
     auto issue = [&](const uint32_t(&of)[NR], uint32_t block, int batch) { // always closes a group: the number of pending ones stays fixed

@@ -83,7 +83,7 @@ __global__ void init_tree_kernel(size_t n, int splits, uint32_t *perm, NodeInfo 
 // ---- large nodes: one warp per (1024-row chunk, 32 dimensions), then one thread per (node, dimension) adds the node's chunk
 // sums in order and divides
 template <bool VEC>
-__global__ void __launch_bounds__(32 * WR_WARPS) chunk_sums_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
+__global__ void __launch_bounds__(32 * WR_WARPS) chunk_sums_kernel(const float *__restrict__ x, size_t dim, const uint32_t *perm,
                                                                    const LevelInfo *level, const ChunkInfo *chunks, float *partial)
 {
     __shared__ __align__(16) WalkRing ring[WR_WARPS];
@@ -118,7 +118,7 @@ __global__ void node_mean_kernel(const NodeInfo *nodes, const LevelInfo *level, 
 // ---- one warp per (node, 32 dimensions): the node's mean (MEAN: the sums of its 1024-row chunks one after the other) and, if
 // it is going to be split, its spread
 template <bool VEC>
-__global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm,
+__global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *__restrict__ x, size_t dim, const uint32_t *perm,
                                                                    const NodeInfo *nodes, const LevelInfo *level, float *centroids, float *spread)
 {
     __shared__ __align__(16) WalkRing ring[WR_WARPS];
@@ -303,7 +303,14 @@ __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const fl
             }
             return r;
         };
-        const float4 cc = load_piece(centroids + (size_t)node * dim + col0 + piece * 4);
+        float4 cc = make_float4(0.f, 0.f, 0.f, 0.f); // (node_mean_kernel may have written it while this kernel was already there: ordinary loads)
+        {
+            const float *c = centroids + (size_t)node * dim + col0 + piece * 4;
+            if (live > 0) cc.x = c[0];
+            if (live > 1) cc.y = c[1];
+            if (live > 2) cc.z = c[2];
+            if (live > 3) cc.w = c[3];
+        }
         // this lane's four dimensions 4 * piece + j, row position sub: a stage begins on 256 bytes, so the four-row group i lies at the
         // address of group 0 with i exchanged into bits 4 to 7
         uint32_t dst[4];
