@@ -165,10 +165,16 @@ int vqb_opq_cross_cov(vqb_ctx *ctx, const float *y, const float *x, size_t n, si
 
 /* Diagnostic for the tensor-core path of the product quantizer (sub-space width 8): the raw scores
  * |c_j|^2/2 - x.c_j of its operands (scores_out: n x m x 256, may be NULL), the codes the path produces (codes_out: n x m) and the number
- * of (row, sub-space) pairs it left to the reference's arithmetic.  Requires m % 4 == 0, 4 <= m <= 64, 2 <= k <= 256.
+ * of (row, sub-space) pairs it left to the reference's arithmetic.  Requires 4 <= m <= 64, 2 <= k <= 256.
  * No counterpart in the reference. */
 int vqb_pq_tensor_scores(vqb_ctx *ctx, const float *x, size_t n, size_t m, const float *codebooks, size_t k,
                          float *scores_out, uint32_t *codes_out, unsigned long long *marked_out);
+/* The whole numbers T = sigma S + K0 that it ranks the centroids by (t_out: n x m x 256; S = |c - mu|^2/2 - (x - mu).(c - mu), or
+ * -x.c/|c| for cosine), each row's sigma and K0 (frames_out: n x m x 2; sigma = 0: the row is left to the reference's arithmetic) and the
+ * sub-spaces' constants (consts_out: m x 32; 0 ..: -mu; 24 .. 31: bit mask of the centroids that are left out of the scale).  Sub-space
+ * widths 4 and 8, metric VQB_SQUARED_EUCLIDEAN, VQB_EUCLIDEAN or VQB_COSINE. */
+int vqb_pq_tensor_fixed_point(vqb_ctx *ctx, const float *x, size_t n, size_t m, size_t sub_dim, const float *codebooks, size_t k,
+                              int metric, float *t_out, float *frames_out, float *consts_out);
 
 /* ---- lbg_quantize (src/utils.rs:32-109) on `n` rows of width d:
  * init_idx = k row indices, centroids_out = k x d (host or device). ------- */

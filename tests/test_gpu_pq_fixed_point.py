@@ -89,6 +89,60 @@ def test_encodes_take_the_kernels_that_are_faster(m, sd, n, euclid, cosine):
             assert ctx.launch_count() - before == (3 if k >= line else 1), (distance, k)
 
 
+@pytest.mark.parametrize("metric", ["euclid", "cosine"])
+@pytest.mark.parametrize("case", ["uniform", "normal", "offset", "far", "tight", "small", "large"])
+@pytest.mark.parametrize("m,sd,k", [(6, 8, 256), (5, 4, 200), (4, 8, 100)])
+def test_fixed_point_scores_against_f64(ctx, m, sd, k, case, metric):
+    """What the decision rests on: T = sigma S + K0 cut to a whole number lies within (-1.25, 0.25) of its value, and within 0.17 of that for
+    the parts that are dropped or rounded before (the header of pq_tc.cu).  The cut is the tensor core's own, so it is measured here."""
+    import ctypes as C
+
+    from vq_b200 import _lib
+
+    rng = np.random.default_rng(m * k + len(case))
+    n = 3000
+    x = rng.normal(size=(n, m * sd)).astype(np.float32)
+    cb = rng.normal(size=(m, k, sd)).astype(np.float32)
+    if case == "uniform":
+        x, cb = rng.random(x.shape, dtype=np.float32), rng.random(cb.shape, dtype=np.float32)
+    elif case == "offset":
+        x, cb = x + np.float32(100), cb + np.float32(100)
+    elif case == "far":
+        cb[:, 7] *= 100
+        x[::3] *= 50
+    elif case == "tight":
+        where = rng.normal(size=(8, m, sd)).astype(np.float32) * 10
+        cb = (where[rng.integers(8, size=k)] + rng.normal(size=(k, m, sd)) * 1e-2).astype(np.float32).transpose(1, 0, 2).copy()
+        x = (where[rng.integers(8, size=n)] + rng.normal(size=(n, m, sd)) * 1e-2).astype(np.float32).reshape(n, m * sd)
+    elif case in ("small", "large"):
+        scale = np.float32(1e-6 if case == "small" else 1e6)
+        x, cb = x * scale, cb * scale
+    t, frames, consts = np.zeros((n, m, 256), np.float32), np.zeros((n, m, 2), np.float32), np.zeros((m, 32), np.float32)
+    rc = _lib.load().vqb_pq_tensor_fixed_point(ctx.handle, x.ctypes.data, n, m, sd, cb.ctypes.data, k, 2 if metric == "cosine" else 0, t.ctypes.data,
+                                               frames.ctypes.data, consts.ctypes.data)
+    assert rc == 0, _lib.load().vqb_last_error(ctx.handle).decode()
+    sigma, k0 = frames[:, :, :1].astype(np.float64), frames[:, :, 1:].astype(np.float64)
+    far = np.unpackbits(consts[:, 24:].copy().view(np.uint8), axis=1, bitorder="little")[:, :k].astype(bool)
+    assert (frames[:, :, 0] > 0).mean() > 0.99 and far.sum() <= (m if case == "far" else 0)
+    mu = -consts[:, :sd].astype(np.float64)
+    y, c = x.astype(np.float64).reshape(n, m, sd) - mu, cb.astype(np.float64) - mu[:, None]
+    if metric == "cosine":
+        assert not mu.any()
+        half, c = np.zeros((m, k)), c / np.linalg.norm(c, axis=-1, keepdims=True)
+    else:
+        half = 0.5 * (c * c).sum(-1)
+    exact = sigma * (half[None] - np.einsum("nmd,mkd->nmk", y, c)) + k0
+    use = (sigma > 0) & ~far[None]
+    error = np.where(use, t[:, :, :k] - exact, 0.0)
+    print(f"T - sigma S - K0: {error.min():.3f} .. {error.max():.3f}; T {t[:, :, :k][use].min()} .. {t[:, :, :k][use].max()}")
+    assert (t == np.floor(t)).all()
+    assert -1.25 - 0.17 < error.min() and error.max() < 0.25 + 0.17
+    assert (exact[use] > 8 - 1).all() and (exact[use] < 65400 + 1).all()
+    beyond = np.broadcast_to(sigma > 0, (n, m, 256)).copy()  # columns without a centroid, and those left out: above all others
+    beyond[:, :, :k] &= far[None]
+    assert (np.abs(t[beyond] - 57344) <= 1).all()
+
+
 CASES = ["far", "very_far", "many_far", "offset", "tight", "equal", "nan", "tiny", "huge", "far_rows"]
 
 

@@ -46,6 +46,7 @@ SIGNATURES = {
     "vqb_tsvq_destroy": (C.c_int, [_P]),
     "vqb_evaluate_f16": (C.c_int, [_P, _P, _P, _SZ, _SZ, _SZ, C.POINTER(C.c_float), C.POINTER(C.c_float)]),
     "vqb_pq_tensor_scores": (C.c_int, [_P, _P, _SZ, _SZ, _P, _SZ, _P, _P, _P]),
+    "vqb_pq_tensor_fixed_point": (C.c_int, [_P, _P, _SZ, _SZ, _SZ, _P, _SZ, C.c_int, _P, _P, _P]),
     "vqb_dense_dots": (C.c_int, [_P, _P, _SZ, _SZ, _P, _SZ, _P, _P]),
     "vqb_opq_rotate_rows": (C.c_int, [_P, _P, _SZ, _P, _SZ, _P]),
     "vqb_opq_cross_cov": (C.c_int, [_P, _P, _P, _SZ, _SZ, _P]),

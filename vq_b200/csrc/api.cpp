@@ -562,6 +562,22 @@ int vqb_pq_tensor_scores(vqb_ctx *ctx, const float *x, size_t n, size_t m, const
     });
 }
 
+int vqb_pq_tensor_fixed_point(vqb_ctx *ctx, const float *x, size_t n, size_t m, size_t sub_dim, const float *codebooks, size_t k, int metric, float *t_out,
+                              float *frames_out, float *consts_out)
+{
+    if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");
+    return locked(ctx, [&] {
+        if (!x || !codebooks || !t_out || !frames_out || !consts_out || n == 0) throw Error(VQB_ERR_BAD_ARGUMENT, "NULL or empty argument");
+        CudaDevice &dev = *ctx->dev;
+        In ix(dev, x, sizeof(float) * n * m * sub_dim), ic(dev, codebooks, sizeof(float) * m * k * sub_dim);
+        Out ot(dev, t_out, sizeof(float) * n * m * 256), of(dev, frames_out, sizeof(float) * n * m * 2), oc(dev, consts_out, sizeof(float) * m * 32);
+        dev.pq_fixed_point_debug(ix.as<float>(), n, m, sub_dim, ic.as<float>(), k, metric, ot.as<float>(), of.as<float>(), oc.as<float>());
+        ot.finish();
+        of.finish();
+        oc.finish();
+    });
+}
+
 int vqb_opq_rotate_rows(vqb_ctx *ctx, const float *rot, size_t dim, const float *x, size_t n, float *y_out)
 {
     if (!ctx) return set_err(nullptr, VQB_ERR_BAD_ARGUMENT, "ctx is NULL");

@@ -575,6 +575,32 @@ void CudaDevice::pq_tensor_debug(const float *x, size_t n, size_t m, const float
     *marked = after - before;
 }
 
+void CudaDevice::pq_fixed_point_debug(const float *x, size_t n, size_t m, size_t sd, const float *codebooks, size_t k, int metric, float *t, float *frames,
+                                      float *consts)
+{
+    AssignParams p = {};
+    p.x = x;
+    p.n = n;
+    p.ld = m * sd;
+    p.m = (int)m;
+    p.k = (int)k;
+    p.sd = (int)sd;
+    p.centroids = codebooks;
+    p.x_vec4 = 1;
+    if (!pq_tensor_enabled_ || !pq_tc_applicable(p, metric)) throw Error(103, "shape not covered by the product-quantizer tensor-core path");
+    bop_fresh_ = nullptr;
+    const PqCodes work(*this, n, m);
+    PqTcBuffers tb;
+    tb.scratch = pq_scratch_;
+    tb.maps = pq_maps_.get();
+    tb.codes = work.codes;
+    tb.error_word = tc_error_;
+    tb.dbg_scores = t;
+    tb.dbg_frames = frames;
+    launch_pq_tc(*this, p, metric, false, 4, tb);
+    copy(consts, pq_scratch_ + pq_tc_consts_offset_floats(), m * 32 * sizeof(float));
+}
+
 void CudaDevice::copy(void *dst, const void *src, size_t bytes)
 {
     if (!bytes) return;

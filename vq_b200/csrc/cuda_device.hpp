@@ -53,7 +53,6 @@ class CudaDevice : public Device {
     void end_arrival();
     bool svd_sweeps(double *gt, double *vt, size_t n) override;
     bool polar_rotation(const double *a_dev, size_t n, float *rot_dev) override;
-    // Zero-filled map of at least `bytes` bytes for the product-quantizer tensor kernel; its users leave it zero-filled.
     void patch_centroids(const Shape &sh, const float *x, uint64_t row_begin, const RowPatch *patches, size_t n_patches,
                          float *centroids, Comm *comm) override;
     void assign_train(const Shape &sh, const float *x, const float *centroids, void *codes, const uint32_t *active,
@@ -84,6 +83,9 @@ class CudaDevice : public Device {
     // Raw scores, codes and the number of pairs left to the exact scan of the product-quantizer tensor-core kernel.
     void pq_tensor_debug(const float *x, size_t n, size_t m, const float *codebooks, size_t k, float *scores, uint32_t *codes,
                          unsigned long long *marked);
+    // The fixed-point scores T of that kernel, the rows' sigma and K0, the sub-spaces' constants.
+    void pq_fixed_point_debug(const float *x, size_t n, size_t m, size_t sd, const float *codebooks, size_t k, int metric, float *t, float *frames,
+                              float *consts);
     // Reconstruction error and windowed recall@k of an f16 reconstruction (the reference's evaluation metrics).
     void evaluate_f16(const float *x, const uint16_t *q, size_t n, size_t dim, size_t k, float *mse_out, float *recall_out);
     void distance_rows(int metric, double p, const float *a, const float *b, size_t d, size_t n, float *out);

@@ -26,7 +26,8 @@
 //
 // Bound behind M.  In units of T (sigma (|x|^2 + rho^2) <= 65300, which covers sigma (|x| + rho)^2 / 2):
 //   last step: the tensor core aligns its addends to 2^23 and cuts each towards zero two bits below the unit (measured: 1, 2, 8 and
-//   16 fractional addends beside 2^23 give errors of 0.25 per addend and one unit downwards for the result).  2^23, K0 and the
+//   16 fractional addends beside 2^23 give errors of 0.25 per addend and one unit downwards for the result; how it cuts is not documented,
+//   so tests/test_gpu_pq_fixed_point.py measures T against f64: -1.02 .. 0.27 over both widths, cosine, offsets, far and tight centroids).  2^23, K0 and the
 //   padding are whole numbers, so that only the accumulator of the steps before is cut: error in (-1.25, 0.25)
 //   steps before: partial sums up to 2^16 in f32: 0.02 each; dropped xl.cl: sd * 8 * 4 * 2^-12 = 0.06, the low parts' rounding as much
 //   again; half norm in f32 9u and in two parts 2^-24: 0.04; x - mu and c - mu, u each: 0.01
@@ -137,7 +138,8 @@ struct PqTcParams {
     const float *sub; // [m][32]
     unsigned long long *stats;
     int *error;
-    float *dbg_scores;              // optional [n][m][256]
+    float *dbg_scores;              // optional [n][m][256]: scores, or T with
+    float *dbg_frames;              // [n][m][2]: sigma and K0
     uint16_t first[MAXM / 4 + 1];   // CTAs first[g] .. first[g + 1] - 1 serve group g
 };
 
@@ -337,7 +339,8 @@ __device__ __noinline__ bool pq_queue_drain(const PqTcParams &Q, const uint4 *qu
     return moved;
 }
 
-template <int SD, bool TRAIN, int METRIC, bool WIDE, bool DUMP>
+// DUMP: diagnostics in place of codes, 1: the chain's result without the fixed-point constants, as scores; 2: T itself and the rows' sigma and K0
+template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP>
 __global__ void __launch_bounds__(NTHREADS, 1)
     pq_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
                  const __grid_constant__ PqTcParams Q)
@@ -498,11 +501,16 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     lo[i] = pack_f16(fmaf(lo2(y[i]), f.mul, -lo2(head)), fmaf(hi2(y[i]), f.mul, -hi2(head)));
                 }
                 cc = pack_f16(f.cr, f.cr);
-                k0 = DUMP ? 0u : pack_f16(2048.0f, f.k0);
+                k0 = DUMP == 1 ? 0u : pack_f16(2048.0f, f.k0);
                 if (__any_sync(0xffffffffu, !f.ok)) { // (rarely: a vote instead of a select per word)
 #pragma unroll
                     for (int i = 0; i < SD / 2; ++i) hi[i] = f.ok ? hi[i] : 0u, lo[i] = f.ok ? lo[i] : 0u;
                     cc = f.ok ? cc : 0u, k0 = f.ok ? k0 : 0u;
+                }
+                if (DUMP == 2 && tile * (unsigned long long)BM + r < P.n) {
+                    float *o = Q.dbg_frames + ((tile * (unsigned long long)BM + r) * m + g * 4 + ss) * 2;
+                    o[0] = f.ok ? f.mul * sub[SUB_SCALE] : 0.0f;
+                    o[1] = __half2float(__float2half_rn(f.k0));
                 }
                 if (!mbar_wait(&bars->aempty[ss], (step & 1u) ^ 1u, abort_flag, Q.error, 11)) {
                     ok = false;
@@ -575,7 +583,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t v[32];
-                if (DUMP) { // diagnostic: the chain's result without the fixed-point constants, as scores
+                if (DUMP) {
                     const unsigned long long row = (unsigned long long)(tile0 + step * tstep) * BM + r;
                     float x[SD], sq[2] = {0.0f, 0.0f}, shift = 0.0f;
 #pragma unroll
@@ -595,7 +603,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         if (valid) {
                             float *o = Q.dbg_scores + ((size_t)row * m + s) * BN + half * 128 + c * 32;
 #pragma unroll
-                            for (int t = 0; t < 32; ++t) o[t] = half * 128 + c * 32 + t < k ? __uint_as_float(v[t]) / sigma - shift : 1e30f;
+                            for (int t = 0; t < 32; ++t) {
+                                if (DUMP == 2) o[t] = __uint_as_float(v[t]) - 8388608.0f;
+                                else o[t] = half * 128 + c * 32 + t < k ? __uint_as_float(v[t]) / sigma - shift : 1e30f;
+                            }
                         }
                     }
                 } else {
@@ -938,13 +949,14 @@ bool pq_tc_encode_pays(const AssignParams &p, int metric)
 
 size_t pq_tc_scratch_floats() { return SCRATCH_FLOATS; }
 size_t pq_tc_stats_offset_floats() { return OFF_STATS; }
+size_t pq_tc_consts_offset_floats() { return OFF_SUB; }
 size_t pq_tc_code_bytes(size_t n, size_t m) { return n * m; }
 
 struct PqMaps {
     CUtensorMap x, b1, b2;
 };
 
-template <int SD, bool TRAIN, int METRIC, bool WIDE, bool DUMP = false>
+template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP = 0>
 static void launch_w(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
 {
     auto kernel = pq_tc_kernel<SD, TRAIN, METRIC, WIDE, DUMP>;
@@ -987,7 +999,12 @@ template <int SD> static void launch_expand(CudaDevice &dev, const AssignParams 
 
 template <int SD> static void launch_sd(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid, int metric, bool train, const uint16_t *c16)
 {
-    if (q.dbg_scores) launch_w<SD, false, M_SQ, true, true>(dev, mp, q, grid);
+    if (q.dbg_frames) { // T itself, and nothing else
+        if (metric == M_COSINE) launch_w<SD, false, M_COSINE, true, 2>(dev, mp, q, grid);
+        else launch_w<SD, false, M_SQ, true, 2>(dev, mp, q, grid);
+        return;
+    }
+    if (q.dbg_scores) launch_w<SD, false, M_SQ, true, 1>(dev, mp, q, grid);
     if (train) {
         launch_t<SD, true, M_SQ>(dev, mp, q, grid);
         return;
@@ -1029,6 +1046,7 @@ void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train
     q.stats = reinterpret_cast<unsigned long long *>(b.scratch + OFF_STATS);
     q.error = b.error_word;
     q.dbg_scores = b.dbg_scores;
+    q.dbg_frames = b.dbg_frames;
     // one CTA per SM, shared out among the groups of four sub-spaces by what they hold: the last one may have fewer than four
     const unsigned long long tiles = (p.n + BM - 1) / BM;
     const unsigned ngroups = ((unsigned)p.m + 3) / 4;

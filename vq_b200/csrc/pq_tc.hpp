@@ -36,12 +36,14 @@ struct PqTcBuffers {
     uint8_t *codes = nullptr;     // encode: pq_tc_code_bytes(n, m) bytes of working memory
     int *error_word = nullptr;    // set when a bounded wait expires
     bool prepare_operand = true;  // false: scratch already holds operand B of p.centroids (written by launch_pq_update_centroids)
-    float *dbg_scores = nullptr;  // optional: n x m x 256 raw scores
+    float *dbg_scores = nullptr;  // optional: n x m x 256 raw scores, or with dbg_frames (n x m x 2: sigma, K0) the fixed-point ones and no codes
+    float *dbg_frames = nullptr;
 };
 void launch_pq_operand_b(CudaDevice &dev, const float *centroids, int m, int k, int sd, bool cosine, float *scratch);
 void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train, size_t code_bytes, const PqTcBuffers &b);
 // number of (row, sub-space) pairs the tensor kernel has left to the reference's arithmetic so far (first u64 of the statistics)
 size_t pq_tc_stats_offset_floats();
+size_t pq_tc_consts_offset_floats(); // the sub-spaces' constants, 32 each
 // centroid update + operand B of the next pass + the iteration's flags, one launch (m CTAs)
 void launch_pq_update_centroids(CudaDevice &dev, int m, int k, int sd, float *sums, uint32_t *counts, uint32_t *moved, bool counts_f32,
                                 const uint32_t *active, float *centroids, float *scratch, const StatusPage &sp, const PeerView &pv);
