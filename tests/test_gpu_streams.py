@@ -77,14 +77,14 @@ def test_a_captured_call_stays_out_of_the_order():
     assert torch.equal(codes, want_a) and torch.equal(got_b, want_b)
 
 
-@pytest.mark.parametrize("m,sd,k", [(16, 8, 256), (7, 8, 100), (9, 4, 60)])
-def test_a_captured_encode_has_working_memory_of_its_own(m, sd, k):
+@pytest.mark.parametrize("m,sd,k,n", [(16, 8, 256, 30_000), (7, 8, 100, 30_000), (9, 4, 60, 30_000), (16, 8, 256, 300_000), (13, 8, 40, 400_000)])
+def test_a_captured_encode_replays_after_larger_calls(m, sd, k, n):
     """The first call of a context may be a captured one, and its graph replays correctly after larger calls of the context and between
-    them: nothing that it works with is the context's to free."""
+    them: nothing that it works with is given back meanwhile.  (Codes of up to 4 MiB lie in the context, more in the graph.)"""
     import torch
-    x = torch.from_numpy(synth.uniform01(60_000, m * sd, 9)).cuda()
+    x = torch.from_numpy(synth.uniform01(2 * n, m * sd, 9)).cuda()
     books = synth.uniform01(m * k, sd, 3).reshape(m, k, sd)
-    rows = x[:30_000].clone()
+    rows = x[:n].clone()
     want, want_all = (vq.ProductQuantizer.from_codebooks(books, vq.Distance.Euclidean).quantize(r, return_codes=True) for r in (rows, x))
     ctx = vq.Context(0)
     q = vq.ProductQuantizer.from_codebooks(books, vq.Distance.Euclidean, ctx=ctx)
@@ -98,8 +98,8 @@ def test_a_captured_encode_has_working_memory_of_its_own(m, sd, k):
         assert torch.equal(codes, want[1]) and torch.equal(out, want[0])
         got = q.quantize(x, return_codes=True)  # larger than anything before it
         assert torch.equal(got[1], want_all[1]) and torch.equal(got[0], want_all[0])
-        rows.copy_(x[30_000:] if turn == 0 else x[:30_000])  # the graph reads its rows anew
+        rows.copy_(x[n:] if turn == 0 else x[:n])  # the graph reads its rows anew
         graph.replay()
-        assert torch.equal(codes, want_all[1][30_000:] if turn == 0 else want[1])
-        rows.copy_(x[:30_000])
+        assert torch.equal(codes, want_all[1][n:] if turn == 0 else want[1])
+        rows.copy_(x[:n])
     del graph

@@ -90,6 +90,7 @@ CudaDevice::~CudaDevice()
         if (stage_) cudaFreeHost(stage_);
         cudaFree(rot_split_);
         cudaFree(pq_scratch_);
+        cudaFree(pq_codes_);
         cudaFree(tc_stats_);
         cudaFree(tc_error_);
         if (status_host_) cudaFreeHost(status_host_);
@@ -392,7 +393,8 @@ void CudaDevice::download(void *dst, const void *src, size_t bytes, void *dst2, 
 void CudaDevice::ensure_tc_buffers()
 {
     if (tc_error_) return;
-    device_allocs_ += 4;
+    device_allocs_ += 5;
+    VQB_CUDA_CHECK(cudaMalloc(&pq_codes_, PQ_KEPT_CODES));
     VQB_CUDA_CHECK(cudaMalloc(&rot_split_, opq_tc_split_floats(128) * sizeof(float)));
     VQB_CUDA_CHECK(cudaMalloc(&pq_scratch_, pq_tc_scratch_floats() * sizeof(float)));
     VQB_CUDA_CHECK(cudaMemsetAsync(pq_scratch_, 0, pq_tc_scratch_floats() * sizeof(float), stream_));
@@ -524,26 +526,28 @@ void CudaDevice::dense_debug(const float *x, size_t n, size_t dim, const float *
     prepared_x_ = nullptr;
 }
 
-// The one-byte codes that an encode on the tensor path goes through.  They belong to the call, in the order of its stream: a call that is
-// being captured makes them part of its graph, which may then be replayed whatever other calls do meanwhile (a buffer that the
-// context keeps and grows is freed under a graph that holds its address, and cannot grow at all during a capture).
+// The one-byte codes that an encode on the tensor path goes through.  Up to PQ_KEPT_CODES bytes they lie in a buffer that the context has from
+// its creation to its end, like the operand tiles (taking them from the pool costs a call that is waited for 3 of 54 us: 60,001 x 96, m 12).
+// More belong to the call, in the order of its stream: a call that is being captured makes them part of its graph, which may then be
+// replayed whatever larger calls come (a buffer that grows is freed under a graph that holds its address, and cannot grow in a capture).
 struct PqCodes {
     CudaDevice &dev;
     size_t rows; // at a time: all of them, or a multiple of 128
-    uint8_t *codes;
-    PqCodes(CudaDevice &d, size_t n, size_t m) : dev(d), rows(n), codes(static_cast<uint8_t *>(d.alloc(pq_tc_code_bytes(n, m)))) {}
-    // As many rows as there is room for, but not less than `least`: none then, and codes is null.
-    PqCodes(CudaDevice &d, size_t n, size_t m, size_t least) : dev(d), rows(n), codes(nullptr)
+    uint8_t *codes, *own = nullptr;
+    // pieces: as many rows as there is room for.  (The kept buffer has room for some at any time.)
+    PqCodes(CudaDevice &d, size_t n, size_t m, bool pieces) : dev(d), rows(n), codes(nullptr)
     {
         static const char *cap = std::getenv("VQB_CODE_ROWS"); // at most so many rows' codes at a time (tests)
-        if (cap) rows = std::min(n, (size_t)std::strtoull(cap, nullptr, 10) / 128 * 128), least = std::min<size_t>(least, 128);
-        for (; rows >= std::min(n, least) && rows; rows = rows / 256 * 128) {
-            codes = static_cast<uint8_t *>(dev.try_alloc(pq_tc_code_bytes(rows, m)));
+        if (cap && pieces) rows = std::min(n, std::max<size_t>(128, std::strtoull(cap, nullptr, 10) / 128 * 128));
+        for (;; rows = rows / 256 * 128) {
+            const size_t bytes = pq_tc_code_bytes(rows, m);
+            if (bytes <= CudaDevice::PQ_KEPT_CODES) codes = dev.pq_kept_codes();
+            else codes = own = static_cast<uint8_t *>(pieces ? dev.try_alloc(bytes) : dev.alloc(bytes));
             if (codes) return;
         }
     }
     PqCodes(const PqCodes &) = delete;
-    ~PqCodes() { dev.release(codes); }
+    ~PqCodes() { dev.release(own); }
 };
 
 void CudaDevice::pq_tensor_debug(const float *x, size_t n, size_t m, const float *codebooks, size_t k, float *scores, uint32_t *codes,
@@ -566,7 +570,7 @@ void CudaDevice::pq_tensor_debug(const float *x, size_t n, size_t m, const float
     PqTcBuffers tb;
     tb.scratch = pq_scratch_;
     tb.maps = pq_maps_.get();
-    const PqCodes work(*this, n, m);
+    const PqCodes work(*this, n, m, false);
     tb.codes = work.codes;
     tb.error_word = tc_error_;
     tb.dbg_scores = scores;
@@ -589,7 +593,7 @@ void CudaDevice::pq_fixed_point_debug(const float *x, size_t n, size_t m, size_t
     p.x_vec4 = 1;
     if (!pq_tensor_enabled_ || !pq_tc_applicable(p, metric)) throw Error(103, "shape not covered by the product-quantizer tensor-core path");
     bop_fresh_ = nullptr;
-    const PqCodes work(*this, n, m);
+    const PqCodes work(*this, n, m, false);
     PqTcBuffers tb;
     tb.scratch = pq_scratch_;
     tb.maps = pq_maps_.get();
@@ -806,35 +810,31 @@ void CudaDevice::pq_encode_impl(const Shape &sh, const float *x, const float *co
     p.x_vec4 = aligned16(x) && (sh.ld % 4 == 0) && (sh.sd % 4 == 0);
     p.out_vec = (!out_f16 || (aligned16(out_f16) && dim % 8 == 0)) && (!out_f32 || (aligned16(out_f32) && dim % 4 == 0));
     const bool tensor = !cuda_cores_only && pq_tensor_enabled_ && pq_tc_applicable(p, metric) && pq_tc_encode_pays(p, metric);
-    // (the lines of the one-launch kernel lie where it meets the other path; narrow or odd shapes keep that of the CUDA cores' kernels)
+    // (the lines of the one-launch kernel: see there; narrow or odd shapes keep the one that was drawn against the CUDA cores' kernels)
     if (direct_encode_applicable(p, tensor && p.sd == 8 && p.m % 4 == 0)) {
         launch_direct_encode(*this, p, metric);
         return;
     }
     if (tensor) {
-        // Where memory is short the rows are taken piece by piece, and pieces of less than 32,768 rows (each is three launches) are left to
-        // the kernels that need no working memory.
-        const PqCodes work(*this, sh.n_local, sh.m, 32768);
-        if (work.codes) {
-            bop_fresh_ = nullptr;
-            PqTcBuffers tb;
-            tb.prepare_operand = !operand_there;
-            tb.scratch = pq_scratch_;
-            tb.maps = pq_maps_.get();
-            tb.codes = work.codes;
-            tb.error_word = tc_error_;
-            for (size_t r0 = 0; r0 < sh.n_local; r0 += work.rows) {
-                AssignParams piece = p;
-                piece.n = std::min(work.rows, sh.n_local - r0);
-                piece.x = x + r0 * sh.ld;
-                piece.out_f16 = out_f16 ? out_f16 + r0 * dim : nullptr;
-                piece.out_codes = out_codes ? out_codes + r0 * sh.m : nullptr;
-                piece.out_f32 = out_f32 ? out_f32 + r0 * dim : nullptr;
-                launch_pq_tc(*this, piece, metric, false, 4, tb);
-                tb.prepare_operand = false;
-            }
-            return;
+        bop_fresh_ = nullptr;
+        const PqCodes work(*this, sh.n_local, sh.m, true);
+        PqTcBuffers tb;
+        tb.prepare_operand = !operand_there;
+        tb.scratch = pq_scratch_;
+        tb.maps = pq_maps_.get();
+        tb.codes = work.codes;
+        tb.error_word = tc_error_;
+        for (size_t r0 = 0; r0 < sh.n_local; r0 += work.rows) { // piece by piece where memory is short
+            AssignParams piece = p;
+            piece.n = std::min(work.rows, sh.n_local - r0);
+            piece.x = x + r0 * sh.ld;
+            piece.out_f16 = out_f16 ? out_f16 + r0 * dim : nullptr;
+            piece.out_codes = out_codes ? out_codes + r0 * sh.m : nullptr;
+            piece.out_f32 = out_f32 ? out_f32 + r0 * dim : nullptr;
+            launch_pq_tc(*this, piece, metric, false, 4, tb);
+            tb.prepare_operand = false;
         }
+        return;
     }
     if (launch_assign_reg(*this, p, metric, false, 4)) return;
     GenericParams g = {};
@@ -1908,7 +1908,7 @@ bool CudaDevice::encode_cross_cov(const Shape &sh, const float *x, const float *
     PqTcBuffers tb;
     tb.scratch = pq_scratch_;
     tb.maps = pq_maps_.get();
-    const PqCodes work(*this, sh.n_local, sh.m);
+    const PqCodes work(*this, sh.n_local, sh.m, false);
     tb.codes = work.codes;
     tb.error_word = tc_error_;
     launch_pq_tc(*this, p, metric, false, 4, tb);

@@ -30,6 +30,9 @@ class CudaDevice : public Device {
 
     void *alloc(size_t bytes) override;
     void *try_alloc(size_t bytes); // null when there is no room
+    // Bytes of the buffer for the one-byte codes of a call (of 64 sub-spaces: 65,536 rows), which lives as long as the context.
+    static constexpr size_t PQ_KEPT_CODES = size_t(4) << 20;
+    uint8_t *pq_kept_codes() const { return pq_codes_; }
     void release(void *p) override;
     void upload(void *dst, const void *src, size_t bytes) override;
     void download(void *dst, const void *src, size_t bytes) override;
@@ -158,6 +161,7 @@ class CudaDevice : public Device {
                       unsigned long long *stats);
     float *pq_scratch_ = nullptr;
     std::unique_ptr<PqTcMaps> pq_maps_; // of pq_scratch_
+    uint8_t *pq_codes_ = nullptr;       // PQ_KEPT_CODES bytes
     float *rot_split_ = nullptr; // TF32 high and low parts of the rotation matrix of the current rotate_rows call (dim <= 128)
     bool opq_tensor_enabled_ = true;
     bool pq_tensor_enabled_ = false;
