@@ -147,10 +147,10 @@ int vqb_tsvq_destroy(vqb_tsvq *t);
 int vqb_evaluate_f16(vqb_ctx *ctx, const float *x, const uint16_t *q_f16, size_t n, size_t dim, size_t k,
                      float *mse_out, float *recall_out);
 
-/* Diagnostic for the tensor-core path used by full-width k-means (residual quantizer): the raw tcgen05 TF32 dot
- * products x_r . c_j (dots_out: n x 256, columns >= k are 0; may be NULL) and shortlist statistics
- * stats_out[3] = {rows, shortlisted candidates, rows that needed a full exact scan}.  Requires 32 <= dim <= 128,
- * dim % 32 == 0, 2 <= k <= 256.  No counterpart in the reference. */
+/* Diagnostic for the tensor-core path used by full-width k-means (residual quantizer): the raw tcgen05 dot
+ * products x_r . c_j of its binary16 images (dots_out: n x 256, columns >= k are 0; may be NULL) and shortlist statistics
+ * stats_out[3] = {rows, shortlisted candidates, rows that needed a full exact scan}.  Requires 17 <= dim <= 128,
+ * 2 <= k <= 256.  No counterpart in the reference. */
 int vqb_dense_dots(vqb_ctx *ctx, const float *x, size_t n, size_t dim, const float *codebook, size_t k,
                    float *dots_out, unsigned long long *stats_out);
 
@@ -240,7 +240,7 @@ int vqb_opq_quantize(vqb_opq *opq, const float *x, size_t n, size_t dim, uint16_
  * request loop: the rotated rows that vqb_opq_quantize keeps in pool memory live here in a fixed array inside
  * the library image (VQB_OPQ_STATIC_MAX_FLOATS floats = 4 MiB, resident on every GPU that loads the library,
  * for the life of the process), and the nearest-centroid step runs on the CUDA-core kernels, which work out of
- * shared memory and registers (the tensor-core kernel of vqb_opq_quantize needs operand tiles and a mark map in
+ * shared memory and registers (the tensor-core kernel of vqb_opq_quantize needs operand tiles and a byte per code in
  * device memory).  The call makes no cudaMalloc / cudaMallocAsync / cudaFree and creates no event, on its first
  * use of a context as on any later one (vqb_ctx_alloc_count stays unchanged across it).
  *   - x, out_f16 and codes must be DEVICE pointers (either output may be NULL, not both); host pointers are

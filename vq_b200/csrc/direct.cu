@@ -462,6 +462,9 @@ static void launch_any(CudaDevice &dev, DirectParams &p, int metric, int m)
 // Where the other kernels take over.  A thread looks at two centroids whatever k is, so this kernel's time follows (row, sub-space)
 // pairs and 2 tk = 64, 128 or 256.  Measured with rows on the GPU, from the call to its result and as one of many in a row (the
 // two agree within a few per cent):
+// These lines are of the kernels on the other side before launches overlapped and the tensor-core one became what it is (3000 x 128 now takes
+// 15.5 us there, in three launches), and before sub-spaces of 4 values and odd numbers of them went to it as well: they have not been
+// drawn anew since, and could lie lower.
 //   the tensor-core kernel (8-wide sub-spaces; 19 us in three launches as one of many, hardly dependent on the rows) passes at
 //       k 256: 10,900 .. 11,100 pairs (m 4, 8, 16, 32), k 200: 10,750, k 128: 15,900 .. 20,000, k 20, 40, 64: 27,100 .. 27,400
 //   the CUDA-core kernels (19 us up to k 20, 33 at 64, 40 .. 46 at 128, 66 .. 83 at 256, until their grids are full, some thousand

@@ -26,9 +26,10 @@
 //
 // Bound behind M.  In units of T (sigma (|x|^2 + rho^2) <= 65300, which covers sigma (|x| + rho)^2 / 2):
 //   last step: the tensor core aligns its addends to 2^23 and cuts each towards zero two bits below the unit (measured: 1, 2, 8 and
-//   16 fractional addends beside 2^23 give errors of 0.25 per addend and one unit downwards for the result; how it cuts is not documented,
-//   so tests/test_gpu_pq_fixed_point.py measures T against f64: -1.02 .. 0.27 over both widths, cosine, offsets, far and tight centroids).  2^23, K0 and the
-//   padding are whole numbers, so that only the accumulator of the steps before is cut: error in (-1.25, 0.25)
+//   16 fractional addends beside 2^23 give errors of 0.25 per addend and one unit downwards for the result).  2^23, K0 and the
+//   padding are whole numbers, so that only the accumulator of the steps before is cut: error in (-1.25, 0.25).  How it cuts is not
+//   documented, so tests/test_gpu_pq_fixed_point.py measures T against f64: -1.02 .. 0.27 in all, over both widths, cosine, offsets, far
+//   and tight centroids
 //   steps before: partial sums up to 2^16 in f32: 0.02 each; dropped xl.cl: sd * 8 * 4 * 2^-12 = 0.06, the low parts' rounding as much
 //   again; half norm in f32 9u and in two parts 2^-24: 0.04; x - mu and c - mu, u each: 0.01
 //   the reference's own arithmetic prefers w over a only if D_w <= D_a (1 + 4u) with (sd + 2)u each: 24u * 65300 = 0.1
@@ -61,9 +62,9 @@
 // Every wait is bounded; on expiry the CTA records a code, stops issuing, frees tensor memory and the host raises an error.
 //
 // Measured, 1M x 128, m 16, k 256: a training pass 0.643 (0.613 and 0.030 for the pairs left to an exact kernel) -> 0.38 ms, an
-// encode 0.682 -> 0.43 ms, against f32 scores of split-TF32 operands with one f32 minimum each.  Per unit 880 cycles; the parts
-// alone: hand-over of the barriers 500, with the producers 720, with the epilogue 860; the MMAs take 385, the minima 256 of a
-// scheduler's integer pipe.  What each choice brought (ms a pass, the others as they are):
+// encode to f16 rows 0.682 -> 0.43 ms (with 32-bit codes too 0.696 -> 0.470), against f32 scores of split-TF32 operands with one f32
+// minimum each.  Per unit 880 cycles; the parts alone: hand-over of the barriers 500, with the producers 720, with the epilogue 860; the
+// MMAs take 385, the minima 256 of a scheduler's integer pipe.  What each choice brought (ms a pass, the others as they are):
 //   * one issuer per accumulator half instead of one per accumulator (0.46), and those instead of one in all (0.71): a half is idle
 //     from its release until its issuer has seen it, and an issuer that waits for one half keeps the other waiting
 //   * eight producer warps instead of four (0.48): 150 dependent instructions a slice, 5 cycles each, are what a warp takes
