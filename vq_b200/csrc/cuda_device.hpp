@@ -30,8 +30,8 @@ class CudaDevice : public Device {
 
     void *alloc(size_t bytes) override;
     void *try_alloc(size_t bytes); // null when there is no room
-    // Bytes of the buffer for the one-byte codes of a call (of 64 sub-spaces: 65,536 rows), which lives as long as the context.
-    static constexpr size_t PQ_KEPT_CODES = size_t(4) << 20;
+    // Bytes of the buffer for the one-byte codes of a call (1M rows of 32 sub-spaces), which lives as long as the context.
+    static constexpr size_t PQ_KEPT_CODES = size_t(32) << 20;
     uint8_t *pq_kept_codes() const { return pq_codes_; }
     void release(void *p) override;
     void upload(void *dst, const void *src, size_t bytes) override;
