@@ -44,7 +44,7 @@
 // radius leaves f32; with a NaN in centroid 0, where the reference's scan starts, the answer is 0 without one.
 // (500,000 x 128, m 16, k 256, encode, before -> now: rows of normal values 358 -> 260 us; 64 clusters of standard deviation 0.05 / 0.001
 // and distance 1: 666 -> 480 / 6100 -> 1640 us; values around 100: 6400 -> 255 us, which the uncentred scores could not separate.  Ties,
-// 300,000 x 128: rows on centroids 212 -> 144, each centroid twice 3750 -> 254, four distinct centroids 3750 -> 1665, all equal 3745 -> 2430,
+// 300,000 x 128: rows on centroids 212 -> 144, each centroid twice 3750 -> 254, four distinct centroids 3750 -> 1665, all equal 3745 -> 2520,
 // rows and centroids of 0 and 1 2605 -> 1350 us.)
 //
 // Cosine (src/distances.rs:141-150).  1 - x.c / (|x| |c|) ranks like S_j = -x.(c_j / |c_j|), with the norm that the reference
@@ -303,30 +303,29 @@ __device__ __noinline__ bool pq_queue_drain(const PqTcParams &Q, const uint4 *qu
         }
     };
     // many candidates (ties): the lanes go through all centroids together, whose loads are then the same for all
-    const bool all = (e.w & Q_WHOLE) || __popc(e.z) * __popc(e.y >> 16) >= 256;
+    constexpr int U = 4; // distances in flight: each is a chain of additions
+    if (P.k < U && (e.w & Q_WHOLE)) e.y |= 0xFFFF0000u, e.z = 3u;
+    const bool all = P.k >= U && ((e.w & Q_WHOLE) || __popc(e.z) * __popc(e.y >> 16) >= 256);
     if (__float_as_uint(sub[SUB_FLAGS]) & SUB_NAN0) {
         nan0 = true;
     } else if (__any_sync(0xffffffffu, all)) {
-        constexpr int U = 4; // distances in flight: each is a chain of additions
         // in ascending order a centroid that is not below the best one's square cannot have the smaller root: the root is taken of new
-        // minima only (300,000 x 128, m 16, k 256, all centroids equal: encode 4.25 -> 2.43 ms with both changes, 4.04 with this one)
+        // minima only (300,000 x 128, m 16, k 256, all centroids equal: encode 4.25 -> 2.52 ms with both changes, 4.04 with this one)
         float best = VQB_INF;
-        auto take = [&](float d, int j) {
-            if (j == 0) nan0 = !(d == d);
-            if (d < best) {
-                const float r = METRIC == M_EUCLID ? __fsqrt_rn(d) : d;
-                if (r < bd) best = d, bd = r, bi = j;
-            }
-        };
-        int j = 0;
-        for (; j + U <= P.k; j += U) {
+        for (int j = 0;;) {
             float d[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) d[u] = distance(j + u);
+            if (j == 0) nan0 = !(d[0] == d[0]);
 #pragma unroll
-            for (int u = 0; u < U; ++u) take(d[u], j + u);
+            for (int u = 0; u < U; ++u)
+                if (d[u] < best) {
+                    const float r = METRIC == M_EUCLID ? __fsqrt_rn(d[u]) : d[u];
+                    if (r < bd) best = d[u], bd = r, bi = j + u;
+                }
+            if (j + U >= P.k) break;
+            j = min(j + U, P.k - U); // (some of the last step's a second time: none of them is below the best)
         }
-        for (; j < P.k; ++j) take(distance(j), j);
     }
     if (!all) {
         bd = VQB_INF, bi = 0x7fffffff, nan0 = false;
