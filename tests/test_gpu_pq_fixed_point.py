@@ -207,3 +207,26 @@ def test_training_on_values_that_strain_the_fixed_point(oracle, case):
     cb_o, _ = oracle.pq_fit(x, m, k, iters, init, so.draw)
     pq = vq.ProductQuantizer.fit(x, m, k, iters, vq.Distance.Euclidean, 3, init_idx=init, draw=sg.draw, accumulate=vq.ACCUM_ORDERED)
     assert np.array_equal(pq.codebooks, cb_o, equal_nan=True)
+
+
+@pytest.mark.parametrize("k", [2, 3, 4, 5, 7, 9])
+@pytest.mark.parametrize("case", ["equal", "equal_but_last", "wild_rows", "void"])
+def test_scans_of_all_centroids(oracle, case, k):
+    """Rows that look at every centroid, around the number of distances that are worked out at a time."""
+    rng = np.random.default_rng(k)
+    n, m = 9_000, 4
+    x = rng.normal(size=(n, m * 8)).astype(np.float32)
+    cb = rng.normal(size=(m, k, 8)).astype(np.float32)
+    if case.startswith("equal"):
+        cb[:] = cb[:, :1]
+        if case == "equal_but_last":
+            cb[:, -1] = np.nextafter(cb[:, -1], np.float32(100))
+    elif case == "wild_rows":
+        x[::3, ::5] = np.nan
+        x[1::3] *= np.float32(1e19)
+        x[5::7, 3] = np.inf
+    else:  # a radius that leaves f32: the whole sub-space is scanned
+        cb *= np.float32(1e-20)
+    with np.errstate(all="ignore"):
+        for metric in ((vq.Distance.Euclidean, ka.EUCLID), (vq.Distance.SquaredEuclidean, ka.SQ), (vq.Distance.CosineDistance, ka.COSINE)):
+            _check(oracle, cb, x, metric)
