@@ -10,6 +10,7 @@ INVARIANT = re.compile(r"\b(__ldg|load_piece(?:<\w+>)?|load_slice(?:<\w+>)?)\(")
 # `perm` of the spreads and splits were written two launches ago or earlier.
 ALLOWED = {
     "walk_rows": set(), "dense_codebook_kernel": set(), "dense_shortlist_kernel": set(), "update_centroids_kernel": set(), "pq_update_centroids_kernel": set(),
+    "rvq_stages_kernel": set(),  # (rows and codebooks by load4: written before the kernel in front of it)
     "pq_operand_b_kernel": set(), "pq_tc_kernel": {"P.x"}, "pq_queue_drain": {"P.x"}, "pq_expand_kernel": {"c16", "centroids"},
     "queue_sums_kernel": {"xp", "i"},  # (its load_piece takes a number)
     "resolve_kernel": {"x", "book", "c", "xr"}, "ordered_hist_kernel": set(), "ordered_lists_kernel": set(),

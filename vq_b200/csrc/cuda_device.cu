@@ -401,8 +401,8 @@ void CudaDevice::ensure_tc_buffers()
     pq_maps_.reset(new PqTcMaps(pq_tc_make_maps(pq_scratch_)));
     VQB_CUDA_CHECK(cudaMalloc(&tc_stats_, 3 * sizeof(unsigned long long)));
     VQB_CUDA_CHECK(cudaMemsetAsync(tc_stats_, 0, 3 * sizeof(unsigned long long), stream_));
-    VQB_CUDA_CHECK(cudaMalloc(&tc_error_, sizeof(int)));
-    VQB_CUDA_CHECK(cudaMemsetAsync(tc_error_, 0, sizeof(int), stream_));
+    VQB_CUDA_CHECK(cudaMalloc(&tc_error_, 16 * sizeof(int))); // the error word, and from the ninth on wait_words()
+    VQB_CUDA_CHECK(cudaMemsetAsync(tc_error_, 0, 16 * sizeof(int), stream_));
     unfinished_ = true; // the first call may come on another stream
 }
 
@@ -924,47 +924,16 @@ void CudaDevice::rvq_quantize(const float *x, size_t n, size_t dim, const float 
     g.out_codes = out_codes;
     g.stages = (int)stages;
     g.epsilon = epsilon;
-    const bool tensor = tensor_enabled_ && stages < 255 && dense_tc_applicable(dim, k, metric);
-    if (direct_rvq_applicable(g, tensor, smem_limit_)) {
-        launch_direct_rvq(*this, g, metric);
-        return;
-    }
-    if (tensor) {
-        // stage by stage: codes from the rows' images, then the residuals with their images for the next stage; the sums of the
-        // chosen centroids are formed from the codes at the end
-        const size_t res_bytes = stages > 1 ? sizeof(float) * dim : 0;
-        const DenseWork &w = dense_work(n, dim, res_bytes + stages + 1);
-        prepared_x_ = nullptr;
-        const size_t piece = std::min(n, dense_rows_);
-        float *res = (float *)alloc((res_bytes + stages + 1) * piece);
-        uint8_t *codes = (uint8_t *)res + res_bytes * piece;
-        for (size_t r0 = 0; r0 < n; r0 += piece) {
-            const size_t rows = std::min(piece, n - r0);
-            const float *xp = x + r0 * dim;
-            uint8_t *ended = codes + rows * stages;
-            VQB_CUDA_CHECK(cudaMemsetAsync(ended, 0xFF, rows, stream_));
-            dense_frame(*this, w, xp, rows, dim, nullptr, nullptr, true);
-            dense_prepare(*this, w, xp, rows, dim);
-            for (size_t st = 0; st < stages; ++st) {
-                const float *cb = codebooks + st * k * dim, *from = st ? res : xp;
-                dense_decide(from, rows, dim, cb, k, metric == M_EUCLID, codes + st * rows, nullptr, nullptr);
-                if (st + 1 == stages) break; // nothing looks at the last residual
-                RvqApply a;
-                a.x = from;
-                a.res = res;
-                a.n = rows;
-                a.dim = dim;
-                a.codebook = cb;
-                a.codes = codes + st * rows;
-                a.ended = ended;
-                a.stage = (int)st;
-                a.epsilon = epsilon;
-                rvq_apply(*this, a, w);
-            }
-            rvq_gather(*this, codes, ended, rows, dim, codebooks, k, (int)stages, out_f16 ? out_f16 + r0 * dim : nullptr,
-                       out_codes ? out_codes + r0 * stages : nullptr);
+    if (tensor_enabled_ && stages > 0 && dense_tc_applicable(dim, k, metric) && rvq_stages_pays(g)) {
+        ensure_tc_buffers();
+        if (void *work = try_alloc(rvq_stages_bytes(dim, k, stages))) {
+            launch_rvq_stages(*this, g, metric == M_EUCLID, work);
+            release(work);
+            return;
         }
-        release(res);
+    }
+    if (direct_rvq_applicable(g, smem_limit_)) {
+        launch_direct_rvq(*this, g, metric);
         return;
     }
     if (out_codes) VQB_CUDA_CHECK(cudaMemsetAsync(out_codes, 0xFF, sizeof(uint32_t) * n * stages, stream_));

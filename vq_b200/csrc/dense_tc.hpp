@@ -57,16 +57,14 @@ struct RvqApply {
     size_t n = 0, dim = 0;
     const float *codebook = nullptr;
     const uint8_t *codes = nullptr;
-    double *norm_sum = nullptr;  // training: the residual norms are added up (src/rvq.rs:131-138)
-    uint8_t *ended = nullptr;    // encode: number of stages of rows that have ended early (src/rvq.rs:204-207), else 255
-    int stage = 0;
-    float epsilon = 0.0f;
+    double *norm_sum = nullptr;  // the residual norms are added up (src/rvq.rs:131-138)
 };
 void rvq_apply(CudaDevice &dev, const RvqApply &a, const DenseWork &w);
 
-// Encode, at the end: sums of the chosen centroids in stage order as binary16 (src/rvq.rs:203,209-213) and the codes.
-// codes: [stages][n]; ended as above.
-void rvq_gather(CudaDevice &dev, const uint8_t *codes, const uint8_t *ended, size_t n, size_t dim, const float *codebooks, size_t k, int stages,
-                uint16_t *out_f16, uint32_t *out_codes);
+// The residual encoder with all its stages in one launch (rvq_tc.cu), for shapes that dense_tc_applicable takes.
+struct GenericParams;
+bool rvq_stages_pays(const GenericParams &g);                        // more rows than direct.cu is faster with
+size_t rvq_stages_bytes(size_t dim, size_t k, size_t stages);        // device memory that it needs
+void launch_rvq_stages(CudaDevice &dev, const GenericParams &g, bool euclid, void *work);
 
 } // namespace vqb

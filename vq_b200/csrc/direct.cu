@@ -491,18 +491,11 @@ void launch_direct_encode(CudaDevice &dev, const AssignParams &a, int metric)
     launch_any(dev, p, metric, a.m);
 }
 
-bool direct_rvq_applicable(const GenericParams &g, bool tensor, size_t smem_limit)
+// Against the CUDA-core kernel this one is ahead at every size that was measured (Manhattan, 80,000 x 128, k 256, 8 stages:
+// 7.2 -> 2.8 ms; cosine: 10.1 -> 2.4 ms).  Where the tensor-core kernel takes over: rvq_stages_pays (rvq_tc.cu).
+bool direct_rvq_applicable(const GenericParams &g, size_t smem_limit)
 {
-    if (g.k > DK_MAX || std::max(direct_smem(8, direct_tk(g.k), g.sd, true), direct_smem(1, direct_tk(g.k), g.sd, true)) > smem_limit - STATIC_SMEM) return false;
-    // Against the CUDA-core kernel this one is ahead at every size that was measured (Manhattan, 80,000 x 128, k 256, 8 stages:
-    // 7.2 -> 2.8 ms; cosine: 10.1 -> 2.4 ms).  The tensor-core path takes about 45 us a stage up to 20,000 rows (five launches), of
-    // which little depends on the rows' width or on k; the two meet at these rows (8 stages; 2 stages within 6 %):
-    //   2 tk 256:  12,700 of 128, 16,600 of 96, 22,400 of 64, 31,700 of 32, 12,300 of 61 (no whole 16-byte pieces: no TMA)
-    //   2 tk 128:  29,900 of 128, 34,400 of 61          2 tk 64:  46,400 of 128, 107,000 of 40, 115,000 of 32, 97,000 of 24
-    if (!tensor) return true;
-    const int tk = direct_tk(g.k), dc = chunk_dims(g.sd), width = (g.sd + dc - 1) / dc * dc;
-    const double rows = (tk == 128 ? 2.0e6 : tk == 64 ? 4.6e6 : 6.8e6) / (width + 32);
-    return (double)g.n <= (whole_pieces(g.sd, g.centroids) ? rows : 0.6 * rows);
+    return g.k <= DK_MAX && std::max(direct_smem(8, direct_tk(g.k), g.sd, true), direct_smem(1, direct_tk(g.k), g.sd, true)) <= smem_limit - STATIC_SMEM;
 }
 
 void launch_direct_rvq(CudaDevice &dev, const GenericParams &g, int metric)

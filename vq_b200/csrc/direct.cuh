@@ -15,7 +15,7 @@ bool direct_encode_applicable(const AssignParams &p, bool tensor);
 void launch_direct_encode(CudaDevice &dev, const AssignParams &p, int metric);
 
 // The same for the residual encoder: all stages of a row in one launch.  g.m == 1, g.centroids [stages][k][sd].
-bool direct_rvq_applicable(const GenericParams &g, bool tensor, size_t smem_limit);
+bool direct_rvq_applicable(const GenericParams &g, size_t smem_limit);
 void launch_direct_rvq(CudaDevice &dev, const GenericParams &g, int metric);
 
 } // namespace vqb

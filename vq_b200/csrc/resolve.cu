@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256) resolve_kernel(const float *__restrict__ 
 // images; the codebook's rows come from L2.
 template <int L, bool VEC>
 __global__ void __launch_bounds__(256) rvq_apply_kernel(const float *x, float *res, unsigned long long n, int dim, int dimp, const float *__restrict__ book,
-                                                        const uint8_t *__restrict__ codes, double *norm_sum, uint8_t *ended, int stage, float epsilon,
+                                                        const uint8_t *__restrict__ codes, double *norm_sum,
                                                         const float *frame, uint16_t *image, float *norms)
 {
     const int lane = threadIdx.x & 31, piece = lane % L;
@@ -91,8 +91,7 @@ __global__ void __launch_bounds__(256) rvq_apply_kernel(const float *x, float *r
     const unsigned long long step = (unsigned long long)gridDim.x * (256 / L);
     double total = 0.0;
     for (unsigned long long row = blockIdx.x * (unsigned long long)(256 / L) + threadIdx.x / L; row - threadIdx.x / L < n; row += step) {
-        bool in = row < n;
-        if (ended && in) in = ended[row] > stage; // the other rows have ended: nothing of them changes
+        const bool in = row < n;
         float v[4], c[4];
         const int code = in ? (int)codes[row] : 0;
         if (VEC) {
@@ -126,62 +125,11 @@ __global__ void __launch_bounds__(256) rvq_apply_kernel(const float *x, float *r
         }
         if (norm_sum && in && piece == 0) total += (double)sqrtf(a);
         if (in && piece == 0) norms[row] = fa * 1.00001f; // an upper bound is what the shortlist needs
-        if (ended) {
-            // The reference compares the root of the SERIAL sum of squares (src/rvq.rs:204-207), which lies within 2 dim 2^-24 of this
-            // one: only a row that close to epsilon is added up in order.
-            const float nrm = sqrtf(a), slack = 1e-4f * epsilon;
-            bool below = nrm < epsilon - slack;
-            const bool close = in && !below && !(nrm > epsilon + slack);
-            __syncwarp(); // the row's residual is in memory for the lane that may read it
-            if (close && piece == 0) {
-                float s = 0.0f;
-                for (int i = 0; i < dim; ++i) {
-                    const float r = *reinterpret_cast<volatile float *>(res + row * dim + i);
-                    s = __fadd_rn(s, __fmul_rn(r, r));
-                }
-                below = __fsqrt_rn(s) < epsilon;
-            }
-            if (in && piece == 0 && below) ended[row] = (uint8_t)(stage + 1);
-            __syncwarp();
-        }
     }
     if (norm_sum) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
         if (lane == 0 && total != 0.0) atomicAdd(norm_sum, total);
-    }
-}
-
-template <int L, bool VEC>
-__global__ void __launch_bounds__(256) rvq_gather_kernel(const uint8_t *__restrict__ codes, const uint8_t *__restrict__ ended, unsigned long long n, int dim,
-                                                         const float *__restrict__ books, int k, int stages, uint16_t *out_f16, uint32_t *out_codes)
-{
-    const int piece = (threadIdx.x & 31) % L;
-    const unsigned long long step = (unsigned long long)gridDim.x * (256 / L);
-    for (unsigned long long row = blockIdx.x * (unsigned long long)(256 / L) + threadIdx.x / L; row < n; row += step) {
-        const int last = min(stages, (int)ended[row]);
-        float q[4] = {0.f, 0.f, 0.f, 0.f};
-        if (out_f16) {
-#pragma unroll 4
-            for (int st = 0; st < last; ++st) {
-                float c[4];
-                load_piece<VEC>(c, books + (size_t)st * k * dim, codes[(size_t)st * n + row], piece, true, dim);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) q[e] = __fadd_rn(q[e], c[e]);
-            }
-            uint16_t *o = out_f16 + row * dim + 4 * piece;
-            if (VEC) {
-                if (4 * piece < dim)
-                    *reinterpret_cast<uint2 *>(o) = make_uint2((uint32_t)f32_to_f16_bits(q[0]) | ((uint32_t)f32_to_f16_bits(q[1]) << 16),
-                                                               (uint32_t)f32_to_f16_bits(q[2]) | ((uint32_t)f32_to_f16_bits(q[3]) << 16));
-            } else {
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (4 * piece + e < dim) o[e] = f32_to_f16_bits(q[e]);
-            }
-        }
-        if (out_codes)
-            for (int st = piece; st < stages; st += L) out_codes[row * stages + st] = st < last ? (uint32_t)codes[(size_t)st * n + row] : 0xFFFFFFFFu;
     }
 }
 
@@ -224,21 +172,7 @@ void rvq_apply(CudaDevice &dev, const RvqApply &a, const DenseWork &w)
     with_lanes(dimp, a.dim % 4 == 0 && aligned(a.x, 16) && aligned(a.res, 16) && aligned(a.codebook, 16), [&](auto lanes, auto vec) {
         constexpr int L = decltype(lanes)::value;
         rvq_apply_kernel<L, decltype(vec)::value><<<grid_rows(dev, a.n, L), 256, 0, dev.stream()>>>(
-            a.x, a.res, a.n, (int)a.dim, (int)dimp, a.codebook, a.codes, a.norm_sum, a.ended, a.stage, a.epsilon, w.frame, w.image, w.norms);
-    });
-    VQB_CUDA_CHECK(cudaGetLastError());
-    dev.count_launch();
-}
-
-void rvq_gather(CudaDevice &dev, const uint8_t *codes, const uint8_t *ended, size_t n, size_t dim, const float *codebooks, size_t k, int stages,
-                uint16_t *out_f16, uint32_t *out_codes)
-{
-    if (n == 0) return;
-    KernelScope ks(dev, "rvq_gather");
-    with_lanes(dense_padded(dim), dim % 4 == 0 && aligned(codebooks, 16) && aligned(out_f16, 8), [&](auto lanes, auto vec) {
-        constexpr int L = decltype(lanes)::value;
-        rvq_gather_kernel<L, decltype(vec)::value><<<grid_rows(dev, n, L), 256, 0, dev.stream()>>>(codes, ended, n, (int)dim, codebooks, (int)k, stages,
-                                                                                               out_f16, out_codes);
+            a.x, a.res, a.n, (int)a.dim, (int)dimp, a.codebook, a.codes, a.norm_sum, w.frame, w.image, w.norms);
     });
     VQB_CUDA_CHECK(cudaGetLastError());
     dev.count_launch();
