@@ -126,10 +126,16 @@ __global__ void __launch_bounds__(256) rvq_apply_kernel(const float *x, float *r
         if (norm_sum && in && piece == 0) total += (double)sqrtf(a);
         if (in && piece == 0) norms[row] = fa * 1.00001f; // an upper bound is what the shortlist needs
     }
-    if (norm_sum) {
+    if (norm_sum) { // one atomic a CTA: one a warp, on the one address, took 45 us of 58 for 33,506 rows
+        __shared__ double s_total[8];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-        if (lane == 0 && total != 0.0) atomicAdd(norm_sum, total);
+        if (lane == 0) s_total[threadIdx.x >> 5] = total;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < 8; ++w) total += s_total[w];
+            if (total != 0.0) atomicAdd(norm_sum, total);
+        }
     }
 }
 
