@@ -38,7 +38,7 @@ namespace {
 constexpr int DT = 256;  // threads of a CTA: DT / TK groups of TK threads, each group with its own R rows
 constexpr int DC = 16;   // dimensions of a codebook chunk
 constexpr int DK_MAX = 256;
-constexpr size_t STATIC_SMEM = 8192; // more than the kernels' own shared arrays
+constexpr size_t STATIC_SMEM = 8192; // more than the kernels' own shared arrays, which count towards the 48 KiB of a launch that asks for no more
 
 struct DirectParams {
     const float *x;
@@ -418,7 +418,7 @@ template <int METRIC, int R> static void launch_rows(CudaDevice &dev, const CUte
     const size_t smem = direct_smem(R, p.tk, p.sd, p.stages > 0);
     static std::atomic<unsigned long long> configured{0}; // bit d: the attribute has been set on device d (it is per device and sticky)
     const unsigned long long bit = 1ull << (dev.device() & 63);
-    if (smem > 48 * 1024 && !(configured.load(std::memory_order_relaxed) & bit)) {
+    if (smem + STATIC_SMEM > 48 * 1024 && !(configured.load(std::memory_order_relaxed) & bit)) {
         VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(dev.smem_limit() - STATIC_SMEM)));
         configured.fetch_or(bit, std::memory_order_relaxed);
     }
