@@ -1841,10 +1841,13 @@ void CudaDevice::cross_cov(const float *y, const float *x, size_t n, size_t dim,
         launch_opq_cross_cov(*this, y, x, n, dim, a, tc_error_);
         return;
     }
-    const unsigned long long rows_per_cta = 2048;
+    // Four CTAs a SM as long as each still has 64 rows for the dim x dim f64 atomics at its end, and at most 2048, whose sums are f32.  (A
+    // fixed 2048 left 6 CTAs of 12,369 x 40: 220 us, now 20; 45,000 x 104 238 -> 73.)
+    const unsigned tiles = (unsigned)((dim + 63) / 64);
+    const unsigned long long wanted = std::max(1ull, (unsigned long long)sm_count_ * 4 / ((unsigned long long)tiles * tiles));
+    const unsigned long long rows_per_cta = std::min<unsigned long long>(2048, std::max<unsigned long long>(64, ((n + wanted - 1) / wanted + 15) / 16 * 16));
     const unsigned long long splits = (n + rows_per_cta - 1) / rows_per_cta;
     const unsigned long long slab = 65535ull;
-    const unsigned tiles = (unsigned)((dim + 63) / 64);
     for (unsigned long long z0 = 0; z0 < splits; z0 += slab) {
         const unsigned long long zs = std::min(slab, splits - z0);
         const unsigned long long r0 = z0 * rows_per_cta;

@@ -373,8 +373,10 @@ __device__ __forceinline__ void polar_max(double v, unsigned long long *out, dou
 
 template <int KC, int CTAS_PER_SM>
 __global__ void __launch_bounds__(POLAR_TILE *POLAR_TILE, CTAS_PER_SM)
-    polar_iterate_kernel(const double *a, int n, PolarWork w, float *rot, int max_steps, const __grid_constant__ PolarSteps steps)
+    polar_iterate_kernel(const double *a, int dim, int n, PolarWork w, float *rot, int max_steps, const __grid_constant__ PolarSteps steps)
 {
+    // dim: the matrix as it is; n: whole tiles.  The rows and columns beyond it are zeros, which every step leaves zeros, and do not count as
+    // missing from the identity.
     __shared__ __align__(16) PolarTiles<KC> tiles;
     __shared__ double red[8];
     __shared__ int failed_sh;
@@ -385,17 +387,18 @@ __global__ void __launch_bounds__(POLAR_TILE *POLAR_TILE, CTAS_PER_SM)
     if (threadIdx.x == 0) failed_sh = 0;
     // scale^2 = |a|_1 |a|_inf: a warp per row sum or column sum
     double best[2] = {0.0, 0.0};
-    for (unsigned int v = (blockIdx.y * gridDim.x + blockIdx.x) * 8u + (threadIdx.x >> 5); v < 2u * (unsigned)n; v += 8u * ctas) {
-        const bool column = v >= (unsigned)n;
-        const size_t first = column ? v - (unsigned)n : (size_t)v * n, step = column ? (size_t)n : 1;
+    for (unsigned int v = (blockIdx.y * gridDim.x + blockIdx.x) * 8u + (threadIdx.x >> 5); v < 2u * (unsigned)dim; v += 8u * ctas) {
+        const bool column = v >= (unsigned)dim;
+        const size_t first = column ? v - (unsigned)dim : (size_t)v * dim, step = column ? (size_t)dim : 1;
         double sum = 0.0;
 #pragma unroll 4
-        for (int u = threadIdx.x & 31; u < n; u += 32) sum += fabs(__ldcg(a + first + u * step));
+        for (int u = threadIdx.x & 31; u < dim; u += 32) sum += fabs(__ldcg(a + first + u * step));
         for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
         best[column] = fmax(best[column], sum); // (a NaN is passed over)
     }
     double *cur = w.x0, *nxt = w.x1;
-    double own = __ldcg(a + (size_t)j * n + i); // this thread's entry of the iterate; X_0 = A^T inv, the factor applied in step 0
+    const bool inside = i < dim && j < dim;
+    double own = inside ? __ldcg(a + (size_t)j * dim + i) : 0.0; // this thread's entry of the iterate; X_0 = A^T inv, the factor applied in step 0
     cur[(size_t)i * n + j] = own;
     polar_max(best[0], w.scale, red);
     __syncthreads();
@@ -409,7 +412,7 @@ __global__ void __launch_bounds__(POLAR_TILE *POLAR_TILE, CTAS_PER_SM)
         // b = X^T X, tile (i-block, j-block), and the step's residual
         const double b = polar_tile<KC, false>(cur, cur, n, i0, j0, tiles) * inv * inv;
         w.b[(size_t)i * n + j] = b;
-        const double dev = fabs(b - (i == j ? 1.0 : 0.0));
+        const double dev = fabs(b - (i == j && inside ? 1.0 : 0.0));
         polar_max(dev == dev ? dev : 1e300, w.resid + step, red);
         if (!polar_grid_barrier(w, ++round, ctas, &failed_sh)) return;
         // nxt = ca X - cb X b, tile (i-block, j-block); the residual arrives with its operands
@@ -426,7 +429,7 @@ __global__ void __launch_bounds__(POLAR_TILE *POLAR_TILE, CTAS_PER_SM)
         cur = nxt;
         nxt = t;
     }
-    rot[(size_t)i * n + j] = (float)(own * inv);
+    if (inside) rot[(size_t)i * dim + j] = (float)(own * inv);
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         w.status[0] = resid < 1e-11 ? 1 : 0;
         w.status[1] = step;
@@ -441,9 +444,10 @@ __global__ void polar_finish_kernel(const double *x, int count, float *rot)
 
 } // namespace
 
-bool CudaDevice::polar_rotation(const double *a_dev, size_t n, float *rot_dev)
+bool CudaDevice::polar_rotation(const double *a_dev, size_t dim, float *rot_dev)
 {
-    if (n == 0 || n % POLAR_TILE != 0 || n > 512) return false;
+    if (dim == 0 || dim > 512) return false;
+    const size_t n = (dim + POLAR_TILE - 1) / POLAR_TILE * POLAR_TILE;
     const size_t bytes = sizeof(double) * n * n;
     const int max_steps = 96;
     {
@@ -475,9 +479,9 @@ bool CudaDevice::polar_rotation(const double *a_dev, size_t n, float *rot_dev)
                 KernelScope ks(*this, "polar_rotation");
                 VQB_CUDA_CHECK(cudaMemsetAsync(w.resid, 0, extra, stream_));
                 const dim3 grid((unsigned)(n / POLAR_TILE), (unsigned)(n / POLAR_TILE));
-                int n_i = (int)n, steps_i = max_steps;
+                int dim_i = (int)dim, n_i = (int)n, steps_i = max_steps;
                 PolarSteps steps = polar_steps(1e-4);
-                void *args[] = {(void *)&a_dev, (void *)&n_i, (void *)&w, (void *)&rot_dev, (void *)&steps_i, (void *)&steps};
+                void *args[] = {(void *)&a_dev, (void *)&dim_i, (void *)&n_i, (void *)&w, (void *)&rot_dev, (void *)&steps_i, (void *)&steps};
                 VQB_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)kernel, grid, dim3(POLAR_TILE * POLAR_TILE), args, 0, stream_));
                 count_launch();
             }
@@ -487,6 +491,7 @@ bool CudaDevice::polar_rotation(const double *a_dev, size_t n, float *rot_dev)
             return status[0] == 1;
         }
     }
+    if (dim != n) return false; // the launches below take whole tiles
     double *x0 = static_cast<double *>(alloc(bytes)), *x1 = static_cast<double *>(alloc(bytes)), *b = static_cast<double *>(alloc(bytes));
     double *fro2 = static_cast<double *>(alloc(sizeof(double)));
     unsigned long long *resid = static_cast<unsigned long long *>(alloc(sizeof(unsigned long long) * 2));
