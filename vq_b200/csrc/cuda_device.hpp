@@ -205,6 +205,21 @@ struct KernelScope {
     }
 };
 
+// As launch_following (below), in clusters of CTAs along x.
+template <typename... P, typename... A>
+void launch_following_clusters(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, cudaStream_t stream, A &&...args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
+    cudaLaunchAttribute attr[2] = {};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster, attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr, cfg.numAttrs = cluster > 1 ? 2 : 1;
+    VQB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+
 // Launches a kernel that may start while the one before it in the stream still runs: it waits itself (after_previous_kernel() of
 // kernels_common.cuh, before its first access to global memory), so that its launch and set-up overlap the other's end.  Between two
 // small kernels that takes 1 to 3 us off: encode of 3000 / 20,000 x 128 (three kernels) 20.9 -> 15.5 / 28.4 -> 24.1 us, fit of 2500 /
@@ -213,13 +228,7 @@ struct KernelScope {
 template <typename... P, typename... A>
 void launch_following(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args)
 {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid, cfg.blockDim = block, cfg.dynamicSmemBytes = smem, cfg.stream = stream;
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr, cfg.numAttrs = 1;
-    VQB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    launch_following_clusters(kernel, grid, block, smem, 1, stream, static_cast<A &&>(args)...);
 }
 
 // assign_launch.cu

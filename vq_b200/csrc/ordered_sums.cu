@@ -4,10 +4,13 @@
 // stable counting sort (two passes over the codes), and then every cluster walks its own list:
 //   ordered_hist_kernel     rows per (chunk of rows, cluster)
 //   ordered_lists_kernel    where each chunk's rows of a cluster start, then the row numbers themselves, ascending
+//   ordered_lists_cluster_kernel  both of these, up to 65,536 rows and 1024 clusters
 //   ordered_sums_kernel     one lane per (cluster, dimension) adds the cluster's rows in list order
 //   ordered_sums_long_kernel the same with eight warps per list, for wide rows
 // The work is O(n) per sub-space.  Walking all n codes once per (cluster, dimension), as this did before, cost 0.44 ms per pass
 // at 10,000 x 128, m 16, k 256 and 1.5 ms at 33,506 x 128, k 62; three launches of this file take ~0.02 ms and ~0.05 ms.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "cuda_device.hpp"
@@ -16,6 +19,8 @@
 #include "row_walk.cuh"
 
 namespace vqb {
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -117,6 +122,105 @@ __global__ void __launch_bounds__(OL_THREADS) ordered_lists_kernel(const CodeT *
         }
         __syncwarp();
     }
+}
+
+// Both steps in one launch: a cluster of CTAs per sub-space, which exchange their counts through distributed shared memory.
+constexpr int OC_CTAS = 8, OC_WARPS = 16, OC_THREADS = 32 * OC_WARPS, OC_MAX_K = 1024; // counters of sixteen warps: 64 KiB
+constexpr unsigned OC_STEPS = 16, OC_MAX_ROWS = OC_CTAS * OC_WARPS * 32 * OC_STEPS; // a lane keeps its rows' codes in registers: 65,536 rows
+
+template <typename CodeT>
+__global__ void __launch_bounds__(OC_THREADS) ordered_lists_cluster_kernel(const CodeT *codes, unsigned n, unsigned per, int m, int k, const uint32_t *active,
+                                                                           uint32_t *__restrict__ start, uint32_t *__restrict__ list)
+{
+    extern __shared__ uint32_t oc_smem[]; // [OC_WARPS][k]: counts, then the next free place of each list; [k]: counts of this CTA
+    __shared__ uint32_t s_part[OC_WARPS];
+    cg::cluster_group cl = cg::this_cluster();
+    const int s = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint32_t *s_at = oc_smem, *s_own = oc_smem + OC_WARPS * k;
+    for (int t = threadIdx.x; t < OC_WARPS * k; t += OC_THREADS) s_at[t] = 0u;
+    after_previous_kernel();
+    next_kernel_may_start();
+    if (active && active[s] == 0) return; // the whole cluster
+    const unsigned c = cl.block_rank(), w0 = (c * OC_WARPS + warp) * per, w1 = min(n, w0 + per); // a warp owns `per` rows in a row, a multiple of 32
+    __syncthreads();
+    uint32_t *mine = s_at + warp * k;
+    uint32_t code[OC_STEPS]; // all on their way at once
+#pragma unroll
+    for (unsigned i = 0; i < OC_STEPS; ++i) {
+        const unsigned r = w0 + 32 * i + lane;
+        code[i] = 32 * i < per && r < w1 ? (uint32_t)codes[(size_t)r * m + s] : 0xFFFFFFFFu;
+    }
+#pragma unroll
+    for (unsigned i = 0; i < OC_STEPS; ++i)
+        if (32 * i < per && code[i] != 0xFFFFFFFFu) atomicAdd(mine + code[i], 1u);
+    __syncthreads();
+    for (int j = threadIdx.x; j < k; j += OC_THREADS) {
+        uint32_t total = 0;
+#pragma unroll
+        for (int w = 0; w < OC_WARPS; ++w) total += s_at[w * k + j];
+        s_own[j] = total;
+    }
+    cl.sync();
+    // thread t: clusters t jt .. t jt + jt - 1
+    const int jt = (k + OC_THREADS - 1) / OC_THREADS, j0 = threadIdx.x * jt;
+    constexpr int JT = OC_MAX_K / OC_THREADS;
+    uint32_t all[JT], before[JT], total = 0;
+#pragma unroll
+    for (int i = 0; i < JT; ++i) {
+        all[i] = before[i] = 0u;
+        if (i >= jt || j0 + i >= k) continue;
+#pragma unroll
+        for (unsigned q = 0; q < OC_CTAS; ++q) {
+            const uint32_t v = *cl.map_shared_rank(s_own + j0 + i, q);
+            all[i] += v;
+            before[i] += q < c ? v : 0u;
+        }
+        total += all[i];
+    }
+    uint32_t incl = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    if (lane == 31) s_part[warp] = incl;
+    cl.barrier_arrive(); // (everybody has read the others' counts once this completes: before leaving)
+    __syncthreads();
+    uint32_t at = incl - total;
+    for (int w = 0; w < warp; ++w) at += s_part[w];
+#pragma unroll
+    for (int i = 0; i < JT; ++i) {
+        const int j = j0 + i;
+        if (i >= jt || j >= k) continue;
+        if (c == 0) start[(size_t)s * (k + 1) + j] = at;
+        uint32_t place = at + before[i];
+#pragma unroll
+        for (int w = 0; w < OC_WARPS; ++w) {
+            const uint32_t cnt = s_at[w * k + j];
+            s_at[w * k + j] = place;
+            place += cnt;
+        }
+        at += all[i];
+    }
+    if (c == 0 && threadIdx.x == 0) start[(size_t)s * (k + 1) + k] = n;
+    __syncthreads();
+    uint32_t *out = list + (size_t)s * n;
+#pragma unroll
+    for (unsigned i = 0; i < OC_STEPS; ++i) {
+        if (32 * i >= per) break;
+        const bool in = code[i] != 0xFFFFFFFFu;
+        const unsigned same = __match_any_sync(0xffffffffu, code[i]);
+        const int rank = __popc(same & ((1u << lane) - 1u));
+        uint32_t place = 0;
+        if (in) place = mine[code[i]] + rank;
+        __syncwarp();
+        if (in) {
+            out[place] = w0 + 32 * i + lane;
+            if (rank == 0) mine[code[i]] += __popc(same);
+        }
+        __syncwarp();
+    }
+    cl.barrier_wait();
 }
 
 // A warp takes 32 / W clusters side by side, W lanes each (W: the power of two that covers the width, at most 32; wider rows
@@ -251,7 +355,17 @@ static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const Cod
     const size_t hist_words = (size_t)m * chunks * k, start_words = (size_t)m * (k + 1), list_words = (size_t)m * n;
     uint32_t *work = static_cast<uint32_t *>(dev.alloc((hist_words + start_words + list_words) * sizeof(uint32_t)));
     uint32_t *hist = work, *start = hist + hist_words, *list = start + start_words;
-    {
+    // One launch instead of two, us a fit of 10 iterations: 60,000 x 128, m 16, k 256 1050 -> 950; 10,000 626 -> 608; 30,000, m 32, k 64 887 -> 864;
+    // residual 33,506 x 128, k 62, 3 stages 2260 -> 2180, 5,000 x 27, k 60 1473 -> 1402 (2,500 x 128, k 256 495 -> 505).
+    if (k <= OC_MAX_K && n <= OC_MAX_ROWS) {
+        KernelScope ks(dev, "ordered_lists");
+        auto kernel = ordered_lists_cluster_kernel<CodeT>;
+        const size_t smem = sizeof(uint32_t) * (OC_WARPS + 1) * k;
+        if (smem > 40 * 1024) VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        const unsigned per = ((n + OC_CTAS * OC_WARPS - 1) / (OC_CTAS * OC_WARPS) + 31) / 32 * 32;
+        launch_following_clusters(kernel, dim3(OC_CTAS, m), OC_THREADS, smem, OC_CTAS, dev.stream(), codes, n, per, m, k, active, start, list);
+        dev.count_launch();
+    } else {
         KernelScope ks(dev, "ordered_lists");
         const size_t smem = sizeof(uint32_t) * k;
         launch_following(ordered_hist_kernel<CodeT>, dim3(chunks, m), OL_THREADS, smem, dev.stream(), codes, n, chunk, m, k, active, hist);
