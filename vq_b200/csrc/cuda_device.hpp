@@ -136,6 +136,9 @@ class CudaDevice : public Device {
     cudaEvent_t order_event_ = nullptr;
     bool lasting(cudaStream_t s) const;
     static constexpr size_t STAGE_BYTES = 1u << 20; // pinned staging for small downloads
+    static constexpr size_t UPLOAD_BYTES = 1u << 20; // behind it, a ring for small uploads
+    size_t upload_at_ = 0;
+    cudaEvent_t upload_event_ = nullptr; // the last of them has been read
     unsigned char *stage_ = nullptr, *stage_dev_ = nullptr; // stage_dev_: the same bytes as kernels on this GPU address them
     cudaEvent_t stage_event_ = nullptr;
     std::atomic<uint64_t> launches_{0}, device_allocs_{0};
