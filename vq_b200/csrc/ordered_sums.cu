@@ -252,92 +252,25 @@ __global__ void __launch_bounds__(32 * OS_WARPS) ordered_sums_kernel(const float
 }
 
 // Few clusters of wide rows, whose lists are long (in the later stages of a residual fit most rows are closest to one centroid): a CTA per
-// (cluster, 32 dimensions).  One warp that does everything takes 25 to 33 cycles a row, its instructions one after the other; here seven warps
-// bring the rows (stages of 128, three ahead) and the eighth adds them up, 7 to 8 cycles a row.
-constexpr int OL_STAGE = 128, OL_SLOTS = 4, OL_PRODUCERS = 7, OL_SHARE = 20; // rows of a stage; stages in the ring; rows of a producer (7 x 20 >= 128)
-constexpr size_t OL_LONG_SMEM = (size_t)OL_SLOTS * OL_STAGE * 32 * sizeof(float);
-
+// (cluster, 32 dimensions) (stream_rows).
 template <bool VEC>
-__global__ void __launch_bounds__(32 * (OL_PRODUCERS + 1)) ordered_sums_long_kernel(const float *__restrict__ x, unsigned n, unsigned long long ld, int m, int k, int sd,
-                                                                                    const uint32_t *active, const uint32_t *start,
-                                                                                    const uint32_t *list, float *sums, uint32_t *counts, int counts_f32)
+__global__ void __launch_bounds__(STREAM_THREADS) ordered_sums_long_kernel(const float *__restrict__ x, unsigned n, unsigned long long ld, int m, int k, int sd,
+                                                                          const uint32_t *active, const uint32_t *start,
+                                                                          const uint32_t *list, float *sums, uint32_t *counts, int counts_f32)
 {
-    extern __shared__ __align__(16) float ol_ring[]; // [OL_SLOTS][OL_STAGE][32]
-    const int s = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    extern __shared__ __align__(16) float ol_ring[];
+    const int s = blockIdx.y, lane = threadIdx.x & 31;
     after_previous_kernel();
     next_kernel_may_start();
     if (active && active[s] == 0) return;
     const int pieces = (sd + 31) / 32, j = blockIdx.x / pieces, d0 = blockIdx.x % pieces * 32, cols = min(32, sd - d0);
-    const uint32_t b = start[(size_t)s * (k + 1) + j], len = start[(size_t)s * (k + 1) + j + 1] - b, stages = (len + OL_STAGE - 1) / OL_STAGE;
-    const uint32_t *rows = list + (size_t)s * n + b;
-    const int first = warp * OL_SHARE, share = min(OL_SHARE, OL_STAGE - first); // producer warp's rows of a stage
-    x += (size_t)s * sd + d0;
-    auto number = [&](uint32_t t) -> uint32_t { // of the producer's row `lane` in stage t
-        const uint32_t at = t * OL_STAGE + first + lane;
-        return lane < share && at < len ? rows[at] : 0u;
-    };
-    auto issue = [&](uint32_t t, uint32_t num) { // always closes a group
-        if (t < stages) {
-            const int here = min(share, (int)(len - min(len, t * OL_STAGE + first))); // rows of this share that the list has
-            float *slot = ol_ring + ((size_t)(t % OL_SLOTS) * OL_STAGE + first) * 32;
-            if (VEC) {
-#pragma unroll
-                for (int i = 0; i < OL_SHARE; i += 4) { // four rows at a time, eight lanes each
-                    const int r = i + (lane >> 3), c = (lane & 7) * 4;
-                    const uint32_t row = __shfl_sync(0xffffffffu, num, r);
-                    if (r < here && c < cols)
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(slot + r * 32 + c)), "l"(x + (size_t)row * ld + c) : "memory");
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < OL_SHARE; ++r) {
-                    const uint32_t row = __shfl_sync(0xffffffffu, num, r);
-                    if (r < here && lane < cols)
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(slot + r * 32 + lane)), "l"(x + (size_t)row * ld + lane) : "memory");
-                }
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    const bool producer = warp < OL_PRODUCERS;
-    uint32_t num = 0;
-    if (producer) {
-#pragma unroll
-        for (uint32_t t = 0; t < OL_SLOTS - 1; ++t) issue(t, number(t));
-        num = number(OL_SLOTS - 1);
-    }
+    const uint32_t b = start[(size_t)s * (k + 1) + j], len = start[(size_t)s * (k + 1) + j + 1] - b;
     float acc = 0.0f;
-    for (uint32_t t = 0; t < stages; ++t) {
-        if (producer) asm volatile("cp.async.wait_group %0;" ::"n"(OL_SLOTS - 2) : "memory"); // stage t of this warp is there
-        __syncthreads();                                                                      // and of all; stage t - 1 is used up
-        if (producer) {
-            issue(t + OL_SLOTS - 1, num);
-            num = number(t + OL_SLOTS);
-        } else {
-            const float *v = ol_ring + (size_t)(t % OL_SLOTS) * OL_STAGE * 32 + lane;
-            const int here = (int)min((uint32_t)OL_STAGE, len - t * OL_STAGE);
-            if (here == OL_STAGE) {
-                float cur[8], next[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) cur[i] = v[i * 32];
-#pragma unroll 4
-                for (int r = 8; r <= OL_STAGE; r += 8) {
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) next[i] = v[(r < OL_STAGE ? r + i : i) * 32];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) acc = __fadd_rn(acc, cur[i]), cur[i] = next[i];
-                }
-            } else {
-#pragma unroll 4
-                for (int r = 0; r < here; ++r) acc = __fadd_rn(acc, v[r * 32]);
-            }
-        }
-    }
-    if (!producer && lane < cols) {
+    stream_rows<VEC>(ol_ring, x + (size_t)s * sd + d0, ld, list + (size_t)s * n + b, len, cols, [&](float v) { acc = __fadd_rn(acc, v); }, [](uint32_t) {});
+    if (threadIdx.x >= 32 * STREAM_PRODUCERS && lane < cols) {
         sums[((size_t)s * k + j) * sd + d0 + lane] = acc;
         if (d0 + lane == 0) counts[(size_t)s * k + j] = counts_f32 ? __float_as_uint((float)len) : len;
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 } // namespace
@@ -383,8 +316,8 @@ static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const Cod
     if (sd > 16 && (long_units * m <= (size_t)dev.sm_count() * 4 || n / k >= 150)) {
         KernelScope ks(dev, "ordered_sums");
         auto kernel = vec ? ordered_sums_long_kernel<true> : ordered_sums_long_kernel<false>;
-        VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OL_LONG_SMEM));
-        launch_following(kernel, dim3((unsigned)long_units, m), 32 * (OL_PRODUCERS + 1), OL_LONG_SMEM, dev.stream(), x, n, sh.ld, m, k, sd, active, start, list, sums, counts,
+        VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STREAM_SMEM));
+        launch_following(kernel, dim3((unsigned)long_units, m), STREAM_THREADS, STREAM_SMEM, dev.stream(), x, n, sh.ld, m, k, sd, active, start, list, sums, counts,
                          counts_f32);
         dev.count_launch();
     } else {

@@ -80,23 +80,21 @@ __global__ void init_tree_kernel(size_t n, int splits, uint32_t *perm, NodeInfo 
     }
 }
 
-// ---- large nodes: one warp per (1024-row chunk, 32 dimensions), then one thread per (node, dimension) adds the node's chunk
+// ---- large nodes: one CTA per (1024-row chunk, 32 dimensions), then one thread per (node, dimension) adds the node's chunk
 // sums in order and divides
 template <bool VEC>
-__global__ void __launch_bounds__(32 * WR_WARPS) chunk_sums_kernel(const float *__restrict__ x, size_t dim, const uint32_t *perm,
-                                                                   const LevelInfo *level, const ChunkInfo *chunks, float *partial)
+__global__ void __launch_bounds__(STREAM_THREADS) chunk_sums_kernel(const float *__restrict__ x, size_t dim, const uint32_t *perm,
+                                                                    const LevelInfo *level, const ChunkInfo *chunks, float *partial)
 {
-    __shared__ __align__(16) WalkRing ring[WR_WARPS];
+    extern __shared__ __align__(16) float ring[];
     after_previous_kernel();
     next_kernel_may_start();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t groups = (dim + 31) / 32, unit = (size_t)blockIdx.x * WR_WARPS + warp, chunk = unit / groups, d0 = unit % groups * 32, d = d0 + lane;
+    const size_t groups = (dim + 31) / 32, chunk = blockIdx.x / groups, d0 = blockIdx.x % groups * 32, d = d0 + (threadIdx.x & 31);
     if (chunk >= (size_t)level->chunks) return;
     const ChunkInfo ch = chunks[chunk];
-    const int cols = (int)min(dim - d0, (size_t)32);
     float acc = 0.0f;
-    walk_rows<32, VEC>(ring[warp], x + d0, dim, perm + ch.start, ch.rows, cols, [&](float v) { acc = __fadd_rn(acc, v); });
-    if (d < dim) partial[chunk * dim + d] = acc;
+    stream_rows<VEC>(ring, x + d0, dim, perm + ch.start, ch.rows, (int)min(dim - d0, (size_t)32), [&](float v) { acc = __fadd_rn(acc, v); }, [](uint32_t) {});
+    if (threadIdx.x >= 32 * STREAM_PRODUCERS && d < dim) partial[chunk * dim + d] = acc;
 }
 
 __global__ void node_mean_kernel(const NodeInfo *nodes, const LevelInfo *level, size_t dim, const float *partial, float *centroids)
@@ -147,6 +145,38 @@ __global__ void __launch_bounds__(32 * WR_WARPS) node_stats_kernel(const float *
         const float e = __fsub_rn(v, c);
         var = __fadd_rn(var, __fmul_rn(e, e));
     });
+    if (live) spread[in_level * dim + d] = var;
+}
+
+// The same by a CTA per (node, 32 dimensions).
+template <bool VEC>
+__global__ void __launch_bounds__(STREAM_THREADS) node_stats_stream_kernel(const float *__restrict__ x, size_t dim, const uint32_t *perm,
+                                                                           const NodeInfo *nodes, const LevelInfo *level, float *centroids, float *spread)
+{
+    extern __shared__ __align__(16) float ring[];
+    after_previous_kernel();
+    next_kernel_may_start();
+    const size_t groups = (dim + 31) / 32, in_level = blockIdx.x / groups, d0 = blockIdx.x % groups * 32, d = d0 + (threadIdx.x & 31);
+    if (in_level >= (size_t)level->count) return;
+    const int node = level->first + (int)in_level;
+    const NodeInfo nd = nodes[node];
+    const bool live = threadIdx.x >= 32 * STREAM_PRODUCERS && d < dim;
+    const int cols = (int)min(dim - d0, (size_t)32);
+    const uint32_t *rows = perm + nd.start;
+    static_assert(MEAN_CHUNK % STREAM_STAGE == 0, "a chunk's sum ends with a stage");
+    float total = 0.0f, acc = 0.0f;
+    const uint32_t last = (nd.count + STREAM_STAGE - 1) / STREAM_STAGE - 1;
+    stream_rows<VEC>(ring, x + d0, dim, rows, nd.count, cols, [&](float v) { acc = __fadd_rn(acc, v); }, [&](uint32_t t) {
+        if (t == last || (t + 1) % (MEAN_CHUNK / STREAM_STAGE) == 0) total = __fadd_rn(total, acc), acc = 0.0f;
+    });
+    const float c = __fdiv_rn(total, __uint2float_rn(nd.count));
+    if (live) centroids[(size_t)node * dim + d] = c;
+    if (!nd.split) return;
+    float var = 0.0f;
+    stream_rows<VEC>(ring, x + d0, dim, rows, nd.count, cols, [&](float v) {
+        const float e = __fsub_rn(v, c);
+        var = __fadd_rn(var, __fmul_rn(e, e));
+    }, [](uint32_t) {});
     if (live) spread[in_level * dim + d] = var;
 }
 
@@ -370,9 +400,12 @@ __global__ void __launch_bounds__(NS_THREADS) node_spread_stream_kernel(const fl
 // radix selection (11 + 11 + 10 bits; the CTAs add up their digit counts through distributed shared memory), for an even
 // count its predecessor, the median, and the stable partition.
 constexpr int SP_THREADS = 512, SP_BINS = 2048, SP_CLUSTER = 8;
+constexpr unsigned SP_KEYS = 16384; // keys that a CTA keeps in shared memory
+constexpr int SP_U = 8;             // loads of a thread in flight
+constexpr int SP_RUN = 4;           // rows of a thread at a time in the partition
 
 __global__ void __launch_bounds__(SP_THREADS) split_kernel(const float *__restrict__ x, size_t dim, const uint32_t *__restrict__ perm, uint32_t *perm_out,
-                                                           NodeInfo *nodes, const LevelInfo *level, const float *spread, uint32_t *keys, int *error)
+                                                           NodeInfo *nodes, const LevelInfo *level, const float *spread, uint32_t *keys, unsigned room, int *error)
 {
     after_previous_kernel();
     next_kernel_may_start();
@@ -384,6 +417,7 @@ __global__ void __launch_bounds__(SP_THREADS) split_kernel(const float *__restri
     const int node = level->first + (int)in_level;
     const NodeInfo nd = nodes[node];
     if (!nd.split) return;
+    extern __shared__ uint32_t s_keys[];
     __shared__ __align__(16) uint32_t s_hist[SP_BINS];
     __shared__ uint32_t s_scan[SP_THREADS / 32], s_bin, s_below, s_left, s_max;
     __shared__ unsigned long long s_best;
@@ -405,12 +439,44 @@ __global__ void __launch_bounds__(SP_THREADS) split_kernel(const float *__restri
 
     const unsigned per = (nd.count + cs - 1) / cs, r0 = min(nd.count, rank * per), r1 = min(nd.count, r0 + per);
     const uint32_t *rows = perm + nd.start;
-    uint32_t *own = keys + nd.start;
-    for (unsigned i = r0 + tid; i < r1; i += SP_THREADS) {
-        const float v = __ldg(x + (size_t)rows[i] * dim + split_dim);
-        if (!(v == v)) atomicExch(error, 105);
-        own[i] = f32_key(v);
+    // f(key of row i) for this CTA's rows, several of a thread's keys on their way at once where they are in memory
+    uint32_t *const far_keys = keys + nd.start;
+    const bool fits = r1 - r0 <= room;
+    auto for_keys = [&](auto f) {
+        if (fits) {
+#pragma unroll 4
+            for (unsigned i = r0 + tid; i < r1; i += SP_THREADS) f(s_keys[i - r0]);
+        } else {
+            for (unsigned i0 = r0 + tid; i0 < r1; i0 += SP_U * SP_THREADS) {
+                uint32_t key[SP_U];
+#pragma unroll
+                for (int u = 0; u < SP_U; ++u) key[u] = i0 + u * SP_THREADS < r1 ? far_keys[i0 + u * SP_THREADS] : 0u;
+#pragma unroll
+                for (int u = 0; u < SP_U; ++u)
+                    if (i0 + u * SP_THREADS < r1) f(key[u]);
+            }
+        }
+    };
+    auto meet = [&] { // all CTAs of the node
+        if (cs > 1) cl.sync();
+        else __syncthreads();
+    };
+    bool nan = false;
+    for (unsigned i0 = r0 + tid; i0 < r1; i0 += SP_U * SP_THREADS) {
+        uint32_t row[SP_U];
+        float v[SP_U];
+#pragma unroll
+        for (int u = 0; u < SP_U; ++u) row[u] = i0 + u * SP_THREADS < r1 ? rows[i0 + u * SP_THREADS] : 0u;
+#pragma unroll
+        for (int u = 0; u < SP_U; ++u) v[u] = i0 + u * SP_THREADS < r1 ? __ldg(x + (size_t)row[u] * dim + split_dim) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < SP_U; ++u) {
+            const unsigned i = i0 + u * SP_THREADS;
+            nan = nan || !(v[u] == v[u]);
+            if (i < r1) (fits ? s_keys[i - r0] : far_keys[i]) = f32_key(v[u]);
+        }
     }
+    if (nan) atomicExch(error, 105);
     __syncthreads(); // from here on a CTA reads the keys of its own rows only
 
     // inclusive scan of one value per thread; the CTA's total in s_scan[last]
@@ -444,11 +510,10 @@ __global__ void __launch_bounds__(SP_THREADS) split_kernel(const float *__restri
         const uint32_t digit = pass == 2 ? 1023u : 2047u;
         for (int b = tid; b < SP_BINS; b += SP_THREADS) s_hist[b] = 0u;
         __syncthreads();
-        for (unsigned i = r0 + tid; i < r1; i += SP_THREADS) {
-            const uint32_t key = own[i];
+        for_keys([&](uint32_t key) {
             if ((key & mask) == prefix) atomicAdd(s_hist + ((key >> shift) & digit), 1u);
-        }
-        cl.sync();
+        });
+        meet();
         uint32_t c[SP_BINS / SP_THREADS], sum = 0u;
 #pragma unroll
         for (int b = 0; b < SP_BINS / SP_THREADS; ++b) c[b] = 0u;
@@ -464,7 +529,7 @@ __global__ void __launch_bounds__(SP_THREADS) split_kernel(const float *__restri
             if (r >= below && r - below < c[b]) s_bin = 4 * tid + b, s_below = below;
             below += c[b];
         }
-        cl.sync(); // the counts have been read everywhere before they are cleared
+        meet(); // the counts have been read everywhere before they are cleared
         prefix |= s_bin << shift, mask |= digit << shift;
         r -= s_below;
     }
@@ -474,13 +539,12 @@ __global__ void __launch_bounds__(SP_THREADS) split_kernel(const float *__restri
         float lo = hi; // r > 0: the predecessor equals it
         if (r == 0) {  // (the same in every CTA)
             uint32_t low = 0u;
-            for (unsigned i = r0 + tid; i < r1; i += SP_THREADS) {
-                const uint32_t key = own[i];
+            for_keys([&](uint32_t key) {
                 if (key < prefix) low = max(low, key);
-            }
+            });
             low = __reduce_max_sync(0xffffffffu, low);
             if (lane == 0) atomicMax(&s_max, low);
-            cl.sync();
+            meet();
             low = 0u;
             for (unsigned q = 0; q < cs; ++q) low = max(low, *cl.map_shared_rank(&s_max, q));
             lo = key_f32(low);
@@ -490,22 +554,35 @@ __global__ void __launch_bounds__(SP_THREADS) split_kernel(const float *__restri
 
     // stable partition: the rows at or below the median first, both sides in their old order
     uint32_t mine = 0u;
-    for (unsigned i = r0 + tid; i < r1; i += SP_THREADS) mine += key_f32(own[i]) <= median ? 1u : 0u;
+    for_keys([&](uint32_t key) { mine += key_f32(key) <= median ? 1u : 0u; });
     mine = __reduce_add_sync(0xffffffffu, mine);
     if (lane == 0) atomicAdd(&s_left, mine);
-    cl.sync();
+    meet();
     uint32_t before = 0u, nleft = 0u;
     for (unsigned q = 0; q < cs; ++q) {
         const uint32_t l = *cl.map_shared_rank(&s_left, q);
         before += q < rank ? l : 0u;
         nleft += l;
     }
-    cl.sync(); // nobody leaves while its shared memory is still being read
-    for (unsigned t0 = r0; t0 < r1; t0 += SP_THREADS) {
-        const unsigned i = t0 + tid;
-        const bool in = i < r1, left = in && key_f32(own[i]) <= median;
-        const uint32_t incl = block_scan(left ? 1u : 0u), lefts = before + incl - (left ? 1u : 0u);
-        if (in) perm_out[nd.start + (left ? lefts : nleft + (i - lefts))] = rows[i];
+    meet(); // nobody leaves while its shared memory is still being read
+    // a thread takes SP_RUN rows in a row, so that the scan is needed once for SP_RUN * SP_THREADS of them
+    for (unsigned t0 = r0; t0 < r1; t0 += SP_RUN * SP_THREADS) {
+        const unsigned i0 = t0 + SP_RUN * tid;
+        uint32_t row[SP_RUN], lefts = 0u;
+        bool left[SP_RUN];
+#pragma unroll
+        for (int u = 0; u < SP_RUN; ++u) {
+            const bool in = i0 + u < r1;
+            row[u] = in ? rows[i0 + u] : 0u;
+            left[u] = in && key_f32(fits ? s_keys[i0 + u - r0] : far_keys[i0 + u]) <= median;
+            lefts += left[u] ? 1u : 0u;
+        }
+        uint32_t at = before + block_scan(lefts) - lefts;
+#pragma unroll
+        for (int u = 0; u < SP_RUN; ++u) {
+            if (i0 + u < r1) perm_out[nd.start + (left[u] ? at : nleft + (i0 + u - at))] = row[u];
+            at += left[u] ? 1u : 0u;
+        }
         before += s_scan[SP_THREADS / 32 - 1];
         // (block_scan's first barrier keeps s_scan until everybody has read the total)
     }
@@ -853,10 +930,9 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
         LevelInfo known = {0, 1, 0, 0}; // the last level that the host has asked about
         auto ask = [&](size_t l) {
             int herr = 0;
-            dev.download(&herr, error, sizeof(int));
+            dev.download(&herr, error, sizeof(int), &known, levels + (l & 1), sizeof known);
             if (herr == NS_ERR_WAIT) throw Error(100, "tsvq: a wait inside the node statistics kernel ran out");
             if (herr) throw Error(herr, "values are not comparable (NaN in the training data)");
-            dev.download(&known, levels + (l & 1), sizeof known);
         };
         size_t most = 1; // nodes that the level can have
         for (size_t l = 0;; ++l) {
@@ -873,12 +949,20 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
             }
             if (small) {
                 KernelScope ks(dev, "tsvq_node_stats");
-                launch_following(vec ? node_stats_kernel<true> : node_stats_kernel<false>, grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st, x, dim, perm, nodes, level, cent, spread);
+                // us a build, a warp / a CTA per node and 32 dimensions from 150 rows on: 100,000 x 128, depth 10 1157 / 1110; 2,475 x 122, depth 9
+                // 414 / 324; 20,000 x 64, depth 8 464 / 417.  (From 600 rows on 1097, 339, 422.)
+                if (n / most >= 150) {
+                    const auto kernel = vec ? node_stats_stream_kernel<true> : node_stats_stream_kernel<false>;
+                    VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STREAM_SMEM));
+                    launch_following(kernel, grid_for(most * groups, 1, 1u << 30), STREAM_THREADS, STREAM_SMEM, st, x, dim, perm, nodes, level, cent, spread);
+                } else launch_following(vec ? node_stats_kernel<true> : node_stats_kernel<false>, grid_for(most * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st, x, dim, perm, nodes, level, cent, spread);
                 dev.count_launch();
             } else {
                 {
                     KernelScope ks(dev, "tsvq_node_means");
-                    launch_following(vec ? chunk_sums_kernel<true> : chunk_sums_kernel<false>, grid_for((n_chunks + most) * groups, WR_WARPS, 1u << 30), 32 * WR_WARPS, 0, st, x, dim, perm, level, chunks, partial);
+                    const auto kernel = vec ? chunk_sums_kernel<true> : chunk_sums_kernel<false>;
+                    VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STREAM_SMEM));
+                    launch_following(kernel, grid_for((n_chunks + most) * groups, 1, 1u << 30), STREAM_THREADS, STREAM_SMEM, st, x, dim, perm, level, chunks, partial);
                     launch_following(node_mean_kernel, grid_for(most * dim, 128, 1u << 30), 128, 0, st, nodes, level, dim, partial, cent);
                     dev.count_launch();
                     dev.count_launch();
@@ -898,9 +982,16 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
             {
                 KernelScope ks(dev, "tsvq_split");
                 cudaLaunchConfig_t cfg = {};
-                const unsigned cluster = small ? 1u : (unsigned)SP_CLUSTER;
+                // CTAs of a node by its rows (on average), us a build: 100,000 x 128, depth 10 1319 with eight above 2048 rows and keys in memory, 1241
+                // with keys in shared memory, 1176 like this; 300,000 x 32 2526, 2439, 2283; 2,475 x 122, depth 9 494, 434, 417.  (One up to 16,384,
+                // then eight: 1192, 2272, 418.)
+                const size_t rows = n / most;
+                const unsigned cluster = rows <= 4096 ? 1u : rows <= 8192 ? 2u : rows <= 16384 ? 4u : (unsigned)SP_CLUSTER;
+                const size_t split_smem = sizeof(uint32_t) * std::min<size_t>(SP_KEYS, 2 * (rows / cluster + 1)); // (nodes are halves, but for ties)
+                VQB_CUDA_CHECK(cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(uint32_t) * SP_KEYS)));
                 cfg.gridDim = dim3((unsigned)most * cluster);
                 cfg.blockDim = dim3(SP_THREADS);
+                cfg.dynamicSmemBytes = split_smem;
                 cfg.stream = st;
                 cudaLaunchAttribute attr[2] = {};
                 attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -910,7 +1001,7 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
                 attr[1].val.programmaticStreamSerializationAllowed = 1;
                 cfg.attrs = attr;
                 cfg.numAttrs = 2;
-                VQB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, split_kernel, x, dim, (const uint32_t *)perm, perm2, nodes, level, (const float *)spread, keys, error));
+                VQB_CUDA_CHECK(cudaLaunchKernelEx(&cfg, split_kernel, x, dim, (const uint32_t *)perm, perm2, nodes, level, (const float *)spread, keys, (unsigned)(split_smem / sizeof(uint32_t)), error));
                 dev.count_launch();
             }
             room_for_chunks(std::min(2 * most, n));
@@ -923,8 +1014,7 @@ void tsvq_fit(CudaDevice &dev, const float *x, size_t n, size_t dim, size_t max_
         out.nodes = (size_t)(known.first + known.count);
         out.h_left.resize(out.nodes);
         out.h_right.resize(out.nodes);
-        dev.download(out.h_left.data(), left, sizeof(int32_t) * out.nodes);
-        dev.download(out.h_right.data(), right, sizeof(int32_t) * out.nodes);
+        dev.download(out.h_left.data(), left, sizeof(int32_t) * out.nodes, out.h_right.data(), right, sizeof(int32_t) * out.nodes);
     } catch (...) {
         cudaStreamSynchronize(st);
         dev.release(cent), dev.release(left), dev.release(right);
