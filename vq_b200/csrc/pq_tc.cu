@@ -35,6 +35,14 @@
 //   the reference's own arithmetic prefers w over a only if D_w <= D_a (1 + 4u) with (sd + 2)u each: 24u * 65300 = 0.1
 //   => T_w <= T_best + 1.5 + 2 * 0.17 + 0.1, i.e. a difference of at most 1.  M = 3 leaves room for twice what was measured.
 //
+// FEW (8-wide, many rows).  Every step reads and writes the whole accumulator, and on large inputs the chip runs at its power limit: the third
+// step cost a tenth of the time (1M x 128, m 16, k 256, back to back at 990 W: encode 475 -> 449 us, fit of 10 iterations 5,340 -> 4,985).  So
+// the constants share a step with the last products, xl.(-ch), and the half norm.  Then eleven addends beside 2^23 have fractions: the
+// accumulator and the eight products, either sign, -2.25 .. 2.25, the half norm's two, never negative, -0.5 .. 0, and the result's unit
+// downwards: error in (-3.75, 2.25) instead of (-1.25, 0.25), measured (tests/test_gpu_pq_two_steps.py) -2.97 .. 1.98.
+//   => T_w <= T_best + 6.0 + 2 * 0.17 + 0.1, i.e. a difference of at most 6: M = 7.  More rows are queued for it: uniform ones 2 % of the time,
+//   64 clusters of standard deviation 0.05 and distance 1 391 -> 497 us for 500,000 rows (of 0.001 1,678 -> 1,460, of 0.3 217 -> 225).
+//
 // Far centroids.  One centroid far from the others would stretch the range for all.  Those farther from mu than four times the
 // mean distance (mu: the mean of the rest, found in up to six rounds) are left out: rho covers the others.  The producers leave a
 // lower bound of what a far one can score against the row, lim^2/2 - lim |x|, in shared memory; a row that has it within reach is
@@ -56,8 +64,8 @@
 // 128-row tile of one sub-space; it uses one of the two 128 x 256 f32 accumulators, in two halves of 128 columns.
 //   warps 0-3    MMA issuers, one per accumulator half; warp 0 first loads the group's operand-B tiles (TMA, no multicast), warp 1
 //                owns tensor memory
-//   warps 4-11   take the row tile that TMA has brought into shared memory (two buffers), scale and split the slices (two sub-spaces a
-//                warp) and write operand-A tiles, one stage per sub-space
+//   warps 4-11   take their 32 rows of two sub-spaces, which TMA brings into the warp's own two buffers, scale and split the slices and
+//                write operand-A tiles, one stage per sub-space
 //   warps 12-27  epilogue: a team of four warps per sub-space (one row per lane, one TMEM lane quadrant per warp)
 // Every wait is bounded; on expiry the CTA records a code, stops issuing, frees tensor memory and the host raises an error.
 //
@@ -74,8 +82,9 @@
 //     instruction, they keep the L1 cache busy for 256 cycles a unit (0.40)
 //   * an encode leaves one byte per pair; pq_expand_kernel turns them into rows and 32-bit codes with whole-line stores, 0.06 ms
 //     (16-byte pieces stored from here: 0.49 in all)
-// The constant in a step of its own (K = 48) rather than beside the last products (K = 32): ten cut addends instead of one would
-// need M = 8 and triple the share of queued rows.
+//   * each of the eight fetches its own rows: with one copy of the 128 rows for all, issued by the first of them once the others had used
+//     the buffer up, that warp's 950 cycles for it were the kernel's longest chain (encode 0.353 -> 0.345, training pass 0.366 -> 0.360, short
+//     runs; at the power limit 456 -> 449 us for the encode)
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -91,6 +100,7 @@ namespace vqb {
 namespace {
 
 constexpr int BM = (int)PQ_TC_TILE, BN = 256, MAXM = 64, NTHREADS = 32 * (4 + 8 + 16);
+constexpr int NRAW = 2; // row buffers of a producer warp
 constexpr int QCAP = 64; // queue entries per epilogue warp: fewer than 32 wait, at most 32 are added at a time
 constexpr float COS_MIN = 1e-17f, COS_MAX = 1e18f;  // cosine: norms that the scores can be trusted for
 constexpr float RHO_MIN = 1e-14f, RHO_MAX = 1e15f;  // Euclidean: radii for which neither 2^+-96 scalings nor distances leave f32
@@ -121,16 +131,18 @@ template <> struct Slots<4> {
 template <> struct Slots<8> {
     static constexpr int STEPS = 3, NORM = 24, CONST = 32, M = 3;
 };
+// FEW: where the constants stand then, and the window
+constexpr int FEW_CONST = 26, FEW_M = 7;
 template <int SD> constexpr uint32_t A1_BYTES = BM * 64;                            // a stage
-template <int SD> constexpr uint32_t A2_BYTES = Slots<SD>::STEPS == 3 ? BM * 32 : 0;
-template <int SD> constexpr uint32_t A_BYTES = A1_BYTES<SD> + A2_BYTES<SD>;
+template <int SD, bool FEW> constexpr uint32_t A2_BYTES = Slots<SD>::STEPS == 3 && !FEW ? BM * 32 : 0;
+template <int SD, bool FEW> constexpr uint32_t A_BYTES = A1_BYTES<SD> + A2_BYTES<SD, FEW>;
 template <int SD> constexpr uint32_t B1_BYTES = BN * 64;                            // a sub-space
-template <int SD> constexpr uint32_t B2_BYTES = Slots<SD>::STEPS == 3 ? BN * 32 : 0;
-template <int SD> constexpr uint32_t B_BYTES = B1_BYTES<SD> + B2_BYTES<SD>;
-template <int SD> constexpr uint32_t RAW_BYTES = BM * 4 * SD * 4;                   // a row tile
+template <int SD, bool FEW> constexpr uint32_t B2_BYTES = Slots<SD>::STEPS == 3 && !FEW ? BN * 32 : 0;
+template <int SD, bool FEW> constexpr uint32_t B_BYTES = B1_BYTES<SD> + B2_BYTES<SD, FEW>;
+template <int SD> constexpr uint32_t RAW_BYTES = 32 * 2 * SD * 4;                   // a producer warp's rows: 32 of them, two sub-spaces wide
 
 struct alignas(8) PqBarriers {
-    unsigned long long afull[4], aempty[4], bfull, rfull[2], rempty[2]; // a...: per sub-space; r...: per row-tile buffer
+    unsigned long long afull[4], aempty[4], bfull, rfull[8][NRAW]; // a...: per sub-space; r...: per producer warp's row buffer
     unsigned long long tfull[8], tempty[8];                             // [2 ss + half]
     uint32_t tmem_base;
     int abort_flag;
@@ -198,8 +210,8 @@ __device__ __forceinline__ float sqrt_approx(float v)
     return r;
 }
 
-template <int SD>
-constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES<SD> + 4 * (size_t)A_BYTES<SD> + 2 * (size_t)RAW_BYTES<SD> + 4 * SUB_FLOATS * sizeof(float) +
+template <int SD, bool FEW>
+constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES<SD, FEW> + 4 * (size_t)A_BYTES<SD, FEW> + 8 * NRAW * (size_t)RAW_BYTES<SD> + 4 * SUB_FLOATS * sizeof(float) +
                               16 * QCAP * sizeof(uint4) + 4 * 4 * BM * sizeof(uint16_t) + sizeof(PqBarriers) + 64;
 
 // What a row contributes besides its (shifted) values: the factor of its operand, the half-norm factor and the two row constants.
@@ -363,7 +375,7 @@ __device__ __noinline__ bool pq_queue_drain(const PqTcParams &Q, const uint4 *qu
 }
 
 // DUMP: diagnostics in place of codes, 1: the chain's result without the fixed-point constants, as scores; 2: T itself and the rows' sigma and K0
-template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP>
+template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP, bool FEW>
 __global__ void __launch_bounds__(NTHREADS, 1)
     pq_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
                  const __grid_constant__ PqTcParams Q)
@@ -371,13 +383,15 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     constexpr bool COSINE = METRIC == M_COSINE;
     constexpr int halves = WIDE ? 2 : 1; // accumulator halves that hold centroids
     using SL = Slots<SD>;
+    constexpr int STEPS = FEW ? 2 : SL::STEPS;
+    constexpr uint32_t M = FEW ? FEW_M : SL::M; // scores this close are decided exactly
     extern __shared__ unsigned char smem_raw[];
     const AssignParams &P = Q.a;
     unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char *b_smem = base;                                                    // [4] 64-byte rows, then [4] 32-byte rows
-    unsigned char *a_smem = base + 4 * (size_t)B_BYTES<SD>;                          // the same
-    unsigned char *raw_smem = a_smem + 4 * (size_t)A_BYTES<SD>;                      // [2] row tiles
-    float *sub_s = reinterpret_cast<float *>(raw_smem + 2 * (size_t)RAW_BYTES<SD>);  // [4][32]
+    unsigned char *a_smem = base + 4 * (size_t)B_BYTES<SD, FEW>;                          // the same
+    unsigned char *raw_smem = a_smem + 4 * (size_t)A_BYTES<SD, FEW>;                      // [8][NRAW] row pieces
+    float *sub_s = reinterpret_cast<float *>(raw_smem + 8 * NRAW * (size_t)RAW_BYTES<SD>);  // [4][32]
     uint4 *queues = reinterpret_cast<uint4 *>(sub_s + 4 * SUB_FLOATS);               // [16][QCAP]
     uint16_t *far_s = reinterpret_cast<uint16_t *>(queues + 16 * QCAP);              // [4][4][128] RowFrame::far of four tiles
     PqBarriers *bars = reinterpret_cast<PqBarriers *>(far_s + 4 * 4 * BM);
@@ -397,10 +411,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             mbar_init(&bars->afull[s], 4);
             mbar_init(&bars->aempty[s], halves); // one commit per accumulator half
         }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&bars->rfull[b], 1);
-            mbar_init(&bars->rempty[b], 8);
-        }
+        for (int b = 0; b < 8 * NRAW; ++b) mbar_init(&bars->rfull[0][b], 1);
         mbar_init(&bars->bfull, 1);
         for (int b = 0; b < 8; ++b) {
             mbar_init(&bars->tfull[b], 1);
@@ -409,7 +420,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (uint32_t i = threadIdx.x; i < 4 * A_BYTES<SD> / 16; i += NTHREADS) // the slots that no row uses stay zero
+    for (uint32_t i = threadIdx.x; i < 4 * A_BYTES<SD, FEW> / 16; i += NTHREADS) // the slots that no row uses stay zero
         reinterpret_cast<uint4 *>(a_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (warp == 1) {
@@ -432,10 +443,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // ------------------------------------------------ operand B: the group's sub-spaces, once
         const bool leader = elect_one();
         if (warp == 0 && leader && act) {
-            mbar_expect_tx(&bars->bfull, (uint32_t)here * B_BYTES<SD>);
+            mbar_expect_tx(&bars->bfull, (uint32_t)here * B_BYTES<SD, FEW>);
             for (int ss = 0; ss < here; ++ss) {
                 tma_load_2d(b_smem + (size_t)ss * B1_BYTES<SD>, &map_b1, 0, (g * 4 + ss) * BN, &bars->bfull);
-                if (B2_BYTES<SD>) tma_load_2d(b_smem + 4 * (size_t)B1_BYTES<SD> + (size_t)ss * B2_BYTES<SD>, &map_b2, 0, (g * 4 + ss) * BN, &bars->bfull);
+                if (B2_BYTES<SD, FEW>) tma_load_2d(b_smem + 4 * (size_t)B1_BYTES<SD> + (size_t)ss * B2_BYTES<SD, FEW>, &map_b2, 0, (g * 4 + ss) * BN, &bars->bfull);
             }
         }
         __syncwarp();
@@ -445,9 +456,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         const uint32_t mine = half < halves ? act >> (2 * acc) & 3u : 0u;
         if (mine) {
             bool ok = mbar_wait(&bars->bfull, 0, abort_flag, Q.error, 12);
-            const uint32_t a1 = (smem_u32(a_smem) + 2 * acc * A1_BYTES<SD>) >> 4, a2 = (smem_u32(a_smem) + 4 * A1_BYTES<SD> + 2 * acc * A2_BYTES<SD>) >> 4;
+            const uint32_t a1 = (smem_u32(a_smem) + 2 * acc * A1_BYTES<SD>) >> 4, a2 = (smem_u32(a_smem) + 4 * A1_BYTES<SD> + 2 * acc * A2_BYTES<SD, FEW>) >> 4;
             const uint32_t b1 = (smem_u32(b_smem) + 2 * acc * B1_BYTES<SD> + half * (B1_BYTES<SD> / 2)) >> 4;
-            const uint32_t b2 = (smem_u32(b_smem) + 4 * B1_BYTES<SD> + 2 * acc * B2_BYTES<SD> + half * (B2_BYTES<SD> / 2)) >> 4;
+            const uint32_t b2 = (smem_u32(b_smem) + 4 * B1_BYTES<SD> + 2 * acc * B2_BYTES<SD, FEW> + half * (B2_BYTES<SD, FEW> / 2)) >> 4;
             const uint32_t td = tmem_base + acc * BN + half * 128;
             uint32_t phase = 0; // parity of the tile's phases
             for (uint32_t tile = tile0; ok && tile < n_tiles; tile += tstep, phase ^= 1u) { // (after an abort the next wait fails)
@@ -467,7 +478,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         const uint32_t o = (uint32_t)h; // 16 halves = 32 bytes = 2 descriptor units per step
                         umma_f16_n128(td, smem_desc_sw64_at(a1 + o * (A1_BYTES<SD> >> 4)), smem_desc_sw64_at(b1 + o * (B1_BYTES<SD> >> 4)), 0u);
                         umma_f16_n128(td, smem_desc_sw64_at(a1 + o * (A1_BYTES<SD> >> 4) + 2), smem_desc_sw64_at(b1 + o * (B1_BYTES<SD> >> 4) + 2), 1u);
-                        if (SL::STEPS == 3) umma_f16_n128(td, smem_desc_sw32_at(a2 + o * (A2_BYTES<SD> >> 4)), smem_desc_sw32_at(b2 + o * (B2_BYTES<SD> >> 4)), 1u);
+                        if (STEPS == 3) umma_f16_n128(td, smem_desc_sw32_at(a2 + o * (A2_BYTES<SD, FEW> >> 4)), smem_desc_sw32_at(b2 + o * (B2_BYTES<SD, FEW> >> 4)), 1u);
                         umma_commit(&bars->tfull[2 * ss + half]);
                         umma_commit(&bars->aempty[ss]);
                     }
@@ -479,20 +490,22 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // ------------------------------------------------ operand A: scaled and split row slices
         const int r = (warp & 3) * 32 + lane; // row of the tile
         const int pair = (warp - 4) >> 2;     // this warp's sub-spaces: 2 pair, 2 pair + 1
-        auto load_tile = [&](uint32_t tile, uint32_t buf) { // rows and columns beyond the matrix arrive as zeros
-            mbar_expect_tx(&bars->rfull[buf], RAW_BYTES<SD>);
-            tma_load_2d(raw_smem + buf * RAW_BYTES<SD>, &map_x, g * 4 * SD, (int)(tile * BM), &bars->rfull[buf]);
+        const uint32_t mine = act >> (2 * pair) & 3u;
+        unsigned char *const raw0 = raw_smem + (size_t)(warp - 4) * NRAW * RAW_BYTES<SD>;
+        unsigned long long *const full = bars->rfull[warp - 4];
+        auto load_rows = [&](uint32_t tile, uint32_t buf) { // rows and columns beyond the matrix arrive as zeros
+            mbar_expect_tx(&full[buf], RAW_BYTES<SD>);
+            tma_load_2d(raw0 + buf * RAW_BYTES<SD>, &map_x, (g * 4 + 2 * pair) * SD, (int)(tile * BM) + (warp & 3) * 32, &full[buf]);
         };
-        if (warp == 4 && lane == 0 && act) {
-            if (tile0 < n_tiles) load_tile(tile0, 0);
-            if (tile0 + tstep < n_tiles) load_tile(tile0 + tstep, 1);
-        }
+        if (lane == 0 && mine)
+            for (uint32_t b = 0; b < NRAW; ++b)
+                if (tile0 + b * tstep < n_tiles) load_rows(tile0 + b * tstep, b);
         __syncwarp();
-        uint32_t step = 0, buf = 0, rphase = 0; // tiles so far (parity: that of the stages); row-tile buffer and its parity
+        uint32_t step = 0, buf = 0, rphase = 0; // tiles so far (parity: that of the stages); row buffer and its parity
         bool ok = true;
-        for (uint32_t tile = tile0; act && ok && tile < n_tiles; tile += tstep, ++step) {
-            if (!mbar_wait(&bars->rfull[buf], rphase, abort_flag, Q.error, 10)) break;
-            const unsigned char *raw = raw_smem + buf * RAW_BYTES<SD> + r * (16 * SD);
+        for (uint32_t tile = tile0; mine && ok && tile < n_tiles; tile += tstep, ++step) {
+            if (!mbar_wait(&full[buf], rphase, abort_flag, Q.error, 10)) break;
+            const unsigned char *raw = raw0 + buf * RAW_BYTES<SD> + lane * (8 * SD);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int ss = 2 * pair + h;
@@ -502,8 +515,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 F2 y[SD / 2];
 #pragma unroll
                 for (int c = 0; c < SD / 4; ++c) {
-                    const int chunk = ss * (SD / 4) + c;
-                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(raw + ((SD == 8 ? chunk ^ (r & 7) : chunk ^ ((r >> 1) & 3)) << 4));
+                    const int chunk = h * (SD / 4) + c;
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(raw + ((SD == 8 ? chunk ^ ((lane >> 1) & 3) : chunk ^ ((lane >> 2) & 1)) << 4));
                     y[2 * c] = v.x, y[2 * c + 1] = v.y;
                     if (!COSINE) {
                         const ulonglong2 mu = reinterpret_cast<const ulonglong2 *>(sub)[c]; // the mean with its sign changed
@@ -550,9 +563,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     *reinterpret_cast<uint4 *>(row1 + ((0 ^ s1) << 4)) = h4;
                     *reinterpret_cast<uint4 *>(row1 + ((1 ^ s1) << 4)) = h4;
                     *reinterpret_cast<uint4 *>(row1 + ((2 ^ s1) << 4)) = make_uint4(lo[0], lo[1], lo[2 % (SD / 2)], lo[3 % (SD / 2)]);
-                    *reinterpret_cast<uint4 *>(row1 + ((3 ^ s1) << 4)) = make_uint4(cc, 0u, 0u, 0u);
-                    unsigned char *row2 = a_smem + 4 * (size_t)A1_BYTES<SD> + (size_t)ss * A2_BYTES<SD> + (size_t)r * 32;
-                    *reinterpret_cast<uint4 *>(row2 + (((r >> 2) & 1) << 4)) = make_uint4(k0, 0u, 0u, 0u);
+                    *reinterpret_cast<uint4 *>(row1 + ((3 ^ s1) << 4)) = make_uint4(cc, FEW ? k0 : 0u, 0u, 0u);
+                    unsigned char *row2 = a_smem + 4 * (size_t)A1_BYTES<SD> + (size_t)ss * A2_BYTES<SD, FEW> + (size_t)r * 32;
+                    if (!FEW) *reinterpret_cast<uint4 *>(row2 + (((r >> 2) & 1) << 4)) = make_uint4(k0, 0u, 0u, 0u);
                 }
                 if (__float_as_uint(sub[SUB_FLAGS]) & SUB_FAR) far_s[(ss * 4 + (step & 3u)) * BM + r] = (uint16_t)f.far;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic writes -> visible to the MMA's reads
@@ -560,17 +573,16 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 if (lane == 0) mbar_arrive(&bars->afull[ss]);
             }
             if (!ok) break;
-            // the row tile is used up: once all eight warps say so, its buffer takes the tile after the next
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->rempty[buf]);
-            if (warp == 4 && tile + 2 * tstep < n_tiles) {
-                ok = mbar_wait(&bars->rempty[buf], rphase, abort_flag, Q.error, 17);
-                if (ok && lane == 0) load_tile(tile + 2 * tstep, buf);
-                __syncwarp();
-            }
-            buf ^= 1u;
-            if (buf == 0) rphase ^= 1u;
+            __syncwarp(); // the rows are read
+            if (lane == 0 && tile + NRAW * tstep < n_tiles) load_rows(tile + NRAW * tstep, buf);
+            if (++buf == NRAW) buf = 0, rphase ^= 1u;
         }
+        // after an abort: rows that are still on their way land before the CTA goes (bounded waits, at once where they are there)
+        if (*abort_flag)
+            for (uint32_t b = 0; mine && b < NRAW; ++b) {
+                mbar_wait(&full[buf], rphase, abort_flag, Q.error, 17);
+                if (++buf == NRAW) buf = 0, rphase ^= 1u;
+            }
     } else {
         // ------------------------------------------------ epilogue: team (warp - 12) / 4 serves that sub-space of the group
         const int q = warp & 3; // TMEM lane quadrant
@@ -660,12 +672,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             }
             const uint32_t best = min(best2 & 0xFFFFu, best2 >> 16);
             const uint32_t minus = ((0u - best) & 0xFFFFu) * 0x10001u; // adding it: the distance from the best, never negative
-            constexpr uint32_t MM = SL::M * 0x10001u;
+            constexpr uint32_t MM = M * 0x10001u;
             // Sums of weight * min(distance, M) over the blocks (weight W0 + block) and over the classes (W0 + class), both halves of a word
             // at once.  What they lack of M times all weights is the sum of weight * (M - distance) over those within M: one with distance 0
             // gives M weights, two or more at least W0 (M + 1) > M (W0 + 15).
-            constexpr uint32_t W0 = 16 * SL::M, NBLK = 8 * halves;
-            constexpr uint32_t WB = 2 * SL::M * (NBLK * W0 + NBLK * (NBLK - 1) / 2), WA = SL::M * (16 * W0 + 120);
+            constexpr uint32_t W0 = 16 * M, NBLK = 8 * halves;
+            constexpr uint32_t WB = 2 * M * (NBLK * W0 + NBLK * (NBLK - 1) / 2), WA = M * (16 * W0 + 120);
             uint32_t sb = 0, sb1 = 0, sa = 0, sa1 = 0;
 #pragma unroll
             for (uint32_t i = 0; i < NBLK; i += 2) {
@@ -678,17 +690,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 sa1 = __dp2a_lo(__viaddmin_u16x2(ga[i + 1], minus, MM), (W0 + 2 * i + 2) + ((W0 + 2 * i + 3) << 8), sa1);
             }
             const uint32_t lb = WB - sb - sb1, la = WA - sa - sa1;
-            const uint32_t idx = ((lb * 16u + la - SL::M * 17u * W0) / SL::M) & 0xFFu; // 16 block + class
+            const uint32_t idx = ((lb * 16u + la - M * 17u * W0) / M) & 0xFFu; // 16 block + class
             const bool whole = best - 1u >= T_HIGH - 1u; // 0: nothing to tell apart; high up: nothing but columns without a centroid
-            bool single = max(lb, la) <= SL::M * (W0 + 15u) && !whole;
+            bool single = max(lb, la) <= M * (W0 + 15u) && !whole;
             // a far centroid may be as close (the entry is written again four tiles on, which takes this unit's end)
-            const bool far = any_far && best + SL::M > far_s[(ss * 4 + (step & 3u)) * BM + r];
+            const bool far = any_far && best + M > far_s[(ss * 4 + (step & 3u)) * BM + r];
             single = single && !far;
             const bool later = valid && !single;
             const uint32_t vote = __ballot_sync(0xffffffffu, later);
             if (vote) {
                 // one bit per half of a word: min(distance, M) + (65536 - M) wraps to 0 for M and stays at least 1 otherwise
-                constexpr uint32_t LESS = (0x10000u - SL::M) * 0x10001u;
+                constexpr uint32_t LESS = (0x10000u - M) * 0x10001u;
                 uint32_t blocks = 0, classes = 0;
 #pragma unroll
                 for (int c = 0; c < 2 * halves; ++c) { // four words at a time: eight bits, weighted by the bytes of dp2a
@@ -875,6 +887,7 @@ __device__ __forceinline__ void write_operand(const float (&v)[SD], int s, int k
         // zeros: the rows' operands are zero as well, every column ties
     } else if (!mine || far) {
         row[SL::CONST] = f32_to_f16_bits(4096.0f + 28.0f); // 2048 * 28 = 57344
+        if (SD == 8) row[FEW_CONST] = row[SL::CONST];
     } else {
 #pragma unroll
         for (int i = 0; i < SD; ++i) {
@@ -891,6 +904,7 @@ __device__ __forceinline__ void write_operand(const float (&v)[SD], int s, int k
         }
         row[SL::CONST] = f32_to_f16_bits(4096.0f);
         row[SL::CONST + 1] = one;
+        if (SD == 8) row[FEW_CONST] = row[SL::CONST], row[FEW_CONST + 1] = one;
     }
     uint4 *o1 = reinterpret_cast<uint4 *>(scratch + OFF_B1) + ((size_t)s * BN + j) * 4, *o2 = reinterpret_cast<uint4 *>(scratch + OFF_B2) + ((size_t)s * BN + j) * 2;
 #pragma unroll
@@ -979,11 +993,11 @@ struct PqMaps {
     CUtensorMap x, b1, b2;
 };
 
-template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP = 0>
-static void launch_w(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
+template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP, bool FEW>
+static void launch_k(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
 {
-    auto kernel = pq_tc_kernel<SD, TRAIN, METRIC, WIDE, DUMP>;
-    constexpr size_t smem = PQ_TC_SMEM<SD>;
+    auto kernel = pq_tc_kernel<SD, TRAIN, METRIC, WIDE, DUMP, FEW>;
+    constexpr size_t smem = PQ_TC_SMEM<SD, FEW>;
     static std::atomic<unsigned long long> configured{0}; // bit d: the attribute has been set on device d (it is per device and sticky)
     const unsigned long long bit = 1ull << (dev.device() & 63);
     if (!(configured.load(std::memory_order_relaxed) & bit)) {
@@ -993,6 +1007,17 @@ static void launch_w(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, uns
     KernelScope ks(dev, TRAIN ? "assign_train" : "pq_encode");
     launch_following(kernel, grid, NTHREADS, smem, dev.stream(), mp.x, mp.b1, mp.b2, q);
     dev.count_launch();
+}
+
+// Two steps instead of three (FEW in the header) for training passes and encodes of many rows, 8-wide.  us, three / two: encode of 1,500 x 128, m 16,
+// k 256 16.6 / 16.9, 4,000 23.3 / 23.7, 8,000 19.0 / 17.9, 20,000 24.8 / 23.0, 300,000 132.6 / 128.8; fits of 10 iterations, 2,500 rows 474 / 462,
+// 20,000 628 / 609, 100,000 939 / 905.
+constexpr unsigned long long FEW_ENCODE_ROWS = 6000;
+
+template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP = 0> static void launch_w(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
+{
+    if (SD == 8 && (TRAIN || q.a.n >= FEW_ENCODE_ROWS)) launch_k<SD, TRAIN, METRIC, WIDE, DUMP, SD == 8>(dev, mp, q, grid);
+    else launch_k<SD, TRAIN, METRIC, WIDE, DUMP, false>(dev, mp, q, grid);
 }
 
 template <int SD, bool TRAIN, int METRIC> static void launch_t(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
@@ -1061,7 +1086,7 @@ void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train
     PqMaps mp;
     mp.b1 = b.maps->b1, mp.b2 = b.maps->b2;
     // the rows as they lie: a box is one tile of a group's columns
-    mp.x = make_tensor_map_2d(p.x, (unsigned long long)p.m * p.sd, p.n, 4 * p.sd, BM, p.sd == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, p.ld);
+    mp.x = make_tensor_map_2d(p.x, (unsigned long long)p.m * p.sd, p.n, 2 * p.sd, 32, p.sd == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, p.ld);
     PqTcParams q = {};
     q.a = p;
     if (!train) q.a.codes = b.codes;
