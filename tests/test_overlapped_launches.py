@@ -14,7 +14,7 @@ ALLOWED = {
     "pq_operand_b_kernel": set(), "pq_tc_kernel": {"P.x"}, "pq_queue_drain": {"P.x"}, "pq_expand_kernel": {"c16", "centroids"},
     "queue_sums_kernel": {"xp", "i"},  # (its load_piece takes a number)
     "resolve_kernel": {"x", "book", "c", "xr"}, "ordered_hist_kernel": set(), "ordered_lists_kernel": set(), "ordered_lists_cluster_kernel": set(),
-    "ordered_sums_kernel": {"x"}, "ordered_sums_long_kernel": {"x"}, "init_tree_kernel": set(), "chunk_sums_kernel": {"x"}, "node_mean_kernel": set(), "node_stats_kernel": {"x"},
+    "ordered_sums_kernel": {"x"}, "ordered_sums_long_kernel": {"x"}, "init_tree_kernel": set(), "chunk_sums_kernel": {"x"}, "node_mean_kernel": set(), "node_stats_kernel": {"x"}, "node_stats_stream_kernel": {"x"},
     "node_spread_stream_kernel": {"x", "perm", "xcol", "p"}, "split_kernel": {"x", "perm"}, "next_level_kernel": set(), "no_children_kernel": set(),
 }
 
