@@ -2,6 +2,7 @@
 // patches, rotation / cross-covariance for OPQ, row-wise distances and the element-wise quantizers.
 // The nearest-centroid kernels live in assign_reg.cuh / assign_generic.cuh (launched from assign_launch.cu).
 #include "cuda_device.hpp"
+#include "dense_image.cuh"
 
 #include <algorithm>
 #include <chrono>
@@ -201,7 +202,7 @@ bool CudaDevice::lasting(cudaStream_t s) const { return s == own_stream_ || s ==
 void CudaDevice::end_call()
 {
     release_dense();
-    bop_fresh_ = nullptr; // the next call's centroids may have the same address
+    bop_fresh_ = dense_fresh_ = nullptr; // the next call's centroids may have the same address
     if (!unfinished_ || lasting(stream_)) return;
     if (captured(stream_)) unfinished_ = false;
     else if (cudaEventRecord(order_event_, stream_) != cudaSuccess) cudaGetLastError(); // (not the next launch's error)
@@ -515,7 +516,7 @@ void CudaDevice::check_tc_error()
 
 void CudaDevice::prepare_rows(const Shape &sh, const float *x)
 {
-    bop_fresh_ = nullptr;
+    bop_fresh_ = dense_fresh_ = nullptr;
     const bool by_apply = prepared_by_apply_ && prepared_x_ == x && prepared_n_ == sh.n_local && prepared_dim_ == sh.sd;
     prepared_by_apply_ = false;
     if (by_apply && sh.m == 1 && dense_tc_applicable(sh.sd, sh.k, M_SQ)) return; // rvq_update has just written these rows and their images
@@ -540,7 +541,8 @@ void CudaDevice::dense_debug(const float *x, size_t n, size_t dim, const float *
     VQB_CUDA_CHECK(cudaMemsetAsync(tc_stats_, 0, 3 * sizeof(unsigned long long), stream_));
     dense_frame(*this, w, x, n, dim, nullptr, nullptr, false); // the caller asked for x.c
     dense_prepare(*this, w, x, n, dim);
-    dense_shortlist(*this, w, n, dim, codebook, k, tc_stats_, tc_error_, dots, nullptr);
+    dense_fresh_ = nullptr;
+    dense_shortlist(*this, w, n, dim, codebook, k, tc_stats_, tc_error_, dots, nullptr, false);
     download(stats3, tc_stats_, 3 * sizeof(unsigned long long));
     prepared_x_ = nullptr;
 }
@@ -692,7 +694,7 @@ void CudaDevice::patch_centroids(const Shape &sh, const float *x, uint64_t row_b
                                  size_t n_patches, float *centroids, Comm *comm)
 {
     if (n_patches == 0) return;
-    bop_fresh_ = nullptr; // the centroids change behind the fused update's back
+    bop_fresh_ = dense_fresh_ = nullptr; // the centroids change behind the fused update's back
     const bool arriving = arrival_.dev && x == arrival_.dev && arrival_.awaited < arrival_.pieces;
     bool here = !arriving && row_begin == 0 && (!comm || comm->world() <= 1);
     for (size_t i = 0; here && i < n_patches; ++i) here = patches[i].row < sh.n_local;
@@ -752,7 +754,7 @@ void CudaDevice::dense_decide(const float *x, size_t n, size_t dim, const float 
         if (n > dense_rows_) dense_prepare(*this, dense_, xp, rows, dim);
         VQB_CUDA_CHECK(cudaMemsetAsync(dense_.list_count, 0, sizeof(uint32_t), stream_));
         const ShortlistTrain tr = {codes + r0, changed};
-        dense_shortlist(*this, dense_, rows, dim, codebook, k, stats, tc_error_, nullptr, &tr);
+        dense_shortlist(*this, dense_, rows, dim, codebook, k, stats, tc_error_, nullptr, &tr, codebook == dense_fresh_);
         dense_resolve(*this, dense_, xp, rows, dim, codebook, k, euclid, codes + r0, changed);
     }
 }
@@ -931,7 +933,8 @@ void CudaDevice::rvq_update(float *res, size_t n, size_t dim, const float *centr
             a.codebook = centroids;
             a.codes = codes + r0;
             a.norm_sum = norm_sum;
-            rvq_apply(*this, a, dense_);
+            rvq_apply(*this, a, dense_); // (a new frame)
+            dense_fresh_ = nullptr;
         }
         release(codes);
         prepared_by_apply_ = n <= dense_rows_; // the next stage's images are there
@@ -1559,7 +1562,7 @@ void CudaDevice::accumulate(const Shape &sh, const float *x, const void *codes, 
 // One CTA of 8 warps per (sub-space, 32 clusters): a warp takes four clusters, its lanes the dimensions.
 // ------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) update_centroids_kernel(float *sums, uint32_t *counts, uint32_t *moved, int counts_f32, const uint32_t *active,
-                                                               int k, int sd, float *centroids, StatusPage sp, const PeerView pv)
+                                                               int k, int sd, float *centroids, StatusPage sp, const PeerView pv, const DenseOperand dense)
 {
     __shared__ uint32_t s_bits;
     const int s = blockIdx.x, word = blockIdx.y;
@@ -1638,6 +1641,20 @@ __global__ void __launch_bounds__(256) update_centroids_kernel(float *sums, uint
             }
             sp.put(sp.idx_moved(s), act ? mv : 0u);
             if (s == 0) sp.put_error();
+        }
+    }
+    // full-width k-means: the images of these centroids for the next assignment pass, while the host looks at the flags (in a kernel of its
+    // own between two passes they took 5 us of an iteration)
+    if (dense.image && act) {
+        const FramePiece frame = load_frame(dense.frame, lane);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int j = word * 32 + warp * 4 + q;
+            const bool in = j < k;
+            float v[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = in && 4 * lane + e < sd ? centroids[(size_t)j * sd + 4 * lane + e] : 0.0f;
+            store_codebook_row(dense.image, dense.half_norms, dense.dimp, j, v, frame, in, lane);
         }
     }
 }
@@ -1754,12 +1771,16 @@ void CudaDevice::update_centroids(const Shape &sh, const IterBuffers &buf, const
     const unsigned wps = (unsigned)((k + 31) / 32);
     if (wps > 65535u) throw Error(103, "more than 2,097,120 clusters per sub-space are not supported");
     const StatusPage sp = status_page(m, k);
+    DenseOperand dense = {};
+    if (prepared_x_ && m == 1 && prepared_dim_ == sh.sd && prepared_n_ == sh.n_local && dense_tc_applicable(sh.sd, k, M_SQ))
+        dense = DenseOperand{dense_.frame, dense_.book_image, dense_.half_norms, (int)dense_padded(sh.sd)};
     {
         KernelScope ks(*this, "update_centroids");
         launch_following(update_centroids_kernel, dim3((unsigned)m, wps), 256, 0, stream_, buf.sums, buf.counts, buf.moved, buf.counts_f32 ? 1 : 0, active, (int)k,
-                         (int)sh.sd, centroids, sp, pv);
+                         (int)sh.sd, centroids, sp, pv, dense);
         count_launch();
     }
+    dense_fresh_ = dense.image ? centroids : nullptr;
     wait_status(sp, m, k, status);
 }
 

@@ -150,6 +150,7 @@ class CudaDevice : public Device {
     void wait_status(const StatusPage &sp, size_t m, size_t k, IterStatus &out);
     // centroids whose operand B (pq_tc.cu) the scratch currently holds, written by the fused centroid update
     const float *bop_fresh_ = nullptr;
+    const float *dense_fresh_ = nullptr; // and those whose images (dense_tc.cu) dense_ holds, in its present frame
     // full-width tensor path (dense_tc.cu): which rows dense_ holds the images of, and the block behind dense_
     bool tensor_enabled_ = true;
     const float *prepared_x_ = nullptr;

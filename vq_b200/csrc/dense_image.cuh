@@ -57,4 +57,22 @@ __device__ __forceinline__ float store_image(uint16_t *row_image, int dimp, int 
     return a;
 }
 
+// What an assignment pass needs of the centroids, for a kernel that has them at hand.
+struct DenseOperand {
+    const float *frame;
+    uint16_t *image; // null: nothing to write
+    float *half_norms;
+    int dimp;
+};
+
+// A warp writes image and half norm of centroid j (zeros and +inf where there is none)
+__device__ __forceinline__ void store_codebook_row(uint16_t *image, float *half_norms, int dimp, int j, const float (&v)[4], FramePiece f, bool in, int lane)
+{
+    if (!in) f.mu[0] = f.mu[1] = f.mu[2] = f.mu[3] = 0.0f;
+    float a = store_image(image + (size_t)j * 2 * dimp, dimp, lane, v, f, true);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (lane == 0) half_norms[j] = in ? 0.5f * a : __int_as_float(0x7f800000);
+}
+
 } // namespace vqb

@@ -478,12 +478,7 @@ __global__ void __launch_bounds__(256) dense_codebook_kernel(const float *c, int
     float v[4]; // (ordinary loads: a centroid update may come directly before)
 #pragma unroll
     for (int e = 0; e < 4; ++e) v[e] = in && 4 * lane + e < dim ? c[(size_t)j * dim + 4 * lane + e] : 0.0f;
-    FramePiece f = load_frame(frame, lane);
-    if (!in) f.mu[0] = f.mu[1] = f.mu[2] = f.mu[3] = 0.0f;
-    float a = store_image(image + (size_t)j * 2 * dimp, dimp, lane, v, f, true);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-    if (lane == 0) hn[j] = in ? 0.5f * a : VQB_DENSE_INF;
+    store_codebook_row(image, hn, dimp, j, v, load_frame(frame, lane), in, lane);
 }
 
 // Images and (upper bounds of the) squared norms of the rows: one read, one write of the same size.  L lanes per row (8, 16 or
@@ -549,11 +544,11 @@ void dense_prepare(CudaDevice &dev, const DenseWork &w, const float *x, size_t n
 }
 
 void dense_shortlist(CudaDevice &dev, const DenseWork &w, size_t n, size_t dim, const float *codebook, size_t k, unsigned long long *stats,
-                     int *error_word, float *debug_dots, const ShortlistTrain *train)
+                     int *error_word, float *debug_dots, const ShortlistTrain *train, bool book_there)
 {
     if (n == 0) return;
     const int dimp = (int)dense_padded(dim);
-    {
+    if (!book_there) {
         KernelScope ks(dev, "dense_codebook");
         launch_following(dense_codebook_kernel, BN / 8, 256, 0, dev.stream(), codebook, (int)k, (int)dim, dimp, w.frame, w.book_image, w.half_norms);
         dev.count_launch();

@@ -37,13 +37,13 @@ void dense_prepare(CudaDevice &dev, const DenseWork &w, const float *x, size_t n
 
 // Decides every row that has a single candidate -- codes[r] is rewritten, *changed gets VQB_MOVED_BITS when a row moved -- and
 // appends the other rows (also those that cannot be ranked: NaN, infinity) to w.list with their masks in w.cand
-// (*w.list_count zero on entry).  Without `train` all rows get their mask and nothing else happens (diagnostics).
+// (*w.list_count zero on entry); book_there: w holds the codebook's image already.  Without `train` all rows get their mask and nothing else happens (diagnostics).
 struct ShortlistTrain {
     uint8_t *codes;
     uint32_t *changed;
 };
 void dense_shortlist(CudaDevice &dev, const DenseWork &w, size_t n, size_t dim, const float *codebook, size_t k, unsigned long long *stats,
-                     int *error_word, float *debug_dots, const ShortlistTrain *train);
+                     int *error_word, float *debug_dots, const ShortlistTrain *train, bool book_there);
 
 // The listed rows: the reference's own arithmetic over their candidates.
 void dense_resolve(CudaDevice &dev, const DenseWork &w, const float *x, size_t n, size_t dim, const float *codebook, size_t k, bool euclid,
