@@ -454,7 +454,7 @@ const DenseWork &CudaDevice::dense_work(size_t n, size_t dim, size_t beside)
     const size_t book = up(256 * 4 * dimp), hn = up(256 * sizeof(float)), frame = up(129 * sizeof(float));
     auto total = [&](size_t rows) {
         image = up(rows * 4 * dimp), norms = up(rows * sizeof(float)), cand = up(rows * DENSE_MASK_WORDS * sizeof(uint32_t));
-        list = up((rows + 1) * sizeof(uint32_t));
+        list = up((rows + 3) * sizeof(uint32_t));
         return image + norms + cand + list + book + hn + frame;
     };
     size_t rows = cap ? std::min(n, std::max<size_t>(128, std::strtoull(cap, nullptr, 10) / 128 * 128)) : n;
@@ -484,7 +484,8 @@ const DenseWork &CudaDevice::dense_work(size_t n, size_t dim, size_t beside)
     dense_.norms = reinterpret_cast<float *>(take(norms));
     dense_.cand = reinterpret_cast<uint32_t *>(take(cand));
     dense_.list_count = reinterpret_cast<uint32_t *>(take(list));
-    dense_.list = dense_.list_count + 1;
+    dense_.list = dense_.list_count + 3;
+    VQB_CUDA_CHECK(cudaMemsetAsync(dense_.list_count, 0, 3 * sizeof(uint32_t), stream_)); // dense_resolve leaves it at zero
     dense_.book_image = reinterpret_cast<uint16_t *>(take(book));
     dense_.half_norms = reinterpret_cast<float *>(take(hn));
     dense_.frame = reinterpret_cast<float *>(take(frame));
@@ -493,7 +494,7 @@ const DenseWork &CudaDevice::dense_work(size_t n, size_t dim, size_t beside)
 
 void CudaDevice::release_dense()
 {
-    prepared_x_ = nullptr;
+    prepared_x_ = dense_fresh_ = nullptr;
     prepared_by_apply_ = false;
     if (!dense_block_) return;
     release(dense_block_);
@@ -752,7 +753,6 @@ void CudaDevice::dense_decide(const float *x, size_t n, size_t dim, const float 
         const size_t rows = std::min(dense_rows_, n - r0);
         const float *xp = x + r0 * dim;
         if (n > dense_rows_) dense_prepare(*this, dense_, xp, rows, dim);
-        VQB_CUDA_CHECK(cudaMemsetAsync(dense_.list_count, 0, sizeof(uint32_t), stream_));
         const ShortlistTrain tr = {codes + r0, changed};
         dense_shortlist(*this, dense_, rows, dim, codebook, k, stats, tc_error_, nullptr, &tr, codebook == dense_fresh_);
         dense_resolve(*this, dense_, xp, rows, dim, codebook, k, euclid, codes + r0, changed);
@@ -774,7 +774,7 @@ void CudaDevice::assign_train(const Shape &sh, const float *x, const float *cent
             unsigned long long st3[3] = {0, 0, 0};
             download(st3, tc_stats_, sizeof st3);
             uint32_t listed = 0;
-            download(&listed, dense_.list_count, sizeof listed);
+            download(&listed, dense_.list_count + 2, sizeof listed);
             std::fprintf(stderr, "[vqb] shortlist: rows %llu candidates %llu (%.2f per row) full scans %llu, %u rows left for the exact kernel\n", st3[0],
                          st3[1], st3[0] ? (double)st3[1] / (double)st3[0] : 0.0, st3[2], listed);
         }

@@ -24,7 +24,7 @@ struct DenseWork {
     float *norms = nullptr;         // [n] upper bounds of |s (x - mu)|^2
     uint32_t *cand = nullptr;       // [n][8] bit j set: centroid j may be the reference's choice (all k bits set: examine all)
     uint32_t *list = nullptr;       // [n] rows with more than one candidate
-    uint32_t *list_count = nullptr;
+    uint32_t *list_count = nullptr; // [3] how many, CTAs that are done with them (both zero between passes), how many the last pass had
     uint16_t *book_image = nullptr; // [256][2 * dense_padded(dim)]
     float *half_norms = nullptr;    // [256]
     float *frame = nullptr;         // [129] mu and s (dense_image.cuh)

@@ -18,7 +18,7 @@ namespace {
 // the way to a few centroids in L2: 16 loads per lane are on their way at once.
 template <bool VEC>
 __global__ void __launch_bounds__(256) resolve_kernel(const float *__restrict__ x, int dim, int k, const float *__restrict__ book, int euclid,
-                                                      const uint32_t *cand, const uint32_t *list, const uint32_t *list_count,
+                                                      const uint32_t *cand, const uint32_t *list, uint32_t *list_count,
                                                       uint8_t *codes, uint32_t *changed)
 {
     __shared__ uint8_t s_number[8][256];
@@ -77,6 +77,9 @@ __global__ void __launch_bounds__(256) resolve_kernel(const float *__restrict__ 
         __syncwarp();
     }
     if (lane == 0 && moved && changed) atomicOr(changed, VQB_MOVED_BITS);
+    // the list is empty again for the next pass (a memset between two passes of few rows took 4 us, and the overlap of their launches)
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(list_count + 1, 1u) == gridDim.x - 1) list_count[0] = list_count[1] = 0u, list_count[2] = total;
 }
 
 // L lanes per row, four values each (as dense_prepare_kernel): one read of the rows, one write of the residuals, one of their
