@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(done) : "l"(P.wait) : "memory");
             if (done < (uint32_t)P.stages) {
                 *abort_flag = 1;
-                atomicCAS(P.error, 0, 34);
+                atomicCAS(P.error, 0, 44);
             }
             asm volatile("fence.proxy.async;" ::: "memory");
         }
@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();
             // ---- 2. scores
-            if (tid == 0 && mbar_wait(&sh.bars.bfull, it & 1u, abort_flag, P.error, 31)) {
+            if (tid == 0 && mbar_wait(&sh.bars.bfull, it & 1u, abort_flag, P.error, 41)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t ad = smem_desc_sw128(smem_u32(a_smem)), bd = smem_desc_sw128(smem_u32(b_smem));
                 auto at = [](int step, uint32_t chunk_bytes) { return (uint64_t)((step >> 2) * (int)(chunk_bytes >> 4) + 2 * (step & 3)); };
@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
                 umma_commit(&sh.bars.tfull);
             }
             __syncwarp();
-            const bool there = mbar_wait(&sh.bars.tfull, it & 1u, abort_flag, P.error, 32);
+            const bool there = mbar_wait(&sh.bars.tfull, it & 1u, abort_flag, P.error, 42);
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (tid == 0 && there && (st + 1 < P.stages || tile + gridDim.x < n_tiles)) load_book(st + 1 < P.stages ? st + 1 : 0), ++loads;
             // ---- 3. the largest score of each row, then the centroids within the bound
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
         }
     }
     // (after an abort: a codebook that is still on its way has to land before the CTA goes; a bounded wait, and at once for a phase that is over)
-    if (!ok && tid == 0 && loads > 0) mbar_wait(&sh.bars.bfull, (loads - 1) & 1u, abort_flag, P.error, 33);
+    if (!ok && tid == 0 && loads > 0) mbar_wait(&sh.bars.bfull, (loads - 1) & 1u, abort_flag, P.error, 43);
     if (P.wait && tid == 0 && atomicAdd(P.wait + 1, 1u) == gridDim.x - 1) P.wait[0] = P.wait[1] = 0u; // nobody looks at them any more
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
