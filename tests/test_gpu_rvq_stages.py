@@ -51,3 +51,26 @@ def test_norms_next_to_epsilon_are_added_up_in_order(oracle):
     assert 100 < (codes_o[:, 1] == 0xFFFFFFFF).sum() < 1_900  # the case is on both sides
     got, codes = vq.ResidualQuantizer.from_codebooks(books, eps, vq.Distance.Euclidean).quantize(x, return_codes=True)
     assert np.array_equal(codes, codes_o) and np.array_equal(got.view(np.uint16), want)
+
+
+@pytest.mark.parametrize("n", [2_000, 20_000])
+def test_captured_encode_follows_its_rows(n):
+    """One launch and two, replayed: the counters that the CTAs of the first wait on are left as they were found."""
+    import torch
+
+    x = torch.from_numpy(synth.gaussian_mixture(n, 128, 7)).cuda()
+    books = (0.3 * synth.normal(3 * 256, 128, 3)).reshape(3, 256, 128)
+    q = vq.ResidualQuantizer.from_codebooks(books, 0.01, vq.Distance.Euclidean)
+    q.quantize(x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out, codes = q.quantize(x, return_codes=True)
+    for seed in (7, 8):
+        x.copy_(torch.from_numpy(synth.gaussian_mixture(n, 128, seed)))
+        graph.replay()
+        graph.replay()
+        torch.cuda.synchronize()
+        got, got_codes = out.clone(), codes.clone()
+        want, want_codes = q.quantize(x, return_codes=True)
+        assert torch.equal(got_codes, want_codes) and torch.equal(got, want)

@@ -632,7 +632,8 @@ template <int THREADS> __global__ void __launch_bounds__(THREADS) rvq_books_kern
     make_book<THREADS>(sh, books, blockIdx.x, k, dim, dimp, bn, vec != 0, frames, image, extra);
 }
 
-template <int KS, int BN, int ROWS> void launch_stages(CudaDevice &dev, const CUtensorMap &map, const RvqStagesParams &p)
+// False: a cooperative launch whose CTAs cannot all be resident (SMs that this process may not use)
+template <int KS, int BN, int ROWS> bool launch_stages(CudaDevice &dev, const CUtensorMap &map, const RvqStagesParams &p)
 {
     auto kernel = rvq_stages_kernel<KS, BN, ROWS>;
     constexpr size_t smem = stages_smem<KS, BN>();
@@ -646,16 +647,22 @@ template <int KS, int BN, int ROWS> void launch_stages(CudaDevice &dev, const CU
     KernelScope ks(dev, "rvq_quantize");
     if (p.wait) {
         void *args[] = {const_cast<CUtensorMap *>(&map), const_cast<RvqStagesParams *>(&p)};
-        VQB_CUDA_CHECK(cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(NT), args, smem, dev.stream()));
+        const cudaError_t e = cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(NT), args, smem, dev.stream());
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            cudaGetLastError();
+            return false;
+        }
+        VQB_CUDA_CHECK(e);
     } else launch_following(kernel, grid, NT, smem, dev.stream(), map, p);
     dev.count_launch();
+    return true;
 }
 
-template <int KS> void launch_ks(CudaDevice &dev, const CUtensorMap &map, const RvqStagesParams &p, int bn)
+template <int KS> bool launch_ks(CudaDevice &dev, const CUtensorMap &map, const RvqStagesParams &p, int bn)
 {
     const bool few = p.n <= (unsigned long long)dev.sm_count() * (BM / 2);
-    if (bn == 256) few ? launch_stages<KS, 256, 4>(dev, map, p) : launch_stages<KS, 256, 8>(dev, map, p);
-    else few ? launch_stages<KS, 128, 4>(dev, map, p) : launch_stages<KS, 128, 8>(dev, map, p);
+    if (bn == 256) return few ? launch_stages<KS, 256, 4>(dev, map, p) : launch_stages<KS, 256, 8>(dev, map, p);
+    return few ? launch_stages<KS, 128, 4>(dev, map, p) : launch_stages<KS, 128, 8>(dev, map, p);
 }
 
 int book_rows(int k) { return k > 128 ? 256 : 128; }
@@ -690,25 +697,33 @@ void launch_rvq_stages(CudaDevice &dev, const GenericParams &g, bool euclid, voi
     // there were several launches a stage, it is two, and no CTA waits for another.
     const int tk = g.k > 128 ? 128 : g.k > 64 ? 64 : 32;
     const bool one = (double)g.n <= (tk == 128 ? 2.0e6 : tk == 64 ? 4.6e6 : 6.8e6) / (dimp + 32) * (whole ? 1.0 : 0.6);
-    if (!one) {
+    auto make_books = [&] {
         KernelScope ks(dev, "rvq_books");
         rvq_books_kernel<1024><<<g.stages, 1024, 0, dev.stream()>>>(g.centroids, g.k, g.sd, dimp, bn, whole, frames, image, extra);
         VQB_CUDA_CHECK(cudaGetLastError());
         dev.count_launch();
-    }
+    };
+    if (!one) make_books();
     const CUtensorMap map = make_tensor_map_2d(image, 2 * (unsigned long long)dimp, rows, CHUNK, (unsigned)bn, CU_TENSOR_MAP_SWIZZLE_128B);
     RvqStagesParams p = {};
     p.x = g.x, p.books = g.centroids, p.n = g.n, p.dim = g.sd, p.k = g.k, p.stages = g.stages, p.euclid = euclid, p.epsilon = g.epsilon;
     p.vec = whole && (reinterpret_cast<uintptr_t>(g.x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(g.out_f16) & 7u) == 0;
     p.frames = frames, p.image = image, p.extra = extra, p.book_vec = whole, p.wait = one ? dev.wait_words() : nullptr, p.out_f16 = g.out_f16, p.out_codes = g.out_codes, p.error = dev.error_word();
-    switch (dimp / 16) {
-    case 2: launch_ks<2>(dev, map, p, bn); break;
-    case 3: launch_ks<3>(dev, map, p, bn); break;
-    case 4: launch_ks<4>(dev, map, p, bn); break;
-    case 5: launch_ks<5>(dev, map, p, bn); break;
-    case 6: launch_ks<6>(dev, map, p, bn); break;
-    case 7: launch_ks<7>(dev, map, p, bn); break;
-    default: launch_ks<8>(dev, map, p, bn); break;
+    auto launch = [&] {
+        switch (dimp / 16) {
+        case 2: return launch_ks<2>(dev, map, p, bn);
+        case 3: return launch_ks<3>(dev, map, p, bn);
+        case 4: return launch_ks<4>(dev, map, p, bn);
+        case 5: return launch_ks<5>(dev, map, p, bn);
+        case 6: return launch_ks<6>(dev, map, p, bn);
+        case 7: return launch_ks<7>(dev, map, p, bn);
+        default: return launch_ks<8>(dev, map, p, bn);
+        }
+    };
+    if (!launch()) {
+        make_books();
+        p.wait = nullptr;
+        launch();
     }
 }
 
