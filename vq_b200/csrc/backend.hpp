@@ -105,6 +105,9 @@ class Device {
     virtual void *alloc(size_t bytes) = 0;
     virtual void release(void *p) = 0;
     virtual void upload(void *dst, const void *src, size_t bytes) = 0;   // host -> device, complete on return
+    // The same for what the call itself goes on to use: the source may be reused on return, and whatever the device is asked for later comes
+    // after the copy, but nobody has waited for it.
+    virtual void upload_queued(void *dst, const void *src, size_t bytes) { upload(dst, src, bytes); }
     virtual void download(void *dst, const void *src, size_t bytes) = 0; // device -> host, complete on return
     virtual void copy(void *dst, const void *src, size_t bytes) = 0;     // device -> device
     virtual void zero(void *dst, size_t bytes) = 0;

@@ -203,6 +203,7 @@ void CudaDevice::end_call()
 {
     release_dense();
     bop_fresh_ = dense_fresh_ = nullptr; // the next call's centroids may have the same address
+    if (upload_at_) upload_at_ = UPLOAD_BYTES; // and its stream another one: its first upload waits for the last of this call
     if (!unfinished_ || lasting(stream_)) return;
     if (captured(stream_)) unfinished_ = false;
     else if (cudaEventRecord(order_event_, stream_) != cudaSuccess) cudaGetLastError(); // (not the next launch's error)
@@ -277,25 +278,31 @@ void CudaDevice::upload(void *dst, const void *src, size_t bytes)
         VQB_CUDA_CHECK(cudaStreamSynchronize(stream_));
         return;
     }
-    // Small ones go through pinned memory, and nobody waits for them: a fit of 10,000 x 128 spent 75 of its 550 us in two copies from pageable
-    // memory (64 KiB of row numbers, 64 bytes of flags) and their waits.
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (stage_ && bytes <= UPLOAD_BYTES / 4 && cudaStreamIsCapturing(stream_, &capturing) == cudaSuccess && capturing == cudaStreamCaptureStatusNone) {
-        const size_t room = (bytes + 63) / 64 * 64;
-        if (upload_at_ + room > UPLOAD_BYTES) { // from the start again, once the copies have read what is there
-            VQB_CUDA_CHECK(cudaEventSynchronize(upload_event_));
-            upload_at_ = 0;
-        }
-        unsigned char *from = stage_ + STAGE_BYTES + upload_at_;
-        std::memcpy(from, src, bytes);
-        VQB_CUDA_CHECK(cudaMemcpyAsync(dst, from, bytes, cudaMemcpyHostToDevice, stream_));
-        VQB_CUDA_CHECK(cudaEventRecord(upload_event_, stream_)); // (a stream comes after the work of the one before: set_stream)
-        upload_at_ += room;
-        unfinished_ = true;
-        return;
-    }
     VQB_CUDA_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream_));
     VQB_CUDA_CHECK(cudaStreamSynchronize(stream_));
+}
+
+// Small ones go through pinned memory, and nobody waits for them: a fit of 10,000 x 128 spent 75 of its 550 us in two copies from pageable
+// memory (64 KiB of row numbers, 64 bytes of flags) and their waits.
+void CudaDevice::upload_queued(void *dst, const void *src, size_t bytes)
+{
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    const bool arriving = arrival_.dev && arrival_.awaited < arrival_.pieces;
+    if (!stage_ || arriving || !bytes || bytes > UPLOAD_BYTES / 4 || cudaStreamIsCapturing(stream_, &capturing) != cudaSuccess || capturing != cudaStreamCaptureStatusNone) {
+        upload(dst, src, bytes);
+        return;
+    }
+    const size_t room = (bytes + 63) / 64 * 64;
+    if (upload_at_ + room > UPLOAD_BYTES) { // from the start again, once the copies have read what is there (also at the first of a call: end_call)
+        VQB_CUDA_CHECK(cudaEventSynchronize(upload_event_));
+        upload_at_ = 0;
+    }
+    unsigned char *from = stage_ + STAGE_BYTES + upload_at_;
+    std::memcpy(from, src, bytes);
+    VQB_CUDA_CHECK(cudaMemcpyAsync(dst, from, bytes, cudaMemcpyHostToDevice, stream_));
+    VQB_CUDA_CHECK(cudaEventRecord(upload_event_, stream_)); // (a call has one stream)
+    upload_at_ += room;
+    unfinished_ = true;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -701,7 +708,7 @@ void CudaDevice::patch_centroids(const Shape &sh, const float *x, uint64_t row_b
     for (size_t i = 0; here && i < n_patches; ++i) here = patches[i].row < sh.n_local;
     if (here) {
         RowPatch *pd = (RowPatch *)alloc(sizeof(RowPatch) * n_patches);
-        upload(pd, patches, sizeof(RowPatch) * n_patches);
+        upload_queued(pd, patches, sizeof(RowPatch) * n_patches);
         {
             KernelScope ks(*this, "patch_centroids");
             patch_copy_kernel<<<blocks_for(n_patches * sh.sd, 256, 4096), 256, 0, stream_>>>(x, sh.ld, (int)sh.k, (int)sh.sd, pd, n_patches, centroids);
@@ -713,7 +720,7 @@ void CudaDevice::patch_centroids(const Shape &sh, const float *x, uint64_t row_b
     }
     RowPatch *pd = (RowPatch *)alloc(sizeof(RowPatch) * n_patches);
     uint32_t *stage = (uint32_t *)alloc(sizeof(uint32_t) * n_patches * sh.sd);
-    upload(pd, patches, sizeof(RowPatch) * n_patches);
+    upload_queued(pd, patches, sizeof(RowPatch) * n_patches);
     const size_t total = n_patches * sh.sd;
     KernelScope ks(*this, "patch_centroids");
     if (arriving) {

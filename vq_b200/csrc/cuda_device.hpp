@@ -35,6 +35,7 @@ class CudaDevice : public Device {
     uint8_t *pq_kept_codes() const { return pq_codes_; }
     void release(void *p) override;
     void upload(void *dst, const void *src, size_t bytes) override;
+    void upload_queued(void *dst, const void *src, size_t bytes) override;
     void download(void *dst, const void *src, size_t bytes) override;
     // two of them with one wait (either may be empty)
     void download(void *dst, const void *src, size_t bytes, void *dst2, const void *src2, size_t bytes2);

@@ -159,7 +159,7 @@ void lbg_fit(Device &dev, Comm *comm, const Shape &sh, const float *x, size_t ma
         for (size_t s = 0; s < m; ++s) any = any || active[s];
         if (!any) break;
         if (active_dirty) { // the mask only changes when a subspace retires
-            dev.upload(act.p, active.data(), sizeof(uint32_t) * m);
+            dev.upload_queued(act.p, active.data(), sizeof(uint32_t) * m);
             active_dirty = false;
         }
         if (direct) buf = pair[it & 1];
