@@ -428,8 +428,8 @@ void CudaDevice::ensure_tc_buffers()
     pq_maps_.reset(new PqTcMaps(pq_tc_make_maps(pq_scratch_)));
     VQB_CUDA_CHECK(cudaMalloc(&tc_stats_, 3 * sizeof(unsigned long long)));
     VQB_CUDA_CHECK(cudaMemsetAsync(tc_stats_, 0, 3 * sizeof(unsigned long long), stream_));
-    VQB_CUDA_CHECK(cudaMalloc(&tc_error_, 16 * sizeof(int))); // the error word, and from the ninth on wait_words()
-    VQB_CUDA_CHECK(cudaMemsetAsync(tc_error_, 0, 16 * sizeof(int), stream_));
+    VQB_CUDA_CHECK(cudaMalloc(&tc_error_, sizeof(int)));
+    VQB_CUDA_CHECK(cudaMemsetAsync(tc_error_, 0, sizeof(int), stream_));
     unfinished_ = true; // the first call may come on another stream
 }
 

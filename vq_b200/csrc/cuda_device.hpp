@@ -107,7 +107,6 @@ class CudaDevice : public Device {
     size_t smem_limit() const { return smem_limit_; }
     void end_call(); // at the end of every call of the C ABI
     int *error_word() const { return tc_error_; } // null with VQB_NO_TENSOR=1
-    uint32_t *wait_words() const { return reinterpret_cast<uint32_t *>(tc_error_) + 8; } // two counters that a launch leaves at zero
     uint64_t launches() const { return launches_.load(); }
     void count_launch(uint64_t n = 1) { launches_ += n, unfinished_ = true; }
     // How often this context has asked CUDA for device or pinned memory (cudaMalloc, cudaMallocAsync, cudaHostAlloc).

@@ -61,7 +61,7 @@ struct RvqApply {
 };
 void rvq_apply(CudaDevice &dev, const RvqApply &a, const DenseWork &w);
 
-// The residual encoder with all its stages in one launch (rvq_tc.cu), for shapes that dense_tc_applicable takes.
+// The residual encoder with all its stages in one kernel (rvq_tc.cu), for shapes that dense_tc_applicable takes.
 struct GenericParams;
 bool rvq_stages_pays(const GenericParams &g);                        // more rows than direct.cu is faster with
 size_t rvq_stages_bytes(size_t dim, size_t k, size_t stages);        // device memory that it needs
