@@ -979,7 +979,10 @@ void CudaDevice::rvq_quantize(const float *x, size_t n, size_t dim, const float 
     g.out_codes = out_codes;
     g.stages = (int)stages;
     g.epsilon = epsilon;
-    if (tensor_enabled_ && stages > 0 && dense_tc_applicable(dim, k, metric) && rvq_stages_pays(g)) {
+    // An encode of few rows that is being captured stays one node without memory of its own (CUDA lets a graph with such memory exist in one
+    // instance only): direct.cu.  4,999 x 128, 8 stages: 154 us instead of 67; 2,000 x 128, 2 stages: 35 instead of 30.
+    const bool bare = rvq_stages_one_launch(g) && captured(stream_) && direct_rvq_applicable(g, smem_limit_);
+    if (tensor_enabled_ && stages > 0 && dense_tc_applicable(dim, k, metric) && rvq_stages_pays(g) && !bare) {
         ensure_tc_buffers();
         if (void *work = try_alloc(rvq_stages_bytes(dim, k, stages))) {
             launch_rvq_stages(*this, g, metric == M_EUCLID, work);

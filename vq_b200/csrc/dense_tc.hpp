@@ -64,6 +64,7 @@ void rvq_apply(CudaDevice &dev, const RvqApply &a, const DenseWork &w);
 // The residual encoder with all its stages in one kernel (rvq_tc.cu), for shapes that dense_tc_applicable takes.
 struct GenericParams;
 bool rvq_stages_pays(const GenericParams &g);                        // more rows than direct.cu is faster with
+bool rvq_stages_one_launch(const GenericParams &g);                  // so few that the kernel lays the codebooks out itself
 size_t rvq_stages_bytes(size_t dim, size_t k, size_t stages);        // device memory that it needs
 void launch_rvq_stages(CudaDevice &dev, const GenericParams &g, bool euclid, void *work);
 

@@ -1,5 +1,4 @@
-// rvq_tc.cu -- the residual encoder (src/rvq.rs:171-215) with all its stages in one kernel (and one before it that lays the
-// codebooks out), for the shapes of the tensor-core path.
+// rvq_tc.cu -- the residual encoder (src/rvq.rs:171-215) with all its stages in one kernel, for the shapes of the tensor-core path.
 //
 // A CTA takes 128 rows through every stage: the residuals and the sums of the chosen centroids stay in registers (a warp has eight rows, a
 // lane four dimensions of each), what goes to memory is the input once and the results once.  Per stage
@@ -25,6 +24,8 @@
 // -> 973); 1,000,000 x 64: 2505 -> 2221, x 32: 1589 -> 1507; 1,000,000 x 61, 4 stages: 1422 -> 1280.  What bounds it is the chain of a stage
 // in a CTA, 9,800 cycles with 64 rows and 13,000 with 128: image 1,600 / 2,000, MMAs 3,750 (3,200 of them the tensor core's), scores 1,450 / 2,100,
 // codes 650 (3,100 for a warp with a row that is not decided, for which the others wait), the centroids' way from L2 2,000, norms 450.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <atomic>
 
@@ -60,6 +61,8 @@ struct RvqStagesParams {
     float *frames;   // [stages][F_FLOATS]
     uint16_t *image; // [stages][bn][2 * DIMP]
     float *extra;    // [stages][bn][8] operand B of the half norms, as the tile lies in shared memory
+    int one;         // a cooperative launch, which lays the codebooks out itself
+    int book_vec;    // centroids are whole 16-byte pieces
     uint16_t *out_f16;
     uint32_t *out_codes;
     int *error;
@@ -127,36 +130,33 @@ __device__ __forceinline__ void split_pair(float v0, float v1, uint32_t &h, uint
     h = *reinterpret_cast<const uint32_t *>(&hh), l = *reinterpret_cast<const uint32_t *>(&ll);
 }
 
-constexpr int BT = 1024, BW = BT / 32; // threads and warps of rvq_books_kernel
-
-struct BookShared {
-    alignas(16) float sum[BW][128];
+template <int W> struct BookShared {
+    alignas(16) float sum[W][128];
     alignas(16) float mu[128];
     alignas(16) uint32_t hash[256];
     uint32_t first[256], count, big, hmax;
 };
 
-// Frame, image and half norms of a stage's codebook, a CTA for each.  A centroid that equals one before it in every value never wins
+// Frame, image and half norms of a stage's codebook, by a whole CTA.  A centroid that equals one before it in every value never wins
 // (equal distances, strict '<' in ascending order), so its column is like one beyond k: training on few rows leaves dozens of equal
 // centroids, zeros mostly, and every row that chose one of them would be left to the exact evaluation with all of them.
-// All of it is in registers from one trip to memory on (a warp has every 32nd centroid, a lane four dimensions of each).
-__global__ void __launch_bounds__(BT) rvq_books_kernel(const float *books, int k, int dim, int dimp, int bn, int vec, float *frames, uint16_t *image, float *extra)
+// All of it is in registers from one trip to memory on (a warp has every THREADS / 32nd centroid, a lane four dimensions of each).
+template <int THREADS>
+__device__ __forceinline__ void make_book(BookShared<THREADS / 32> &s, const float *books, int st, int k, int dim, int dimp, int bn, bool vec, float *frames, uint16_t *image, float *extra)
 {
-    constexpr int C = 256 / BW; // centroids of a warp
-    __shared__ BookShared s;
-    next_kernel_may_start();
-    const int st = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int W = THREADS / 32, C = 256 / W; // centroids of a warp
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const float *book = books + (size_t)st * k * dim;
     if (tid == 0) s.count = s.big = s.hmax = 0u;
     if (tid < 256) s.first[tid] = tid;
     float v[C][4], sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int i = 0; i < C; ++i) load4(v[i], book + (size_t)(warp + BW * i) * dim, lane, dim, vec != 0, warp + BW * i < k);
+    for (int i = 0; i < C; ++i) load4(v[i], book + (size_t)(warp + W * i) * dim, lane, dim, vec, warp + W * i < k);
     __syncthreads();
     uint32_t count = 0;
 #pragma unroll
     for (int i = 0; i < C; ++i) {
-        const int j = warp + BW * i;
+        const int j = warp + W * i;
         const float big = fmaxf(fmaxf(fabsf(v[i][0]), fabsf(v[i][1])), fmaxf(fabsf(v[i][2]), fabsf(v[i][3])));
         const bool nan = !(v[i][0] + v[i][1] + v[i][2] + v[i][3] == v[i][0] + v[i][1] + v[i][2] + v[i][3]);
         if (j < k && __all_sync(0xffffffffu, big < 1e37f && !nan)) { // what is not finite has no say
@@ -177,17 +177,17 @@ __global__ void __launch_bounds__(BT) rvq_books_kernel(const float *books, int k
     if (tid < 128) {
         float t = 0.0f;
 #pragma unroll
-        for (int w = 0; w < BW; ++w) t += s.sum[w][tid];
+        for (int w = 0; w < W; ++w) t += s.sum[w][tid];
         const float mu = t / fmaxf((float)s.count, 1.0f);
         s.mu[tid] = fabsf(mu) < VQB_DENSE_INF ? mu : 0.0f;
         fr[tid] = s.mu[tid];
     }
     {
-        const int j = tid & 255, from = (tid >> 8) * (256 / (BT / 256)); // BT / 256 threads look for the first centroid with the same hash
+        const int j = tid & 255, from = (tid >> 8) * (256 / (THREADS / 256)); // THREADS / 256 threads look for the first centroid with the same hash
         const uint32_t mine = s.hash[j];
         int first = 256;
 #pragma unroll 4
-        for (int i = 256 / (BT / 256) - 4; i >= 0; i -= 4) {
+        for (int i = 256 / (THREADS / 256) - 4; i >= 0; i -= 4) {
             const uint4 h = *reinterpret_cast<const uint4 *>(&s.hash[from + i]);
             first = h.w == mine ? from + i + 3 : first, first = h.z == mine ? from + i + 2 : first;
             first = h.y == mine ? from + i + 1 : first, first = h.x == mine ? from + i : first;
@@ -200,11 +200,11 @@ __global__ void __launch_bounds__(BT) rvq_books_kernel(const float *books, int k
     float a[C];
 #pragma unroll
     for (int i = 0; i < C; ++i) {
-        const int j = warp + BW * i;
+        const int j = warp + W * i;
         bool same = j >= k;
         if (!same && s.first[j] < (uint32_t)j) { // equal indeed?
             float w[4];
-            load4(w, book + (size_t)s.first[j] * dim, lane, dim, vec != 0, true);
+            load4(w, book + (size_t)s.first[j] * dim, lane, dim, vec, true);
             same = __all_sync(0xffffffffu, v[i][0] == w[0] && v[i][1] == w[1] && v[i][2] == w[2] && v[i][3] == w[3]);
         }
         gone |= (same ? 1u : 0u) << i;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(BT) rvq_books_kernel(const float *books, int k
     const float beta = power_of_two(eb);
 #pragma unroll
     for (int i = 0; i < C; ++i) {
-        const int j = warp + BW * i;
+        const int j = warp + W * i;
         uint32_t h[2], l[2];
 #pragma unroll
         for (int e = 0; e < 2; ++e) split_pair(gone >> i & 1u ? 0.0f : v[i][2 * e] * beta, gone >> i & 1u ? 0.0f : v[i][2 * e + 1] * beta, h[e], l[e]);
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(BT) rvq_books_kernel(const float *books, int k
             *reinterpret_cast<uint2 *>(o + dimp) = make_uint2(l[0], l[1]);
         }
     }
-    const int j = warp + BW * (lane / LPC);
+    const int j = warp + W * (lane / LPC);
     if (lane % LPC == 0 && j < bn) {
         const float hn = 0.5f * beta * beta * sq;
         if (here) atomicMax(&s.hmax, __float_as_uint(fmaxf(hn, 0.0f))); // (NaN counts as 0)
@@ -294,6 +294,16 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
         for (int i = tid; i < (BM - TILE) * 2; i += NT) reinterpret_cast<uint4 *>(ax_smem + TILE * 32)[i] = make_uint4(0u, 0u, 0u, 0u);
     }
     bool ok = true;
+    if (P.one) { // the codebooks' images by the first CTAs, then all wait for them at the launch's own barrier
+        BookShared<NWARP> &scratch = *reinterpret_cast<BookShared<NWARP> *>(b_smem);
+        for (int st = blockIdx.x; st < P.stages; st += gridDim.x) {
+            make_book<NT>(scratch, P.books, st, k, dim, DIMP, BN, P.book_vec != 0, P.frames, P.image, P.extra);
+            asm volatile("fence.proxy.async;" ::: "memory"); // TMA reads them
+            __syncthreads();
+        }
+        cooperative_groups::this_grid().sync();
+        asm volatile("fence.proxy.async;" ::: "memory");
+    }
     auto load_book = [&](int st) { // by one thread
         mbar_expect_tx(&sh.bars.bfull, kchunks * BOOK_CHUNK<BN> + BN * 32);
         for (int kc = 0; kc < kchunks; ++kc) tma_load_2d(b_smem + (size_t)kc * BOOK_CHUNK<BN>, &map_b, kc * CHUNK, st * BN, &sh.bars.bfull);
@@ -602,7 +612,15 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
     }
 }
 
-template <int KS, int BN, int ROWS> void launch_stages(CudaDevice &dev, const CUtensorMap &map, const RvqStagesParams &p)
+template <int THREADS> __global__ void __launch_bounds__(THREADS) rvq_books_kernel(const float *books, int k, int dim, int dimp, int bn, int vec, float *frames, uint16_t *image, float *extra)
+{
+    __shared__ BookShared<THREADS / 32> sh;
+    next_kernel_may_start();
+    make_book<THREADS>(sh, books, blockIdx.x, k, dim, dimp, bn, vec != 0, frames, image, extra);
+}
+
+// False: a cooperative launch whose CTAs cannot all be resident (SMs that this process may not use)
+template <int KS, int BN, int ROWS> bool launch_stages(CudaDevice &dev, const CUtensorMap &map, const RvqStagesParams &p)
 {
     auto kernel = rvq_stages_kernel<KS, BN, ROWS>;
     constexpr size_t smem = stages_smem<KS, BN>();
@@ -614,20 +632,31 @@ template <int KS, int BN, int ROWS> void launch_stages(CudaDevice &dev, const CU
     }
     const unsigned grid = (unsigned)std::min<unsigned long long>((p.n + NWARP * ROWS - 1) / (NWARP * ROWS), (unsigned long long)dev.sm_count());
     KernelScope ks(dev, "rvq_quantize");
-    launch_following(kernel, grid, NT, smem, dev.stream(), map, p);
+    if (p.one) {
+        void *args[] = {const_cast<CUtensorMap *>(&map), const_cast<RvqStagesParams *>(&p)};
+        const cudaError_t e = cudaLaunchCooperativeKernel((const void *)kernel, dim3(grid), dim3(NT), args, smem, dev.stream());
+        if (e == cudaErrorCooperativeLaunchTooLarge) {
+            cudaGetLastError();
+            return false;
+        }
+        VQB_CUDA_CHECK(e);
+    } else launch_following(kernel, grid, NT, smem, dev.stream(), map, p);
     dev.count_launch();
+    return true;
 }
 
-template <int KS> void launch_ks(CudaDevice &dev, const CUtensorMap &map, const RvqStagesParams &p, int bn)
+template <int KS> bool launch_ks(CudaDevice &dev, const CUtensorMap &map, const RvqStagesParams &p, int bn)
 {
     const bool few = p.n <= (unsigned long long)dev.sm_count() * (BM / 2);
-    if (bn == 256) few ? launch_stages<KS, 256, 4>(dev, map, p) : launch_stages<KS, 256, 8>(dev, map, p);
-    else few ? launch_stages<KS, 128, 4>(dev, map, p) : launch_stages<KS, 128, 8>(dev, map, p);
+    if (bn == 256) return few ? launch_stages<KS, 256, 4>(dev, map, p) : launch_stages<KS, 256, 8>(dev, map, p);
+    return few ? launch_stages<KS, 128, 4>(dev, map, p) : launch_stages<KS, 128, 8>(dev, map, p);
 }
 
 int book_rows(int k) { return k > 128 ? 256 : 128; }
 
 } // namespace
+
+static bool whole_pieces(const GenericParams &g) { return g.sd % 4 == 0 && (reinterpret_cast<uintptr_t>(g.centroids) & 15u) == 0; }
 
 // Against direct.cu (us a call, here / there): a stage takes 3 to 6 us here up to 64 rows per SM whatever the rows, and 17 us come before; there it
 // is the rows' time.  The two meet (256 centroids) at 1300 x 128, 2 stages: 29 / 29; 800 x 96, 4: 39 / 39; 700 x 64, 8: 48 / 48;
@@ -635,8 +664,19 @@ int book_rows(int k) { return k > 128 ? 256 : 128; }
 // one is ahead from 300 rows on, but with codebooks of many equal centroids, which cost it nothing: not a line to draw for others.
 bool rvq_stages_pays(const GenericParams &g)
 {
-    if (!(g.sd % 4 == 0 && (reinterpret_cast<uintptr_t>(g.centroids) & 15u) == 0)) return g.n >= 300;
+    if (!whole_pieces(g)) return g.n >= 300;
     return (double)g.n >= (500.0 + 1600.0 / g.stages) * (g.sd < 64 ? 1.5 : 1.0);
+}
+
+// Up to the rows that direct.cu used to take, the encode stays one launch of one kernel, as callers have it: the first CTAs make the codebooks'
+// images and all wait for them.  They wait at the barrier that every cooperative launch has of its own; counters of the context, which an earlier
+// form had, were also those of a captured encode that is replayed beside other calls.  (All CTAs of such a launch are resident, and none leaves
+// before the barrier.)  4,999 x 128, 8 stages: 67 us (63 in two launches); beyond, where there were several launches a stage, it is two, and no CTA
+// waits for another.
+bool rvq_stages_one_launch(const GenericParams &g)
+{
+    const double rows = (g.k > 128 ? 2.0e6 : g.k > 64 ? 4.6e6 : 6.8e6) / (double)(dense_padded(g.sd) + 32);
+    return (double)g.n <= rows * (whole_pieces(g) ? 1.0 : 0.6);
 }
 
 size_t rvq_stages_bytes(size_t dim, size_t k, size_t stages)
@@ -651,26 +691,35 @@ void launch_rvq_stages(CudaDevice &dev, const GenericParams &g, bool euclid, voi
     const size_t rows = (size_t)g.stages * bn;
     uint16_t *image = static_cast<uint16_t *>(work); // (whole multiples of 16 bytes follow each other)
     float *extra = reinterpret_cast<float *>(image + rows * 2 * dimp), *frames = extra + rows * 8;
-    const bool whole = g.sd % 4 == 0 && (reinterpret_cast<uintptr_t>(g.centroids) & 15u) == 0;
-    {
+    const bool whole = whole_pieces(g);
+    const bool one = rvq_stages_one_launch(g);
+    auto make_books = [&] {
         KernelScope ks(dev, "rvq_books");
-        rvq_books_kernel<<<g.stages, BT, 0, dev.stream()>>>(g.centroids, g.k, g.sd, dimp, bn, whole, frames, image, extra);
+        rvq_books_kernel<1024><<<g.stages, 1024, 0, dev.stream()>>>(g.centroids, g.k, g.sd, dimp, bn, whole, frames, image, extra);
         VQB_CUDA_CHECK(cudaGetLastError());
         dev.count_launch();
-    }
+    };
+    if (!one) make_books();
     const CUtensorMap map = make_tensor_map_2d(image, 2 * (unsigned long long)dimp, rows, CHUNK, (unsigned)bn, CU_TENSOR_MAP_SWIZZLE_128B);
     RvqStagesParams p = {};
     p.x = g.x, p.books = g.centroids, p.n = g.n, p.dim = g.sd, p.k = g.k, p.stages = g.stages, p.euclid = euclid, p.epsilon = g.epsilon;
     p.vec = whole && (reinterpret_cast<uintptr_t>(g.x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(g.out_f16) & 7u) == 0;
-    p.frames = frames, p.image = image, p.extra = extra, p.out_f16 = g.out_f16, p.out_codes = g.out_codes, p.error = dev.error_word();
-    switch (dimp / 16) {
-    case 2: launch_ks<2>(dev, map, p, bn); break;
-    case 3: launch_ks<3>(dev, map, p, bn); break;
-    case 4: launch_ks<4>(dev, map, p, bn); break;
-    case 5: launch_ks<5>(dev, map, p, bn); break;
-    case 6: launch_ks<6>(dev, map, p, bn); break;
-    case 7: launch_ks<7>(dev, map, p, bn); break;
-    default: launch_ks<8>(dev, map, p, bn);
+    p.frames = frames, p.image = image, p.extra = extra, p.book_vec = whole, p.one = one, p.out_f16 = g.out_f16, p.out_codes = g.out_codes, p.error = dev.error_word();
+    auto launch = [&] {
+        switch (dimp / 16) {
+        case 2: return launch_ks<2>(dev, map, p, bn);
+        case 3: return launch_ks<3>(dev, map, p, bn);
+        case 4: return launch_ks<4>(dev, map, p, bn);
+        case 5: return launch_ks<5>(dev, map, p, bn);
+        case 6: return launch_ks<6>(dev, map, p, bn);
+        case 7: return launch_ks<7>(dev, map, p, bn);
+        default: return launch_ks<8>(dev, map, p, bn);
+        }
+    };
+    if (!launch()) {
+        make_books();
+        p.one = 0;
+        launch();
     }
 }
 
