@@ -6,8 +6,9 @@
 //   2. one thread issues the MMAs against the stage's codebook image, which TMA has brought into shared memory (the next stage's
 //      follows as soon as these MMAs are done): D_j = v.c_j - |c_j|^2/2 in tensor memory,
 //   3. sixteen warps look at the 128 x 256 scores: largest one per row, then a mask of the centroids within the error bound,
-//   4. rows with one candidate have their code; the others' candidates are evaluated with the reference's serial f32 chain, a
-//      warp loading whole centroids and one lane per candidate adding up,
+//   4. rows with one candidate have their code; the others' candidates are evaluated with the reference's serial f32 chain: up to
+//      eight by the row's own warp (whole centroids loaded, one lane per candidate adding up), more by all warps together against all
+//      centroids, a row with a value that is not finite not at all (no distance is below +inf: centroid 0),
 //   5. residual, running sum, norm against epsilon.
 // The multi-launch path that this replaces wrote residual, image and norms of every row in every stage (1 KB a row).
 //
@@ -73,6 +74,9 @@ template <int BN> struct Shared { // behind the operand tiles
     float vn2[BM], alpha[BM];    // |v|^2 (upper bound), scale of a row
     uint32_t mask[BM][BN / 32];  // candidates
     uint8_t nan0[BM];
+    uint8_t open[BM];             // rows with many candidates, in any order
+    uint32_t n_open;
+    unsigned long long least[BM]; // of each of them: bits of the smallest distance so far (never negative: ordered like the numbers), its centroid
     RvqBarriers bars;
 };
 
@@ -106,6 +110,13 @@ template <int N, int L> __device__ __forceinline__ float sum_rows(const float (&
         for (int i = 0; i < N / 2; ++i) b[i] = (up ? a[i + N / 2] : a[i]) + __shfl_xor_sync(0xffffffffu, up ? a[i] : a[i + N / 2], L / 2);
         return sum_rows<N / 2, L / 2>(b, lane);
     }
+}
+
+// the reference's serial sum, four terms on
+__device__ __forceinline__ void square_differences(float &d, const float4 &x, const float4 &c)
+{
+    const float e0 = __fsub_rn(x.x, c.x), e1 = __fsub_rn(x.y, c.y), e2 = __fsub_rn(x.z, c.z), e3 = __fsub_rn(x.w, c.w);
+    d = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(d, __fmul_rn(e0, e0)), __fmul_rn(e1, e1)), __fmul_rn(e2, e2)), __fmul_rn(e3, e3));
 }
 
 // exponent that brings a norm, given its square, to [32, 64)
@@ -330,6 +341,14 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
         }
     };
     constexpr int PER = ROWS * 128 / (4 * DIMP); // scratch rows in them
+    // Rows with more candidates than FEW_CANDIDATES (a batch of four takes a warp 2,900 cycles): PASS of them at a time against all centroids, PL
+    // pieces of 16 bytes at a time; a warp has PASS_ROWS of them and 64 centroids, two a lane.  us a call, 8 stages of 256, 128 wide, every row
+    // by its own warp / now / with direct.cu and resolve.cu: 1,500 rows far from all centroids 3,428 / 444 / 563, families of 32 centroids a
+    // rounding apart 450 / 345 / 204, values that are not finite 4,394 / 107 / 569, in 1 % of the rows 768 / 72 / 283; 40,000 rows 17,652 / 3,104 / 19,329,
+    // 2,190 / 2,132 / 4,420, 23,828 / 438 / 19,675, 2,291 / 238 / 3,816.  4 stages of 64 wide, 1,500 rows far 1,013 / 153 / 135.  Rows that are
+    // decided pay 2 % for it (4,999 x 128 67.3 / 69.0, 40,000 211 / 215: registers, a barrier a stage).
+    constexpr int FEW_CANDIDATES = 8, PASS_ROWS = ROWS == 8 ? 4 : 8, PASS = PASS_ROWS * NWARP * 2 / WORDS, PL = KS == 8 ? 8 : kchunks > 1 ? 4 : 2, PC = (PL * BN + NT - 1) / NT;
+    static_assert((4 * KS) % PL == 0 && PASS * 4 * DIMP + PL * BN * 16 <= kchunks * BM * 128, "rows and centroids of a pass lie in operand A");
     constexpr int BATCH = PER * kchunks < 4 ? PER * kchunks : 4; // candidates at a time (eight: 116 bytes of registers spilled, 5 % slower)
     auto scratch = [&](int b, int p) { // 16-byte piece p of scratch row b
         return reinterpret_cast<float4 *>(own + (size_t)(b / PER) * (BM * 128) + (b % PER) * (4 * DIMP)) + (p ^ (b & 3));
@@ -410,6 +429,7 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic writes -> visible to the MMA's reads
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncthreads();
+            if (tid == 0) sh.n_open = 0u;
             // ---- 2. scores
             if (tid == 0 && mbar_wait(&sh.bars.bfull, it & 1u, abort_flag, P.error, 41)) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -498,7 +518,18 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
                 }
 #pragma unroll
                 for (int o = LPR / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o), code = max(code, __shfl_xor_sync(0xffffffffu, code, o));
-                uint32_t open = __ballot_sync(0xffffffffu, live && cnt != 1 && sub == 0);
+                bool many = live && cnt > FEW_CANDIDATES;
+                const bool any_many = __syncthreads_or(many);
+                if (any_many) {
+                    // a value that is not finite leaves no distance below +inf: centroid 0
+#pragma unroll
+                    for (int i = 0; i < NI; ++i) {
+                        const bool off = !(fabsf(v[i][0]) < VQB_DENSE_INF && fabsf(v[i][1]) < VQB_DENSE_INF && fabsf(v[i][2]) < VQB_DENSE_INF && fabsf(v[i][3]) < VQB_DENSE_INF);
+                        const uint32_t lanes = __ballot_sync(0xffffffffu, off) >> (side * L) & (0xFFFFFFFFu >> (32 - L));
+                        if (lanes && piece / LPR == i && many) code = 0, cnt = 1, many = false;
+                    }
+                }
+                uint32_t open = __ballot_sync(0xffffffffu, live && cnt != 1 && !many && sub == 0);
                 while (open) {
                     const int r = row_of(__ffs(open) - 1);
                     open &= open - 1;
@@ -539,6 +570,82 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
                         __syncwarp();
                     }
                     if (own_row == r) code = stuck ? 0 : chosen;
+                }
+                if (any_many) { // all warps look at these rows together (the scratch in operand A is free: dense passes below)
+                    int place = 0;
+                    if (many && sub == 0) {
+                        place = (int)atomicAdd(&sh.n_open, 1u);
+                        sh.open[place] = (uint8_t)(first + own_row);
+                        sh.least[place] = 0xFFFFFFFF00000000ull; // centroid 0 where nothing is below +inf
+                    }
+                    place = __shfl_sync(0xffffffffu, many ? place : 1 << 20, lane - sub);
+                    __syncthreads();
+                    const int n_open = (int)sh.n_open;
+                    float4 *const rows = reinterpret_cast<float4 *>(a_smem), *const planes = rows + PASS * (DIMP / 4); // [PASS][DIMP / 4], [PL][BN]
+                    const int lo = 64 * (warp % (WORDS / 2)), at = PASS_ROWS * (warp / (WORDS / 2)); // this warp's candidates, two a lane, and rows of a pass
+                    for (int pass = 0; pass < n_open; pass += PASS) {
+#pragma unroll
+                        for (int i = 0; i < NI; ++i) {
+                            const int pos = __shfl_sync(0xffffffffu, place, side * L + i * LPR) - pass;
+                            if (pos >= 0 && pos < PASS && 4 * piece < DIMP) rows[pos * (DIMP / 4) + piece] = make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
+                        }
+                        const int here = min(PASS_ROWS, n_open - pass - at); // (below 1: none)
+                        float d[2][PASS_ROWS];
+#pragma unroll
+                        for (int g = 0; g < PASS_ROWS; ++g) d[0][g] = d[1][g] = 0.0f;
+#pragma unroll 1
+                        for (int p0 = 0; p0 < DIMP / 4; p0 += PL) {
+                            float c[PC][4]; // (beyond dim: zeros on both sides, which change no sum of squares)
+#pragma unroll
+                            for (int i = 0; i < PC; ++i) {
+                                const int j = (tid + i * NT) / PL;
+                                load4(c[i], book + (size_t)j * dim, p0 + tid % PL, dim, vec, j < k);
+                            }
+#pragma unroll
+                            for (int i = 0; i < PC; ++i) {
+                                const int j = (tid + i * NT) / PL, p = tid % PL;
+                                if (PL * BN >= NT || j < BN) planes[p * BN + (j ^ p)] = make_float4(c[i][0], c[i][1], c[i][2], c[i][3]);
+                            }
+                            __syncthreads();
+                            if (here > 0 && lo < k) {
+#pragma unroll 1
+                                for (int p = 0; p < PL; ++p) {
+                                    const float4 c0 = planes[p * BN + ((lo + lane) ^ p)], c1 = planes[p * BN + ((lo + 32 + lane) ^ p)];
+                                    const float4 *xp = rows + at * (DIMP / 4) + p0 + p;
+#pragma unroll
+                                    for (int g0 = 0; g0 < PASS_ROWS; g0 += 4) { // (beyond the last row: what lies there, to no effect)
+                                        if (g0 >= here) break;
+                                        float4 x4[4];
+#pragma unroll
+                                        for (int g = 0; g < 4; ++g) x4[g] = xp[(g0 + g) * (DIMP / 4)];
+#pragma unroll
+                                        for (int g = 0; g < 4; ++g) square_differences(d[0][g0 + g], x4[g], c0), square_differences(d[1][g0 + g], x4[g], c1);
+                                    }
+                                }
+                            }
+                            __syncthreads();
+                        }
+#pragma unroll
+                        for (int g = 0; g < PASS_ROWS; ++g) {
+                            if (g >= here || lo >= k) break;
+                            const int pos = pass + at + g;
+                            const uint32_t *mask = &sh.mask[sh.open[pos]][lo >> 5];
+                            uint32_t u = 0xFFFFFFFFu, j = 0u;
+                            bool stuck = false; // the reference's scan starts at centroid 0: a NaN there stays
+#pragma unroll
+                            for (int half = 0; half < 2; ++half) {
+                                const float dist = P.euclid ? __fsqrt_rn(d[half][g]) : d[half][g];
+                                if (!(mask[half] >> lane & 1u)) continue;
+                                if (dist < VQB_DENSE_INF && __float_as_uint(dist) < u) u = __float_as_uint(dist), j = lo + 32 * half + lane;
+                                stuck = stuck || (lo + 32 * half + lane == 0 && !(dist == dist));
+                            }
+                            stuck = __any_sync(0xffffffffu, stuck);
+                            const uint32_t low = __reduce_min_sync(0xffffffffu, u), first_j = __reduce_min_sync(0xffffffffu, u == low ? j : 0xFFFFFFFFu); // of equal ones the first
+                            if (lane == 0 && (stuck || low != 0xFFFFFFFFu)) atomicMin(&sh.least[pos], stuck ? 0ull : (unsigned long long)low << 32 | first_j);
+                        }
+                    }
+                    __syncthreads();
+                    if (many) code = (int)(uint32_t)sh.least[place];
                 }
             }
             if (P.out_codes && sub == 0 && my_row < P.n) P.out_codes[my_row * P.stages + st] = live ? (uint32_t)code : 0xFFFFFFFFu;
