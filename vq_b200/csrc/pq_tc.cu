@@ -35,14 +35,6 @@
 //   the reference's own arithmetic prefers w over a only if D_w <= D_a (1 + 4u) with (sd + 2)u each: 24u * 65300 = 0.1
 //   => T_w <= T_best + 1.5 + 2 * 0.17 + 0.1, i.e. a difference of at most 1.  M = 3 leaves room for twice what was measured.
 //
-// FEW (8-wide, many rows).  Every step reads and writes the whole accumulator, and on large inputs the chip runs at its power limit: the third
-// step cost a tenth of the time (1M x 128, m 16, k 256, back to back at 990 W: encode 475 -> 449 us, fit of 10 iterations 5,340 -> 4,985).  So
-// the constants share a step with the last products, xl.(-ch), and the half norm.  Then eleven addends beside 2^23 have fractions: the
-// accumulator and the eight products, either sign, -2.25 .. 2.25, the half norm's two, never negative, -0.5 .. 0, and the result's unit
-// downwards: error in (-3.75, 2.25) instead of (-1.25, 0.25), measured (tests/test_gpu_pq_two_steps.py) -2.97 .. 1.98.
-//   => T_w <= T_best + 6.0 + 2 * 0.17 + 0.1, i.e. a difference of at most 6: M = 7.  More rows are queued for it: uniform ones 2 % of the time,
-//   64 clusters of standard deviation 0.05 and distance 1 391 -> 497 us for 500,000 rows (of 0.001 1,678 -> 1,460, of 0.3 217 -> 225).
-//
 // Far centroids.  One centroid far from the others would stretch the range for all.  Those farther from mu than four times the
 // mean distance (mu: the mean of the rest, found in up to six rounds) are left out: rho covers the others.  The producers leave a
 // lower bound of what a far one can score against the row, lim^2/2 - lim |x|, in shared memory; a row that has it within reach is
@@ -84,7 +76,11 @@
 //     (16-byte pieces stored from here: 0.49 in all)
 //   * each of the eight fetches its own rows: with one copy of the 128 rows for all, issued by the first of them once the others had used
 //     the buffer up, that warp's 950 cycles for it were the kernel's longest chain (encode 0.353 -> 0.345, training pass 0.366 -> 0.360, short
-//     runs; at the power limit 456 -> 449 us for the encode)
+//     runs)
+// The constant in a step of its own (K = 48) rather than beside the last products (K = 32): eleven cut addends instead of one need M = 7, with
+// 0.6 units to spare for how the tensor core cuts instead of 1.1, and queue up to twice the rows.  Uniform rows are 5 to 7 % faster with two steps
+// (1M x 128, m 16, k 256 at the power limit: encode 477 / 450 us, fit of 10 iterations 5,370 / 5,000), clustered ones slower (500,000 rows in 64
+// clusters, standard deviation 0.05 of their distance: 437 / 589, 4,880 / 6,010; 0.1: 309 / 378, 3,700 / 4,210).
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -131,14 +127,12 @@ template <> struct Slots<4> {
 template <> struct Slots<8> {
     static constexpr int STEPS = 3, NORM = 24, CONST = 32, M = 3;
 };
-// FEW: where the constants stand then, and the window
-constexpr int FEW_CONST = 26, FEW_M = 7;
 template <int SD> constexpr uint32_t A1_BYTES = BM * 64;                            // a stage
-template <int SD, bool FEW> constexpr uint32_t A2_BYTES = Slots<SD>::STEPS == 3 && !FEW ? BM * 32 : 0;
-template <int SD, bool FEW> constexpr uint32_t A_BYTES = A1_BYTES<SD> + A2_BYTES<SD, FEW>;
+template <int SD> constexpr uint32_t A2_BYTES = Slots<SD>::STEPS == 3 ? BM * 32 : 0;
+template <int SD> constexpr uint32_t A_BYTES = A1_BYTES<SD> + A2_BYTES<SD>;
 template <int SD> constexpr uint32_t B1_BYTES = BN * 64;                            // a sub-space
-template <int SD, bool FEW> constexpr uint32_t B2_BYTES = Slots<SD>::STEPS == 3 && !FEW ? BN * 32 : 0;
-template <int SD, bool FEW> constexpr uint32_t B_BYTES = B1_BYTES<SD> + B2_BYTES<SD, FEW>;
+template <int SD> constexpr uint32_t B2_BYTES = Slots<SD>::STEPS == 3 ? BN * 32 : 0;
+template <int SD> constexpr uint32_t B_BYTES = B1_BYTES<SD> + B2_BYTES<SD>;
 template <int SD> constexpr uint32_t RAW_BYTES = 32 * 2 * SD * 4;                   // a producer warp's rows: 32 of them, two sub-spaces wide
 
 struct alignas(8) PqBarriers {
@@ -210,8 +204,8 @@ __device__ __forceinline__ float sqrt_approx(float v)
     return r;
 }
 
-template <int SD, bool FEW>
-constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES<SD, FEW> + 4 * (size_t)A_BYTES<SD, FEW> + 8 * NRAW * (size_t)RAW_BYTES<SD> + 4 * SUB_FLOATS * sizeof(float) +
+template <int SD>
+constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES<SD> + 4 * (size_t)A_BYTES<SD> + 8 * NRAW * (size_t)RAW_BYTES<SD> + 4 * SUB_FLOATS * sizeof(float) +
                               16 * QCAP * sizeof(uint4) + 4 * 4 * BM * sizeof(uint16_t) + sizeof(PqBarriers) + 64;
 
 // What a row contributes besides its (shifted) values: the factor of its operand, the half-norm factor and the two row constants.
@@ -375,7 +369,7 @@ __device__ __noinline__ bool pq_queue_drain(const PqTcParams &Q, const uint4 *qu
 }
 
 // DUMP: diagnostics in place of codes, 1: the chain's result without the fixed-point constants, as scores; 2: T itself and the rows' sigma and K0
-template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP, bool FEW>
+template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP>
 __global__ void __launch_bounds__(NTHREADS, 1)
     pq_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_b1, const __grid_constant__ CUtensorMap map_b2,
                  const __grid_constant__ PqTcParams Q)
@@ -383,14 +377,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     constexpr bool COSINE = METRIC == M_COSINE;
     constexpr int halves = WIDE ? 2 : 1; // accumulator halves that hold centroids
     using SL = Slots<SD>;
-    constexpr int STEPS = FEW ? 2 : SL::STEPS;
-    constexpr uint32_t M = FEW ? FEW_M : SL::M; // scores this close are decided exactly
+    constexpr uint32_t M = SL::M; // scores this close are decided exactly
     extern __shared__ unsigned char smem_raw[];
     const AssignParams &P = Q.a;
     unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char *b_smem = base;                                                    // [4] 64-byte rows, then [4] 32-byte rows
-    unsigned char *a_smem = base + 4 * (size_t)B_BYTES<SD, FEW>;                          // the same
-    unsigned char *raw_smem = a_smem + 4 * (size_t)A_BYTES<SD, FEW>;                      // [8][NRAW] row pieces
+    unsigned char *a_smem = base + 4 * (size_t)B_BYTES<SD>;                          // the same
+    unsigned char *raw_smem = a_smem + 4 * (size_t)A_BYTES<SD>;                      // [8][NRAW] row pieces
     float *sub_s = reinterpret_cast<float *>(raw_smem + 8 * NRAW * (size_t)RAW_BYTES<SD>);  // [4][32]
     uint4 *queues = reinterpret_cast<uint4 *>(sub_s + 4 * SUB_FLOATS);               // [16][QCAP]
     uint16_t *far_s = reinterpret_cast<uint16_t *>(queues + 16 * QCAP);              // [4][4][128] RowFrame::far of four tiles
@@ -420,7 +413,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         bars->abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    for (uint32_t i = threadIdx.x; i < 4 * A_BYTES<SD, FEW> / 16; i += NTHREADS) // the slots that no row uses stay zero
+    for (uint32_t i = threadIdx.x; i < 4 * A_BYTES<SD> / 16; i += NTHREADS) // the slots that no row uses stay zero
         reinterpret_cast<uint4 *>(a_smem)[i] = make_uint4(0u, 0u, 0u, 0u);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (warp == 1) {
@@ -443,10 +436,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // ------------------------------------------------ operand B: the group's sub-spaces, once
         const bool leader = elect_one();
         if (warp == 0 && leader && act) {
-            mbar_expect_tx(&bars->bfull, (uint32_t)here * B_BYTES<SD, FEW>);
+            mbar_expect_tx(&bars->bfull, (uint32_t)here * B_BYTES<SD>);
             for (int ss = 0; ss < here; ++ss) {
                 tma_load_2d(b_smem + (size_t)ss * B1_BYTES<SD>, &map_b1, 0, (g * 4 + ss) * BN, &bars->bfull);
-                if (B2_BYTES<SD, FEW>) tma_load_2d(b_smem + 4 * (size_t)B1_BYTES<SD> + (size_t)ss * B2_BYTES<SD, FEW>, &map_b2, 0, (g * 4 + ss) * BN, &bars->bfull);
+                if (B2_BYTES<SD>) tma_load_2d(b_smem + 4 * (size_t)B1_BYTES<SD> + (size_t)ss * B2_BYTES<SD>, &map_b2, 0, (g * 4 + ss) * BN, &bars->bfull);
             }
         }
         __syncwarp();
@@ -456,9 +449,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         const uint32_t mine = half < halves ? act >> (2 * acc) & 3u : 0u;
         if (mine) {
             bool ok = mbar_wait(&bars->bfull, 0, abort_flag, Q.error, 12);
-            const uint32_t a1 = (smem_u32(a_smem) + 2 * acc * A1_BYTES<SD>) >> 4, a2 = (smem_u32(a_smem) + 4 * A1_BYTES<SD> + 2 * acc * A2_BYTES<SD, FEW>) >> 4;
+            const uint32_t a1 = (smem_u32(a_smem) + 2 * acc * A1_BYTES<SD>) >> 4, a2 = (smem_u32(a_smem) + 4 * A1_BYTES<SD> + 2 * acc * A2_BYTES<SD>) >> 4;
             const uint32_t b1 = (smem_u32(b_smem) + 2 * acc * B1_BYTES<SD> + half * (B1_BYTES<SD> / 2)) >> 4;
-            const uint32_t b2 = (smem_u32(b_smem) + 4 * B1_BYTES<SD> + 2 * acc * B2_BYTES<SD, FEW> + half * (B2_BYTES<SD, FEW> / 2)) >> 4;
+            const uint32_t b2 = (smem_u32(b_smem) + 4 * B1_BYTES<SD> + 2 * acc * B2_BYTES<SD> + half * (B2_BYTES<SD> / 2)) >> 4;
             const uint32_t td = tmem_base + acc * BN + half * 128;
             uint32_t phase = 0; // parity of the tile's phases
             for (uint32_t tile = tile0; ok && tile < n_tiles; tile += tstep, phase ^= 1u) { // (after an abort the next wait fails)
@@ -478,7 +471,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                         const uint32_t o = (uint32_t)h; // 16 halves = 32 bytes = 2 descriptor units per step
                         umma_f16_n128(td, smem_desc_sw64_at(a1 + o * (A1_BYTES<SD> >> 4)), smem_desc_sw64_at(b1 + o * (B1_BYTES<SD> >> 4)), 0u);
                         umma_f16_n128(td, smem_desc_sw64_at(a1 + o * (A1_BYTES<SD> >> 4) + 2), smem_desc_sw64_at(b1 + o * (B1_BYTES<SD> >> 4) + 2), 1u);
-                        if (STEPS == 3) umma_f16_n128(td, smem_desc_sw32_at(a2 + o * (A2_BYTES<SD, FEW> >> 4)), smem_desc_sw32_at(b2 + o * (B2_BYTES<SD, FEW> >> 4)), 1u);
+                        if (SL::STEPS == 3) umma_f16_n128(td, smem_desc_sw32_at(a2 + o * (A2_BYTES<SD> >> 4)), smem_desc_sw32_at(b2 + o * (B2_BYTES<SD> >> 4)), 1u);
                         umma_commit(&bars->tfull[2 * ss + half]);
                         umma_commit(&bars->aempty[ss]);
                     }
@@ -563,9 +556,9 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                     *reinterpret_cast<uint4 *>(row1 + ((0 ^ s1) << 4)) = h4;
                     *reinterpret_cast<uint4 *>(row1 + ((1 ^ s1) << 4)) = h4;
                     *reinterpret_cast<uint4 *>(row1 + ((2 ^ s1) << 4)) = make_uint4(lo[0], lo[1], lo[2 % (SD / 2)], lo[3 % (SD / 2)]);
-                    *reinterpret_cast<uint4 *>(row1 + ((3 ^ s1) << 4)) = make_uint4(cc, FEW ? k0 : 0u, 0u, 0u);
-                    unsigned char *row2 = a_smem + 4 * (size_t)A1_BYTES<SD> + (size_t)ss * A2_BYTES<SD, FEW> + (size_t)r * 32;
-                    if (!FEW) *reinterpret_cast<uint4 *>(row2 + (((r >> 2) & 1) << 4)) = make_uint4(k0, 0u, 0u, 0u);
+                    *reinterpret_cast<uint4 *>(row1 + ((3 ^ s1) << 4)) = make_uint4(cc, 0u, 0u, 0u);
+                    unsigned char *row2 = a_smem + 4 * (size_t)A1_BYTES<SD> + (size_t)ss * A2_BYTES<SD> + (size_t)r * 32;
+                    *reinterpret_cast<uint4 *>(row2 + (((r >> 2) & 1) << 4)) = make_uint4(k0, 0u, 0u, 0u);
                 }
                 if (__float_as_uint(sub[SUB_FLAGS]) & SUB_FAR) far_s[(ss * 4 + (step & 3u)) * BM + r] = (uint16_t)f.far;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // generic writes -> visible to the MMA's reads
@@ -887,7 +880,6 @@ __device__ __forceinline__ void write_operand(const float (&v)[SD], int s, int k
         // zeros: the rows' operands are zero as well, every column ties
     } else if (!mine || far) {
         row[SL::CONST] = f32_to_f16_bits(4096.0f + 28.0f); // 2048 * 28 = 57344
-        if (SD == 8) row[FEW_CONST] = row[SL::CONST];
     } else {
 #pragma unroll
         for (int i = 0; i < SD; ++i) {
@@ -904,7 +896,6 @@ __device__ __forceinline__ void write_operand(const float (&v)[SD], int s, int k
         }
         row[SL::CONST] = f32_to_f16_bits(4096.0f);
         row[SL::CONST + 1] = one;
-        if (SD == 8) row[FEW_CONST] = row[SL::CONST], row[FEW_CONST + 1] = one;
     }
     uint4 *o1 = reinterpret_cast<uint4 *>(scratch + OFF_B1) + ((size_t)s * BN + j) * 4, *o2 = reinterpret_cast<uint4 *>(scratch + OFF_B2) + ((size_t)s * BN + j) * 2;
 #pragma unroll
@@ -993,11 +984,11 @@ struct PqMaps {
     CUtensorMap x, b1, b2;
 };
 
-template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP, bool FEW>
-static void launch_k(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
+template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP = 0>
+static void launch_w(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
 {
-    auto kernel = pq_tc_kernel<SD, TRAIN, METRIC, WIDE, DUMP, FEW>;
-    constexpr size_t smem = PQ_TC_SMEM<SD, FEW>;
+    auto kernel = pq_tc_kernel<SD, TRAIN, METRIC, WIDE, DUMP>;
+    constexpr size_t smem = PQ_TC_SMEM<SD>;
     static std::atomic<unsigned long long> configured{0}; // bit d: the attribute has been set on device d (it is per device and sticky)
     const unsigned long long bit = 1ull << (dev.device() & 63);
     if (!(configured.load(std::memory_order_relaxed) & bit)) {
@@ -1007,17 +998,6 @@ static void launch_k(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, uns
     KernelScope ks(dev, TRAIN ? "assign_train" : "pq_encode");
     launch_following(kernel, grid, NTHREADS, smem, dev.stream(), mp.x, mp.b1, mp.b2, q);
     dev.count_launch();
-}
-
-// Two steps instead of three (FEW in the header) for training passes and encodes of many rows, 8-wide.  us, three / two: encode of 1,500 x 128, m 16,
-// k 256 16.6 / 16.9, 4,000 23.3 / 23.7, 8,000 19.0 / 17.9, 20,000 24.8 / 23.0, 300,000 132.6 / 128.8; fits of 10 iterations, 2,500 rows 474 / 462,
-// 20,000 628 / 609, 100,000 939 / 905.
-constexpr unsigned long long FEW_ENCODE_ROWS = 6000;
-
-template <int SD, bool TRAIN, int METRIC, bool WIDE, int DUMP = 0> static void launch_w(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
-{
-    if (SD == 8 && (TRAIN || q.a.n >= FEW_ENCODE_ROWS)) launch_k<SD, TRAIN, METRIC, WIDE, DUMP, SD == 8>(dev, mp, q, grid);
-    else launch_k<SD, TRAIN, METRIC, WIDE, DUMP, false>(dev, mp, q, grid);
 }
 
 template <int SD, bool TRAIN, int METRIC> static void launch_t(CudaDevice &dev, const PqMaps &mp, const PqTcParams &q, unsigned grid)
