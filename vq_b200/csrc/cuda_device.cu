@@ -1327,7 +1327,7 @@ __global__ void __launch_bounds__(256) accum_pairs_moved_kernel(const float *__r
 // fetch the row in 16-byte pieces and add it to the new cluster's running sums and subtract it from the old one's with
 // 128-bit atomics on global memory.  Few rows move, so neither per-CTA sums (whose clearing and flushing would dominate)
 // nor an ownership split are worth their fixed cost here.
-template <typename CodeT, bool VEC>
+template <typename CodeT>
 __global__ void __launch_bounds__(256) accum_rows_moved_kernel(const float *__restrict__ x, unsigned long long n, unsigned long long ld, int m, int k, int sd,
                                                                CodeT *codes_prev, const CodeT *codes,
                                                                const uint32_t *active, float *sums, uint32_t *counts, int counts_f32)
@@ -1350,18 +1350,10 @@ __global__ void __launch_bounds__(256) accum_rows_moved_kernel(const float *__re
             moved &= moved - 1;
             const uint32_t cw = __shfl_sync(0xffffffffu, was, src), cn = __shfl_sync(0xffffffffu, now, src);
             const float *xr = xs + (r0 + src) * ld;
-            if (VEC) {
-                for (int d = 4 * lane; d < sd; d += 128) {
-                    const float4 v = __ldg(reinterpret_cast<const float4 *>(xr + d));
-                    atomicAdd(reinterpret_cast<float4 *>(gsum + (size_t)cn * sd + d), v);
-                    atomicAdd(reinterpret_cast<float4 *>(gsum + (size_t)cw * sd + d), make_float4(-v.x, -v.y, -v.z, -v.w));
-                }
-            } else {
-                for (int d = lane; d < sd; d += 32) {
-                    const float v = __ldg(xr + d);
-                    atomicAdd(gsum + (size_t)cn * sd + d, v);
-                    atomicAdd(gsum + (size_t)cw * sd + d, -v);
-                }
+            for (int d = 4 * lane; d < sd; d += 128) {
+                const float4 v = __ldg(reinterpret_cast<const float4 *>(xr + d));
+                atomicAdd(reinterpret_cast<float4 *>(gsum + (size_t)cn * sd + d), v);
+                atomicAdd(reinterpret_cast<float4 *>(gsum + (size_t)cw * sd + d), make_float4(-v.x, -v.y, -v.z, -v.w));
             }
             if (lane == 0) {
                 if (counts_f32) {
@@ -1492,16 +1484,12 @@ static bool accumulate_moved_t(CudaDevice &dev, const Shape &sh, const float *x,
     const int m = (int)sh.m, k = (int)sh.k, sd = (int)sh.sd;
     const size_t budget = dev.smem_limit() - 1024;
     const size_t per_sub = (size_t)k * (sd + 2) * sizeof(float); // sums, count changes, touched flags
-    const bool whole = sd % 4 == 0 && sh.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(sums) & 15u) == 0;
-    // Wide rows in no whole 16-byte pieces, for which there are no queues, from 80,000 rows on.  us a pass, all rows / the moved ones, and a fit:
-    // 162,920 x 70, k 256 39 / 19, 2375 -> 1950; 300,000 x 61, k 16 62 / 18, 2124 -> 1512; 700,000 x 33, k 100 127 / 50, 4922 -> 3623; 80,000 x 127,
-    // k 40 23 / 22, 1380 -> 1350; but 66,000 x 99, k 256 25 / 15, 1725 -> 1786 (the copies of sums and codes).
-    if (whole ? sd >= 64 : sd > 32 && sh.n_local >= 80000) {
+    if (sd >= 64 && sd % 4 == 0 && sh.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(sums) & 15u) == 0) {
         const unsigned long long groups = (sh.n_local + 31) / 32;
         const unsigned gx = (unsigned)std::max<unsigned long long>(1, std::min<unsigned long long>((groups + 7) / 8, (unsigned long long)dev.sm_count() * 8 / m + 1));
         KernelScope ks(dev, "accumulate_moved");
-        auto kernel = whole ? accum_rows_moved_kernel<CodeT, true> : accum_rows_moved_kernel<CodeT, false>;
-        kernel<<<dim3(gx, m), 256, 0, dev.stream()>>>(x, sh.n_local, sh.ld, m, k, sd, codes_prev, codes, active, sums, counts, counts_f32);
+        accum_rows_moved_kernel<CodeT><<<dim3(gx, m), 256, 0, dev.stream()>>>(x, sh.n_local, sh.ld, m, k, sd, codes_prev, codes, active, sums, counts,
+                                                                              counts_f32);
         VQB_CUDA_CHECK(cudaGetLastError());
         dev.count_launch();
         return true;
