@@ -8,6 +8,7 @@
 #include <chrono>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include <cstdlib>
@@ -168,6 +169,19 @@ std::string CudaDevice::timing_report()
         out += "\"" + kv.first + "\": {\"launches\": " + std::to_string(kv.second.first) + ", \"ms\": " + std::to_string(kv.second.second) + "}";
     }
     return out + "}";
+}
+
+void allow_shared_memory(const CudaDevice &dev, const void *kernel)
+{
+    static std::mutex mu;
+    static std::vector<std::pair<const void *, int>> done; // (as many as there are kernels that ask, times devices)
+    const std::pair<const void *, int> key(kernel, dev.device());
+    std::lock_guard<std::mutex> lk(mu);
+    if (std::find(done.begin(), done.end(), key) != done.end()) return;
+    cudaFuncAttributes own;
+    VQB_CUDA_CHECK(cudaFuncGetAttributes(&own, kernel));
+    VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(dev.smem_limit() - own.sharedSizeBytes)));
+    done.push_back(key);
 }
 
 // A stream that is being captured into a graph takes no part in the order of calls: an event from outside may not be waited for
@@ -1434,7 +1448,7 @@ static void accumulate_t(CudaDevice &dev, const Shape &sh, const float *x, const
         const size_t smem = (size_t)group * per_sub;
         const int ctas_per_sm = (int)std::max<size_t>(1, std::min<size_t>(2, budget / (smem + 1024)));
         auto kernel = accum_small_kernel<CodeT>;
-        VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_shared_memory(dev, kernel);
         const int threads = 1024;
         const unsigned long long pairs = (unsigned long long)sh.n_local * group;
         const unsigned ny = (unsigned)((m + group - 1) / group);
@@ -1453,7 +1467,7 @@ static void accumulate_t(CudaDevice &dev, const Shape &sh, const float *x, const
     if (owner_smem <= budget && sd % 4 == 0 && sh.ld % 4 == 0 && sd >= 64 && k >= 2 * AO_WARPS && k <= (1 << 24) &&
         (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && getenv("VQB_ACCUM_ATOMICS") == nullptr) {
         auto kernel = accum_owner_kernel<CodeT>;
-        VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)owner_smem));
+        allow_shared_memory(dev, kernel);
         const unsigned long long pieces = (sh.n_local + AO_PIECE - 1) / AO_PIECE;
         unsigned gx = (unsigned)std::min<unsigned long long>(pieces, (unsigned long long)std::max(1, dev.sm_count() / m));
         dim3 grid(std::max(1u, gx), m);
@@ -1464,7 +1478,7 @@ static void accumulate_t(CudaDevice &dev, const Shape &sh, const float *x, const
     }
     if (per_sub <= budget) {
         auto kernel = accum_wide_kernel<CodeT, true>;
-        VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)per_sub));
+        allow_shared_memory(dev, kernel);
         unsigned gx = (unsigned)std::min<unsigned long long>((sh.n_local + 15) / 16, (unsigned long long)std::max(1, dev.sm_count() / m));
         dim3 grid(std::max(1u, gx), m);
         kernel<<<grid, threads, per_sub, st>>>(x, sh.n_local, sh.ld, m, k, sd, codes, active, sums, counts, counts_f32);
@@ -1513,7 +1527,7 @@ static bool accumulate_moved_t(CudaDevice &dev, const Shape &sh, const float *x,
     const size_t smem = (size_t)group * per_sub;
     const int ctas_per_sm = (int)std::max<size_t>(1, std::min<size_t>(2, budget / (smem + 1024)));
     auto kernel = accum_moved_kernel<CodeT>;
-    VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared_memory(dev, kernel);
     const int threads = 1024;
     const unsigned long long pairs = (unsigned long long)sh.n_local * group;
     const unsigned ny = (unsigned)((m + group - 1) / group);

@@ -209,6 +209,12 @@ struct KernelScope {
     }
 };
 
+// Lets a kernel be launched with all the dynamic shared memory that there is beside its own arrays.  Always the same figure, set once: the attribute
+// is the kernel's and not the launch's, so that a thread that sets what its own launch needs takes it away from another one's (two contexts,
+// fits with different numbers of centroids) between that one's call and launch.
+void allow_shared_memory(const CudaDevice &dev, const void *kernel);
+template <typename... P> void allow_shared_memory(const CudaDevice &dev, void (*kernel)(P...)) { allow_shared_memory(dev, reinterpret_cast<const void *>(kernel)); }
+
 // As launch_following (below), in clusters of CTAs along x.
 template <typename... P, typename... A>
 void launch_following_clusters(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, unsigned cluster, cudaStream_t stream, A &&...args)

@@ -151,7 +151,7 @@ void CudaDevice::evaluate_f16(const float *x, const uint16_t *q, size_t n, size_
     {
         KernelScope ks(*this, "recall");
         auto kernel = recall_kernel<32>;
-        VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_shared_memory(*this, kernel);
         kernel<<<(unsigned)queries, 256, smem, stream_>>>(x, q, n, (int)dim, (int)k, step, window, hits);
         VQB_CUDA_CHECK(cudaGetLastError());
         count_launch();

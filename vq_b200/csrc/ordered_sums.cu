@@ -294,7 +294,7 @@ static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const Cod
         KernelScope ks(dev, "ordered_lists");
         auto kernel = ordered_lists_cluster_kernel<CodeT>;
         const size_t smem = sizeof(uint32_t) * (OC_WARPS + 1) * k;
-        if (smem > 40 * 1024) VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        allow_shared_memory(dev, kernel);
         const unsigned per = ((n + OC_CTAS * OC_WARPS - 1) / (OC_CTAS * OC_WARPS) + 31) / 32 * 32;
         launch_following_clusters(kernel, dim3(OC_CTAS, m), OC_THREADS, smem, OC_CTAS, dev.stream(), codes, n, per, m, k, active, start, list);
         dev.count_launch();
@@ -304,8 +304,7 @@ static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const Cod
         launch_following(ordered_hist_kernel<CodeT>, dim3(chunks, m), OL_THREADS, smem, dev.stream(), codes, n, chunk, m, k, active, hist);
         dev.count_launch();
         auto kernel = ordered_lists_kernel<CodeT>;
-        if (OL_WARPS * smem > 48 * 1024)
-            VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(OL_WARPS * smem)));
+        allow_shared_memory(dev, kernel);
         launch_following(kernel, dim3(chunks, m), OL_THREADS, OL_WARPS * smem, dev.stream(), codes, n, chunk, m, k, active, hist, start, list);
         dev.count_launch();
     }
@@ -333,7 +332,7 @@ static void launch_t(CudaDevice &dev, const Shape &sh, const float *x, const Cod
         const size_t rings = sizeof(WalkRing) * OS_WARPS;
         const size_t spread = (size_t)grid.x * grid.y <= (size_t)dev.sm_count() && dev.smem_limit() / 2 > rings ? dev.smem_limit() / 2 - rings : 0;
         auto go = [&](auto kernel) {
-            if (spread) VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spread));
+            if (spread) allow_shared_memory(dev, kernel);
             launch_following(kernel, grid, 32 * OS_WARPS, spread, dev.stream(), x, n, sh.ld, m, k, sd, active, start, list, sums, counts, counts_f32);
         };
         if (w == 4) go(vec ? ordered_sums_kernel<4, true> : ordered_sums_kernel<4, false>);

@@ -216,7 +216,7 @@ Plan plan(size_t m, size_t k, size_t sd, size_t budget)
 template <int LE, int G> void launch(CudaDevice &dev, const QsParams &q, dim3 grid, size_t smem)
 {
     auto kernel = q.prev ? queue_sums_kernel<LE, G, true> : queue_sums_kernel<LE, G, false>;
-    VQB_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_shared_memory(dev, kernel);
     launch_following(kernel, grid, qs_threads(LE), smem, dev.stream(), q);
     dev.count_launch();
 }

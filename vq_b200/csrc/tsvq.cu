@@ -1060,7 +1060,7 @@ static void launch_quantize(CudaDevice &dev, const TsvqTree &t, double p, const 
     const size_t tile_smem = sizeof(float) * TQ_ROWS * (t.dim + 4);
     const bool aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(out_f16) % 16 == 0;
     if (t.dim % 8 == 0 && tile_smem <= 200 * 1024 && aligned && getenv("VQB_TSVQ_SERIAL_WALK") == nullptr) {
-        VQB_CUDA_CHECK(cudaFuncSetAttribute(tsvq_quantize_tile_kernel<METRIC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem));
+        allow_shared_memory(dev, tsvq_quantize_tile_kernel<METRIC>);
         const size_t tiles = (n + TQ_ROWS - 1) / TQ_ROWS;
         const unsigned per_sm = (unsigned)std::max<size_t>(1, std::min<size_t>(8, (220 * 1024) / (tile_smem + 1024)));
         const unsigned grid = (unsigned)std::min<size_t>(tiles, (size_t)dev.sm_count() * per_sm);
