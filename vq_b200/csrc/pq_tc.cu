@@ -56,8 +56,8 @@
 // 128-row tile of one sub-space; it uses one of the two 128 x 256 f32 accumulators, in two halves of 128 columns.
 //   warps 0-3    MMA issuers, one per accumulator half; warp 0 first loads the group's operand-B tiles (TMA, no multicast), warp 1
 //                owns tensor memory
-//   warps 4-11   take their 32 rows of two sub-spaces, which TMA brings into the warp's own two buffers, scale and split the slices and
-//                write operand-A tiles, one stage per sub-space
+//   warps 4-11   take the row tile that TMA has brought into shared memory (two buffers), scale and split the slices (two sub-spaces a
+//                warp) and write operand-A tiles, one stage per sub-space
 //   warps 12-27  epilogue: a team of four warps per sub-space (one row per lane, one TMEM lane quadrant per warp)
 // Every wait is bounded; on expiry the CTA records a code, stops issuing, frees tensor memory and the host raises an error.
 //
@@ -74,13 +74,12 @@
 //     instruction, they keep the L1 cache busy for 256 cycles a unit (0.40)
 //   * an encode leaves one byte per pair; pq_expand_kernel turns them into rows and 32-bit codes with whole-line stores, 0.06 ms
 //     (16-byte pieces stored from here: 0.49 in all)
-//   * each of the eight fetches its own rows: with one copy of the 128 rows for all, issued by the first of them once the others had used
-//     the buffer up, that warp's 950 cycles for it were the kernel's longest chain (encode 0.353 -> 0.345, training pass 0.366 -> 0.360, short
-//     runs)
 // The constant in a step of its own (K = 48) rather than beside the last products (K = 32): eleven cut addends instead of one need M = 7, with
 // 0.6 units to spare for how the tensor core cuts instead of 1.1, and queue up to twice the rows.  Uniform rows are 5 to 7 % faster with two steps
-// (1M x 128, m 16, k 256 at the power limit: encode 477 / 450 us, fit of 10 iterations 5,370 / 5,000), clustered ones slower (500,000 rows in 64
-// clusters, standard deviation 0.05 of their distance: 437 / 589, 4,880 / 6,010; 0.1: 309 / 378, 3,700 / 4,210).
+// (1M x 128, m 16, k 256 at the power limit: encode 469 / 442 us, fit of 10 iterations 5,300 / 4,960), clustered ones slower (500,000 rows in 64
+// clusters, standard deviation 0.05 of their distance: 443 / 589, 4,890 / 6,010; 0.1: 321 / 378, 3,750 / 4,210).  Rows that each producer warp fetches
+// for itself instead of one copy for all eight gained nothing with three steps (1M 466.7 / 466.0) and cost short calls 4 % (cosine, 60,001 x 96, k 200:
+// 36.7 / 35.1).
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
@@ -96,7 +95,6 @@ namespace vqb {
 namespace {
 
 constexpr int BM = (int)PQ_TC_TILE, BN = 256, MAXM = 64, NTHREADS = 32 * (4 + 8 + 16);
-constexpr int NRAW = 2; // row buffers of a producer warp
 constexpr int QCAP = 64; // queue entries per epilogue warp: fewer than 32 wait, at most 32 are added at a time
 constexpr float COS_MIN = 1e-17f, COS_MAX = 1e18f;  // cosine: norms that the scores can be trusted for
 constexpr float RHO_MIN = 1e-14f, RHO_MAX = 1e15f;  // Euclidean: radii for which neither 2^+-96 scalings nor distances leave f32
@@ -133,10 +131,10 @@ template <int SD> constexpr uint32_t A_BYTES = A1_BYTES<SD> + A2_BYTES<SD>;
 template <int SD> constexpr uint32_t B1_BYTES = BN * 64;                            // a sub-space
 template <int SD> constexpr uint32_t B2_BYTES = Slots<SD>::STEPS == 3 ? BN * 32 : 0;
 template <int SD> constexpr uint32_t B_BYTES = B1_BYTES<SD> + B2_BYTES<SD>;
-template <int SD> constexpr uint32_t RAW_BYTES = 32 * 2 * SD * 4;                   // a producer warp's rows: 32 of them, two sub-spaces wide
+template <int SD> constexpr uint32_t RAW_BYTES = BM * 4 * SD * 4;                   // a row tile
 
 struct alignas(8) PqBarriers {
-    unsigned long long afull[4], aempty[4], bfull, rfull[8][NRAW]; // a...: per sub-space; r...: per producer warp's row buffer
+    unsigned long long afull[4], aempty[4], bfull, rfull[2], rempty[2]; // a...: per sub-space; r...: per row-tile buffer
     unsigned long long tfull[8], tempty[8];                             // [2 ss + half]
     uint32_t tmem_base;
     int abort_flag;
@@ -205,7 +203,7 @@ __device__ __forceinline__ float sqrt_approx(float v)
 }
 
 template <int SD>
-constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES<SD> + 4 * (size_t)A_BYTES<SD> + 8 * NRAW * (size_t)RAW_BYTES<SD> + 4 * SUB_FLOATS * sizeof(float) +
+constexpr size_t PQ_TC_SMEM = 1024 + 4 * (size_t)B_BYTES<SD> + 4 * (size_t)A_BYTES<SD> + 2 * (size_t)RAW_BYTES<SD> + 4 * SUB_FLOATS * sizeof(float) +
                               16 * QCAP * sizeof(uint4) + 4 * 4 * BM * sizeof(uint16_t) + sizeof(PqBarriers) + 64;
 
 // What a row contributes besides its (shifted) values: the factor of its operand, the half-norm factor and the two row constants.
@@ -377,14 +375,13 @@ __global__ void __launch_bounds__(NTHREADS, 1)
     constexpr bool COSINE = METRIC == M_COSINE;
     constexpr int halves = WIDE ? 2 : 1; // accumulator halves that hold centroids
     using SL = Slots<SD>;
-    constexpr uint32_t M = SL::M; // scores this close are decided exactly
     extern __shared__ unsigned char smem_raw[];
     const AssignParams &P = Q.a;
     unsigned char *base = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char *b_smem = base;                                                    // [4] 64-byte rows, then [4] 32-byte rows
     unsigned char *a_smem = base + 4 * (size_t)B_BYTES<SD>;                          // the same
-    unsigned char *raw_smem = a_smem + 4 * (size_t)A_BYTES<SD>;                      // [8][NRAW] row pieces
-    float *sub_s = reinterpret_cast<float *>(raw_smem + 8 * NRAW * (size_t)RAW_BYTES<SD>);  // [4][32]
+    unsigned char *raw_smem = a_smem + 4 * (size_t)A_BYTES<SD>;                      // [2] row tiles
+    float *sub_s = reinterpret_cast<float *>(raw_smem + 2 * (size_t)RAW_BYTES<SD>);  // [4][32]
     uint4 *queues = reinterpret_cast<uint4 *>(sub_s + 4 * SUB_FLOATS);               // [16][QCAP]
     uint16_t *far_s = reinterpret_cast<uint16_t *>(queues + 16 * QCAP);              // [4][4][128] RowFrame::far of four tiles
     PqBarriers *bars = reinterpret_cast<PqBarriers *>(far_s + 4 * 4 * BM);
@@ -404,7 +401,10 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             mbar_init(&bars->afull[s], 4);
             mbar_init(&bars->aempty[s], halves); // one commit per accumulator half
         }
-        for (int b = 0; b < 8 * NRAW; ++b) mbar_init(&bars->rfull[0][b], 1);
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&bars->rfull[b], 1);
+            mbar_init(&bars->rempty[b], 8);
+        }
         mbar_init(&bars->bfull, 1);
         for (int b = 0; b < 8; ++b) {
             mbar_init(&bars->tfull[b], 1);
@@ -483,22 +483,20 @@ __global__ void __launch_bounds__(NTHREADS, 1)
         // ------------------------------------------------ operand A: scaled and split row slices
         const int r = (warp & 3) * 32 + lane; // row of the tile
         const int pair = (warp - 4) >> 2;     // this warp's sub-spaces: 2 pair, 2 pair + 1
-        const uint32_t mine = act >> (2 * pair) & 3u;
-        unsigned char *const raw0 = raw_smem + (size_t)(warp - 4) * NRAW * RAW_BYTES<SD>;
-        unsigned long long *const full = bars->rfull[warp - 4];
-        auto load_rows = [&](uint32_t tile, uint32_t buf) { // rows and columns beyond the matrix arrive as zeros
-            mbar_expect_tx(&full[buf], RAW_BYTES<SD>);
-            tma_load_2d(raw0 + buf * RAW_BYTES<SD>, &map_x, (g * 4 + 2 * pair) * SD, (int)(tile * BM) + (warp & 3) * 32, &full[buf]);
+        auto load_tile = [&](uint32_t tile, uint32_t buf) { // rows and columns beyond the matrix arrive as zeros
+            mbar_expect_tx(&bars->rfull[buf], RAW_BYTES<SD>);
+            tma_load_2d(raw_smem + buf * RAW_BYTES<SD>, &map_x, g * 4 * SD, (int)(tile * BM), &bars->rfull[buf]);
         };
-        if (lane == 0 && mine)
-            for (uint32_t b = 0; b < NRAW; ++b)
-                if (tile0 + b * tstep < n_tiles) load_rows(tile0 + b * tstep, b);
+        if (warp == 4 && lane == 0 && act) {
+            if (tile0 < n_tiles) load_tile(tile0, 0);
+            if (tile0 + tstep < n_tiles) load_tile(tile0 + tstep, 1);
+        }
         __syncwarp();
-        uint32_t step = 0, buf = 0, rphase = 0; // tiles so far (parity: that of the stages); row buffer and its parity
+        uint32_t step = 0, buf = 0, rphase = 0; // tiles so far (parity: that of the stages); row-tile buffer and its parity
         bool ok = true;
-        for (uint32_t tile = tile0; mine && ok && tile < n_tiles; tile += tstep, ++step) {
-            if (!mbar_wait(&full[buf], rphase, abort_flag, Q.error, 10)) break;
-            const unsigned char *raw = raw0 + buf * RAW_BYTES<SD> + lane * (8 * SD);
+        for (uint32_t tile = tile0; act && ok && tile < n_tiles; tile += tstep, ++step) {
+            if (!mbar_wait(&bars->rfull[buf], rphase, abort_flag, Q.error, 10)) break;
+            const unsigned char *raw = raw_smem + buf * RAW_BYTES<SD> + r * (16 * SD);
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int ss = 2 * pair + h;
@@ -508,8 +506,8 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 F2 y[SD / 2];
 #pragma unroll
                 for (int c = 0; c < SD / 4; ++c) {
-                    const int chunk = h * (SD / 4) + c;
-                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(raw + ((SD == 8 ? chunk ^ ((lane >> 1) & 3) : chunk ^ ((lane >> 2) & 1)) << 4));
+                    const int chunk = ss * (SD / 4) + c;
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(raw + ((SD == 8 ? chunk ^ (r & 7) : chunk ^ ((r >> 1) & 3)) << 4));
                     y[2 * c] = v.x, y[2 * c + 1] = v.y;
                     if (!COSINE) {
                         const ulonglong2 mu = reinterpret_cast<const ulonglong2 *>(sub)[c]; // the mean with its sign changed
@@ -566,16 +564,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 if (lane == 0) mbar_arrive(&bars->afull[ss]);
             }
             if (!ok) break;
-            __syncwarp(); // the rows are read
-            if (lane == 0 && tile + NRAW * tstep < n_tiles) load_rows(tile + NRAW * tstep, buf);
-            if (++buf == NRAW) buf = 0, rphase ^= 1u;
-        }
-        // after an abort: rows that are still on their way land before the CTA goes (bounded waits, at once where they are there)
-        if (*abort_flag)
-            for (uint32_t b = 0; mine && b < NRAW; ++b) {
-                mbar_wait(&full[buf], rphase, abort_flag, Q.error, 17);
-                if (++buf == NRAW) buf = 0, rphase ^= 1u;
+            // the row tile is used up: once all eight warps say so, its buffer takes the tile after the next
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->rempty[buf]);
+            if (warp == 4 && tile + 2 * tstep < n_tiles) {
+                ok = mbar_wait(&bars->rempty[buf], rphase, abort_flag, Q.error, 17);
+                if (ok && lane == 0) load_tile(tile + 2 * tstep, buf);
+                __syncwarp();
             }
+            buf ^= 1u;
+            if (buf == 0) rphase ^= 1u;
+        }
     } else {
         // ------------------------------------------------ epilogue: team (warp - 12) / 4 serves that sub-space of the group
         const int q = warp & 3; // TMEM lane quadrant
@@ -665,12 +664,12 @@ __global__ void __launch_bounds__(NTHREADS, 1)
             }
             const uint32_t best = min(best2 & 0xFFFFu, best2 >> 16);
             const uint32_t minus = ((0u - best) & 0xFFFFu) * 0x10001u; // adding it: the distance from the best, never negative
-            constexpr uint32_t MM = M * 0x10001u;
+            constexpr uint32_t MM = SL::M * 0x10001u;
             // Sums of weight * min(distance, M) over the blocks (weight W0 + block) and over the classes (W0 + class), both halves of a word
             // at once.  What they lack of M times all weights is the sum of weight * (M - distance) over those within M: one with distance 0
             // gives M weights, two or more at least W0 (M + 1) > M (W0 + 15).
-            constexpr uint32_t W0 = 16 * M, NBLK = 8 * halves;
-            constexpr uint32_t WB = 2 * M * (NBLK * W0 + NBLK * (NBLK - 1) / 2), WA = M * (16 * W0 + 120);
+            constexpr uint32_t W0 = 16 * SL::M, NBLK = 8 * halves;
+            constexpr uint32_t WB = 2 * SL::M * (NBLK * W0 + NBLK * (NBLK - 1) / 2), WA = SL::M * (16 * W0 + 120);
             uint32_t sb = 0, sb1 = 0, sa = 0, sa1 = 0;
 #pragma unroll
             for (uint32_t i = 0; i < NBLK; i += 2) {
@@ -683,17 +682,17 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                 sa1 = __dp2a_lo(__viaddmin_u16x2(ga[i + 1], minus, MM), (W0 + 2 * i + 2) + ((W0 + 2 * i + 3) << 8), sa1);
             }
             const uint32_t lb = WB - sb - sb1, la = WA - sa - sa1;
-            const uint32_t idx = ((lb * 16u + la - M * 17u * W0) / M) & 0xFFu; // 16 block + class
+            const uint32_t idx = ((lb * 16u + la - SL::M * 17u * W0) / SL::M) & 0xFFu; // 16 block + class
             const bool whole = best - 1u >= T_HIGH - 1u; // 0: nothing to tell apart; high up: nothing but columns without a centroid
-            bool single = max(lb, la) <= M * (W0 + 15u) && !whole;
+            bool single = max(lb, la) <= SL::M * (W0 + 15u) && !whole;
             // a far centroid may be as close (the entry is written again four tiles on, which takes this unit's end)
-            const bool far = any_far && best + M > far_s[(ss * 4 + (step & 3u)) * BM + r];
+            const bool far = any_far && best + SL::M > far_s[(ss * 4 + (step & 3u)) * BM + r];
             single = single && !far;
             const bool later = valid && !single;
             const uint32_t vote = __ballot_sync(0xffffffffu, later);
             if (vote) {
                 // one bit per half of a word: min(distance, M) + (65536 - M) wraps to 0 for M and stays at least 1 otherwise
-                constexpr uint32_t LESS = (0x10000u - M) * 0x10001u;
+                constexpr uint32_t LESS = (0x10000u - SL::M) * 0x10001u;
                 uint32_t blocks = 0, classes = 0;
 #pragma unroll
                 for (int c = 0; c < 2 * halves; ++c) { // four words at a time: eight bits, weighted by the bytes of dp2a
@@ -1066,7 +1065,7 @@ void launch_pq_tc(CudaDevice &dev, const AssignParams &p, int metric, bool train
     PqMaps mp;
     mp.b1 = b.maps->b1, mp.b2 = b.maps->b2;
     // the rows as they lie: a box is one tile of a group's columns
-    mp.x = make_tensor_map_2d(p.x, (unsigned long long)p.m * p.sd, p.n, 2 * p.sd, 32, p.sd == 8 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, p.ld);
+    mp.x = make_tensor_map_2d(p.x, (unsigned long long)p.m * p.sd, p.n, 4 * p.sd, BM, p.sd == 8 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, p.ld);
     PqTcParams q = {};
     q.a = p;
     if (!train) q.a.codes = b.codes;
