@@ -343,10 +343,10 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
     constexpr int PER = ROWS * 128 / (4 * DIMP); // scratch rows in them
     // Rows with more candidates than FEW_CANDIDATES (a batch of four takes a warp 2,900 cycles): PASS of them at a time against all centroids, PL
     // pieces of 16 bytes at a time; a warp has PASS_ROWS of them and 64 centroids, two a lane.  us a call, 8 stages of 256, 128 wide, every row
-    // by its own warp / now / with direct.cu and resolve.cu: 1,500 rows far from all centroids 3,428 / 444 / 563, families of 32 centroids a
-    // rounding apart 450 / 345 / 204, values that are not finite 4,394 / 107 / 569, in 1 % of the rows 768 / 72 / 283; 40,000 rows 17,652 / 3,104 / 19,329,
-    // 2,190 / 2,132 / 4,420, 23,828 / 438 / 19,675, 2,291 / 238 / 3,816.  4 stages of 64 wide, 1,500 rows far 1,013 / 153 / 135.  Rows that are
-    // decided pay 2 % for it (4,999 x 128 67.3 / 69.0, 40,000 211 / 215: registers, a barrier a stage).
+    // by its own warp / now / with direct.cu and resolve.cu: 1,500 rows far from all centroids 3,428 / 455 / 563, families of 32 centroids a
+    // rounding apart 450 / 358 / 204, values that are not finite 4,394 / 107 / 569, in 1 % of the rows 768 / 72 / 283; 40,000 rows 17,652 / 3,043 / 19,329,
+    // 2,190 / 2,080 / 4,420, 23,828 / 428 / 19,675, 2,291 / 215 / 3,816.  4 stages of 64 wide, 1,500 rows far 1,013 / 151 / 135.  Rows that are
+    // decided: 4,999 x 128 67.1 / 68.6, 40,000 210 / 207 (this code in line with the rest instead of behind __builtin_expect 215).
     constexpr int FEW_CANDIDATES = 8, PASS_ROWS = ROWS == 8 ? 4 : 8, PASS = PASS_ROWS * NWARP * 2 / WORDS, PL = KS == 8 ? 8 : kchunks > 1 ? 4 : 2, PC = (PL * BN + NT - 1) / NT;
     static_assert((4 * KS) % PL == 0 && PASS * 4 * DIMP + PL * BN * 16 <= kchunks * BM * 128, "rows and centroids of a pass lie in operand A");
     constexpr int BATCH = PER * kchunks < 4 ? PER * kchunks : 4; // candidates at a time (eight: 116 bytes of registers spilled, 5 % slower)
@@ -478,6 +478,7 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
                 ok = false;
                 break;
             }
+            int found = 0; // candidates in this thread's columns
             if (mine_q) {
                 const float best = -fmaxf(fmaxf(sh.part[0][er], sh.part[1][er]), fmaxf(sh.part[2][er], sh.part[3][er])); // smallest score
                 const float *fr = P.frames + (size_t)st * F_FLOATS;
@@ -500,11 +501,13 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
                     for (int i = 0; i < 32; ++i) m = __funnelshift_l(__float_as_uint(__uint_as_float(t[i]) - lim_d), m, 1);
                     const int lo = quarter * COLS + c;
                     const uint32_t in_range = k >= lo + 32 ? 0xFFFFFFFFu : k > lo ? (1u << (k - lo)) - 1u : 0u;
-                    sh.mask[er][lo >> 5] = (scan_all ? 0xFFFFFFFFu : ~__brev(m)) & in_range;
+                    const uint32_t word = (scan_all ? 0xFFFFFFFFu : ~__brev(m)) & in_range;
+                    sh.mask[er][lo >> 5] = word;
+                    found += __popc(word);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncthreads();
+            const bool maybe_many = __syncthreads_or(found > FEW_CANDIDATES / 4); // (more than that in all four quarters: one has more than a fourth)
             // ---- 4. codes: a row's lanes look at its mask
             const float *book = P.books + (size_t)st * k * dim;
             int code = -1;
@@ -518,9 +521,10 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
                 }
 #pragma unroll
                 for (int o = LPR / 2; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o), code = max(code, __shfl_xor_sync(0xffffffffu, code, o));
-                bool many = live && cnt > FEW_CANDIDATES;
-                const bool any_many = __syncthreads_or(many);
-                if (any_many) {
+                bool many = false, any_many = false;
+                if (__builtin_expect(maybe_many, 0)) {
+                    many = live && cnt > FEW_CANDIDATES;
+                    any_many = __syncthreads_or(many);
                     // a value that is not finite leaves no distance below +inf: centroid 0
 #pragma unroll
                     for (int i = 0; i < NI; ++i) {
@@ -571,7 +575,7 @@ __global__ void __launch_bounds__(NT, 1) rvq_stages_kernel(const __grid_constant
                     }
                     if (own_row == r) code = stuck ? 0 : chosen;
                 }
-                if (any_many) { // all warps look at these rows together (the scratch in operand A is free: dense passes below)
+                if (__builtin_expect(any_many, 0)) { // all warps look at these rows together (the scratch in operand A is free: dense passes below)
                     int place = 0;
                     if (many && sub == 0) {
                         place = (int)atomicAdd(&sh.n_open, 1u);
