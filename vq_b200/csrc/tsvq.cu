@@ -11,7 +11,8 @@
 //
 // The levels follow each other without the host: the device numbers the children and lays out the next level, the host
 // launches for as many nodes as the level can have and surplus CTAs leave at once.  Per level: centroids and spreads (one warp per
-// node and 32 dimensions where nodes are small; chunk sums, means and a streaming kernel where they are large), split_kernel (split
+// node and 32 dimensions where nodes have fewer than 150 rows, a CTA up to 2048; chunk sums, a CTA per 1024 rows, means and a streaming kernel
+// above), split_kernel (split
 // dimension, keys, median by radix selection, stable partition; one cluster of CTAs per node), next_level_kernel.  A full
 // 64-bit sort of all rows per level, and two round trips to the host, took 0.16 + 0.08 ms of the 0.39 ms of a level of 100,000 x 128.
 // The build is not sharded: every rank of a multi-GPU job builds the same tree.
