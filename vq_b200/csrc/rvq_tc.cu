@@ -20,7 +20,7 @@
 //   limit = S_min + 2 E + 1.05 (dim + 6) 2^-24 (|v|^2 / rho + 2 S_min + 2 E)
 // alpha is kept within 2^-60 .. 2^20 of beta: |v|^2 / rho and rho |c|^2 stay far inside f32.
 //
-// Measured (us a call, before -> now; 128 values, 256 centroids, 8 stages): 4,999 rows 193 -> 64, 12,000 rows 466 -> 84, 40,000 rows 912 -> 201,
+// Measured (us a call, before -> now; 128 values, 256 centroids, 8 stages): 4,999 rows 193 -> 66, 12,000 rows 466 -> 83, 40,000 rows 912 -> 200,
 // 1,000,000 rows 16,200 -> 3,340 (in these codebooks dozens of centroids are equal; 2 stages, few equal ones: 48 -> 29, 102 -> 35, 125 -> 66, 1121
 // -> 973); 1,000,000 x 64: 2505 -> 2221, x 32: 1589 -> 1507; 1,000,000 x 61, 4 stages: 1422 -> 1280.  What bounds it is the chain of a stage
 // in a CTA, 9,800 cycles with 64 rows and 13,000 with 128: image 1,600 / 2,000, MMAs 3,750 (3,200 of them the tensor core's), scores 1,450 / 2,100,
